@@ -69,6 +69,9 @@ SIGNATURES = {
     "f2c_pairwise_distance": [p, p, p, i64, i64, i64, ci, p],
     "f2c_kmeans_assign_workspace": [i64, i64, i64],
     "f2c_kmeans_assign": [p, p, p, i64, i64, i64, ci, p, p],
+    "f2c_kmeans_fit_workspace": [i64, i64, i64],
+    "f2c_kmeans_fit_begin": [p, i64, i64, i64, p, p],
+    "f2c_kmeans_fit_iterate": [p, p, i64, i64, i64, ci, C.c_double, ci, p, p],
     "f2c_kmeans_assign_static": [p, p, p, i64, i64, i64, ci, p],
     "f2c_kmeans_assign_static_status": [p, p, p],
     "f2c_device_status": [p, p],
@@ -83,7 +86,8 @@ SIGNATURES = {
     "f2c_last_error": [],
     "f2c_version": [],
 }
-_RESTYPE = {"f2c_last_error": C.c_char_p, "f2c_kmeans_assign_workspace": C.c_int64, "f2c_relabel_capacity": C.c_int64,
+_RESTYPE = {"f2c_last_error": C.c_char_p, "f2c_kmeans_assign_workspace": C.c_int64, "f2c_kmeans_fit_workspace": C.c_int64,
+            "f2c_relabel_capacity": C.c_int64,
             "f2c_sample_block_workspace": C.c_int64, "f2c_peer_hot_first_cold_id": C.c_int64}
 
 for _name, _args in SIGNATURES.items():

@@ -25,7 +25,8 @@ __device__ __forceinline__ float finish_cosine(float dot, float xx, float cc) {
 template <int METRIC, bool WRITE_DIST, bool WRITE_LABEL>
 __global__ void __launch_bounds__(256) kmeans_warp_kernel(const float* __restrict__ x, const float* __restrict__ y,
                                                           float* __restrict__ dist, int64_t* __restrict__ labels, int64_t n,
-                                                          int k, int d) {
+                                                          int k, int d, const int32_t* done) {
+  if (done != nullptr && *(volatile const int32_t*)done != 0) return;
   const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -70,14 +71,10 @@ __global__ void __launch_bounds__(256) kmeans_warp_kernel(const float* __restric
 // Centres are staged KC at a time as [KC][DMAX] (zero padded) plus their squared norms.
 template <int DMAX, int METRIC>
 __global__ void __launch_bounds__(256) kmeans_thread_kernel(const float* __restrict__ x, const float* __restrict__ y,
-                                                            int64_t* __restrict__ labels, const int32_t* __restrict__ subset,
-                                                            const int32_t* __restrict__ count_dev, int64_t n, int k, int d, int kc) {
+                                                            int64_t* __restrict__ labels, const int32_t* __restrict__ subset, int64_t n,
+                                                            int k, int d, int kc, const int32_t* done) {
+  if (done != nullptr && *(volatile const int32_t*)done != 0) return;  // a fit that has converged (kmeans_fit.cu)
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  // count_dev != nullptr: the number of listed points is only known on the device; a small grid walks the list
-  if (count_dev != nullptr) {
-    const int64_t cnt = *count_dev;
-    n = cnt < n ? cnt : n;
-  }
   float* yc_s = reinterpret_cast<float*>(smem_raw);  // [kc][DMAX]
   float* cc_s = yc_s + (size_t)kc * DMAX;            // [kc]
   for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n; base += (int64_t)gridDim.x * blockDim.x) {
@@ -133,24 +130,145 @@ __global__ void __launch_bounds__(256) kmeans_thread_kernel(const float* __restr
   }
 }
 
+// ---------------------------------------------------------------- listed points
+// Exact scores of the points the tensor-core kernel left undecided: a list whose length only the device knows, usually a
+// few hundred points.  The centres are staged once per CTA (rows padded by 16 bytes: eight lanes that read one 16-byte
+// piece of eight different centres touch eight bank groups).  A short list is worked one warp per point, lanes over the
+// centres, so that its latency is k / 32 centres instead of k (256 centres of 32 dimensions: 17 us of dependent FMAs in one
+// thread before); a list longer than the grid's warps could take in kShortRounds rounds goes one thread per point, where a
+// centre is read once for 32 points.  Both add a centre's terms in the order of kmeans_thread_kernel: same distances.
+constexpr int kListThreads = 256;
+constexpr int kShortRounds = 32;
+
+template <int DMAX, int METRIC>
+__global__ void __launch_bounds__(kListThreads) kmeans_listed_kernel(const float* __restrict__ x, const float* __restrict__ y,
+                                                                     int64_t* __restrict__ labels, const int32_t* __restrict__ list,
+                                                                     const int32_t* __restrict__ count_dev, int64_t max_count, int k, int d,
+                                                                     int kc) {
+  constexpr int STRIDE = DMAX + 4;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int64_t cnt = *count_dev < max_count ? *count_dev : max_count;
+  const int lane = threadIdx.x & 31;
+  const int64_t warp = ((int64_t)blockIdx.x * kListThreads + threadIdx.x) >> 5, n_warps = ((int64_t)gridDim.x * kListThreads) >> 5;
+  const bool by_warp = cnt <= n_warps * kShortRounds && kc >= k;
+  if (by_warp ? (int64_t)blockIdx.x * (kListThreads / 32) >= cnt : (int64_t)blockIdx.x * kListThreads >= cnt) return;
+  float* yc_s = reinterpret_cast<float*>(smem_raw);  // [kc][STRIDE]
+  float* cc_s = yc_s + (size_t)kc * STRIDE;          // [kc]
+  auto stage = [&](int c0, int nc) {
+    for (int e = threadIdx.x; e < nc * DMAX; e += kListThreads) {
+      const int c = e / DMAX, t = e - c * DMAX;
+      yc_s[c * STRIDE + t] = t < d ? __ldg(y + (int64_t)(c0 + c) * d + t) : 0.0f;
+    }
+    __syncthreads();
+    if (METRIC == F2C_COSINE) {
+      for (int c = threadIdx.x; c < nc; c += kListThreads) {
+        float cc = 0.0f;
+#pragma unroll
+        for (int t = 0; t < DMAX; ++t) cc = fmaf(yc_s[c * STRIDE + t], yc_s[c * STRIDE + t], cc);
+        cc_s[c] = cc;
+      }
+      __syncthreads();
+    }
+  };
+  auto distance = [&](const float (&xr)[DMAX], float xx, int c) {
+    const float4* yc4 = reinterpret_cast<const float4*>(yc_s + (size_t)c * STRIDE);
+    float acc = 0.0f;
+#pragma unroll
+    for (int q = 0; q < DMAX / 4; ++q) {
+      const float4 b = yc4[q];
+      if (METRIC == F2C_L2) {
+        const float d0 = xr[4 * q] - b.x, d1 = xr[4 * q + 1] - b.y, d2 = xr[4 * q + 2] - b.z, d3 = xr[4 * q + 3] - b.w;
+        acc = fmaf(d0, d0, acc); acc = fmaf(d1, d1, acc); acc = fmaf(d2, d2, acc); acc = fmaf(d3, d3, acc);
+      } else {
+        acc = fmaf(xr[4 * q], b.x, acc); acc = fmaf(xr[4 * q + 1], b.y, acc);
+        acc = fmaf(xr[4 * q + 2], b.z, acc); acc = fmaf(xr[4 * q + 3], b.w, acc);
+      }
+    }
+    const float v = METRIC == F2C_L2 ? acc : finish_cosine(acc, xx, cc_s[c]);
+    return v != v ? 1.0f : v;
+  };
+  float xr[DMAX];
+  float xx = 0.0f;
+  auto load_point = [&](int64_t i) {
+    xx = 0.0f;
+#pragma unroll
+    for (int t = 0; t < DMAX; ++t) {
+      xr[t] = (i >= 0 && t < d) ? __ldg(x + i * d + t) : 0.0f;
+      if (METRIC == F2C_COSINE) xx = fmaf(xr[t], xr[t], xx);
+    }
+  };
+  if (by_warp) {
+    stage(0, k);
+    for (int64_t s = warp; s < cnt; s += n_warps) {
+      const int64_t i = list[s];
+      load_point(i);
+      float best = INFINITY;
+      int best_c = 0x7fffffff;
+      for (int c = lane; c < k; c += 32) {
+        const float v = distance(xr, xx, c);
+        if (v < best) { best = v; best_c = c; }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+        const int oc = __shfl_xor_sync(0xffffffffu, best_c, o);
+        if (ob < best || (ob == best && oc < best_c)) { best = ob; best_c = oc; }
+      }
+      if (lane == 0) labels[i] = best_c == 0x7fffffff ? 0 : best_c;
+    }
+    return;
+  }
+  for (int64_t base = (int64_t)blockIdx.x * kListThreads; base < cnt; base += (int64_t)gridDim.x * kListThreads) {
+    const int64_t s = base + threadIdx.x;
+    const int64_t i = s < cnt ? (int64_t)list[s] : -1;
+    load_point(i);
+    float best = INFINITY;
+    int best_c = 0;
+    for (int c0 = 0; c0 < k; c0 += kc) {
+      const int nc = min(kc, k - c0);
+      __syncthreads();
+      stage(c0, nc);
+      for (int c = 0; c < nc; ++c) {
+        const float v = distance(xr, xx, c);
+        if (v < best) { best = v; best_c = c0 + c; }
+      }
+    }
+    if (i >= 0) labels[i] = best_c;
+  }
+}
+
+template <int DMAX>
+static int launch_listed(const float* x, const float* y, int64_t* labels, const int32_t* list, const int32_t* count_dev, int64_t max_count,
+                         int64_t k, int64_t d, int metric, cudaStream_t st) {
+  int kc = (int)k;
+  while ((size_t)kc * (DMAX + 5) * sizeof(float) > 96 * 1024) kc = (kc + 1) / 2;
+  const size_t smem = (size_t)kc * (DMAX + 5) * sizeof(float);
+  auto kern = metric == F2C_COSINE ? kmeans_listed_kernel<DMAX, F2C_COSINE> : kmeans_listed_kernel<DMAX, F2C_L2>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "kmeans_assign: %s", cudaGetErrorString(e));
+  int64_t grid = ceil_div(max_count, kListThreads / 32);
+  if (grid > 2 * current_sm_count()) grid = 2 * current_sm_count();
+  kern<<<(unsigned)grid, kListThreads, smem, st>>>(x, y, labels, list, count_dev, max_count, (int)k, (int)d, kc);
+  return check_launch("kmeans_assign");
+}
+
 template <int DMAX>
 static int launch_thread_assign(const float* x, const float* y, int64_t* labels, const int32_t* subset, int64_t n, int64_t k,
-                                int64_t d, int metric, cudaStream_t st, const int32_t* count_dev = nullptr) {
+                                int64_t d, int metric, cudaStream_t st, const int32_t* done) {
   int kc = (int)k;
   const size_t budget = 96 * 1024;
   while ((size_t)kc * (DMAX + 1) * sizeof(float) > budget) kc = (kc + 1) / 2;
   size_t smem = (size_t)kc * (DMAX + 1) * sizeof(float);
   unsigned grid = (unsigned)ceil_div(n, 256);
-  if (count_dev != nullptr && grid > 2u * current_sm_count()) grid = 2u * current_sm_count();  // the list is short: a small grid walks it
   cudaError_t e;
   if (metric == F2C_COSINE) {
     auto kern = kmeans_thread_kernel<DMAX, F2C_COSINE>;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) kern<<<grid, 256, smem, st>>>(x, y, labels, subset, count_dev, n, (int)k, (int)d, kc);
+    if (e == cudaSuccess) kern<<<grid, 256, smem, st>>>(x, y, labels, subset, n, (int)k, (int)d, kc, done);
   } else {
     auto kern = kmeans_thread_kernel<DMAX, F2C_L2>;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) kern<<<grid, 256, smem, st>>>(x, y, labels, subset, count_dev, n, (int)k, (int)d, kc);
+    if (e == cudaSuccess) kern<<<grid, 256, smem, st>>>(x, y, labels, subset, n, (int)k, (int)d, kc, done);
   }
   if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "kmeans_assign: %s", cudaGetErrorString(e));
   return check_launch("kmeans_assign");
@@ -158,20 +276,20 @@ static int launch_thread_assign(const float* x, const float* y, int64_t* labels,
 
 // Exact fp32 assignment of all points (subset == nullptr) or of the listed ones.
 int kmeans_assign_exact(const float* x, const float* y, int64_t* labels, const int32_t* subset, int64_t n, int64_t k,
-                        int64_t d, int metric, cudaStream_t st) {
+                        int64_t d, int metric, cudaStream_t st, const int32_t* done) {
   if (n == 0) return F2C_OK;
-  if (d <= 8) return launch_thread_assign<8>(x, y, labels, subset, n, k, d, metric, st);
-  if (d <= 16) return launch_thread_assign<16>(x, y, labels, subset, n, k, d, metric, st);
-  if (d <= 32) return launch_thread_assign<32>(x, y, labels, subset, n, k, d, metric, st);
-  if (d <= 64) return launch_thread_assign<64>(x, y, labels, subset, n, k, d, metric, st);
-  if (d <= 128) return launch_thread_assign<128>(x, y, labels, subset, n, k, d, metric, st);
+  if (d <= 8) return launch_thread_assign<8>(x, y, labels, subset, n, k, d, metric, st, done);
+  if (d <= 16) return launch_thread_assign<16>(x, y, labels, subset, n, k, d, metric, st, done);
+  if (d <= 32) return launch_thread_assign<32>(x, y, labels, subset, n, k, d, metric, st, done);
+  if (d <= 64) return launch_thread_assign<64>(x, y, labels, subset, n, k, d, metric, st, done);
+  if (d <= 128) return launch_thread_assign<128>(x, y, labels, subset, n, k, d, metric, st, done);
   if (subset != nullptr) return set_error(F2C_ERR_UNSUPPORTED, "kmeans_assign: subset re-scoring needs d <= 128");
   int64_t blocks = ceil_div(n, 8);
   if (blocks > current_sm_count() * 32) blocks = current_sm_count() * 32;
   if (metric == F2C_COSINE)
-    kmeans_warp_kernel<F2C_COSINE, false, true><<<(unsigned)blocks, 256, 0, st>>>(x, y, nullptr, labels, n, (int)k, (int)d);
+    kmeans_warp_kernel<F2C_COSINE, false, true><<<(unsigned)blocks, 256, 0, st>>>(x, y, nullptr, labels, n, (int)k, (int)d, done);
   else
-    kmeans_warp_kernel<F2C_L2, false, true><<<(unsigned)blocks, 256, 0, st>>>(x, y, nullptr, labels, n, (int)k, (int)d);
+    kmeans_warp_kernel<F2C_L2, false, true><<<(unsigned)blocks, 256, 0, st>>>(x, y, nullptr, labels, n, (int)k, (int)d, done);
   return check_launch("kmeans_assign");
 }
 
@@ -179,18 +297,17 @@ int kmeans_assign_exact(const float* x, const float* y, int64_t* labels, const i
 int kmeans_assign_exact_listed(const float* x, const float* y, int64_t* labels, const int32_t* list, const int32_t* count_dev,
                                int64_t max_count, int64_t k, int64_t d, int metric, cudaStream_t st) {
   if (max_count == 0) return F2C_OK;
-  if (d <= 8) return launch_thread_assign<8>(x, y, labels, list, max_count, k, d, metric, st, count_dev);
-  if (d <= 16) return launch_thread_assign<16>(x, y, labels, list, max_count, k, d, metric, st, count_dev);
-  if (d <= 32) return launch_thread_assign<32>(x, y, labels, list, max_count, k, d, metric, st, count_dev);
-  if (d <= 64) return launch_thread_assign<64>(x, y, labels, list, max_count, k, d, metric, st, count_dev);
-  if (d <= 128) return launch_thread_assign<128>(x, y, labels, list, max_count, k, d, metric, st, count_dev);
-  return set_error(F2C_ERR_UNSUPPORTED, "kmeans_assign: listed re-scoring needs d <= 128");
+  if (d <= 8) return launch_listed<8>(x, y, labels, list, count_dev, max_count, k, d, metric, st);
+  if (d <= 16) return launch_listed<16>(x, y, labels, list, count_dev, max_count, k, d, metric, st);
+  if (d <= 32) return launch_listed<32>(x, y, labels, list, count_dev, max_count, k, d, metric, st);
+  if (d <= 64) return launch_listed<64>(x, y, labels, list, count_dev, max_count, k, d, metric, st);
+  return set_error(F2C_ERR_UNSUPPORTED, "kmeans_assign: listed re-scoring needs d <= 64");
 }
 
 bool kmeans_tc_supported(int64_t n, int64_t k, int64_t d);
 int64_t kmeans_tc_workspace(int64_t n);
 int kmeans_assign_tc(const float* x, const float* y, int64_t* labels, int64_t n, int64_t k, int64_t d, int metric, void* workspace,
-                     cudaStream_t st);
+                     cudaStream_t st, const int32_t* done);
 
 static int validate_km(const char* op, int64_t n, int64_t k, int64_t d, int metric) {
   F2C_REQUIRE(n >= 0 && k >= 1 && d >= 1, F2C_ERR_INVALID, "%s: bad shape n=%lld k=%lld d=%lld", op, (long long)n, (long long)k,
@@ -214,9 +331,9 @@ extern "C" int f2c_pairwise_distance(const float* x, const float* y, float* dist
   if (blocks > current_sm_count() * 32) blocks = current_sm_count() * 32;
   cudaStream_t st = (cudaStream_t)stream;
   if (metric == F2C_COSINE)
-    kmeans_warp_kernel<F2C_COSINE, true, false><<<(unsigned)blocks, 256, 0, st>>>(x, y, dist, nullptr, n, (int)k, (int)d);
+    kmeans_warp_kernel<F2C_COSINE, true, false><<<(unsigned)blocks, 256, 0, st>>>(x, y, dist, nullptr, n, (int)k, (int)d, nullptr);
   else
-    kmeans_warp_kernel<F2C_L2, true, false><<<(unsigned)blocks, 256, 0, st>>>(x, y, dist, nullptr, n, (int)k, (int)d);
+    kmeans_warp_kernel<F2C_L2, true, false><<<(unsigned)blocks, 256, 0, st>>>(x, y, dist, nullptr, n, (int)k, (int)d, nullptr);
   return check_launch("pairwise_distance");
 }
 
@@ -237,6 +354,6 @@ extern "C" int f2c_kmeans_assign(const float* x, const float* centers, int64_t* 
   //  the CUDA-core scorer reads so little per point that the 128-point tiles only add latency)
   const bool prefer_tc = d >= 8 || scorer == F2C_SCORER_TENSOR;
   if (workspace != nullptr && kmeans_tc_supported(n, k, d) && prefer_tc && scorer != F2C_SCORER_EXACT && aligned(workspace, 16))
-    return kmeans_assign_tc(x, centers, labels, n, k, d, metric, workspace, (cudaStream_t)stream);
-  return kmeans_assign_exact(x, centers, labels, nullptr, n, k, d, metric, (cudaStream_t)stream);
+    return kmeans_assign_tc(x, centers, labels, n, k, d, metric, workspace, (cudaStream_t)stream, nullptr);
+  return kmeans_assign_exact(x, centers, labels, nullptr, n, k, d, metric, (cudaStream_t)stream, nullptr);
 }

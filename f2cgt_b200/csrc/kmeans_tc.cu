@@ -36,8 +36,6 @@
 
 namespace f2c {
 
-int kmeans_assign_exact(const float* x, const float* y, int64_t* labels, const int32_t* subset, int64_t n, int64_t k, int64_t d,
-                        int metric, cudaStream_t st);
 int kmeans_assign_exact_listed(const float* x, const float* y, int64_t* labels, const int32_t* list, const int32_t* count_dev,
                                int64_t max_count, int64_t k, int64_t d, int metric, cudaStream_t st);
 
@@ -127,6 +125,7 @@ struct Params {
   int metric;
   int vec4;    // rows of x can be read as float4
   float eps;   // relative error bound of one score
+  const int32_t* done;  // when set and non-zero: nothing to do (a fit that has converged, kmeans_fit.cu)
 };
 
 constexpr int kGroupThreads = 256;  // two threads per point of the tile
@@ -165,6 +164,7 @@ struct Top2 {
 template <bool BF16>
 __global__ void __launch_bounds__(kCtaThreads, 1) kmeans_tc_kernel(const Params p) {
   extern __shared__ __align__(128) unsigned char smem[];
+  if (p.done != nullptr && *(volatile const int32_t*)p.done != 0) return;
   const int tid = threadIdx.x;
   const int g = tid >> 8;            // group
   const int lt = tid & 255;          // thread within the group
@@ -466,8 +466,9 @@ bool kmeans_tc_supported(int64_t n, int64_t k, int64_t d) { return n >= 1 && n <
 int64_t kmeans_tc_workspace(int64_t n) { return 256 + 4 * n; }  // [count, error, pad][index list]
 
 int kmeans_assign_tc(const float* x, const float* y, int64_t* labels, int64_t n, int64_t k, int64_t d, int metric, void* workspace,
-                     cudaStream_t st) {
+                     cudaStream_t st, const int32_t* done) {
   tc::Params p{};
+  p.done = done;
   p.x = x; p.y = y; p.labels = labels; p.n = n; p.k = (int)k; p.d = (int)d; p.metric = metric;
   p.dp = (int)((d + 7) / 8 * 8);
   p.terms = p.dp <= 32 ? 3 : 1;
@@ -557,7 +558,7 @@ extern "C" int f2c_kmeans_assign_static(const float* x, const float* centers, in
   int rc = tc::static_scratch(op, &scratch);
   if (rc) return rc;
   // same kernels as kmeans_assign; the header (count, error code) is cleared inside
-  return kmeans_assign_tc(x, centers, labels, n, k, d, metric, scratch, (cudaStream_t)stream);
+  return kmeans_assign_tc(x, centers, labels, n, k, d, metric, scratch, (cudaStream_t)stream, nullptr);
 }
 
 // What the last f2c_kmeans_assign_static call on the current device left in the header of the built-in array: the

@@ -1,13 +1,14 @@
 """Lloyd iterations for ``KMeans.fit`` (reference: RAFT ``kmeans::fit`` behind src/kmeans.cu:61-75, and
 the torch loop around ``capi.pairwise_distance`` in examples/my_kmeans.py:73-113).
 
-The assignment step - the n*k*d contraction - is the library's k-means kernel; torch only does the
-O(n*d) centre update and the k-means++ / random initialisation.  Initial centres are random, so a fit
+The iterations - assignment, the n*k*d contraction, and centre update - are the library's kernels; torch only does the
+k-means++ / random initialisation.  Initial centres are random, so a fit
 is comparable with the reference's by inertia only, never label by label.
 """
 import torch
 
 from . import ops
+from ._lib import check, lib
 
 
 def _init_random(x, k, gen):
@@ -35,20 +36,42 @@ def _init_kmeanspp(x, k, gen):
     return centers
 
 
-def _update(x, labels, centers):
-    """Mean of every cluster's points, deterministically (a scatter-add would sum in whatever order its atomics land, and
-    a fit would not be reproducible): points sorted by label, float64 prefix sums, one difference per cluster."""
+_AHEAD = 8  # iterations queued between two looks at the convergence flag (those behind the converged one cost a few empty launches)
+
+
+def _iterate(x, centers, metric, max_iter, tol):
+    """Lloyd iterations from ``centers`` (float32, replaced in place) until the summed squared shift is at most ``tol``.  The
+    whole loop runs on the device (``f2c_kmeans_fit_iterate``); the host queues a few iterations ahead and reads one flag."""
+    if x.dim() != 2 or centers.dim() != 2 or x.shape[1] != centers.shape[1]:
+        raise RuntimeError("data must be [n, d] and centers [k, d]")
+    n, d = x.shape
     k = centers.shape[0]
-    order = torch.argsort(labels, stable=True)
-    csum = torch.cumsum(x[order].double(), dim=0)
-    cnt = torch.bincount(labels, minlength=k)
-    end = torch.cumsum(cnt, 0)                      # one past the last point of every cluster, in sorted order
-    zero = torch.zeros((1, x.shape[1]), dtype=torch.float64, device=x.device)
-    padded = torch.cat([zero, csum], dim=0)         # padded[j] = sum of the first j sorted points
-    sums = (padded[end] - padded[end - cnt]).float()
-    cntf = cnt.to(torch.float32).unsqueeze(1)
-    # empty clusters keep their previous centre (examples/my_kmeans.py:133-144)
-    return torch.where(cntf > 0, sums / cntf.clamp_min(1), centers)
+    ws = torch.empty((lib.f2c_kmeans_fit_workspace(n, k, d),), dtype=torch.uint8, device=x.device)
+    words = ws[:16].view(torch.int32)
+    seen = [(torch.empty(4, dtype=torch.int32, pin_memory=True), torch.cuda.Event()) for _ in range(2)]
+    stream = torch.cuda.current_stream(x.device)
+    queued = rounds = 0
+    with ops._on(x):
+        check(lib.f2c_kmeans_fit_begin(x.data_ptr(), n, k, d, ws.data_ptr(), stream.cuda_stream))
+        while True:
+            take = min(_AHEAD, max_iter - queued)
+            if take > 0:
+                check(lib.f2c_kmeans_fit_iterate(x.data_ptr(), centers.data_ptr(), n, k, d, ops._metric(metric), float(tol), take,
+                                                 ws.data_ptr(), stream.cuda_stream))
+                queued += take
+            host, event = seen[rounds % 2]
+            host.copy_(words, non_blocking=True)
+            event.record(stream)
+            rounds += 1
+            if take > 0 and rounds == 1:
+                continue  # look at a round's flag only when the next round is queued: the GPU never waits for the host
+            host, event = seen[rounds % 2] if take > 0 else (host, event)
+            event.synchronize()
+            done, _, not_finite, error = host.tolist()
+            if error != 0:
+                raise RuntimeError("f2cgt_b200: kmeans_assign: tensor-core kernel reported a timed-out wait")
+            if done or take <= 0:
+                return bool(not_finite)
 
 
 def _inertia(x, labels, centers, metric):
@@ -69,16 +92,13 @@ def lloyd_fit(x, k, metric, init, init_centers, max_iter, tol, n_init, seed=None
             centers = _init_random(x, k, gen)
         else:
             centers = _init_kmeanspp(x, k, gen)
-        labels = None
-        for _it in range(max_iter):
-            labels = ops.kmeans_assign(x, centers.contiguous(), metric)
-            new_centers = _update(x, labels, centers)
-            shift = float(((new_centers - centers) ** 2).sum())
-            centers = new_centers
-            if shift <= tol:
-                break
-        labels = ops.kmeans_assign(x, centers.contiguous(), metric)
-        inertia = _inertia(x, labels, centers, metric)
+        centers = centers.contiguous()
+        not_finite = x.shape[0] > 0 and max_iter > 0 and _iterate(x, centers, metric, max_iter, tol)
+        if max(1, n_init) == 1 or init == "array":
+            if not_finite or not bool(torch.isfinite(centers).all()):
+                raise RuntimeError("KMeans.fit: the data or the centres are not finite")
+            return centers
+        inertia = float("nan") if not_finite else _inertia(x, ops.kmeans_assign(x, centers, metric), centers, metric)
         if inertia < best_inertia:
             best, best_inertia = centers, inertia
     return best

@@ -231,6 +231,20 @@ int64_t f2c_kmeans_assign_workspace(int64_t n, int64_t k, int64_t d);
 int f2c_kmeans_assign(const float* x, const float* centers, int64_t* labels, int64_t n, int64_t k, int64_t d,
                       int metric, void* workspace, void* stream);
 
+/* Lloyd iterations of KMeans.fit(data)  -  src/kmeans.cu:61-75 (RAFT kmeans::fit; the loop as restated by the reference in
+ * examples/my_kmeans.py:73-113): labels = nearest centre, centres = mean of their points (a cluster without points keeps its
+ * centre), until the summed squared shift of the centres is at most tol.
+ *   f2c_kmeans_fit_begin    clears `workspace` (f2c_kmeans_fit_workspace(n, k, d) bytes, 256-byte aligned) for one fit of x
+ *   f2c_kmeans_fit_iterate  queues `iterations` iterations on `centers` [k, d] (in place) without waiting for any of them;
+ *                           those behind the converged one do nothing, so a caller queues a few at a time and looks at the
+ *                           first four int32 words of the workspace between the calls: {done, iterations taken, the data
+ *                           hold inf or NaN (then nothing is iterated), error code of the assignment kernel}.
+ * The sums are exact fixed-point integers: a fit is reproducible bit for bit. */
+int64_t f2c_kmeans_fit_workspace(int64_t n, int64_t k, int64_t d);
+int f2c_kmeans_fit_begin(const float* x, int64_t n, int64_t k, int64_t d, void* workspace, void* stream);
+int f2c_kmeans_fit_iterate(const float* x, float* centers, int64_t n, int64_t k, int64_t d, int metric, double tol, int iterations,
+                           void* workspace, void* stream);
+
 /* K-means assignment for callers that cannot allocate device memory - no counterpart in the reference.
  * Same result as f2c_kmeans_assign, but the scratch it needs is a fixed 4 MiB + 256 B array inside the library
  * (present on every GPU that loads it, until exit) instead of a caller-supplied workspace, and the call itself

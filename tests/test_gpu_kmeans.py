@@ -121,3 +121,31 @@ def test_tensor_core_assignment_at_table_scale(capi, d):
         assert ops.kmeans_assign.last_undecided <= (0.02 if d <= 32 else 0.05) * n
         exact = ops.kmeans_assign(x, c, metric, scorer="exact")
         assert torch.equal(tc, exact), (metric, d, int((tc != exact).sum()))
+
+
+@pytest.mark.parametrize("metric", ["l2", "cosine"])
+@pytest.mark.parametrize("n,k,d", [(1, 1, 1), (257, 16, 5), (5000, 256, 8), (1023, 17, 600), (150_001, 256, 64), (200_000, 100, 24),
+                                   (3000, 300, 100)])
+def test_fit_iterations_equal_the_restated_loop(capi, metric, n, k, d):
+    """The queued Lloyd iterations (fixed-point sums, convergence flag on the device) against the loop of
+    examples/my_kmeans.py:73-113 written with the assignment operator and float64 sums."""
+    g = torch.Generator(device="cuda").manual_seed(n + k + d)
+    x = torch.randn(n, d, device="cuda", generator=g) * torch.logspace(-3, 2, d, device="cuda")
+    start = x[torch.randint(0, n, (k,), device="cuda", generator=g)] + 1e-3
+    for max_iter, tol in ((1, 0.0), (11, 0.0), (20, 1e30)):
+        want = start.clone()
+        for _ in range(max_iter):
+            labels = capi.kmeans_assign(x, want, metric)
+            sums = torch.zeros(k, d, dtype=torch.float64, device="cuda").index_add_(0, labels, x.double())
+            cnt = torch.bincount(labels, minlength=k).unsqueeze(1)
+            new = torch.where(cnt > 0, sums.float() / cnt.clamp_min(1), want)
+            shift, want = float(((new - want) ** 2).sum()), new
+            if shift <= tol:
+                break
+        km = capi.KMeans(start.clone(), metric, max_iter=max_iter, tol=tol)
+        km.fit(x)
+        got = km.get_centers()
+        assert float((got - want).norm() / want.norm()) < 1e-5
+        again = capi.KMeans(start.clone(), metric, max_iter=max_iter, tol=tol)
+        again.fit(x)
+        assert torch.equal(got, again.get_centers())
