@@ -47,6 +47,9 @@ SIGNATURES = {
     "f2c_packbits": [p, p, i64, i64, ci, p],
     "f2c_unpackbits": [p, p, i64, i64, i64, ci, p],
     "f2c_sq_compress": [p, p, p, i64, i64, i64, ci, i64, p],
+    "f2c_sq_statistics_workspace": [],
+    "f2c_sq_statistics": [p, i64, p, i64, i64, i64, C.POINTER(i64), p, p, p],
+    "f2c_sq_encode": [p, p, p, i64, i64, i64, ci, i64, p],
     "f2c_sq_decompress": [p, ci, p, i64, p, i64, i64, i64, ci, i64, p],
     "f2c_vq_decompress": [p, ci, p, ci, p, i64, i64, i64, i64, i64, p],
     "f2c_spmm_csr": [p, ci, p, p, ci, p, i64, i64, ci, p],
@@ -86,7 +89,7 @@ SIGNATURES = {
     "f2c_last_error": [],
     "f2c_version": [],
 }
-_RESTYPE = {"f2c_last_error": C.c_char_p, "f2c_kmeans_assign_workspace": C.c_int64, "f2c_kmeans_fit_workspace": C.c_int64,
+_RESTYPE = {"f2c_last_error": C.c_char_p, "f2c_kmeans_assign_workspace": C.c_int64, "f2c_kmeans_fit_workspace": C.c_int64, "f2c_sq_statistics_workspace": C.c_int64,
             "f2c_relabel_capacity": C.c_int64,
             "f2c_sample_block_workspace": C.c_int64, "f2c_peer_hot_first_cold_id": C.c_int64}
 

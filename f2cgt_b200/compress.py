@@ -17,11 +17,13 @@ initialisations are seeded per column slice, so the split artefact equals the si
 ``configs`` = (column_slice, target_bits) per level, ``feat_dim``, ``data``, ``seeds``) plus the tables;
 ``save`` / ``load`` write and read ``compression_meta.pt``, ``compression_data.pt`` and ``seeds_compression_data.pt``.
 """
+import ctypes
 import os
 
 import torch
 
 from . import ops
+from ._lib import check, lib
 
 
 def normalize(data):
@@ -53,20 +55,63 @@ def _percentiles(a, qs):
     return out
 
 
+_QUANTILES = (0.005, 0.995)
+
+
+def _ranks(n):
+    """Ranks around the two percentiles of n values, and the weight of the upper neighbour (numpy's linear interpolation)."""
+    ranks, weights = [], []
+    for q in _QUANTILES:
+        pos = q * (n - 1)
+        lo = int(pos)
+        ranks += [lo, min(lo + 1, n - 1)]
+        weights.append(pos - lo)
+    return ranks, weights
+
+
+def _statistics(x, rows, n_rows, col, width, out, workspace):
+    """Queue the order statistics and the mean of |x[rows, col:col+width]| (rows=None: the first n_rows); ``out``: float64 [5]."""
+    ranks = (ctypes.c_int64 * 4)(*_ranks(n_rows * width)[0])
+    with ops._on(x):
+        check(lib.f2c_sq_statistics(x.data_ptr(), x.stride(0), 0 if rows is None else rows.data_ptr(), n_rows, col, width, ranks,
+                                    out.data_ptr(), workspace.data_ptr(), ops._stream(x)))
+
+
+def _by_kernel(n_rows, width):
+    return 0 < n_rows * width < 2**31 and width < 8192
+
+
+def _codebook_rows(limits):
+    """[fmin, fmax, emin, emax, mean] per (low percentile, high percentile, mean)."""
+    eps = 1e-5
+    rows = []
+    for v_lo, v_hi, mean in limits:
+        rows.append([max(float(v_lo), eps), max(float(v_hi), 2 * eps), 0.0, 0.0, mean + 0.1 if mean < 0.1 else mean])
+    # emin / emax are float32 values in the reference (torch.log2 of a float32 tensor, then + epsilon)
+    logs = torch.log2(torch.tensor([r[:2] for r in rows], dtype=torch.float32).reshape(-1, 2))
+    logs[:, 1] += eps
+    for r, (emin, emax) in zip(rows, logs.tolist()):
+        r[2], r[3] = emin, emax
+    return rows
+
+
+def _limits(stats, n):
+    """(low percentile, high percentile, mean) from what ``_statistics`` measured over n values."""
+    weights = _ranks(n)[1]
+    return tuple(stats[2 * i] + (stats[2 * i + 1] - stats[2 * i]) * weights[i] for i in (0, 1)) + (stats[4],)
+
+
 def sq_metadata(sample):
     """One codebook row from a sample of one column slice (examples/process_compress.py:43-68)."""
-    eps = 1e-5
+    if sample.is_cuda and sample.dim() == 2 and _by_kernel(*sample.shape):
+        x = sample.float().contiguous()
+        out = torch.empty(5, dtype=torch.float64, device=x.device)
+        ws = torch.empty(lib.f2c_sq_statistics_workspace(), dtype=torch.uint8, device=x.device)
+        _statistics(x, None, x.shape[0], 0, x.shape[1], out, ws)
+        return _codebook_rows([_limits(out.tolist(), x.numel())])[0]
     a = sample.float().abs().flatten()
-    q = _percentiles(a, (0.005, 0.995))
-    fmin = max(float(q[0]), eps)
-    fmax = max(float(q[1]), 2 * eps)
-    mean = float(a.mean())
-    if mean < 0.1:
-        mean += 0.1
-    # emin / emax are float32 values in the reference (torch.log2 of a float32 tensor, then + epsilon)
-    emin = float(torch.log2(torch.tensor(fmin, dtype=torch.float32)))
-    emax = float(torch.log2(torch.tensor(fmax, dtype=torch.float32)) + eps)
-    return [fmin, fmax, emin, emax, mean]
+    q = _percentiles(a, _QUANTILES)
+    return _codebook_rows([(q[0], q[1], float(a.mean()))])[0]
 
 
 # ---------------------------------------------------------------------------------------------- rank split (host logic)
@@ -114,27 +159,50 @@ def sq_compress_features(features, target_bits, column_slice, hotness=None, samp
     n_slices = (D + column_slice - 1) // column_slice
     (s_lo, s_hi), (r_lo, r_hi) = split_plan(n, n_slices, world, rank)
     gen = torch.Generator(device=features.device)
-    rows = []
+    # The statistics of all slices are queued before the first is read: one host read per call.
+    direct = features.dtype == torch.float32 and features.is_cuda and features.is_contiguous()
+    rows = [None] * (s_hi - s_lo)
+    pending = []
+    if features.is_cuda:
+        stats = torch.empty((s_hi - s_lo, 5), dtype=torch.float64, device=features.device)
+        ws = torch.empty(lib.f2c_sq_statistics_workspace(), dtype=torch.uint8, device=features.device)
     for i in range(s_lo, s_hi):
         gen.manual_seed(seed * 1000003 + i)  # per slice, so that the row is the same whichever rank computes it
-        idx = _sample_rows(n, sample_size, hotness, gen)
-        rows.append(sq_metadata(features[idx, i * column_slice:(i + 1) * column_slice]))
-    codebooks = torch.tensor(rows, dtype=torch.float32, device=features.device).reshape(-1, 5)
+        lo, hi = i * column_slice, min((i + 1) * column_slice, D)
+        idx = None if direct and sample_size >= n else _sample_rows(n, sample_size, hotness, gen)
+        n_sample = n if idx is None else idx.numel()
+        if not direct or not _by_kernel(n_sample, hi - lo):
+            rows[i - s_lo] = sq_metadata((features if idx is None else features[idx])[:, lo:hi])
+            continue
+        _statistics(features, idx, n_sample, lo, hi - lo, stats[i - s_lo], ws)
+        pending.append((i - s_lo, n_sample * (hi - lo)))
+    if pending:
+        staging = torch.empty(stats.shape, dtype=torch.float64, pin_memory=True)
+        staging.copy_(stats, non_blocking=True)
+        torch.cuda.current_stream(features.device).synchronize()
+        host = staging.tolist()
+        for (r, _), row in zip(pending, _codebook_rows([_limits(host[r], count) for r, count in pending])):
+            rows[r] = row
+    codebooks = torch.tensor(rows, dtype=torch.float32, pin_memory=features.is_cuda).reshape(-1, 5).to(features.device, non_blocking=True)
     if group is not None:
         codebooks = gather_parts(codebooks, group)
-    parts = []
+    width = (D * target_bits + 7) // 8 if target_bits <= 8 else D
+    dtype = torch.int8 if target_bits <= 8 else torch.int16  # packed bytes are stored as int8 (:109-111,141)
+    table = torch.empty((r_hi - r_lo, width), dtype=dtype, device=features.device)
     for s in range(r_lo, r_hi, batch_rows):
         x = features[s:min(s + batch_rows, r_hi)].float().contiguous()
+        part = table[s - r_lo:s - r_lo + x.shape[0]]
+        ops._chk(x, "features")
+        if D <= 1024 and n_slices <= 512 and part.data_ptr() % 4 == 0:
+            with ops._on(x):
+                check(lib.f2c_sq_encode(x.data_ptr(), part.data_ptr(), codebooks.data_ptr(), codebooks.shape[0], x.shape[0], D, target_bits,
+                                        column_slice, ops._stream(x)))
+            continue
         c = ops.sq_compress(x, codebooks, target_bits, column_slice)
         if target_bits < 8:
-            parts.append(ops.packbits(c.to(torch.uint8), target_bits).view(torch.int8))  # stored as int8 (:109-111,141)
-        elif target_bits == 8:
-            parts.append(c.to(torch.int8))
+            part.copy_(ops.packbits(c.to(torch.uint8), target_bits).view(torch.int8))
         else:
-            parts.append(c.to(torch.int16))
-    width = (D * target_bits + 7) // 8 if target_bits <= 8 else D
-    table = torch.cat(parts) if parts else torch.empty((0, width), dtype=torch.int8 if target_bits <= 8 else torch.int16,
-                                                       device=features.device)
+            part.copy_(c.to(dtype))
     if group is not None and gather:
         table = gather_parts(table, group)
     return table, codebooks

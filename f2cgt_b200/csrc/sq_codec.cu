@@ -8,27 +8,11 @@
 // the same math flags, so codes and decoded values carry the reference kernel's bits.
 #include <type_traits>
 
-#include "common.cuh"
+#include "sq_encode.cuh"
 
 namespace f2c {
 
 // ---------------------------------------------------------------- compress
-template <int BITS>
-__device__ __forceinline__ float sq_encode(float x, const float* __restrict__ cb) {
-  if (BITS == 1) return x <= 0.0f ? 0.0f : 1.0f;
-  constexpr float drange = (float)(1 << (BITS - 1));
-  float fmin = __ldg(cb + 0), fmax = __ldg(cb + 1), emin = __ldg(cb + 2), emax = __ldg(cb + 3);
-  bool neg = x <= 0.0f;
-  float v = fabsf(x);
-  v = fminf(fmaxf(v, fmin), fmax);
-  v = log2f(v);
-  v = (v - emin) / (emax - emin) * drange;
-  v = floorf(v);
-  v = neg ? -1.0f - v : v;
-  if (BITS < 8) v += drange;
-  return v;
-}
-
 template <int BITS>
 __global__ void __launch_bounds__(256) sq_compress_vec_kernel(const float4* __restrict__ src, float4* __restrict__ dst,
                                                               const float* __restrict__ codebooks, int64_t n_vec,

@@ -93,6 +93,21 @@ int f2c_unpackbits(const uint8_t* pack, uint8_t* unpack, int64_t rows, int64_t p
 int f2c_sq_compress(const float* src, float* dst, const float* codebooks, int64_t n_codebooks, int64_t rows,
                     int64_t feat_dim, int bits, int64_t column_slice, void* stream);
 
+/* What the offline compressor does around sq_compress (no single counterpart in the reference).
+ *   f2c_sq_statistics  the numbers a codebook row is made of (examples/process_compress.py:43-68): over the columns
+ *                      [col, col + width) of the given rows (`rows` int64 device array, NULL = rows 0 .. n_rows - 1) of a matrix
+ *                      with `ld` floats per row, the values of |x| at four ranks of its ascending order (NaN last) and the mean of
+ *                      |x|, as five doubles in `out` (device).  ranks_host: HOST array of four ranks in [0, n_rows * width).
+ *                      n_rows * width < 2^31, width < 8192; workspace: f2c_sq_statistics_workspace() bytes.
+ *   f2c_sq_encode      sq_compress + cast + packbits in one pass (:120-141): x [rows, feat_dim] f32 -> codes as stored: packed
+ *                      bytes [rows, ceil(feat_dim * bits / 8)] (1, 2, 4 bits), int8 (8) or int16 (16) [rows, feat_dim].  Same
+ *                      codes as the separate operators.  feat_dim <= 1024 and at most 512 codebook rows, else F2C_ERR_LIMIT. */
+int64_t f2c_sq_statistics_workspace(void);
+int f2c_sq_statistics(const float* x, int64_t ld, const int64_t* rows, int64_t n_rows, int64_t col, int64_t width,
+                      const int64_t* ranks_host, double* out, void* workspace, void* stream);
+int f2c_sq_encode(const float* x, void* codes, const float* codebooks, int64_t n_codebooks, int64_t rows, int64_t feat_dim,
+                  int bits, int64_t column_slice, void* stream);
+
 /* sq_decompress(compress_data, codebooks, target_bits, column_slice, feat_dim)  -
  * src/sq_quantization.cu:158-182 (kernel :85-156).  codes [rows, src_dim] -> out [rows, feat_dim] f32. */
 int f2c_sq_decompress(const void* codes, int code_dtype, const float* codebooks, int64_t n_codebooks,

@@ -100,3 +100,53 @@ def test_rank_split_equals_single_process(capi):
             assert c["row_range"] == (0, 20000) and torch.equal(c["compression_data"], a["compression_data"])
     finally:
         dist.destroy_process_group()
+
+
+@pytest.mark.parametrize("bits", [1, 2, 4, 8, 16])
+@pytest.mark.parametrize("rows,D,cs", [(1, 1, 8), (5, 7, 8), (3001, 33, 16), (2049, 100, 104), (1000, 128, 32), (777, 200, 100), (513, 36, 5),
+                                       (70, 1024, 1024), (64, 1021, 256), (257, 64, 64)])
+def test_one_pass_encoder_equals_the_separate_operators(capi, bits, rows, D, cs):
+    """sq_encode == sq_compress + cast + packbits, clamped, zero, infinite and NaN values and equal features included."""
+    from f2cgt_b200 import compress, ops
+    from f2cgt_b200._lib import check, lib
+    g = torch.Generator(device="cuda").manual_seed(rows + D)
+    for kind in range(3):
+        x = torch.randn(rows, D, generator=g, device="cuda") * torch.logspace(-2, 2, D, device="cuda")
+        if kind == 1:
+            x.flatten()[::3] = 0
+            x.flatten()[1::17] = float("inf")
+            x.flatten()[5::19] = float("nan")
+        cbs = torch.tensor([compress.sq_metadata(x[:, b:b + cs].nan_to_num(0, 3, -3)) for b in range(0, D, cs)], device="cuda")
+        if kind == 2:  # nearly constant features: a level is a few floats wide
+            cbs[:, 1] = cbs[:, 0] * 1.0001
+            cbs[:, 3] = cbs[:, 2] + 1e-4
+        width = (D * bits + 7) // 8 if bits <= 8 else D
+        got = torch.empty((rows, width), dtype=torch.int8 if bits <= 8 else torch.int16, device="cuda")
+        check(lib.f2c_sq_encode(x.data_ptr(), got.data_ptr(), cbs.data_ptr(), cbs.shape[0], rows, D, bits, cs, ops._stream(x)))
+        c = capi.sq_compress(x, cbs, bits, cs)
+        want = capi.packbits(c.to(torch.uint8), bits).view(torch.int8) if bits < 8 else c.to(got.dtype)
+        assert torch.equal(got, want), (kind, int((got != want).sum()))
+
+
+@pytest.mark.parametrize("rows,D,col,width,sampled", [(1, 1, 0, 1, False), (2, 3, 1, 2, False), (1000, 128, 0, 128, True), (5000, 100, 96, 4, True),
+                                                      (33, 7, 2, 5, True), (70_000, 64, 32, 32, True)])
+def test_sample_statistics_equal_a_sort(capi, rows, D, col, width, sampled):
+    from f2cgt_b200 import compress
+    from f2cgt_b200._lib import lib
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    ws = torch.empty(lib.f2c_sq_statistics_workspace(), dtype=torch.uint8, device="cuda")
+    for kind in range(3):
+        x = torch.randn(rows, D, generator=g, device="cuda")
+        if kind == 1:
+            x[torch.rand(rows, D, generator=g, device="cuda") < 0.9] = 0
+        if kind == 2:
+            x.fill_(-2.5)
+        idx = torch.randperm(rows, generator=g, device="cuda")[:(rows + 1) // 2] if sampled else None
+        part = (x if idx is None else x[idx])[:, col:col + width].abs()
+        out = torch.empty(5, dtype=torch.float64, device="cuda")
+        compress._statistics(x, idx, part.shape[0], col, width, out, ws)
+        ordered = part.flatten().sort().values
+        want = [float(ordered[r]) for r in compress._ranks(part.numel())[0]]
+        got = out.tolist()
+        assert got[:4] == want, (kind, got, want)
+        assert abs(got[4] - float(part.double().mean())) <= 1e-12 * max(1.0, got[4])
