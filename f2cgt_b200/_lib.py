@@ -25,6 +25,17 @@ class Epilogue(C.Structure):
                 ("offset", C.c_uint64), ("kernel", C.c_int)]
 
 
+MAX_HOPS = 16
+
+
+class Minibatch(C.Structure):  # f2c_minibatch
+    _fields_ = [("indptr", C.c_void_p), ("indices", C.c_void_p), ("seeds", C.c_void_p), ("n_nodes", C.c_int64), ("n_seeds", C.c_int64),
+                ("index_dtype", C.c_int), ("n_hops", C.c_int), ("num_pick", C.c_int * MAX_HOPS), ("rng_seed", C.c_uint64),
+                ("rng_offset", C.c_uint64), ("unique", C.c_void_p), ("sub_indptr", C.c_void_p * MAX_HOPS), ("ids", C.c_void_p * MAX_HOPS),
+                ("local", C.c_void_p * MAX_HOPS), ("node_map", C.c_void_p), ("header", C.c_void_p), ("workspace", C.c_void_p),
+                ("workspace_bytes", C.c_int64), ("epoch", C.c_uint32)]
+
+
 class F2CError(RuntimeError):
     pass
 
@@ -86,12 +97,14 @@ SIGNATURES = {
     "f2c_sample_neighbors": [p, p, p, p, p, i64, ci, i64, ci, u64, u64, p],
     "f2c_sample_block_workspace": [i64, ci, ci],
     "f2c_sample_block": [p, p, p, ci, i64, ci, u64, u64, p, p, p, p, p, p, i64, p],
+    "f2c_sample_minibatch_workspace": [i64, i64, ci, C.POINTER(ci)],
+    "f2c_sample_minibatch": [C.POINTER(Minibatch), p],
     "f2c_last_error": [],
     "f2c_version": [],
 }
 _RESTYPE = {"f2c_last_error": C.c_char_p, "f2c_kmeans_assign_workspace": C.c_int64, "f2c_kmeans_fit_workspace": C.c_int64, "f2c_sq_statistics_workspace": C.c_int64,
             "f2c_relabel_capacity": C.c_int64,
-            "f2c_sample_block_workspace": C.c_int64, "f2c_peer_hot_first_cold_id": C.c_int64}
+            "f2c_sample_block_workspace": C.c_int64, "f2c_sample_minibatch_workspace": C.c_int64, "f2c_peer_hot_first_cold_id": C.c_int64}
 
 for _name, _args in SIGNATURES.items():
     _fn = getattr(lib, _name)  # AttributeError here = header and library out of step

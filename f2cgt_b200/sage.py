@@ -353,12 +353,10 @@ class SAGE(nn.Module):
 class GPUSamplingDataloader:
     """Seeds are split contiguously over the ranks (examples/dataloader.py:102-108), shuffled per epoch.
 
-    ``ahead=True`` (default) builds every minibatch one step early on a CUDA stream of its own.  A block is a chain of
-    small dependent kernels with one host read per hop; on the training stream that chain would sit on the critical path
-    of every step although it needs nothing from the model.  Here ``__next__`` hands out the minibatch built during the
-    previous step and queues the first hop of the next; each later hop is queued by ``poke()`` - which the training loop
-    calls between its phases and which never blocks - or, at the latest, by the next ``__next__``.  The minibatches are
-    the same either way: sampling draws are keyed by epoch, step and hop.  In this mode the loader works in two sets of
+    ``ahead=True`` (default) builds every minibatch one step early, as one kernel on a CUDA stream of its own
+    (``ops.sample_minibatch_launch``): ``__next__`` hands out the minibatch built during the previous step and queues the next
+    one, so neither its latency nor its host read is on the critical path of a step that does more than sample.  The minibatches
+    are the same either way: sampling draws are keyed by epoch, step and hop.  In this mode the loader works in two sets of
     buffers it allocates once (sized for the largest possible hop), used alternately: the tensors of a minibatch are
     views of one set and stay valid until the next-but-one ``__next__``."""
 
@@ -374,8 +372,10 @@ class GPUSamplingDataloader:
         per = (seeds.numel() + world - 1) // world
         self.seeds = seeds[rank * per:(rank + 1) * per]
         self.rank = rank
+        # (what one kernel does not take - more than 2^31 ids in a hop - is built hop by hop inside its step)
+        ahead = ahead and ops.minibatch_fits(indptr.numel() - 1, self.batchsize, self.num_picks)
         self.side = torch.cuda.Stream(device=indptr.device) if ahead else None
-        self._gen = self._result = self._wait = None
+        self._pending = None  # buffers of the minibatch under construction
         self._sets, self._consumed, self._built = None, [None, None], 0
 
     def __len__(self):
@@ -390,87 +390,69 @@ class GPUSamplingDataloader:
         else:
             self.order = self.seeds
         self.epoch += 1
-        self._gen = self._result = self._wait = None
+        self._pending = None
         if self.side is not None:
             self.side.wait_stream(torch.cuda.current_stream(self.indptr.device))  # the shuffled order is read over there
             self._start()
         return self
 
-    def _buffer_sets(self):
-        if self._sets is None:
-            n_nodes, bound, sizes = self.indptr.numel() - 1, self.batchsize, []
-            for num_pick in reversed(self.num_picks):
-                sizes.append((bound, num_pick))
-                bound = min(bound * (num_pick + 1), n_nodes)  # a hop's distinct nodes are the next hop's seeds
-            self._sets = [[ops.BlockBuffers(b, k, self.indptr.dtype, self.indptr.device) for b, k in sizes] for _ in range(2)]
-        return self._sets
-
-    def _hops(self, seeds, step, buffers=None):
-        """Generator over one minibatch: yields the pending hop after queueing it, returns the minibatch."""
+    def _hops(self, seeds, step):
+        """One minibatch hop by hop on the current stream, in fresh tensors."""
         output_nodes, blocks = seeds, []
         for hop, num_pick in enumerate(reversed(self.num_picks)):
             # one library call and one host read (the number of distinct nodes) per hop; the index tensors carry a tail
             # behind indptr[-1] that no kernel reads
-            pending = ops.sample_block_launch(self.indptr, self.indices, seeds, num_pick,
-                                              rng_seed=(self.rng_seed * 7919 + self.epoch) * 65536 + self.rank, rng_offset=step * 8 + hop,
-                                              buffers=None if buffers is None else buffers[hop])
-            yield pending
+            pending = ops.sample_block_launch(self.indptr, self.indices, seeds, num_pick, rng_seed=self._rng_seed(), rng_offset=step * 8 + hop)
             sub_indptr, sub_indices, unique, local = ops.sample_block_finish(pending)
             blocks.insert(0, dict(dst_nodes=seeds, src_nodes=unique, indptr=sub_indptr, indices_global=sub_indices, indices_local=local,
                                   n_edges=pending.n_edges))
             seeds = unique
         return seeds, output_nodes, blocks
 
+    def _rng_seed(self):
+        return (self.rng_seed * 7919 + self.epoch) * 65536 + self.rank
+
     def _start(self):
+        self._pending = None
         if self.curr >= len(self):
-            self._gen = None
             return
-        seeds = self.order[self.curr * self.batchsize:(self.curr + 1) * self.batchsize]
+        if self._sets is None:
+            picks = self.num_picks[::-1]
+            first = ops.MinibatchBuffers(self.indptr, self.indices, self.batchsize, picks)
+            self._sets = [first, ops.MinibatchBuffers(self.indptr, self.indices, self.batchsize, picks, share=first)]
+            self.side.wait_stream(torch.cuda.current_stream(self.indptr.device))  # the node words are set over there
         which = self._built % 2
         self._built += 1
         if self._consumed[which] is not None:  # the minibatch that last lived in this set: its step must be through
             self.side.wait_event(self._consumed[which])
-        self._gen = self._hops(seeds, self.curr, self._buffer_sets()[which])
+        ops.sample_minibatch_launch(self._sets[which], self.order[self.curr * self.batchsize:(self.curr + 1) * self.batchsize],
+                                    rng_seed=self._rng_seed(), rng_offset=self.curr * 8, stream=self.side)
+        self._pending = self._sets[which]
         self.curr += 1
-        self._advance()
-
-    def _advance(self):
-        """Finish the pending hop (blocks until the GPU is done with it) and queue the next one."""
-        with torch.cuda.stream(self.side):
-            try:
-                self._wait = next(self._gen)
-            except StopIteration as done:
-                self._result, self._gen, self._wait = done.value, None, None
 
     def poke(self):
-        """Move the minibatch under construction one hop forward if that needs no waiting; call it wherever the host has
-        just queued a stretch of GPU work."""
-        if self._gen is not None and self._wait is not None and self._wait.event.query():
-            self._advance()
+        """Nothing to do: a minibatch under construction needs no help from the host (kept for training loops that call it)."""
 
     def __next__(self):
         if self.side is None:
             if self.curr >= len(self):
                 raise StopIteration
-            gen = self._hops(self.order[self.curr * self.batchsize:(self.curr + 1) * self.batchsize], self.curr)
             self.curr += 1
-            try:
-                while True:
-                    next(gen)
-            except StopIteration as done:
-                return done.value
-        if self._gen is None and self._result is None:
+            return self._hops(self.order[(self.curr - 1) * self.batchsize:self.curr * self.batchsize], self.curr - 1)
+        built = self._pending
+        if built is None:
             raise StopIteration
-        while self._result is None:
-            self._advance()
-        batch, self._result = self._result, None
-        cur = torch.cuda.current_stream(self.indptr.device)
-        cur.wait_stream(self.side)
-        # Everything queued on this stream so far belongs to earlier minibatches: once it has run, the set of the
-        # minibatch handed out before this one may be overwritten (which is what the _start below goes on to do).
+        built.event.synchronize()
+        # Everything queued on the current stream so far belongs to earlier minibatches: once it has run, the set of the
+        # minibatch handed out before this one may be overwritten, which is what the next one goes on to do.
         previous = self._built % 2
         if self._consumed[previous] is None:
             self._consumed[previous] = torch.cuda.Event()
-        self._consumed[previous].record(cur)
+        self._consumed[previous].record(torch.cuda.current_stream(self.indptr.device))
         self._start()
-        return batch
+        hops, input_nodes = ops.sample_minibatch_finish(built)
+        blocks = []
+        for i, (seeds, sub_indptr, sub_indices, local) in enumerate(hops):
+            blocks.insert(0, dict(dst_nodes=seeds, src_nodes=hops[i + 1][0] if i + 1 < len(hops) else input_nodes, indptr=sub_indptr,
+                                  indices_global=sub_indices, indices_local=local, n_edges=sub_indices.numel()))
+        return input_nodes, hops[0][0], blocks

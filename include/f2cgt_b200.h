@@ -328,6 +328,42 @@ int f2c_sample_block(const void* indptr, const void* indices, const void* seeds,
                      uint64_t rng_seed, uint64_t rng_offset, void* sub_indptr, void* keys, void* unique, void* relabelled,
                      int64_t* header_device, void* workspace, int64_t workspace_bytes, void* stream);
 
+/* A whole minibatch in one call: the loop of examples/dataloader.py:167-182, i.e. f2c_sample_block for every hop where the
+ * seeds of hop h + 1 are the distinct nodes of hop h, without a host read in between.  Same draws (hop h uses stream offset
+ * rng_offset + h) and same numbering.  Hops are in sampling order (from the seeds outwards).
+ *   sub_indptr[h] [n_h + 1], ids[h] and local[h] [n_h * num_pick[h]]: CSC offsets, global ids and new numbers of the hop's edges,
+ *       n_0 = n_seeds, n_h = min(n_{h-1} * (num_pick[h-1] + 1), n_nodes) being upper bounds; entries behind the edges are not written
+ *   unique [n_{n_hops}]   distinct nodes in order of first occurrence; those of hop h are a prefix of those of hop h + 1
+ *   node_map [n_nodes]    64-bit words, all ones before the first call; kept by the caller between calls
+ *   epoch                 number of this minibatch: larger than that of any earlier call on node_map, below 2^32 - 1
+ *   header                HOST memory the device can write (pinned), 2 * n_hops + 1 entries, valid when the stream has got past
+ *                         the call: {edges, distinct nodes} per hop, then 0 or the error (2 negative id, 3 id >= n_nodes)
+ *   workspace             f2c_sample_minibatch_workspace() bytes, 256-byte aligned */
+#define F2C_MAX_HOPS 16
+typedef struct {
+  const void* indptr;
+  const void* indices;
+  const void* seeds;
+  int64_t n_nodes;
+  int64_t n_seeds;
+  int index_dtype;
+  int n_hops;
+  int num_pick[F2C_MAX_HOPS];
+  uint64_t rng_seed;
+  uint64_t rng_offset;
+  void* unique;
+  void* sub_indptr[F2C_MAX_HOPS];
+  void* ids[F2C_MAX_HOPS];
+  void* local[F2C_MAX_HOPS];
+  void* node_map;
+  int64_t* header;
+  void* workspace;
+  int64_t workspace_bytes;
+  uint32_t epoch;
+} f2c_minibatch;
+int64_t f2c_sample_minibatch_workspace(int64_t n_nodes, int64_t n_seeds, int n_hops, const int* num_pick_host);
+int f2c_sample_minibatch(const f2c_minibatch* args, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -148,3 +148,49 @@ def test_sample_block_of_isolated_seeds(capi):
     ip, ix, uniq, local = ops.sample_block(indptr, indices, seeds, 5)
     assert ip.tolist() == [0, 0, 0, 0] and uniq.tolist() == [4, 2, 9]
     assert ix.tolist() == [4] * 15 and local.tolist() == [0] * 15
+
+
+@pytest.mark.parametrize("idx", [torch.int64, torch.int32])
+@pytest.mark.parametrize("picks,n_seeds", [((1,), 1), ((3, 2), 1), ((8, 9), 700), ((12, 12, 12), 300), ((16, 17, 5), 65), ((33, 64), 40),
+                                           ((2, 2, 2, 2, 2, 2, 2, 2), 5)])
+def test_minibatch_kernel_equals_hops_one_by_one(capi, idx, picks, n_seeds):
+    """All hops in one kernel == one sample_block per hop, over several minibatches in the same buffers (the node words carry
+    over), with repeated seeds, isolated nodes and nodes of a high degree."""
+    from f2cgt_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(len(picks) + n_seeds)
+    n = 4000
+    deg = torch.randint(0, 40, (n,), generator=g, device="cuda")
+    deg[::50] = 0
+    deg[7] = 3000
+    indptr = torch.cat([torch.zeros(1, dtype=torch.int64, device="cuda"), deg.cumsum(0)]).to(idx)
+    indices = torch.randint(0, n, (int(indptr[-1]),), generator=g, device="cuda").to(idx)
+    buffers = ops.MinibatchBuffers(indptr, indices, n_seeds, picks)
+    second = ops.MinibatchBuffers(indptr, indices, n_seeds, picks, share=buffers)
+    for step in range(4):
+        seeds = torch.randint(0, n, (max(1, n_seeds - step),), generator=g, device="cuda").to(idx)
+        seeds[0] = 7
+        b = (buffers, second)[step % 2]
+        ops.sample_minibatch_launch(b, seeds, rng_seed=9 + step, rng_offset=8 * step)
+        hops, nodes = ops.sample_minibatch_finish(b)
+        frontier = seeds
+        for h, k in enumerate(picks):
+            ip, ix, uniq, local = ops.sample_block(indptr, indices, frontier, k, rng_seed=9 + step, rng_offset=8 * step + h)
+            nnz = int(ip[-1])
+            got_seeds, got_ip, got_ix, got_local = hops[h]
+            assert torch.equal(got_seeds, frontier) and torch.equal(got_ip, ip)
+            assert torch.equal(got_ix, ix[:nnz]) and torch.equal(got_local, local[:nnz])
+            frontier = uniq
+        assert torch.equal(nodes, frontier)
+
+
+def test_minibatch_kernel_rejects_ids_outside_the_graph(capi):
+    from f2cgt_b200 import ops
+    indptr = torch.tensor([0, 2, 3, 3], device="cuda")
+    for bad in (-5, 3):
+        indices = torch.tensor([1, bad, 2], device="cuda")
+        b = ops.MinibatchBuffers(indptr, indices, 2, (4, 4))
+        ops.sample_minibatch_launch(b, torch.tensor([0, 1], device="cuda"))
+        with pytest.raises(RuntimeError, match="id"):
+            ops.sample_minibatch_finish(b)
+        ops.sample_minibatch_launch(b, torch.tensor([1], device="cuda"))
+        assert ops.sample_minibatch_finish(b)[1].tolist() == [1, 2]
