@@ -45,7 +45,8 @@ def _load():
         raise ImportError(
             f"{LIB_PATH} not found: build it with `python -m f2cgt_b200.build` (needs nvcc); "
             "f2cgt_b200 has no fallback path")
-    return C.CDLL(LIB_PATH)
+    # an override must also serve the native module, which is linked to the library beside it: global scope comes first
+    return C.CDLL(LIB_PATH, mode=C.RTLD_GLOBAL if os.environ.get("F2CGT_B200_LIB") else C.DEFAULT_MODE)
 
 
 lib = _load()

@@ -1,0 +1,206 @@
+// The per-call part of f2cgt_b200/ops.py for the decoders and the aggregations: argument checks, output allocation, stream
+// lookup and the library call.  In Python these cost 10-14 us per call, several times the launch itself; here 3-4 us.
+#include "native.h"
+
+namespace f2c_native {
+
+PyObject* g_error_class = nullptr;
+
+void arguments(const char* name, Py_ssize_t got, Py_ssize_t want) {
+  if (got != want) fail(PyExc_TypeError, "%s: expected %zd arguments, got %zd", name, want, got);
+}
+
+namespace {
+
+struct Csc { const at::Tensor &indptr, &indices; int64_t n_dst; int tag; };
+
+Csc csc(PyObject* ip, PyObject* ix) {
+  const at::Tensor& indptr = tensor(ip, "indptr", kIndex);
+  const at::Tensor& indices = tensor(ix, "indices", kIndex);
+  if (indptr.scalar_type() != indices.scalar_type()) fail(PyExc_RuntimeError, "indptr and indices must have the same dtype");
+  if (indptr.dim() != 1 || indptr.numel() < 1) fail(PyExc_RuntimeError, "indptr must be 1-D with at least one element");
+  return Csc{indptr, indices, indptr.numel() - 1, dtype_tag(indptr.scalar_type())};
+}
+
+// [max(n_dst, out_rows), width]; rows behind n_dst are zero
+at::Tensor block_out(int64_t n_dst, int64_t width, at::ScalarType dtype, const at::Device& device, PyObject* out_rows, cudaStream_t st) {
+  const int64_t rows = out_rows == Py_None ? n_dst : std::max(n_dst, integer(out_rows));
+  if (width < 0) fail(PyExc_RuntimeError, "negative width");
+  at::Tensor out = empty({rows, width}, dtype, device);
+  if (rows > n_dst) {
+    const size_t row = (size_t)width * out.element_size();
+    C10_CUDA_CHECK(cudaMemsetAsync((char*)out.data_ptr() + (size_t)n_dst * row, 0, (size_t)(rows - n_dst) * row, st));
+  }
+  return out;
+}
+
+// dropout: None or a mapping with p, seed, offset, training, scale; kernel: an f2c_kernel value
+struct Options {
+  f2c_epilogue e{};
+  bool set = false;
+  const f2c_epilogue* get() const { return set ? &e : nullptr; }
+};
+
+Options options(PyObject* dropout, PyObject* kernel) {
+  Options o;
+  o.e.kernel = (int)integer(kernel);
+  o.set = o.e.kernel != 0;
+  if (dropout == Py_None) return o;
+  o.set = true;
+  PyObject* d = PyDict_Check(dropout) ? Py_NewRef(dropout) : PyObject_CallOneArg((PyObject*)&PyDict_Type, dropout);
+  if (d == nullptr) throw PythonError{};
+  struct Drop { PyObject* o; ~Drop() { Py_DECREF(o); } } keep{d};
+  auto item = [&](const char* k) -> PyObject* { return PyDict_GetItemString(d, k); };
+  PyObject* p = item("p");
+  if (p == nullptr) fail(PyExc_KeyError, "p");
+  o.e.p = (float)real(p);
+  auto whole = [&](const char* k, int64_t otherwise) -> int64_t {
+    PyObject* v = item(k);
+    if (v == nullptr) return otherwise;
+    if (PyLong_Check(v)) {
+      const unsigned long long u = PyLong_AsUnsignedLongLongMask(v);
+      if (u == (unsigned long long)-1 && PyErr_Occurred()) throw PythonError{};
+      return (int64_t)u;
+    }
+    return integer(v);
+  };
+  o.e.training = item("training") ? (PyObject_IsTrue(item("training")) ? 1 : 0) : 1;
+  o.e.scale = item("scale") ? (PyObject_IsTrue(item("scale")) ? 1 : 0) : 0;
+  o.e.seed = (uint64_t)whole("seed", 0);
+  o.e.offset = (uint64_t)whole("offset", 0);
+  return o;
+}
+
+PyObject* sq_decompress(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    arguments("sq_decompress", n, 5);
+    const at::Tensor& codes = tensor(a[0], "compress_data", kCodes);
+    const at::Tensor& cb = tensor(a[1], "codebooks", kF32);
+    if (codes.dim() != 2) fail(PyExc_RuntimeError, "compress_data must be 2-D");
+    const int64_t bits = integer(a[2]), cs = integer(a[3]), dim = integer(a[4]);
+    c10::cuda::CUDAGuard guard(codes.device());
+    at::Tensor out = block_out(codes.size(0), dim, at::kFloat, codes.device(), Py_None, nullptr);
+    check_status(f2c_sq_decompress(codes.data_ptr(), dtype_tag(codes.scalar_type()), cb.const_data_ptr<float>(), cb.size(0),
+                                   out.mutable_data_ptr<float>(), codes.size(0), codes.size(1), dim, (int)bits, cs, stream_of(codes)));
+    return THPVariable_Wrap(std::move(out));
+  });
+}
+
+PyObject* vq_decompress(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    arguments("vq_decompress", n, 3);
+    const at::Tensor& codes = tensor(a[0], "index_tensor", kCodes);
+    const at::Tensor& cb = tensor(a[1], "codebooks", kF32 | bit(F2C_F16));
+    if (codes.dim() != 2 || cb.dim() != 3 || codes.size(1) != cb.size(0))
+      fail(PyExc_RuntimeError, "index_tensor must be [rows, n_codebooks] and codebooks [n_codebooks, length, column_slice]");
+    const int64_t dim = integer(a[2]);
+    c10::cuda::CUDAGuard guard(codes.device());
+    at::Tensor out = block_out(codes.size(0), dim, at::kFloat, codes.device(), Py_None, nullptr);
+    check_status(f2c_vq_decompress(codes.data_ptr(), dtype_tag(codes.scalar_type()), cb.data_ptr(), dtype_tag(cb.scalar_type()),
+                                   out.mutable_data_ptr<float>(), codes.size(0), cb.size(0), cb.size(1), cb.size(2), dim, stream_of(codes)));
+    return THPVariable_Wrap(std::move(out));
+  });
+}
+
+PyObject* spmm(PyObject*, PyObject* const* a, Py_ssize_t n) {  // feat, indptr, indices, reduce, out_rows
+  return guarded([&]() -> PyObject* {
+    arguments("spmm", n, 5);
+    const at::Tensor& feat = tensor(a[0], "feat", kF32 | bit(F2C_F16) | bit(F2C_F64));
+    const Csc c = csc(a[1], a[2]);
+    if (feat.dim() != 2) fail(PyExc_RuntimeError, "feat must be 2-D");
+    c10::cuda::CUDAGuard guard(feat.device());
+    cudaStream_t st = stream_of(feat);
+    at::Tensor out = block_out(c.n_dst, feat.size(1), feat.scalar_type(), feat.device(), a[4], st);
+    check_status(f2c_spmm_csr(feat.data_ptr(), dtype_tag(feat.scalar_type()), c.indptr.data_ptr(), c.indices.data_ptr(), c.tag, out.data_ptr(),
+                              c.n_dst, feat.size(1), (int)integer(a[3]), st));
+    return THPVariable_Wrap(std::move(out));
+  });
+}
+
+// codes, codebooks, indptr, indices, bits, column_slice, feat_dim, reduce, dropout, kernel, out_rows
+PyObject* sq_spmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    arguments("sq_spmm", n, 11);
+    const at::Tensor& codes = tensor(a[0], "compress_feat", kCodes);
+    const at::Tensor& cb = tensor(a[1], "codebooks", kF32);
+    const Csc c = csc(a[2], a[3]);
+    if (codes.dim() != 2) fail(PyExc_RuntimeError, "compress_feat must be 2-D");
+    const int64_t bits = integer(a[4]), cs = integer(a[5]), dim = integer(a[6]);
+    const Options o = options(a[8], a[9]);
+    c10::cuda::CUDAGuard guard(codes.device());
+    cudaStream_t st = stream_of(codes);
+    at::Tensor out = block_out(c.n_dst, dim, at::kFloat, codes.device(), a[10], st);
+    check_status(f2c_sq_spmm_csr(codes.data_ptr(), dtype_tag(codes.scalar_type()), cb.const_data_ptr<float>(), cb.size(0), c.indptr.data_ptr(),
+                                 c.indices.data_ptr(), c.tag, out.mutable_data_ptr<float>(), c.n_dst, codes.size(0), codes.size(1), dim,
+                                 (int)bits, cs, (int)integer(a[7]), o.get(), st));
+    return THPVariable_Wrap(std::move(out));
+  });
+}
+
+// codes, codebooks, indptr, indices, feat_dim, reduce, dropout, kernel, out_rows
+PyObject* vq_spmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    arguments("vq_spmm", n, 9);
+    const at::Tensor& codes = tensor(a[0], "compress_feat", kCodes);
+    const at::Tensor& cb = tensor(a[1], "codebooks", kF32);
+    const Csc c = csc(a[2], a[3]);
+    if (codes.dim() != 2 || cb.dim() != 3 || codes.size(1) != cb.size(0))
+      fail(PyExc_RuntimeError, "compress_feat must be [rows, n_codebooks] and codebooks [n_codebooks, length, column_slice]");
+    const int64_t dim = integer(a[4]);
+    const Options o = options(a[6], a[7]);
+    c10::cuda::CUDAGuard guard(codes.device());
+    cudaStream_t st = stream_of(codes);
+    at::Tensor out = block_out(c.n_dst, dim, at::kFloat, codes.device(), a[8], st);
+    check_status(f2c_vq_spmm_csr(codes.data_ptr(), dtype_tag(codes.scalar_type()), cb.const_data_ptr<float>(), c.indptr.data_ptr(),
+                                 c.indices.data_ptr(), c.tag, out.mutable_data_ptr<float>(), c.n_dst, cb.size(0), cb.size(1), cb.size(2), dim,
+                                 (int)integer(a[5]), o.get(), st));
+    return THPVariable_Wrap(std::move(out));
+  });
+}
+
+// sq codes, sq codebooks, bits, column_slice, vq codes, vq codebooks, slot, indptr, indices, feat_dim, reduce, dropout, kernel, out_rows
+PyObject* two_level_spmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    arguments("two_level_spmm", n, 14);
+    const at::Tensor& sq = tensor(a[0], "sq_data", kCodes);
+    const at::Tensor& sq_cb = tensor(a[1], "sq_codebooks", kF32);
+    const at::Tensor& vq = tensor(a[4], "vq_data", kCodes);
+    const at::Tensor& vq_cb = tensor(a[5], "vq_codebooks", kF32);
+    const int32_t* slot = a[6] == Py_None ? nullptr : tensor(a[6], "slot", bit(F2C_I32)).const_data_ptr<int32_t>();
+    const Csc c = csc(a[7], a[8]);
+    if (vq_cb.dim() != 3 || sq.dim() != 2 || vq.dim() != 2) fail(PyExc_RuntimeError, "sq_data and vq_data must be 2-D and vq_codebooks 3-D");
+    const int64_t dim = integer(a[9]);
+    const Options o = options(a[11], a[12]);
+    c10::cuda::CUDAGuard guard(vq.device());
+    cudaStream_t st = stream_of(vq);
+    at::Tensor out = block_out(c.n_dst, dim, at::kFloat, vq.device(), a[13], st);
+    check_status(f2c_hybrid_spmm_csr(sq.data_ptr(), dtype_tag(sq.scalar_type()), sq_cb.const_data_ptr<float>(), sq_cb.size(0),
+                                     (int)integer(a[2]), integer(a[3]), sq.size(1), vq.data_ptr(), dtype_tag(vq.scalar_type()),
+                                     vq_cb.const_data_ptr<float>(), vq_cb.size(0), vq_cb.size(1), vq_cb.size(2), slot, sq.size(0),
+                                     c.indptr.data_ptr(), c.indices.data_ptr(), c.tag, out.mutable_data_ptr<float>(), c.n_dst, dim,
+                                     (int)integer(a[10]), o.get(), st));
+    return THPVariable_Wrap(std::move(out));
+  });
+}
+
+PyObject* set_error_class(PyObject*, PyObject* cls) {
+  Py_XSETREF(g_error_class, Py_NewRef(cls));
+  Py_RETURN_NONE;
+}
+
+PyMethodDef g_methods[] = {
+    {"sq_decompress", (PyCFunction)(void*)sq_decompress, METH_FASTCALL, nullptr},
+    {"vq_decompress", (PyCFunction)(void*)vq_decompress, METH_FASTCALL, nullptr},
+    {"spmm", (PyCFunction)(void*)spmm, METH_FASTCALL, nullptr},
+    {"sq_spmm", (PyCFunction)(void*)sq_spmm, METH_FASTCALL, nullptr},
+    {"vq_spmm", (PyCFunction)(void*)vq_spmm, METH_FASTCALL, nullptr},
+    {"two_level_spmm", (PyCFunction)(void*)two_level_spmm, METH_FASTCALL, nullptr},
+    {"set_error_class", set_error_class, METH_O, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+
+PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, g_methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+}  // namespace f2c_native
+
+PyMODINIT_FUNC PyInit__native(void) { return PyModule_Create(&f2c_native::g_module); }

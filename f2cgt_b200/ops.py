@@ -16,7 +16,10 @@ torch is used for memory and streams only; every computation is a kernel of libf
 import torch
 
 from . import _lib
+from . import _native  # the checks, allocation and launch of the calls below whose host time counts (native/ops.cpp)
 from ._lib import lib, check, Epilogue
+
+_native.set_error_class(_lib.F2CError)
 
 _DT = {torch.uint8: _lib.U8, torch.int8: _lib.I8, torch.int16: _lib.I16, torch.int32: _lib.I32,
        torch.int64: _lib.I64, torch.float16: _lib.F16, torch.float32: _lib.F32, torch.float64: _lib.F64}
@@ -72,11 +75,11 @@ def _epilogue(dropout, kernel="auto"):
                     int(dropout.get("seed", 0)) & 0xFFFFFFFFFFFFFFFF, int(dropout.get("offset", 0)), _lib.KERNELS[kernel])
 
 
-def _check_block(check, indptr, indices, n_src):
-    """check=True: verify the CSC block on the device first (indptr non-decreasing from 0, every index in [0, n_src));
+def _check_block(table, indptr, indices):
+    """check=True: verify the CSC block on the device first (indptr non-decreasing from 0, every index in [0, rows of the table));
     the fused kernels trust ``indices`` like the reference does, so a debugging caller can ask."""
-    if not check:
-        return
+    _csc(indptr, indices)
+    n_src = table.shape[0]
     flag = torch.zeros(1, dtype=torch.int32, device=indptr.device)
     with _on(indptr):
         _lib.check(lib.f2c_check_csc(_ptr(indptr), _ptr(indices), _DT[indptr.dtype], indptr.numel() - 1, int(n_src), _ptr(flag),
@@ -141,32 +144,13 @@ def sq_compress(src, codebooks, target_bits, column_slice):
 
 def sq_decompress(compress_data, codebooks, target_bits, column_slice, feat_dim):
     """src/sq_quantization.cu:158-182.  Codes [rows, src_dim] -> float32 [rows, feat_dim]."""
-    _chk(compress_data, "compress_data", (torch.uint8, torch.int8, torch.int16))
-    _chk(codebooks, "codebooks", (torch.float32,))
-    if compress_data.dim() != 2:
-        raise RuntimeError("compress_data must be 2-D")
-    rows, src_dim = compress_data.shape
-    out = torch.empty((rows, feat_dim), dtype=torch.float32, device=compress_data.device)
-    with _on(compress_data):
-        check(lib.f2c_sq_decompress(_ptr(compress_data), _DT[compress_data.dtype], _ptr(codebooks), codebooks.shape[0],
-                                    _ptr(out), rows, src_dim, feat_dim, target_bits, column_slice, _stream(compress_data)))
-    return out
+    return _native.sq_decompress(compress_data, codebooks, target_bits, column_slice, feat_dim)
 
 
 # ------------------------------------------------------------------ vector quantisation
 def vq_decompress(index_tensor, codebooks, feat_dim):
     """src/vq_quantization.cu:35-60.  Codes [rows, n_cb], codebooks [n_cb, K, cs] (fp32/fp16) -> fp32."""
-    _chk(index_tensor, "index_tensor", (torch.uint8, torch.int8, torch.int16))
-    _chk(codebooks, "codebooks", (torch.float32, torch.float16))
-    if index_tensor.dim() != 2 or codebooks.dim() != 3 or index_tensor.shape[1] != codebooks.shape[0]:
-        raise RuntimeError("index_tensor must be [rows, n_codebooks] and codebooks [n_codebooks, length, column_slice]")
-    rows = index_tensor.shape[0]
-    n_cb, K, cs = codebooks.shape
-    out = torch.empty((rows, feat_dim), dtype=torch.float32, device=index_tensor.device)
-    with _on(index_tensor):
-        check(lib.f2c_vq_decompress(_ptr(index_tensor), _DT[index_tensor.dtype], _ptr(codebooks), _DT[codebooks.dtype],
-                                    _ptr(out), rows, n_cb, K, cs, feat_dim, _stream(index_tensor)))
-    return out
+    return _native.vq_decompress(index_tensor, codebooks, feat_dim)
 
 
 # ------------------------------------------------------------------ aggregation
@@ -193,15 +177,7 @@ def _block_out(n_dst, width, dtype, device, out_rows):
 
 def spmm_csr(feat, indptr, indices, reduce="mean", out_rows=None):
     """src/fusion_spmm.cu:45-70.  Mean of neighbour rows; output has the dtype of ``feat``."""
-    _chk(feat, "feat", (torch.float32, torch.float16, torch.float64))
-    n_dst = _csc(indptr, indices)
-    if feat.dim() != 2:
-        raise RuntimeError("feat must be 2-D")
-    out = _block_out(n_dst, feat.shape[1], feat.dtype, feat.device, out_rows)
-    with _on(feat):
-        check(lib.f2c_spmm_csr(_ptr(feat), _DT[feat.dtype], _ptr(indptr), _ptr(indices), _DT[indptr.dtype], _ptr(out), n_dst,
-                               feat.shape[1], _REDUCE[reduce], _stream(feat)))
-    return out
+    return _native.spmm(feat, indptr, indices, _REDUCE[reduce], out_rows)
 
 
 def spmm_csr_backward(grad_out, indptr, indices, n_src, reduce="mean"):
@@ -221,20 +197,10 @@ def spmm_csr_backward(grad_out, indptr, indices, n_src, reduce="mean"):
 def sq_decompress_spmm_csr(compress_feat, codebooks, indptr, indices, target_bit, column_slice, feat_dim, reduce="mean",
                            dropout=None, kernel="auto", check=False, out_rows=None):
     """src/fusion_spmm.cu:240-272.  Fused SQ decode + mean aggregation -> float32 [n_dst, feat_dim]."""
-    _chk(compress_feat, "compress_feat", (torch.uint8, torch.int8, torch.int16))
-    _chk(codebooks, "codebooks", (torch.float32,))
-    n_dst = _csc(indptr, indices)
-    if compress_feat.dim() != 2:
-        raise RuntimeError("compress_feat must be 2-D")
-    _check_block(check, indptr, indices, compress_feat.shape[0])
-    out = _block_out(n_dst, feat_dim, torch.float32, compress_feat.device, out_rows)
-    ep = _epilogue(dropout, kernel)
-    with _on(compress_feat):
-        _lib.check(lib.f2c_sq_spmm_csr(_ptr(compress_feat), _DT[compress_feat.dtype], _ptr(codebooks), codebooks.shape[0],
-                                  _ptr(indptr), _ptr(indices), _DT[indptr.dtype], _ptr(out), n_dst, compress_feat.shape[0],
-                                       compress_feat.shape[1], feat_dim, target_bit, column_slice, _REDUCE[reduce], ep,
-                                       _stream(compress_feat)))
-    return out
+    if check:
+        _check_block(compress_feat, indptr, indices)
+    return _native.sq_spmm(compress_feat, codebooks, indptr, indices, target_bit, column_slice, feat_dim, _REDUCE[reduce], dropout,
+                           _lib.KERNELS[kernel], out_rows)
 
 
 def peer_first_cold_id(n_replicated, rows_per_shard):
@@ -277,20 +243,9 @@ def sq_decompress_spmm_csr_peer(peer_table, codebooks, indptr, indices, target_b
 def vq_decompress_spmm_csr(compress_feat, codebooks, indptr, indices, feat_dim, reduce="mean", dropout=None, kernel="auto",
                            check=False, out_rows=None):
     """src/fusion_spmm.cu:107-141.  Fused VQ decode + mean aggregation -> float32 [n_dst, feat_dim]."""
-    _chk(compress_feat, "compress_feat", (torch.uint8, torch.int8, torch.int16))
-    _chk(codebooks, "codebooks", (torch.float32,))
-    n_dst = _csc(indptr, indices)
-    if compress_feat.dim() != 2 or codebooks.dim() != 3 or compress_feat.shape[1] != codebooks.shape[0]:
-        raise RuntimeError("compress_feat must be [rows, n_codebooks] and codebooks [n_codebooks, length, column_slice]")
-    n_cb, K, cs = codebooks.shape
-    _check_block(check, indptr, indices, compress_feat.shape[0])
-    out = _block_out(n_dst, feat_dim, torch.float32, compress_feat.device, out_rows)
-    ep = _epilogue(dropout, kernel)
-    with _on(compress_feat):
-        _lib.check(lib.f2c_vq_spmm_csr(_ptr(compress_feat), _DT[compress_feat.dtype], _ptr(codebooks), _ptr(indptr), _ptr(indices),
-                                  _DT[indptr.dtype], _ptr(out), n_dst, n_cb, K, cs, feat_dim, _REDUCE[reduce], ep,
-                                  _stream(compress_feat)))
-    return out
+    if check:
+        _check_block(compress_feat, indptr, indices)
+    return _native.vq_spmm(compress_feat, codebooks, indptr, indices, feat_dim, _REDUCE[reduce], dropout, _lib.KERNELS[kernel], out_rows)
 
 
 def fusion_decompress(sq_data, sq_codebooks, target_bits, column_slice, vq_data, vq_codebooks, feat_dim):
@@ -315,23 +270,10 @@ def two_level_decompress_spmm_csr(sq_data, sq_codebooks, target_bits, column_sli
     """Two-level aggregation in one launch.  Source row s is decoded from row ``slot[s]`` of the SQ table
     when ``slot[s] >= 0`` (int32), from row s of the VQ table otherwise; then the reference mean.
     ``slot=None``: hot-first numbering - the hot nodes are ids ``0 .. len(sq_data) - 1`` and node s reads SQ row s."""
-    _chk(sq_data, "sq_data", (torch.uint8, torch.int8, torch.int16))
-    _chk(sq_codebooks, "sq_codebooks", (torch.float32,))
-    _chk(vq_data, "vq_data", (torch.uint8, torch.int8, torch.int16))
-    _chk(vq_codebooks, "vq_codebooks", (torch.float32,))
-    if slot is not None:
-        _chk(slot, "slot", (torch.int32,))
-    n_dst = _csc(indptr, indices)
-    n_cb, K, cs = vq_codebooks.shape
-    _check_block(check, indptr, indices, vq_data.shape[0])
-    out = _block_out(n_dst, feat_dim, torch.float32, vq_data.device, out_rows)
-    ep = _epilogue(dropout, kernel)
-    with _on(vq_data):
-        _lib.check(lib.f2c_hybrid_spmm_csr(_ptr(sq_data), _DT[sq_data.dtype], _ptr(sq_codebooks), sq_codebooks.shape[0],
-                                      target_bits, column_slice, sq_data.shape[1], _ptr(vq_data), _DT[vq_data.dtype],
-                                      _ptr(vq_codebooks), n_cb, K, cs, _ptr(slot), sq_data.shape[0], _ptr(indptr), _ptr(indices),
-                                      _DT[indptr.dtype], _ptr(out), n_dst, feat_dim, _REDUCE[reduce], ep, _stream(vq_data)))
-    return out
+    if check:
+        _check_block(vq_data, indptr, indices)
+    return _native.two_level_spmm(sq_data, sq_codebooks, target_bits, column_slice, vq_data, vq_codebooks, slot, indptr, indices, feat_dim,
+                                  _REDUCE[reduce], dropout, _lib.KERNELS[kernel], out_rows)
 
 
 def two_level_decompress_spmm_csr_peer(sq_peers, sq_codebooks, target_bits, column_slice, vq_peers, vq_codebooks, slot_peers, indptr,
