@@ -6,6 +6,7 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/Dtype.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "../../include/f2cgt_b200.h"
@@ -105,6 +106,9 @@ inline int unlocked(F&& call) {
   PyEval_RestoreThread(s);
   return rc;
 }
+
+
+extern PyMethodDef g_sage_methods[];  // sage.cpp
 
 void arguments(const char* name, Py_ssize_t got, Py_ssize_t want);
 

@@ -203,4 +203,8 @@ PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, g_methods
 }  // namespace
 }  // namespace f2c_native
 
-PyMODINIT_FUNC PyInit__native(void) { return PyModule_Create(&f2c_native::g_module); }
+PyMODINIT_FUNC PyInit__native(void) {
+  PyObject* m = PyModule_Create(&f2c_native::g_module);
+  if (m != nullptr && PyModule_AddFunctions(m, f2c_native::g_sage_methods) != 0) Py_CLEAR(m);
+  return m;
+}

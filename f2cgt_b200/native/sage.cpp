@@ -1,0 +1,289 @@
+// A GraphSAGE network over a minibatch's blocks as ONE autograd node: what f2cgt_b200/sage.py's layers do (products, bias, ReLU,
+// dropout, mean aggregation over the hidden layers), forward and backward, without an interpreter or an autograd node in
+// between.  A training step was bound by the host: about seventy launches, each behind 10-20 us of Python and dispatcher.
+//
+// The forward products are the library's kernel where products may use tf32 (csrc/sage_gemm.cu: both products of a layer, bias
+// and ReLU in one launch, the same sums as the two library products it replaces, see use_own()).  All other products are
+// torch's, on row counts padded by sage._bucket as in the Python layers: their sums over 10^3 .. 10^5 rows depend on how they
+// are split, and a weight gradient that differs by 10^-5 is enough for Adam's first steps to go the other way on a weight whose
+// gradient is nearly zero.  What changes there is the time around them: the mask of ReLU and dropout, with the bias gradient, is
+// one pass (csrc/sage_mask.cu), and the weight gradients, which cuBLAS gives to a few CTAs each, run on a second stream
+// beside the input gradients and each other.  Dropout is torch's own, over the padded rows, so that masks are the ones
+// torch.nn.Dropout would draw.
+#include "native.h"
+
+#include <array>
+
+#include <ATen/cuda/CUDAEvent.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/autograd/variable.h>
+
+namespace f2c_native {
+namespace {
+
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+
+struct Layer {
+  int64_t rows = 0, padded = 0;       // destination rows of the block, and the row count dropout sees
+  at::Tensor indptr, indices;         // hidden layers: the block over the previous layer's rows
+};
+
+struct Net {
+  std::vector<Layer> layers;
+  double p = 0.0;                     // dropout between the layers (0 outside training)
+  bool tf32 = false;                  // forward products may be the library's
+  c10::optional<at::ScalarType> cast; // operand type of torch's products
+  double scale() const { return p < 1.0 ? 1.0 / (1.0 - p) : 0.0; }
+};
+
+struct Status {  // library status inside a node (no Python exception there)
+  void operator=(int rc) const { TORCH_CHECK(rc == F2C_OK, "f2cgt_b200: ", f2c_last_error()); }
+};
+constexpr Status checked{};
+
+float* f32(const at::Tensor& t) { return (float*)t.data_ptr(); }
+
+at::Tensor mm(const Net& net, const at::Tensor& a, const at::Tensor& b) {
+  return net.cast ? at::mm(a.to(*net.cast), b.to(*net.cast)).to(at::kFloat) : at::mm(a, b);
+}
+void addmm_(const Net& net, at::Tensor& y, const at::Tensor& a, const at::Tensor& b) {
+  if (net.cast) y.add_(mm(net, a, b)); else y.addmm_(a, b);
+}
+
+// Whether a layer's forward product is the library's kernel.  Its result equals torch's two products bit for bit for k % 32 == 0
+// (checked for k = 64 .. 256, n = 16 .. 256, 2 .. 61,440 rows) and, for other k, from some ten thousand rows on; below that cuBLAS sums in
+// another order, which a training run would notice (see above) and inference does not.
+bool use_own(const Net& net, int64_t rows, int64_t k, bool record) {
+  return net.tf32 && k % 4 == 0 && rows > 1 && (!record || k % 32 == 0 || rows >= 16384);
+}
+
+void zero_tail(at::Tensor& t, int64_t rows, cudaStream_t st) {
+  if (t.size(0) > rows) C10_CUDA_CHECK(cudaMemsetAsync(f32(t) + rows * t.size(1), 0, (size_t)((t.size(0) - rows) * t.size(1)) * 4, st));
+}
+
+// y of one layer (before dropout), `padded` rows
+at::Tensor layer_forward(const Net& net, const at::Tensor& x1, const at::Tensor& x2, const at::Tensor* w, const Layer& l, bool relu, bool record,
+                         cudaStream_t st) {
+  const at::Tensor &w1 = w[0], &w2 = w[1], &bias = w[2];
+  if (use_own(net, l.rows, w1.size(1), record)) {
+    at::Tensor y = empty({l.padded, w1.size(0)}, at::kFloat, x1.device());
+    checked = f2c_sage_forward(f32(x1), f32(x2), f32(w1), f32(w2), bias.defined() ? f32(bias) : nullptr, f32(y), l.rows, w1.size(0), w1.size(1),
+                               relu ? 1 : 0, st);
+    zero_tail(y, l.rows, st);
+    return y;
+  }
+  const at::Tensor a = x1.narrow(0, 0, l.padded), b = x2.narrow(0, 0, l.padded);
+  at::Tensor y;
+  if (bias.defined() && !net.cast) {
+    y = at::addmm(bias, a, w1.t());
+  } else {
+    y = mm(net, a, w1.t());
+    if (bias.defined()) y.add_(bias);
+  }
+  addmm_(net, y, b, w2.t());
+  if (relu) y.relu_();
+  return y;
+}
+
+// The stream beside the caller's on which weight gradients run, and the events that tie the two; one set per thread and device.
+struct Beside {
+  c10::optional<c10::cuda::CUDAStream> stream;
+  at::cuda::CUDAEvent fork{cudaEventDisableTiming}, join{cudaEventDisableTiming};
+};
+Beside& beside(c10::DeviceIndex device) {
+  // never freed: at thread exit the CUDA context may be gone before the events
+  static thread_local std::array<Beside*, 64> all{};
+  Beside*& b = all[(size_t)device & 63];
+  if (b == nullptr) {
+    b = new Beside();
+    b->stream = c10::cuda::getStreamFromPool(false, device);
+  }
+  return *b;
+}
+constexpr int64_t kBesideRows = 4096;  // fewer rows: a product is shorter than the calls that would move it
+
+struct SageBackward : public torch::autograd::Node {
+  Net net;
+  std::vector<SavedVariable> weights;   // per layer: self, neigh, bias
+  std::vector<at::Tensor> x1, x2;       // inputs of the layers' products
+  std::vector<at::Tensor> out;          // outputs after ReLU and dropout (all layers but the last)
+  bool released = false;
+
+  std::string name() const override { return "SageBackward"; }
+  void release_variables() override {
+    released = true;
+    weights.clear(); x1.clear(); x2.clear(); out.clear();
+  }
+
+  variable_list apply(variable_list&& grads) override {
+    TORCH_CHECK(!released, "Trying to backward through the graph a second time: its saved tensors have been freed");
+    const size_t L = net.layers.size();
+    variable_list result(3 * L);
+    if (!grads[0].defined()) return result;
+    at::NoGradGuard no_grad;
+    const at::Tensor given = grads[0].to(at::kFloat);
+    c10::cuda::CUDAGuard guard(given.device());
+    const c10::cuda::CUDAStream main = at::cuda::getCurrentCUDAStream(given.device().index());
+    cudaStream_t st = main.stream();
+    auto self = shared_from_this();
+    std::vector<at::Tensor> w(3 * L);
+    int64_t biases = 0;
+    for (size_t i = 0; i < 3 * L; ++i) {
+      w[i] = weights[i].unpack(self);
+      if (i % 3 == 2 && w[i].defined()) biases += (w[i].numel() + 63) / 64 * 64;
+    }
+    at::Tensor bias_grads = empty({biases}, at::kFloat, given.device());  // the mask kernel adds to it
+    if (biases > 0) C10_CUDA_CHECK(cudaMemsetAsync(bias_grads.data_ptr(), 0, (size_t)biases * 4, st));
+
+    // gradient of the last layer's output on its padded rows
+    at::Tensor g = given.contiguous();
+    if (net.layers[L - 1].padded > g.size(0)) {
+      at::Tensor padded = empty({net.layers[L - 1].padded, g.size(1)}, at::kFloat, g.device());
+      C10_CUDA_CHECK(cudaMemcpyAsync(padded.data_ptr(), g.data_ptr(), (size_t)g.numel() * 4, cudaMemcpyDeviceToDevice, st));
+      zero_tail(padded, g.size(0), st);
+      g = padded;
+    }
+    Beside& side = beside(given.device().index());
+    bool forked = false;
+    std::vector<at::Tensor> keep;  // what the side stream reads, until the streams have joined
+    int64_t bias_at = 0;
+    for (size_t i = L; i-- > 0;) {
+      const Layer& l = net.layers[i];
+      const at::Tensor* wi = &w[3 * i];
+      const int64_t n = wi[0].size(0), k = wi[0].size(1), m = g.size(0);
+      at::Tensor db;
+      if (wi[2].defined()) {
+        db = bias_grads.narrow(0, bias_at, n);
+        bias_at += (n + 63) / 64 * 64;
+      }
+      at::Tensor dy = g;
+      if (i + 1 < L) {
+        dy = empty({m, n}, at::kFloat, g.device());
+        checked = f2c_sage_mask(f32(g), f32(out[i]), (float)net.scale(), f32(dy), db.defined() ? f32(db) : nullptr, m, n, st);
+      } else if (db.defined()) {
+        at::sum_out(db, dy, 0);
+      }
+      result[3 * i + 2] = db;
+      const at::Tensor dyt = dy.t();
+      const bool apart = m >= kBesideRows;
+      if (apart) {
+        side.fork.record(main);
+        side.fork.block(*side.stream);
+        c10::cuda::CUDAStreamGuard on_side(*side.stream);
+        result[3 * i + 1] = mm(net, dyt, x2[i].narrow(0, 0, m));
+        if (i > 0) result[3 * i] = mm(net, dyt, x1[i].narrow(0, 0, m));
+        side.join.record(*side.stream);
+        forked = true;
+        keep.push_back(dy);
+      } else {
+        result[3 * i + 1] = mm(net, dyt, x2[i].narrow(0, 0, m));
+      }
+      if (!apart || i == 0) result[3 * i] = mm(net, dyt, x1[i].narrow(0, 0, m));
+      if (i > 0) {
+        at::Tensor dh = empty({net.layers[i - 1].padded, k}, at::kFloat, g.device());  // gradient of the previous layer's output
+        const at::Tensor d_neigh = mm(net, dy, wi[1]);
+        checked = f2c_spmm_csr_backward(f32(d_neigh), l.indptr.data_ptr(), l.indices.data_ptr(), dtype_tag(l.indptr.scalar_type()), f32(dh), l.rows,
+                                        dh.size(0), k, F2C_MEAN, st);
+        at::Tensor head = dh.narrow(0, 0, m);
+        addmm_(net, head, dy, wi[0]);
+        g = dh;
+      }
+    }
+    if (forked) side.join.block(main);
+    for (size_t i = 0; i < 3 * L; ++i)
+      if (!task_should_compute_output(i)) result[i] = at::Tensor();
+    return result;
+  }
+};
+
+// h_self, h_neigh, indptrs (list, layers 1..), indices (list), rows (list), padded (list), weights (list of 3 L, None = no bias),
+// dropout p, tf32 products allowed (bool), operand type of torch's products (torch.dtype or None)
+PyObject* sage_net(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    arguments("sage_net", n, 10);
+    const at::Tensor& h_self = tensor(a[0], "h_self", kF32);
+    const at::Tensor& h_neigh = tensor(a[1], "h_neigh", kF32);
+    auto list = [](PyObject* o, Py_ssize_t want) {
+      if (!PyList_Check(o) || (want >= 0 && PyList_GET_SIZE(o) != want)) fail(PyExc_TypeError, "sage_net: lists of matching lengths are wanted");
+      return PyList_GET_SIZE(o);
+    };
+    const Py_ssize_t L = list(a[4], -1);
+    list(a[2], L - 1); list(a[3], L - 1); list(a[5], L); list(a[6], 3 * L);
+    Net net;
+    net.layers.resize(L);
+    std::vector<at::Tensor> w(3 * L);
+    for (Py_ssize_t i = 0; i < L; ++i) {
+      Layer& l = net.layers[i];
+      l.rows = integer(PyList_GET_ITEM(a[4], i));
+      l.padded = integer(PyList_GET_ITEM(a[5], i));
+      if (l.rows < 0 || l.padded < l.rows) fail(PyExc_RuntimeError, "sage_net: bad row counts");
+      if (i > 0) {
+        l.indptr = tensor(PyList_GET_ITEM(a[2], i - 1), "indptr", kIndex);
+        l.indices = tensor(PyList_GET_ITEM(a[3], i - 1), "indices", kIndex);
+        if (l.indptr.scalar_type() != l.indices.scalar_type()) fail(PyExc_RuntimeError, "indptr and indices must have the same dtype");
+        if (l.indptr.numel() != l.rows + 1 || l.rows > net.layers[i - 1].rows || l.padded > net.layers[i - 1].padded) fail(PyExc_RuntimeError, "sage_net: blocks do not fit together");
+      }
+      for (int j = 0; j < 3; ++j) {
+        PyObject* o = PyList_GET_ITEM(a[6], 3 * i + j);
+        if (j == 2 && o == Py_None) continue;
+        w[3 * i + j] = tensor(o, "weight", kF32);
+      }
+      const at::Tensor &w1 = w[3 * i], &w2 = w[3 * i + 1];
+      const int64_t in = i == 0 ? h_self.size(1) : w[3 * i - 3].size(0);
+      if (w1.dim() != 2 || w1.sizes() != w2.sizes() || w1.size(1) != in || (w[3 * i + 2].defined() && w[3 * i + 2].numel() != w1.size(0)))
+        fail(PyExc_RuntimeError, "sage_net: weights do not fit together");
+    }
+    net.p = real(a[7]);
+    net.tf32 = PyObject_IsTrue(a[8]) == 1;
+    if (a[9] != Py_None) net.cast = reinterpret_cast<THPDtype*>(a[9])->scalar_type;
+    if (h_self.dim() != 2 || h_self.sizes() != h_neigh.sizes() || h_self.size(0) < net.layers[0].padded) fail(PyExc_RuntimeError, "sage_net: bad inputs");
+    const bool record = at::GradMode::is_enabled() && torch::autograd::compute_requires_grad(w);
+
+    c10::cuda::CUDAGuard guard(h_self.device());
+    cudaStream_t st = stream_of(h_self);
+    std::shared_ptr<SageBackward> node;
+    if (record) {
+      node = std::shared_ptr<SageBackward>(new SageBackward(), torch::autograd::deleteNode);
+      node->set_next_edges(torch::autograd::collect_next_edges(w));
+    }
+    at::Tensor h;
+    {
+      at::AutoDispatchBelowADInplaceOrView below;
+      at::Tensor x1 = h_self, x2 = h_neigh;
+      for (Py_ssize_t i = 0; i < L; ++i) {
+        const Layer& l = net.layers[i];
+        const bool last = i + 1 == L;
+        if (i > 0) {
+          x1 = h;
+          x2 = empty({l.padded, h.size(1)}, at::kFloat, h.device());
+          zero_tail(x2, l.rows, st);
+          checked = f2c_spmm_csr(h.data_ptr(), F2C_F32, l.indptr.data_ptr(), l.indices.data_ptr(), dtype_tag(l.indptr.scalar_type()), x2.data_ptr(),
+                                 l.rows, h.size(1), F2C_MEAN, st);
+        }
+        h = layer_forward(net, x1, x2, &w[3 * i], l, !last, record, st);
+        if (!last && net.p > 0) h = at::dropout(h, net.p, true);
+        if (record) {
+          node->x1.push_back(x1);
+          node->x2.push_back(x2);
+          if (!last) node->out.push_back(h);
+        }
+      }
+      if (h.size(0) > net.layers[L - 1].rows) h = h.narrow(0, 0, net.layers[L - 1].rows);
+    }
+    if (record) {
+      for (const at::Tensor& t : w) node->weights.emplace_back(t, false);
+      node->net = std::move(net);
+      torch::autograd::set_history(h, node);
+    }
+    return THPVariable_Wrap(std::move(h));
+  });
+}
+
+}  // namespace
+
+PyMethodDef g_sage_methods[] = {{"sage_net", (PyCFunction)(void*)sage_net, METH_FASTCALL, nullptr}, {nullptr, nullptr, 0, nullptr}};
+
+}  // namespace f2c_native

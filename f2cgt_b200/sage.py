@@ -341,6 +341,9 @@ class SAGE(nn.Module):
         self.dropout = nn.Dropout(dropout)
 
     def forward(self, blocks, x=None):
+        weights = self._plain_weights() if x is None and len(blocks) == len(self.layers) else None
+        if weights is not None:
+            return self._forward_as_one_node(blocks, weights)
         h = x
         for i, (layer, block) in enumerate(zip(self.layers, blocks)):
             h = layer.forward_padded(block, h)
@@ -348,6 +351,49 @@ class SAGE(nn.Module):
                 h = self.dropout(torch.relu(h))
         n_out = blocks[-1]["dst_nodes"].numel()
         return h if h.shape[0] == n_out else h[:n_out]
+
+    def _plain_weights(self):
+        """[self, neigh, bias] of every layer, or None when the layers are not just these tensors (subclasses, hooks,
+        parametrisations, other dtypes, autocast): then every layer is called on its own."""
+        if torch.is_autocast_enabled("cuda") or type(self.dropout) is not nn.Dropout or _hooked(self.dropout):
+            return None
+        weights = []
+        for i, layer in enumerate(self.layers._modules.values()):
+            if type(layer) is not (SAGEConv if i else MySAGEConv) or _hooked(layer):
+                return None
+            parts = layer._modules
+            fc_self, fc_neigh = parts["fc_self"], parts["fc_neigh"]
+            for fc in (fc_self, fc_neigh):
+                if type(fc) is not nn.Linear or _hooked(fc):
+                    return None
+            bias = fc_self._parameters["bias"]
+            three = [fc_self._parameters["weight"], fc_neigh._parameters["weight"], bias]
+            for w in three:
+                if w is not None and (w.dtype is not torch.float32 or not w.is_cuda or not w.is_contiguous()):
+                    return None
+            if fc_neigh._parameters["bias"] is not None:
+                return None
+            weights += three
+        return weights
+
+    def _forward_as_one_node(self, blocks, weights):
+        """The whole network as one autograd node (native/sage.cpp): the layers' arithmetic without their host time."""
+        first = blocks[0]
+        sm, neighbours, dst = first.get("first_layer_input") or self.layers[0].sm.for_block(first)
+        rows, padded = [dst.numel()], [_bucket(dst.numel())]
+        for block in blocks[1:]:
+            rows.append(block["dst_nodes"].numel())
+            padded.append(min(_bucket(rows[-1]), padded[-1]))
+        h_neigh = sm.aggregate(first["indptr"], neighbours, out_rows=padded[0])  # raw codes in, no autograd through it
+        h_self = sm.decode_rows(dst, out_rows=padded[0])
+        p = self.dropout.p if self.dropout.training else 0.0
+        tf32 = _PRODUCT_DTYPE is None and torch.backends.cuda.matmul.allow_tf32
+        return ops._native.sage_net(h_self, h_neigh, [b["indptr"] for b in blocks[1:]], [b["indices_local"] for b in blocks[1:]], rows, padded,
+                                    weights, p, tf32, _PRODUCT_DTYPE)
+
+
+def _hooked(module):
+    return bool(module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks)
 
 
 class GPUSamplingDataloader:

@@ -131,6 +131,16 @@ int f2c_spmm_csr(const void* feat, int feat_dtype, const void* indptr, const voi
 int f2c_spmm_csr_backward(const float* grad_out, const void* indptr, const void* indices, int index_dtype,
                           float* grad_src, int64_t n_dst, int64_t n_src, int64_t feat_dim, int reduce, void* stream);
 
+/* Forward product of a SAGE layer (fc_self and fc_neigh of examples/conv.py:62-76 together), fp32 storage, tf32 operands
+ * (rounded to nearest), fp32 accumulation: y [m, n] = (x1 [m, k] w1 [n, k]^T + bias [n]) + x2 w2^T (bias may be NULL), then
+ * max(0, .) when relu != 0.  Row-major, operands 16-byte aligned, k % 4 == 0 (else F2C_ERR_UNSUPPORTED). */
+int f2c_sage_forward(const float* x1, const float* x2, const float* w1, const float* w2, const float* bias, float* y, int64_t m,
+                     int64_t n, int64_t k, int relu, void* stream);
+
+/* Gradient through dropout and ReLU of a layer whose output after both is h: dy = h > 0 ? scale * g : 0 (scale = what dropout
+ * multiplies survivors with), and db [n] += column sums of dy (db may be NULL; no fixed order).  g, h, dy [rows, n] f32. */
+int f2c_sage_mask(const float* g, const float* h, float scale, float* dy, float* db, int64_t rows, int64_t n, void* stream);
+
 /* sq_decompress_spmm_csr(compress_feat, codebooks, indptr, indices, target_bit, column_slice, feat_dim)
  *  -  src/fusion_spmm.cu:240-272 (kernel :143-238).  out [n_dst, feat_dim] f32; the decoded rows are
  * never written to memory.  n_src = number of rows of `codes` (compress_feat.size(0)); every index

@@ -248,3 +248,79 @@ def test_bf16_product_operands_stay_close_to_fp32(capi):
         assert p.grad.dtype == torch.float32 and torch.isfinite(p.grad).all()
         assert float((p.grad - a).abs().max()) < 0.15 * float(a.abs().max()) + 1e-6
     assert sage._PRODUCT_DTYPE is None  # the context manager restored the default
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 1, 4), (127, 16, 32), (128, 128, 128), (129, 172, 100), (1000, 171, 64), (4097, 128, 256), (300, 300, 260),
+                                   (40_001, 64, 128), (600, 47, 12)])
+def test_layer_product_on_tensor_cores(capi, m, n, k):
+    """Forward product of a layer against float64 (operands carry 10 mantissa bits); rows behind m stay untouched."""
+    from f2cgt_b200 import ops
+    from f2cgt_b200._lib import check, lib
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    x1, x2, w1, w2, b = rnd(m, k), rnd(m, k), rnd(n, k), rnd(n, k), rnd(n)
+    sums = x1.double() @ w1.double().t() + x2.double() @ w2.double().t()
+    parts = x1.double().abs() @ w1.double().abs().t() + x2.double().abs() @ w2.double().abs().t()
+    for relu in (0, 1):
+        for bias in (b, None):
+            y = torch.full((m + 1, n), float("nan"), device="cuda")
+            check(lib.f2c_sage_forward(x1.data_ptr(), x2.data_ptr(), w1.data_ptr(), w2.data_ptr(), 0 if bias is None else bias.data_ptr(),
+                                       y.data_ptr(), m, n, k, relu, ops._stream(x1)))
+            want = sums if bias is None else sums + bias.double()
+            want = want.clamp_min(0) if relu else want
+            assert bool(((y[:m].double() - want).abs() <= 1.5e-3 * parts + 1e-6).all()) and bool(y[m].isnan().all())
+    assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("rows,n", [(1, 1), (1000, 128), (4097, 47), (333, 260), (5, 1500)])
+def test_relu_dropout_mask_and_bias_gradient(capi, rows, n):
+    from f2cgt_b200 import ops
+    from f2cgt_b200._lib import check, lib
+    g = torch.Generator(device="cuda").manual_seed(rows + n)
+    grad, h, db = torch.randn(rows, n, generator=g, device="cuda"), torch.randn(rows, n, generator=g, device="cuda"), torch.ones(n, device="cuda")
+    dy = torch.empty_like(grad)
+    check(lib.f2c_sage_mask(grad.data_ptr(), h.data_ptr(), 2.0, dy.data_ptr(), db.data_ptr(), rows, n, ops._stream(h)))
+    want = torch.where(h > 0, grad * 2.0, 0.0)
+    assert torch.equal(dy, want)
+    assert torch.allclose(db.double(), 1 + want.double().sum(0), rtol=1e-5, atol=1e-5 * rows**0.5)
+
+
+@pytest.mark.parametrize("tf32,product,D,hidden,classes,dropout", [(True, None, 128, 128, 172, 0.5), (True, None, 100, 64, 47, 0.0), (False, None, 64, 96, 10, 0.5),
+                                                                   (True, torch.bfloat16, 128, 64, 20, 0.3), (True, None, 64, 30, 7, 0.5)])
+def test_network_as_one_node_equals_the_layers(capi, tf32, product, D, hidden, classes, dropout):
+    """One autograd node for the whole network == its layers called one by one (same dropout masks), forward and gradients;
+    a batch that is no multiple of the padding, with and without gradients."""
+    from f2cgt_b200 import sage, synth
+    n = 20000
+    indptr, indices = synth.power_law_graph(n, 12, 2.1, seed=1, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(5)
+    codes = torch.randint(0, 256, (n, (D + 31) // 32), generator=g, dtype=torch.uint8, device="cuda")
+    cm = sage.CompressionManager(D, ["vq"], [(32, -1)], [torch.randn((D + 31) // 32, 256, 32, generator=g, device="cuda")], [codes])
+    seeds = torch.randperm(n, generator=g, device="cuda")[:233]
+    before = torch.backends.cuda.matmul.allow_tf32
+    torch.backends.cuda.matmul.allow_tf32 = tf32
+    try:
+        torch.manual_seed(1)
+        model = sage.SAGE(D, hidden, classes, 3, dropout, cm).to("cuda")
+        _, _, blocks = next(iter(sage.GPUSamplingDataloader(indptr, indices, seeds, 233, (6, 5, 4), shuffle=False)))
+        weight = torch.randn(233, classes, generator=g, device="cuda")
+        got = []
+        for one_node in (True, False):
+            handle = None if one_node else model.layers[1].register_forward_pre_hook(lambda *_: None)  # a hook: layer by layer
+            assert (model._plain_weights() is not None) == one_node
+            torch.manual_seed(7)
+            model.zero_grad(set_to_none=True)
+            with sage.products_in(product):
+                out = model(blocks)
+                (out * weight).sum().backward()
+            with torch.no_grad():
+                quiet = model.eval()(blocks)
+            model.train()
+            got.append([out.detach(), quiet] + [p.grad for p in model.parameters()])
+            if handle is not None:
+                handle.remove()
+        tol = 1e-5 if not tf32 else 5e-3 if product is None else 2e-2
+        for a, b in zip(*got):
+            assert a.shape == b.shape and float((a - b).norm() / b.norm()) < tol
+    finally:
+        torch.backends.cuda.matmul.allow_tf32 = before
