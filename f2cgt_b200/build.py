@@ -72,7 +72,7 @@ def build_native(force=False, jobs=8):
     if commands or not os.path.exists(NATIVE):
         libs = [f"-L{d}" for d in library_paths() + [os.path.join(cuda, "lib64"), PKG]]
         link = ["g++", "-shared", "-o", NATIVE] + objs + libs + ["-l:libf2cgt_b200.so", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda",
-                                                                "-ltorch_python", "-ltorch", "-lcudart", "-Wl,-rpath,$ORIGIN"]
+                                                                "-ltorch_python", "-ltorch", "-lcudart", "-lcublas", "-Wl,-rpath,$ORIGIN"]
         _run_all([(link, NATIVE)], 1)
     return NATIVE
 

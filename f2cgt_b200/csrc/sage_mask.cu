@@ -10,7 +10,8 @@ namespace {
 
 constexpr int kThreads = 256;
 
-template <bool VEC>
+// MASK = false: only the column sums of g
+template <bool VEC, bool MASK>
 __global__ void __launch_bounds__(kThreads) sage_mask_kernel(const float* __restrict__ g, const float* __restrict__ h, float scale,
                                                              float* __restrict__ dy, float* __restrict__ db, int64_t rows, int n, int units) {
   constexpr int E = VEC ? 4 : 1;
@@ -27,14 +28,19 @@ __global__ void __launch_bounds__(kThreads) sage_mask_kernel(const float* __rest
     for (int64_t r = (int64_t)blockIdx.x * lanes + local; r < rows; r += step) {
       const int64_t at = r * n + c;
       if (VEC) {
-        const float4 a = __ldcs(reinterpret_cast<const float4*>(g + at)), b = __ldcs(reinterpret_cast<const float4*>(h + at));
-        const float4 v = make_float4(b.x > 0.f ? a.x * scale : 0.f, b.y > 0.f ? a.y * scale : 0.f, b.z > 0.f ? a.z * scale : 0.f,
-                                     b.w > 0.f ? a.w * scale : 0.f);
-        *reinterpret_cast<float4*>(dy + at) = v;
+        float4 v = __ldcs(reinterpret_cast<const float4*>(g + at));
+        if (MASK) {
+          const float4 b = __ldcs(reinterpret_cast<const float4*>(h + at));
+          v = make_float4(b.x > 0.f ? v.x * scale : 0.f, b.y > 0.f ? v.y * scale : 0.f, b.z > 0.f ? v.z * scale : 0.f, b.w > 0.f ? v.w * scale : 0.f);
+          *reinterpret_cast<float4*>(dy + at) = v;
+        }
         s[0] += v.x; s[E > 1 ? 1 : 0] += v.y; s[E > 2 ? 2 : 0] += v.z; s[E > 3 ? 3 : 0] += v.w;
       } else {
-        const float v = h[at] > 0.f ? g[at] * scale : 0.f;
-        dy[at] = v;
+        float v = g[at];
+        if (MASK) {
+          v = h[at] > 0.f ? v * scale : 0.f;
+          dy[at] = v;
+        }
         s[0] += v;
       }
     }
@@ -58,13 +64,53 @@ extern "C" int f2c_sage_mask(const float* g, const float* h, float scale, float*
   const char* op = "sage_mask";
   F2C_REQUIRE(rows >= 0 && n >= 0 && n <= 8192, F2C_ERR_LIMIT, "%s: bad shape", op);
   if (rows * n == 0) return F2C_OK;
-  F2C_REQUIRE(g && h && dy, F2C_ERR_INVALID, "%s: null pointer", op);
+  F2C_REQUIRE(g && (h != nullptr ? dy != nullptr : db != nullptr), F2C_ERR_INVALID, "%s: null pointer", op);
   const bool vec = n % 4 == 0 && aligned(g, 16) && aligned(h, 16) && aligned(dy, 16);
   const int units = (int)(vec ? n / 4 : n);
   const int lanes = units < kThreads ? kThreads / units : 1;
   int64_t grid = ceil_div(rows, (int64_t)lanes * 4);
   if (grid > 8 * current_sm_count()) grid = 8 * current_sm_count();
-  auto kern = vec ? sage_mask_kernel<true> : sage_mask_kernel<false>;
+  auto kern = h != nullptr ? (vec ? sage_mask_kernel<true, true> : sage_mask_kernel<false, true>)
+                           : (vec ? sage_mask_kernel<true, false> : sage_mask_kernel<false, false>);
   kern<<<(unsigned)grid, kThreads, (size_t)n * 4, (cudaStream_t)stream>>>(g, h, scale, dy, db, rows, (int)n, units);
+  return check_launch(op);
+}
+
+namespace f2c {
+namespace {
+
+constexpr int kMaxRanges = 32;
+struct Ranges {
+  uint32_t* at[kMaxRanges];
+  int64_t words[kMaxRanges];
+  int count;
+};
+
+__global__ void __launch_bounds__(256) zero_ranges_kernel(const Ranges r) {
+  for (int i = 0; i < r.count; ++i)
+    for (int64_t w = (int64_t)blockIdx.x * 256 + threadIdx.x; w < r.words[i]; w += (int64_t)gridDim.x * 256) r.at[i][w] = 0u;
+}
+
+}  // namespace
+}  // namespace f2c
+
+extern "C" int f2c_zero_ranges(void* const* ranges_host, const int64_t* bytes_host, int count, void* stream) {
+  const char* op = "zero_ranges";
+  F2C_REQUIRE(count >= 0 && count <= kMaxRanges && (count == 0 || (ranges_host && bytes_host)), F2C_ERR_INVALID, "%s: at most %d ranges", op,
+              kMaxRanges);
+  Ranges r{};
+  int64_t most = 0;
+  for (int i = 0; i < count; ++i) {
+    F2C_REQUIRE(bytes_host[i] >= 0 && bytes_host[i] % 4 == 0 && (bytes_host[i] == 0 || (ranges_host[i] && aligned(ranges_host[i], 4))),
+                F2C_ERR_INVALID, "%s: ranges are whole, aligned words", op);
+    if (bytes_host[i] == 0) continue;
+    r.at[r.count] = (uint32_t*)ranges_host[i];
+    r.words[r.count++] = bytes_host[i] / 4;
+    if (bytes_host[i] / 4 > most) most = bytes_host[i] / 4;
+  }
+  if (r.count == 0) return F2C_OK;
+  int64_t grid = ceil_div(most, 1024);
+  if (grid > 2 * current_sm_count()) grid = 2 * current_sm_count();
+  zero_ranges_kernel<<<(unsigned)grid, 256, 0, (cudaStream_t)stream>>>(r);
   return check_launch(op);
 }

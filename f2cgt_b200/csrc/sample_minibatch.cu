@@ -266,6 +266,7 @@ __global__ void __launch_bounds__(kThreads) minibatch_kernel(const Params<IdxT> 
   }
   if (gtid == 0) {
     p.header[2 * p.n_hops] = (int64_t)*(volatile int32_t*)p.error;
+    *p.error = 0;  // for the next minibatch
     __threadfence_system();
   }
 }
@@ -276,11 +277,11 @@ static Scratch plan(int64_t max_positions) {
   auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
   Scratch w{};
   size_t at = 0;
+  w.error = at; at += 256;
   w.val = at; at += up((size_t)max_positions * 4);
   w.rank = at; at += up((size_t)max_positions * 4);
   w.warp_prefix = at; at += up((size_t)kMaxCtas * kWarps * 4);
   w.cta_sum = at; at += up((size_t)2 * kMaxCtas * 4);
-  w.error = at; at += 256;
   w.total = at;
   return w;
 }
@@ -324,8 +325,6 @@ static int launch(const f2c_minibatch* a, int64_t max_positions, cudaStream_t st
   p.cta_sum = (uint32_t*)(ws + w.cta_sum); p.error = (int32_t*)(ws + w.error);
   p.header = a->header;
   p.rng_seed = a->rng_seed; p.rng_offset = a->rng_offset;
-  cudaError_t e = cudaMemsetAsync(p.error, 0, 4, st);
-  if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "%s: %s", op, cudaGetErrorString(e));
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) dev = 0;
   int grid = resident_ctas<IdxT>(dev);
@@ -333,7 +332,7 @@ static int launch(const f2c_minibatch* a, int64_t max_positions, cudaStream_t st
   const int64_t tiles = ceil_div(max_positions, kThreads);
   if (grid > tiles) grid = (int)tiles;
   void* args[] = {(void*)&p};
-  e = cudaLaunchCooperativeKernel((const void*)minibatch_kernel<IdxT>, dim3((unsigned)grid), dim3(kThreads), args, 0, st);
+  cudaError_t e = cudaLaunchCooperativeKernel((const void*)minibatch_kernel<IdxT>, dim3((unsigned)grid), dim3(kThreads), args, 0, st);
   if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "%s: cooperative launch: %s", op, cudaGetErrorString(e));
   return check_launch(op);
 }

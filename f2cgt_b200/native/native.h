@@ -108,7 +108,7 @@ inline int unlocked(F&& call) {
 }
 
 
-extern PyMethodDef g_sage_methods[];  // sage.cpp
+extern PyMethodDef g_sage_methods[], g_loader_methods[];  // sage.cpp, loader.cpp
 
 void arguments(const char* name, Py_ssize_t got, Py_ssize_t want);
 

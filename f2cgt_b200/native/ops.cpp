@@ -22,12 +22,13 @@ Csc csc(PyObject* ip, PyObject* ix) {
   return Csc{indptr, indices, indptr.numel() - 1, dtype_tag(indptr.scalar_type())};
 }
 
-// [max(n_dst, out_rows), width]; rows behind n_dst are zero
+// [max(n_dst, |out_rows|), width]; rows behind n_dst are zero, or - negative out_rows - left as they are
 at::Tensor block_out(int64_t n_dst, int64_t width, at::ScalarType dtype, const at::Device& device, PyObject* out_rows, cudaStream_t st) {
-  const int64_t rows = out_rows == Py_None ? n_dst : std::max(n_dst, integer(out_rows));
+  const int64_t asked = out_rows == Py_None ? n_dst : integer(out_rows);
+  const int64_t rows = std::max(n_dst, std::abs(asked));
   if (width < 0) fail(PyExc_RuntimeError, "negative width");
   at::Tensor out = empty({rows, width}, dtype, device);
-  if (rows > n_dst) {
+  if (rows > n_dst && asked > 0) {
     const size_t row = (size_t)width * out.element_size();
     C10_CUDA_CHECK(cudaMemsetAsync((char*)out.data_ptr() + (size_t)n_dst * row, 0, (size_t)(rows - n_dst) * row, st));
   }
@@ -205,6 +206,7 @@ PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, g_methods
 
 PyMODINIT_FUNC PyInit__native(void) {
   PyObject* m = PyModule_Create(&f2c_native::g_module);
-  if (m != nullptr && PyModule_AddFunctions(m, f2c_native::g_sage_methods) != 0) Py_CLEAR(m);
+  for (PyMethodDef* more : {f2c_native::g_sage_methods, f2c_native::g_loader_methods})
+    if (m != nullptr && PyModule_AddFunctions(m, more) != 0) Py_CLEAR(m);
   return m;
 }

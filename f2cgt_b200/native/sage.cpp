@@ -15,6 +15,7 @@
 #include <array>
 
 #include <ATen/cuda/CUDAEvent.h>
+#include <cublas_v2.h>
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
@@ -60,8 +61,35 @@ bool use_own(const Net& net, int64_t rows, int64_t k, bool record) {
   return net.tf32 && k % 4 == 0 && rows > 1 && (!record || k % 32 == 0 || rows >= 16384);
 }
 
-void zero_tail(at::Tensor& t, int64_t rows, cudaStream_t st) {
-  if (t.size(0) > rows) C10_CUDA_CHECK(cudaMemsetAsync(f32(t) + rows * t.size(1), 0, (size_t)((t.size(0) - rows) * t.size(1)) * 4, st));
+// Ranges to be set to zero in one launch: a memset each costs the host as much as a kernel.
+struct Zeros {
+  void* at[32];
+  int64_t bytes[32];
+  int count = 0;
+  void add(void* p, int64_t n) {
+    if (n <= 0) return;
+    TORCH_CHECK(count < 32, "sage_net: too many layers");
+    at[count] = p;
+    bytes[count++] = n;
+  }
+  void tail(const at::Tensor& t, int64_t rows) { add(f32(t) + rows * t.size(1), (t.size(0) - rows) * t.size(1) * 4); }
+  void run(cudaStream_t st) { checked = f2c_zero_ranges(at, bytes, count, st); }
+};
+
+// Products of the backward pass as at::mm computes them (same library call, same operands), without its dispatch: out is
+// [a.size(1), b.size(1)] = a^T (first rows of b), or - plain - [a.size(0), b.size(1)] = a b, added to what out holds when add.
+void product(const Net& net, at::Tensor& out, const at::Tensor& a, bool a_turned, const at::Tensor& b, bool add) {
+  const int64_t inner = a_turned ? a.size(0) : b.size(0), rows = out.size(0), cols = out.size(1);
+  if (net.cast) {
+    const at::Tensor r = mm(net, a_turned ? a.t() : a, b.narrow(0, 0, inner));
+    if (add) out.add_(r); else out.copy_(r);
+    return;
+  }
+  const float one = 1.0f, beta = add ? 1.0f : 0.0f;
+  const cublasStatus_t rc = cublasSgemm(at::cuda::getCurrentCUDABlasHandle(), CUBLAS_OP_N, a_turned ? CUBLAS_OP_T : CUBLAS_OP_N, (int)cols,
+                                        (int)rows, (int)inner, &one, f32(b), (int)cols, f32(a), (int)(a_turned ? rows : inner), &beta, f32(out),
+                                        (int)cols);
+  TORCH_CHECK(rc == CUBLAS_STATUS_SUCCESS, "cublasSgemm failed with status ", (int)rc);
 }
 
 // y of one layer (before dropout), `padded` rows
@@ -72,7 +100,6 @@ at::Tensor layer_forward(const Net& net, const at::Tensor& x1, const at::Tensor&
     at::Tensor y = empty({l.padded, w1.size(0)}, at::kFloat, x1.device());
     checked = f2c_sage_forward(f32(x1), f32(x2), f32(w1), f32(w2), bias.defined() ? f32(bias) : nullptr, f32(y), l.rows, w1.size(0), w1.size(1),
                                relu ? 1 : 0, st);
-    zero_tail(y, l.rows, st);
     return y;
   }
   const at::Tensor a = x1.narrow(0, 0, l.padded), b = x2.narrow(0, 0, l.padded);
@@ -136,16 +163,24 @@ struct SageBackward : public torch::autograd::Node {
       if (i % 3 == 2 && w[i].defined()) biases += (w[i].numel() + 63) / 64 * 64;
     }
     at::Tensor bias_grads = empty({biases}, at::kFloat, given.device());  // the mask kernel adds to it
-    if (biases > 0) C10_CUDA_CHECK(cudaMemsetAsync(bias_grads.data_ptr(), 0, (size_t)biases * 4, st));
+    // The weight gradients' products run over padded rows, where the gradients are zero; what they meet there must be finite.
+    Zeros zeros;
+    zeros.add(bias_grads.data_ptr(), biases * 4);
+    for (size_t i = 0; i < L; ++i) {
+      if (i == 0) zeros.tail(x1[0], net.layers[0].rows);
+      zeros.tail(x2[i], net.layers[i].rows);
+      if (i + 1 < L) zeros.tail(out[i], net.layers[i].rows);
+    }
 
     // gradient of the last layer's output on its padded rows
     at::Tensor g = given.contiguous();
     if (net.layers[L - 1].padded > g.size(0)) {
       at::Tensor padded = empty({net.layers[L - 1].padded, g.size(1)}, at::kFloat, g.device());
       C10_CUDA_CHECK(cudaMemcpyAsync(padded.data_ptr(), g.data_ptr(), (size_t)g.numel() * 4, cudaMemcpyDeviceToDevice, st));
-      zero_tail(padded, g.size(0), st);
+      zeros.tail(padded, g.size(0));
       g = padded;
     }
+    zeros.run(st);
     Beside& side = beside(given.device().index());
     bool forked = false;
     std::vector<at::Tensor> keep;  // what the side stream reads, until the streams have joined
@@ -164,31 +199,33 @@ struct SageBackward : public torch::autograd::Node {
         dy = empty({m, n}, at::kFloat, g.device());
         checked = f2c_sage_mask(f32(g), f32(out[i]), (float)net.scale(), f32(dy), db.defined() ? f32(db) : nullptr, m, n, st);
       } else if (db.defined()) {
-        at::sum_out(db, dy, 0);
+        checked = f2c_sage_mask(f32(dy), nullptr, 1.0f, nullptr, f32(db), m, n, st);
       }
       result[3 * i + 2] = db;
-      const at::Tensor dyt = dy.t();
-      const bool apart = m >= kBesideRows;
-      if (apart) {
+      at::Tensor both = empty({2, n, k}, at::kFloat, g.device());
+      at::Tensor d_self = result[3 * i] = both.select(0, 0), d_nb = result[3 * i + 1] = both.select(0, 1);
+      if (m >= kBesideRows) {
         side.fork.record(main);
         side.fork.block(*side.stream);
         c10::cuda::CUDAStreamGuard on_side(*side.stream);
-        result[3 * i + 1] = mm(net, dyt, x2[i].narrow(0, 0, m));
-        if (i > 0) result[3 * i] = mm(net, dyt, x1[i].narrow(0, 0, m));
+        product(net, d_nb, dy, true, x2[i], false);
+        if (i > 0) product(net, d_self, dy, true, x1[i], false);
         side.join.record(*side.stream);
         forked = true;
         keep.push_back(dy);
       } else {
-        result[3 * i + 1] = mm(net, dyt, x2[i].narrow(0, 0, m));
+        product(net, d_nb, dy, true, x2[i], false);
+        if (i > 0) product(net, d_self, dy, true, x1[i], false);
       }
-      if (!apart || i == 0) result[3 * i] = mm(net, dyt, x1[i].narrow(0, 0, m));
+      if (i == 0) product(net, d_self, dy, true, x1[i], false);
       if (i > 0) {
         at::Tensor dh = empty({net.layers[i - 1].padded, k}, at::kFloat, g.device());  // gradient of the previous layer's output
-        const at::Tensor d_neigh = mm(net, dy, wi[1]);
-        checked = f2c_spmm_csr_backward(f32(d_neigh), l.indptr.data_ptr(), l.indices.data_ptr(), dtype_tag(l.indptr.scalar_type()), f32(dh), l.rows,
+        at::Tensor d_rows = empty({m, k}, at::kFloat, g.device());
+        product(net, d_rows, dy, false, wi[1], false);
+        checked = f2c_spmm_csr_backward(f32(d_rows), l.indptr.data_ptr(), l.indices.data_ptr(), dtype_tag(l.indptr.scalar_type()), f32(dh), l.rows,
                                         dh.size(0), k, F2C_MEAN, st);
         at::Tensor head = dh.narrow(0, 0, m);
-        addmm_(net, head, dy, wi[0]);
+        product(net, head, dy, false, wi[0], true);
         g = dh;
       }
     }
@@ -259,12 +296,11 @@ PyObject* sage_net(PyObject*, PyObject* const* a, Py_ssize_t n) {
         if (i > 0) {
           x1 = h;
           x2 = empty({l.padded, h.size(1)}, at::kFloat, h.device());
-          zero_tail(x2, l.rows, st);
           checked = f2c_spmm_csr(h.data_ptr(), F2C_F32, l.indptr.data_ptr(), l.indices.data_ptr(), dtype_tag(l.indptr.scalar_type()), x2.data_ptr(),
                                  l.rows, h.size(1), F2C_MEAN, st);
         }
         h = layer_forward(net, x1, x2, &w[3 * i], l, !last, record, st);
-        if (!last && net.p > 0) h = at::dropout(h, net.p, true);
+        if (!last && net.p > 0) h = net.p < 1 && h.numel() > 0 ? std::get<0>(at::native_dropout(h, net.p, true)) : at::dropout(h, net.p, true);
         if (record) {
           node->x1.push_back(x1);
           node->x2.push_back(x2);

@@ -601,64 +601,45 @@ class MinibatchBuffers:
         ws_bytes = _minibatch_workspace(n_nodes, self.max_seeds, self.num_picks)
         if ws_bytes <= 0:
             raise RuntimeError("sample_minibatch: 1 to 16 hops, num_pick in [1, 64], at most 2^31 - 2 ids per hop")
-        self.ws = torch.empty((ws_bytes,), dtype=torch.uint8, device=dev)
-        # [node words], number of the last minibatch built with them
+        # [node words, number of the last minibatch built with them]
         self.shared = share.shared if share is not None else [torch.full((n_nodes,), -1, dtype=torch.int64, device=dev), 0]
-        self.header = torch.zeros((2 * hops + 1,), dtype=torch.int64, pin_memory=True)
-        self.event = torch.cuda.Event()
-        self.sub_indptr, self.ids, self.local = [], [], []
-        rows = self.max_seeds
+        ws = torch.empty((ws_bytes,), dtype=torch.uint8, device=dev)
+        ws[:256].zero_()
+        sub_indptr, ids, local, rows = [], [], [], self.max_seeds
         for k in self.num_picks:
-            self.sub_indptr.append(torch.empty((rows + 1,), dtype=dt, device=dev))
+            sub_indptr.append(torch.empty((rows + 1,), dtype=dt, device=dev))
             edges = torch.empty((2, rows * k), dtype=dt, device=dev)
-            self.ids.append(edges[0])
-            self.local.append(edges[1])
+            ids.append(edges[0])
+            local.append(edges[1])
             rows = min(rows * (k + 1), n_nodes)
-        self.unique = torch.empty((rows,), dtype=dt, device=dev)
-        a = self.args = _lib.Minibatch()
-        a.indptr, a.indices, a.n_nodes, a.index_dtype, a.n_hops = _ptr(indptr), _ptr(indices), n_nodes, _DT[dt], hops
-        a.unique, a.node_map, a.header, a.workspace, a.workspace_bytes = (_ptr(self.unique), _ptr(self.shared[0]), _ptr(self.header),
-                                                                          _ptr(self.ws), ws_bytes)
-        for h in range(hops):
-            a.num_pick[h], a.sub_indptr[h], a.ids[h], a.local[h] = (self.num_picks[h], _ptr(self.sub_indptr[h]), _ptr(self.ids[h]),
-                                                                    _ptr(self.local[h]))
+        unique = torch.empty((rows,), dtype=dt, device=dev)
+        header = torch.zeros((2 * hops + 1,), dtype=torch.int64, pin_memory=True)
+        self.native = _native.minibatch_new(indptr, indices, ws, self.shared[0], header, unique, sub_indptr, ids, local, self.num_picks)
+
+    def next_epoch(self, stream):
+        """Number of the minibatch about to be built (the node words are set again before it could wrap)."""
+        if self.shared[1] >= 2**32 - 2:
+            with torch.cuda.stream(stream):
+                self.shared[0].fill_(-1)
+            self.shared[1] = 0
+        self.shared[1] += 1
+        return self.shared[1]
 
 
 def sample_minibatch_launch(buffers, seeds, rng_seed=0, rng_offset=0, stream=None):
     """Queue every hop of a minibatch on ``stream`` (default: the current one) as one kernel, without waiting: hop h draws like
-    ``sample_block(..., rng_offset=rng_offset + h)`` from the distinct nodes of hop h - 1.  ``buffers.event`` tells when it is through."""
-    b, a = buffers, buffers.args
-    _chk(seeds, "seeds", (b.indptr.dtype,))
+    ``sample_block(..., rng_offset=rng_offset + h)`` from the distinct nodes of hop h - 1."""
     n = seeds.numel()
-    if n == 0 or n > b.max_seeds:
-        raise RuntimeError(f"sample_minibatch: between 1 and {b.max_seeds} seeds")
+    if n == 0 or n > buffers.max_seeds:
+        raise RuntimeError(f"sample_minibatch: between 1 and {buffers.max_seeds} seeds")
     if stream is None:
-        stream = torch.cuda.current_stream(b.indptr.device)
-    if b.shared[1] >= 2**32 - 2:
-        with torch.cuda.stream(stream):
-            b.shared[0].fill_(-1)
-        b.shared[1] = 0
-    b.shared[1] += 1
-    b.seeds = seeds
-    a.seeds, a.n_seeds, a.epoch, a.rng_seed, a.rng_offset = _ptr(seeds), n, b.shared[1], int(rng_seed) & 0xFFFFFFFFFFFFFFFF, int(rng_offset)
-    with _on(b.indptr):
-        check(lib.f2c_sample_minibatch(a, stream.cuda_stream))
-        b.event.record(stream)
+        stream = torch.cuda.current_stream(buffers.indptr.device)
+    _native.minibatch_launch(buffers.native, seeds, 0, n, buffers.next_epoch(stream), int(rng_seed), int(rng_offset), stream.cuda_stream)
 
 
 def sample_minibatch_finish(buffers):
     """Wait (on the host) for the minibatch in ``buffers`` and return ``(blocks, unique)``: per hop, from the seeds outwards,
     ``(seeds, sub_indptr, sub_indices, local_indices)``, and the distinct nodes of all hops (those of hop h are a prefix).
     The tensors are views of the buffers."""
-    b = buffers
-    b.event.synchronize()
-    *sizes, err = b.header.tolist()
-    if err != 0:
-        raise RuntimeError("sample_minibatch: negative id in the graph or the seeds" if err == 2 else
-                           "sample_minibatch: id beyond the graph's nodes in the graph or the seeds")
-    out, seeds = [], b.seeds
-    for h in range(len(b.num_picks)):
-        edges, n = sizes[2 * h], sizes[2 * h + 1]
-        out.append((seeds, b.sub_indptr[h][:seeds.numel() + 1], b.ids[h][:edges], b.local[h][:edges]))
-        seeds = b.unique[:n]
-    return out, seeds
+    input_nodes, _, blocks = _native.minibatch_take(buffers.native)
+    return [(b["dst_nodes"], b["indptr"], b["indices_global"], b["indices_local"]) for b in blocks[::-1]], input_nodes

@@ -40,7 +40,7 @@ class CompressionManager:
             raise ValueError("two-level compression is hot SQ rows over a VQ table, with a slot array or hot-first numbering")
 
     def aggregate(self, indptr, indices_global, dropout=None, out_rows=None):
-        """``out_rows``: allocate that many output rows (zero behind the block's own), see ``ops._block_out``."""
+        """``out_rows``: allocate that many output rows (zero behind the block's own; negative: left unwritten)."""
         if self.is_two_level:
             cs, bits = self.configs[0]
             return ops.two_level_decompress_spmm_csr(self.tables[0], self.codebooks[0], bits, cs, self.tables[1], self.codebooks[1],
@@ -384,8 +384,9 @@ class SAGE(nn.Module):
         for block in blocks[1:]:
             rows.append(block["dst_nodes"].numel())
             padded.append(min(_bucket(rows[-1]), padded[-1]))
-        h_neigh = sm.aggregate(first["indptr"], neighbours, out_rows=padded[0])  # raw codes in, no autograd through it
-        h_self = sm.decode_rows(dst, out_rows=padded[0])
+        out_rows = -padded[0] if type(sm) is CompressionManager else padded[0]  # rows behind the block's own are nobody's input yet
+        h_neigh = sm.aggregate(first["indptr"], neighbours, out_rows=out_rows)  # raw codes in, no autograd through it
+        h_self = sm.decode_rows(dst, out_rows=out_rows)
         p = self.dropout.p if self.dropout.training else 0.0
         tf32 = _PRODUCT_DTYPE is None and torch.backends.cuda.matmul.allow_tf32
         return ops._native.sage_net(h_self, h_neigh, [b["indptr"] for b in blocks[1:]], [b["indices_local"] for b in blocks[1:]], rows, padded,
@@ -422,7 +423,7 @@ class GPUSamplingDataloader:
         ahead = ahead and ops.minibatch_fits(indptr.numel() - 1, self.batchsize, self.num_picks)
         self.side = torch.cuda.Stream(device=indptr.device) if ahead else None
         self._pending = None  # buffers of the minibatch under construction
-        self._sets, self._consumed, self._built = None, [None, None], 0
+        self._sets, self._built = None, 0
 
     def __len__(self):
         return (self.seeds.numel() + self.batchsize - 1) // self.batchsize
@@ -438,7 +439,8 @@ class GPUSamplingDataloader:
         self.epoch += 1
         self._pending = None
         if self.side is not None:
-            self.side.wait_stream(torch.cuda.current_stream(self.indptr.device))  # the shuffled order is read over there
+            # the shuffled order is read over there, and minibatches of an epoch cut short may still be in use here
+            self.side.wait_stream(torch.cuda.current_stream(self.indptr.device))
             self._start()
         return self
 
@@ -459,6 +461,7 @@ class GPUSamplingDataloader:
         return (self.rng_seed * 7919 + self.epoch) * 65536 + self.rank
 
     def _start(self):
+        """Queue the first minibatch of an epoch."""
         self._pending = None
         if self.curr >= len(self):
             return
@@ -467,14 +470,11 @@ class GPUSamplingDataloader:
             first = ops.MinibatchBuffers(self.indptr, self.indices, self.batchsize, picks)
             self._sets = [first, ops.MinibatchBuffers(self.indptr, self.indices, self.batchsize, picks, share=first)]
             self.side.wait_stream(torch.cuda.current_stream(self.indptr.device))  # the node words are set over there
-        which = self._built % 2
+        b = self._sets[self._built % 2]
         self._built += 1
-        if self._consumed[which] is not None:  # the minibatch that last lived in this set: its step must be through
-            self.side.wait_event(self._consumed[which])
-        ops.sample_minibatch_launch(self._sets[which], self.order[self.curr * self.batchsize:(self.curr + 1) * self.batchsize],
-                                    rng_seed=self._rng_seed(), rng_offset=self.curr * 8, stream=self.side)
-        self._pending = self._sets[which]
-        self.curr += 1
+        ops.sample_minibatch_launch(b, self.order[:self.batchsize], self._rng_seed(), 0, self.side)
+        self._pending = b
+        self.curr = 1
 
     def poke(self):
         """Nothing to do: a minibatch under construction needs no help from the host (kept for training loops that call it)."""
@@ -488,17 +488,15 @@ class GPUSamplingDataloader:
         built = self._pending
         if built is None:
             raise StopIteration
-        built.event.synchronize()
-        # Everything queued on the current stream so far belongs to earlier minibatches: once it has run, the set of the
-        # minibatch handed out before this one may be overwritten, which is what the next one goes on to do.
-        previous = self._built % 2
-        if self._consumed[previous] is None:
-            self._consumed[previous] = torch.cuda.Event()
-        self._consumed[previous].record(torch.cuda.current_stream(self.indptr.device))
-        self._start()
-        hops, input_nodes = ops.sample_minibatch_finish(built)
-        blocks = []
-        for i, (seeds, sub_indptr, sub_indices, local) in enumerate(hops):
-            blocks.insert(0, dict(dst_nodes=seeds, src_nodes=hops[i + 1][0] if i + 1 < len(hops) else input_nodes, indptr=sub_indptr,
-                                  indices_global=sub_indices, indices_local=local, n_edges=sub_indices.numel()))
-        return input_nodes, hops[0][0], blocks
+        first = self.curr * self.batchsize
+        left = self.order.numel() - first
+        if left <= 0:
+            self._pending = None
+            return ops._native.minibatch_next(built.native, None, None, 0, 0, 0, 0, 0, 0)
+        # the other set: its minibatch was handed out before this one, so what is queued by now is all that reads it
+        b = self._pending = self._sets[self._built % 2]
+        self._built += 1
+        rng_offset = self.curr * 8
+        self.curr += 1
+        return ops._native.minibatch_next(built.native, b.native, self.order, first, min(left, self.batchsize), b.next_epoch(self.side),
+                                          self._rng_seed(), rng_offset, self.side.cuda_stream)

@@ -86,11 +86,12 @@ class DirectFusedAdam:
         self.lr, self.betas, self.eps = float(lr), betas, float(eps)
         self.exp_avg = [torch.zeros_like(p) for p in self.params]
         self.exp_avg_sq = [torch.zeros_like(p) for p in self.params]
-        self.steps = [torch.zeros((), dtype=torch.float32, device=p.device) for p in self.params]
+        # one step counter for all parameters: they are always updated together
+        self.steps = [torch.zeros((), dtype=torch.float32, device=self.params[0].device)] * len(self.params) if self.params else []
 
     @staticmethod
     def available():
-        return hasattr(torch, "_fused_adam_") and hasattr(torch, "_foreach_add_")
+        return hasattr(torch, "_fused_adam_")
 
     def zero_grad(self, set_to_none=True):
         for p in self.params:
@@ -101,7 +102,9 @@ class DirectFusedAdam:
 
     @torch.no_grad()
     def step(self):
-        torch._foreach_add_(self.steps, 1)
+        if not self.params:
+            return
+        self.steps[0].add_(1)
         torch._fused_adam_(self.params, [p.grad for p in self.params], self.exp_avg, self.exp_avg_sq, [], self.steps, amsgrad=False,
                            lr=self.lr, beta1=self.betas[0], beta2=self.betas[1], weight_decay=0.0, eps=self.eps, maximize=False,
                            grad_scale=None, found_inf=None)

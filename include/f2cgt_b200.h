@@ -138,8 +138,12 @@ int f2c_sage_forward(const float* x1, const float* x2, const float* w1, const fl
                      int64_t n, int64_t k, int relu, void* stream);
 
 /* Gradient through dropout and ReLU of a layer whose output after both is h: dy = h > 0 ? scale * g : 0 (scale = what dropout
- * multiplies survivors with), and db [n] += column sums of dy (db may be NULL; no fixed order).  g, h, dy [rows, n] f32. */
+ * multiplies survivors with), and db [n] += column sums of dy (db may be NULL; no fixed order).  g, h, dy [rows, n] f32.
+ * h == NULL: dy is not written, db += column sums of g. */
 int f2c_sage_mask(const float* g, const float* h, float scale, float* dy, float* db, int64_t rows, int64_t n, void* stream);
+
+/* Set up to 32 ranges of device memory (whole 4-byte words) to zero in one launch; the arrays are HOST arrays. */
+int f2c_zero_ranges(void* const* ranges_host, const int64_t* bytes_host, int count, void* stream);
 
 /* sq_decompress_spmm_csr(compress_feat, codebooks, indptr, indices, target_bit, column_slice, feat_dim)
  *  -  src/fusion_spmm.cu:240-272 (kernel :143-238).  out [n_dst, feat_dim] f32; the decoded rows are
@@ -348,7 +352,7 @@ int f2c_sample_block(const void* indptr, const void* indices, const void* seeds,
  *   epoch                 number of this minibatch: larger than that of any earlier call on node_map, below 2^32 - 1
  *   header                HOST memory the device can write (pinned), 2 * n_hops + 1 entries, valid when the stream has got past
  *                         the call: {edges, distinct nodes} per hop, then 0 or the error (2 negative id, 3 id >= n_nodes)
- *   workspace             f2c_sample_minibatch_workspace() bytes, 256-byte aligned */
+ *   workspace             f2c_sample_minibatch_workspace() bytes, 256-byte aligned, its first 256 bytes zero before the first call */
 #define F2C_MAX_HOPS 16
 typedef struct {
   const void* indptr;
