@@ -39,6 +39,23 @@ static inline int dtype_size(int dt) {
 static inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; }
 static inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
+// ---- launches that overlap the kernel before them on the stream ----
+// A kernel launched with launch_dependent() may be brought onto the SMs while the previous kernel of the stream still runs;
+// it calls dependency_wait() before it touches memory (that returns when the previous kernel is complete and its writes are
+// visible) and, having done so, release_dependents() so that the next one can do the same.  What overlaps is the launch itself:
+// ~2 us of every call in a row of short ones.
+template <typename... K, typename... A>
+static inline cudaError_t launch_dependent(void (*kern)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st; cfg.attrs = &attr; cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+__device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void release_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- device helpers ----
 
 // Read-only, L1-bypassing vector loads for streamed gathers.

@@ -12,6 +12,8 @@ namespace f2c {
 
 __global__ void __launch_bounds__(256) dropout_kernel(float* __restrict__ x, int64_t numel, int64_t n_vec, int vec_ok,
                                                       const DropoutArgs a) {
+  dependency_wait();
+  release_dependents();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_vec) return;
   int64_t base = i * 4;
@@ -40,6 +42,6 @@ extern "C" int f2c_dropout(float* x, int64_t numel, float p, int training, uint6
   f2c_epilogue ep{p, training, scale, seed, offset};
   DropoutArgs a = make_dropout(&ep);
   int64_t n_vec = ceil_div(numel, 4);
-  dropout_kernel<<<(unsigned)ceil_div(n_vec, 256), 256, 0, (cudaStream_t)stream>>>(x, numel, n_vec, aligned(x, 16) ? 1 : 0, a);
+  launch_dependent(dropout_kernel, (unsigned)ceil_div(n_vec, 256), 256, 0, (cudaStream_t)stream, x, numel, n_vec, aligned(x, 16) ? 1 : 0, a);
   return check_launch("dropout_inplace");
 }

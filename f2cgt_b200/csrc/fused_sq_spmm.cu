@@ -96,6 +96,8 @@ struct SqParams {
 template <int BITS, int VEC, int U, typename IdxT, int DEC, bool PEER = false>
 __global__ void __launch_bounds__(SqCta<BITS, DEC>::kThreads, SqCta<BITS, DEC>::kCtasPerSm)
 sq_spmm_kernel(const SqParams p) {
+  dependency_wait();
+  release_dependents();
   constexpr bool ALIGNED = SqCta<BITS, DEC>::kAligned;
   constexpr int EPL = BITS == 16 ? VEC / 2 : VEC * 8 / BITS;  // output columns per lane
   constexpr bool PACKED = DEC == DEC_LUT && BITS <= 4;
@@ -275,6 +277,8 @@ __global__ void __launch_bounds__(256) sq_spmm_generic_kernel(const void* __rest
                                                               const IdxT* __restrict__ indptr, const IdxT* __restrict__ indices,
                                                               float* __restrict__ out, int64_t n_dst, int64_t src_dim, int feat_dim,
                                                               int column_slice, int reduce, DropoutArgs drop) {
+  dependency_wait();
+  release_dependents();
   constexpr int PER = BITS >= 8 ? 1 : 8 / BITS;
   constexpr int B = BITS >= 8 ? 8 : BITS;
   const int lane = threadIdx.x & 31;
@@ -374,7 +378,7 @@ static int launch_fast(SqParams p, bool vec_store, cudaStream_t st) {
   int rows_per_cta = kWarpsPerCta * (32 >> p.logG);
   int64_t grid = ceil_div(p.n_dst, rows_per_cta);
   if (grid > (int64_t)sms * resident) grid = (int64_t)sms * resident;
-  kern<<<(unsigned)grid, kThreads, smem, st>>>(p);
+  launch_dependent(kern, (unsigned)grid, kThreads, smem, st, p);
   return check_launch("sq_decompress_spmm_csr");
 }
 
@@ -463,7 +467,7 @@ static int launch_sq_spmm(const void* codes, int code_dtype, const float* codebo
     return set_error(F2C_ERR_UNSUPPORTED, "%s: shape not served by the register-prefetch kernel", op);
   int64_t blocks = ceil_div(n_dst, 8);
   if (blocks > current_sm_count() * 32) blocks = current_sm_count() * 32;
-#define F2C_GEN(T) sq_spmm_generic_kernel<BITS, T, IdxT><<<(unsigned)blocks, 256, 0, st>>>( \
+#define F2C_GEN(T) launch_dependent(sq_spmm_generic_kernel<BITS, T, IdxT>, (unsigned)blocks, 256, 0, st,  \
       codes, codebooks, (const IdxT*)indptr, (const IdxT*)indices, out, n_dst, src_dim, (int)D, (int)cs, reduce, drop)
   if (code_dtype == F2C_I8) F2C_GEN(int8_t);
   else if (code_dtype == F2C_U8) F2C_GEN(uint8_t);

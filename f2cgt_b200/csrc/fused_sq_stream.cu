@@ -60,6 +60,8 @@ struct Params {
 
 template <int BITS, typename IdxT, bool PEER>
 __global__ void __launch_bounds__(Geo<BITS>::kThreads, 1) sq_stream_kernel(const Params p) {
+  dependency_wait();
+  release_dependents();
   using L = Lut<BITS>;
   constexpr int VEC = Geo<BITS>::VEC, EPL = Geo<BITS>::EPL, C = Geo<BITS>::kConsumers, kProducers = Geo<BITS>::kProducers;
   constexpr bool PACKED = BITS <= 4;
@@ -313,7 +315,7 @@ static int launch_stream(const void* codes, int code_dtype, const float* codeboo
     auto launch = [&](auto kern) -> int {
       cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemTotal);
       if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "sq_decompress_spmm_csr: %s", cudaGetErrorString(e));
-      kern<<<(unsigned)grid, G_::kThreads, kSmemTotal, st>>>(p);
+      launch_dependent(kern, (unsigned)grid, G_::kThreads, kSmemTotal, st, p);
       return check_launch("sq_decompress_spmm_csr");
     };
     *served = true;

@@ -75,6 +75,8 @@ template <int ROWW> __device__ __forceinline__ void load_code_row(CodeRow<ROWW>&
 // other ranks are read with ordinary loads over NVLink (no collective, no staging copy, nothing waits on another rank).
 template <int HB, typename IdxT, int ROWW, bool PEER = false>
 __global__ void __launch_bounds__(VqCta<HB>::kThreads, 1) vq_fast_kernel(const VqParams p) {
+  dependency_wait();
+  release_dependents();
   constexpr int kThreads = VqCta<HB>::kThreads, kWarps = VqCta<HB>::kWarps;
   extern __shared__ __align__(128) unsigned char smem[];
   unsigned char* cb_s = smem;
@@ -344,7 +346,7 @@ static int launch_rows(const VqParams& p, int roww, dim3 grid, size_t smem, cuda
     auto kern = vq_fast_kernel<HB, IdxT, RW, PEER>;                                                      \
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
     if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "%s: %s", op, cudaGetErrorString(e));           \
-    kern<<<grid, VqCta<HB>::kThreads, smem, st>>>(p);                                                               \
+    launch_dependent(kern, grid, VqCta<HB>::kThreads, smem, st, p);                                                               \
     return check_launch(op);                                                                             \
   }
   if (roww == 1) F2C_VQF(1)

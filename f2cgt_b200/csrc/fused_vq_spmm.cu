@@ -72,6 +72,8 @@ __device__ __forceinline__ float4 sq_decode4(const uint8_t* __restrict__ row, in
 // HB = 0: pure VQ.  HB in {1,2,4,8,16}: two-level, SQ width HB.
 template <int HB, typename IdxT, bool CB_SMEM>
 __global__ void __launch_bounds__(kVqThreads) vq_spmm_kernel(const VqParams p) {
+  dependency_wait();
+  release_dependents();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float* cb_s = reinterpret_cast<float*>(smem_raw);
   const int part = blockIdx.y;
@@ -170,6 +172,8 @@ __global__ void __launch_bounds__(kVqThreads) vq_spmm_kernel(const VqParams p) {
 // j, j+32, ...; codebooks through the read-only cache.
 template <typename IdxT>
 __global__ void __launch_bounds__(256) vq_spmm_generic_kernel(const VqParams p) {
+  dependency_wait();
+  release_dependents();
   const IdxT* __restrict__ indptr = reinterpret_cast<const IdxT*>(p.indptr);
   const IdxT* __restrict__ indices = reinterpret_cast<const IdxT*>(p.indices);
   const int lane = threadIdx.x & 31;
@@ -219,9 +223,9 @@ static int launch_vq(VqParams& p, cudaStream_t st, const char* op) {
     auto kern = vq_spmm_kernel<HB, IdxT, true>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "%s: %s", op, cudaGetErrorString(e));
-    kern<<<grid, kVqThreads, smem, st>>>(p);
+    launch_dependent(kern, grid, kVqThreads, smem, st, p);
   } else {
-    vq_spmm_kernel<HB, IdxT, false><<<grid, kVqThreads, 0, st>>>(p);
+    launch_dependent(vq_spmm_kernel<HB, IdxT, false>, grid, kVqThreads, 0, st, p);
   }
   return check_launch(op);
 }
@@ -252,8 +256,8 @@ extern "C" int f2c_vq_spmm_csr(const void* codes, int code_dtype, const float* c
   if (!fast) {
     int64_t blocks = ceil_div(n_dst, 8);
     if (blocks > current_sm_count() * 32) blocks = current_sm_count() * 32;
-    if (index_dtype == F2C_I32) vq_spmm_generic_kernel<int32_t><<<(unsigned)blocks, 256, 0, st>>>(p);
-    else vq_spmm_generic_kernel<int64_t><<<(unsigned)blocks, 256, 0, st>>>(p);
+    if (index_dtype == F2C_I32) launch_dependent(vq_spmm_generic_kernel<int32_t>, (unsigned)blocks, 256, 0, st, p);
+    else launch_dependent(vq_spmm_generic_kernel<int64_t>, (unsigned)blocks, 256, 0, st, p);
     return check_launch(op);
   }
   const int variant = kernel_variant(epilogue);

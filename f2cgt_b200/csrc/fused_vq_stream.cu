@@ -87,6 +87,8 @@ template <int ROWW> __device__ __forceinline__ void store_code_row(uint32_t a, c
 template <int HB, typename IdxT, int ROWW>
 __global__ void __launch_bounds__(kThreads, 1) vq_stream_kernel(const VqParams p, const Layout lay, const int rows_per_chunk,
                                                                 const int64_t n_chunks, int* const error) {
+  dependency_wait();
+  release_dependents();
   extern __shared__ __align__(128) unsigned char smem[];
   constexpr int C = kConsumers;
   constexpr uint32_t ROWB = ROWW * 4;
@@ -428,7 +430,7 @@ static int launch_stream_rows(const VqParams& p, const vqs::Layout& lay, int row
     auto kern = vqs::vq_stream_kernel<HB, IdxT, RW>;                                                     \
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
     if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "%s: %s", op, cudaGetErrorString(e));           \
-    kern<<<grid, vqs::kThreads, smem, st>>>(p, lay, rows_per_chunk, n_chunks, error);                    \
+    launch_dependent(kern, grid, vqs::kThreads, smem, st, p, lay, rows_per_chunk, n_chunks, error);                    \
     return check_launch(op);                                                                             \
   }
   if (roww == 1) F2C_VQS(1)

@@ -23,6 +23,8 @@ struct HybridDecodeParams {
 
 template <int BITS>
 __global__ void __launch_bounds__(256) hybrid_decode_kernel(const HybridDecodeParams p) {
+  dependency_wait();
+  release_dependents();
   const int vec_per_row = p.feat_dim / 4;
   const int64_t n_vec = (p.sq_rows + p.vq_rows) * vec_per_row;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -114,11 +116,11 @@ extern "C" int f2c_hybrid_decompress(const void* sq_codes, int sq_dtype, const f
   unsigned grid = (unsigned)ceil_div(n_vec, 256);
   cudaStream_t st = (cudaStream_t)stream;
   switch (bits) {
-    case 1: hybrid_decode_kernel<1><<<grid, 256, 0, st>>>(p); break;
-    case 2: hybrid_decode_kernel<2><<<grid, 256, 0, st>>>(p); break;
-    case 4: hybrid_decode_kernel<4><<<grid, 256, 0, st>>>(p); break;
-    case 8: hybrid_decode_kernel<8><<<grid, 256, 0, st>>>(p); break;
-    default: hybrid_decode_kernel<16><<<grid, 256, 0, st>>>(p); break;
+    case 1: launch_dependent(hybrid_decode_kernel<1>, grid, 256, 0, st, p); break;
+    case 2: launch_dependent(hybrid_decode_kernel<2>, grid, 256, 0, st, p); break;
+    case 4: launch_dependent(hybrid_decode_kernel<4>, grid, 256, 0, st, p); break;
+    case 8: launch_dependent(hybrid_decode_kernel<8>, grid, 256, 0, st, p); break;
+    default: launch_dependent(hybrid_decode_kernel<16>, grid, 256, 0, st, p); break;
   }
   return check_launch(op);
 }

@@ -26,6 +26,8 @@ template <int METRIC, bool WRITE_DIST, bool WRITE_LABEL>
 __global__ void __launch_bounds__(256) kmeans_warp_kernel(const float* __restrict__ x, const float* __restrict__ y,
                                                           float* __restrict__ dist, int64_t* __restrict__ labels, int64_t n,
                                                           int k, int d, const int32_t* done) {
+  dependency_wait();
+  release_dependents();
   if (done != nullptr && *(volatile const int32_t*)done != 0) return;
   const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -73,6 +75,8 @@ template <int DMAX, int METRIC>
 __global__ void __launch_bounds__(256) kmeans_thread_kernel(const float* __restrict__ x, const float* __restrict__ y,
                                                             int64_t* __restrict__ labels, const int32_t* __restrict__ subset, int64_t n,
                                                             int k, int d, int kc, const int32_t* done) {
+  dependency_wait();
+  release_dependents();
   if (done != nullptr && *(volatile const int32_t*)done != 0) return;  // a fit that has converged (kmeans_fit.cu)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float* yc_s = reinterpret_cast<float*>(smem_raw);  // [kc][DMAX]
@@ -145,6 +149,8 @@ __global__ void __launch_bounds__(kListThreads) kmeans_listed_kernel(const float
                                                                      int64_t* __restrict__ labels, const int32_t* __restrict__ list,
                                                                      const int32_t* __restrict__ count_dev, int64_t max_count, int k, int d,
                                                                      int kc) {
+  dependency_wait();
+  release_dependents();
   constexpr int STRIDE = DMAX + 4;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int64_t cnt = *count_dev < max_count ? *count_dev : max_count;
@@ -248,7 +254,7 @@ static int launch_listed(const float* x, const float* y, int64_t* labels, const 
   if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "kmeans_assign: %s", cudaGetErrorString(e));
   int64_t grid = ceil_div(max_count, kListThreads / 32);
   if (grid > 2 * current_sm_count()) grid = 2 * current_sm_count();
-  kern<<<(unsigned)grid, kListThreads, smem, st>>>(x, y, labels, list, count_dev, max_count, (int)k, (int)d, kc);
+  launch_dependent(kern, (unsigned)grid, kListThreads, smem, st, x, y, labels, list, count_dev, max_count, (int)k, (int)d, kc);
   return check_launch("kmeans_assign");
 }
 
@@ -264,11 +270,11 @@ static int launch_thread_assign(const float* x, const float* y, int64_t* labels,
   if (metric == F2C_COSINE) {
     auto kern = kmeans_thread_kernel<DMAX, F2C_COSINE>;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) kern<<<grid, 256, smem, st>>>(x, y, labels, subset, n, (int)k, (int)d, kc, done);
+    if (e == cudaSuccess) launch_dependent(kern, grid, 256, smem, st, x, y, labels, subset, n, (int)k, (int)d, kc, done);
   } else {
     auto kern = kmeans_thread_kernel<DMAX, F2C_L2>;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) kern<<<grid, 256, smem, st>>>(x, y, labels, subset, n, (int)k, (int)d, kc, done);
+    if (e == cudaSuccess) launch_dependent(kern, grid, 256, smem, st, x, y, labels, subset, n, (int)k, (int)d, kc, done);
   }
   if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "kmeans_assign: %s", cudaGetErrorString(e));
   return check_launch("kmeans_assign");
@@ -287,9 +293,9 @@ int kmeans_assign_exact(const float* x, const float* y, int64_t* labels, const i
   int64_t blocks = ceil_div(n, 8);
   if (blocks > current_sm_count() * 32) blocks = current_sm_count() * 32;
   if (metric == F2C_COSINE)
-    kmeans_warp_kernel<F2C_COSINE, false, true><<<(unsigned)blocks, 256, 0, st>>>(x, y, nullptr, labels, n, (int)k, (int)d, done);
+    launch_dependent(kmeans_warp_kernel<F2C_COSINE, false, true>, (unsigned)blocks, 256, 0, st, x, y, nullptr, labels, n, (int)k, (int)d, done);
   else
-    kmeans_warp_kernel<F2C_L2, false, true><<<(unsigned)blocks, 256, 0, st>>>(x, y, nullptr, labels, n, (int)k, (int)d, done);
+    launch_dependent(kmeans_warp_kernel<F2C_L2, false, true>, (unsigned)blocks, 256, 0, st, x, y, nullptr, labels, n, (int)k, (int)d, done);
   return check_launch("kmeans_assign");
 }
 
@@ -331,9 +337,9 @@ extern "C" int f2c_pairwise_distance(const float* x, const float* y, float* dist
   if (blocks > current_sm_count() * 32) blocks = current_sm_count() * 32;
   cudaStream_t st = (cudaStream_t)stream;
   if (metric == F2C_COSINE)
-    kmeans_warp_kernel<F2C_COSINE, true, false><<<(unsigned)blocks, 256, 0, st>>>(x, y, dist, nullptr, n, (int)k, (int)d, nullptr);
+    launch_dependent(kmeans_warp_kernel<F2C_COSINE, true, false>, (unsigned)blocks, 256, 0, st, x, y, dist, nullptr, n, (int)k, (int)d, nullptr);
   else
-    kmeans_warp_kernel<F2C_L2, true, false><<<(unsigned)blocks, 256, 0, st>>>(x, y, dist, nullptr, n, (int)k, (int)d, nullptr);
+    launch_dependent(kmeans_warp_kernel<F2C_L2, true, false>, (unsigned)blocks, 256, 0, st, x, y, dist, nullptr, n, (int)k, (int)d, nullptr);
   return check_launch("pairwise_distance");
 }
 

@@ -48,6 +48,8 @@ __device__ __forceinline__ int fraction_bits(int64_t n) {
 }
 
 __global__ void __launch_bounds__(256) max_abs_kernel(const float* __restrict__ x, int64_t numel, State* st) {
+  dependency_wait();
+  release_dependents();
   uint32_t m = 0;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < numel; i += (int64_t)gridDim.x * blockDim.x)
     m = max(m, __float_as_uint(__ldg(x + i)) & 0x7fffffffu);  // NaN has larger bits than inf
@@ -56,6 +58,8 @@ __global__ void __launch_bounds__(256) max_abs_kernel(const float* __restrict__ 
 }
 
 __global__ void begin_kernel(State* st) {
+  dependency_wait();
+  release_dependents();
   if (threadIdx.x == 0 && st->max_bits >= 0x7f800000u) { st->not_finite = 1; st->done = 1; }
 }
 
@@ -96,6 +100,8 @@ template <bool SHARED>
 __global__ void __launch_bounds__(kThreads) accumulate_kernel(const float* __restrict__ x, const int64_t* __restrict__ labels,
                                                               float* __restrict__ centers, long long* sums, unsigned int* counts,
                                                               int64_t n, int k, int d, double tol, const int32_t* assign_error, State* st) {
+  dependency_wait();
+  release_dependents();
   if (*(volatile int32_t*)&st->done != 0) return;
   extern __shared__ __align__(16) unsigned char smem[];
   const int kd = k * d;
@@ -213,8 +219,8 @@ extern "C" int f2c_kmeans_fit_begin(const float* x, int64_t n, int64_t k, int64_
   fit::State* state = (fit::State*)workspace;
   int64_t blocks = ceil_div(n * d, 256 * 8);
   if (blocks > 8 * current_sm_count()) blocks = 8 * current_sm_count();
-  fit::max_abs_kernel<<<(unsigned)blocks, 256, 0, st>>>(x, n * d, state);
-  fit::begin_kernel<<<1, 32, 0, st>>>(state);
+  launch_dependent(fit::max_abs_kernel, (unsigned)blocks, 256, 0, st, x, n * d, state);
+  launch_dependent(fit::begin_kernel, 1, 32, 0, st, state);
   return check_launch(op);
 }
 
@@ -248,7 +254,7 @@ extern "C" int f2c_kmeans_fit_iterate(const float* x, float* centers, int64_t n,
     rc = tc ? kmeans_assign_tc(x, centers, labels, n, k, d, metric, ws + w.assign, st, &state->done)
             : kmeans_assign_exact(x, centers, labels, nullptr, n, k, d, metric, st, &state->done);
     if (rc) return rc;
-    kern<<<(unsigned)grid, fit::kThreads, shared ? smem : 0, st>>>(x, labels, centers, sums, counts, n, (int)k, (int)d, tol, assign_error,
+    launch_dependent(kern, (unsigned)grid, fit::kThreads, shared ? smem : 0, st, x, labels, centers, sums, counts, n, (int)k, (int)d, tol, assign_error,
                                                                   state);
     rc = check_launch(op);
     if (rc) return rc;

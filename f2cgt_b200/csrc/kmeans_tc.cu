@@ -163,6 +163,8 @@ struct Top2 {
 // [tmem slot][2 fail flags][2 x 128 floats |x|^2]
 template <bool BF16>
 __global__ void __launch_bounds__(kCtaThreads, 1) kmeans_tc_kernel(const Params p) {
+  dependency_wait();
+  release_dependents();
   extern __shared__ __align__(128) unsigned char smem[];
   if (p.done != nullptr && *(volatile const int32_t*)p.done != 0) return;
   const int tid = threadIdx.x;
@@ -492,7 +494,7 @@ int kmeans_assign_tc(const float* x, const float* y, int64_t* labels, int64_t n,
   int64_t tiles = ceil_div(n, tc::kTileM);
   int64_t grid = ceil_div(tiles, 2);  // one CTA per SM (it owns all 512 TMEM columns), two tiles in flight per CTA
   if (grid > current_sm_count()) grid = current_sm_count();
-  kern<<<(unsigned)grid, tc::kCtaThreads, smem, st>>>(p);
+  launch_dependent(kern, (unsigned)grid, tc::kCtaThreads, smem, st, p);
   int rc = check_launch("kmeans_assign (tensor cores)");
   if (rc) return rc;
   // undecided points: exact fp32 scorer over the device-side list

@@ -29,6 +29,8 @@ __device__ __forceinline__ uint32_t pack_word(const uint8_t* __restrict__ src) {
 template <int BITS>
 __global__ void __launch_bounds__(256) pack_flat_kernel(const uint8_t* __restrict__ unpack,
                                                         uint32_t* __restrict__ pack, int64_t n_words) {
+  dependency_wait();
+  release_dependents();
   constexpr int PER = 8 / BITS;
   constexpr int IN_BYTES = 4 * PER;  // 8, 16 or 32
   int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -49,6 +51,8 @@ template <int BITS>
 __global__ void __launch_bounds__(256) pack_generic_kernel(const uint8_t* __restrict__ unpack,
                                                            uint8_t* __restrict__ pack, int64_t n_out,
                                                            int64_t unpack_dim, int64_t pack_dim) {
+  dependency_wait();
+  release_dependents();
   constexpr int PER = 8 / BITS;
   constexpr uint32_t MASK = (1u << BITS) - 1u;
   int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -65,6 +69,8 @@ __global__ void __launch_bounds__(256) pack_generic_kernel(const uint8_t* __rest
 template <int BITS>
 __global__ void __launch_bounds__(256) unpack_flat_kernel(const uint32_t* __restrict__ pack,
                                                           uint8_t* __restrict__ unpack, int64_t n_words) {
+  dependency_wait();
+  release_dependents();
   constexpr int PER = 8 / BITS;
   constexpr int OUT_BYTES = 4 * PER;
   constexpr uint32_t MASK = (1u << BITS) - 1u;
@@ -87,6 +93,8 @@ template <int BITS>
 __global__ void __launch_bounds__(256) unpack_generic_kernel(const uint8_t* __restrict__ pack,
                                                              uint8_t* __restrict__ unpack, int64_t n_out,
                                                              int64_t unpack_dim, int64_t pack_dim) {
+  dependency_wait();
+  release_dependents();
   constexpr int PER = 8 / BITS;
   constexpr uint32_t MASK = (1u << BITS) - 1u;
   int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -104,9 +112,9 @@ static int launch_pack(const uint8_t* unpack, uint8_t* pack, int64_t rows, int64
   bool flat = unpack_dim % PER == 0 && n_out % 4 == 0 && aligned(unpack, 16) && aligned(pack, 4);
   if (flat) {
     int64_t n_words = n_out / 4;
-    pack_flat_kernel<BITS><<<(unsigned)ceil_div(n_words, 256), 256, 0, st>>>(unpack, (uint32_t*)pack, n_words);
+    launch_dependent(pack_flat_kernel<BITS>, (unsigned)ceil_div(n_words, 256), 256, 0, st, unpack, (uint32_t*)pack, n_words);
   } else {
-    pack_generic_kernel<BITS><<<(unsigned)ceil_div(n_out, 256), 256, 0, st>>>(unpack, pack, n_out, unpack_dim, pack_dim);
+    launch_dependent(pack_generic_kernel<BITS>, (unsigned)ceil_div(n_out, 256), 256, 0, st, unpack, pack, n_out, unpack_dim, pack_dim);
   }
   return check_launch("packbits");
 }
@@ -120,9 +128,9 @@ static int launch_unpack(const uint8_t* pack, uint8_t* unpack, int64_t rows, int
   bool flat = unpack_dim == pack_dim * PER && (rows * pack_dim) % 4 == 0 && aligned(unpack, 16) && aligned(pack, 4);
   if (flat) {
     int64_t n_words = rows * pack_dim / 4;
-    unpack_flat_kernel<BITS><<<(unsigned)ceil_div(n_words, 256), 256, 0, st>>>((const uint32_t*)pack, unpack, n_words);
+    launch_dependent(unpack_flat_kernel<BITS>, (unsigned)ceil_div(n_words, 256), 256, 0, st, (const uint32_t*)pack, unpack, n_words);
   } else {
-    unpack_generic_kernel<BITS><<<(unsigned)ceil_div(n_out, 256), 256, 0, st>>>(pack, unpack, n_out, unpack_dim, pack_dim);
+    launch_dependent(unpack_generic_kernel<BITS>, (unsigned)ceil_div(n_out, 256), 256, 0, st, pack, unpack, n_out, unpack_dim, pack_dim);
   }
   return check_launch("unpackbits");
 }

@@ -120,6 +120,8 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
 __global__ void __launch_bounds__(kThreads, 1) sage_forward_kernel(const __grid_constant__ CUtensorMap x1, const __grid_constant__ CUtensorMap x2,
                                                                    const __grid_constant__ CUtensorMap w1, const __grid_constant__ CUtensorMap w2,
                                                                    const Params p) {
+  dependency_wait();
+  release_dependents();
   extern __shared__ unsigned char smem_raw[];
   __shared__ Bars bars;
   __shared__ __align__(16) float epi_s[4 * kEpiFloats];
@@ -353,7 +355,7 @@ extern "C" int f2c_sage_forward(const float* x1, const float* x2, const float* w
   int64_t grid = current_sm_count() / col_tiles;
   if (grid < 1) grid = 1;
   if (grid > p.tiles) grid = p.tiles;
-  sg::sage_forward_kernel<<<dim3((unsigned)grid, (unsigned)col_tiles), sg::kThreads, smem, (cudaStream_t)stream>>>(maps[0], maps[1], maps[2],
+  launch_dependent(sg::sage_forward_kernel, dim3((unsigned)grid, (unsigned)col_tiles), sg::kThreads, smem, (cudaStream_t)stream, maps[0], maps[1], maps[2],
                                                                                                                maps[3], p);
   return check_launch(op);
 }

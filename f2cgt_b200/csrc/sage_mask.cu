@@ -14,6 +14,8 @@ constexpr int kThreads = 256;
 template <bool VEC, bool MASK>
 __global__ void __launch_bounds__(kThreads) sage_mask_kernel(const float* __restrict__ g, const float* __restrict__ h, float scale,
                                                              float* __restrict__ dy, float* __restrict__ db, int64_t rows, int n, int units) {
+  dependency_wait();
+  release_dependents();
   constexpr int E = VEC ? 4 : 1;
   extern __shared__ float sums[];
   for (int i = threadIdx.x; i < n; i += kThreads) sums[i] = 0.0f;
@@ -72,7 +74,7 @@ extern "C" int f2c_sage_mask(const float* g, const float* h, float scale, float*
   if (grid > 8 * current_sm_count()) grid = 8 * current_sm_count();
   auto kern = h != nullptr ? (vec ? sage_mask_kernel<true, true> : sage_mask_kernel<false, true>)
                            : (vec ? sage_mask_kernel<true, false> : sage_mask_kernel<false, false>);
-  kern<<<(unsigned)grid, kThreads, (size_t)n * 4, (cudaStream_t)stream>>>(g, h, scale, dy, db, rows, (int)n, units);
+  launch_dependent(kern, (unsigned)grid, kThreads, (size_t)n * 4, (cudaStream_t)stream, g, h, scale, dy, db, rows, (int)n, units);
   return check_launch(op);
 }
 
@@ -87,6 +89,8 @@ struct Ranges {
 };
 
 __global__ void __launch_bounds__(256) zero_ranges_kernel(const Ranges r) {
+  dependency_wait();
+  release_dependents();
   for (int i = 0; i < r.count; ++i)
     for (int64_t w = (int64_t)blockIdx.x * 256 + threadIdx.x; w < r.words[i]; w += (int64_t)gridDim.x * 256) r.at[i][w] = 0u;
 }
@@ -111,6 +115,6 @@ extern "C" int f2c_zero_ranges(void* const* ranges_host, const int64_t* bytes_ho
   if (r.count == 0) return F2C_OK;
   int64_t grid = ceil_div(most, 1024);
   if (grid > 2 * current_sm_count()) grid = 2 * current_sm_count();
-  zero_ranges_kernel<<<(unsigned)grid, 256, 0, (cudaStream_t)stream>>>(r);
+  launch_dependent(zero_ranges_kernel, (unsigned)grid, 256, 0, (cudaStream_t)stream, r);
   return check_launch(op);
 }

@@ -35,6 +35,8 @@ template <typename T, typename IdxT, int VEC>
 __global__ void __launch_bounds__(256) spmm_csr_kernel(const T* __restrict__ feat, T* __restrict__ out,
                                                        const IdxT* __restrict__ indptr, const IdxT* __restrict__ indices,
                                                        int64_t n_dst, int feat_dim, int reduce) {
+  dependency_wait();
+  release_dependents();
   using A = Acc<T>;
   struct alignas(sizeof(T) * VEC) Vec { T v[VEC]; };
   const int lane = threadIdx.x & 31;
@@ -87,10 +89,10 @@ static int launch_spmm(const void* feat, const void* indptr, const void* indices
   if (blocks > current_sm_count() * 64) blocks = current_sm_count() * 64;
   bool vec = D % VEC == 0 && aligned(feat, 16) && aligned(out, 16);
   if (vec)
-    spmm_csr_kernel<T, IdxT, VEC><<<(unsigned)blocks, 256, 0, st>>>((const T*)feat, (T*)out, (const IdxT*)indptr,
+    launch_dependent(spmm_csr_kernel<T, IdxT, VEC>, (unsigned)blocks, 256, 0, st, (const T*)feat, (T*)out, (const IdxT*)indptr,
                                                                      (const IdxT*)indices, n_dst, (int)D, reduce);
   else
-    spmm_csr_kernel<T, IdxT, 1><<<(unsigned)blocks, 256, 0, st>>>((const T*)feat, (T*)out, (const IdxT*)indptr,
+    launch_dependent(spmm_csr_kernel<T, IdxT, 1>, (unsigned)blocks, 256, 0, st, (const T*)feat, (T*)out, (const IdxT*)indptr,
                                                                    (const IdxT*)indices, n_dst, (int)D, reduce);
   return check_launch("spmm_csr");
 }
@@ -134,6 +136,8 @@ template <typename IdxT, bool VEC4>
 __global__ void __launch_bounds__(256) spmm_backward_kernel(const float* __restrict__ grad_out, float* __restrict__ grad_src,
                                                             const IdxT* __restrict__ indptr, const IdxT* __restrict__ indices,
                                                             int64_t n_dst, int feat_dim, int reduce) {
+  dependency_wait();
+  release_dependents();
   const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -172,7 +176,7 @@ extern "C" int f2c_spmm_csr_backward(const float* grad_out, const void* indptr, 
   int64_t blocks = ceil_div(n_dst, 8);
   if (blocks > current_sm_count() * 16) blocks = current_sm_count() * 16;
   const bool vec = feat_dim % 4 == 0 && aligned(grad_out, 16) && aligned(grad_src, 16);
-#define F2C_BW(T, V) spmm_backward_kernel<T, V><<<(unsigned)blocks, 256, 0, st>>>(grad_out, grad_src, (const T*)indptr, (const T*)indices, n_dst, (int)feat_dim, reduce)
+#define F2C_BW(T, V) launch_dependent(spmm_backward_kernel<T, V>, (unsigned)blocks, 256, 0, st, grad_out, grad_src, (const T*)indptr, (const T*)indices, n_dst, (int)feat_dim, reduce)
   if (index_dtype == F2C_I32) { if (vec) F2C_BW(int32_t, true); else F2C_BW(int32_t, false); }
   else { if (vec) F2C_BW(int64_t, true); else F2C_BW(int64_t, false); }
 #undef F2C_BW

@@ -17,6 +17,8 @@ template <int BITS>
 __global__ void __launch_bounds__(256) sq_compress_vec_kernel(const float4* __restrict__ src, float4* __restrict__ dst,
                                                               const float* __restrict__ codebooks, int64_t n_vec,
                                                               int vec_per_row, int column_slice) {
+  dependency_wait();
+  release_dependents();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_vec) return;
   int c0 = (int)(i % vec_per_row) * 4;
@@ -32,6 +34,8 @@ template <int BITS>
 __global__ void __launch_bounds__(256) sq_compress_scalar_kernel(const float* __restrict__ src, float* __restrict__ dst,
                                                                  const float* __restrict__ codebooks, int64_t numel,
                                                                  int feat_dim, int column_slice) {
+  dependency_wait();
+  release_dependents();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= numel) return;
   int c = (int)(i % feat_dim);
@@ -45,10 +49,10 @@ static int launch_compress(const float* src, float* dst, const float* cb, int64_
   if (numel == 0) return F2C_OK;
   if (D % 4 == 0 && aligned(src, 16) && aligned(dst, 16)) {
     int64_t n_vec = numel / 4;
-    sq_compress_vec_kernel<BITS><<<(unsigned)ceil_div(n_vec, 256), 256, 0, st>>>(
+    launch_dependent(sq_compress_vec_kernel<BITS>, (unsigned)ceil_div(n_vec, 256), 256, 0, st, 
         (const float4*)src, (float4*)dst, cb, n_vec, (int)(D / 4), (int)cs);
   } else {
-    sq_compress_scalar_kernel<BITS><<<(unsigned)ceil_div(numel, 256), 256, 0, st>>>(src, dst, cb, numel, (int)D, (int)cs);
+    launch_dependent(sq_compress_scalar_kernel<BITS>, (unsigned)ceil_div(numel, 256), 256, 0, st, src, dst, cb, numel, (int)D, (int)cs);
   }
   return check_launch("sq_compress");
 }
@@ -64,6 +68,8 @@ template <int BITS, typename CodeT>
 __global__ void __launch_bounds__(256) sq_decompress_scalar_kernel(const void* __restrict__ codes, float* __restrict__ out,
                                                                    const float* __restrict__ codebooks, int64_t numel,
                                                                    int64_t src_dim, int feat_dim, int column_slice) {
+  dependency_wait();
+  release_dependents();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= numel) return;
   int64_t row = i / feat_dim;
@@ -89,6 +95,8 @@ __global__ void __launch_bounds__(256) sq_decompress_vec_kernel(const void* __re
                                                                 const float* __restrict__ codebooks, int64_t n_chunks,
                                                                 int64_t src_dim, int feat_dim, int chunks_per_row,
                                                                 int column_slice) {
+  dependency_wait();
+  release_dependents();
   constexpr int EPT = BITS == 1 ? 8 : 4;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_chunks) return;
@@ -151,6 +159,8 @@ template <int BITS>
 __global__ void __launch_bounds__(kSqLutThreads) sq_decompress_lut_kernel(
     const uint8_t* __restrict__ codes, float* __restrict__ out, const float* __restrict__ codebooks, int64_t rows,
     int64_t row_bytes, int feat_dim, int chunks_per_row, int column_slice, int n_cb, int log_copies, int is_signed) {
+  dependency_wait();
+  release_dependents();
   constexpr int EPT = BITS == 1 ? 8 : 4;
   constexpr int NCODE = 1 << BITS;
   constexpr uint32_t MASK = NCODE - 1;
@@ -244,7 +254,7 @@ static bool try_decompress_lut(const void* codes, float* out, const float* cb, i
   int64_t grid = ceil_div(rows, rows_per_cta);
   const int64_t cap = (int64_t)current_sm_count() * (smem > 32 * 1024 ? 3 : 6);
   if (grid > cap) grid = cap;
-  kern<<<(unsigned)grid, kSqLutThreads, smem, st>>>((const uint8_t*)codes, out, cb, rows, src_dim, (int)D, (int)cpr, (int)cs,
+  launch_dependent(kern, (unsigned)grid, kSqLutThreads, smem, st, (const uint8_t*)codes, out, cb, rows, src_dim, (int)D, (int)cpr, (int)cs,
                                                     (int)n_cb, log_copies, std::is_signed<CodeT>::value ? 1 : 0);
   return true;
 }
@@ -262,10 +272,10 @@ static int launch_decompress(const void* codes, float* out, const float* cb, int
   if (try_decompress_lut<BITS, CodeT>(codes, out, cb, rows, src_dim, D, cs, st)) return check_launch("sq_decompress");
   if (vec) {
     int64_t n_chunks = numel / EPT;
-    sq_decompress_vec_kernel<BITS, CodeT><<<(unsigned)ceil_div(n_chunks, 256), 256, 0, st>>>(
+    launch_dependent(sq_decompress_vec_kernel<BITS, CodeT>, (unsigned)ceil_div(n_chunks, 256), 256, 0, st, 
         codes, out, cb, n_chunks, src_dim, (int)D, (int)(D / EPT), (int)cs);
   } else {
-    sq_decompress_scalar_kernel<BITS, CodeT><<<(unsigned)ceil_div(numel, 256), 256, 0, st>>>(
+    launch_dependent(sq_decompress_scalar_kernel<BITS, CodeT>, (unsigned)ceil_div(numel, 256), 256, 0, st, 
         codes, out, cb, numel, src_dim, (int)D, (int)cs);
   }
   return check_launch("sq_decompress");

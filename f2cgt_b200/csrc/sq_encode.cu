@@ -98,6 +98,8 @@ struct Args {
 // dim % 4 == 0, x 16-byte aligned, at most kThreads units per row.
 template <int BITS>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm) encode_vec_kernel(const Args a) {
+  dependency_wait();
+  release_dependents();
   constexpr int E = BITS >= 8 ? 4 : 8;  // columns per thread and row
   constexpr int Q = E / 4;
   constexpr int F = BITS >= 8 ? 4 : 2;  // rows in flight per thread
@@ -181,6 +183,8 @@ constexpr int kTileFloats = 6144;
 
 template <int BITS>
 __global__ void __launch_bounds__(kThreads) encode_tile_kernel(const Args a, int tile_rows, int aligned_in) {
+  dependency_wait();
+  release_dependents();
   constexpr int B = BITS >= 8 ? 8 : BITS;
   constexpr int PER = 8 / B;           // elements per stored byte (16 bits: per stored pair of bytes)
   extern __shared__ __align__(16) float tile_smem[];
@@ -245,7 +249,7 @@ static int launch_encode(Args a, cudaStream_t st, const char* op) {
     int64_t grid = ceil_div(a.rows, kThreads / a.units);
     const int64_t cap = kCtasPerSm * (int64_t)current_sm_count();
     if (grid > cap) grid = cap;
-    kern<<<(unsigned)grid, kThreads, par_bytes, st>>>(a);
+    launch_dependent(kern, (unsigned)grid, kThreads, par_bytes, st, a);
     return check_launch(op);
   }
   F2C_REQUIRE(aligned(a.out, 4), F2C_ERR_INVALID, "%s: the codes must be 4-byte aligned", op);
@@ -260,7 +264,7 @@ static int launch_encode(Args a, cudaStream_t st, const char* op) {
   int64_t grid = ceil_div(a.rows, tile_rows);
   const int64_t cap = 5 * (int64_t)current_sm_count();
   if (grid > cap) grid = cap;
-  kern<<<(unsigned)grid, kThreads, smem, st>>>(a, tile_rows, aligned(a.x, 16) ? 1 : 0);
+  launch_dependent(kern, (unsigned)grid, kThreads, smem, st, a, tile_rows, aligned(a.x, 16) ? 1 : 0);
   return check_launch(op);
 }
 

@@ -82,6 +82,8 @@ __device__ void locate(const uint32_t* __restrict__ hist, unsigned long long ran
 // PASS 1, 2, 3; VEC = 4: rows and columns allow 16-byte loads
 template <int PASS, int VEC>
 __global__ void __launch_bounds__(kThreads) select_kernel(const Args a) {
+  dependency_wait();
+  release_dependents();
   extern __shared__ __align__(16) uint32_t hist_s[];
   __shared__ bool last;
   __shared__ double warp_total[kThreads / 32];
@@ -248,7 +250,7 @@ static cudaError_t launch(const Args& a, int grid, cudaStream_t st) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
   }
-  kern<<<(unsigned)grid, kThreads, smem, st>>>(a);
+  launch_dependent(kern, (unsigned)grid, kThreads, smem, st, a);
   return cudaGetLastError();
 }
 

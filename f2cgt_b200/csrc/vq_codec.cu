@@ -33,6 +33,8 @@ template <typename CodeT, typename CbT>
 __global__ void __launch_bounds__(256) vq_decompress_vec_kernel(const void* __restrict__ codes, const CbT* __restrict__ cbs,
                                                                 float* __restrict__ out, int64_t n_vec, int vec_per_row,
                                                                 int n_cb, uint32_t length, int cs, int feat_dim) {
+  dependency_wait();
+  release_dependents();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_vec) return;
   int64_t row = i / vec_per_row;
@@ -47,6 +49,8 @@ template <typename CodeT, typename CbT>
 __global__ void __launch_bounds__(256) vq_decompress_scalar_kernel(const void* __restrict__ codes, const CbT* __restrict__ cbs,
                                                                    float* __restrict__ out, int64_t numel, int n_cb,
                                                                    uint32_t length, int cs, int feat_dim) {
+  dependency_wait();
+  release_dependents();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= numel) return;
   int64_t row = i / feat_dim;
@@ -67,6 +71,8 @@ constexpr size_t kVqStreamSmem = 200 * 1024;
 __global__ void __launch_bounds__(kVqStreamThreads, 1) vq_decompress_stream_kernel(
     const uint8_t* __restrict__ codes, const float* __restrict__ cbs, float* __restrict__ out, int64_t rows, int vec_per_row,
     int n_cb, int K, int cs, int feat_dim, int spq, int stride) {
+  dependency_wait();
+  release_dependents();
   extern __shared__ __align__(128) unsigned char vq_smem[];
   {  // consecutive threads write consecutive 16-byte pieces of shared memory (no bank conflicts while staging)
     const int lg4 = 31 - __clz(cs >> 2);
@@ -133,7 +139,7 @@ static bool try_vq_decompress_stream(const void* codes, const float* cbs, float*
   const int rows_per_cta = kVqStreamThreads / (int)(D / 4);
   int64_t grid = ceil_div(rows, rows_per_cta);
   if (grid > current_sm_count()) grid = current_sm_count();
-  vq_decompress_stream_kernel<<<(unsigned)grid, kVqStreamThreads, smem, st>>>(
+  launch_dependent(vq_decompress_stream_kernel, (unsigned)grid, kVqStreamThreads, smem, st, 
       (const uint8_t*)codes, cbs, out, rows, (int)(D / 4), (int)n_cb, (int)K, (int)cs, (int)D, spq, stride);
   return true;
 }
@@ -149,10 +155,10 @@ static int launch_vq_decompress(const void* codes, const void* cbs, float* out, 
     return check_launch("vq_decompress");
   if (vec) {
     int64_t n_vec = numel / 4;
-    vq_decompress_vec_kernel<CodeT, CbT><<<(unsigned)ceil_div(n_vec, 256), 256, 0, st>>>(
+    launch_dependent(vq_decompress_vec_kernel<CodeT, CbT>, (unsigned)ceil_div(n_vec, 256), 256, 0, st, 
         codes, (const CbT*)cbs, out, n_vec, (int)(D / 4), (int)n_cb, (uint32_t)length, (int)cs, (int)D);
   } else {
-    vq_decompress_scalar_kernel<CodeT, CbT><<<(unsigned)ceil_div(numel, 256), 256, 0, st>>>(
+    launch_dependent(vq_decompress_scalar_kernel<CodeT, CbT>, (unsigned)ceil_div(numel, 256), 256, 0, st, 
         codes, (const CbT*)cbs, out, numel, (int)n_cb, (uint32_t)length, (int)cs, (int)D);
   }
   return check_launch("vq_decompress");
