@@ -64,6 +64,27 @@ __device__ __forceinline__ uint32_t ldg_nc_u32(const void* p) {
   asm volatile("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
   return v;
 }
+__device__ __forceinline__ uint32_t ldg_nc_u32_if(const void* p, bool on) {  // 0 without a load when !on; no branch
+  uint32_t v = 0u;
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.global.nc.L1::no_allocate.u32 %0, [%1];\n\t}" : "+r"(v) : "l"(p), "r"((uint32_t)on));
+  return v;
+}
+__device__ __forceinline__ uint2 ldg_nc_u64_if(const void* p, bool on) {
+  uint2 v = make_uint2(0u, 0u);
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\t@q ld.global.nc.L1::no_allocate.v2.u32 {%0,%1}, [%2];\n\t}" : "+r"(v.x), "+r"(v.y) : "l"(p), "r"((uint32_t)on));
+  return v;
+}
+// low 32 bits of a neighbour id, 0 without a load when !on
+__device__ __forceinline__ uint32_t ld_id_if(const int32_t* p, bool on) {
+  uint32_t v = 0u;
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.global.nc.u32 %0, [%1];\n\t}" : "+r"(v) : "l"(p), "r"((uint32_t)on));
+  return v;
+}
+__device__ __forceinline__ uint32_t ld_id_if(const int64_t* p, bool on) {
+  uint32_t v = 0u;
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.global.nc.u32 %0, [%1];\n\t}" : "+r"(v) : "l"(p), "r"((uint32_t)on));
+  return v;
+}
 __device__ __forceinline__ uint2 ldg_nc_u64(const void* p) {
   uint2 v;
   asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));

@@ -86,6 +86,8 @@ struct SqParams {
   uint32_t rows_per_shard;
   unsigned long long shard_magic;  // floor(2^64 / rows_per_shard) + 1: exact 32-bit division by one multiply-high
   int staged;        // 1: rows leave through the shared-memory staging area (feat_dim % 4 == 0)
+  // RAGGED kernels: blockIdx.y = part; a column slice is cut into slice_parts parts of part_cols columns (the last may be short)
+  int slice_parts, part_cols;
   int stage_offset;  // byte offset of that area in dynamic shared memory
   DropoutArgs drop;
 };
@@ -93,7 +95,11 @@ struct SqParams {
 // U = neighbours held in registers per destination row (rows with more take extra, unpipelined rounds).
 // PEER: the table is row-sharded over the GPUs of one NVSwitch box and every shard is mapped into this process;
 // a neighbour's row is read from its owner's HBM with an ordinary load over NVLink (no collective, no staging copy).
-template <int BITS, int VEC, int U, typename IdxT, int DEC, bool PEER = false>
+// RAGGED: rows of any length at any alignment (VEC = 4), worked in column parts of at most 31 words that lie in one column slice.
+// Lane w loads the w-th ALIGNED word that the part touches in a neighbour's row (one lane more than the part has words, so a
+// group is one power of two wider at times); at the decode it takes the next lane's word by a shuffle and joins the two with
+// a funnel shift.  Nothing beyond the word of the row's last byte is read.
+template <int BITS, int VEC, int U, typename IdxT, int DEC, bool PEER = false, bool RAGGED = false>
 __global__ void __launch_bounds__(SqCta<BITS, DEC>::kThreads, SqCta<BITS, DEC>::kCtasPerSm)
 sq_spmm_kernel(const SqParams p) {
   dependency_wait();
@@ -113,11 +119,24 @@ sq_spmm_kernel(const SqParams p) {
   const int sub = lane >> p.logG;
   const int rows_per_warp = 32 >> p.logG;
   const uint32_t byte0 = (uint32_t)lane_g * VEC;
-  const bool lane_active = byte0 < p.row_bytes;
+  // column part of this CTA: columns [col_base, col_base + cols), bytes [byte_base, byte_base + part_bytes) of a row
+  int col_base = 0, cols = p.feat_dim, slice = 0;
+  uint32_t byte_base = 0, part_bytes = p.row_bytes;
+  if (RAGGED) {
+    slice = (int)blockIdx.y / p.slice_parts;
+    const int within = ((int)blockIdx.y - slice * p.slice_parts) * p.part_cols;
+    col_base = slice * p.column_slice + within;
+    cols = min(min(p.part_cols, p.column_slice - within), p.feat_dim - col_base);
+    if (cols <= 0) return;  // a short last slice has fewer parts
+    byte_base = (uint32_t)col_base * BITS / 8u;
+    part_bytes = ((uint32_t)cols * BITS + 7u) / 8u;
+  }
+  const bool lane_active = byte0 < part_bytes + (RAGGED ? 4u : 0u);  // RAGGED: has a word to load
+  const bool lane_stores = byte0 < part_bytes;
   const int c0 = lane_g * EPL;
 
   // Codebook row of this lane's columns (the host guarantees they share one row on this path).
-  int cb_row = c0 / p.column_slice;
+  int cb_row = RAGGED ? slice : c0 / p.column_slice;
   if (cb_row >= p.n_cb) cb_row = p.n_cb - 1;
   const float emin = __ldg(p.codebooks + cb_row * kCodebookDim + 2);
   const float emax = __ldg(p.codebooks + cb_row * kCodebookDim + 3);
@@ -133,7 +152,7 @@ sq_spmm_kernel(const SqParams p) {
   const IdxT* __restrict__ indices = reinterpret_cast<const IdxT*>(p.indices);
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t stride = (((int64_t)gridDim.x * blockDim.x) >> 5) * rows_per_warp;
-  const uint8_t* __restrict__ my_codes = p.codes + byte0;
+  const uint8_t* __restrict__ my_codes = p.codes + byte_base + byte0;
   // address of this lane's slice of source row `id`
   auto row_ptr = [&](uint32_t id) -> const uint8_t* {
     if (!PEER) return my_codes + (uint64_t)id * p.row_bytes;
@@ -155,6 +174,19 @@ sq_spmm_kernel(const SqParams p) {
   // overwrites them with the ids of the row after (the hardware scoreboard orders the two).
   uint32_t nidx[U];
   VecLoad<VEC> data[2][U];
+  uint32_t shifts[2] = {0u, 0u};  // RAGGED: misalignment of slot u in bytes, at bit 2 u
+  static_assert(!RAGGED || (VEC == 4 && U <= 16 && !PEER), "ragged rows: one word per lane");
+  // this lane's aligned word of a row (0 where it has none or `on` is false), without a branch; returns the misalignment, 0 when
+  // !on: a slot without a neighbour has to stay 0 through the join, because its table copy has a single slab
+  auto load_word = [&](uint32_t id, bool on, VecLoad<VEC>& v) -> uint32_t {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(row_ptr(id));
+    const uint32_t off = (uint32_t)at & 3u;
+    v.w[0] = ldg_nc_u32_if(reinterpret_cast<const void*>(at - off), on && byte0 < off + part_bytes);
+    return on ? off : 0u;
+  };
+  auto joined = [&](uint32_t word, uint32_t off) -> uint32_t {  // all lanes of the warp call
+    return __funnelshift_r(word, __shfl_down_sync(0xffffffffu, word, 1), off * 8u);
+  };
   auto prime = [&]() {
     if (d < n_dst && lane_active) { int64_t b = (int64_t)indptr[d]; degA = (int)((int64_t)indptr[d + 1] - b); idsA = indices + b; }
     if (d + istride < n_dst && lane_active) {
@@ -164,21 +196,24 @@ sq_spmm_kernel(const SqParams p) {
       int64_t b = (int64_t)indptr[d + 2 * istride]; degC = (int)((int64_t)indptr[d + 2 * istride + 1] - b); idsC = indices + b;
     }
 #pragma unroll
-    for (int u = 0; u < U; ++u) nidx[u] = u < degA ? (uint32_t)idsA[u] : 0u;
+    for (int u = 0; u < U; ++u) nidx[u] = ld_id_if(idsA + u, u < degA);
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      data[0][u].zero();
-      if (u < degA) data[0][u].load(row_ptr(nidx[u]));
+      if constexpr (RAGGED) {
+        shifts[0] |= load_word(nidx[u], u < degA, data[0][u]) << (2 * u);
+      } else {
+        data[0][u].load_if(row_ptr(nidx[u]), u < degA);
+      }
     }
 #pragma unroll
-    for (int u = 0; u < U; ++u) nidx[u] = u < degB ? (uint32_t)idsB[u] : 0u;
+    for (int u = 0; u < U; ++u) nidx[u] = ld_id_if(idsB + u, u < degB);
   };
   if (PRIME_EARLY) prime();
   uint32_t lane_off = 0;
   if (DEC == DEC_LUT) {
     using L = Lut<BITS>;
-    build_sq_table<BITS, EPL>(smem_raw, reinterpret_cast<float*>(smem_raw + L::TABLE_BYTES + 256), p.codebooks, p.n_cb, p.column_slice,
-                              G, p.code_kind, (int)threadIdx.x, (int)blockDim.x, [] { __syncthreads(); });
+    build_sq_table<BITS, EPL>(smem_raw, reinterpret_cast<float*>(smem_raw + L::TABLE_BYTES + 256),
+                              p.codebooks + (RAGGED ? cb_row * kCodebookDim : 0), RAGGED ? 1 : p.n_cb, p.column_slice, RAGGED ? 1 : G, p.code_kind, (int)threadIdx.x, (int)blockDim.x, [] { __syncthreads(); });
     lane_off = L::lane_offset(lane);
     if (ALIGNED) lane_off |= (uint32_t)__cvta_generic_to_shared(smem_raw);  // low 16 bits of the base are zero
   }
@@ -201,12 +236,16 @@ sq_spmm_kernel(const SqParams p) {
         // (1) code rows of the next destination row -> data[P^1]
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-          data[P ^ 1][u].zero();
-          if (u < degB) data[P ^ 1][u].load(row_ptr(nidx[u]));
+          if (RAGGED && u == 0) shifts[P ^ 1] = 0u;
+          if constexpr (RAGGED) {
+            shifts[P ^ 1] |= load_word(nidx[u], u < degB, data[P ^ 1][u]) << (2 * u);
+          } else {
+            data[P ^ 1][u].load_if(row_ptr(nidx[u]), u < degB);
+          }
         }
         // (2) neighbour ids of the row after it
 #pragma unroll
-        for (int u = 0; u < U; ++u) nidx[u] = u < degC ? (uint32_t)idsC[u] : 0u;
+        for (int u = 0; u < U; ++u) nidx[u] = ld_id_if(idsC + u, u < degC);
         // (3) indptr pair three rows ahead
         const IdxT* idsD = indices;
         int degD = 0;
@@ -223,7 +262,8 @@ sq_spmm_kernel(const SqParams p) {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
           if (u < umax) {  // warp uniform
-            const VecLoad<VEC>& row = data[P][u];
+            VecLoad<VEC> row = data[P][u];
+            if constexpr (RAGGED) row.w[0] = joined(row.w[0], (shifts[P] >> (2 * u)) & 3u);
             if (DEC == DEC_LUT) {
               sq_accumulate<BITS, VEC, DEC, ALIGNED>(acc, row, table, u < degA ? lane_off : lane_off_zero, p.code_kind, scale, emin, mean);
             } else if (u < degA) {
@@ -232,19 +272,32 @@ sq_spmm_kernel(const SqParams p) {
           }
         }
         // destination rows with more than U neighbours: further rounds of four, not pipelined
-        for (int k = U; k < degA; k += 4) {
+        const int degX = RAGGED ? __reduce_max_sync(0xffffffffu, degA) : degA;  // the shuffles below are the warp's
+        for (int k = U; k < degX; k += 4) {
           VecLoad<VEC> extra[4];
+          uint32_t off[4];
 #pragma unroll
-          for (int u = 0; u < 4; ++u)
-            if (k + u < degA) extra[u].load(row_ptr((uint32_t)idsA[k + u]));
+          for (int u = 0; u < 4; ++u) {
+            const bool on = k + u < degA;
+            if constexpr (RAGGED) off[u] = load_word(on ? (uint32_t)idsA[k + u] : 0u, on, extra[u]);
+            else if (on) extra[u].load(row_ptr((uint32_t)idsA[k + u]));
+          }
+          if constexpr (RAGGED) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) extra[u].w[0] = joined(extra[u].w[0], off[u]);
+          }
 #pragma unroll
           for (int u = 0; u < 4; ++u)
             if (k + u < degA) sq_accumulate<BITS, VEC, DEC, ALIGNED>(acc, extra[u], table, lane_off, p.code_kind, scale, emin, mean);
         }
 
         // (5) mean / dropout / store
-        const bool have_row = d < n_dst && lane_active;
-        if (p.staged) {
+        const bool have_row = d < n_dst && lane_stores;
+        if constexpr (RAGGED) {
+          float* stage = reinterpret_cast<float*>(smem_raw + p.stage_offset) + (threadIdx.x >> 5) * (32 * EPL);
+          sq_store_ragged<EPL>(acc, stage, lane, p.logG, degA, have_row, (int64_t)row_base, (int64_t)(n_dst - row_base), cols, col_base,
+                               p.feat_dim, p.reduce, div_safe, p.drop, p.out);
+        } else if (p.staged) {
           float4* stage = reinterpret_cast<float4*>(smem_raw + p.stage_offset) + (threadIdx.x >> 5) * (32 * (EPL / 4));
           sq_store_rows<EPL>(acc, stage, lane, p.logG, degA, have_row, (int64_t)row_base, (int64_t)(n_dst - row_base), p.feat_dim,
                              p.reduce, div_safe, p.drop, p.out);
@@ -334,15 +387,15 @@ struct ResidentCache {
   size_t smem[64] = {};
 };
 
-template <int BITS, int VEC, int U, typename IdxT, int DEC, bool PEER = false>
-static int launch_fast(SqParams p, bool vec_store, cudaStream_t st) {
-  auto kern = sq_spmm_kernel<BITS, VEC, U, IdxT, DEC, PEER>;
+template <int BITS, int VEC, int U, typename IdxT, int DEC, bool PEER = false, bool RAGGED = false>
+static int launch_fast(SqParams p, bool vec_store, cudaStream_t st, int parts = 1) {
+  auto kern = sq_spmm_kernel<BITS, VEC, U, IdxT, DEC, PEER, RAGGED>;
   constexpr int EPL = BITS == 16 ? VEC / 2 : VEC * 8 / BITS;
   // decode table (64 KB) + the decoded code values of each distinct codebook row
   size_t smem = 0;
   if (DEC == DEC_LUT) {
     using L = Lut<BITS>;
-    int n_rows = (1 << p.logG) < L::COPIES ? (1 << p.logG) : L::COPIES;
+    int n_rows = RAGGED ? 1 : (1 << p.logG) < L::COPIES ? (1 << p.logG) : L::COPIES;
     smem = L::TABLE_BYTES + 256 + (size_t)n_rows * L::NCODE * sizeof(float);
   }
   constexpr int kThreads = SqCta<BITS, DEC>::kThreads;
@@ -350,7 +403,7 @@ static int launch_fast(SqParams p, bool vec_store, cudaStream_t st) {
   // staging area for coalesced output: warps x 32 lanes x EPL floats
   p.staged = 0;
   p.stage_offset = (int)smem;
-  if (vec_store && EPL >= 4) {
+  if (RAGGED || (vec_store && EPL >= 4)) {
     p.staged = 1;
     smem += (size_t)kWarpsPerCta * 32 * EPL * sizeof(float);
   }
@@ -377,8 +430,9 @@ static int launch_fast(SqParams p, bool vec_store, cudaStream_t st) {
   }
   int rows_per_cta = kWarpsPerCta * (32 >> p.logG);
   int64_t grid = ceil_div(p.n_dst, rows_per_cta);
-  if (grid > (int64_t)sms * resident) grid = (int64_t)sms * resident;
-  launch_dependent(kern, (unsigned)grid, kThreads, smem, st, p);
+  const int64_t most = (int64_t)sms * resident >= parts ? (int64_t)sms * resident / parts : 1;
+  if (grid > most) grid = most;
+  launch_dependent(kern, dim3((unsigned)grid, (unsigned)parts), kThreads, smem, st, p);
   return check_launch("sq_decompress_spmm_csr");
 }
 
@@ -404,12 +458,12 @@ static int launch_sq_spmm(const void* codes, int code_dtype, const float* codebo
                           int reduce, const DropoutArgs& drop, int variant, cudaStream_t st, const PeerInfo* peer = nullptr) {
   if (n_dst == 0 || D == 0) return F2C_OK;
   const char* op = peer ? "sq_decompress_spmm_csr_peer" : "sq_decompress_spmm_csr";
-  // ---- streamed kernel (producer warps + shared-memory ring).  Measured on B200 (2,449,029-row table, outermost block
-  //      of 1024 seeds x fan-out 12,12,12, cold L2): 2-bit codes 36.9 us against 41.9 us for the register-prefetch kernel;
-  //      1 bit 41-43 against 41, 4 bit 49.5 against 43.7, 8 bit 61.4 against 49.2 - staging the rows costs shared-memory
-  //      wavefronts (7.0 M against 4.5 M at 4 bits) that the table decode needs itself, so only the 2-bit shape, whose
-  //      rows are cheap to stage and whose prefetch kernel is the most latency-bound, gains.
-  const bool stream_by_default = BITS == 2 && peer == nullptr;
+  // ---- streamed kernel (producer warps + shared-memory ring): 2-bit codes and many rows only.  Staging the rows costs
+  //      shared-memory wavefronts that the table decode needs itself (cold L2, 59,000 rows x 12 neighbours x 128 columns: 4 bits 49.5
+  //      against 43.7 us, 8 bits 61.4 against 49.2), so only the width whose rows are cheap to stage gains (36.9 against 41.9 us),
+  //      and its start costs 3 us more: 2 bits, 128 columns, 8,000 / 16,000 / 32,000 rows 9.7 / 13.6 / 20.1 against 7.9 / 11.8 / 20.1 us, 256
+  //      columns 13.1 / 18.9 / 29.4 against 11.8 / 19.2 / 31.2 us - even at four million sums.
+  const bool stream_by_default = BITS == 2 && peer == nullptr && n_dst * D >= (4ll << 20);
   if (variant == F2C_KERNEL_STREAM && peer != nullptr && peer->n_replicated > 0)
     return set_error(F2C_ERR_UNSUPPORTED, "%s: the streamed kernel does not serve a table with replicated leading rows", op);
   if ((variant == F2C_KERNEL_AUTO && stream_by_default) || variant == F2C_KERNEL_STREAM) {
@@ -447,6 +501,10 @@ static int launch_sq_spmm(const void* codes, int code_dtype, const float* codebo
     // table copies are shared by lanes l and l + COPIES: they must own the same columns
     int copies = BITS >= 4 ? 32 : BITS == 2 ? 16 : 8;
     bool lut = (n_cb == 1 || copies % G == 0) && variant != F2C_KERNEL_PREFETCH_ARITH;
+    // Few sums do not pay for the 64 KB table: 128 columns, 1,000 / 2,000 / 4,000 rows of 12 neighbours take 6.5 / 6.7 / 9.0 us by
+    // exp2f against 7.8 / 8.0 / 8.1 us at 8 bits, 7.7 / 8.0 / 8.1 against 8.1 / 8.2 / 8.3 us at 4 bits; 1-bit codes need no exp2f (8,000 rows:
+    // 7.4 against 8.0 us); 2-bit tables are quicker to build than the codes to decode.
+    if (variant == F2C_KERNEL_AUTO && peer == nullptr && BITS != 2 && n_dst * D <= (BITS == 1 ? 1ll << 20 : 1ll << 18)) lut = false;
     if (peer != nullptr) {
       const int head_slots = (int)ceil_div(peer->n_replicated, peer->rows_per_shard);
       for (int k = 0; k < 16; ++k) {
@@ -463,6 +521,30 @@ static int launch_sq_spmm(const void* codes, int code_dtype, const float* codebo
     return dispatch_fast<BITS, IdxT>(p, vec, lut, D % 4 == 0 && aligned(out, 16), st);
   }
   if (peer != nullptr) return set_error(F2C_ERR_UNSUPPORTED, "%s: shape not served by the peer kernel", op);
+  // ---- rows of any length and alignment, in column parts of at most 31 words, each inside one column slice
+  if (natural_dtype && n_src < (1ll << 32) && n_dst < (1ll << 30) && row_bytes < (1ll << 31) && variant == F2C_KERNEL_AUTO) {
+    constexpr int kLaneCols = BITS == 16 ? 2 : 32 / BITS;
+    const int64_t width = n_cb == 1 ? D : cs < D ? cs : D, slices = ceil_div(D, width);
+    const int64_t slice_parts = ceil_div(width, 31 * kLaneCols);
+    int64_t part_cols = ceil_div(ceil_div(width, slice_parts), 8) * 8;
+    if (part_cols > 31 * kLaneCols) part_cols = 31 * kLaneCols / 8 * 8;
+    if ((BITS < 16 || n_dst * D <= 1ll << 18) && part_cols * slice_parts >= width && slices * slice_parts <= 64 && (slices == 1 || width * BITS % 8 == 0)) {
+      SqParams p{};
+      p.codes = (const uint8_t*)codes; p.codebooks = codebooks; p.indptr = indptr; p.indices = indices; p.out = out;
+      p.n_dst = n_dst; p.row_bytes = (uint32_t)row_bytes; p.feat_dim = (int)D; p.column_slice = (int)width; p.n_cb = (int)n_cb;
+      p.logG = ilog2((int)ceil_div((part_cols < width ? part_cols : width) * BITS, 32) + 1);
+      p.code_kind = code_dtype == F2C_I8 ? CODE_I8 : code_dtype == F2C_U8 ? CODE_U8 : CODE_I16;
+      p.reduce = reduce; p.drop = drop; p.slice_parts = (int)slice_parts; p.part_cols = (int)part_cols;
+      const int parts = (int)(slices * slice_parts);
+      // Measured on B200, 12 neighbours per row, general kernel -> this one: 90,000 rows of 200 2-bit columns 196 -> 89 us, 301 1-bit 240 -> 126,
+      // 380 4-bit 335 -> 211, 357 8-bit 391 -> 276; 300 rows of 357 8-bit columns 18.4 -> 5.8.  16-bit codes have no table: two elements
+      // per lane and word leave too little work beside the row's addresses (90,000 x 110: 143 -> 209), so only few rows go here.
+      if constexpr (BITS <= 8)
+        if (BITS == 2 || n_dst * D > (BITS == 1 ? 1ll << 20 : 1ll << 18))
+          return launch_fast<BITS, 4, 12, IdxT, DEC_LUT, false, true>(p, false, st, parts);
+      return launch_fast<BITS, 4, 12, IdxT, DEC_ARITH, false, true>(p, false, st, parts);
+    }
+  }
   if (variant == F2C_KERNEL_PREFETCH || variant == F2C_KERNEL_PREFETCH_ARITH)
     return set_error(F2C_ERR_UNSUPPORTED, "%s: shape not served by the register-prefetch kernel", op);
   int64_t blocks = ceil_div(n_dst, 8);

@@ -14,12 +14,14 @@ template <int VEC> struct VecLoad;
 template <> struct VecLoad<4> {
   uint32_t w[1];
   __device__ __forceinline__ void load(const void* p) { w[0] = ldg_nc_u32(p); }
+  __device__ __forceinline__ void load_if(const void* p, bool on) { w[0] = ldg_nc_u32_if(p, on); }
   __device__ __forceinline__ void load_shared(uint32_t a) { asm volatile("ld.shared.b32 %0, [%1];" : "=r"(w[0]) : "r"(a)); }
   __device__ __forceinline__ void zero() { w[0] = 0u; }
 };
 template <> struct VecLoad<8> {
   uint32_t w[2];
   __device__ __forceinline__ void load(const void* p) { uint2 v = ldg_nc_u64(p); w[0] = v.x; w[1] = v.y; }
+  __device__ __forceinline__ void load_if(const void* p, bool on) { uint2 v = ldg_nc_u64_if(p, on); w[0] = v.x; w[1] = v.y; }
   __device__ __forceinline__ void load_shared(uint32_t a) {
     asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(w[0]), "=r"(w[1]) : "r"(a));
   }
@@ -224,6 +226,39 @@ __device__ __forceinline__ void sq_store_rows(const AccT& acc, float4* stage, in
       }
       if (drop.enabled) v = dropout_apply4(v, (uint64_t)(dr * feat_dim + 4 * c), drop);
       stg_cs_f4(out + dr * feat_dim + 4 * c, v);
+    }
+  }
+  __syncwarp();
+}
+
+// The same for a column part of rows of any width: sums staged as plain rows, read back so that the lanes of the warp write
+// consecutive columns, four bytes each (a row of the output need not start on a 16-byte boundary).
+//   stage   the warp's area of 32 * EPL floats; a lane's columns are rotated by its number, so that neither the writes (stride
+//           EPL between lanes) nor the reads (stride 1) meet in a bank
+template <int EPL, typename AccT>
+__device__ __forceinline__ void sq_store_ragged(const AccT& acc, float* stage, int lane, int logG, int deg, bool have_row, int64_t row_base,
+                                                int64_t n_rows_left, int cols, int col_base, int feat_dim, int reduce, bool div_safe,
+                                                const DropoutArgs& drop, float* __restrict__ out) {
+  const int rows_per_warp = 32 >> logG;
+  if (have_row) {
+#pragma unroll
+    for (int e = 0; e < EPL; ++e) stage[lane * EPL + ((e + lane) & (EPL - 1))] = acc.get(e);
+  }
+  float my_rcp = 0.0f;
+  if (reduce == F2C_MEAN && deg > 1) my_rcp = 1.0f / (float)deg;
+  __syncwarp();
+  for (int row = 0; row < rows_per_warp; ++row) {
+    if (row >= n_rows_left) break;
+    const int64_t dr = row_base + row;
+    const float rcp = __shfl_sync(0xffffffffu, my_rcp, row << logG);
+    const float degf = (float)__shfl_sync(0xffffffffu, deg, row << logG);
+    for (int c = lane; c < cols; c += 32) {
+      const int writer = (row << logG) + c / EPL;
+      float v = stage[writer * EPL + ((c + writer) & (EPL - 1))];
+      if (rcp != 0.0f) v = div_safe ? div_exact_fast(v, degf, rcp) : div_exact(v, degf, rcp);
+      const int64_t at = dr * feat_dim + col_base + c;
+      if (drop.enabled) v = dropout_apply1(v, (uint64_t)at, drop);
+      __stcs(out + at, v);
     }
   }
   __syncwarp();

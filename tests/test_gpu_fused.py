@@ -507,3 +507,29 @@ def test_two_level_over_sharded_tables_equals_whole_tables(capi, oracle, hot_bit
     got = ops.two_level_decompress_spmm_csr_peer(Peers(sq_t, n_hot), dev(cb), hot_bits, D, vq_peers, cbs, slot_peers, ip, ix, D)
     want = capi.two_level_decompress_spmm_csr(sq_t, dev(cb), hot_bits, D, codes, cbs, slot, ip, ix, D)
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("bits", [1, 2, 4, 8, 16])
+@pytest.mark.parametrize("D,cs", [(1, 8), (7, 8), (33, 40), (71, 24), (127, 128), (129, 136), (200, 200), (257, 264), (100, 56), (513, 520), (1025, 1032), (300, 8)])
+def test_fused_sq_rows_of_any_length(capi, oracle, bits, D, cs):
+    """Rows whose length or start is no multiple of a word, several column parts and slices: same bits as the general kernel,
+    also from a table that starts at an odd address (8-bit and packed codes) and with dropout."""
+    rng = np.random.default_rng(bits * 31 + D)
+    n_src, n_dst = 200, 301
+    _, cb, stored = sq_table(oracle, rng, n_src, D, bits, cs)
+    codes, t_cb = dev(stored), dev(cb)
+    tables = [codes]
+    if bits <= 8:
+        shifted = torch.empty(codes.numel() + 3, dtype=codes.dtype, device="cuda")[3:].view_as(codes)
+        tables.append(shifted.copy_(codes))
+    for n in (n_dst, 40 * n_dst):  # few rows: decoded by exp2f; many: by the table
+        deg = rng.integers(0, 20, n)
+        deg[::9] = 0
+        deg[7] = 150
+        indptr = np.concatenate([[0], np.cumsum(deg)]).astype(np.int64)
+        indices = rng.integers(0, n_src, int(indptr[-1])).astype(np.int64)
+        for table in tables:
+            for idx in (np.int64, np.int32):
+                args = (table, t_cb, dev(indptr.astype(idx)), dev(indices.astype(idx)), bits, cs, D)
+                for kw in (dict(), dict(reduce="sum"), dict(dropout=dict(p=0.4, seed=3, offset=2, training=True, scale=True))):
+                    assert torch.equal(capi.sq_decompress_spmm_csr(*args, **kw), capi.sq_decompress_spmm_csr(*args, kernel="general", **kw)), (kw, idx, n)
