@@ -263,8 +263,16 @@ extern "C" int f2c_vq_spmm_csr(const void* codes, int code_dtype, const float* c
   const int variant = kernel_variant(epilogue);
   bool served = false;
   if (variant != F2C_KERNEL_GENERAL) {
+    if (variant == F2C_KERNEL_AUTO && feat_dim <= 64) {  // half a warp per row (64 columns in 4 x 16 or 8 x 8)
+      rc = launch_vq_rows(p, index_dtype, st, op, &served);
+      if (served || rc) return rc;
+    }
     rc = launch_vq_fast(p, 0, index_dtype, variant, st, op, &served);
     if (served || rc) return rc;
+    if (variant == F2C_KERNEL_AUTO) {
+      rc = launch_vq_rows(p, index_dtype, st, op, &served);
+      if (served || rc) return rc;
+    }
     if (variant != F2C_KERNEL_AUTO) return set_error(F2C_ERR_UNSUPPORTED, "%s: shape not served by the requested kernel family", op);
   }
   return index_dtype == F2C_I32 ? launch_vq<0, int32_t>(p, st, op) : launch_vq<0, int64_t>(p, st, op);

@@ -47,6 +47,9 @@ struct VqParams {
 int launch_vq_fast(VqParams& p, int hot_bits, int index_dtype, int variant, cudaStream_t st, const char* op, bool* served,
                    bool peer = false);
 
+// Two destination rows per warp, nearly any shape (fused_vq_rows.cu), for VQ tables of this GPU.
+int launch_vq_rows(VqParams& p, int index_dtype, cudaStream_t st, const char* op, bool* served);
+
 // Make sure the current device can read `ptr` (device memory of this or another GPU of the box): peer access is
 // one-directional and is requested here when needed (idempotent).  Returns a status with the error text set.
 int ensure_readable_from_current_device(const void* ptr, const char* op, const char* what, int index);

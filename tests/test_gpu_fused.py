@@ -533,3 +533,29 @@ def test_fused_sq_rows_of_any_length(capi, oracle, bits, D, cs):
                 args = (table, t_cb, dev(indptr.astype(idx)), dev(indices.astype(idx)), bits, cs, D)
                 for kw in (dict(), dict(reduce="sum"), dict(dropout=dict(p=0.4, seed=3, offset=2, training=True, scale=True))):
                     assert torch.equal(capi.sq_decompress_spmm_csr(*args, **kw), capi.sq_decompress_spmm_csr(*args, kernel="general", **kw)), (kw, idx, n)
+
+
+@pytest.mark.parametrize("n_cb,cs,D,K,dtype", [(1, 4, 3, 256, np.uint8), (2, 64, 128, 256, np.uint8), (3, 8, 24, 7, np.uint8), (7, 16, 110, 256, np.uint8), (13, 8, 100, 256, np.uint8),
+                                               (14, 8, 110, 256, np.uint8), (25, 8, 200, 256, np.uint8), (32, 8, 256, 256, np.uint8), (5, 32, 157, 200, np.uint8), (16, 16, 256, 256, np.uint8),
+                                               (8, 16, 128, 1024, np.int16), (3, 8, 23, 300, np.int16), (9, 12, 101, 33, np.uint8), (4, 32, 128, 600, np.int16), (6, 20, 120, 256, np.uint8),
+                                               (4, 16, 64, 256, np.uint8), (8, 8, 64, 256, np.uint8), (2, 32, 64, 255, np.uint8)])
+def test_fused_vq_any_shape_equals_the_general_kernel(capi, n_cb, cs, D, K, dtype):
+    """Two rows per warp: any code row length, part count, code width and output width; rows with more than 16 neighbours, empty
+    rows, an odd number of rows, a table at an odd address, codes beyond the codebook."""
+    rng = np.random.default_rng(n_cb * 100 + cs)
+    n_src, n_dst = 500, 2001
+    codes = dev(rng.integers(0, min(K + 3, 256) if dtype == np.uint8 else K + 3, (n_src, n_cb)).astype(dtype))
+    cbs = dev(rng.standard_normal((n_cb, K, cs)).astype(np.float32))
+    deg = rng.integers(0, 19, n_dst)
+    deg[::11] = 0
+    deg[5::400] = 75
+    indptr = np.concatenate([[0], np.cumsum(deg)]).astype(np.int64)
+    indices = rng.integers(0, n_src, int(indptr[-1])).astype(np.int64)
+    tables = [codes]
+    if dtype == np.uint8:
+        tables.append(torch.empty(codes.numel() + 3, dtype=codes.dtype, device="cuda")[3:].view_as(codes).copy_(codes))
+    for table in tables:
+        for idx in (np.int64, np.int32):
+            args = (table, cbs, dev(indptr.astype(idx)), dev(indices.astype(idx)), D)
+            for kw in (dict(), dict(reduce="sum"), dict(dropout=dict(p=0.4, seed=3, offset=2, training=True, scale=True))):
+                assert torch.equal(capi.vq_decompress_spmm_csr(*args, **kw), capi.vq_decompress_spmm_csr(*args, kernel="general", **kw)), (kw, idx)
