@@ -92,26 +92,8 @@ __global__ void __launch_bounds__(VqCta<HB>::kThreads, 1) vq_fast_kernel(const V
   const int col_end = min(s_end * p.cs, p.feat_dim);
   const int K = (int)p.K, cs = p.cs, spq = p.fast_spq, stride = p.fast_stride;
 
-  // ---- stage this part's codebooks (layout in the header comment); column_slice is a power of two here.
-  //      Consecutive threads write consecutive 16-byte pieces of shared memory (no bank conflicts while staging).
-  {
-    const int lg4 = 31 - __clz(cs >> 2);  // log2(float4 pieces per centroid)
-    const int n_sub = s_end - s_begin;
-    const float4* src = reinterpret_cast<const float4*>(p.codebooks + (int64_t)s_begin * K * cs);
-    float4* dst = reinterpret_cast<float4*>(cb_s);
-    if (spq > 1) {  // 128-byte line = the centroids `code` of spq consecutive subspaces
-      const int n16 = ((n_sub + spq - 1) / spq) * K * 8;
-      for (int i = threadIdx.x; i < n16; i += kThreads) {
-        const int piece = i & 7, line = i >> 3;
-        const int code = line % K, grp = line / K;
-        const int sl = grp * spq + (piece >> lg4), q = piece & ((1 << lg4) - 1);
-        dst[i] = sl < n_sub ? __ldg(src + ((sl * K + code) << lg4) + q) : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-    } else {        // natural layout: the staged image equals the global one
-      const int n16 = (n_sub * K) << lg4;
-      for (int i = threadIdx.x; i < n16; i += kThreads) dst[i] = __ldg(src + i);
-    }
-  }
+  // ---- stage this part's codebooks (layout in the header comment); the hot-row table is built while they arrive
+  stage_codebooks(cb_s, p.codebooks + (int64_t)s_begin * K * cs, s_end - s_begin, K, cs, spq, kThreads);
   // ---- hot-row decode table: entry (byte, lane) = the floats that `byte` decodes to with the codebook row of
   //      that lane's columns; slab `byte` starts at byte * 256, a lane's entry is 4 (8-bit) or 8 (4-bit) bytes
   if (HB != 0) {
@@ -133,6 +115,7 @@ __global__ void __launch_bounds__(VqCta<HB>::kThreads, 1) vq_fast_kernel(const V
       }
     }
   }
+  codebooks_staged();
   __syncthreads();
 
   // ---- lane constants

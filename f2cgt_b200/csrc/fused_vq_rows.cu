@@ -96,24 +96,7 @@ __global__ void __launch_bounds__(kThreads, 1) vq_rows_kernel(const VqParams p) 
   const int s_begin = (int)blockIdx.y * p.cb_per_part, s_end = min(s_begin + p.cb_per_part, p.n_cb), n_sub = s_end - s_begin;
   const int col_begin = s_begin * p.cs, col_end = min(s_end * p.cs, p.feat_dim);
   const int K = (int)p.K, cs = p.cs, spq = p.fast_spq, stride = p.fast_stride;
-  // ---- stage this part's codebooks
-  {
-    const float4* src = reinterpret_cast<const float4*>(p.codebooks + (int64_t)s_begin * K * cs);
-    float4* dst = reinterpret_cast<float4*>(cb_s);
-    if (spq > 1) {  // 128-byte line = the centroids `code` of spq consecutive subspaces; column_slice is a power of two
-      const int lg4 = 31 - __clz(cs >> 2);
-      const int n16 = ((n_sub + spq - 1) / spq) * K * 8;
-      for (int i = threadIdx.x; i < n16; i += kThreads) {
-        const int piece = i & 7, line = i >> 3;
-        const int code = line % K, grp = line / K;
-        const int sl = grp * spq + (piece >> lg4), q = piece & ((1 << lg4) - 1);
-        dst[i] = sl < n_sub ? __ldg(src + ((sl * K + code) << lg4) + q) : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-    } else {
-      const int n16 = n_sub * K * (cs / 4);
-      for (int i = threadIdx.x; i < n16; i += kThreads) dst[i] = __ldg(src + i);
-    }
-  }
+  stage_codebooks(cb_s, p.codebooks + (int64_t)s_begin * K * cs, n_sub, K, cs, spq, kThreads);
   // ---- lane constants
   uint32_t cb_addr[NCH], code_addr[NCH];
   bool active[NCH];
@@ -126,6 +109,7 @@ __global__ void __launch_bounds__(kThreads, 1) vq_rows_kernel(const VqParams p) 
     cb_addr[c] = smem_u32(cb_s) + (spq > 1 ? (uint32_t)((sl / spq) * K * 128 + (sl % spq) * cs * 4 + off * 4) : (uint32_t)(sl * K * stride + off * 4));
     code_addr[c] = smem_u32(tile) + (uint32_t)(half * HALF + sl * kNb * EB);
   }
+  codebooks_staged();
   __syncthreads();
 
   const IdxT* __restrict__ indptr = reinterpret_cast<const IdxT*>(p.indptr);

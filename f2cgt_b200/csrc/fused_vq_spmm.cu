@@ -83,10 +83,8 @@ __global__ void __launch_bounds__(kVqThreads) vq_spmm_kernel(const VqParams p) {
   const int col_end = min(s_end * p.cs, p.feat_dim);
   const float* __restrict__ cb_g = p.codebooks + (int64_t)s_begin * p.K * p.cs;
   if (CB_SMEM) {
-    const int n4 = (s_end - s_begin) * (int)p.K * p.cs / 4;
-    const float4* src = reinterpret_cast<const float4*>(cb_g);
-    float4* dst = reinterpret_cast<float4*>(cb_s);
-    for (int i = threadIdx.x; i < n4; i += blockDim.x) dst[i] = __ldg(src + i);
+    stage_codebooks(smem_raw, cb_g, s_end - s_begin, (int)p.K, p.cs, 1, kVqThreads);
+    codebooks_staged();
     __syncthreads();
   }
   const float* cb = CB_SMEM ? cb_s : cb_g;
@@ -197,11 +195,19 @@ __global__ void __launch_bounds__(256) vq_spmm_generic_kernel(const VqParams p) 
   }
 }
 
+// Few rows and narrow subspaces: no codebooks in shared memory at all, every centroid is read through L2.  While each row has a
+// warp of its own (32 per SM) and one tile of 128 columns, that takes 7 to 8 us whatever the shape, less than staging the
+// interleaved codebooks first (256 centroids, 12 neighbours, 300 / 2,000 / 4,000 rows: 110 columns in slices of 8 8.5 / 8.6 / 10.2 us against
+// 6.9 / 7.3 / 7.3, 128 two-level 8.5 / 10.1 / 11.8 against 7.7 / 7.9 / 8.0); slices of 32 and more stage in 5 us, 64 columns in 4.
+static bool unstaged_is_faster(const VqParams& p) {
+  return p.cs < 32 && p.feat_dim > 64 && p.feat_dim <= 128 && p.n_dst <= (int64_t)current_sm_count() * (kVqThreads / 32);
+}
+
 template <int HB, typename IdxT>
-static int launch_vq(VqParams& p, cudaStream_t st, const char* op) {
+static int launch_vq(VqParams& p, cudaStream_t st, const char* op, bool few = false) {
   // split the subspaces over blockIdx.y until one part's codebooks fit in shared memory
   size_t one_cb = (size_t)p.K * p.cs * sizeof(float);
-  bool use_smem = one_cb <= kVqSmemBudget;
+  bool use_smem = one_cb <= kVqSmemBudget && !few;
   int parts = 1;
   if (use_smem) {
     while (ceil_div(p.n_cb, parts) * one_cb > kVqSmemBudget) ++parts;
@@ -261,8 +267,9 @@ extern "C" int f2c_vq_spmm_csr(const void* codes, int code_dtype, const float* c
     return check_launch(op);
   }
   const int variant = kernel_variant(epilogue);
+  const bool few = variant == F2C_KERNEL_AUTO && unstaged_is_faster(p);
   bool served = false;
-  if (variant != F2C_KERNEL_GENERAL) {
+  if (variant != F2C_KERNEL_GENERAL && !few) {
     if (variant == F2C_KERNEL_AUTO && feat_dim <= 64) {  // half a warp per row (64 columns in 4 x 16 or 8 x 8)
       rc = launch_vq_rows(p, index_dtype, st, op, &served);
       if (served || rc) return rc;
@@ -275,7 +282,7 @@ extern "C" int f2c_vq_spmm_csr(const void* codes, int code_dtype, const float* c
     }
     if (variant != F2C_KERNEL_AUTO) return set_error(F2C_ERR_UNSUPPORTED, "%s: shape not served by the requested kernel family", op);
   }
-  return index_dtype == F2C_I32 ? launch_vq<0, int32_t>(p, st, op) : launch_vq<0, int64_t>(p, st, op);
+  return index_dtype == F2C_I32 ? launch_vq<0, int32_t>(p, st, op, few) : launch_vq<0, int64_t>(p, st, op, few);
 }
 
 extern "C" int f2c_hybrid_spmm_csr(const void* sq_codes, int sq_dtype, const float* sq_codebooks, int64_t sq_n_codebooks,
@@ -313,14 +320,15 @@ extern "C" int f2c_hybrid_spmm_csr(const void* sq_codes, int sq_dtype, const flo
   p.sq_cs = (int)sq_column_slice; p.sq_n_cb = (int)sq_n_codebooks; p.sq_signed = sq_dtype == F2C_I8;
   cudaStream_t st = (cudaStream_t)stream;
   const int variant = kernel_variant(epilogue);
+  const bool few = variant == F2C_KERNEL_AUTO && unstaged_is_faster(p);
   bool served = false;
-  if (variant != F2C_KERNEL_GENERAL) {
+  if (variant != F2C_KERNEL_GENERAL && !few) {
     rc = launch_vq_fast(p, bits, index_dtype, variant, st, op, &served);
     if (served || rc) return rc;
     if (variant != F2C_KERNEL_AUTO) return set_error(F2C_ERR_UNSUPPORTED, "%s: shape not served by the requested kernel family", op);
   }
 #define F2C_HY(B) \
-  return index_dtype == F2C_I32 ? launch_vq<B, int32_t>(p, st, op) : launch_vq<B, int64_t>(p, st, op)
+  return index_dtype == F2C_I32 ? launch_vq<B, int32_t>(p, st, op, few) : launch_vq<B, int64_t>(p, st, op, few)
   switch (bits) {
     case 1: F2C_HY(1);
     case 2: F2C_HY(2);

@@ -8,7 +8,7 @@
 // clamped to the last centroid so that a bad table cannot fault the device.
 #include <type_traits>
 
-#include "common.cuh"
+#include "vq_params.cuh"
 
 namespace f2c {
 
@@ -74,23 +74,8 @@ __global__ void __launch_bounds__(kVqStreamThreads, 1) vq_decompress_stream_kern
   dependency_wait();
   release_dependents();
   extern __shared__ __align__(128) unsigned char vq_smem[];
-  {  // consecutive threads write consecutive 16-byte pieces of shared memory (no bank conflicts while staging)
-    const int lg4 = 31 - __clz(cs >> 2);
-    const float4* src = reinterpret_cast<const float4*>(cbs);
-    float4* dst = reinterpret_cast<float4*>(vq_smem);
-    if (spq > 1) {  // 128-byte line = the centroids `code` of spq consecutive subspaces
-      const int n16 = ((n_cb + spq - 1) / spq) * K * 8;
-      for (int i = threadIdx.x; i < n16; i += kVqStreamThreads) {
-        const int piece = i & 7, line = i >> 3;
-        const int code = line % K, grp = line / K;
-        const int sl = grp * spq + (piece >> lg4), q = piece & ((1 << lg4) - 1);
-        dst[i] = sl < n_cb ? __ldg(src + ((sl * K + code) << lg4) + q) : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-    } else {
-      const int n16 = (n_cb * K) << lg4;
-      for (int i = threadIdx.x; i < n16; i += kVqStreamThreads) dst[i] = __ldg(src + i);
-    }
-  }
+  stage_codebooks(vq_smem, cbs, n_cb, K, cs, spq, kVqStreamThreads);
+  codebooks_staged();
   __syncthreads();
   const int rows_per_cta = kVqStreamThreads / vec_per_row;
   const int j = (threadIdx.x % vec_per_row) * 4;

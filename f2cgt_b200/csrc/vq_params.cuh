@@ -42,6 +42,34 @@ struct VqParams {
   VqPeer peer;        // only read by PEER kernels
 };
 
+// Codebooks of n_sub subspaces (n_sub x K centroids of cs floats, cs % 4 == 0, 16-byte aligned) into shared memory with threads
+// 0 .. nthr-1: as they are (spq = 1), or - cs a power of two below 32 - with the centroids `code` of spq consecutive subspaces
+// side by side in a 128-byte line.  Copies are asynchronous, so that all of a thread's are in flight at once (loads through
+// registers with a division per piece took 2.4 us more for 16 x 256 x 8 floats); they are complete after
+// codebooks_staged() and a barrier.
+__device__ __forceinline__ void copy16_async(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void stage_codebooks(unsigned char* dst, const float* __restrict__ src, int n_sub, int K, int cs, int spq, int nthr) {
+  const uint32_t to = (uint32_t)__cvta_generic_to_shared(dst);
+  if (spq > 1) {
+    const int lg4 = 31 - __clz(cs >> 2);
+    const int piece = threadIdx.x & 7, q = piece & ((1 << lg4) - 1);  // nthr is a multiple of 8
+    for (int grp = 0; grp * spq < n_sub; ++grp) {
+      const int sl = grp * spq + (piece >> lg4);
+      const uint32_t line0 = to + (uint32_t)grp * K * 128 + piece * 16;
+      if (sl < n_sub) {
+        const float* from = src + (int64_t)sl * K * cs + 4 * q;
+        for (int code = threadIdx.x >> 3; code < K; code += nthr >> 3) copy16_async(line0 + code * 128, from + code * cs);
+      }
+    }
+  } else {
+    const int n16 = n_sub * K * (cs / 4);
+    for (int i = threadIdx.x; i < n16; i += nthr) copy16_async(to + i * 16, src + 4 * i);
+  }
+}
+__device__ __forceinline__ void codebooks_staged() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // Streamed (fused_vq_stream.cu) or register-prefetch (fused_vq_fast.cu) kernel for the common shapes, by `variant`
 // (an f2c_kernel value); sets *served = false (and launches nothing) when the shape is not one of theirs.
 int launch_vq_fast(VqParams& p, int hot_bits, int index_dtype, int variant, cudaStream_t st, const char* op, bool* served,

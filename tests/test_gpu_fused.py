@@ -543,7 +543,7 @@ def test_fused_vq_any_shape_equals_the_general_kernel(capi, n_cb, cs, D, K, dtyp
     """Two rows per warp: any code row length, part count, code width and output width; rows with more than 16 neighbours, empty
     rows, an odd number of rows, a table at an odd address, codes beyond the codebook."""
     rng = np.random.default_rng(n_cb * 100 + cs)
-    n_src, n_dst = 500, 2001
+    n_src, n_dst = 500, 6001  # more rows than one per warp of the general kernel
     codes = dev(rng.integers(0, min(K + 3, 256) if dtype == np.uint8 else K + 3, (n_src, n_cb)).astype(dtype))
     cbs = dev(rng.standard_normal((n_cb, K, cs)).astype(np.float32))
     deg = rng.integers(0, 19, n_dst)
