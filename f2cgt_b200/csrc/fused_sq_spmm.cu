@@ -86,8 +86,10 @@ struct SqParams {
   uint32_t rows_per_shard;
   unsigned long long shard_magic;  // floor(2^64 / rows_per_shard) + 1: exact 32-bit division by one multiply-high
   int staged;        // 1: rows leave through the shared-memory staging area (feat_dim % 4 == 0)
-  // RAGGED kernels: blockIdx.y = part; a column slice is cut into slice_parts parts of part_cols columns (the last may be short)
-  int slice_parts, part_cols;
+  // RAGGED kernels: blockIdx.y = part; a column slice is cut into slice_parts parts of part_cols columns (the last may be short).
+  // slice_parts = 0: parts of part_cols columns of the whole row, whose lanes may belong to different slices.  words_aligned: every
+  // part of every row starts on a word
+  int slice_parts, part_cols, words_aligned;
   int stage_offset;  // byte offset of that area in dynamic shared memory
   DropoutArgs drop;
 };
@@ -123,20 +125,22 @@ sq_spmm_kernel(const SqParams p) {
   int col_base = 0, cols = p.feat_dim, slice = 0;
   uint32_t byte_base = 0, part_bytes = p.row_bytes;
   if (RAGGED) {
-    slice = (int)blockIdx.y / p.slice_parts;
+    slice = p.slice_parts > 0 ? (int)blockIdx.y / p.slice_parts : 0;
     const int within = ((int)blockIdx.y - slice * p.slice_parts) * p.part_cols;
     col_base = slice * p.column_slice + within;
-    cols = min(min(p.part_cols, p.column_slice - within), p.feat_dim - col_base);
+    cols = min(p.part_cols, p.feat_dim - col_base);
+    if (p.slice_parts > 0) cols = min(cols, p.column_slice - within);
     if (cols <= 0) return;  // a short last slice has fewer parts
     byte_base = (uint32_t)col_base * BITS / 8u;
     part_bytes = ((uint32_t)cols * BITS + 7u) / 8u;
   }
-  const bool lane_active = byte0 < part_bytes + (RAGGED ? 4u : 0u);  // RAGGED: has a word to load
+  const bool lane_active = byte0 < part_bytes + (RAGGED && !p.words_aligned ? 4u : 0u);  // RAGGED: has a word to load
   const bool lane_stores = byte0 < part_bytes;
   const int c0 = lane_g * EPL;
 
   // Codebook row of this lane's columns (the host guarantees they share one row on this path).
-  int cb_row = RAGGED ? slice : c0 / p.column_slice;
+  const bool one_slice = RAGGED && p.slice_parts > 0;
+  int cb_row = one_slice ? slice : (col_base + c0) / p.column_slice;
   if (cb_row >= p.n_cb) cb_row = p.n_cb - 1;
   const float emin = __ldg(p.codebooks + cb_row * kCodebookDim + 2);
   const float emax = __ldg(p.codebooks + cb_row * kCodebookDim + 3);
@@ -213,7 +217,8 @@ sq_spmm_kernel(const SqParams p) {
   if (DEC == DEC_LUT) {
     using L = Lut<BITS>;
     build_sq_table<BITS, EPL>(smem_raw, reinterpret_cast<float*>(smem_raw + L::TABLE_BYTES + 256),
-                              p.codebooks + (RAGGED ? cb_row * kCodebookDim : 0), RAGGED ? 1 : p.n_cb, p.column_slice, RAGGED ? 1 : G, p.code_kind, (int)threadIdx.x, (int)blockDim.x, [] { __syncthreads(); });
+                              p.codebooks + (one_slice ? slice * kCodebookDim : 0), one_slice ? 1 : p.n_cb, p.column_slice, one_slice ? 1 : G,
+                              RAGGED && !one_slice ? col_base : 0, p.code_kind, (int)threadIdx.x, (int)blockDim.x, [] { __syncthreads(); });
     lane_off = L::lane_offset(lane);
     if (ALIGNED) lane_off |= (uint32_t)__cvta_generic_to_shared(smem_raw);  // low 16 bits of the base are zero
   }
@@ -395,7 +400,7 @@ static int launch_fast(SqParams p, bool vec_store, cudaStream_t st, int parts = 
   size_t smem = 0;
   if (DEC == DEC_LUT) {
     using L = Lut<BITS>;
-    int n_rows = RAGGED ? 1 : (1 << p.logG) < L::COPIES ? (1 << p.logG) : L::COPIES;
+    int n_rows = (1 << p.logG) < L::COPIES ? (1 << p.logG) : L::COPIES;
     smem = L::TABLE_BYTES + 256 + (size_t)n_rows * L::NCODE * sizeof(float);
   }
   constexpr int kThreads = SqCta<BITS, DEC>::kThreads;
@@ -524,24 +529,45 @@ static int launch_sq_spmm(const void* codes, int code_dtype, const float* codebo
   // ---- rows of any length and alignment, in column parts of at most 31 words, each inside one column slice
   if (natural_dtype && n_src < (1ll << 32) && n_dst < (1ll << 30) && row_bytes < (1ll << 31) && variant == F2C_KERNEL_AUTO) {
     constexpr int kLaneCols = BITS == 16 ? 2 : 32 / BITS;
-    const int64_t width = n_cb == 1 ? D : cs < D ? cs : D, slices = ceil_div(D, width);
-    const int64_t slice_parts = ceil_div(width, 31 * kLaneCols);
-    int64_t part_cols = ceil_div(ceil_div(width, slice_parts), 8) * 8;
-    if (part_cols > 31 * kLaneCols) part_cols = 31 * kLaneCols / 8 * 8;
-    if ((BITS < 16 || n_dst * D <= 1ll << 18) && part_cols * slice_parts >= width && slices * slice_parts <= 64 && (slices == 1 || width * BITS % 8 == 0)) {
+    const bool few = BITS != 2 && n_dst * D <= (BITS == 1 ? 1ll << 20 : 1ll << 18);  // decoded by exp2f, as above
+    const bool rows_aligned = row_bytes % 4 == 0 && aligned(codes, 4);  // then a part needs no word more than it has
+    const int64_t slices = n_cb == 1 || cs >= D ? 1 : ceil_div(D, cs);
+    const int copies = BITS >= 4 ? 32 : BITS == 2 ? 16 : 8;  // of the table: lanes further apart share one
+    struct Plan { int64_t slice_parts, part_cols, parts; int logG; bool words_aligned, ok; };
+    // parts of every slice, or (across) of the whole row
+    auto plan = [&](bool across) {
+      Plan q{};
+      const int64_t width = slices == 1 || across ? D : cs;
+      q.words_aligned = rows_aligned && (slices == 1 || across || width * BITS % 32 == 0);
+      const int64_t step = (q.words_aligned || across) && kLaneCols > 8 ? kLaneCols : 8;
+      const int64_t max_cols = (q.words_aligned ? 32 : 31) * kLaneCols / step * step;
+      q.slice_parts = ceil_div(width, max_cols);
+      q.part_cols = q.slice_parts == 1 ? width : ceil_div(ceil_div(width, q.slice_parts), step) * step;
+      q.parts = (slices == 1 || across ? 1 : slices) * q.slice_parts;
+      q.logG = ilog2((int)ceil_div(q.part_cols * BITS, 32) + (q.words_aligned ? 0 : 1));
+      q.ok = q.parts <= 64 && (slices == 1 || (across ? cs % kLaneCols == 0 && (few || BITS > 8 || copies % (1 << q.logG) == 0) : width * BITS % 8 == 0));
+      return q;
+    };
+    Plan q = plan(false);
+    bool across = false;
+    if (slices > 1) {
+      const Plan wide = plan(true);
+      if (wide.ok && (!q.ok || wide.parts < q.parts)) { q = wide; across = true; }
+    }
+    if ((BITS < 16 || n_dst * D <= 1ll << 18) && q.ok) {
       SqParams p{};
       p.codes = (const uint8_t*)codes; p.codebooks = codebooks; p.indptr = indptr; p.indices = indices; p.out = out;
-      p.n_dst = n_dst; p.row_bytes = (uint32_t)row_bytes; p.feat_dim = (int)D; p.column_slice = (int)width; p.n_cb = (int)n_cb;
-      p.logG = ilog2((int)ceil_div((part_cols < width ? part_cols : width) * BITS, 32) + 1);
+      p.n_dst = n_dst; p.row_bytes = (uint32_t)row_bytes; p.feat_dim = (int)D; p.column_slice = (int)(slices > 1 ? cs : D);
+      p.n_cb = (int)n_cb; p.logG = q.logG;
       p.code_kind = code_dtype == F2C_I8 ? CODE_I8 : code_dtype == F2C_U8 ? CODE_U8 : CODE_I16;
-      p.reduce = reduce; p.drop = drop; p.slice_parts = (int)slice_parts; p.part_cols = (int)part_cols;
-      const int parts = (int)(slices * slice_parts);
+      p.reduce = reduce; p.drop = drop; p.slice_parts = across ? 0 : (int)q.slice_parts; p.part_cols = (int)q.part_cols;
+      p.words_aligned = q.words_aligned;
+      const int parts = (int)q.parts;
       // Measured on B200, 12 neighbours per row, general kernel -> this one: 90,000 rows of 200 2-bit columns 196 -> 89 us, 301 1-bit 240 -> 126,
       // 380 4-bit 335 -> 211, 357 8-bit 391 -> 276; 300 rows of 357 8-bit columns 18.4 -> 5.8.  16-bit codes have no table: two elements
       // per lane and word leave too little work beside the row's addresses (90,000 x 110: 143 -> 209), so only few rows go here.
       if constexpr (BITS <= 8)
-        if (BITS == 2 || n_dst * D > (BITS == 1 ? 1ll << 20 : 1ll << 18))
-          return launch_fast<BITS, 4, 12, IdxT, DEC_LUT, false, true>(p, false, st, parts);
+        if (!few) return launch_fast<BITS, 4, 12, IdxT, DEC_LUT, false, true>(p, false, st, parts);
       return launch_fast<BITS, 4, 12, IdxT, DEC_ARITH, false, true>(p, false, st, parts);
     }
   }

@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(Geo<BITS>::kThreads, 1) sq_stream_kernel(const
     } else {
       // =========================================================== consumer warps
       if (!table_built) {
-        build_sq_table<BITS, EPL>(table_g, values, p.codebooks, p.n_cb, p.column_slice, G, p.code_kind, tid, C * 32,
+        build_sq_table<BITS, EPL>(table_g, values, p.codebooks, p.n_cb, p.column_slice, G, 0, p.code_kind, tid, C * 32,
                                   [] { asm volatile("bar.sync 1, %0;" ::"n"(C * 32) : "memory"); });
         table_built = true;
       }

@@ -20,6 +20,7 @@
 // Measured on B200, 90,000 rows x 12 neighbours, general kernel -> this one: 110 columns in slices of 8 95 -> 58 us, 200 in 32
 // 173 -> 62, 100 in 16 89 -> 40, 128 in 16 with 1024 centroids 280 -> 122; 128 columns in 8 or 32 tie with the pipelined kernel (39,
 // 32 us), which stays for them because it starts faster (300 rows: 7.9 against 8.6 us).
+#include "sq_fused.cuh"
 #include "vq_params.cuh"
 
 namespace f2c {
@@ -227,12 +228,7 @@ __global__ void __launch_bounds__(kThreads, 1) vq_rows_kernel(const VqParams p) 
         }
         __syncwarp();
         if (row < n_dst)
-          for (int c = hl; c < col_end - col_begin; c += 16) {
-            float v = out_s[half * 64 * NCH + c];
-            const int64_t at = (int64_t)row * p.feat_dim + col_begin + c;
-            if (p.drop.enabled) v = dropout_apply1(v, (uint64_t)at, p.drop);
-            __stcs(p.out + at, v);
-          }
+          store_run(p.out, (int64_t)row * p.feat_dim + col_begin, col_end - col_begin, hl, 16, p.drop, [&](int c) { return out_s[half * 64 * NCH + c]; });
       }
     }
     // ---- stage 2: ids have arrived; fetch the code rows

@@ -145,12 +145,12 @@ __device__ __forceinline__ void sq_accumulate(AccT& acc, const VecLoad<VEC>& dat
 // bank-replicated table from those values, 16 bytes per store.
 template <int BITS, int EPL, typename Sync>
 __device__ __forceinline__ void build_sq_table(unsigned char* table, float* values, const float* __restrict__ codebooks, int n_cb,
-                                               int column_slice, int G, int code_kind, int tid, int nthr, Sync sync) {
+                                               int column_slice, int G, int first_col, int code_kind, int tid, int nthr, Sync sync) {
   using L = Lut<BITS>;
   const int n_rows = G < L::COPIES ? G : L::COPIES;
   for (int i = tid; i < n_rows * L::NCODE; i += nthr) {
     int code = i & (L::NCODE - 1), g = i / L::NCODE;
-    int row = (g * EPL) / column_slice;
+    int row = (first_col + g * EPL) / column_slice;
     if (row >= n_cb) row = n_cb - 1;
     float e0 = __ldg(codebooks + row * kCodebookDim + 2), e1 = __ldg(codebooks + row * kCodebookDim + 3);
     float m = __ldg(codebooks + row * kCodebookDim + 4);
@@ -231,35 +231,65 @@ __device__ __forceinline__ void sq_store_rows(const AccT& acc, float4* stage, in
   __syncwarp();
 }
 
-// The same for a column part of rows of any width: sums staged as plain rows, read back so that the lanes of the warp write
-// consecutive columns, four bytes each (a row of the output need not start on a 16-byte boundary).
-//   stage   the warp's area of 32 * EPL floats; a lane's columns are rotated by its number, so that neither the writes (stride
-//           EPL between lanes) nor the reads (stride 1) meet in a bank
+// `count` consecutive floats of the output, from flat index `base` on, written by lanes 0 .. lanes-1 as aligned groups of four:
+// whatever the row width, a lane makes one 16-byte store and one Philox call per group, and single stores only where a group
+// reaches over an end of the run.  value(t) is the run's t-th number.
+template <typename F>
+__device__ __forceinline__ void store_run(float* __restrict__ out, int64_t base, int count, int lane, int lanes, const DropoutArgs& drop, F value) {
+  const bool vec = (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
+  const int head = (int)(base & 3);  // the run starts `head` numbers into its first group
+  const int groups = (head + count + 3) >> 2;
+  for (int g = lane; g < groups; g += lanes) {
+    const int t0 = 4 * g - head;
+    const int64_t at = base - head + 4 * (int64_t)g;
+    float v[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[e] = t0 + e >= 0 && t0 + e < count ? value(t0 + e) : 0.0f;
+    if (drop.enabled) {
+      const float4 d = dropout_apply4(make_float4(v[0], v[1], v[2], v[3]), (uint64_t)at, drop);
+      v[0] = d.x; v[1] = d.y; v[2] = d.z; v[3] = d.w;
+    }
+    if (vec && t0 >= 0 && t0 + 4 <= count) {
+      stg_cs_f4(out + at, make_float4(v[0], v[1], v[2], v[3]));
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (t0 + e >= 0 && t0 + e < count) __stcs(out + at + e, v[e]);
+    }
+  }
+}
+
+// Mean / dropout / store of a column part of rows of any width.
+//   stage   the warp's area of 32 * EPL floats; a lane's columns are rotated so that neither the writes (EPL apart) nor the
+//           reads (4 apart) meet in a bank
+// A part that is the whole row makes one run of the warp's rows, which lie one behind the other.
 template <int EPL, typename AccT>
 __device__ __forceinline__ void sq_store_ragged(const AccT& acc, float* stage, int lane, int logG, int deg, bool have_row, int64_t row_base,
                                                 int64_t n_rows_left, int cols, int col_base, int feat_dim, int reduce, bool div_safe,
                                                 const DropoutArgs& drop, float* __restrict__ out) {
-  const int rows_per_warp = 32 >> logG;
+  const int rows = (int)min((int64_t)(32 >> logG), n_rows_left);
+  auto place = [&](int writer, int e) { return writer * EPL + ((e + ((writer * EPL) >> 5)) & (EPL - 1)); };
   if (have_row) {
+    float rcp = 0.0f;
+    const float degf = (float)deg;
+    if (reduce == F2C_MEAN && deg > 1) rcp = 1.0f / degf;
 #pragma unroll
-    for (int e = 0; e < EPL; ++e) stage[lane * EPL + ((e + lane) & (EPL - 1))] = acc.get(e);
-  }
-  float my_rcp = 0.0f;
-  if (reduce == F2C_MEAN && deg > 1) my_rcp = 1.0f / (float)deg;
-  __syncwarp();
-  for (int row = 0; row < rows_per_warp; ++row) {
-    if (row >= n_rows_left) break;
-    const int64_t dr = row_base + row;
-    const float rcp = __shfl_sync(0xffffffffu, my_rcp, row << logG);
-    const float degf = (float)__shfl_sync(0xffffffffu, deg, row << logG);
-    for (int c = lane; c < cols; c += 32) {
-      const int writer = (row << logG) + c / EPL;
-      float v = stage[writer * EPL + ((c + writer) & (EPL - 1))];
+    for (int e = 0; e < EPL; ++e) {
+      float v = acc.get(e);
       if (rcp != 0.0f) v = div_safe ? div_exact_fast(v, degf, rcp) : div_exact(v, degf, rcp);
-      const int64_t at = dr * feat_dim + col_base + c;
-      if (drop.enabled) v = dropout_apply1(v, (uint64_t)at, drop);
-      __stcs(out + at, v);
+      stage[place(lane, e)] = v;
     }
+  }
+  __syncwarp();
+  if (cols == feat_dim) {
+    const uint32_t magic = 0xffffffffu / (uint32_t)cols + 1u;  // t / cols for t < 32 * 32 (cols = 1: every t is its own row)
+    store_run(out, row_base * feat_dim, rows * cols, lane, 32, drop, [&](int t) {
+      const int r = cols == 1 ? t : (int)__umulhi((uint32_t)t, magic), c = t - r * cols;
+      return stage[place((r << logG) + c / EPL, c & (EPL - 1))];
+    });
+  } else {
+    for (int r = 0; r < rows; ++r)
+      store_run(out, (row_base + r) * feat_dim + col_base, cols, lane, 32, drop, [&](int c) { return stage[place((r << logG) + c / EPL, c & (EPL - 1))]; });
   }
   __syncwarp();
 }

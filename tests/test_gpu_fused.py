@@ -510,7 +510,7 @@ def test_two_level_over_sharded_tables_equals_whole_tables(capi, oracle, hot_bit
 
 
 @pytest.mark.parametrize("bits", [1, 2, 4, 8, 16])
-@pytest.mark.parametrize("D,cs", [(1, 8), (7, 8), (33, 40), (71, 24), (127, 128), (129, 136), (200, 200), (257, 264), (100, 56), (513, 520), (1025, 1032), (300, 8)])
+@pytest.mark.parametrize("D,cs", [(1, 8), (7, 8), (33, 40), (71, 24), (127, 128), (129, 136), (200, 200), (257, 264), (100, 56), (513, 520), (1025, 1032), (300, 8), (110, 32), (368, 368), (64, 8), (200, 104), (255, 128)])
 def test_fused_sq_rows_of_any_length(capi, oracle, bits, D, cs):
     """Rows whose length or start is no multiple of a word, several column parts and slices: same bits as the general kernel,
     also from a table that starts at an odd address (8-bit and packed codes) and with dropout."""
