@@ -2,22 +2,15 @@
 // (reference operator vq_decompress, src/vq_quantization.cu:5-60).
 //
 // A pure gather bound by the fp32 output stream (4 B per element against 1/cs code bytes); the
-// codebooks (<= a few hundred KB) are served by L1/L2 through the read-only path.  Each thread
-// emits one float4 when the slice width and feat_dim are multiples of four.  A code outside
-// [0, length) cannot be told from a valid one by the reference (it reads out of bounds); here it is
-// clamped to the last centroid so that a bad table cannot fault the device.
+// codebooks (a few hundred KB) are read from shared memory or L2.  A code outside [0, length) cannot be told from a valid one
+// by the reference (it reads out of bounds); here it is clamped to the last centroid so that a bad table cannot fault the device.
+#include <algorithm>
 #include <type_traits>
 
+#include "row_lanes.cuh"
 #include "vq_params.cuh"
 
 namespace f2c {
-
-template <typename CodeT>
-__device__ __forceinline__ uint32_t load_code(const void* codes, int64_t pos, uint32_t length) {
-  int v = (int)reinterpret_cast<const CodeT*>(codes)[pos];
-  uint32_t u = (uint32_t)v;
-  return u < length ? u : length - 1;
-}
 
 __device__ __forceinline__ float4 load_cb4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
 __device__ __forceinline__ float4 load_cb4(const __half* p) {
@@ -29,124 +22,124 @@ __device__ __forceinline__ float4 load_cb4(const __half* p) {
 __device__ __forceinline__ float load_cb1(const float* p) { return __ldg(p); }
 __device__ __forceinline__ float load_cb1(const __half* p) { return __half2float(__ldg(p)); }
 
-template <typename CodeT, typename CbT>
-__global__ void __launch_bounds__(256) vq_decompress_vec_kernel(const void* __restrict__ codes, const CbT* __restrict__ cbs,
-                                                                float* __restrict__ out, int64_t n_vec, int vec_per_row,
-                                                                int n_cb, uint32_t length, int cs, int feat_dim) {
-  dependency_wait();
-  release_dependents();
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_vec) return;
-  int64_t row = i / vec_per_row;
-  int j = (int)(i % vec_per_row) * 4;
-  int s = j / cs, off = j - s * cs;
-  uint32_t code = load_code<CodeT>(codes, row * n_cb + s, length);
-  float4 v = load_cb4(cbs + ((int64_t)s * length + code) * cs + off);
-  stg_cs_f4(out + row * feat_dim + j, v);
-}
+// A thread keeps EPT neighbouring columns for its whole life (a CTA holds as many whole rows of columns as fit), so its subspace
+// and its offset in the centroid are found once, the next row is an add away and any row width costs the same; the codes of
+// several rows are in flight per thread, and all their centroid pieces are asked for before the first is stored.
+//   EPT     4 where a centroid is read and a row written in 16-byte pieces, else 1
+//   STAGED  the codebooks of the CTA's columns lie in shared memory instead of L1 and L2.  Where those of a whole row do not fit,
+//           the columns are cut into parts (grid.y) whose codebooks do.  Subspaces narrower than 32 columns (a power of two) are
+//           interleaved inside 128-byte lines: lanes on neighbouring columns read different banks whatever the codes.
+// Row widths that are no multiple of 4 columns took one thread and two 64-bit divisions per element before: 200,000 x 110 of
+// 8-column subspaces 91.3 us, now 23.7; x 357 of 64 columns 279, now 71.  Widths of 4 n columns: 200,000 x 128 of 8 columns
+// 23.5 us, now 18.7; x 200 of 32 41.3, now 27.8.
+constexpr int kVqStagedThreads = 1024;
+constexpr size_t kVqStagedSmem = 200 * 1024;
+constexpr int kVqThreads = 512;
 
-template <typename CodeT, typename CbT>
-__global__ void __launch_bounds__(256) vq_decompress_scalar_kernel(const void* __restrict__ codes, const CbT* __restrict__ cbs,
-                                                                   float* __restrict__ out, int64_t numel, int n_cb,
-                                                                   uint32_t length, int cs, int feat_dim) {
-  dependency_wait();
-  release_dependents();
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= numel) return;
-  int64_t row = i / feat_dim;
-  int j = (int)(i % feat_dim);
-  int s = j / cs, off = j - s * cs;
-  uint32_t code = load_code<CodeT>(codes, row * n_cb + s, length);
-  out[i] = load_cb1(cbs + ((int64_t)s * length + code) * cs + off);
-}
-
-// Streaming variant for the common shapes (uint8 codes, fp32 codebooks that fit in shared memory, vec_per_row
-// dividing the CTA size): the codebooks are staged once per CTA of a persistent grid, a thread keeps one float4
-// column position for its whole life (so its subspace and offset are computed once, and row advance is an add),
-// and eight rows are in flight per thread.  Subspaces narrower than 32 columns are interleaved inside 128-byte
-// lines, so that the eight lanes of a quarter-warp read eight different 16-byte bank groups whatever the codes.
-constexpr int kVqStreamThreads = 1024;
-constexpr size_t kVqStreamSmem = 200 * 1024;
-
-__global__ void __launch_bounds__(kVqStreamThreads, 1) vq_decompress_stream_kernel(
-    const uint8_t* __restrict__ codes, const float* __restrict__ cbs, float* __restrict__ out, int64_t rows, int vec_per_row,
-    int n_cb, int K, int cs, int feat_dim, int spq, int stride) {
+template <typename CodeT, typename CbT, int EPT, bool STAGED>
+__global__ void __launch_bounds__(STAGED ? kVqStagedThreads : kVqThreads, STAGED ? 1 : 3) vq_decompress_kernel(
+    const CodeT* __restrict__ codes, const CbT* __restrict__ cbs, float* __restrict__ out, int64_t rows, int units, int part, int rows_per_cta,
+    int n_cb, int K, int cs, int feat_dim, int sub_per_part, int spq, int stride) {
   dependency_wait();
   release_dependents();
   extern __shared__ __align__(128) unsigned char vq_smem[];
-  stage_codebooks(vq_smem, cbs, n_cb, K, cs, spq, kVqStreamThreads);
-  codebooks_staged();
-  __syncthreads();
-  const int rows_per_cta = kVqStreamThreads / vec_per_row;
-  const int j = (threadIdx.x % vec_per_row) * 4;
+  const int s0 = STAGED ? (int)blockIdx.y * sub_per_part : 0;  // first subspace of the part
+  if constexpr (STAGED) {
+    stage_codebooks(vq_smem, cbs + (int64_t)s0 * K * cs, min(sub_per_part, n_cb - s0), K, cs, spq, (int)blockDim.x);
+    codebooks_staged();
+    __syncthreads();
+  }
+  const int sub = threadIdx.x / part;
+  const int unit = blockIdx.y * part + (threadIdx.x - sub * part);
+  if (sub >= rows_per_cta || unit >= units) return;
+  const int j = unit * EPT;
   const int s = j / cs, off = j - s * cs;
-  const uint32_t lane_base = (uint32_t)__cvta_generic_to_shared(vq_smem) +
-                             (spq > 1 ? (uint32_t)((s / spq) * K * 128 + (s % spq) * cs * 4 + off * 4) : (uint32_t)(s * K * stride + off * 4));
+  const int sl = s - s0;
+  const uint32_t lane_base = STAGED ? (uint32_t)__cvta_generic_to_shared(vq_smem) +
+                                          (spq > 1 ? (uint32_t)((sl / spq) * K * 128 + (sl % spq) * cs * 4 + off * 4) : (uint32_t)(sl * K * stride + off * 4))
+                                    : 0u;
+  const CbT* const cb = cbs + (int64_t)s * K * cs + off;
   const int64_t step = (int64_t)gridDim.x * rows_per_cta;
-  int64_t row = (int64_t)blockIdx.x * rows_per_cta + threadIdx.x / vec_per_row;
-  const uint8_t* cp = codes + row * n_cb + s;
+  int64_t row = (int64_t)blockIdx.x * rows_per_cta + sub;
+  const CodeT* cp = codes + row * n_cb + s;
   float* op = out + row * feat_dim + j;
   const int64_t cstep = step * n_cb, ostep = step * feat_dim;
   const uint32_t kmax = (uint32_t)K - 1u;
-  constexpr int kInFlight = 8;  // rows in flight per thread
-  for (; row + (kInFlight - 1) * step < rows; row += kInFlight * step, cp += kInFlight * cstep, op += kInFlight * ostep) {
+  auto fetch = [&](const CodeT* q) { return min((uint32_t)(int)__ldg(q), kmax); };
+  constexpr int kInFlight = EPT == 4 ? 4 : 8;  // rows in flight per thread: what the registers of three CTAs hold
+  auto value1 = [&](uint32_t c) {
+    float v;
+    if constexpr (STAGED) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(lane_base + c * (uint32_t)stride));
+    else v = load_cb1(cb + (int64_t)c * cs);
+    return v;
+  };
+  auto batch = [&](auto on) {
     uint32_t c[kInFlight];
 #pragma unroll
-    for (int u = 0; u < kInFlight; ++u) c[u] = min((uint32_t)__ldg(cp + u * cstep), kmax);
+    for (int u = 0; u < kInFlight; ++u) c[u] = on(u) ? fetch(cp + u * cstep) : 0u;
+    if constexpr (EPT == 4) {
+      float4 v[kInFlight];
 #pragma unroll
-    for (int u = 0; u < kInFlight; ++u) {
-      float4 v;
-      asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(lane_base + c[u] * (uint32_t)stride));
-      stg_cs_f4(op + u * ostep, v);
+      for (int u = 0; u < kInFlight; ++u) if (on(u)) v[u] = load_cb4(cb + (int64_t)c[u] * cs);
+#pragma unroll
+      for (int u = 0; u < kInFlight; ++u) if (on(u)) stg_cs_f4(op + u * ostep, v[u]);
+    } else {
+      float v[kInFlight];
+#pragma unroll
+      for (int u = 0; u < kInFlight; ++u) if (on(u)) v[u] = value1(c[u]);
+#pragma unroll
+      for (int u = 0; u < kInFlight; ++u) if (on(u)) __stcs(op + u * ostep, v[u]);
     }
-  }
-  for (; row < rows; row += step, cp += cstep, op += ostep) {
-    const uint32_t c = min((uint32_t)__ldg(cp), kmax);
-    float4 v;
-    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(lane_base + c * (uint32_t)stride));
-    stg_cs_f4(op, v);
-  }
+  };
+  for (; row + (kInFlight - 1) * step < rows; row += kInFlight * step, cp += kInFlight * cstep, op += kInFlight * ostep) batch([](int) { return true; });
+  if (row < rows) batch([&](int u) { return row + u * step < rows; });
 }
 
-// Returns true when the streaming kernel was launched.
-static bool try_vq_decompress_stream(const void* codes, const float* cbs, float* out, int64_t rows, int64_t n_cb, int64_t K,
-                                     int64_t cs, int64_t D, cudaStream_t st) {
-  if (K > 256 || cs < 4 || (cs & (cs - 1)) != 0 || D % 4 != 0 || D / 4 > kVqStreamThreads || kVqStreamThreads % (D / 4) != 0) return false;
-  if (!aligned(out, 16) || !aligned(cbs, 16) || rows < 4096) return false;
-  const int spq = cs < 32 ? (int)(32 / cs) : 1;
-  const int stride = cs < 32 ? 128 : (int)cs * 4;
-  const size_t smem = spq > 1 ? (size_t)ceil_div(n_cb, spq) * K * 128 : (size_t)n_cb * K * cs * 4;
-  if (smem > kVqStreamSmem) return false;
-  if (cudaFuncSetAttribute(vq_decompress_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kVqStreamSmem) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return false;
+template <typename CodeT, typename CbT, int EPT>
+static int launch_vq_ept(const CodeT* codes, const CbT* cbs, float* out, int64_t rows, int64_t n_cb, int64_t K, int64_t cs, int64_t D, cudaStream_t st) {
+  const int sms = current_sm_count();
+  const int64_t units = D / EPT;
+  if constexpr (std::is_same<CbT, float>::value && EPT == 1) {
+    // Reads of single floats from narrow centroids spread a warp over many lines of L1, so 8 and 16 columns are staged once there
+    // is work for the copy of up to 200 KB per multiprocessor: 200,000 x 110 of 8 columns 23.7 us against 33.6 from L1, x 375 of
+    // 16 69 against 78, but 27,000 x 110 8.9 against 7.5.  From 32 columns on L1 is as good or better (x 357 of 64: 88 against
+    // 71), and so it is for 16-byte reads of any width.
+    const int64_t used = ceil_div(D, cs);  // subspaces that hold columns
+    const int spq = (cs & (cs - 1)) == 0 && cs < 32 ? (int)(32 / cs) : 1;
+    const int64_t line = spq > 1 ? 128 * K : 4 * K * cs;  // bytes of spq subspaces
+    const int64_t fit = (int64_t)kVqStagedSmem / line * spq;
+    if (fit > 0 && cs < 32 && cs % 4 == 0 && aligned(cbs, 16) && rows * D >= (8 << 20)) {
+      int64_t parts = ceil_div(used, fit);
+      while (parts < used && ceil_div(ceil_div(used, parts), spq) * spq * cs > kVqStagedThreads) ++parts;
+      const int64_t spp = ceil_div(ceil_div(used, parts), spq) * spq;
+      parts = ceil_div(used, spp);
+      const int64_t part = spp < used ? spp * cs : D;
+      if (part <= kVqStagedThreads && parts <= sms) {
+        const Lanes ln = lanes_of_rows(part, rows, sms, kVqStagedThreads);
+        const size_t smem = (size_t)(ceil_div(spp < n_cb ? spp : n_cb, spq) * line);
+        auto kern = vq_decompress_kernel<CodeT, CbT, EPT, true>;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kVqStagedSmem) != cudaSuccess) return check_launch("vq_decompress");
+        const int64_t grid = std::min(ceil_div(rows, ln.rows_per_cta), (int64_t)sms / parts);
+        launch_dependent(kern, dim3((unsigned)grid, (unsigned)parts), ln.threads, smem, st, codes, cbs, out, rows, (int)units, (int)part,
+                         ln.rows_per_cta, (int)n_cb, (int)K, (int)cs, (int)D, (int)spp, spq, spq > 1 ? 128 : (int)cs * 4);
+        return check_launch("vq_decompress");
+      }
+    }
   }
-  const int rows_per_cta = kVqStreamThreads / (int)(D / 4);
-  int64_t grid = ceil_div(rows, rows_per_cta);
-  if (grid > current_sm_count()) grid = current_sm_count();
-  launch_dependent(vq_decompress_stream_kernel, (unsigned)grid, kVqStreamThreads, smem, st, 
-      (const uint8_t*)codes, cbs, out, rows, (int)(D / 4), (int)n_cb, (int)K, (int)cs, (int)D, spq, stride);
-  return true;
+  const Lanes ln = lanes_of_rows(units, rows, sms, kVqThreads);
+  const int64_t grid = std::min(ceil_div(rows, ln.rows_per_cta), ceil_div((int64_t)sms * 3 * kVqThreads / ln.threads, ln.parts));
+  launch_dependent(vq_decompress_kernel<CodeT, CbT, EPT, false>, dim3((unsigned)grid, (unsigned)ln.parts), ln.threads, 0, st, codes, cbs, out, rows,
+                   (int)units, ln.part, ln.rows_per_cta, (int)n_cb, (int)K, (int)cs, (int)D, 0, 1, 0);
+  return check_launch("vq_decompress");
 }
 
 template <typename CodeT, typename CbT>
 static int launch_vq_decompress(const void* codes, const void* cbs, float* out, int64_t rows, int64_t n_cb, int64_t length,
                                 int64_t cs, int64_t D, cudaStream_t st) {
-  int64_t numel = rows * D;
-  if (numel == 0) return F2C_OK;
-  bool vec = cs % 4 == 0 && D % 4 == 0 && aligned(out, 16) && aligned(cbs, 4 * sizeof(CbT));
-  if (sizeof(CodeT) == 1 && !std::is_signed<CodeT>::value && std::is_same<CbT, float>::value &&
-      try_vq_decompress_stream(codes, (const float*)cbs, out, rows, n_cb, length, cs, D, st))
-    return check_launch("vq_decompress");
-  if (vec) {
-    int64_t n_vec = numel / 4;
-    launch_dependent(vq_decompress_vec_kernel<CodeT, CbT>, (unsigned)ceil_div(n_vec, 256), 256, 0, st, 
-        codes, (const CbT*)cbs, out, n_vec, (int)(D / 4), (int)n_cb, (uint32_t)length, (int)cs, (int)D);
-  } else {
-    launch_dependent(vq_decompress_scalar_kernel<CodeT, CbT>, (unsigned)ceil_div(numel, 256), 256, 0, st, 
-        codes, (const CbT*)cbs, out, numel, (int)n_cb, (uint32_t)length, (int)cs, (int)D);
-  }
-  return check_launch("vq_decompress");
+  if (rows * D == 0) return F2C_OK;
+  if (cs % 4 == 0 && D % 4 == 0 && aligned(out, 16) && aligned(cbs, 4 * sizeof(CbT)))
+    return launch_vq_ept<CodeT, CbT, 4>((const CodeT*)codes, (const CbT*)cbs, out, rows, n_cb, length, cs, D, st);
+  return launch_vq_ept<CodeT, CbT, 1>((const CodeT*)codes, (const CbT*)cbs, out, rows, n_cb, length, cs, D, st);
 }
 
 int validate_vq(const char* op, int code_dtype, int64_t n_cb, int64_t length, int64_t cs, int64_t feat_dim) {

@@ -169,6 +169,31 @@ def test_vq_decompress_streaming_kernel(capi, oracle, n_cb, K, cs, D):
 
 
 @pytest.mark.parametrize("bits", [1, 2, 4, 8, 16])
+@pytest.mark.parametrize("rows,D,cs", [(1, 357, 360), (4099, 357, 184), (9001, 101, 104), (5003, 200, 56), (4500, 3, 8), (4097, 1030, 520), (30011, 36, 40)])
+def test_sq_decompress_rows_of_any_width(capi, oracle, bits, rows, D, cs):
+    """Widths that leave threads of a CTA idle, that are cut into column parts, whose codes straddle bytes or slices; one row, a
+    last batch of rows that is not full; codes and output at an odd address."""
+    rng = np.random.default_rng(bits * 7 + D)
+    _, cb, stored = sq_table(oracle, rng, rows, D, bits, cs)
+    got = capi.sq_decompress(dev(stored), dev(cb), bits, cs, D)
+    assert ulp_diff(host(got), oracle.sq_decompress(stored, cb, bits, cs, D)).max() <= SQ_MAX_ULP
+    if rows > 1:
+        assert torch.equal(capi.sq_decompress(dev(stored)[1:], dev(cb), bits, cs, D), got[1:])
+
+
+@pytest.mark.parametrize("code_dtype", [np.uint8, np.int16, np.int8])
+@pytest.mark.parametrize("rows,n_cb,K,cs,D", [(1, 4, 256, 32, 110), (4099, 14, 256, 8, 110), (6007, 6, 256, 64, 357), (5001, 7, 256, 32, 200),
+                                              (4500, 8, 1024, 16, 128), (4097, 33, 256, 32, 1041), (4200, 3, 256, 24, 70), (4300, 5, 60, 5, 23),
+                                              (77001, 14, 256, 8, 110), (23003, 24, 256, 16, 375), (130001, 3, 256, 24, 70), (8500, 130, 100, 8, 1037)])
+def test_vq_decompress_rows_of_any_width(capi, oracle, code_dtype, rows, n_cb, K, cs, D):
+    """Codebooks that fit in shared memory at once, in column parts, or not at all; rows that are no multiple of four columns."""
+    rng = np.random.default_rng(n_cb + K + cs)
+    cbs = rng.standard_normal((n_cb, K, cs)).astype(np.float32)
+    codes = rng.integers(0, min(K, np.iinfo(code_dtype).max + 1), (rows, n_cb)).astype(code_dtype)
+    assert np.array_equal(host(capi.vq_decompress(dev(codes), dev(cbs), D)), oracle.vq_decompress(codes, cbs, D))
+
+
+@pytest.mark.parametrize("bits", [1, 2, 4, 8, 16])
 @pytest.mark.parametrize("D,sq_cs,n_cb,cs", [(128, 128, 4, 32), (128, 32, 16, 8), (256, 256, 4, 64), (110, 110, 2, 60)])
 def test_fusion_decompress_is_concatenation(capi, oracle, bits, D, sq_cs, n_cb, cs):
     # tests/test_fusion_decompress.py:32-43 of the reference
