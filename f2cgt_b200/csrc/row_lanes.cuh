@@ -7,9 +7,9 @@ namespace f2c {
 
 struct Lanes { int parts, part, rows_per_cta, threads; };
 
-// Of the CTA sizes between half of `most` and `most` (multiples of 32; `most` alone when a part needs it), the one with the
-// fewest idle threads: 101 columns fill 505 of 512 threads, 357 columns 357 of 384.
-// Small CTAs that spread over all multiprocessors when the work does not fill them anyway.
+// Of the CTA sizes between half of `most` and `most` (multiples of 32 that hold a part) the one with the fewest idle threads:
+// 101 columns fill 505 of 512 threads, 357 columns 357 of 384.  Work that does not fill the chip is spread over all its
+// multiprocessors in CTAs of 128 threads.
 static inline Lanes lanes_of_rows(int64_t units, int64_t rows, int sms, int most) {
   Lanes l;
   if (rows * units < (int64_t)sms * 3 * 512) most = 128;

@@ -66,7 +66,13 @@ __global__ void __launch_bounds__(STAGED ? kVqStagedThreads : kVqThreads, STAGED
   const int64_t cstep = step * n_cb, ostep = step * feat_dim;
   const uint32_t kmax = (uint32_t)K - 1u;
   auto fetch = [&](const CodeT* q) { return min((uint32_t)(int)__ldg(q), kmax); };
-  constexpr int kInFlight = EPT == 4 ? 4 : 8;  // rows in flight per thread: what the registers of three CTAs hold
+  constexpr int kInFlight = EPT == 4 && !STAGED ? 4 : 8;  // rows in flight per thread: what the registers of three CTAs hold
+  auto value4 = [&](uint32_t c) {
+    float4 v;
+    if constexpr (STAGED) asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(lane_base + c * (uint32_t)stride));
+    else v = load_cb4(cb + (int64_t)c * cs);
+    return v;
+  };
   auto value1 = [&](uint32_t c) {
     float v;
     if constexpr (STAGED) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(lane_base + c * (uint32_t)stride));
@@ -80,7 +86,7 @@ __global__ void __launch_bounds__(STAGED ? kVqStagedThreads : kVqThreads, STAGED
     if constexpr (EPT == 4) {
       float4 v[kInFlight];
 #pragma unroll
-      for (int u = 0; u < kInFlight; ++u) if (on(u)) v[u] = load_cb4(cb + (int64_t)c[u] * cs);
+      for (int u = 0; u < kInFlight; ++u) if (on(u)) v[u] = value4(c[u]);
 #pragma unroll
       for (int u = 0; u < kInFlight; ++u) if (on(u)) stg_cs_f4(op + u * ostep, v[u]);
     } else {
@@ -99,21 +105,23 @@ template <typename CodeT, typename CbT, int EPT>
 static int launch_vq_ept(const CodeT* codes, const CbT* cbs, float* out, int64_t rows, int64_t n_cb, int64_t K, int64_t cs, int64_t D, cudaStream_t st) {
   const int sms = current_sm_count();
   const int64_t units = D / EPT;
-  if constexpr (std::is_same<CbT, float>::value && EPT == 1) {
+  if constexpr (std::is_same<CbT, float>::value) {
     // Reads of single floats from narrow centroids spread a warp over many lines of L1, so 8 and 16 columns are staged once there
     // is work for the copy of up to 200 KB per multiprocessor: 200,000 x 110 of 8 columns 23.7 us against 33.6 from L1, x 375 of
     // 16 69 against 78, but 27,000 x 110 8.9 against 7.5.  From 32 columns on L1 is as good or better (x 357 of 64: 88 against
-    // 71), and so it is for 16-byte reads of any width.
+    // 71), and so it is for 16-byte reads up to some 100 M outputs, beyond which the copy is nothing (400,000 x 128 of 32 columns
+    // 35.0 us staged, 34.6 not; 1,000,003 x 128 86.8 and 90.5).
     const int64_t used = ceil_div(D, cs);  // subspaces that hold columns
     const int spq = (cs & (cs - 1)) == 0 && cs < 32 ? (int)(32 / cs) : 1;
     const int64_t line = spq > 1 ? 128 * K : 4 * K * cs;  // bytes of spq subspaces
     const int64_t fit = (int64_t)kVqStagedSmem / line * spq;
-    if (fit > 0 && cs < 32 && cs % 4 == 0 && aligned(cbs, 16) && rows * D >= (8 << 20)) {
+    const bool worth = EPT == 1 ? cs < 32 && rows * D >= (8 << 20) : used <= fit && rows * D >= (96 << 20);
+    if (fit > 0 && worth && cs % 4 == 0 && aligned(cbs, 16)) {
       int64_t parts = ceil_div(used, fit);
-      while (parts < used && ceil_div(ceil_div(used, parts), spq) * spq * cs > kVqStagedThreads) ++parts;
+      while (parts < used && ceil_div(ceil_div(used, parts), spq) * spq * cs / EPT > kVqStagedThreads) ++parts;
       const int64_t spp = ceil_div(ceil_div(used, parts), spq) * spq;
       parts = ceil_div(used, spp);
-      const int64_t part = spp < used ? spp * cs : D;
+      const int64_t part = spp < used ? spp * cs / EPT : units;
       if (part <= kVqStagedThreads && parts <= sms) {
         const Lanes ln = lanes_of_rows(part, rows, sms, kVqStagedThreads);
         const size_t smem = (size_t)(ceil_div(spp < n_cb ? spp : n_cb, spq) * line);
