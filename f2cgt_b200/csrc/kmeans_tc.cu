@@ -14,12 +14,12 @@
 //    (half the bytes per value), accurate to ~2^-16.
 //  * The whole score comes out of the GEMM.  argmin_c |y_c|^2 - 2 x.y_c = argmax_c (x.y_c - |y_c|^2 / 2): one
 //    more K step carries [1, 1, 0...] on the point side and the split of -|y_c|^2/2 on the centre side
-//    (cosine: the centre rows are pre-scaled by 1/|y_c| instead), so the epilogue is a pure running
-//    arg-max - five instructions per (point, centre) - with no per-centre term to fetch.
-//  * The epilogue reads the 128 x 256 scores with tcgen05.ld (one point per thread) and keeps the best and
-//    second best score.  A point whose two best scores are closer than the error bound of the product is
-//    NOT decided here: its index is appended to a scratch list and the exact fp32 scorer (kmeans.cu)
-//    assigns it afterwards, so every label equals the label of the exact fp32 kernel.
+//    (cosine: the centre rows are pre-scaled by 1/|y_c| instead), so the epilogue is a pure arg-max - one three-operand
+//    max per (point, centre) - with no per-centre term to fetch.
+//  * The epilogue reads the 128 x 256 scores with tcgen05.ld (one point per thread) and finds the best score and whether it is
+//    the only one within the error bound of the product.  A point where it is not is NOT decided here: its index is appended to
+//    a scratch list and the exact fp32 scorer (kmeans.cu) assigns it afterwards, so every label equals the label of the exact
+//    fp32 kernel.
 //  * Overlap.  A CTA is two groups of eight warps that share the staged centre tile; each group has its own
 //    point tile, mbarrier and 256 TMEM columns and runs load -> MMA -> epilogue on alternate tiles, so the
 //    tensor pipe works on one group's tile while the other group is in its epilogue.  A point of the tile
@@ -109,6 +109,13 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
       : "r"(taddr));
 }
 
+// The loads issued so far are complete; naming the registers keeps their uses behind the wait.
+__device__ __forceinline__ void tmem_wait(uint32_t (&r)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]),
+                 "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])::"memory");
+}
+
 struct Params {
   const float* x;
   const float* y;
@@ -140,27 +147,14 @@ __device__ __forceinline__ void split4(const float (&v)[4], float4& hi, float4& 
   hi.w = __uint_as_float(__float_as_uint(v[3]) & 0xFFFFE000u); lo.w = v[3] - hi.w;
 }
 
-// running (best, second best, index of best) over a stream of scores, larger = better
-struct Top2 {
-  float best, second;
-  int idx;
-  __device__ __forceinline__ void init() { best = -INFINITY; second = -INFINITY; idx = 0; }
-  __device__ __forceinline__ void push(float s, int c) {
-    const bool gt = s > best;
-    second = gt ? best : fmaxf(second, s);
-    idx = gt ? c : idx;
-    best = gt ? s : best;
-  }
-  __device__ __forceinline__ void merge(const Top2& o) {
-    const bool gt = o.best > best || (o.best == best && o.idx < idx);
-    second = gt ? fmaxf(best, o.second) : fmaxf(second, o.best);
-    idx = gt ? o.idx : idx;
-    best = gt ? o.best : best;
-  }
-};
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
 
-// Shared memory: [B tile][A tile group 0][A tile group 1][scratch 256 floats][exchange 2 x 128 x 16 B][2 mbarriers]
-// [tmem slot][2 fail flags][2 x 128 floats |x|^2]
+// Shared memory: [B tile][A tile group 0][A tile group 1][scratch 256 floats][exchange 2 x 128 x 8 B][2 mbarriers]
+// [tmem slot][2 fail flags][2 x 2 x 128 floats |x|^2]
 template <bool BF16>
 __global__ void __launch_bounds__(kCtaThreads, 1) kmeans_tc_kernel(const Params p) {
   dependency_wait();
@@ -180,11 +174,11 @@ __global__ void __launch_bounds__(kCtaThreads, 1) kmeans_tc_kernel(const Params 
   unsigned char* b_tile = smem;
   unsigned char* a_tile = smem + (size_t)kc * lbo_b + (size_t)g * kc * lbo_a;
   float* scratch = reinterpret_cast<float*>(smem + (size_t)kc * lbo_b + (size_t)2 * kc * lbo_a);
-  float4* exch = reinterpret_cast<float4*>(scratch + kMaxN) + g * kTileM;  // (best, second, index, |x|^2 part) of half 1
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(scratch + kMaxN + 2 * kTileM * 4);
+  float2* exch = reinterpret_cast<float2*>(scratch + kMaxN) + g * kTileM;  // (best, its centre or -1) of half 1
+  uint64_t* mbar = reinterpret_cast<uint64_t*>(scratch + kMaxN + 2 * kTileM * 2);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mbar + 2);
   volatile uint32_t* fail = tmem_slot + 1;
-  float* xx_s = reinterpret_cast<float*>(mbar + 8) + g * kTileM;  // |x|^2 of the tile's points (bf16 path)
+  float* xx_s = reinterpret_cast<float*>(mbar + 8) + g * 2 * kTileM;  // |x|^2 of the tile's points (tf32: two parts of it)
 
   // ---- one-time setup: TMEM (all 512 columns: 256 per group), mbarriers, centre tile ----
   if (tid < 32) {
@@ -311,8 +305,8 @@ __global__ void __launch_bounds__(kCtaThreads, 1) kmeans_tc_kernel(const Params 
   for (int64_t tile = first; tile < n_tiles; tile += stride) {
     // ---- A tile: the two threads of point tile*128 + pt split and store alternate 16-byte chunks of its row ----
     const int64_t i = tile * kTileM + pt;
-    float xx = 0.0f;
     {
+      float xx = 0.0f;
       const int G = p.dp / 4;
       if (BF16) {
         const int C = p.dp / 8;
@@ -358,6 +352,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) kmeans_tc_kernel(const Params 
           }
         }
       }
+      if (!BF16) xx_s[half * kTileM + pt] = xx;
       // norm-term columns: ones against the pieces of -|y|^2 / 2 (two tf32 ones, or three bf16 ones = 0x3F80 each)
       *reinterpret_cast<uint4*>(a_tile + (size_t)(kc_x + half) * lbo_a + pt * 16) =
           half != 0 ? make_uint4(0u, 0u, 0u, 0u)
@@ -367,7 +362,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) kmeans_tc_kernel(const Params 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     group_sync(g);  // A tile complete; every warp of the group has finished reading the previous tile's accumulators
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (BF16) xx = half == 0 ? xx_s[pt] : 0.0f;  // read before the next tile's split overwrites it (two group syncs away)
+    const float xx = BF16 ? xx_s[pt] : xx_s[pt] + xx_s[kTileM + pt];  // read before the next tile's split overwrites it (two group syncs away)
 
     // ---- S = A' * B'^T into this group's TMEM columns ----
     if (lt == 0) {
@@ -399,55 +394,77 @@ __global__ void __launch_bounds__(kCtaThreads, 1) kmeans_tc_kernel(const Params 
     }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
-    // ---- epilogue: TMEM lane pt = point i; its two threads scan one half of the centres each, with four
-    //      independent trackers over interleaved columns; half 1 hands its result to half 0 through shared memory ----
-    Top2 t0, t1, t2, t3;
-    t0.init(); t1.init(); t2.init(); t3.init();
+    // ---- epilogue: TMEM lane pt = point i; its two threads scan one half of the centres each ----
+    // Maxima only, one three-operand max per score: of the 16-column groups (row_max) and of the columns with the same number in
+    // their group (col_max).  Scores within 2 tol of the best lie in the crossings of the groups and columns whose maximum does,
+    // so the best centre is decided exactly when that is one group and one column - at the crossing.  (A running best, second
+    // best and index took five compare instructions per score, which issue at half rate: 2,449,029 points of 8 columns
+    // against 256 centres 275 us, now @K8@.)
+    const float xn = sqrtf(xx);
+    // error bound of a score: L2  eps*|x||y|max ;  cosine  eps*|x|
+    const float tol2 = 2.0f * (p.metric == F2C_L2 ? p.eps * xn * cmax : p.eps * xn);
     const uint32_t lane_addr = tmem_base + ((uint32_t)(lane_quarter * 32) << 16);
     const int c_split = ((p.n_pad / 32 + 1) / 2) * 32;
     const int c_begin = half == 0 ? 0 : c_split, c_end = half == 0 ? c_split : p.n_pad;
+    constexpr int kGroups = kMaxN / 2 / 16;
+    float row_max[kGroups], col_max[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) col_max[j] = -INFINITY;
     {
       uint32_t ra[16], rb[16];  // two 16-column loads alternate: one is consumed while the other is in flight
-      auto scan = [&](const uint32_t (&r)[16], int c0) {
-#pragma unroll
-        for (int j = 0; j < 16; j += 4) {
-          t0.push(__uint_as_float(r[j]), c0 + j);
-          t1.push(__uint_as_float(r[j + 1]), c0 + j + 1);
-          t2.push(__uint_as_float(r[j + 2]), c0 + j + 2);
-          t3.push(__uint_as_float(r[j + 3]), c0 + j + 3);
-        }
+      auto group_max = [&](const uint32_t (&r)[16]) {
+        auto f = [&](int j) { return __uint_as_float(r[j]); };
+        const float m0 = max3(f(0), f(1), f(2)), m1 = max3(f(3), f(4), f(5)), m2 = max3(f(6), f(7), f(8)), m3 = max3(f(9), f(10), f(11));
+        const float m4 = max3(f(12), f(13), f(14));
+        return fmaxf(max3(m0, m1, m2), max3(m3, m4, f(15)));
       };
       if (c_begin < c_end) tmem_ld16(lane_addr + (uint32_t)c_begin, ra);
-      for (int c0 = c_begin; c0 < c_end; c0 += 32) {  // c_end - c_begin is a multiple of 32
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        tmem_ld16(lane_addr + (uint32_t)(c0 + 16), rb);
-        scan(ra, c0);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (c0 + 32 < c_end) tmem_ld16(lane_addr + (uint32_t)(c0 + 32), ra);
-        scan(rb, c0 + 16);
+#pragma unroll
+      for (int q = 0; q < kGroups; q += 2) {  // c_end - c_begin is a multiple of 32
+        const int c0 = c_begin + 16 * q;
+        row_max[q] = -INFINITY;
+        row_max[q + 1] = -INFINITY;
+        if (c0 < c_end) {
+          tmem_wait(ra);
+          tmem_ld16(lane_addr + (uint32_t)(c0 + 16), rb);
+          row_max[q] = group_max(ra);
+          float own[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) own[j] = __uint_as_float(ra[j]);
+          tmem_wait(rb);
+          if (c0 + 32 < c_end) tmem_ld16(lane_addr + (uint32_t)(c0 + 32), ra);
+          row_max[q + 1] = group_max(rb);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) col_max[j] = max3(col_max[j], own[j], __uint_as_float(rb[j]));
+        }
       }
     }
-    t0.merge(t1); t2.merge(t3); t0.merge(t2);
-    if (half == 1) exch[pt] = make_float4(t0.best, t0.second, __int_as_float(t0.idx), xx);
+    static_assert(kGroups == 8, "the tree below");
+    float best = max3(max3(row_max[0], row_max[1], row_max[2]), max3(row_max[3], row_max[4], row_max[5]), fmaxf(row_max[6], row_max[7]));
+    // hits, each counted as 64 + its number: below 128 there was one
+    const float from = best - tol2;
+    int rows_hit = 0, cols_hit = 0;
+#pragma unroll
+    for (int q = 0; q < kGroups; ++q) rows_hit += row_max[q] >= from ? 64 + q : 0;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) cols_hit += col_max[j] >= from ? 64 + j : 0;
+    int centre = rows_hit < 128 && cols_hit < 128 ? c_begin + 16 * (rows_hit - 64) + cols_hit - 64 : -1;
+    if (half == 1) exch[pt] = make_float2(best, __int_as_float(centre));
     group_sync(g);
     if (half == 1) continue;
     {
-      const float4 o = exch[pt];
-      Top2 other;
-      other.best = o.x; other.second = o.y; other.idx = __float_as_int(o.z);
-      t0.merge(other);
-      xx += o.w;
+      const float2 o = exch[pt];
+      const bool mine = best - tol2 > o.x, other = o.x - tol2 > best;
+      centre = mine ? centre : (other ? __float_as_int(o.y) : -1);
+      best = fmaxf(best, o.x);
     }
-    const float xn = sqrtf(xx);
-    // error bound of a score: L2  eps*|x||y|max ;  cosine  eps*|x|
-    const float tol = p.metric == F2C_L2 ? p.eps * xn * cmax : p.eps * xn;
-    const bool odd = bad_centres || !(xx < INFINITY) || !(t0.best > -INFINITY);  // NaN / inf somewhere: exact scorer
+    const bool odd = bad_centres || !(xx < INFINITY) || !(best > -INFINITY);  // NaN / inf somewhere: exact scorer
     if (i < p.n) {
-      if (odd || !(t0.best - t0.second > 2.0f * tol)) {  // undecided: the exact scorer assigns it afterwards
+      if (odd || centre < 0) {  // undecided: the exact scorer assigns it afterwards
         const int slot = atomicAdd(p.amb_count, 1);
         p.amb_list[slot] = (int32_t)i;
       } else {
-        p.labels[i] = t0.idx;
+        p.labels[i] = centre;
       }
     }
   }
@@ -486,7 +503,7 @@ int kmeans_assign_tc(const float* x, const float* y, int64_t* labels, int64_t n,
   cudaError_t e = cudaMemsetAsync(head, 0, 256, st);
   if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "kmeans_assign: %s", cudaGetErrorString(e));
   const int kc = (p.bf16 ? 3 * p.dp / 8 : p.terms * p.dp / 4) + 2;
-  size_t smem = (size_t)kc * (tc::kMaxN + 2 * tc::kTileM) * 16 + tc::kMaxN * 4 + 2 * tc::kTileM * 16 + 64 + 2 * tc::kTileM * 4;
+  size_t smem = (size_t)kc * (tc::kMaxN + 2 * tc::kTileM) * 16 + tc::kMaxN * 4 + 2 * tc::kTileM * 8 + 64 + 4 * tc::kTileM * 4;
   if (smem < 120 * 1024) smem = 120 * 1024;  // one CTA per SM: a second one would only wait for the TMEM columns
   auto kern = p.bf16 ? tc::kmeans_tc_kernel<true> : tc::kmeans_tc_kernel<false>;
   e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
