@@ -147,13 +147,14 @@ constexpr int kShortRounds = 32;
 template <int DMAX, int METRIC>
 __global__ void __launch_bounds__(kListThreads) kmeans_listed_kernel(const float* __restrict__ x, const float* __restrict__ y,
                                                                      int64_t* __restrict__ labels, const int32_t* __restrict__ list,
-                                                                     const int32_t* __restrict__ count_dev, int64_t max_count, int k, int d,
-                                                                     int kc) {
+                                                                     const int32_t* __restrict__ count_dev, const int32_t* __restrict__ all_dev,
+                                                                     int64_t max_count, int k, int d, int kc, int y_vec4) {
   dependency_wait();
   release_dependents();
   constexpr int STRIDE = DMAX + 4;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int64_t cnt = *count_dev < max_count ? *count_dev : max_count;
+  const bool all = all_dev != nullptr && *all_dev != 0;  // every point instead of the listed ones
+  const int64_t cnt = !all && *count_dev < max_count ? *count_dev : max_count;
   const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * kListThreads + threadIdx.x) >> 5, n_warps = ((int64_t)gridDim.x * kListThreads) >> 5;
   const bool by_warp = cnt <= n_warps * kShortRounds && kc >= k;
@@ -161,9 +162,20 @@ __global__ void __launch_bounds__(kListThreads) kmeans_listed_kernel(const float
   float* yc_s = reinterpret_cast<float*>(smem_raw);  // [kc][STRIDE]
   float* cc_s = yc_s + (size_t)kc * STRIDE;          // [kc]
   auto stage = [&](int c0, int nc) {
-    for (int e = threadIdx.x; e < nc * DMAX; e += kListThreads) {
-      const int c = e / DMAX, t = e - c * DMAX;
-      yc_s[c * STRIDE + t] = t < d ? __ldg(y + (int64_t)(c0 + c) * d + t) : 0.0f;
+    if (y_vec4) {  // d % 4 == 0; eight 16-byte loads in flight per thread (single floats: 15 us for 256 x 64, now @L64@)
+#pragma unroll 8
+      for (int e = threadIdx.x; e < nc * (DMAX / 4); e += kListThreads) {
+        const int c = e / (DMAX / 4), t = 4 * (e - c * (DMAX / 4));
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (t < d) v = __ldg(reinterpret_cast<const float4*>(y + (int64_t)(c0 + c) * d + t));
+        *reinterpret_cast<float4*>(yc_s + c * STRIDE + t) = v;
+      }
+    } else {
+#pragma unroll 8
+      for (int e = threadIdx.x; e < nc * DMAX; e += kListThreads) {
+        const int c = e / DMAX, t = e - c * DMAX;
+        yc_s[c * STRIDE + t] = t < d ? __ldg(y + (int64_t)(c0 + c) * d + t) : 0.0f;
+      }
     }
     __syncthreads();
     if (METRIC == F2C_COSINE) {
@@ -206,7 +218,7 @@ __global__ void __launch_bounds__(kListThreads) kmeans_listed_kernel(const float
   if (by_warp) {
     stage(0, k);
     for (int64_t s = warp; s < cnt; s += n_warps) {
-      const int64_t i = list[s];
+      const int64_t i = all ? s : (int64_t)list[s];
       load_point(i);
       float best = INFINITY;
       int best_c = 0x7fffffff;
@@ -226,7 +238,7 @@ __global__ void __launch_bounds__(kListThreads) kmeans_listed_kernel(const float
   }
   for (int64_t base = (int64_t)blockIdx.x * kListThreads; base < cnt; base += (int64_t)gridDim.x * kListThreads) {
     const int64_t s = base + threadIdx.x;
-    const int64_t i = s < cnt ? (int64_t)list[s] : -1;
+    const int64_t i = s < cnt ? (all ? s : (int64_t)list[s]) : -1;
     load_point(i);
     float best = INFINITY;
     int best_c = 0;
@@ -244,8 +256,8 @@ __global__ void __launch_bounds__(kListThreads) kmeans_listed_kernel(const float
 }
 
 template <int DMAX>
-static int launch_listed(const float* x, const float* y, int64_t* labels, const int32_t* list, const int32_t* count_dev, int64_t max_count,
-                         int64_t k, int64_t d, int metric, cudaStream_t st) {
+static int launch_listed(const float* x, const float* y, int64_t* labels, const int32_t* list, const int32_t* count_dev, const int32_t* all_dev,
+                         int64_t max_count, int64_t k, int64_t d, int metric, cudaStream_t st) {
   int kc = (int)k;
   while ((size_t)kc * (DMAX + 5) * sizeof(float) > 96 * 1024) kc = (kc + 1) / 2;
   const size_t smem = (size_t)kc * (DMAX + 5) * sizeof(float);
@@ -254,7 +266,8 @@ static int launch_listed(const float* x, const float* y, int64_t* labels, const 
   if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "kmeans_assign: %s", cudaGetErrorString(e));
   int64_t grid = ceil_div(max_count, kListThreads / 32);
   if (grid > 2 * current_sm_count()) grid = 2 * current_sm_count();
-  launch_dependent(kern, (unsigned)grid, kListThreads, smem, st, x, y, labels, list, count_dev, max_count, (int)k, (int)d, kc);
+  launch_dependent(kern, (unsigned)grid, kListThreads, smem, st, x, y, labels, list, count_dev, all_dev, max_count, (int)k, (int)d, kc,
+                   d % 4 == 0 && aligned(y, 16) ? 1 : 0);
   return check_launch("kmeans_assign");
 }
 
@@ -299,14 +312,15 @@ int kmeans_assign_exact(const float* x, const float* y, int64_t* labels, const i
   return check_launch("kmeans_assign");
 }
 
-// Exact assignment of the points listed in `list`; their number sits in device memory (*count_dev <= max_count).
+// Exact assignment of the points listed in `list`; their number sits in device memory (*count_dev <= max_count).  Of all
+// max_count points instead when all_dev is set and *all_dev is not 0.
 int kmeans_assign_exact_listed(const float* x, const float* y, int64_t* labels, const int32_t* list, const int32_t* count_dev,
-                               int64_t max_count, int64_t k, int64_t d, int metric, cudaStream_t st) {
+                               const int32_t* all_dev, int64_t max_count, int64_t k, int64_t d, int metric, cudaStream_t st) {
   if (max_count == 0) return F2C_OK;
-  if (d <= 8) return launch_listed<8>(x, y, labels, list, count_dev, max_count, k, d, metric, st);
-  if (d <= 16) return launch_listed<16>(x, y, labels, list, count_dev, max_count, k, d, metric, st);
-  if (d <= 32) return launch_listed<32>(x, y, labels, list, count_dev, max_count, k, d, metric, st);
-  if (d <= 64) return launch_listed<64>(x, y, labels, list, count_dev, max_count, k, d, metric, st);
+  if (d <= 8) return launch_listed<8>(x, y, labels, list, count_dev, all_dev, max_count, k, d, metric, st);
+  if (d <= 16) return launch_listed<16>(x, y, labels, list, count_dev, all_dev, max_count, k, d, metric, st);
+  if (d <= 32) return launch_listed<32>(x, y, labels, list, count_dev, all_dev, max_count, k, d, metric, st);
+  if (d <= 64) return launch_listed<64>(x, y, labels, list, count_dev, all_dev, max_count, k, d, metric, st);
   return set_error(F2C_ERR_UNSUPPORTED, "kmeans_assign: listed re-scoring needs d <= 64");
 }
 
@@ -355,10 +369,10 @@ extern "C" int f2c_kmeans_assign(const float* x, const float* centers, int64_t* 
   if (rc) return rc;
   if (n == 0) return F2C_OK;
   F2C_REQUIRE(x && centers && labels, F2C_ERR_INVALID, "kmeans_assign: null pointer");
-  // tensor-core path when a scratch buffer is supplied and the shape fits; the exact fp32 scorer otherwise
-  // (measured on B200 with 256 centres: the tensor-core path is faster from d = 8 up for both metrics; below that
-  //  the CUDA-core scorer reads so little per point that the 128-point tiles only add latency)
-  const bool prefer_tc = d >= 8 || scorer == F2C_SCORER_TENSOR;
+  // tensor-core path when a scratch buffer is supplied and the shape fits; the exact fp32 scorer otherwise, and below four
+  // dimensions, where many points' best two centres are too close for the split product (2,449,029 x 4 against 256 centres:
+  // exact scorer 982 us, tensor cores @K4@)
+  const bool prefer_tc = d >= 4 || scorer == F2C_SCORER_TENSOR;
   if (workspace != nullptr && kmeans_tc_supported(n, k, d) && prefer_tc && scorer != F2C_SCORER_EXACT && aligned(workspace, 16))
     return kmeans_assign_tc(x, centers, labels, n, k, d, metric, workspace, (cudaStream_t)stream, nullptr);
   return kmeans_assign_exact(x, centers, labels, nullptr, n, k, d, metric, (cudaStream_t)stream, nullptr);

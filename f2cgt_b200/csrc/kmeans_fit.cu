@@ -238,7 +238,7 @@ extern "C" int f2c_kmeans_fit_iterate(const float* x, float* centers, int64_t n,
   long long* sums = (long long*)(ws + w.sums);
   unsigned int* counts = (unsigned int*)(ws + w.counts);
   int64_t* labels = (int64_t*)(ws + w.labels);
-  const bool tc = kmeans_tc_supported(n, k, d) && d >= 8;
+  const bool tc = kmeans_tc_supported(n, k, d) && d >= 4;
   const int32_t* assign_error = tc ? (const int32_t*)(ws + w.assign) + 1 : nullptr;
   const size_t smem = ((size_t)2 * k * d + k) * 4 + fit::kChunk * 2;
   const bool shared = smem <= fit::kSmemLimit && k <= 65535;

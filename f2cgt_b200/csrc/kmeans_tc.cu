@@ -26,8 +26,8 @@
 //    belongs to two threads of its group (same TMEM lane, warps w and w + 4): they load and split alternate
 //    chunks of its row and scan one half of the centres each - the epilogue, not the MMA, is what the kernel
 //    spends its issue slots on, and twice the warps fill them better.  The group's first thread issues the
-//    MMAs.  Every wait on an MMA-completion mbarrier is bounded; on expiry the group records an error code
-//    and leaves, and the CTA frees its TMEM at the common exit.
+//    MMAs.  Every wait on an MMA-completion mbarrier is bounded; on expiry an error code is recorded, which makes the exact
+//    scorer assign every point, no further wait is made, and the CTA frees its TMEM at the common exit.
 #include <mutex>
 
 #include <cuda_bf16.h>
@@ -37,7 +37,7 @@
 namespace f2c {
 
 int kmeans_assign_exact_listed(const float* x, const float* y, int64_t* labels, const int32_t* list, const int32_t* count_dev,
-                               int64_t max_count, int64_t k, int64_t d, int metric, cudaStream_t st);
+                               const int32_t* all_dev, int64_t max_count, int64_t k, int64_t d, int metric, cudaStream_t st);
 
 namespace tc {
 
@@ -90,17 +90,6 @@ __device__ __forceinline__ void split8_bf16(const float (&v)[8], uint4& c1, uint
   c2 = make_uint4(w2[0], w2[1], w2[2], w2[3]);
 }
 
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
-        "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
-        "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
-}
-
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
@@ -126,11 +115,11 @@ struct Params {
   int64_t n;
   int k, d;
   int dp;      // d padded to a multiple of 8
-  int terms;   // 3: split product, 1: plain TF32
   int bf16;    // 1: operands are bf16 pairs (x = b1 + b2), A' = [x1 | x2 | x1], B' = [y1 | y1 | y2], kind::f16 (32 < d <= 64)
   int n_pad;   // k padded to a multiple of 32 (epilogue reads 32 columns at a time; MMA N needs 16)
   int metric;
   int vec4;    // rows of x can be read as float4
+  int y_vec4;  // and rows of y
   float eps;   // relative error bound of one score
   const int32_t* done;  // when set and non-zero: nothing to do (a fit that has converged, kmeans_fit.cu)
 };
@@ -153,8 +142,8 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   return r;
 }
 
-// Shared memory: [B tile][A tile group 0][A tile group 1][scratch 256 floats][exchange 2 x 128 x 8 B][2 mbarriers]
-// [tmem slot][2 fail flags][2 x 2 x 128 floats |x|^2]
+// Shared memory: [B tile][A tile group 0][A tile group 1][scratch 256 floats][exchange 2 x 2 x 128 x 8 B][2 mbarriers]
+// [tmem slot][2 x 2 x 2 x 128 floats |x|^2]
 template <bool BF16>
 __global__ void __launch_bounds__(kCtaThreads, 1) kmeans_tc_kernel(const Params p) {
   dependency_wait();
@@ -168,17 +157,16 @@ __global__ void __launch_bounds__(kCtaThreads, 1) kmeans_tc_kernel(const Params 
   const int half = lt >> 7;          // which half of the row's K chunks it loads and which half of the centres it scans
   const int lane_quarter = (lt >> 5) & 3;
   // 16-byte K chunks per operand row (the last two carry the norm term): 4 tf32 or 8 bf16 values per chunk
-  const int kc_x = BF16 ? 3 * p.dp / 8 : p.terms * p.dp / 4;
+  const int kc_x = BF16 ? 3 * p.dp / 8 : 3 * p.dp / 4;
   const int kc = kc_x + 2;
   const uint32_t lbo_b = kMaxN * 16, lbo_a = kTileM * 16, sbo = 128;
   unsigned char* b_tile = smem;
   unsigned char* a_tile = smem + (size_t)kc * lbo_b + (size_t)g * kc * lbo_a;
   float* scratch = reinterpret_cast<float*>(smem + (size_t)kc * lbo_b + (size_t)2 * kc * lbo_a);
-  float2* exch = reinterpret_cast<float2*>(scratch + kMaxN) + g * kTileM;  // (best, its centre or -1) of half 1
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(scratch + kMaxN + 2 * kTileM * 2);
+  float2* exch = reinterpret_cast<float2*>(scratch + kMaxN) + g * 2 * kTileM;  // (best, its centre or -1) of half 1, for two tiles
+  uint64_t* mbar = reinterpret_cast<uint64_t*>(scratch + kMaxN + 4 * kTileM * 2);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mbar + 2);
-  volatile uint32_t* fail = tmem_slot + 1;
-  float* xx_s = reinterpret_cast<float*>(mbar + 8) + g * 2 * kTileM;  // |x|^2 of the tile's points (tf32: two parts of it)
+  float* xx_all = reinterpret_cast<float*>(mbar + 8) + g * 4 * kTileM;  // |x|^2 of the points (tf32: two parts of it) of two tiles
 
   // ---- one-time setup: TMEM (all 512 columns: 256 per group), mbarriers, centre tile ----
   if (tid < 32) {
@@ -189,48 +177,68 @@ __global__ void __launch_bounds__(kCtaThreads, 1) kmeans_tc_kernel(const Params 
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(mbar)) : "memory");
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(mbar + 1)) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    fail[0] = 0u; fail[1] = 0u;
   }
   // centre c = tid (first 256 threads, 256 rows); padded rows are zero with a norm term that never wins
   if (tid < kMaxN) {
     const int c = tid;
     const int G = p.dp / 4;
+    // sixteen numbers of the row at a time, their loads in flight together (one at a time: 30 us for 256 x 64, whatever n)
+    auto row16 = [&](int t0, float (&v)[16]) {
+      const float* yc = p.y + (int64_t)c * p.d;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int t = t0 + 4 * q;
+        float4 w = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (c < p.k && p.y_vec4) {
+          if (t < p.d) w = __ldg(reinterpret_cast<const float4*>(yc + t));
+        } else if (c < p.k) {
+          if (t < p.d) w.x = __ldg(yc + t);
+          if (t + 1 < p.d) w.y = __ldg(yc + t + 1);
+          if (t + 2 < p.d) w.z = __ldg(yc + t + 2);
+          if (t + 3 < p.d) w.w = __ldg(yc + t + 3);
+        }
+        v[4 * q] = w.x; v[4 * q + 1] = w.y; v[4 * q + 2] = w.z; v[4 * q + 3] = w.w;
+      }
+    };
     float nrm = 0.0f;
-    if (c < p.k)
-      for (int t = 0; t < p.d; ++t) { const float v = __ldg(p.y + (int64_t)c * p.d + t); nrm = fmaf(v, v, nrm); }
+    for (int t0 = 0; t0 < p.d; t0 += 16) {
+      float v[16];
+      row16(t0, v);
+#pragma unroll
+      for (int e = 0; e < 16; ++e) nrm = fmaf(v[e], v[e], nrm);
+    }
     // cosine: rows are scaled to unit length (zero rows stay zero); L2: rows as they are
     const float row_scale = p.metric == F2C_COSINE ? (nrm > 0.0f ? 1.0f / sqrtf(nrm) : 0.0f) : 1.0f;
-    if (BF16) {
-      const int C = p.dp / 8;
-      for (int cq = 0; cq < C; ++cq) {
-        float v[8];
+    for (int t0 = 0; t0 < p.dp; t0 += 16) {
+      float v[16];
+      row16(t0, v);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const int t = 8 * cq + e;
-          v[e] = (c < p.k && t < p.d) ? __ldg(p.y + (int64_t)c * p.d + t) * row_scale : 0.0f;
+      for (int e = 0; e < 16; ++e) v[e] *= row_scale;
+      if constexpr (BF16) {
+        const int C = p.dp / 8;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int cq = t0 / 8 + h;
+          const float w[8] = {v[8 * h], v[8 * h + 1], v[8 * h + 2], v[8 * h + 3], v[8 * h + 4], v[8 * h + 5], v[8 * h + 6], v[8 * h + 7]};
+          uint4 c1, c2;
+          split8_bf16(w, c1, c2);  // B' = [y1 | y1 | y2]; dp is a multiple of 16
+          *reinterpret_cast<uint4*>(b_tile + (size_t)(cq) * lbo_b + c * 16) = c1;
+          *reinterpret_cast<uint4*>(b_tile + (size_t)(C + cq) * lbo_b + c * 16) = c1;
+          *reinterpret_cast<uint4*>(b_tile + (size_t)(2 * C + cq) * lbo_b + c * 16) = c2;
         }
-        uint4 c1, c2;
-        split8_bf16(v, c1, c2);  // B' = [y1 | y1 | y2]
-        *reinterpret_cast<uint4*>(b_tile + (size_t)(cq) * lbo_b + c * 16) = c1;
-        *reinterpret_cast<uint4*>(b_tile + (size_t)(C + cq) * lbo_b + c * 16) = c1;
-        *reinterpret_cast<uint4*>(b_tile + (size_t)(2 * C + cq) * lbo_b + c * 16) = c2;
-      }
-    }
-    for (int gq = 0; gq < (BF16 ? 0 : G); ++gq) {
-      float v[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int t = 4 * gq + e;
-        v[e] = (c < p.k && t < p.d) ? __ldg(p.y + (int64_t)c * p.d + t) * row_scale : 0.0f;
-      }
-      float4 hi, lo;
-      split4(v, hi, lo);
-      if (p.terms == 3) {  // B' = [y_hi | y_hi | y_lo]
-        *reinterpret_cast<float4*>(b_tile + (size_t)(gq) * lbo_b + c * 16) = hi;
-        *reinterpret_cast<float4*>(b_tile + (size_t)(G + gq) * lbo_b + c * 16) = hi;
-        *reinterpret_cast<float4*>(b_tile + (size_t)(2 * G + gq) * lbo_b + c * 16) = lo;
       } else {
-        *reinterpret_cast<float4*>(b_tile + (size_t)gq * lbo_b + c * 16) = make_float4(v[0], v[1], v[2], v[3]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int gq = t0 / 4 + q;
+          if (gq < G) {
+            const float w[4] = {v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]};
+            float4 hi, lo;
+            split4(w, hi, lo);  // B' = [y_hi | y_hi | y_lo]
+            *reinterpret_cast<float4*>(b_tile + (size_t)(gq) * lbo_b + c * 16) = hi;
+            *reinterpret_cast<float4*>(b_tile + (size_t)(G + gq) * lbo_b + c * 16) = hi;
+            *reinterpret_cast<float4*>(b_tile + (size_t)(2 * G + gq) * lbo_b + c * 16) = lo;
+          }
+        }
       }
     }
     // norm term: -|y_c|^2 / 2 split in two TF32 values (L2), 0 (cosine), a value that never wins (padding)
@@ -269,8 +277,8 @@ __global__ void __launch_bounds__(kCtaThreads, 1) kmeans_tc_kernel(const Params 
   const int64_t n_tiles = (p.n + kTileM - 1) / kTileM;
   const int64_t first = (int64_t)blockIdx.x * 2 + g, stride = (int64_t)gridDim.x * 2;
   // This thread's chunks of its point's row, fetched one tile ahead so that the global-load latency hides behind the
-  // previous tile's MMA and epilogue: chunk q of the thread is 16-byte chunk half + 2q of the row (at most 8: d <= 64).
-  constexpr int kMaxChunks = 8;
+  // previous tile's MMA and epilogue: chunk q of the thread is 16-byte chunk half + 2q of the row (tf32: d <= 32).
+  constexpr int kMaxChunks = BF16 ? 8 : 4;
   float4 xv[kMaxChunks];
   // bf16 path (rows of 132 to 256 bytes): the tile's rows are fetched and split by a different thread mapping than the
   // one of the epilogue, so that a warp-wide load covers 8 rows x 128 contiguous bytes instead of 32 rows x 16 bytes
@@ -301,12 +309,35 @@ __global__ void __launch_bounds__(kCtaThreads, 1) kmeans_tc_kernel(const Params 
       }
     }
   };
+  // One barrier of the group per tile: it completes the A tile, ends the reading of the previous tile's accumulators and hands
+  // half 1's result for that tile to half 0, which writes the labels while the next MMAs run.  What crosses it is kept for two
+  // tiles in turn.
+  bool gave_up = false;  // a wait ran out: the error word makes the exact scorer assign every point, so just leave the loop's rhythm intact
+  float best = 0.0f, tol2 = 0.0f, xx = 0.0f;
+  int centre = -1;
+  int64_t i = -1;  // this thread's point of the tile before
+  int turn = 0;
+  auto finish = [&](int t) {  // half 0: labels of the tile before
+    const float2 o = exch[t * kTileM + pt];
+    const bool mine = best - tol2 > o.x, other = o.x - tol2 > best;
+    const int c = mine ? centre : (other ? __float_as_int(o.y) : -1);
+    const bool odd = bad_centres || !(xx < INFINITY) || !(fmaxf(best, o.x) > -INFINITY);  // NaN / inf somewhere: exact scorer
+    const bool mine_to_write = i >= 0 && i < p.n, undecided = mine_to_write && (odd || c < 0);
+    const uint32_t listed = __ballot_sync(0xffffffffu, undecided);  // the exact scorer assigns them afterwards
+    if (listed != 0u) {
+      int slot = 0;
+      if ((threadIdx.x & 31) == 0) slot = atomicAdd(p.amb_count, __popc(listed));
+      slot = __shfl_sync(0xffffffffu, slot, 0);
+      if (undecided) p.amb_list[slot + __popc(listed & ((1u << (threadIdx.x & 31)) - 1u))] = (int32_t)i;
+    }
+    if (mine_to_write && !undecided) p.labels[i] = c;
+  };
   fetch_row(first);
-  for (int64_t tile = first; tile < n_tiles; tile += stride) {
+  for (int64_t tile = first; tile < n_tiles; tile += stride, turn ^= 1) {
+    float* xx_s = xx_all + turn * 2 * kTileM;
     // ---- A tile: the two threads of point tile*128 + pt split and store alternate 16-byte chunks of its row ----
-    const int64_t i = tile * kTileM + pt;
     {
-      float xx = 0.0f;
+      float sum = 0.0f;
       const int G = p.dp / 4;
       if (BF16) {
         const int C = p.dp / 8;
@@ -340,19 +371,16 @@ __global__ void __launch_bounds__(kCtaThreads, 1) kmeans_tc_kernel(const Params 
         const int gq = half + 2 * q;
         if (gq < G) {
           const float v[4] = {xv[q].x, xv[q].y, xv[q].z, xv[q].w};
-          xx = fmaf(v[0], v[0], xx); xx = fmaf(v[1], v[1], xx); xx = fmaf(v[2], v[2], xx); xx = fmaf(v[3], v[3], xx);
+          sum = fmaf(v[0], v[0], sum); sum = fmaf(v[1], v[1], sum); sum = fmaf(v[2], v[2], sum); sum = fmaf(v[3], v[3], sum);
           float4 hi, lo;
           split4(v, hi, lo);
-          if (p.terms == 3) {  // A' = [x_hi | x_lo | x_hi]
-            *reinterpret_cast<float4*>(a_tile + (size_t)(gq) * lbo_a + pt * 16) = hi;
-            *reinterpret_cast<float4*>(a_tile + (size_t)(G + gq) * lbo_a + pt * 16) = lo;
-            *reinterpret_cast<float4*>(a_tile + (size_t)(2 * G + gq) * lbo_a + pt * 16) = hi;
-          } else {
-            *reinterpret_cast<float4*>(a_tile + (size_t)gq * lbo_a + pt * 16) = xv[q];
-          }
+          // A' = [x_hi | x_lo | x_hi]
+          *reinterpret_cast<float4*>(a_tile + (size_t)(gq) * lbo_a + pt * 16) = hi;
+          *reinterpret_cast<float4*>(a_tile + (size_t)(G + gq) * lbo_a + pt * 16) = lo;
+          *reinterpret_cast<float4*>(a_tile + (size_t)(2 * G + gq) * lbo_a + pt * 16) = hi;
         }
       }
-      if (!BF16) xx_s[half * kTileM + pt] = xx;
+      if (!BF16) xx_s[half * kTileM + pt] = sum;
       // norm-term columns: ones against the pieces of -|y|^2 / 2 (two tf32 ones, or three bf16 ones = 0x3F80 each)
       *reinterpret_cast<uint4*>(a_tile + (size_t)(kc_x + half) * lbo_a + pt * 16) =
           half != 0 ? make_uint4(0u, 0u, 0u, 0u)
@@ -360,9 +388,8 @@ __global__ void __launch_bounds__(kCtaThreads, 1) kmeans_tc_kernel(const Params 
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    group_sync(g);  // A tile complete; every warp of the group has finished reading the previous tile's accumulators
+    group_sync(g);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const float xx = BF16 ? xx_s[pt] : xx_s[pt] + xx_s[kTileM + pt];  // read before the next tile's split overwrites it (two group syncs away)
 
     // ---- S = A' * B'^T into this group's TMEM columns ----
     if (lt == 0) {
@@ -376,9 +403,12 @@ __global__ void __launch_bounds__(kCtaThreads, 1) kmeans_tc_kernel(const Params 
       asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar_addr) : "memory");
     }
     fetch_row(tile + stride);  // next tile's row, in flight during this tile's MMA and epilogue
+    if (half == 0) finish(turn ^ 1);
+    i = tile * kTileM + pt;
+    xx = BF16 ? xx_s[pt] : xx_s[pt] + xx_s[kTileM + pt];
     // ---- bounded wait for the MMAs ----
     uint32_t done = 0;
-    for (uint32_t it = 0; it < kWaitLimit && !done; ++it) {
+    for (uint32_t it = 0; it < kWaitLimit && !done && !gave_up; ++it) {
       asm volatile(
           "{\n\t.reg .pred p;\n\t"
           "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
@@ -386,12 +416,11 @@ __global__ void __launch_bounds__(kCtaThreads, 1) kmeans_tc_kernel(const Params 
           : "=r"(done) : "r"(mbar_addr), "r"(parity) : "memory");
     }
     parity ^= 1u;
-    if (!done) fail[g] = 1u;
-    group_sync(g);
-    if (fail[g] != 0u) {  // somebody gave up: record it and leave through the common exit
-      if (lt == 0) atomicExch(p.error, 1 + (int)((tile - first) / stride));  // 1 + how many tiles this group had finished
-      break;
+    if (!done && !gave_up) {
+      gave_up = true;
+      atomicExch(p.error, 1 + (int)((tile - first) / stride));  // 1 + how many tiles this group had finished
     }
+    __syncwarp();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
     // ---- epilogue: TMEM lane pt = point i; its two threads scan one half of the centres each ----
@@ -402,7 +431,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) kmeans_tc_kernel(const Params 
     // against 256 centres 275 us, now @K8@.)
     const float xn = sqrtf(xx);
     // error bound of a score: L2  eps*|x||y|max ;  cosine  eps*|x|
-    const float tol2 = 2.0f * (p.metric == F2C_L2 ? p.eps * xn * cmax : p.eps * xn);
+    tol2 = 2.0f * (p.metric == F2C_L2 ? p.eps * xn * cmax : p.eps * xn);
     const uint32_t lane_addr = tmem_base + ((uint32_t)(lane_quarter * 32) << 16);
     const int c_split = ((p.n_pad / 32 + 1) / 2) * 32;
     const int c_begin = half == 0 ? 0 : c_split, c_end = half == 0 ? c_split : p.n_pad;
@@ -440,7 +469,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) kmeans_tc_kernel(const Params 
       }
     }
     static_assert(kGroups == 8, "the tree below");
-    float best = max3(max3(row_max[0], row_max[1], row_max[2]), max3(row_max[3], row_max[4], row_max[5]), fmaxf(row_max[6], row_max[7]));
+    best = max3(max3(row_max[0], row_max[1], row_max[2]), max3(row_max[3], row_max[4], row_max[5]), fmaxf(row_max[6], row_max[7]));
     // hits, each counted as 64 + its number: below 128 there was one
     const float from = best - tol2;
     int rows_hit = 0, cols_hit = 0;
@@ -448,26 +477,11 @@ __global__ void __launch_bounds__(kCtaThreads, 1) kmeans_tc_kernel(const Params 
     for (int q = 0; q < kGroups; ++q) rows_hit += row_max[q] >= from ? 64 + q : 0;
 #pragma unroll
     for (int j = 0; j < 16; ++j) cols_hit += col_max[j] >= from ? 64 + j : 0;
-    int centre = rows_hit < 128 && cols_hit < 128 ? c_begin + 16 * (rows_hit - 64) + cols_hit - 64 : -1;
-    if (half == 1) exch[pt] = make_float2(best, __int_as_float(centre));
-    group_sync(g);
-    if (half == 1) continue;
-    {
-      const float2 o = exch[pt];
-      const bool mine = best - tol2 > o.x, other = o.x - tol2 > best;
-      centre = mine ? centre : (other ? __float_as_int(o.y) : -1);
-      best = fmaxf(best, o.x);
-    }
-    const bool odd = bad_centres || !(xx < INFINITY) || !(best > -INFINITY);  // NaN / inf somewhere: exact scorer
-    if (i < p.n) {
-      if (odd || centre < 0) {  // undecided: the exact scorer assigns it afterwards
-        const int slot = atomicAdd(p.amb_count, 1);
-        p.amb_list[slot] = (int32_t)i;
-      } else {
-        p.labels[i] = centre;
-      }
-    }
+    centre = rows_hit < 128 && cols_hit < 128 ? c_begin + 16 * (rows_hit - 64) + cols_hit - 64 : -1;
+    if (half == 1) exch[turn * kTileM + pt] = make_float2(best, __int_as_float(centre));
   }
+  group_sync(g);
+  if (half == 0) finish(turn ^ 1);
 
   // ---- common exit: all TMEM reads retired, then the allocating warp frees the columns ----
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -490,11 +504,11 @@ int kmeans_assign_tc(const float* x, const float* y, int64_t* labels, int64_t n,
   p.done = done;
   p.x = x; p.y = y; p.labels = labels; p.n = n; p.k = (int)k; p.d = (int)d; p.metric = metric;
   p.dp = (int)((d + 7) / 8 * 8);
-  p.terms = p.dp <= 32 ? 3 : 1;
   p.bf16 = p.dp > 32 ? 1 : 0;  // 3 x tf32 does not fit in shared memory beyond d = 32; 3 x bf16 does up to d = 64
   if (p.bf16) p.dp = (int)((d + 15) / 16 * 16);  // one bf16 MMA consumes 16 values of K
   p.n_pad = (int)((k + 31) / 32 * 32);
   p.vec4 = d % 4 == 0 && aligned(x, 16);
+  p.y_vec4 = d % 4 == 0 && aligned(y, 16);
   // relative error bound of one score: 2^-16 for the tf32 split (true error ~2^-18.4); 2^-14 for the bf16 split
   // (neglected terms x2.y2 + x.y3 + x3.y <= 3 * 2^-18 |x||y| = 2^-16.4)
   p.eps = p.bf16 ? 1.0f / 16384.0f : 1.0f / 65536.0f;
@@ -502,8 +516,8 @@ int kmeans_assign_tc(const float* x, const float* y, int64_t* labels, int64_t n,
   p.amb_count = head; p.error = head + 1; p.amb_list = head + 64;
   cudaError_t e = cudaMemsetAsync(head, 0, 256, st);
   if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "kmeans_assign: %s", cudaGetErrorString(e));
-  const int kc = (p.bf16 ? 3 * p.dp / 8 : p.terms * p.dp / 4) + 2;
-  size_t smem = (size_t)kc * (tc::kMaxN + 2 * tc::kTileM) * 16 + tc::kMaxN * 4 + 2 * tc::kTileM * 8 + 64 + 4 * tc::kTileM * 4;
+  const int kc = (p.bf16 ? 3 * p.dp / 8 : 3 * p.dp / 4) + 2;
+  size_t smem = (size_t)kc * (tc::kMaxN + 2 * tc::kTileM) * 16 + tc::kMaxN * 4 + 4 * tc::kTileM * 8 + 64 + 8 * tc::kTileM * 4;
   if (smem < 120 * 1024) smem = 120 * 1024;  // one CTA per SM: a second one would only wait for the TMEM columns
   auto kern = p.bf16 ? tc::kmeans_tc_kernel<true> : tc::kmeans_tc_kernel<false>;
   e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -514,8 +528,8 @@ int kmeans_assign_tc(const float* x, const float* y, int64_t* labels, int64_t n,
   launch_dependent(kern, (unsigned)grid, tc::kCtaThreads, smem, st, p);
   int rc = check_launch("kmeans_assign (tensor cores)");
   if (rc) return rc;
-  // undecided points: exact fp32 scorer over the device-side list
-  return kmeans_assign_exact_listed(x, y, labels, p.amb_list, p.amb_count, n, k, d, metric, st);
+  // undecided points (all of them after a wait that ran out): exact fp32 scorer over the device-side list
+  return kmeans_assign_exact_listed(x, y, labels, p.amb_list, p.amb_count, p.error, n, k, d, metric, st);
 }
 
 // ------------------------------------------------------------------------------------------------------
@@ -582,7 +596,7 @@ extern "C" int f2c_kmeans_assign_static(const float* x, const float* centers, in
 
 // What the last f2c_kmeans_assign_static call on the current device left in the header of the built-in array: the
 // number of points the tensor-core pass handed to the exact scorer, and the code the kernel writes when one of its
-// bounded barrier waits ran out (0 = none; labels of the unfinished tiles are then unwritten).  Waits for `stream`,
+// bounded barrier waits ran out (0 = none; the exact scorer then assigned every point).  Waits for `stream`,
 // copies the eight header bytes to the host, allocates nothing.  Returns F2C_ERR_CUDA when the code is non-zero.
 extern "C" int f2c_kmeans_assign_static_status(int32_t* undecided_host, int32_t* error_host, void* stream) {
   using namespace f2c;

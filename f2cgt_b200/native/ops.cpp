@@ -184,6 +184,35 @@ PyObject* two_level_spmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
+PyObject* kmeans_assign(PyObject*, PyObject* const* a, Py_ssize_t n) {  // x, centers, metric and scorer flags -> labels, [undecided, error]
+  return guarded([&]() -> PyObject* {
+    arguments("kmeans_assign", n, 3);
+    const at::Tensor& x = tensor(a[0], "data", kF32);
+    const at::Tensor& centers = tensor(a[1], "centers", kF32);
+    if (x.dim() != 2 || centers.dim() != 2 || x.size(1) != centers.size(1)) fail(PyExc_RuntimeError, "data must be [n, d] and centers [k, d]");
+    const int metric = (int)integer(a[2]);
+    c10::cuda::CUDAGuard guard(x.device());
+    const cudaStream_t st = stream_of(x);
+    const int64_t rows = x.size(0), k = centers.size(0), d = x.size(1);
+    at::Tensor labels = empty({rows}, at::kLong, x.device()), head = empty({2}, at::kInt, x.device());
+    const int64_t bytes = f2c_kmeans_assign_workspace(rows, k, d);
+    at::Tensor ws;
+    if (bytes > 0) {
+      ws = empty({bytes}, at::kByte, x.device());
+      C10_CUDA_CHECK(cudaMemsetAsync(ws.data_ptr(), 0, 256, st));  // the exact scorer leaves it as it is
+    }
+    check_status(f2c_kmeans_assign(x.const_data_ptr<float>(), centers.const_data_ptr<float>(), labels.mutable_data_ptr<int64_t>(), rows, k, d,
+                                   metric, bytes > 0 ? ws.data_ptr() : nullptr, st));
+    if (bytes > 0) C10_CUDA_CHECK(cudaMemcpyAsync(head.data_ptr(), ws.data_ptr(), 8, cudaMemcpyDeviceToDevice, st));
+    else C10_CUDA_CHECK(cudaMemsetAsync(head.data_ptr(), 0, 8, st));
+    PyObject* l = THPVariable_Wrap(std::move(labels));
+    PyObject* h = THPVariable_Wrap(std::move(head));
+    PyObject* r = PyTuple_Pack(2, l, h);
+    Py_DECREF(l); Py_DECREF(h);
+    return r;
+  });
+}
+
 PyObject* set_error_class(PyObject*, PyObject* cls) {
   Py_XSETREF(g_error_class, Py_NewRef(cls));
   Py_RETURN_NONE;
@@ -196,6 +225,7 @@ PyMethodDef g_methods[] = {
     {"sq_spmm", (PyCFunction)(void*)sq_spmm, METH_FASTCALL, nullptr},
     {"vq_spmm", (PyCFunction)(void*)vq_spmm, METH_FASTCALL, nullptr},
     {"two_level_spmm", (PyCFunction)(void*)two_level_spmm, METH_FASTCALL, nullptr},
+    {"kmeans_assign", (PyCFunction)(void*)kmeans_assign, METH_FASTCALL, nullptr},
     {"set_error_class", set_error_class, METH_O, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 

@@ -337,31 +337,28 @@ def pairwise_distance(x, y, metric):
     return dist
 
 
-def kmeans_assign(x, centers, metric, scorer="auto"):
+_SCORER = {"auto": 0, "exact": _lib.SCORER_EXACT, "tensor": _lib.SCORER_TENSOR}
+
+
+class _KMeansAssign:
     """labels[i] = first argmin_c dist(x_i, centers_c), int64 (src/kmeans.cu:77-98).  scorer = "auto" | "exact" (fp32 FMA) |
-    "tensor" (tcgen05 + exact re-score of undecided points): same labels, pinned per call for tests and timing."""
-    _chk(x, "data", (torch.float32,))
-    _chk(centers, "centers", (torch.float32,))
-    if x.dim() != 2 or centers.dim() != 2 or x.shape[1] != centers.shape[1]:
-        raise RuntimeError("data must be [n, d] and centers [k, d]")
-    n, d = x.shape
-    k = centers.shape[0]
-    labels = torch.empty((n,), dtype=torch.int64, device=x.device)
-    ws_bytes = lib.f2c_kmeans_assign_workspace(n, k, d)
-    ws = torch.empty((ws_bytes,), dtype=torch.uint8, device=x.device) if ws_bytes > 0 else None
-    if ws is not None:
-        ws[:256].zero_()  # header: [undecided count, error code]; the library clears it again when it uses the scratch
-    with _on(x):
-        flags = {"auto": 0, "exact": _lib.SCORER_EXACT, "tensor": _lib.SCORER_TENSOR}[scorer]
-        check(lib.f2c_kmeans_assign(_ptr(x), _ptr(centers), _ptr(labels), n, k, d, _metric(metric) | flags, _ptr(ws) if ws is not None else 0,
-                                    _stream(x)))
-    if ws is not None:
-        # word 1 of the scratch header is set when the tensor-core kernel gave up on a bounded wait
-        head = ws[:8].view(torch.int32).cpu()
-        if int(head[1]) != 0:
-            raise RuntimeError("f2cgt_b200: kmeans_assign: tensor-core kernel reported a timed-out wait")
-        kmeans_assign.last_undecided = int(head[0])
-    return labels
+    "tensor" (tcgen05 + exact re-score of undecided points): same labels, pinned per call for tests and timing.
+
+    The call does not wait for the device: a tensor-core kernel that gave up on a bounded wait makes the exact scorer assign
+    every point.  ``last_undecided`` (points of the last call that the exact scorer assigned) waits when it is read."""
+
+    _head = None
+
+    def __call__(self, x, centers, metric, scorer="auto"):
+        labels, self._head = _native.kmeans_assign(x, centers, _metric(metric) | _SCORER[scorer])
+        return labels
+
+    @property
+    def last_undecided(self):
+        return int(self._head[0]) if self._head is not None else 0
+
+
+kmeans_assign = _KMeansAssign()
 
 
 class KMeans:
