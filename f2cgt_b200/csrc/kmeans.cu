@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(kListThreads) kmeans_listed_kernel(const float
   float* yc_s = reinterpret_cast<float*>(smem_raw);  // [kc][STRIDE]
   float* cc_s = yc_s + (size_t)kc * STRIDE;          // [kc]
   auto stage = [&](int c0, int nc) {
-    if (y_vec4) {  // d % 4 == 0; eight 16-byte loads in flight per thread (single floats: 15 us for 256 x 64, now @L64@)
+    if (y_vec4) {  // d % 4 == 0; eight 16-byte loads in flight per thread (single floats: 15 us for 256 x 64, now 8)
 #pragma unroll 8
       for (int e = threadIdx.x; e < nc * (DMAX / 4); e += kListThreads) {
         const int c = e / (DMAX / 4), t = 4 * (e - c * (DMAX / 4));
@@ -371,7 +371,7 @@ extern "C" int f2c_kmeans_assign(const float* x, const float* centers, int64_t* 
   F2C_REQUIRE(x && centers && labels, F2C_ERR_INVALID, "kmeans_assign: null pointer");
   // tensor-core path when a scratch buffer is supplied and the shape fits; the exact fp32 scorer otherwise, and below four
   // dimensions, where many points' best two centres are too close for the split product (2,449,029 x 4 against 256 centres:
-  // exact scorer 982 us, tensor cores @K4@)
+  // exact scorer 982 us, tensor cores 159)
   const bool prefer_tc = d >= 4 || scorer == F2C_SCORER_TENSOR;
   if (workspace != nullptr && kmeans_tc_supported(n, k, d) && prefer_tc && scorer != F2C_SCORER_EXACT && aligned(workspace, 16))
     return kmeans_assign_tc(x, centers, labels, n, k, d, metric, workspace, (cudaStream_t)stream, nullptr);

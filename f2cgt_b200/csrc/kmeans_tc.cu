@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) kmeans_tc_kernel(const Params 
   if (tid < kMaxN) {
     const int c = tid;
     const int G = p.dp / 4;
-    // sixteen numbers of the row at a time, their loads in flight together (one at a time: 30 us for 256 x 64, whatever n)
+    // sixteen numbers of the row at a time, their loads in flight together (one at a time: 31 us for 256 x 64 and few points, now 18)
     auto row16 = [&](int t0, float (&v)[16]) {
       const float* yc = p.y + (int64_t)c * p.d;
 #pragma unroll
@@ -428,7 +428,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) kmeans_tc_kernel(const Params 
     // their group (col_max).  Scores within 2 tol of the best lie in the crossings of the groups and columns whose maximum does,
     // so the best centre is decided exactly when that is one group and one column - at the crossing.  (A running best, second
     // best and index took five compare instructions per score, which issue at half rate: 2,449,029 points of 8 columns
-    // against 256 centres 275 us, now @K8@.)
+    // against 256 centres 275 us, 152 with this and one barrier per tile instead of three.)
     const float xn = sqrtf(xx);
     // error bound of a score: L2  eps*|x||y|max ;  cosine  eps*|x|
     tol2 = 2.0f * (p.metric == F2C_L2 ? p.eps * xn * cmax : p.eps * xn);
