@@ -149,16 +149,8 @@ __global__ void __launch_bounds__(kListThreads) kmeans_listed_kernel(const float
                                                                      int64_t* __restrict__ labels, const int32_t* __restrict__ list,
                                                                      const int32_t* __restrict__ count_dev, const int32_t* __restrict__ all_dev,
                                                                      int64_t max_count, int k, int d, int kc, int y_vec4) {
-  dependency_wait();
-  release_dependents();
   constexpr int STRIDE = DMAX + 4;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const bool all = all_dev != nullptr && *all_dev != 0;  // every point instead of the listed ones
-  const int64_t cnt = !all && *count_dev < max_count ? *count_dev : max_count;
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = ((int64_t)blockIdx.x * kListThreads + threadIdx.x) >> 5, n_warps = ((int64_t)gridDim.x * kListThreads) >> 5;
-  const bool by_warp = cnt <= n_warps * kShortRounds && kc >= k;
-  if (by_warp ? (int64_t)blockIdx.x * (kListThreads / 32) >= cnt : (int64_t)blockIdx.x * kListThreads >= cnt) return;
   float* yc_s = reinterpret_cast<float*>(smem_raw);  // [kc][STRIDE]
   float* cc_s = yc_s + (size_t)kc * STRIDE;          // [kc]
   auto stage = [&](int c0, int nc) {
@@ -188,6 +180,16 @@ __global__ void __launch_bounds__(kListThreads) kmeans_listed_kernel(const float
       __syncthreads();
     }
   };
+  // The kernel before on the stream, which makes the list, has waited for the centres, so they may be staged before it is done.
+  if (kc >= k) stage(0, k);
+  dependency_wait();
+  release_dependents();
+  const bool all = all_dev != nullptr && *all_dev != 0;  // every point instead of the listed ones
+  const int64_t cnt = !all && *count_dev < max_count ? *count_dev : max_count;
+  const int lane = threadIdx.x & 31;
+  const int64_t warp = ((int64_t)blockIdx.x * kListThreads + threadIdx.x) >> 5, n_warps = ((int64_t)gridDim.x * kListThreads) >> 5;
+  const bool by_warp = cnt <= n_warps * kShortRounds && kc >= k;
+  if (by_warp ? (int64_t)blockIdx.x * (kListThreads / 32) >= cnt : (int64_t)blockIdx.x * kListThreads >= cnt) return;
   auto distance = [&](const float (&xr)[DMAX], float xx, int c) {
     const float4* yc4 = reinterpret_cast<const float4*>(yc_s + (size_t)c * STRIDE);
     float acc = 0.0f;
@@ -216,7 +218,6 @@ __global__ void __launch_bounds__(kListThreads) kmeans_listed_kernel(const float
     }
   };
   if (by_warp) {
-    stage(0, k);
     for (int64_t s = warp; s < cnt; s += n_warps) {
       const int64_t i = all ? s : (int64_t)list[s];
       load_point(i);
@@ -244,8 +245,10 @@ __global__ void __launch_bounds__(kListThreads) kmeans_listed_kernel(const float
     int best_c = 0;
     for (int c0 = 0; c0 < k; c0 += kc) {
       const int nc = min(kc, k - c0);
-      __syncthreads();
-      stage(c0, nc);
+      if (kc < k) {
+        __syncthreads();
+        stage(c0, nc);
+      }
       for (int c = 0; c < nc; ++c) {
         const float v = distance(xr, xx, c);
         if (v < best) { best = v; best_c = c0 + c; }
@@ -327,7 +330,7 @@ int kmeans_assign_exact_listed(const float* x, const float* y, int64_t* labels, 
 bool kmeans_tc_supported(int64_t n, int64_t k, int64_t d);
 int64_t kmeans_tc_workspace(int64_t n);
 int kmeans_assign_tc(const float* x, const float* y, int64_t* labels, int64_t n, int64_t k, int64_t d, int metric, void* workspace,
-                     cudaStream_t st, const int32_t* done);
+                     cudaStream_t st, const int32_t* done, bool head_is_clear);
 
 static int validate_km(const char* op, int64_t n, int64_t k, int64_t d, int metric) {
   F2C_REQUIRE(n >= 0 && k >= 1 && d >= 1, F2C_ERR_INVALID, "%s: bad shape n=%lld k=%lld d=%lld", op, (long long)n, (long long)k,
@@ -374,6 +377,6 @@ extern "C" int f2c_kmeans_assign(const float* x, const float* centers, int64_t* 
   // exact scorer 982 us, tensor cores 159)
   const bool prefer_tc = d >= 4 || scorer == F2C_SCORER_TENSOR;
   if (workspace != nullptr && kmeans_tc_supported(n, k, d) && prefer_tc && scorer != F2C_SCORER_EXACT && aligned(workspace, 16))
-    return kmeans_assign_tc(x, centers, labels, n, k, d, metric, workspace, (cudaStream_t)stream, nullptr);
+    return kmeans_assign_tc(x, centers, labels, n, k, d, metric, workspace, (cudaStream_t)stream, nullptr, false);
   return kmeans_assign_exact(x, centers, labels, nullptr, n, k, d, metric, (cudaStream_t)stream, nullptr);
 }

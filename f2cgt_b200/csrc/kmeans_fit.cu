@@ -22,7 +22,7 @@ namespace f2c {
 bool kmeans_tc_supported(int64_t n, int64_t k, int64_t d);
 int64_t kmeans_tc_workspace(int64_t n);
 int kmeans_assign_tc(const float* x, const float* y, int64_t* labels, int64_t n, int64_t k, int64_t d, int metric, void* workspace,
-                     cudaStream_t st, const int32_t* done);
+                     cudaStream_t st, const int32_t* done, bool head_is_clear);
 int kmeans_assign_exact(const float* x, const float* y, int64_t* labels, const int32_t* subset, int64_t n, int64_t k, int64_t d,
                         int metric, cudaStream_t st, const int32_t* done);
 
@@ -65,18 +65,31 @@ __global__ void begin_kernel(State* st) {
 
 // Centres <- sums / counts (clusters without points keep theirs), sums and counts <- 0, shift, done.  One CTA.
 __device__ void finish_iteration(float* __restrict__ centers, long long* sums, unsigned int* counts, int k, int d, double unit,
-                                 double tol, const int32_t* assign_error, State* st) {
+                                 double tol, int32_t* assign_head, State* st) {
   __shared__ double part[kThreads / 32];
   double shift = 0.0;
-  for (int i = threadIdx.x; i < k * d; i += kThreads) {
-    const unsigned int cnt = __ldcg(counts + i / d);
-    const long long s = __ldcg(sums + i);
-    sums[i] = 0;
-    if (cnt != 0u) {
-      const float next = (float)((double)s * unit) / (float)cnt;
-      const float diff = next - centers[i];
-      shift += (double)(diff * diff);
-      centers[i] = next;
+  // this CTA alone works now: the loads of eight entries are in flight together (one at a time: 11 of 23 us for 256 x 32)
+  constexpr int U = 8;
+  for (int i0 = threadIdx.x; i0 < k * d; i0 += U * kThreads) {
+    unsigned int cnt[U];
+    long long sum[U];
+    float old[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + u * kThreads;
+      cnt[u] = 0u;
+      if (i < k * d) { cnt[u] = __ldcg(counts + i / d); sum[u] = __ldcg(sums + i); old[u] = centers[i]; }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + u * kThreads;
+      if (cnt[u] != 0u) {  // sums of clusters without points are zero
+        sums[i] = 0;
+        const float next = (float)((double)sum[u] * unit) / (float)cnt[u];
+        const float diff = next - old[u];
+        shift += (double)(diff * diff);
+        centers[i] = next;
+      }
     }
   }
 #pragma unroll
@@ -90,7 +103,10 @@ __device__ void finish_iteration(float* __restrict__ centers, long long* sums, u
     st->shift = total;
     st->iterations += 1;
     st->arrived = 0u;
-    if (assign_error != nullptr && *assign_error != 0) { st->assign_error = *assign_error; st->done = 1; }
+    if (assign_head != nullptr) {
+      if (assign_head[1] != 0) { st->assign_error = assign_head[1]; st->done = 1; }
+      assign_head[0] = 0;  // the next assignment's list is empty
+    }
     if ((double)(float)total <= tol) st->done = 1;
   }
 }
@@ -99,10 +115,7 @@ __device__ void finish_iteration(float* __restrict__ centers, long long* sums, u
 template <bool SHARED>
 __global__ void __launch_bounds__(kThreads) accumulate_kernel(const float* __restrict__ x, const int64_t* __restrict__ labels,
                                                               float* __restrict__ centers, long long* sums, unsigned int* counts,
-                                                              int64_t n, int k, int d, double tol, const int32_t* assign_error, State* st) {
-  dependency_wait();
-  release_dependents();
-  if (*(volatile int32_t*)&st->done != 0) return;
+                                                              int64_t n, int k, int d, double tol, int32_t* assign_head, State* st) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int kd = k * d;
   uint32_t* lo = reinterpret_cast<uint32_t*>(smem);
@@ -111,6 +124,11 @@ __global__ void __launch_bounds__(kThreads) accumulate_kernel(const float* __res
   uint16_t* lab = reinterpret_cast<uint16_t*>(cnt + (SHARED ? k : 0));  // labels of the chunk (k <= 65535 here)
   __shared__ bool last;
   const int tid = (int)threadIdx.x;
+  if (SHARED)  // while the kernel before still runs
+    for (int i = tid; i < 2 * kd + k; i += kThreads) lo[i] = 0u;
+  dependency_wait();
+  release_dependents();
+  if (*(volatile int32_t*)&st->done != 0) return;
   // |x| <= 2^e: unit of the last place = 2^(e - bits)
   const uint32_t mb = st->max_bits;
   const int e = mb == 0u ? 0 : (int)(mb >> 23) - 126;
@@ -120,10 +138,7 @@ __global__ void __launch_bounds__(kThreads) accumulate_kernel(const float* __res
   // chunks are dealt so that every CTA gets almost the same number of points
   const int64_t rounds = (n + (int64_t)gridDim.x * kChunk - 1) / ((int64_t)gridDim.x * kChunk);
   const int64_t per = (n + rounds * gridDim.x - 1) / (rounds * gridDim.x);
-  if (SHARED) {
-    for (int i = tid; i < 2 * kd + k; i += kThreads) lo[i] = 0u;
-    __syncthreads();
-  }
+  if (SHARED) __syncthreads();
   for (int64_t r = 0; r < rounds; ++r) {
     const int64_t p0 = (r * gridDim.x + blockIdx.x) * per;
     const int pts = (int)max((int64_t)0, min(per, n - p0));
@@ -173,7 +188,7 @@ __global__ void __launch_bounds__(kThreads) accumulate_kernel(const float* __res
   __syncthreads();
   if (last) {
     __threadfence();
-    finish_iteration(centers, sums, counts, k, d, unit, tol, assign_error, st);
+    finish_iteration(centers, sums, counts, k, d, unit, tol, assign_head, st);
   }
 }
 
@@ -215,6 +230,7 @@ extern "C" int f2c_kmeans_fit_begin(const float* x, int64_t n, int64_t k, int64_
   cudaStream_t st = (cudaStream_t)stream;
   const fit::Layout w = fit::plan(n, k, d);
   cudaError_t e = cudaMemsetAsync(workspace, 0, w.labels, st);  // state, sums and counts
+  if (e == cudaSuccess && kmeans_tc_supported(n, k, d)) e = cudaMemsetAsync((unsigned char*)workspace + w.assign, 0, 256, st);
   if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "%s: %s", op, cudaGetErrorString(e));
   fit::State* state = (fit::State*)workspace;
   int64_t blocks = ceil_div(n * d, 256 * 8);
@@ -239,7 +255,7 @@ extern "C" int f2c_kmeans_fit_iterate(const float* x, float* centers, int64_t n,
   unsigned int* counts = (unsigned int*)(ws + w.counts);
   int64_t* labels = (int64_t*)(ws + w.labels);
   const bool tc = kmeans_tc_supported(n, k, d) && d >= 4;
-  const int32_t* assign_error = tc ? (const int32_t*)(ws + w.assign) + 1 : nullptr;
+  int32_t* assign_head = tc ? (int32_t*)(ws + w.assign) : nullptr;  // [undecided points, error]; cleared by f2c_kmeans_fit_begin, then by every iteration
   const size_t smem = ((size_t)2 * k * d + k) * 4 + fit::kChunk * 2;
   const bool shared = smem <= fit::kSmemLimit && k <= 65535;
   auto kern = shared ? fit::accumulate_kernel<true> : fit::accumulate_kernel<false>;
@@ -251,11 +267,11 @@ extern "C" int f2c_kmeans_fit_iterate(const float* x, float* centers, int64_t n,
   int64_t grid = shared ? ceil_div(n, 256) : ceil_div(n * d, fit::kThreads);
   if (grid > current_sm_count()) grid = current_sm_count();
   for (int it = 0; it < iterations; ++it) {
-    rc = tc ? kmeans_assign_tc(x, centers, labels, n, k, d, metric, ws + w.assign, st, &state->done)
+    rc = tc ? kmeans_assign_tc(x, centers, labels, n, k, d, metric, ws + w.assign, st, &state->done, true)
             : kmeans_assign_exact(x, centers, labels, nullptr, n, k, d, metric, st, &state->done);
     if (rc) return rc;
-    launch_dependent(kern, (unsigned)grid, fit::kThreads, shared ? smem : 0, st, x, labels, centers, sums, counts, n, (int)k, (int)d, tol, assign_error,
-                                                                  state);
+    launch_dependent(kern, (unsigned)grid, fit::kThreads, shared ? smem : 0, st, x, labels, centers, sums, counts, n, (int)k, (int)d, tol, assign_head,
+                     state);
     rc = check_launch(op);
     if (rc) return rc;
   }

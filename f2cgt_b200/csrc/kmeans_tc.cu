@@ -263,7 +263,13 @@ __global__ void __launch_bounds__(kCtaThreads, 1) kmeans_tc_kernel(const Params 
   const uint32_t tmem_base = *tmem_slot + (uint32_t)g * 256u;
   // largest centre norm (tolerance of the L2 score); a non-finite centre sends every point to the exact scorer
   float cmax = 0.0f, poison = 0.0f;
-  for (int c = 0; c < p.k; ++c) { cmax = fmaxf(cmax, scratch[c]); poison = fmaf(scratch[c], 0.0f, poison); }  // inf, NaN -> NaN
+#pragma unroll
+  for (int c = threadIdx.x & 31; c < kMaxN; c += 32) { cmax = fmaxf(cmax, scratch[c]); poison = fmaf(scratch[c], 0.0f, poison); }  // inf, NaN -> NaN
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    cmax = fmaxf(cmax, __shfl_xor_sync(0xffffffffu, cmax, o));
+    poison += __shfl_xor_sync(0xffffffffu, poison, o);
+  }
   const bool bad_centres = !(poison == 0.0f);
   cmax = sqrtf(cmax);
 
@@ -499,7 +505,7 @@ bool kmeans_tc_supported(int64_t n, int64_t k, int64_t d) { return n >= 1 && n <
 int64_t kmeans_tc_workspace(int64_t n) { return 256 + 4 * n; }  // [count, error, pad][index list]
 
 int kmeans_assign_tc(const float* x, const float* y, int64_t* labels, int64_t n, int64_t k, int64_t d, int metric, void* workspace,
-                     cudaStream_t st, const int32_t* done) {
+                     cudaStream_t st, const int32_t* done, bool head_is_clear) {
   tc::Params p{};
   p.done = done;
   p.x = x; p.y = y; p.labels = labels; p.n = n; p.k = (int)k; p.d = (int)d; p.metric = metric;
@@ -514,7 +520,7 @@ int kmeans_assign_tc(const float* x, const float* y, int64_t* labels, int64_t n,
   p.eps = p.bf16 ? 1.0f / 16384.0f : 1.0f / 65536.0f;
   int32_t* head = reinterpret_cast<int32_t*>(workspace);
   p.amb_count = head; p.error = head + 1; p.amb_list = head + 64;
-  cudaError_t e = cudaMemsetAsync(head, 0, 256, st);
+  cudaError_t e = head_is_clear ? cudaSuccess : cudaMemsetAsync(head, 0, 256, st);
   if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "kmeans_assign: %s", cudaGetErrorString(e));
   const int kc = (p.bf16 ? 3 * p.dp / 8 : 3 * p.dp / 4) + 2;
   size_t smem = (size_t)kc * (tc::kMaxN + 2 * tc::kTileM) * 16 + tc::kMaxN * 4 + 4 * tc::kTileM * 8 + 64 + 8 * tc::kTileM * 4;
@@ -591,7 +597,7 @@ extern "C" int f2c_kmeans_assign_static(const float* x, const float* centers, in
   int rc = tc::static_scratch(op, &scratch);
   if (rc) return rc;
   // same kernels as kmeans_assign; the header (count, error code) is cleared inside
-  return kmeans_assign_tc(x, centers, labels, n, k, d, metric, scratch, (cudaStream_t)stream, nullptr);
+  return kmeans_assign_tc(x, centers, labels, n, k, d, metric, scratch, (cudaStream_t)stream, nullptr, false);
 }
 
 // What the last f2c_kmeans_assign_static call on the current device left in the header of the built-in array: the
