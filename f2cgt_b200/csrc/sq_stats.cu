@@ -44,44 +44,71 @@ struct Args {
   double* out;          // [5]: the four order statistics, the mean
 };
 
-// exclusive scan position of `rank` in hist[0 .. NB): bin and rank inside it; all threads call, NB a multiple of kThreads or smaller
-template <int NB>
-__device__ void locate(const uint32_t* __restrict__ hist, unsigned long long rank, uint32_t* bin, unsigned long long* inside) {
+struct Found { uint32_t bin[4], count[4]; unsigned long long inside[4]; };
+
+// For each wanted rank the bin of its histogram that holds it, the rank inside the bin and the bin's count.  H histograms of NB
+// bins; rank r lies in histogram owner[r].  One trip to memory for all of them: the CTA that does this works alone.
+template <int H, int NB>
+__device__ void locate(const uint32_t* __restrict__ hist, const int (&owner)[4], const unsigned long long (&rank)[4], Found* found) {
   constexpr int PER = NB >= kThreads ? NB / kThreads : 1;
-  __shared__ unsigned long long warp_sum[kThreads / 32];
-  const int tid = threadIdx.x, lane = tid & 31;
-  uint32_t v[PER];
-  unsigned long long mine = 0;
+  __shared__ unsigned long long warp_sum[H][kThreads / 32];
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  uint32_t v[H][PER];
+  unsigned long long before[H];
 #pragma unroll
-  for (int i = 0; i < PER; ++i) {
-    const int b = tid * PER + i;
-    v[i] = b < NB ? __ldcg(hist + b) : 0u;
-    mine += v[i];
-  }
-  unsigned long long inc = mine;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned long long t = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += t;
-  }
-  if (lane == 31) warp_sum[tid >> 5] = inc;
-  __syncthreads();
-  unsigned long long before = inc - mine;
-  for (int w = 0; w < (tid >> 5); ++w) before += warp_sum[w];
-  if (rank >= before && rank < before + mine) {
-    unsigned long long at = before;
+  for (int h = 0; h < H; ++h)
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
-      if (rank >= at && rank < at + v[i]) { *bin = (uint32_t)(tid * PER + i); *inside = rank - at; }
-      at += v[i];
+      const int b = tid * PER + i;
+      v[h][i] = b < NB ? __ldcg(hist + h * NB + b) : 0u;
+    }
+#pragma unroll
+  for (int h = 0; h < H; ++h) {
+    unsigned long long mine = 0;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) mine += v[h][i];
+    unsigned long long inc = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long t = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += t;
+    }
+    if (lane == 31) warp_sum[h][wid] = inc;
+    before[h] = inc - mine;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int h = 0; h < H; ++h) {
+#pragma unroll
+    for (int w = 0; w < kThreads / 32; ++w) before[h] += w < wid ? warp_sum[h][w] : 0ull;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      if (owner[r] != h) continue;
+      unsigned long long at = before[h];
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        if (rank[r] >= at && rank[r] < at + v[h][i]) { found->bin[r] = (uint32_t)(tid * PER + i); found->inside[r] = rank[r] - at; found->count[r] = v[h][i]; }
+        at += v[h][i];
+      }
     }
   }
   __syncthreads();
 }
 
+// A value that shares the fixed bits with wanted rank r (rare, so one copy of the code, and nothing captured by it).
+template <int PASS>
+__device__ __noinline__ void near_value(uint32_t key, int r, uint32_t* hist, bool keep, uint32_t* near_s, uint32_t* n_near, Work* w) {
+  const uint32_t bin = PASS == 2 ? (key >> kShift2) & (kBins2 - 1) : key & (kBins3 - 1);
+  atomicAdd(hist + r * (PASS == 2 ? kBins2 : kBins3) + bin, 1u);
+  if (PASS == 2 && keep) {
+    const uint32_t at = atomicAdd(n_near, 1u);
+    if (at < kNear) near_s[at] = key; else w->list[atomicAdd(&w->listed, 1u)] = key;
+  }
+}
+
 // PASS 1, 2, 3; VEC = 4: rows and columns allow 16-byte loads
 template <int PASS, int VEC>
-__global__ void __launch_bounds__(kThreads) select_kernel(const Args a) {
+__global__ void __launch_bounds__(kThreads, 2) select_kernel(const Args a) {
   dependency_wait();
   release_dependents();
   extern __shared__ __align__(16) uint32_t hist_s[];
@@ -94,35 +121,25 @@ __global__ void __launch_bounds__(kThreads) select_kernel(const Args a) {
   Work* w = a.work;
   for (int i = tid; i < kShared; i += kThreads) hist_s[i] = 0u;
   if (tid == 0) n_near = 0u;
-  // distinct prefixes of the wanted ranks (lower ranks own the histogram of a shared one)
-  uint32_t want[4];
-  int n_want = 0;
+  // distinct prefixes of the wanted ranks (the lowest rank owns the histogram of a shared one)
+  uint32_t prefix[4], want[4];
+  int owner[4] = {0, 0, 0, 0};
   if (PASS > 1) {
 #pragma unroll
+    for (int r = 0; r < 4; ++r) prefix[r] = __ldcg(&w->prefix[r]);
+#pragma unroll
     for (int r = 0; r < 4; ++r) {
-      const uint32_t pf = __ldcg(&w->prefix[r]);
-      bool seen = false;
+      owner[r] = r;
 #pragma unroll
-      for (int q = 0; q < r; ++q) seen |= q < n_want && want[q] == pf;
-      if (!seen) want[n_want++] = pf;
+      for (int q = r - 1; q >= 0; --q)
+        if (prefix[q] == prefix[r]) owner[r] = q;
+      want[r] = owner[r] == r ? prefix[r] : 0xffffffffu;
     }
-#pragma unroll
-    for (int r = 0; r < 4; ++r) if (r >= n_want) want[r] = 0xffffffffu;
   }
   __syncthreads();
   double sum = 0.0;
   const bool keep = PASS > 1 && __ldcg(&w->fits) != 0u;
   uint32_t* mine = hist_s + (PASS == 1 ? (wid & 1) * kBins1 : 0);
-  // a value that shares the fixed bits with a wanted rank (rare; one copy of the code)
-  auto near = [&](uint32_t key, uint32_t pf) __attribute__((noinline)) {
-    const int r = pf == want[0] ? 0 : pf == want[1] ? 1 : pf == want[2] ? 2 : 3;
-    const uint32_t bin = PASS == 2 ? (key >> kShift2) & (kBins2 - 1) : key & (kBins3 - 1);
-    atomicAdd(mine + r * (PASS == 2 ? kBins2 : kBins3) + bin, 1u);
-    if (PASS == 2 && keep) {
-      const uint32_t at = atomicAdd(&n_near, 1u);
-      if (at < kNear) near_s[at] = key; else w->list[atomicAdd(&w->listed, 1u)] = key;
-    }
-  };
   auto count = [&](float f) {
     const uint32_t key = __float_as_uint(f) & 0x7fffffffu;
     if (PASS == 1) {
@@ -130,7 +147,8 @@ __global__ void __launch_bounds__(kThreads) select_kernel(const Args a) {
       atomicAdd(mine + (key >> kShift1), 1u);
     } else {
       const uint32_t pf = PASS == 2 ? key >> kShift1 : key >> kShift2;
-      if (pf == want[0] || pf == want[1] || pf == want[2] || pf == want[3]) near(key, pf);
+      if (pf == want[0] || pf == want[1] || pf == want[2] || pf == want[3])
+        near_value<PASS>(key, pf == want[0] ? 0 : pf == want[1] ? 1 : pf == want[2] ? 2 : 3, mine, keep, near_s, &n_near, w);
     }
   };
   if (PASS == 3 && keep) {
@@ -203,41 +221,36 @@ __global__ void __launch_bounds__(kThreads) select_kernel(const Args a) {
   if (!last) return;
   __threadfence();
   // ---- the last CTA: which bin holds each wanted rank
-  unsigned long long bin_count[4];
+  // (it works alone, so its trips to memory count: one after the other they were 30 of the 37 us of the first pass over 3.2 M values)
+  __shared__ Found found;
+  __shared__ double cta_sum[PASS == 1 ? kMaxCtas : 1];
+  unsigned long long rank[4];
 #pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    __shared__ uint32_t bin;
-    __shared__ unsigned long long inside;
-    if (PASS == 1) {
-      locate<kBins1>(w->hist, a.rank[r], &bin, &inside);
-      if (tid == 0) { w->prefix[r] = bin; w->rank[r] = inside; }
-      bin_count[r] = __ldcg(w->hist + bin);
-    } else {
-      const uint32_t pf = __ldcg(&w->prefix[r]);
-      int owner = 0;
-      while (owner < 3 && want[owner] != pf) ++owner;
-      if (PASS == 2) {
-        locate<kBins2>(w->hist + owner * kBins2, __ldcg(&w->rank[r]), &bin, &inside);
-        if (tid == 0) { w->prefix[r] = (pf << 12) | bin; w->rank[r] = inside; }
-      } else {
-        locate<kBins3>(w->hist + owner * kBins3, __ldcg(&w->rank[r]), &bin, &inside);
-        if (tid == 0) a.out[r] = (double)__uint_as_float((pf << 6) | bin);
-      }
-    }
-    __syncthreads();
-  }
+  for (int r = 0; r < 4; ++r) rank[r] = PASS == 1 ? a.rank[r] : __ldcg(&w->rank[r]);
+  if (PASS == 1)
+    for (int i = tid; i < (int)gridDim.x; i += kThreads) cta_sum[i] = __ldcg(&w->sum[i]);
+  locate<PASS == 1 ? 1 : 4, PASS == 1 ? kBins1 : PASS == 2 ? kBins2 : kBins3>(w->hist, owner, rank, &found);
   if (PASS < 3)
     for (int i = tid; i < 4 * kBins2; i += kThreads) w->hist[i] = 0u;
+  if (tid < 4) {
+    const uint32_t pf = PASS == 1 ? 0u : tid == 0 ? prefix[0] : tid == 1 ? prefix[1] : tid == 2 ? prefix[2] : prefix[3];
+    if (PASS < 3) {
+      w->prefix[tid] = PASS == 1 ? found.bin[tid] : pf << 12 | found.bin[tid];
+      w->rank[tid] = found.inside[tid];
+    } else {
+      a.out[tid] = (double)__uint_as_float(pf << 6 | found.bin[tid]);
+    }
+  }
   if (PASS == 1 && tid == 0) {
     unsigned long long candidates = 0;
     for (int r = 0; r < 4; ++r) {
       bool seen = false;
-      for (int q = 0; q < r; ++q) seen |= w->prefix[q] == w->prefix[r];
-      if (!seen) candidates += bin_count[r];
+      for (int q = 0; q < r; ++q) seen |= found.bin[q] == found.bin[r];
+      if (!seen) candidates += found.count[r];
     }
     w->fits = candidates <= kListMax ? 1u : 0u;
     double t = 0.0;
-    for (int i = 0; i < (int)gridDim.x; ++i) t += __ldcg(&w->sum[i]);
+    for (int i = 0; i < (int)gridDim.x; ++i) t += cta_sum[i];
     a.out[4] = t / ((double)a.n_rows * (double)a.width);
   }
 }
