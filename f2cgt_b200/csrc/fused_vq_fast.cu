@@ -1,6 +1,6 @@
 // Pipelined fused VQ decode + aggregation and the single-launch two-level (hot rows SQ, all other rows VQ)
-// aggregation for the common shapes: uint8 codes, 4/8/16 code bytes per row, column_slice in {4,...,128} dividing
-// 128, hot rows 8- or 4-bit SQ.  Same arithmetic and CSC summation order as the general kernels of
+// aggregation for the common shapes: uint8 codes, 4/8/16 code bytes per row (two-level: any number), column_slice in
+// {4,...,128} dividing 128, hot rows 8- or 4-bit SQ.  Same arithmetic and CSC summation order as the general kernels of
 // fused_vq_spmm.cu (reference: src/fusion_spmm.cu:72-141 for VQ, src/sq_quantization.cu:123-153 for the hot rows).
 //
 // Why it is shaped like this.  A VQ row is 4..16 bytes, so HBM moves little; every edge pulls feat_dim floats out
@@ -70,10 +70,35 @@ template <int ROWW> __device__ __forceinline__ void load_code_row(CodeRow<ROWW>&
   else { uint4 v = ldg_nc_u128(p); c.w[0] = v.x; c.w[1] = v.y; c.w[ROWW > 2 ? 2 : 0] = v.z; c.w[ROWW > 3 ? 3 : 0] = v.w; }
 }
 
-// HB = 0: VQ only.  HB = 8 / 4: two-level with 8- / 4-bit hot rows.  ROWW = 32-bit words of one VQ code row.
+// A code row (ANY: the part's piece of it, which may start anywhere) as it arrives from memory.
+template <int ROWW, bool ANY> struct Arriving {
+  uint32_t w[ROWW + (ANY ? 1 : 0)];
+  uint32_t off = 0u;  // misalignment in bytes
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int i = 0; i < ROWW + (ANY ? 1 : 0); ++i) w[i] = 0u;
+  }
+  __device__ __forceinline__ void fetch(const uint8_t* at, uint32_t bytes) {
+    if (ANY) {  // the aligned words that hold a byte of it
+      off = (uint32_t)(reinterpret_cast<uintptr_t>(at) & 3u);
+#pragma unroll
+      for (int i = 0; i < ROWW + (ANY ? 1 : 0); ++i) w[i] = ldg_nc_u32_if(at - off + 4 * i, 4u * i < off + bytes);
+    } else {
+      CodeRow<ROWW> c;
+      load_code_row<ROWW>(c, at);
+#pragma unroll
+      for (int i = 0; i < ROWW; ++i) w[i] = c.w[i];
+    }
+  }
+  __device__ __forceinline__ uint32_t word(int i) const { return ANY ? __funnelshift_r(w[i], w[i + (ANY ? 1 : 0)], off * 8u) : w[i]; }
+};
+
+// HB = 0: VQ only.  HB = 8 / 4: two-level with 8- / 4-bit hot rows.  ROWW = 32-bit words of one VQ code row, or (ANY) of the
+// part's piece of a row of any length and alignment: two-level shapes whose rows are not 4, 8 or 16 bytes took the general kernel
+// before (90,000 rows x 12: 100 columns in 16 117 us, now @T100@; 128 in 64 @T128@; 256 in 8 @T256@).
 // PEER: the three tables are row-sharded over the GPUs of the box and every shard is mapped into this process; rows of
 // other ranks are read with ordinary loads over NVLink (no collective, no staging copy, nothing waits on another rank).
-template <int HB, typename IdxT, int ROWW, bool PEER = false>
+template <int HB, typename IdxT, int ROWW, bool ANY = false, bool PEER = false>
 __global__ void __launch_bounds__(VqCta<HB>::kThreads, 1) vq_fast_kernel(const VqParams p) {
   dependency_wait();
   release_dependents();
@@ -127,7 +152,7 @@ __global__ void __launch_bounds__(VqCta<HB>::kThreads, 1) vq_fast_kernel(const V
                                      : (uint32_t)(sl * K * stride + off * 4);
   const uint32_t cb_addr = smem_u32(cb_s) + lane_base;
   uint32_t* wbuf = reinterpret_cast<uint32_t*>(wbuf_all) + wid * 32 * ROWW;
-  const uint32_t wb_addr = smem_u32(wbuf) + (uint32_t)s;  // byte s of every staged code row
+  const uint32_t wb_addr = smem_u32(wbuf) + (uint32_t)(ANY ? sl : s);  // byte s of every staged code row
   const uint32_t hot_col_off = (uint32_t)((colc * (HB == 0 ? 8 : HB)) / 8);
   const uint8_t* hot_base = (HB != 0 && !PEER) ? p.sq_codes + hot_col_off : nullptr;
   const uint32_t hot_row_bytes = (uint32_t)p.sq_row_bytes;
@@ -135,7 +160,8 @@ __global__ void __launch_bounds__(VqCta<HB>::kThreads, 1) vq_fast_kernel(const V
 
   const IdxT* __restrict__ indptr = reinterpret_cast<const IdxT*>(p.indptr);
   const IdxT* __restrict__ indices = reinterpret_cast<const IdxT*>(p.indices);
-  const uint8_t* __restrict__ codes = reinterpret_cast<const uint8_t*>(p.codes);
+  const uint8_t* __restrict__ codes = reinterpret_cast<const uint8_t*>(p.codes) + (ANY ? s_begin : 0);
+  const uint32_t code_bytes = ANY ? (uint32_t)p.n_cb : (uint32_t)ROWB;  // from one row to the next
 
   float4 acc;
   auto add_vq = [&](uint32_t edge_byte_addr) {
@@ -166,14 +192,14 @@ __global__ void __launch_bounds__(VqCta<HB>::kThreads, 1) vq_fast_kernel(const V
     return HB == 8 ? ldg_nc_u32(q) : ldg_nc_u16(q);
   };
   // code row and slot of source node `id`
-  auto fetch_node = [&](int64_t id, CodeRow<ROWW>& c, int& sl_) {
+  auto fetch_node = [&](int64_t id, Arriving<ROWW, ANY>& c, int& sl_) {
     if (PEER) {
       const uint32_t owner = (uint32_t)__umul64hi((unsigned long long)id, p.peer.magic_nodes);
       const uint32_t local = (uint32_t)id - owner * p.peer.rps_nodes;
-      load_code_row<ROWW>(c, p.peer.code[owner] + (uint64_t)local * ROWB);
+      c.fetch(p.peer.code[owner] + (uint64_t)local * ROWB, ROWB);
       if (HB != 0) sl_ = p.peer.slot[0] != nullptr ? __ldg(p.peer.slot[owner] + local) : (id < p.n_hot ? (int)id : -1);
     } else {
-      load_code_row<ROWW>(c, codes + id * ROWB);
+      c.fetch(codes + id * code_bytes, (uint32_t)(s_end - s_begin));
       if (HB != 0) sl_ = hot_slot_of(p, id);
     }
   };
@@ -202,7 +228,7 @@ __global__ void __launch_bounds__(VqCta<HB>::kThreads, 1) vq_fast_kernel(const V
   int64_t beg1 = 0; int deg1 = 0;    // row of stage 1 -> 2
   IdxT idx2 = 0;                     // neighbour id of lane   (loaded by stage 1, read by stage 2)
   int64_t beg2 = 0; int deg2 = 0;    // row of stage 2 -> 3
-  CodeRow<ROWW> code3;               // code row of lane's edge (loaded by stage 2, read by stage 3)
+  Arriving<ROWW, ANY> code3;         // code row of lane's edge (loaded by stage 2, read by stage 3)
   int slot3 = -1;                    // slot of lane's edge     (loaded by stage 2, read by stage 3)
   int64_t beg3 = 0; int deg3 = 0;
   CodeRow<ROWW> code4;               // handed from stage 3 to stage 4
@@ -210,7 +236,8 @@ __global__ void __launch_bounds__(VqCta<HB>::kThreads, 1) vq_fast_kernel(const V
   int64_t beg4 = 0; int deg4 = 0;
   uint32_t hot[HB != 0 ? U : 1];     // hot-row bytes of this lane's columns (loaded by stage 3, read by stage 4)
 #pragma unroll
-  for (int w = 0; w < ROWW; ++w) { code3.w[w] = 0u; code4.w[w] = 0u; }
+  for (int w = 0; w < ROWW; ++w) code4.w[w] = 0u;
+  code3.clear();
 #pragma unroll
   for (int u = 0; u < (HB != 0 ? U : 1); ++u) hot[u] = 0u;
 
@@ -253,14 +280,16 @@ __global__ void __launch_bounds__(VqCta<HB>::kThreads, 1) vq_fast_kernel(const V
       // rows with more than 32 neighbours: further batches, fetched on the spot
       for (int64_t k0 = beg4 + 32; k0 < beg4 + deg4; k0 += 32) {
         const int cnt = (int)min((int64_t)32, beg4 + deg4 - k0);
-        CodeRow<ROWW> c;
-#pragma unroll
-        for (int w = 0; w < ROWW; ++w) c.w[w] = 0u;
+        Arriving<ROWW, ANY> more;
+        more.clear();
         int sl_mine = -1;
         if (lane < cnt) {
           const int64_t id = (int64_t)indices[k0 + lane];
-          fetch_node(id, c, sl_mine);
+          fetch_node(id, more, sl_mine);
         }
+        CodeRow<ROWW> c;
+#pragma unroll
+        for (int w = 0; w < ROWW; ++w) c.w[w] = more.word(w);
         __syncwarp();
         stage_codes(c, cnt);
         __syncwarp();
@@ -286,7 +315,7 @@ __global__ void __launch_bounds__(VqCta<HB>::kThreads, 1) vq_fast_kernel(const V
       const bool on = rH >= r0 && rH < n_dst;
       beg4 = beg3; deg4 = on ? deg3 : 0;
 #pragma unroll
-      for (int w = 0; w < ROWW; ++w) code4.w[w] = code3.w[w];
+      for (int w = 0; w < ROWW; ++w) code4.w[w] = code3.word(w);
       if (HB != 0) {
         slot4 = on ? slot3 : -1;
         mask4 = __ballot_sync(0xffffffffu, slot4 >= 0);
@@ -322,11 +351,11 @@ __global__ void __launch_bounds__(VqCta<HB>::kThreads, 1) vq_fast_kernel(const V
   }
 }
 
-template <int HB, typename IdxT, bool PEER>
+template <int HB, typename IdxT, bool ANY, bool PEER>
 static int launch_rows(const VqParams& p, int roww, dim3 grid, size_t smem, cudaStream_t st, const char* op) {
 #define F2C_VQF(RW)                                                                                      \
   {                                                                                                      \
-    auto kern = vq_fast_kernel<HB, IdxT, RW, PEER>;                                                      \
+    auto kern = vq_fast_kernel<HB, IdxT, RW, ANY, PEER>;                                                 \
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
     if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "%s: %s", op, cudaGetErrorString(e));           \
     launch_dependent(kern, grid, VqCta<HB>::kThreads, smem, st, p);                                                               \
@@ -355,7 +384,9 @@ int launch_vq_fast(VqParams& p, int hot_bits, int index_dtype, int variant, cuda
   const int cs = p.cs;
   const int64_t row_bytes = p.n_cb;  // uint8 codes
   if (p.code_kind != 0 || p.K > 256 || p.n_dst >= (1ll << 30)) return F2C_OK;
-  if (!(row_bytes == 4 || row_bytes == 8 || row_bytes == 16) || !aligned(codes_base, (size_t)row_bytes)) return F2C_OK;
+  // code rows of other lengths or alignments: two-level tables of this GPU here, VQ alone in fused_vq_rows.cu
+  const bool any = !(row_bytes == 4 || row_bytes == 8 || row_bytes == 16) || !aligned(codes_base, (size_t)row_bytes);
+  if (any && (peer || hot_bits == 0)) return F2C_OK;
   if (cs < 4 || cs > 128 || (128 % cs) != 0 || p.feat_dim % 4 != 0 || !aligned(p.out, 16) || !aligned(p.codebooks, 16)) return F2C_OK;
   if (!(hot_bits == 0 || hot_bits == 8 || hot_bits == 4)) return F2C_OK;
   if (hot_bits != 0) {
@@ -365,12 +396,16 @@ int launch_vq_fast(VqParams& p, int hot_bits, int index_dtype, int variant, cuda
   }
   // a column part = at most 128 columns whose codebooks fit beside the table and the code tiles
   const int sub_per_128 = 128 / cs;
-  const int roww = (int)row_bytes / 4;
+  int per_part = sub_per_128 < p.n_cb ? sub_per_128 : p.n_cb;
+  if (any) {
+    if (per_part > 16) per_part = 16;  // code bytes a lane holds
+    per_part = (int)ceil_div(p.n_cb, ceil_div(p.n_cb, per_part));  // even parts
+  }
+  const int words = (int)ceil_div(any ? per_part : row_bytes, 4), roww = words > 2 ? 4 : words;
   const int kWarps = hot_bits != 0 ? VqCta<8>::kWarps : VqCta<0>::kWarps;
   const size_t fixed = (hot_bits != 0 ? kLutBytes : 0) + (size_t)kWarps * 32 * roww * 4;
   const int spq = cs < 32 ? 32 / cs : 1;
   const int stride = cs < 32 ? 128 : cs * 4;
-  int per_part = sub_per_128 < p.n_cb ? sub_per_128 : p.n_cb;
   auto cb_bytes = [&](int n_sub) -> size_t {
     return spq > 1 ? (size_t)ceil_div(n_sub, spq) * p.K * 128 : (size_t)n_sub * p.K * cs * 4;
   };
@@ -389,10 +424,13 @@ int launch_vq_fast(VqParams& p, int hot_bits, int index_dtype, int variant, cuda
   *served = true;
 #define F2C_VQF_IDX(HB)                                                                                                            \
   if (peer)                                                                                                                        \
-    return index_dtype == F2C_I32 ? launch_rows<HB, int32_t, true>(p, roww, grid, smem, st, op)                                    \
-                                  : launch_rows<HB, int64_t, true>(p, roww, grid, smem, st, op);                                   \
-  return index_dtype == F2C_I32 ? launch_rows<HB, int32_t, false>(p, roww, grid, smem, st, op)                                     \
-                                : launch_rows<HB, int64_t, false>(p, roww, grid, smem, st, op)
+    return index_dtype == F2C_I32 ? launch_rows<HB, int32_t, false, true>(p, roww, grid, smem, st, op)                             \
+                                  : launch_rows<HB, int64_t, false, true>(p, roww, grid, smem, st, op);                            \
+  if (any)                                                                                                                         \
+    return index_dtype == F2C_I32 ? launch_rows<HB, int32_t, HB != 0, false>(p, roww, grid, smem, st, op)                          \
+                                  : launch_rows<HB, int64_t, HB != 0, false>(p, roww, grid, smem, st, op);                         \
+  return index_dtype == F2C_I32 ? launch_rows<HB, int32_t, false, false>(p, roww, grid, smem, st, op)                              \
+                                : launch_rows<HB, int64_t, false, false>(p, roww, grid, smem, st, op)
   if (hot_bits == 0) { F2C_VQF_IDX(0); }
   if (hot_bits == 8) { F2C_VQF_IDX(8); }
   F2C_VQF_IDX(4);

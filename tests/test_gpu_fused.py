@@ -298,6 +298,28 @@ def test_pipelined_vq_kernel_equals_general_kernel(capi, oracle, n_cb, K, cs, D,
                     assert all(torch.equal(a, b) for a in fast), (kw, signed)
 
 
+@pytest.mark.parametrize("n_cb,K,cs,D", [(7, 256, 16, 100), (13, 256, 8, 100), (2, 256, 64, 100), (1, 256, 64, 64), (32, 256, 8, 256), (3, 100, 32, 96), (5, 256, 128, 580)])
+@pytest.mark.parametrize("hot_bits,hot_cs", [(8, 0), (4, 56)])
+def test_two_level_code_rows_of_any_length_equal_the_general_kernel(capi, oracle, n_cb, K, cs, D, hot_bits, hot_cs):
+    """Code rows of 1 .. 32 bytes that start anywhere, in one or several column parts, from a table that starts at an odd address."""
+    rng = np.random.default_rng(n_cb * 5 + cs + hot_bits)
+    n_src, n_hot, n_dst, hcs = 701, 90, 2001, hot_cs or D
+    cbs = rng.standard_normal((n_cb, K, cs)).astype(np.float32)
+    codes = dev(rng.integers(0, 256, (n_src + 1, n_cb)).astype(np.uint8))[1:]  # some codes >= K when K < 256
+    deg = rng.integers(0, 14, n_dst)
+    deg[::11] = rng.integers(15, 80, len(deg[::11]))
+    indptr = np.concatenate([[0], np.cumsum(deg)])
+    indices = rng.integers(0, n_src, int(indptr[-1]))
+    _, cb, sq = sq_table(oracle, rng, n_hot, D, hot_bits, hcs)
+    slot = np.full(n_src, -1, np.int32)
+    slot[rng.choice(n_src, n_hot, replace=False)] = rng.permutation(n_hot).astype(np.int32)
+    for idx in (np.int64, np.int32):
+        for kw in (dict(), dict(reduce="sum", dropout=dict(p=0.3, seed=5, offset=1, training=True))):
+            run = lambda k: capi.two_level_decompress_spmm_csr(dev(sq), dev(cb), hot_bits, hcs, codes, dev(cbs), dev(slot),  # noqa: E731
+                                                               dev(indptr.astype(idx)), dev(indices.astype(idx)), D, kernel=k, **kw)
+            assert torch.equal(run("prefetch"), run("general")), (idx, kw)
+
+
 def test_config5_shape_at_scale(capi, oracle):
     """Configuration 5's codecs on a block of realistic size: D = 256, hot 2 % SQ 4 bits + VQ 4 x 64 (256 KB of
     codebooks: two column parts), 150,000 source rows, 12,000 destination rows of up to 15 neighbours.  Every kernel
