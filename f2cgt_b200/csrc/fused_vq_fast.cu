@@ -64,38 +64,10 @@ __device__ __forceinline__ uint32_t ldg_nc_u16(const void* p) {
 }
 
 template <int ROWW> struct CodeRow { uint32_t w[ROWW]; };
-template <int ROWW> __device__ __forceinline__ void load_code_row(CodeRow<ROWW>& c, const void* p) {
-  if (ROWW == 1) c.w[0] = ldg_nc_u32(p);
-  else if (ROWW == 2) { uint2 v = ldg_nc_u64(p); c.w[0] = v.x; c.w[1] = v.y; }
-  else { uint4 v = ldg_nc_u128(p); c.w[0] = v.x; c.w[1] = v.y; c.w[ROWW > 2 ? 2 : 0] = v.z; c.w[ROWW > 3 ? 3 : 0] = v.w; }
-}
-
-// A code row (ANY: the part's piece of it, which may start anywhere) as it arrives from memory.
-template <int ROWW, bool ANY> struct Arriving {
-  uint32_t w[ROWW + (ANY ? 1 : 0)];
-  uint32_t off = 0u;  // misalignment in bytes
-  __device__ __forceinline__ void clear() {
-#pragma unroll
-    for (int i = 0; i < ROWW + (ANY ? 1 : 0); ++i) w[i] = 0u;
-  }
-  __device__ __forceinline__ void fetch(const uint8_t* at, uint32_t bytes) {
-    if (ANY) {  // the aligned words that hold a byte of it
-      off = (uint32_t)(reinterpret_cast<uintptr_t>(at) & 3u);
-#pragma unroll
-      for (int i = 0; i < ROWW + (ANY ? 1 : 0); ++i) w[i] = ldg_nc_u32_if(at - off + 4 * i, 4u * i < off + bytes);
-    } else {
-      CodeRow<ROWW> c;
-      load_code_row<ROWW>(c, at);
-#pragma unroll
-      for (int i = 0; i < ROWW; ++i) w[i] = c.w[i];
-    }
-  }
-  __device__ __forceinline__ uint32_t word(int i) const { return ANY ? __funnelshift_r(w[i], w[i + (ANY ? 1 : 0)], off * 8u) : w[i]; }
-};
 
 // HB = 0: VQ only.  HB = 8 / 4: two-level with 8- / 4-bit hot rows.  ROWW = 32-bit words of one VQ code row, or (ANY) of the
 // part's piece of a row of any length and alignment: two-level shapes whose rows are not 4, 8 or 16 bytes took the general kernel
-// before (90,000 rows x 12: 100 columns in 16 117 us, now @T100@; 128 in 64 @T128@; 256 in 8 @T256@).
+// before (90,000 rows x 12: 100 columns in 16 118 us, now 74; 128 in 64 115, now 53; 256 in 8 246, now 121).
 // PEER: the three tables are row-sharded over the GPUs of the box and every shard is mapped into this process; rows of
 // other ranks are read with ordinary loads over NVLink (no collective, no staging copy, nothing waits on another rank).
 template <int HB, typename IdxT, int ROWW, bool ANY = false, bool PEER = false>
@@ -192,14 +164,14 @@ __global__ void __launch_bounds__(VqCta<HB>::kThreads, 1) vq_fast_kernel(const V
     return HB == 8 ? ldg_nc_u32(q) : ldg_nc_u16(q);
   };
   // code row and slot of source node `id`
-  auto fetch_node = [&](int64_t id, Arriving<ROWW, ANY>& c, int& sl_) {
+  auto fetch_node = [&](int64_t id, CodePiece<ROWW, ANY>& c, int& sl_) {
     if (PEER) {
       const uint32_t owner = (uint32_t)__umul64hi((unsigned long long)id, p.peer.magic_nodes);
       const uint32_t local = (uint32_t)id - owner * p.peer.rps_nodes;
-      c.fetch(p.peer.code[owner] + (uint64_t)local * ROWB, ROWB);
+      c.fetch(p.peer.code[owner] + (uint64_t)local * ROWB, ROWB, true);
       if (HB != 0) sl_ = p.peer.slot[0] != nullptr ? __ldg(p.peer.slot[owner] + local) : (id < p.n_hot ? (int)id : -1);
     } else {
-      c.fetch(codes + id * code_bytes, (uint32_t)(s_end - s_begin));
+      c.fetch(codes + id * code_bytes, (uint32_t)(s_end - s_begin), true);
       if (HB != 0) sl_ = hot_slot_of(p, id);
     }
   };
@@ -228,7 +200,7 @@ __global__ void __launch_bounds__(VqCta<HB>::kThreads, 1) vq_fast_kernel(const V
   int64_t beg1 = 0; int deg1 = 0;    // row of stage 1 -> 2
   IdxT idx2 = 0;                     // neighbour id of lane   (loaded by stage 1, read by stage 2)
   int64_t beg2 = 0; int deg2 = 0;    // row of stage 2 -> 3
-  Arriving<ROWW, ANY> code3;         // code row of lane's edge (loaded by stage 2, read by stage 3)
+  CodePiece<ROWW, ANY> code3;         // code row of lane's edge (loaded by stage 2, read by stage 3)
   int slot3 = -1;                    // slot of lane's edge     (loaded by stage 2, read by stage 3)
   int64_t beg3 = 0; int deg3 = 0;
   CodeRow<ROWW> code4;               // handed from stage 3 to stage 4
@@ -280,7 +252,7 @@ __global__ void __launch_bounds__(VqCta<HB>::kThreads, 1) vq_fast_kernel(const V
       // rows with more than 32 neighbours: further batches, fetched on the spot
       for (int64_t k0 = beg4 + 32; k0 < beg4 + deg4; k0 += 32) {
         const int cnt = (int)min((int64_t)32, beg4 + deg4 - k0);
-        Arriving<ROWW, ANY> more;
+        CodePiece<ROWW, ANY> more;
         more.clear();
         int sl_mine = -1;
         if (lane < cnt) {
@@ -288,8 +260,7 @@ __global__ void __launch_bounds__(VqCta<HB>::kThreads, 1) vq_fast_kernel(const V
           fetch_node(id, more, sl_mine);
         }
         CodeRow<ROWW> c;
-#pragma unroll
-        for (int w = 0; w < ROWW; ++w) c.w[w] = more.word(w);
+        more.join(c.w);
         __syncwarp();
         stage_codes(c, cnt);
         __syncwarp();
@@ -314,8 +285,7 @@ __global__ void __launch_bounds__(VqCta<HB>::kThreads, 1) vq_fast_kernel(const V
       const int rH = rP - 3 * W;
       const bool on = rH >= r0 && rH < n_dst;
       beg4 = beg3; deg4 = on ? deg3 : 0;
-#pragma unroll
-      for (int w = 0; w < ROWW; ++w) code4.w[w] = code3.word(w);
+      code3.join(code4.w);
       if (HB != 0) {
         slot4 = on ? slot3 : -1;
         mask4 = __ballot_sync(0xffffffffu, slot4 >= 0);

@@ -10,7 +10,7 @@
 //  * half a warp owns a destination row: a lane owns four columns of each 64-column chunk of the part, and the work per row
 //    is done for two rows at once; additions are packed (add.f32x2), the mean is one reciprocal per row and two exact
 //    corrections per column, loads are predicated instead of branched around;
-//  * lane t of a half holds neighbour t's code bytes as aligned words, joined by funnel shifts where rows start anywhere,
+//  * lane t of a half holds neighbour t's code bytes as aligned blocks, joined by shifts where rows start anywhere,
 //    and turns them into a tile [subspace][neighbour]: a lane then reads the codes of its subspace of all 16 neighbours
 //    at once.
 // Codebooks of a column part of at most 128 columns are staged once per persistent CTA, subspaces narrower than 32 columns
@@ -57,30 +57,6 @@ __device__ __forceinline__ float4 div4(float4 a, float b, float rcp) {
   return make_float4(a.x / b, a.y / b, a.z / b, a.w / b);
 }
 
-// A neighbour's code bytes of this part: WORDS aligned words (+ one when the row may start anywhere), joined on use.
-template <int WORDS, bool ANY> struct Codes {
-  uint32_t w[WORDS + (ANY ? 1 : 0)];
-  uint32_t off;  // misalignment in bytes
-  __device__ __forceinline__ void fetch(const uint8_t* at, uint32_t bytes, bool on) {
-    off = 0;
-    if (ANY) {
-      off = (uint32_t)(reinterpret_cast<uintptr_t>(at) & 3u);
-      const uint8_t* base = at - off;
-#pragma unroll
-      for (int i = 0; i < WORDS + (ANY ? 1 : 0); ++i) w[i] = ldg_nc_u32_if(base + 4 * i, on && 4u * i < off + bytes);
-    } else if (WORDS == 1) {
-      w[0] = ldg_nc_u32_if(at, on);
-    } else if (WORDS == 2) {
-      const uint2 v = ldg_nc_u64_if(at, on);
-      w[0] = v.x; w[WORDS > 1 ? 1 : 0] = v.y;
-    } else {
-      const uint4 v = ldg_nc_u128_if(at, on);
-      w[0] = v.x; w[WORDS > 1 ? 1 : 0] = v.y; w[WORDS > 2 ? 2 : 0] = v.z; w[WORDS > 3 ? 3 : 0] = v.w;
-    }
-  }
-  __device__ __forceinline__ uint32_t word(int i) const { return ANY ? __funnelshift_r(w[i], w[i + (ANY ? 1 : 0)], off * 8u) : w[i]; }
-};
-
 // NCH: 64-column chunks per part (1, 2).  WORDS: words of a row's code bytes in the part.  ANY: any alignment.  EB: bytes per code.
 template <typename IdxT, int NCH, int WORDS, bool ANY, int EB>
 __global__ void __launch_bounds__(kThreads, 1) vq_rows_kernel(const VqParams p) {
@@ -120,12 +96,12 @@ __global__ void __launch_bounds__(kThreads, 1) vq_rows_kernel(const VqParams p) 
   const int n_dst = (int)p.n_dst;
   const bool clamp = (uint32_t)K < (EB == 1 ? 256u : 65536u);
 
-  auto stage_codes = [&](const Codes<WORDS, ANY>& c, int cnt) {  // lane hl of a half holds neighbour hl
+  auto stage_codes = [&](const CodePiece<WORDS, ANY>& c, int cnt) {  // lane hl of a half holds neighbour hl
     if (hl < cnt) {
       uint32_t x[WORDS];
+      c.join(x);
 #pragma unroll
       for (int i = 0; i < WORDS; ++i) {
-        x[i] = c.word(i);
         if (clamp) {  // codes >= K read the last centroid, as in the general kernel
           uint32_t y = 0;
 #pragma unroll
@@ -182,7 +158,7 @@ __global__ void __launch_bounds__(kThreads, 1) vq_rows_kernel(const VqParams p) 
   int64_t beg1 = 0; int deg1 = 0;   // row of stage 1 -> 2
   IdxT id1 = 0;                     // this lane's neighbour   (loaded by stage 1, read by stage 2)
   int64_t beg2 = 0; int deg2 = 0;   // row of stage 2 -> 3
-  Codes<WORDS, ANY> code2;          // its code row            (loaded by stage 2, read by stage 3)
+  CodePiece<WORDS, ANY> code2;          // its code row            (loaded by stage 2, read by stage 3)
   code2.fetch(codes, 0u, false);
   for (int q = q0;; q += W) {
     const int qa = q - 3 * W;  // pair aggregated in this iteration
@@ -199,7 +175,7 @@ __global__ void __launch_bounds__(kThreads, 1) vq_rows_kernel(const VqParams p) 
       const int most = max(deg2, __shfl_xor_sync(0xffffffffu, deg2, 16));
       for (int k0 = kNb; k0 < most; k0 += kNb) {
         const int n = max(0, min(deg2 - k0, kNb));
-        Codes<WORDS, ANY> more;
+        CodePiece<WORDS, ANY> more;
         const int64_t id = hl < n ? (int64_t)indices[beg2 + k0 + hl] : 0;
         more.fetch(codes + id * row_bytes, part_bytes, hl < n);
         __syncwarp();

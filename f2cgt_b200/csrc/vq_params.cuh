@@ -70,6 +70,49 @@ __device__ __forceinline__ void stage_codebooks(unsigned char* dst, const float*
 }
 __device__ __forceinline__ void codebooks_staged() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
+// A code row (ANY: the part's piece of it, which may start anywhere) as it arrives from memory.  A piece of up to ROWW words is
+// read as the two aligned blocks of ROWW words it may touch and shifted into place by whole words, then by bytes (one load per
+// word it may touch instead: two-level, 90,000 rows x 12, 100 columns in 8 121 us against 84).
+template <int ROWW, bool ANY> struct CodePiece {
+  uint32_t w[ROWW * (ANY ? 2 : 1)];
+  uint32_t off = 0u;  // bytes before the piece
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int i = 0; i < ROWW * (ANY ? 2 : 1); ++i) w[i] = 0u;
+  }
+  __device__ __forceinline__ void block(int at, const uint8_t* q, bool on) {
+    if (ROWW == 1) w[at] = ldg_nc_u32_if(q, on);
+    else if (ROWW == 2) { const uint2 v = ldg_nc_u64_if(q, on); w[at] = v.x; w[at + (ROWW > 1 ? 1 : 0)] = v.y; }
+    else { const uint4 v = ldg_nc_u128_if(q, on); w[at] = v.x; w[at + (ROWW > 1 ? 1 : 0)] = v.y; w[at + (ROWW > 2 ? 2 : 0)] = v.z; w[at + (ROWW > 3 ? 3 : 0)] = v.w; }
+  }
+  __device__ __forceinline__ void fetch(const uint8_t* at, uint32_t bytes, bool on) {
+    if (ANY) {  // only blocks that hold a byte of it are read
+      off = (uint32_t)(reinterpret_cast<uintptr_t>(at) & (4u * ROWW - 1u));
+      block(0, at - off, on);
+      block(ANY ? ROWW : 0, at - off + 4 * ROWW, on && off + bytes > 4u * ROWW);
+    } else {
+      block(0, at, on);
+    }
+  }
+  __device__ __forceinline__ void join(uint32_t (&c)[ROWW]) const {
+    if constexpr (!ANY) {
+#pragma unroll
+      for (int i = 0; i < ROWW; ++i) c[i] = w[i];
+    } else {
+      uint32_t x[ROWW + 2];
+#pragma unroll
+      for (int i = 0; i < ROWW + 2; ++i) {  // whole words: 2 of ROWW = 4 here, then 1
+        const int j = i < 2 * ROWW ? i : 2 * ROWW - 1, k = i + 2 < 2 * ROWW ? i + 2 : 2 * ROWW - 1;
+        x[i] = ROWW == 4 && (off & 8u) ? w[k] : w[j];
+      }
+#pragma unroll
+      for (int i = 0; i < ROWW + 1; ++i) x[i] = ROWW > 1 && (off & 4u) ? x[i + 1] : x[i];
+#pragma unroll
+      for (int i = 0; i < ROWW; ++i) c[i] = __funnelshift_r(x[i], x[i + 1], (off & 3u) * 8u);
+    }
+  }
+};
+
 // Streamed (fused_vq_stream.cu) or register-prefetch (fused_vq_fast.cu) kernel for the common shapes, by `variant`
 // (an f2c_kernel value); sets *served = false (and launches nothing) when the shape is not one of theirs.
 int launch_vq_fast(VqParams& p, int hot_bits, int index_dtype, int variant, cudaStream_t st, const char* op, bool* served,
