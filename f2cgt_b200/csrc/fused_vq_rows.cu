@@ -17,8 +17,8 @@
 // interleaved in 128-byte lines: the eight lanes of a quarter-warp read eight different bank groups whatever the codes are.
 // Pipeline over the row pairs of a warp: the code rows of a pair, the ids of the next and the offsets of the one after are in
 // flight between two iterations.
-// Measured on B200, 90,000 rows x 12 neighbours, general kernel -> this one: 110 columns in slices of 8 95 -> 58 us, 200 in 32
-// 173 -> 62, 100 in 16 89 -> 40, 128 in 16 with 1024 centroids 280 -> 122; 128 columns in 8 or 32 tie with the pipelined kernel (39,
+// Measured on B200, 90,000 rows x 12 neighbours, general kernel -> this one: 110 columns in slices of 8 95 -> 51 us, 200 in 32
+// 173 -> 62, 100 in 16 89 -> 37, 128 in 16 with 1024 centroids 280 -> 122; 128 columns in 8 or 32 tie with the pipelined kernel (39,
 // 32 us), which stays for them because it starts faster (300 rows: 7.9 against 8.6 us).
 #include "sq_fused.cuh"
 #include "vq_params.cuh"
