@@ -63,8 +63,8 @@ static int launch_compress(const float* src, float* dst, const float* cb, int64_
 // slices and addresses allow it, else 1.
 // Bound by HBM: bits/8 + 4 B per element.  One exp2f per element hides behind that; a table of decoded values in shared memory
 // was never faster (27,000 x 128 8-bit codes 6.0 us with one, 4.2 without).  Row widths that are no multiple of 4 columns took one
-// thread and two 64-bit divisions per element before: 200,000 x 357 4-bit codes 288 us, now 77; x 101 8-bit 78, now 24;
-// x 255 16-bit 198, now 68.
+// thread and two 64-bit divisions per element before: 200,000 x 357 4-bit codes 288 us, now 77; x 101 8-bit 78, now 18
+// (by groups, below); x 201 1-bit 142, now 32.
 constexpr int kSqDecThreads = 512;
 
 template <int BITS, typename CodeT, int EPT>
@@ -124,6 +124,130 @@ __global__ void __launch_bounds__(kSqDecThreads, 3) sq_decompress_kernel(
     if (row + u * step < rows) emit(raw[u], op + u * ostep);
 }
 
+// Rows that are no multiple of four columns (or whose slices or codes forbid one load for four): two or four of them make a
+// super-row of whole 16-byte groups, and a thread keeps one group of it for its whole life - four columns with their own row,
+// code position and codebook row, found once.  Stores are whole and aligned whatever the width; a warp of single columns starts
+// its 128 bytes anywhere, which is two partly written sectors per store.
+//   ONE   the rows' codes follow each other without a gap, so that a group's codes are one aligned load; else four loads
+// 200,000 x 101 8-bit codes 24.4 us by columns, 18.4 by groups; x 110 8-bit 33.2, 21.1; x 255 16-bit 68, 58; x 399 8-bit 118, 94.
+template <int BITS, typename CodeT, bool ONE>
+__global__ void __launch_bounds__(kSqDecThreads, 2) sq_decompress_groups_kernel(
+    const uint8_t* __restrict__ codes, float* __restrict__ out, const float* __restrict__ codebooks, int64_t rows, int64_t row_bytes,
+    int feat_dim, int rows_per_super, int groups, int part, int supers_per_cta, int column_slice, int n_cb) {
+  dependency_wait();
+  release_dependents();
+  constexpr int B = BITS >= 8 ? 8 * (int)sizeof(CodeT) : BITS;  // stored bits of a code
+  constexpr uint32_t MASK = (1u << B) - 1u;
+  constexpr int LOADS = ONE ? 1 : 4;
+  const int sub = threadIdx.x / part;
+  const int group = blockIdx.y * part + (threadIdx.x - sub * part);
+  if (sub >= supers_per_cta || group >= groups) return;
+  int row_of[4], shift[4];
+  int64_t at[4];
+  float emin[4], scale[4], mean[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int f = 4 * group + e;
+    row_of[e] = f / feat_dim;
+    const int c = f - row_of[e] * feat_dim;
+    at[e] = row_of[e] * row_bytes + (((int64_t)c * B) >> 3);
+    shift[e] = (c * B) & 7;
+    int cb_row = c / column_slice;
+    if (cb_row >= n_cb) cb_row = n_cb - 1;
+    const float* cb = codebooks + (int64_t)cb_row * kCodebookDim;
+    emin[e] = __ldg(cb + 2);
+    scale[e] = sq_scale<BITS>(emin[e], __ldg(cb + 3));
+    mean[e] = __ldg(cb + 4);
+  }
+  struct Raw { uint32_t w[ONE ? 2 : 4]; };
+  auto fetch = [&](const uint8_t* super, int live, Raw& r) {  // the first `live` columns of the group exist
+    if constexpr (ONE) {
+      constexpr int BYTES = 4 * B / 8 > 0 ? 4 * B / 8 : 1;
+      const uint8_t* q = super + at[0];
+      if (live == 4) {
+        if (BYTES == 8) { const uint2 v = *reinterpret_cast<const uint2*>(q); r.w[0] = v.x; r.w[1] = v.y; }
+        else if (BYTES == 4) r.w[0] = *reinterpret_cast<const uint32_t*>(q);
+        else if (BYTES == 2) r.w[0] = *reinterpret_cast<const uint16_t*>(q);
+        else r.w[0] = *q;
+      } else {
+        r.w[0] = r.w[1] = 0u;
+#pragma unroll
+        for (int b = 0; b < BYTES; ++b)
+          if (8 * b < live * B) r.w[b / 4] |= (uint32_t)q[b] << (8 * (b % 4));
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (e < live) r.w[e] = B == 16 ? (uint32_t)*reinterpret_cast<const uint16_t*>(super + at[e]) : (uint32_t)super[at[e]] >> shift[e];
+    }
+  };
+  auto emit = [&](const Raw& r, float* o, int live) {
+    float v[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const uint32_t code = (ONE ? (B * e >= 32 ? r.w[1] : r.w[0]) >> ((B * e) & 31) : r.w[ONE ? 0 : e]) & MASK;
+      v[e] = sq_decode<BITS>(BITS >= 8 ? (float)(CodeT)code : (float)code, scale[e], emin[e], mean[e]);
+    }
+    if (live == 4) {
+      stg_cs_f4(o, make_float4(v[0], v[1], v[2], v[3]));
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (e < live) o[e] = v[e];
+    }
+  };
+  const int64_t step = (int64_t)gridDim.x * supers_per_cta, full = rows / rows_per_super;
+  int64_t s = (int64_t)blockIdx.x * supers_per_cta + sub;
+  const int64_t cstep = step * rows_per_super * row_bytes, ostep = step * rows_per_super * feat_dim;
+  const uint8_t* cp = codes + s * rows_per_super * row_bytes;
+  float* op = out + s * rows_per_super * feat_dim + 4 * group;
+  constexpr int kInFlight = LOADS == 1 ? 8 : 4;  // super-rows in flight per thread
+  for (; s + (kInFlight - 1) * step < full; s += kInFlight * step, cp += kInFlight * cstep, op += kInFlight * ostep) {
+    Raw r[kInFlight];
+#pragma unroll
+    for (int u = 0; u < kInFlight; ++u) fetch(cp + u * cstep, 4, r[u]);
+#pragma unroll
+    for (int u = 0; u < kInFlight; ++u) emit(r[u], op + u * ostep, 4);
+  }
+  // what is left of the full super-rows, and the rows behind them
+  Raw r[kInFlight];
+  const int rest = (int)(rows - full * rows_per_super);
+  int tail = 0;  // columns of the group that lie in those rows
+#pragma unroll
+  for (int e = 0; e < 4; ++e) tail += row_of[e] < rest ? 1 : 0;
+#pragma unroll
+  for (int u = 0; u < kInFlight; ++u) {
+    const int live = s + u * step < full ? 4 : s + u * step == full ? tail : 0;
+    if (live > 0) fetch(cp + u * cstep, live, r[u]);
+  }
+#pragma unroll
+  for (int u = 0; u < kInFlight; ++u) {
+    const int live = s + u * step < full ? 4 : s + u * step == full ? tail : 0;
+    if (live > 0) emit(r[u], op + u * ostep, live);
+  }
+}
+
+template <int BITS, typename CodeT>
+static int launch_decompress_groups(const void* codes, float* out, const float* cb, int64_t rows, int64_t row_bytes, int64_t D, int64_t cs,
+                                    cudaStream_t st, bool* served) {
+  constexpr int B = BITS >= 8 ? 8 * (int)sizeof(CodeT) : BITS;
+  const int per = D % 4 == 0 ? 1 : D % 2 == 0 ? 2 : 4;
+  const int64_t groups = D * per / 4, supers = ceil_div(rows, per);
+  const int sms = current_sm_count();
+  const Lanes ln = lanes_of_rows(groups, supers, sms, kSqDecThreads);
+  const int64_t grid = std::min(ceil_div(supers, ln.rows_per_cta), ceil_div((int64_t)sms * 2 * kSqDecThreads / ln.threads, ln.parts));
+  const bool one = 4 * B % 8 == 0 && row_bytes * 8 == D * B && aligned(codes, 4 * B / 8 > 0 ? 4 * B / 8 : 1);
+  // Fewer groups than columns means fewer threads, so it takes some work before whole stores pay: 27,000 x 101 8-bit codes 5.2 us
+  // against 4.7 by columns, x 255 16-bit 7.8 against 8.4.  Four loads per group pay later and only for the narrowest codes
+  // (200,000 x 357 4-bit codes 94 us against 77; x 333 2-bit 79 against 87; 27,000 x 201 1-bit 7.1 against 6.8).
+  *served = aligned(out, 16) && rows * D >= (one ? 3 << 20 : 8 << 20) && (one || BITS <= 2);
+  if (!*served) return F2C_OK;
+  auto kern = one ? sq_decompress_groups_kernel<BITS, CodeT, true> : sq_decompress_groups_kernel<BITS, CodeT, BITS <= 2 ? false : true>;
+  launch_dependent(kern, dim3((unsigned)grid, (unsigned)ln.parts), ln.threads, 0, st, (const uint8_t*)codes, out, cb, rows, row_bytes, (int)D, per,
+                   (int)groups, ln.part, ln.rows_per_cta, (int)cs, (int)ceil_div(D, cs));
+  return check_launch("sq_decompress");
+}
+
 template <int BITS, typename CodeT, int EPT>
 static int launch_decompress_ept(const void* codes, float* out, const float* cb, int64_t rows, int64_t row_bytes, int64_t D, int64_t cs,
                                  cudaStream_t st) {
@@ -144,8 +268,11 @@ static int launch_decompress(const void* codes, float* out, const float* cb, int
   constexpr int LOAD_BYTES = BITS >= 8 ? 4 * (int)sizeof(CodeT) : (BITS == 4 ? 2 : 1);
   const int64_t row_bytes = src_dim * (int64_t)sizeof(CodeT);
   const bool vec = D % 4 == 0 && aligned(out, 16) && aligned(codes, LOAD_BYTES) && row_bytes % LOAD_BYTES == 0 && (cs >= D || cs % 4 == 0);
-  return vec ? launch_decompress_ept<BITS, CodeT, 4>(codes, out, cb, rows, row_bytes, D, cs, st)
-             : launch_decompress_ept<BITS, CodeT, 1>(codes, out, cb, rows, row_bytes, D, cs, st);
+  if (vec) return launch_decompress_ept<BITS, CodeT, 4>(codes, out, cb, rows, row_bytes, D, cs, st);
+  bool served = false;
+  const int rc = launch_decompress_groups<BITS, CodeT>(codes, out, cb, rows, row_bytes, D, cs, st, &served);
+  if (served || rc) return rc;
+  return launch_decompress_ept<BITS, CodeT, 1>(codes, out, cb, rows, row_bytes, D, cs, st);
 }
 
 }  // namespace f2c

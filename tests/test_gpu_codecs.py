@@ -169,7 +169,8 @@ def test_vq_decompress_streaming_kernel(capi, oracle, n_cb, K, cs, D):
 
 
 @pytest.mark.parametrize("bits", [1, 2, 4, 8, 16])
-@pytest.mark.parametrize("rows,D,cs", [(1, 357, 360), (4099, 357, 184), (9001, 101, 104), (5003, 200, 56), (4500, 3, 8), (4097, 1030, 520), (30011, 36, 40)])
+@pytest.mark.parametrize("rows,D,cs", [(1, 357, 360), (4099, 357, 184), (9001, 101, 104), (5003, 200, 56), (4500, 3, 8), (4097, 1030, 520), (30011, 36, 40),
+                                        (52003, 101, 40), (40002, 110, 56), (131075, 71, 72), (3150001, 1, 8)])
 def test_sq_decompress_rows_of_any_width(capi, oracle, bits, rows, D, cs):
     """Widths that leave threads of a CTA idle, that are cut into column parts, whose codes straddle bytes or slices; one row, a
     last batch of rows that is not full; codes and output at an odd address."""
