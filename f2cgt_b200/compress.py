@@ -18,6 +18,7 @@ initialisations are seeded per column slice, so the split artefact equals the si
 ``save`` / ``load`` write and read ``compression_meta.pt``, ``compression_data.pt`` and ``seeds_compression_data.pt``.
 """
 import ctypes
+import functools
 import os
 
 import torch
@@ -72,6 +73,11 @@ def _ranks(n):
 # A slice's three passes each end in one CTA that works alone, so the slices of a call run side by side, on this many streams
 # (100,000 x 110 in four slices: 406 us a call on one stream, 373 on four, of which the host takes 250).
 _STATISTICS_STREAMS = 4
+
+
+@functools.lru_cache(maxsize=None)
+def _side_streams(device_index):
+    return tuple(torch.cuda.Stream(device_index) for _ in range(_STATISTICS_STREAMS))
 
 
 def _statistics(x, rows, n_rows, col, width, out, workspace, stream=None):
@@ -172,7 +178,8 @@ def sq_compress_features(features, target_bits, column_slice, hotness=None, samp
         stats = torch.empty((s_hi - s_lo, 5), dtype=torch.float64, device=features.device)
         main = torch.cuda.current_stream(features.device)
         lanes = min(_STATISTICS_STREAMS, s_hi - s_lo)
-        streams = [main] if lanes <= 1 else [torch.cuda.Stream(features.device) for _ in range(lanes)]
+        streams = (main,) if lanes <= 1 else _side_streams(main.device_index)[:lanes]
+        ready = None
         ws = torch.empty((max(lanes, 1), (lib.f2c_sq_statistics_workspace() + 255) // 256 * 256), dtype=torch.uint8, device=features.device)
         samples = []  # alive until the host has read the results
     for i in range(s_lo, s_hi):
@@ -185,7 +192,10 @@ def sq_compress_features(features, target_bits, column_slice, hotness=None, samp
             continue
         lane = len(pending) % lanes
         if streams[lane] is not main:
-            streams[lane].wait_stream(main)  # the sample's row numbers
+            if ready is None or idx is not None:
+                ready = main.record_event()  # the features, the workspaces, the sample's row numbers
+            if idx is not None or len(pending) < lanes:
+                streams[lane].wait_event(ready)
         _statistics(features, idx, n_sample, lo, hi - lo, stats[i - s_lo], ws[lane], streams[lane])
         samples.append(idx)
         pending.append((i - s_lo, n_sample * (hi - lo)))
