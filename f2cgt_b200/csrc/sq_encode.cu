@@ -11,10 +11,14 @@
 // expression (the bound exceeds a hundredth of a level), 1-bit codes are a sign test.
 //
 // Rows whose length is a multiple of 4 columns are read as float4 by threads that keep their columns (and so their codebook
-// row's constants) for life; other rows go through shared memory in whole tiles, so that their loads are aligned too.
+// row's constants) for life, other rows as groups over super-rows or, where codes do not end with a row, through shared memory
+// in whole tiles, so that their loads are aligned too.
 // Measured on B200 (fp32 in + codes out): 1,000,000 x 128 at 1 / 2 / 4 / 8 / 16 bits 76 / 106 / 113 / 141 / 301 us = 6.9 / 5.1 / 5.1 /
 // 4.5 / 2.5 TB/s (4 bits as three passes before: 800 us); 500,001 x 117 58 / 125 / 129 / 154 / 219 us through the tiles.  Two rows in
 // flight per thread and four CTAs per SM: more rows in flight cost registers, i.e. warps (4 rows, two CTAs: +9 %).
+#include <algorithm>
+
+#include "row_lanes.cuh"
 #include "sq_encode.cuh"
 
 namespace f2c {
@@ -44,7 +48,7 @@ template <int BITS>
 __device__ void build_params(float* par, const float* __restrict__ codebooks, int n_cb) {
   if (BITS != 1 && BITS != 16) {
     constexpr float drange = (float)(1 << (BITS - 1));
-    for (int row = threadIdx.x; row < n_cb; row += kThreads) {
+    for (int row = threadIdx.x; row < n_cb; row += blockDim.x) {
       const float* cb = codebooks + row * kCodebookDim;
       const float fmin = __ldg(cb), fmax = __ldg(cb + 1), emin = __ldg(cb + 2), emax = __ldg(cb + 3);
       const float scale = drange / (emax - emin);
@@ -177,6 +181,80 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) encode_vec_kernel(const 
   }
 }
 
+// Codes of 4, 8 or 16 bits in rows that are no multiple of four columns but follow each other without a gap (4 bits: an even
+// number of columns): two or four rows make a super-row of whole 16-byte groups of features, whose four codes are one aligned
+// store.  A thread keeps its group - four columns with their codebook rows - for its whole life and walks over super-rows, two
+// in flight (rows through shared memory in tiles: 500,001 x 117 8-bit codes 154 us, now @E8@; 16-bit 219, now @E16@;
+// 100,000 x 110 8-bit 45, now @E110@).
+constexpr int kGroupThreads = 512;
+
+template <int BITS>
+__global__ void __launch_bounds__(kGroupThreads, 2) encode_groups_kernel(const Args a, int rows_per_super, int groups, int part, int supers_per_cta) {
+  dependency_wait();
+  release_dependents();
+  extern __shared__ float par[];
+  build_params<BITS>(par, a.codebooks, a.n_cb);
+  const int sub = (int)threadIdx.x / part, group = (int)blockIdx.y * part + ((int)threadIdx.x - sub * part);
+  if (sub >= supers_per_cta || group >= groups) return;
+  int row_of_column[4], book[4];
+  Row prow[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    row_of_column[e] = (4 * group + e) / a.dim;
+    book[e] = (4 * group + e - row_of_column[e] * a.dim) / a.column_slice;
+    prow[e] = BITS == 16 ? Row{} : row_of(par + book[e] * kParams);
+  }
+  auto codes_of = [&](float4 x, uint32_t (&c)[4]) {
+    const float v[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float* cb = a.codebooks + book[e] * kCodebookDim;
+      float worst = 0.0f;
+      c[e] = encode_fast<BITS>(v[e], prow[e], cb, worst);
+      if (BITS != 16 && worst >= prow[e].limit) c[e] = encode_exact<BITS>(v[e], cb);
+      c[e] &= (1u << BITS) - 1u;
+    }
+  };
+  const int64_t step = (int64_t)gridDim.x * supers_per_cta, full = a.rows / rows_per_super;
+  const int64_t super = (int64_t)rows_per_super * a.dim;  // columns
+  int64_t s = (int64_t)blockIdx.x * supers_per_cta + sub;
+  constexpr int F = 2;  // super-rows in flight
+  for (; s < full; s += F * step) {
+    float4 x[F];
+#pragma unroll
+    for (int f = 0; f < F; ++f)
+      x[f] = s + f * step < full ? __ldcs(reinterpret_cast<const float4*>(a.x + (s + f * step) * super) + group) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int f = 0; f < F; ++f) {
+      if (s + f * step >= full) break;
+      uint32_t c[4];
+      codes_of(x[f], c);
+      unsigned char* o = a.out + ((s + f * step) * super + 4 * group) * BITS / 8;
+      if (BITS == 16) *reinterpret_cast<uint2*>(o) = make_uint2(c[0] | (c[1] << 16), c[2] | (c[3] << 16));
+      else if (BITS == 8) *reinterpret_cast<uint32_t*>(o) = c[0] | (c[1] << 8) | (c[2] << 16) | (c[3] << 24);
+      else *reinterpret_cast<uint16_t*>(o) = (uint16_t)(c[0] | (c[1] << 4) | (c[2] << 8) | (c[3] << 12));
+    }
+  }
+  // the rows behind the full super-rows: one thread per group of the super-row that they begin
+  const int rest = (int)(a.rows - full * rows_per_super);
+  if (rest == 0 || blockIdx.x != 0 || sub != 0) return;
+  int live = 0;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) live += row_of_column[e] < rest ? 1 : 0;
+  if (live == 0) return;
+  const float* q = a.x + full * super + 4 * group;
+  uint32_t c[4];
+  codes_of(make_float4(q[0], live > 1 ? q[1] : 0.f, live > 2 ? q[2] : 0.f, live > 3 ? q[3] : 0.f), c);
+  unsigned char* o = a.out + (full * super + 4 * group) * BITS / 8;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    if (e >= live) break;
+    if (BITS == 16) reinterpret_cast<uint16_t*>(o)[e] = (uint16_t)c[e];
+    else if (BITS == 8) o[e] = (unsigned char)c[e];
+    else if (e % 2 == 1) o[e / 2] = (unsigned char)(c[e - (e > 0)] | (c[e] << 4));  // an even number is live
+  }
+}
+
 // Any row length up to kTileFloats / 4: tiles of `tile_rows` rows (a multiple of 4, so that a tile starts on a 16-byte boundary
 // of an aligned matrix) are copied to shared memory, encoded byte by byte into a second tile, and copied out.
 constexpr int kTileFloats = 6144;
@@ -251,6 +329,18 @@ static int launch_encode(Args a, cudaStream_t st, const char* op) {
     if (grid > cap) grid = cap;
     launch_dependent(kern, (unsigned)grid, kThreads, par_bytes, st, a);
     return check_launch(op);
+  }
+  if constexpr (BITS == 4 || BITS == 8 || BITS == 16) {
+    if (a.dim * BITS % 8 == 0 && aligned(a.x, 16) && aligned(a.out, BITS / 2)) {
+      const int per = a.dim % 4 == 0 ? 1 : a.dim % 2 == 0 ? 2 : 4;
+      const int64_t groups = (int64_t)a.dim * per / 4, supers = ceil_div(a.rows, per);
+      const int sms = current_sm_count();
+      const Lanes ln = lanes_of_rows(groups, supers, sms, kGroupThreads);
+      const int64_t grid = std::min(ceil_div(supers, ln.rows_per_cta), ceil_div((int64_t)sms * 2 * kGroupThreads / ln.threads, ln.parts));
+      launch_dependent(encode_groups_kernel<BITS>, dim3((unsigned)grid, (unsigned)ln.parts), ln.threads, par_bytes, st, a, per, (int)groups,
+                       ln.part, ln.rows_per_cta);
+      return check_launch(op);
+    }
   }
   F2C_REQUIRE(aligned(a.out, 4), F2C_ERR_INVALID, "%s: the codes must be 4-byte aligned", op);
   int tile_rows = kTileFloats / a.dim / 4 * 4;

@@ -128,6 +128,13 @@ def test_one_pass_encoder_equals_the_separate_operators(capi, bits, rows, D, cs)
         assert torch.equal(got, want), (kind, int((got != want).sum()))
 
 
+@pytest.mark.parametrize("bits", [4, 8, 16])
+@pytest.mark.parametrize("rows,D,cs", [(400_003, 101, 40), (300_001, 110, 56), (60_002, 357, 96), (700_002, 3, 8)])
+def test_one_pass_encoder_groups_over_several_rows(capi, bits, rows, D, cs):
+    """Odd widths with several super-rows per thread and rows left over behind the last whole one."""
+    test_one_pass_encoder_equals_the_separate_operators(capi, bits, rows, D, cs)
+
+
 @pytest.mark.parametrize("rows,D,col,width,sampled", [(1, 1, 0, 1, False), (2, 3, 1, 2, False), (1000, 128, 0, 128, True), (5000, 100, 96, 4, True),
                                                       (33, 7, 2, 5, True), (70_000, 64, 32, 32, True)])
 def test_sample_statistics_equal_a_sort(capi, rows, D, col, width, sampled):
