@@ -14,7 +14,7 @@
 // row's constants) for life, other rows as groups over super-rows or, where codes do not end with a row, through shared memory
 // in whole tiles, so that their loads are aligned too.
 // Measured on B200 (fp32 in + codes out): 1,000,000 x 128 at 1 / 2 / 4 / 8 / 16 bits 76 / 106 / 113 / 141 / 301 us = 6.9 / 5.1 / 5.1 /
-// 4.5 / 2.5 TB/s (4 bits as three passes before: 800 us); 500,001 x 117 58 / 125 / 129 / 154 / 219 us through the tiles.  Two rows in
+// 4.5 / 2.5 TB/s (4 bits as three passes before: 800 us); 500,001 x 117 58 / 125 / 129 us at 1 / 2 / 4 bits through the tiles.  Two rows in
 // flight per thread and four CTAs per SM: more rows in flight cost registers, i.e. warps (4 rows, two CTAs: +9 %).
 #include <algorithm>
 
@@ -184,8 +184,8 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) encode_vec_kernel(const 
 // Codes of 4, 8 or 16 bits in rows that are no multiple of four columns but follow each other without a gap (4 bits: an even
 // number of columns): two or four rows make a super-row of whole 16-byte groups of features, whose four codes are one aligned
 // store.  A thread keeps its group - four columns with their codebook rows - for its whole life and walks over super-rows, two
-// in flight (rows through shared memory in tiles: 500,001 x 117 8-bit codes 154 us, now @E8@; 16-bit 219, now @E16@;
-// 100,000 x 110 8-bit 45, now @E110@).
+// in flight (rows through shared memory in tiles: 500,001 x 117 8-bit codes 154 us, now 114; 16-bit 219, now 154;
+// 100,000 x 110 8-bit 45, now 16.  One branch for a group of four instead of one per column: 8 bits 130).
 constexpr int kGroupThreads = 512;
 
 template <int BITS>
