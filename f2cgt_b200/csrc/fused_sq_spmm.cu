@@ -554,7 +554,11 @@ static int launch_sq_spmm(const void* codes, int code_dtype, const float* codebo
       const Plan wide = plan(true);
       if (wide.ok && (!q.ok || wide.parts < q.parts)) { q = wide; across = true; }
     }
-    if ((BITS < 16 || n_dst * D <= 1ll << 18) && q.ok) {
+    // Three parts or more of 8-bit columns that fill less than two thirds of their lanes read the ids and offsets too often for
+    // their work: 30,000 rows of 255 columns 102 us against 97 of the general kernel, whose warps fill 8 x 32 columns; of 262, 99
+    // against 107; 6,000 rows, where the general kernel's launch counts more, 24 against 28.
+    const bool thin = BITS == 8 && q.parts >= 3 && 3 * D < 2 * q.parts * ((int64_t)kLaneCols << q.logG) && n_dst * D >= 3ll << 20;
+    if ((BITS < 16 || n_dst * D <= 1ll << 18) && q.ok && !thin) {
       SqParams p{};
       p.codes = (const uint8_t*)codes; p.codebooks = codebooks; p.indptr = indptr; p.indices = indices; p.out = out;
       p.n_dst = n_dst; p.row_bytes = (uint32_t)row_bytes; p.feat_dim = (int)D; p.column_slice = (int)(slices > 1 ? cs : D);
