@@ -320,6 +320,18 @@ def test_two_level_code_rows_of_any_length_equal_the_general_kernel(capi, oracle
             assert torch.equal(run("prefetch"), run("general")), (idx, kw)
 
 
+@pytest.mark.parametrize("D,cs", [(241, 248), (255, 128), (256 + 1, 264)])
+def test_fused_sq_wide_ragged_rows_on_either_side_of_two_thirds(capi, oracle, D, cs):
+    """8-bit rows of three column parts, fewer (general kernel) and more than two thirds of whose lanes hold columns: decode, then mean."""
+    rng = np.random.default_rng(D)
+    n_src, n_dst = 3001, 13_100
+    _, cb, sq = sq_table(oracle, rng, n_src, D, 8, cs)
+    indptr = np.concatenate([[0], np.cumsum(rng.integers(0, 14, n_dst))]).astype(np.int64)
+    indices = rng.integers(0, n_src, int(indptr[-1])).astype(np.int64)
+    got = capi.sq_decompress_spmm_csr(dev(sq), dev(cb), dev(indptr), dev(indices), 8, cs, D)
+    assert torch.equal(got, capi.spmm_csr(capi.sq_decompress(dev(sq), dev(cb), 8, cs, D), dev(indptr), dev(indices)))
+
+
 def test_config5_shape_at_scale(capi, oracle):
     """Configuration 5's codecs on a block of realistic size: D = 256, hot 2 % SQ 4 bits + VQ 4 x 64 (256 KB of
     codebooks: two column parts), 150,000 source rows, 12,000 destination rows of up to 15 neighbours.  Every kernel
