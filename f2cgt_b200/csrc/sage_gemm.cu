@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(kThreads, 1) sage_forward_kernel(const __grid_
             float a = __uint_as_float(r1[j]);
             if (p.bias != nullptr) a += bias_s[c0 + j];
             a += __uint_as_float(r2[j]);
-            v[e] = p.relu ? fmaxf(a, 0.f) : a;
+            v[e] = p.relu && a <= 0.f ? 0.f : a;  // a NaN stays one, as in torch.relu
           }
           *reinterpret_cast<float4*>(epi + lane * 36 + 4 * q) = make_float4(v[0], v[1], v[2], v[3]);
         }

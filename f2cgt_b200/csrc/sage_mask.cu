@@ -1,8 +1,10 @@
-// Gradient through dropout and ReLU, and the bias gradient behind them, in one pass: dy = h > 0 ? scale * g : 0 where h is the
-// layer's output after both (zero exactly where the ReLU or the dropout made it so), db += column sums of dy.  As torch
-// operators this is a mask product, a ReLU backward and a vector-matrix product: 36 us for 59,000 x 128 on a B200.
-// HBM bound: two matrices in, one out.  A thread keeps four columns for life, so its column sums stay in registers; a CTA adds
-// them up in shared memory and to db once.  Measured: 16 us (5.7 TB/s).
+// Gradient through dropout and ReLU, and the bias gradient behind them, in one pass: dy = h <= 0 ? 0 : g * keep * scale where h is
+// what the ReLU gave and keep the mask (0 or 1) that dropout drew, db += column sums of dy.  The products and the comparison are
+// torch's (native_dropout_backward, threshold_backward), so a NaN or an infinity in h or g goes where it goes there: a NaN
+// activation passes its gradient, a dropped element of an infinite gradient is NaN.
+// As torch operators this is a mask product, a ReLU backward and a vector-matrix product: 36 us for 59,000 x 128 on a B200.
+// HBM bound: two matrices and the mask in, one matrix out.  A thread keeps four columns for life, so its column sums stay in
+// registers; a CTA adds them up in shared memory and to db once.
 #include "common.cuh"
 
 namespace f2c {
@@ -10,10 +12,12 @@ namespace {
 
 constexpr int kThreads = 256;
 
-// MASK = false: only the column sums of g
-template <bool VEC, bool MASK>
-__global__ void __launch_bounds__(kThreads) sage_mask_kernel(const float* __restrict__ g, const float* __restrict__ h, float scale,
-                                                             float* __restrict__ dy, float* __restrict__ db, int64_t rows, int n, int units) {
+enum Mask { kSums, kRelu, kReluDropout };  // only the column sums of g; h; h and keep
+
+template <bool VEC, Mask MASK>
+__global__ void __launch_bounds__(kThreads) sage_mask_kernel(const float* __restrict__ g, const float* __restrict__ h, const uint8_t* __restrict__ keep,
+                                                             float scale, float* __restrict__ dy, float* __restrict__ db, int64_t rows, int n,
+                                                             int units) {
   dependency_wait();
   release_dependents();
   constexpr int E = VEC ? 4 : 1;
@@ -23,6 +27,10 @@ __global__ void __launch_bounds__(kThreads) sage_mask_kernel(const float* __rest
   const int lanes = units < kThreads ? kThreads / units : 1;  // rows a CTA works on at a time
   const int local = units < kThreads ? (int)threadIdx.x / units : 0;
   const int64_t step = (int64_t)gridDim.x * lanes;
+  auto masked = [&](float v, float b, float k) {
+    if (MASK == kReluDropout) v *= k;
+    return b <= 0.f ? 0.f : v * scale;
+  };
   for (int u = units < kThreads ? (int)threadIdx.x - local * units : (int)threadIdx.x; u < units && local < lanes; u += kThreads) {
     float s[E] = {};
     const int c = u * E;
@@ -31,16 +39,18 @@ __global__ void __launch_bounds__(kThreads) sage_mask_kernel(const float* __rest
       const int64_t at = r * n + c;
       if (VEC) {
         float4 v = __ldcs(reinterpret_cast<const float4*>(g + at));
-        if (MASK) {
+        if (MASK != kSums) {
           const float4 b = __ldcs(reinterpret_cast<const float4*>(h + at));
-          v = make_float4(b.x > 0.f ? v.x * scale : 0.f, b.y > 0.f ? v.y * scale : 0.f, b.z > 0.f ? v.z * scale : 0.f, b.w > 0.f ? v.w * scale : 0.f);
+          uchar4 k = make_uchar4(1, 1, 1, 1);
+          if (MASK == kReluDropout) k = __ldcs(reinterpret_cast<const uchar4*>(keep + at));
+          v = make_float4(masked(v.x, b.x, k.x), masked(v.y, b.y, k.y), masked(v.z, b.z, k.z), masked(v.w, b.w, k.w));
           *reinterpret_cast<float4*>(dy + at) = v;
         }
         s[0] += v.x; s[E > 1 ? 1 : 0] += v.y; s[E > 2 ? 2 : 0] += v.z; s[E > 3 ? 3 : 0] += v.w;
       } else {
         float v = g[at];
-        if (MASK) {
-          v = h[at] > 0.f ? v * scale : 0.f;
+        if (MASK != kSums) {
+          v = masked(v, h[at], MASK == kReluDropout ? keep[at] : 1);
           dy[at] = v;
         }
         s[0] += v;
@@ -62,20 +72,26 @@ __global__ void __launch_bounds__(kThreads) sage_mask_kernel(const float* __rest
 
 using namespace f2c;
 
-extern "C" int f2c_sage_mask(const float* g, const float* h, float scale, float* dy, float* db, int64_t rows, int64_t n, void* stream) {
+extern "C" int f2c_sage_mask_dropout(const float* g, const float* h, const uint8_t* keep, float scale, float* dy, float* db, int64_t rows, int64_t n,
+                                     void* stream) {
   const char* op = "sage_mask";
   F2C_REQUIRE(rows >= 0 && n >= 0 && n <= 8192, F2C_ERR_LIMIT, "%s: bad shape", op);
   if (rows * n == 0) return F2C_OK;
-  F2C_REQUIRE(g && (h != nullptr ? dy != nullptr : db != nullptr), F2C_ERR_INVALID, "%s: null pointer", op);
-  const bool vec = n % 4 == 0 && aligned(g, 16) && aligned(h, 16) && aligned(dy, 16);
+  F2C_REQUIRE(g && (h != nullptr ? dy != nullptr : db != nullptr && keep == nullptr), F2C_ERR_INVALID, "%s: null pointer", op);
+  const bool vec = n % 4 == 0 && aligned(g, 16) && aligned(h, 16) && aligned(dy, 16) && aligned(keep, 4);
   const int units = (int)(vec ? n / 4 : n);
   const int lanes = units < kThreads ? kThreads / units : 1;
   int64_t grid = ceil_div(rows, (int64_t)lanes * 4);
   if (grid > 8 * current_sm_count()) grid = 8 * current_sm_count();
-  auto kern = h != nullptr ? (vec ? sage_mask_kernel<true, true> : sage_mask_kernel<false, true>)
-                           : (vec ? sage_mask_kernel<true, false> : sage_mask_kernel<false, false>);
-  launch_dependent(kern, (unsigned)grid, kThreads, (size_t)n * 4, (cudaStream_t)stream, g, h, scale, dy, db, rows, (int)n, units);
+  auto kern = h == nullptr      ? (vec ? sage_mask_kernel<true, kSums> : sage_mask_kernel<false, kSums>)
+              : keep == nullptr ? (vec ? sage_mask_kernel<true, kRelu> : sage_mask_kernel<false, kRelu>)
+                                : (vec ? sage_mask_kernel<true, kReluDropout> : sage_mask_kernel<false, kReluDropout>);
+  launch_dependent(kern, (unsigned)grid, kThreads, (size_t)n * 4, (cudaStream_t)stream, g, h, keep, scale, dy, db, rows, (int)n, units);
   return check_launch(op);
+}
+
+extern "C" int f2c_sage_mask(const float* g, const float* h, float scale, float* dy, float* db, int64_t rows, int64_t n, void* stream) {
+  return f2c_sage_mask_dropout(g, h, nullptr, scale, dy, db, rows, n, stream);
 }
 
 namespace f2c {

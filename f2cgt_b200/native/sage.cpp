@@ -136,13 +136,13 @@ struct SageBackward : public torch::autograd::Node {
   Net net;
   std::vector<SavedVariable> weights;   // per layer: self, neigh, bias
   std::vector<at::Tensor> x1, x2;       // inputs of the layers' products
-  std::vector<at::Tensor> out;          // outputs after ReLU and dropout (all layers but the last)
+  std::vector<at::Tensor> out, active, keep;  // all layers but the last: output, what the ReLU gave, dropout's mask (undefined: none)
   bool released = false;
 
   std::string name() const override { return "SageBackward"; }
   void release_variables() override {
     released = true;
-    weights.clear(); x1.clear(); x2.clear(); out.clear();
+    weights.clear(); x1.clear(); x2.clear(); out.clear(); active.clear(); keep.clear();
   }
 
   variable_list apply(variable_list&& grads) override {
@@ -183,7 +183,7 @@ struct SageBackward : public torch::autograd::Node {
     zeros.run(st);
     Beside& side = beside(given.device().index());
     bool forked = false;
-    std::vector<at::Tensor> keep;  // what the side stream reads, until the streams have joined
+    std::vector<at::Tensor> read_beside;  // what the side stream reads, until the streams have joined
     int64_t bias_at = 0;
     for (size_t i = L; i-- > 0;) {
       const Layer& l = net.layers[i];
@@ -197,7 +197,8 @@ struct SageBackward : public torch::autograd::Node {
       at::Tensor dy = g;
       if (i + 1 < L) {
         dy = empty({m, n}, at::kFloat, g.device());
-        checked = f2c_sage_mask(f32(g), f32(out[i]), (float)net.scale(), f32(dy), db.defined() ? f32(db) : nullptr, m, n, st);
+        checked = f2c_sage_mask_dropout(f32(g), f32(active[i]), keep[i].defined() ? (const uint8_t*)keep[i].data_ptr() : nullptr, (float)net.scale(),
+                                        f32(dy), db.defined() ? f32(db) : nullptr, m, n, st);
       } else if (db.defined()) {
         checked = f2c_sage_mask(f32(dy), nullptr, 1.0f, nullptr, f32(db), m, n, st);
       }
@@ -212,7 +213,7 @@ struct SageBackward : public torch::autograd::Node {
         if (i > 0) product(net, d_self, dy, true, x1[i], false);
         side.join.record(*side.stream);
         forked = true;
-        keep.push_back(dy);
+        read_beside.push_back(dy);
       } else {
         product(net, d_nb, dy, true, x2[i], false);
         if (i > 0) product(net, d_self, dy, true, x1[i], false);
@@ -300,11 +301,20 @@ PyObject* sage_net(PyObject*, PyObject* const* a, Py_ssize_t n) {
                                  l.rows, h.size(1), F2C_MEAN, st);
         }
         h = layer_forward(net, x1, x2, &w[3 * i], l, !last, record, st);
-        if (!last && net.p > 0) h = net.p < 1 && h.numel() > 0 ? std::get<0>(at::native_dropout(h, net.p, true)) : at::dropout(h, net.p, true);
+        const at::Tensor active = h;
+        at::Tensor keep;
+        if (!last && net.p > 0) {
+          if (net.p < 1 && h.numel() > 0) std::tie(h, keep) = at::native_dropout(h, net.p, true);
+          else h = at::dropout(h, net.p, true);
+        }
         if (record) {
           node->x1.push_back(x1);
           node->x2.push_back(x2);
-          if (!last) node->out.push_back(h);
+          if (!last) {
+            node->out.push_back(h);
+            node->active.push_back(active);
+            node->keep.push_back(keep);
+          }
         }
       }
       if (h.size(0) > net.layers[L - 1].rows) h = h.narrow(0, 0, net.layers[L - 1].rows);

@@ -133,14 +133,19 @@ int f2c_spmm_csr_backward(const float* grad_out, const void* indptr, const void*
 
 /* Forward product of a SAGE layer (fc_self and fc_neigh of examples/conv.py:62-76 together), fp32 storage, tf32 operands
  * (rounded to nearest), fp32 accumulation: y [m, n] = (x1 [m, k] w1 [n, k]^T + bias [n]) + x2 w2^T (bias may be NULL), then
- * max(0, .) when relu != 0.  Row-major, operands 16-byte aligned, k % 4 == 0 (else F2C_ERR_UNSUPPORTED). */
+ * max(0, .) when relu != 0 (a NaN stays NaN).  Row-major, operands 16-byte aligned, k % 4 == 0 (else F2C_ERR_UNSUPPORTED). */
 int f2c_sage_forward(const float* x1, const float* x2, const float* w1, const float* w2, const float* bias, float* y, int64_t m,
                      int64_t n, int64_t k, int relu, void* stream);
 
-/* Gradient through dropout and ReLU of a layer whose output after both is h: dy = h > 0 ? scale * g : 0 (scale = what dropout
- * multiplies survivors with), and db [n] += column sums of dy (db may be NULL; no fixed order).  g, h, dy [rows, n] f32.
- * h == NULL: dy is not written, db += column sums of g. */
+/* Gradient through ReLU and dropout of a layer, and its bias gradient: dy = h <= 0 ? 0 : g * keep * scale (h = what the ReLU
+ * gave, keep [rows, n] = 0 where dropout dropped and 1 elsewhere, scale = what it multiplied survivors with), and db [n] += column
+ * sums of dy (db may be NULL; no fixed order).  g, h, dy [rows, n] f32.  A NaN in h passes its gradient, and NaN or infinite
+ * gradients of dropped elements give NaN, as in torch.  h == NULL (then keep == NULL): dy is not written, db += column sums of g.
+ * f2c_sage_mask: keep all ones (h may then also be the output behind dropout, which is zero where dropout dropped, for
+ * finite gradients). */
 int f2c_sage_mask(const float* g, const float* h, float scale, float* dy, float* db, int64_t rows, int64_t n, void* stream);
+int f2c_sage_mask_dropout(const float* g, const float* h, const uint8_t* keep, float scale, float* dy, float* db, int64_t rows,
+                          int64_t n, void* stream);
 
 /* Set up to 32 ranges of device memory (whole 4-byte words) to zero in one launch; the arrays are HOST arrays. */
 int f2c_zero_ranges(void* const* ranges_host, const int64_t* bytes_host, int count, void* stream);

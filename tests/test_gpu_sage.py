@@ -324,3 +324,104 @@ def test_network_as_one_node_equals_the_layers(capi, tf32, product, D, hidden, c
             assert a.shape == b.shape and float((a - b).norm() / b.norm()) < tol
     finally:
         torch.backends.cuda.matmul.allow_tf32 = before
+
+
+@pytest.mark.parametrize("m,n,k", [(5, 7, 64), (300, 128, 128), (129, 172, 100)])
+def test_layer_product_keeps_not_a_number(capi, m, n, k):
+    """ReLU as torch.relu has it: a NaN sum stays NaN, infinities keep their sign's side."""
+    from f2cgt_b200 import ops
+    from f2cgt_b200._lib import check, lib
+    g = torch.Generator(device="cuda").manual_seed(m)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    x1, x2, w1, w2, b = rnd(m, k), rnd(m, k), rnd(n, k), rnd(n, k), rnd(n)
+    x1[1, 3], x2[3, k - 1], b[2], b[3], b[4] = float("nan"), float("inf"), float("nan"), float("inf"), float("-inf")
+    y = torch.empty((m, n), device="cuda")
+    check(lib.f2c_sage_forward(x1.data_ptr(), x2.data_ptr(), w1.data_ptr(), w2.data_ptr(), b.data_ptr(), y.data_ptr(), m, n, k, 1, ops._stream(x1)))
+    want = torch.relu(x1.double() @ w1.double().t() + b.double() + x2.double() @ w2.double().t())
+    assert torch.equal(y.isnan(), want.isnan()) and torch.equal(y.isinf(), want.isinf())
+
+
+def _with_specials(shape, g, values):
+    t = torch.randn(*shape, generator=g, device="cuda")
+    pick = torch.randint(0, 3 * len(values), shape, generator=g, device="cuda")
+    for i, v in enumerate(values):
+        t[pick == i] = v
+    return t
+
+
+@pytest.mark.parametrize("rows,n", [(1, 3), (700, 96), (333, 47), (6, 1500)])
+@pytest.mark.parametrize("dropout", [False, True])
+def test_relu_dropout_gradient_equals_torch_for_every_value(capi, rows, n, dropout):
+    """Zeros, infinities and NaN in the activations and in the gradient: element by element what torch's own backward gives."""
+    from f2cgt_b200 import ops
+    from f2cgt_b200._lib import check, lib
+    inf, nan = float("inf"), float("nan")
+    g = torch.Generator(device="cuda").manual_seed(rows + n)
+    grad, x = _with_specials((rows, n), g, [0.0, inf, -inf, nan]), _with_specials((rows, n), g, [0.0, -0.0, inf, -inf, nan])
+    x.requires_grad_()
+    active = torch.relu(x)
+    keep = torch.rand(rows, n, generator=g, device="cuda") < 0.6
+    out = torch.ops.aten.native_dropout_backward(grad, keep, 2.5) if dropout else grad * 1.0
+    active.backward(out)
+    dy, db = torch.empty_like(grad), torch.zeros(n, device="cuda")
+    if dropout:
+        check(lib.f2c_sage_mask_dropout(grad.data_ptr(), active.data_ptr(), keep.data_ptr(), 2.5, dy.data_ptr(), db.data_ptr(), rows, n, ops._stream(dy)))
+    else:
+        check(lib.f2c_sage_mask(grad.data_ptr(), active.data_ptr(), 1.0, dy.data_ptr(), db.data_ptr(), rows, n, ops._stream(dy)))
+    assert torch.equal(dy.nan_to_num(7.0, 8.0, 9.0), x.grad.nan_to_num(7.0, 8.0, 9.0))
+    assert torch.equal(db.isnan(), x.grad.sum(0).isnan())
+
+
+def _small_network(dropout, classes=10, hidden=64, layers=3, codebook=None, n=20000, D=128):
+    from f2cgt_b200 import sage, synth
+    indptr, indices = synth.power_law_graph(n, 12, 2.1, seed=1, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(5)
+    codes = torch.randint(0, 256, (n, D // 32), generator=g, dtype=torch.uint8, device="cuda")
+    books = torch.randn(D // 32, 256, 32, generator=g, device="cuda")
+    if codebook is not None:
+        codebook(books)
+    cm = sage.CompressionManager(D, ["vq"], [(32, -1)], [books], [codes])
+    torch.manual_seed(1)
+    model = sage.SAGE(D, hidden, classes, layers, dropout, cm).to("cuda")
+    seeds = torch.randperm(n, generator=g, device="cuda")[:233]
+    _, _, blocks = next(iter(sage.GPUSamplingDataloader(indptr, indices, seeds, 233, (6, 5, 4)[:layers], shuffle=False)))
+    return model, blocks, g
+
+
+@pytest.mark.parametrize("tf32", [True, False])
+@pytest.mark.parametrize("dropout", [0.0, 0.5, 1.0])
+@pytest.mark.parametrize("where", ["features", "gradient", "weight"])
+def test_network_as_one_node_keeps_not_a_number_where_the_layers_do(capi, tf32, dropout, where):
+    """NaN and infinities in the features, in a weight or in the gradient of the output show up in the same outputs and gradients
+    as when the layers are called one by one."""
+    inf, nan = float("inf"), float("nan")
+
+    def spoil(books):
+        books[0, 3, 5], books[1, 7, 2] = nan, inf
+    model, blocks, g = _small_network(dropout, codebook=spoil if where == "features" else None)
+    if where == "weight":
+        with torch.no_grad():
+            model.layers[0].fc_self.weight[3, 4] = nan
+            model.layers[1].fc_neigh.weight[5, 6] = inf
+    weight = torch.randn(233, 10, generator=g, device="cuda")
+    if where == "gradient":
+        weight[5, 3], weight[100, 4], weight[7] = nan, inf, 0.0
+    before = torch.backends.cuda.matmul.allow_tf32
+    torch.backends.cuda.matmul.allow_tf32 = tf32
+    try:
+        got = []
+        for one_node in (True, False):
+            handle = None if one_node else model.layers[1].register_forward_pre_hook(lambda *_: None)  # a hook: layer by layer
+            torch.manual_seed(7)
+            model.zero_grad(set_to_none=True)
+            out = model(blocks)
+            out.backward(weight)
+            got.append([out.detach()] + [p.grad for p in model.parameters()])
+            if handle is not None:
+                handle.remove()
+    finally:
+        torch.backends.cuda.matmul.allow_tf32 = before
+    assert any(bool(t.isnan().any()) for t in got[1])
+    for i, (a, b) in enumerate(zip(*got)):
+        assert torch.equal(a.isnan(), b.isnan()), (i, int(a.isnan().sum()), int(b.isnan().sum()))
+        assert torch.equal(a.isinf(), b.isinf()), i
