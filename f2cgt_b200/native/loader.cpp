@@ -80,8 +80,11 @@ void launch(Set& s, const at::Tensor& order, int64_t first, int64_t count, int64
   s.seeds = view(order, first, count);
   s.args.seeds = s.seeds.data_ptr(); s.args.n_seeds = count; s.args.epoch = (uint32_t)epoch;
   s.args.rng_seed = rng_seed; s.args.rng_offset = rng_offset;
-  check_status(unlocked([&] { return f2c_sample_minibatch(&s.args, st); }));
-  C10_CUDA_CHECK(cudaEventRecord(s.built, st));
+  check_status(unlocked([&] {
+    const int rc = f2c_sample_minibatch(&s.args, st);
+    if (rc == F2C_OK) C10_CUDA_CHECK(cudaEventRecord(s.built, st));
+    return rc;
+  }));
 }
 
 uint64_t bits64(PyObject* o) {
@@ -153,7 +156,7 @@ PyObject* hand_out(Set& s) {
 PyObject* minibatch_take(PyObject*, PyObject* o) {
   return guarded([&]() -> PyObject* {
     Set& s = set_of(o);
-    C10_CUDA_CHECK((cudaError_t)unlocked([&] { return (int)cudaEventSynchronize(s.built); }));
+    C10_CUDA_CHECK(unlocked([&] { return cudaEventSynchronize(s.built); }));
     return hand_out(s);
   });
 }
@@ -164,7 +167,7 @@ PyObject* minibatch_next(PyObject*, PyObject* const* a, Py_ssize_t n) {
     arguments("minibatch_next", n, 9);
     Set& s = set_of(a[0]);
     c10::cuda::CUDAGuard guard(s.indptr.device());
-    C10_CUDA_CHECK((cudaError_t)unlocked([&] { return (int)cudaEventSynchronize(s.built); }));
+    C10_CUDA_CHECK(unlocked([&] { return cudaEventSynchronize(s.built); }));
     if (a[1] != Py_None) {
       Set& next = set_of(a[1]);
       const int64_t first = integer(a[3]), count = integer(a[4]);
@@ -172,8 +175,11 @@ PyObject* minibatch_next(PyObject*, PyObject* const* a, Py_ssize_t n) {
       if (next.lent) {
         // Everything queued on the current stream so far belongs to earlier minibatches: once it has run, the minibatch that
         // was handed out of this set may be overwritten.
-        C10_CUDA_CHECK(cudaEventRecord(next.consumed, stream_of(s.indptr)));
-        C10_CUDA_CHECK(cudaStreamWaitEvent(handle(a[8]), next.consumed, 0));
+        const cudaStream_t side = handle(a[8]);
+        unlocked([&] {
+          C10_CUDA_CHECK(cudaEventRecord(next.consumed, stream_of(s.indptr)));
+          C10_CUDA_CHECK(cudaStreamWaitEvent(side, next.consumed, 0));
+        });
       }
       launch(next, order, first, count, integer(a[5]), bits64(a[6]), bits64(a[7]), handle(a[8]));
     }

@@ -98,13 +98,15 @@ inline PyObject* guarded(F&& body) {
   return nullptr;
 }
 
-// Calls into the library without the interpreter lock (a full launch queue blocks).
+// Runs `body` without the interpreter lock: an allocation may wait for the device, a launch for a place in its stream's queue, and
+// other Python threads (a loader's, a server's) go on meanwhile.  `body` may throw; it touches no Python object.
 template <typename F>
-inline int unlocked(F&& call) {
-  PyThreadState* s = PyEval_SaveThread();
-  const int rc = call();
-  PyEval_RestoreThread(s);
-  return rc;
+inline auto unlocked(F&& body) {
+  struct Released {
+    PyThreadState* state = PyEval_SaveThread();
+    ~Released() { PyEval_RestoreThread(state); }
+  } released;
+  return body();
 }
 
 

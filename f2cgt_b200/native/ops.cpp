@@ -22,11 +22,15 @@ Csc csc(PyObject* ip, PyObject* ix) {
   return Csc{indptr, indices, indptr.numel() - 1, dtype_tag(indptr.scalar_type())};
 }
 
-// [max(n_dst, |out_rows|), width]; rows behind n_dst are zero, or - negative out_rows - left as they are
-at::Tensor block_out(int64_t n_dst, int64_t width, at::ScalarType dtype, const at::Device& device, PyObject* out_rows, cudaStream_t st) {
-  const int64_t asked = out_rows == Py_None ? n_dst : integer(out_rows);
-  const int64_t rows = std::max(n_dst, std::abs(asked));
+// Rows asked for by out_rows (None: the block's own), and the width checked: what block_out() needs of Python.
+int64_t asked_rows(int64_t n_dst, int64_t width, PyObject* out_rows) {
   if (width < 0) fail(PyExc_RuntimeError, "negative width");
+  return out_rows == Py_None ? n_dst : integer(out_rows);
+}
+
+// [max(n_dst, |asked|), width]; rows behind n_dst are zero, or - asked negative - left as they are
+at::Tensor block_out(int64_t n_dst, int64_t asked, int64_t width, at::ScalarType dtype, const at::Device& device, cudaStream_t st) {
+  const int64_t rows = std::max(n_dst, std::abs(asked));
   at::Tensor out = empty({rows, width}, dtype, device);
   if (rows > n_dst && asked > 0) {
     const size_t row = (size_t)width * out.element_size();
@@ -79,10 +83,15 @@ PyObject* sq_decompress(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const at::Tensor& cb = tensor(a[1], "codebooks", kF32);
     if (codes.dim() != 2) fail(PyExc_RuntimeError, "compress_data must be 2-D");
     const int64_t bits = integer(a[2]), cs = integer(a[3]), dim = integer(a[4]);
-    c10::cuda::CUDAGuard guard(codes.device());
-    at::Tensor out = block_out(codes.size(0), dim, at::kFloat, codes.device(), Py_None, nullptr);
-    check_status(f2c_sq_decompress(codes.data_ptr(), dtype_tag(codes.scalar_type()), cb.const_data_ptr<float>(), cb.size(0),
-                                   out.mutable_data_ptr<float>(), codes.size(0), codes.size(1), dim, (int)bits, cs, stream_of(codes)));
+    const int64_t rows = asked_rows(codes.size(0), dim, Py_None);
+    at::Tensor out;
+    check_status(unlocked([&] {
+      c10::cuda::CUDAGuard guard(codes.device());
+      cudaStream_t st = stream_of(codes);
+      out = block_out(rows, rows, dim, at::kFloat, codes.device(), st);
+      return f2c_sq_decompress(codes.data_ptr(), dtype_tag(codes.scalar_type()), cb.const_data_ptr<float>(), cb.size(0),
+                               out.mutable_data_ptr<float>(), codes.size(0), codes.size(1), dim, (int)bits, cs, st);
+    }));
     return THPVariable_Wrap(std::move(out));
   });
 }
@@ -95,10 +104,15 @@ PyObject* vq_decompress(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (codes.dim() != 2 || cb.dim() != 3 || codes.size(1) != cb.size(0))
       fail(PyExc_RuntimeError, "index_tensor must be [rows, n_codebooks] and codebooks [n_codebooks, length, column_slice]");
     const int64_t dim = integer(a[2]);
-    c10::cuda::CUDAGuard guard(codes.device());
-    at::Tensor out = block_out(codes.size(0), dim, at::kFloat, codes.device(), Py_None, nullptr);
-    check_status(f2c_vq_decompress(codes.data_ptr(), dtype_tag(codes.scalar_type()), cb.data_ptr(), dtype_tag(cb.scalar_type()),
-                                   out.mutable_data_ptr<float>(), codes.size(0), cb.size(0), cb.size(1), cb.size(2), dim, stream_of(codes)));
+    const int64_t rows = asked_rows(codes.size(0), dim, Py_None);
+    at::Tensor out;
+    check_status(unlocked([&] {
+      c10::cuda::CUDAGuard guard(codes.device());
+      cudaStream_t st = stream_of(codes);
+      out = block_out(rows, rows, dim, at::kFloat, codes.device(), st);
+      return f2c_vq_decompress(codes.data_ptr(), dtype_tag(codes.scalar_type()), cb.data_ptr(), dtype_tag(cb.scalar_type()),
+                               out.mutable_data_ptr<float>(), codes.size(0), cb.size(0), cb.size(1), cb.size(2), dim, st);
+    }));
     return THPVariable_Wrap(std::move(out));
   });
 }
@@ -109,11 +123,16 @@ PyObject* spmm(PyObject*, PyObject* const* a, Py_ssize_t n) {  // feat, indptr, 
     const at::Tensor& feat = tensor(a[0], "feat", kF32 | bit(F2C_F16) | bit(F2C_F64));
     const Csc c = csc(a[1], a[2]);
     if (feat.dim() != 2) fail(PyExc_RuntimeError, "feat must be 2-D");
-    c10::cuda::CUDAGuard guard(feat.device());
-    cudaStream_t st = stream_of(feat);
-    at::Tensor out = block_out(c.n_dst, feat.size(1), feat.scalar_type(), feat.device(), a[4], st);
-    check_status(f2c_spmm_csr(feat.data_ptr(), dtype_tag(feat.scalar_type()), c.indptr.data_ptr(), c.indices.data_ptr(), c.tag, out.data_ptr(),
-                              c.n_dst, feat.size(1), (int)integer(a[3]), st));
+    const int64_t rows = asked_rows(c.n_dst, feat.size(1), a[4]);
+    const int reduce = (int)integer(a[3]);
+    at::Tensor out;
+    check_status(unlocked([&] {
+      c10::cuda::CUDAGuard guard(feat.device());
+      cudaStream_t st = stream_of(feat);
+      out = block_out(c.n_dst, rows, feat.size(1), feat.scalar_type(), feat.device(), st);
+      return f2c_spmm_csr(feat.data_ptr(), dtype_tag(feat.scalar_type()), c.indptr.data_ptr(), c.indices.data_ptr(), c.tag, out.data_ptr(),
+                          c.n_dst, feat.size(1), reduce, st);
+    }));
     return THPVariable_Wrap(std::move(out));
   });
 }
@@ -128,12 +147,17 @@ PyObject* sq_spmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (codes.dim() != 2) fail(PyExc_RuntimeError, "compress_feat must be 2-D");
     const int64_t bits = integer(a[4]), cs = integer(a[5]), dim = integer(a[6]);
     const Options o = options(a[8], a[9]);
-    c10::cuda::CUDAGuard guard(codes.device());
-    cudaStream_t st = stream_of(codes);
-    at::Tensor out = block_out(c.n_dst, dim, at::kFloat, codes.device(), a[10], st);
-    check_status(f2c_sq_spmm_csr(codes.data_ptr(), dtype_tag(codes.scalar_type()), cb.const_data_ptr<float>(), cb.size(0), c.indptr.data_ptr(),
-                                 c.indices.data_ptr(), c.tag, out.mutable_data_ptr<float>(), c.n_dst, codes.size(0), codes.size(1), dim,
-                                 (int)bits, cs, (int)integer(a[7]), o.get(), st));
+    const int64_t rows = asked_rows(c.n_dst, dim, a[10]);
+    const int reduce = (int)integer(a[7]);
+    at::Tensor out;
+    check_status(unlocked([&] {
+      c10::cuda::CUDAGuard guard(codes.device());
+      cudaStream_t st = stream_of(codes);
+      out = block_out(c.n_dst, rows, dim, at::kFloat, codes.device(), st);
+      return f2c_sq_spmm_csr(codes.data_ptr(), dtype_tag(codes.scalar_type()), cb.const_data_ptr<float>(), cb.size(0), c.indptr.data_ptr(),
+                             c.indices.data_ptr(), c.tag, out.mutable_data_ptr<float>(), c.n_dst, codes.size(0), codes.size(1), dim,
+                             (int)bits, cs, reduce, o.get(), st);
+    }));
     return THPVariable_Wrap(std::move(out));
   });
 }
@@ -149,12 +173,17 @@ PyObject* vq_spmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
       fail(PyExc_RuntimeError, "compress_feat must be [rows, n_codebooks] and codebooks [n_codebooks, length, column_slice]");
     const int64_t dim = integer(a[4]);
     const Options o = options(a[6], a[7]);
-    c10::cuda::CUDAGuard guard(codes.device());
-    cudaStream_t st = stream_of(codes);
-    at::Tensor out = block_out(c.n_dst, dim, at::kFloat, codes.device(), a[8], st);
-    check_status(f2c_vq_spmm_csr(codes.data_ptr(), dtype_tag(codes.scalar_type()), cb.const_data_ptr<float>(), c.indptr.data_ptr(),
-                                 c.indices.data_ptr(), c.tag, out.mutable_data_ptr<float>(), c.n_dst, cb.size(0), cb.size(1), cb.size(2), dim,
-                                 (int)integer(a[5]), o.get(), st));
+    const int64_t rows = asked_rows(c.n_dst, dim, a[8]);
+    const int reduce = (int)integer(a[5]);
+    at::Tensor out;
+    check_status(unlocked([&] {
+      c10::cuda::CUDAGuard guard(codes.device());
+      cudaStream_t st = stream_of(codes);
+      out = block_out(c.n_dst, rows, dim, at::kFloat, codes.device(), st);
+      return f2c_vq_spmm_csr(codes.data_ptr(), dtype_tag(codes.scalar_type()), cb.const_data_ptr<float>(), c.indptr.data_ptr(),
+                             c.indices.data_ptr(), c.tag, out.mutable_data_ptr<float>(), c.n_dst, cb.size(0), cb.size(1), cb.size(2), dim,
+                             reduce, o.get(), st);
+    }));
     return THPVariable_Wrap(std::move(out));
   });
 }
@@ -172,14 +201,19 @@ PyObject* two_level_spmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (vq_cb.dim() != 3 || sq.dim() != 2 || vq.dim() != 2) fail(PyExc_RuntimeError, "sq_data and vq_data must be 2-D and vq_codebooks 3-D");
     const int64_t dim = integer(a[9]);
     const Options o = options(a[11], a[12]);
-    c10::cuda::CUDAGuard guard(vq.device());
-    cudaStream_t st = stream_of(vq);
-    at::Tensor out = block_out(c.n_dst, dim, at::kFloat, vq.device(), a[13], st);
-    check_status(f2c_hybrid_spmm_csr(sq.data_ptr(), dtype_tag(sq.scalar_type()), sq_cb.const_data_ptr<float>(), sq_cb.size(0),
-                                     (int)integer(a[2]), integer(a[3]), sq.size(1), vq.data_ptr(), dtype_tag(vq.scalar_type()),
-                                     vq_cb.const_data_ptr<float>(), vq_cb.size(0), vq_cb.size(1), vq_cb.size(2), slot, sq.size(0),
-                                     c.indptr.data_ptr(), c.indices.data_ptr(), c.tag, out.mutable_data_ptr<float>(), c.n_dst, dim,
-                                     (int)integer(a[10]), o.get(), st));
+    const int64_t rows = asked_rows(c.n_dst, dim, a[13]);
+    const int64_t bits = integer(a[2]), cs = integer(a[3]);
+    const int reduce = (int)integer(a[10]);
+    at::Tensor out;
+    check_status(unlocked([&] {
+      c10::cuda::CUDAGuard guard(vq.device());
+      cudaStream_t st = stream_of(vq);
+      out = block_out(c.n_dst, rows, dim, at::kFloat, vq.device(), st);
+      return f2c_hybrid_spmm_csr(sq.data_ptr(), dtype_tag(sq.scalar_type()), sq_cb.const_data_ptr<float>(), sq_cb.size(0), (int)bits, cs, sq.size(1),
+                                 vq.data_ptr(), dtype_tag(vq.scalar_type()), vq_cb.const_data_ptr<float>(), vq_cb.size(0), vq_cb.size(1),
+                                 vq_cb.size(2), slot, sq.size(0), c.indptr.data_ptr(), c.indices.data_ptr(), c.tag, out.mutable_data_ptr<float>(),
+                                 c.n_dst, dim, reduce, o.get(), st);
+    }));
     return THPVariable_Wrap(std::move(out));
   });
 }
@@ -191,20 +225,25 @@ PyObject* kmeans_assign(PyObject*, PyObject* const* a, Py_ssize_t n) {  // x, ce
     const at::Tensor& centers = tensor(a[1], "centers", kF32);
     if (x.dim() != 2 || centers.dim() != 2 || x.size(1) != centers.size(1)) fail(PyExc_RuntimeError, "data must be [n, d] and centers [k, d]");
     const int metric = (int)integer(a[2]);
-    c10::cuda::CUDAGuard guard(x.device());
-    const cudaStream_t st = stream_of(x);
     const int64_t rows = x.size(0), k = centers.size(0), d = x.size(1);
-    at::Tensor labels = empty({rows}, at::kLong, x.device()), head = empty({2}, at::kInt, x.device());
-    const int64_t bytes = f2c_kmeans_assign_workspace(rows, k, d);
-    at::Tensor ws;
-    if (bytes > 0) {
-      ws = empty({bytes}, at::kByte, x.device());
-      C10_CUDA_CHECK(cudaMemsetAsync(ws.data_ptr(), 0, 256, st));  // the exact scorer leaves it as it is
-    }
-    check_status(f2c_kmeans_assign(x.const_data_ptr<float>(), centers.const_data_ptr<float>(), labels.mutable_data_ptr<int64_t>(), rows, k, d,
-                                   metric, bytes > 0 ? ws.data_ptr() : nullptr, st));
-    if (bytes > 0) C10_CUDA_CHECK(cudaMemcpyAsync(head.data_ptr(), ws.data_ptr(), 8, cudaMemcpyDeviceToDevice, st));
-    else C10_CUDA_CHECK(cudaMemsetAsync(head.data_ptr(), 0, 8, st));
+    at::Tensor labels, head;
+    check_status(unlocked([&] {
+      c10::cuda::CUDAGuard guard(x.device());
+      const cudaStream_t st = stream_of(x);
+      labels = empty({rows}, at::kLong, x.device());
+      head = empty({2}, at::kInt, x.device());
+      const int64_t bytes = f2c_kmeans_assign_workspace(rows, k, d);
+      at::Tensor ws;
+      if (bytes > 0) {
+        ws = empty({bytes}, at::kByte, x.device());
+        C10_CUDA_CHECK(cudaMemsetAsync(ws.data_ptr(), 0, 256, st));  // the exact scorer leaves it as it is
+      }
+      const int rc = f2c_kmeans_assign(x.const_data_ptr<float>(), centers.const_data_ptr<float>(), labels.mutable_data_ptr<int64_t>(), rows, k, d,
+                                       metric, bytes > 0 ? ws.data_ptr() : nullptr, st);
+      if (bytes > 0) C10_CUDA_CHECK(cudaMemcpyAsync(head.data_ptr(), ws.data_ptr(), 8, cudaMemcpyDeviceToDevice, st));
+      else C10_CUDA_CHECK(cudaMemsetAsync(head.data_ptr(), 0, 8, st));
+      return rc;
+    }));
     PyObject* l = THPVariable_Wrap(std::move(labels));
     PyObject* h = THPVariable_Wrap(std::move(head));
     PyObject* r = PyTuple_Pack(2, l, h);

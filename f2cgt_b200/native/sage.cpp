@@ -279,52 +279,54 @@ PyObject* sage_net(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (a[9] != Py_None) net.cast = reinterpret_cast<THPDtype*>(a[9])->scalar_type;
     if (h_self.dim() != 2 || h_self.sizes() != h_neigh.sizes() || h_self.size(0) < net.layers[0].padded) fail(PyExc_RuntimeError, "sage_net: bad inputs");
     const bool record = at::GradMode::is_enabled() && torch::autograd::compute_requires_grad(w);
-
-    c10::cuda::CUDAGuard guard(h_self.device());
-    cudaStream_t st = stream_of(h_self);
-    std::shared_ptr<SageBackward> node;
-    if (record) {
-      node = std::shared_ptr<SageBackward>(new SageBackward(), torch::autograd::deleteNode);
-      node->set_next_edges(torch::autograd::collect_next_edges(w));
-    }
-    at::Tensor h;
-    {
-      at::AutoDispatchBelowADInplaceOrView below;
-      at::Tensor x1 = h_self, x2 = h_neigh;
-      for (Py_ssize_t i = 0; i < L; ++i) {
-        const Layer& l = net.layers[i];
-        const bool last = i + 1 == L;
-        if (i > 0) {
-          x1 = h;
-          x2 = empty({l.padded, h.size(1)}, at::kFloat, h.device());
-          checked = f2c_spmm_csr(h.data_ptr(), F2C_F32, l.indptr.data_ptr(), l.indices.data_ptr(), dtype_tag(l.indptr.scalar_type()), x2.data_ptr(),
-                                 l.rows, h.size(1), F2C_MEAN, st);
-        }
-        h = layer_forward(net, x1, x2, &w[3 * i], l, !last, record, st);
-        const at::Tensor active = h;
-        at::Tensor keep;
-        if (!last && net.p > 0) {
-          if (net.p < 1 && h.numel() > 0) std::tie(h, keep) = at::native_dropout(h, net.p, true);
-          else h = at::dropout(h, net.p, true);
-        }
-        if (record) {
-          node->x1.push_back(x1);
-          node->x2.push_back(x2);
-          if (!last) {
-            node->out.push_back(h);
-            node->active.push_back(active);
-            node->keep.push_back(keep);
+    at::Tensor result = unlocked([&] {
+      c10::cuda::CUDAGuard guard(h_self.device());
+      cudaStream_t st = stream_of(h_self);
+      std::shared_ptr<SageBackward> node;
+      if (record) {
+        node = std::shared_ptr<SageBackward>(new SageBackward(), torch::autograd::deleteNode);
+        node->set_next_edges(torch::autograd::collect_next_edges(w));
+      }
+      at::Tensor h;
+      {
+        at::AutoDispatchBelowADInplaceOrView below;
+        at::Tensor x1 = h_self, x2 = h_neigh;
+        for (Py_ssize_t i = 0; i < L; ++i) {
+          const Layer& l = net.layers[i];
+          const bool last = i + 1 == L;
+          if (i > 0) {
+            x1 = h;
+            x2 = empty({l.padded, h.size(1)}, at::kFloat, h.device());
+            checked = f2c_spmm_csr(h.data_ptr(), F2C_F32, l.indptr.data_ptr(), l.indices.data_ptr(), dtype_tag(l.indptr.scalar_type()), x2.data_ptr(),
+                                   l.rows, h.size(1), F2C_MEAN, st);
+          }
+          h = layer_forward(net, x1, x2, &w[3 * i], l, !last, record, st);
+          const at::Tensor active = h;
+          at::Tensor keep;
+          if (!last && net.p > 0) {
+            if (net.p < 1 && h.numel() > 0) std::tie(h, keep) = at::native_dropout(h, net.p, true);
+            else h = at::dropout(h, net.p, true);
+          }
+          if (record) {
+            node->x1.push_back(x1);
+            node->x2.push_back(x2);
+            if (!last) {
+              node->out.push_back(h);
+              node->active.push_back(active);
+              node->keep.push_back(keep);
+            }
           }
         }
+        if (h.size(0) > net.layers[L - 1].rows) h = h.narrow(0, 0, net.layers[L - 1].rows);
       }
-      if (h.size(0) > net.layers[L - 1].rows) h = h.narrow(0, 0, net.layers[L - 1].rows);
-    }
-    if (record) {
-      for (const at::Tensor& t : w) node->weights.emplace_back(t, false);
-      node->net = std::move(net);
-      torch::autograd::set_history(h, node);
-    }
-    return THPVariable_Wrap(std::move(h));
+      if (record) {
+        for (const at::Tensor& t : w) node->weights.emplace_back(t, false);
+        node->net = std::move(net);
+        torch::autograd::set_history(h, node);
+      }
+      return h;
+    });
+    return THPVariable_Wrap(std::move(result));
   });
 }
 
