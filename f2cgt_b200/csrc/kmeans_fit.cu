@@ -35,8 +35,8 @@ constexpr size_t kSmemLimit = 200 * 1024;
 struct State {       // first 256 bytes of the workspace; the host reads the first four words
   int32_t done;
   int32_t iterations;
-  int32_t not_finite;   // the data hold inf or NaN: nothing is iterated, the caller takes another path
-  int32_t assign_error; // a bounded wait of the tensor-core kernel ran out
+  int32_t not_finite;   // the data hold inf or NaN: nothing is iterated, the caller says so
+  int32_t assign_error; // code of the last bounded wait of the tensor-core kernel that ran out (the exact scorer then assigned every point)
   uint32_t max_bits;    // largest |x| as float bits
   uint32_t arrived;
   double shift;
@@ -104,8 +104,9 @@ __device__ void finish_iteration(float* __restrict__ centers, long long* sums, u
     st->iterations += 1;
     st->arrived = 0u;
     if (assign_head != nullptr) {
-      if (assign_head[1] != 0) { st->assign_error = assign_head[1]; st->done = 1; }
-      assign_head[0] = 0;  // the next assignment's list is empty
+      // after a wait that ran out the labels are the exact scorer's, so the iteration counts and the next one starts afresh
+      if (assign_head[1] != 0) st->assign_error = assign_head[1];
+      assign_head[0] = assign_head[1] = 0;
     }
     if ((double)(float)total <= tol) st->done = 1;
   }

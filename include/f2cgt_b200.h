@@ -272,7 +272,8 @@ int f2c_kmeans_assign(const float* x, const float* centers, int64_t* labels, int
  *   f2c_kmeans_fit_iterate  queues `iterations` iterations on `centers` [k, d] (in place) without waiting for any of them;
  *                           those behind the converged one do nothing, so a caller queues a few at a time and looks at the
  *                           first four int32 words of the workspace between the calls: {done, iterations taken, the data
- *                           hold inf or NaN (then nothing is iterated), error code of the assignment kernel}.
+ *                           hold inf or NaN (then nothing is iterated), code of the last bounded wait of the tensor-core
+ *                           assignment that ran out (0 = none; that iteration's labels are the exact scorer's, nothing is lost)}.
  * The sums are exact fixed-point integers: a fit is reproducible bit for bit. */
 int64_t f2c_kmeans_fit_workspace(int64_t n, int64_t k, int64_t d);
 int f2c_kmeans_fit_begin(const float* x, int64_t n, int64_t k, int64_t d, void* workspace, void* stream);
@@ -291,7 +292,7 @@ int f2c_kmeans_assign_static(const float* x, const float* centers, int64_t* labe
 /* Companion of f2c_kmeans_assign_static (no counterpart in the reference either): its caller cannot read the
  * built-in array, so this copies the array's 8-byte header to the host after `stream` has drained - the number of
  * points the exact scorer had to settle and the code the kernel writes when one of its bounded waits ran out
- * (then some labels are unwritten).  Returns F2C_ERR_CUDA when that code is non-zero.  Allocates nothing.
+ * (then the exact scorer assigned every point).  Returns F2C_ERR_CUDA when that code is non-zero.  Allocates nothing.
  * (f2c_kmeans_assign reports the same two words as int32 words 0 and 1 of the caller's workspace.) */
 int f2c_kmeans_assign_static_status(int32_t* undecided_host, int32_t* error_host, void* stream);
 

@@ -149,3 +149,33 @@ def test_fit_iterations_equal_the_restated_loop(capi, metric, n, k, d):
         again = capi.KMeans(start.clone(), metric, max_iter=max_iter, tol=tol)
         again.fit(x)
         assert torch.equal(got, again.get_centers())
+
+
+def _fit(x, centers, iterations, spoil=False, each=None):
+    """Lloyd iterations by the C entry points, queued at once or (each) one call after the other; centres and state words."""
+    from f2cgt_b200 import ops
+    from f2cgt_b200._lib import check, lib
+    n, d = x.shape
+    k = centers.shape[0]
+    up = lambda v: (v + 255) // 256 * 256  # noqa: E731
+    ws = torch.empty(lib.f2c_kmeans_fit_workspace(n, k, d), dtype=torch.uint8, device="cuda")
+    head = ws[256 + up(k * d * 8) + up(k * 4) + up(n * 8):][:8].view(torch.int32)
+    check(lib.f2c_kmeans_fit_begin(x.data_ptr(), n, k, d, ws.data_ptr(), ops._stream(x)))
+    for take in each or [iterations]:
+        if spoil:
+            head[1] = 3
+        check(lib.f2c_kmeans_fit_iterate(x.data_ptr(), centers.data_ptr(), n, k, d, 0, 0.0, take, ws.data_ptr(), ops._stream(x)))
+        if each:
+            torch.cuda.synchronize()
+    return centers, ws[:16].view(torch.int32).tolist()
+
+
+def test_fit_goes_on_after_an_assignment_whose_wait_ran_out(capi):
+    """The tensor-core kernel's word for a bounded wait that ran out makes the exact scorer assign every point; the fit takes those
+    labels and goes on.  The word is set by the host here."""
+    g = torch.Generator(device="cuda").manual_seed(0)
+    x = torch.randn(5000, 16, generator=g, device="cuda")
+    want, words = _fit(x, x[:64].clone(), 6)
+    got, spoiled = _fit(x, x[:64].clone(), 6, spoil=True)
+    assert spoiled[:3] == words[:3]
+    assert spoiled[3] == 3 and torch.equal(want, got)
