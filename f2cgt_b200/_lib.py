@@ -94,6 +94,8 @@ SIGNATURES = {
     "f2c_kmeans_assign_static": [p, p, p, i64, i64, i64, ci, p],
     "f2c_kmeans_assign_static_status": [p, p, p],
     "f2c_device_status": [p, p],
+    "f2c_device_status_seen": [p],
+    "f2c_device_status_report": [C.c_int32, p],
     "f2c_check_csc": [p, p, ci, i64, i64, p, p],
     "f2c_relabel_capacity": [i64],
     "f2c_relabel_mark": [p, ci, i64, p, p, i64, p, p, p],

@@ -58,6 +58,19 @@ __device__ __forceinline__ void release_dependents() { asm volatile("griddepcont
 
 // ---- device helpers ----
 
+// What a kernel leaves behind when a bounded wait ran out: one record per device (api.cu).  `seen` is the same word in mapped host
+// memory, which the host reads without waiting for the device; null until it has been set up.
+struct WaitReport { int code; int pad; int* seen; };
+__device__ __forceinline__ void report_wait(int* word, int code) {
+  if (word == nullptr) return;
+  atomicExch(word, code);
+  int* const seen = *reinterpret_cast<int* volatile*>(&reinterpret_cast<WaitReport*>(word)->seen);
+  if (seen != nullptr) {
+    *reinterpret_cast<volatile int*>(seen) = code;
+    __threadfence_system();
+  }
+}
+
 // Read-only, L1-bypassing vector loads for streamed gathers.
 __device__ __forceinline__ uint32_t ldg_nc_u32(const void* p) {
   uint32_t v;

@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(Geo<BITS>::kThreads, 1) sq_stream_kernel(const
   const uint32_t cap = (a_bytes - ptr_bytes - ids_bytes) / rb - gmax;   // must be >= (kRowLag + 1) * batch + gmax
   if (ptr_bytes + ids_bytes + ((kRowLag + 1) * batch + 2u * gmax) * rb > a_bytes) {
     // the shared window starts somewhere the host did not expect: a ring too small could stall, so do nothing
-    if (threadIdx.x == 0 && p.error != nullptr) atomicExch(p.error, 3);
+    if (threadIdx.x == 0) report_wait(p.error, 3);
     return;
   }
 

@@ -13,7 +13,8 @@
 //    layer's operands turns that into 2^-11, and a ReLU near zero into a different gradient);
 //  * four warps add bias and the two sums, apply the ReLU and write 128-byte pieces of rows through shared memory, while the
 //    next tile is loaded and multiplied.
-// Every wait is bounded: when one runs out the CTA's roles all leave, the error word is raised and TMEM is freed.
+// Every wait is bounded: when one runs out the CTA's roles all leave, the rows it has not finished become NaN (whoever uses them
+// sees it), the copies and products still in flight are waited for, the error word is raised and TMEM is freed.
 #include <cuda.h>
 
 #include <mutex>
@@ -155,6 +156,8 @@ __global__ void __launch_bounds__(kThreads, 1) sage_forward_kernel(const __grid_
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = bars.tmem;
+  int s = 0;  // loading thread: stage and round of its next load
+  uint32_t round = 0;
 
   if (wid == 0) {
     // ================= loads
@@ -164,8 +167,6 @@ __global__ void __launch_bounds__(kThreads, 1) sage_forward_kernel(const __grid_
         for (int i = 0; i < steps; ++i)
           tma_load(i < per_segment ? &w1 : &w2, smem_u32(weights + (size_t)i * b_bytes), &bars.weights, (i % per_segment) * kK, col0);
       }
-      int s = 0;
-      uint32_t round = 0;
       for (int tile = blockIdx.x; tile < p.tiles; tile += gridDim.x) {
         for (int i = 0; i < steps; ++i) {
           if (round > 0 && !wait_bar(bars.empty + s, (round - 1) & 1, failed)) { tile = p.tiles; break; }
@@ -177,18 +178,6 @@ __global__ void __launch_bounds__(kThreads, 1) sage_forward_kernel(const __grid_
           if (++s == p.stages) { s = 0; ++round; }
         }
       }
-      // loads in flight write to this CTA's shared memory: on the early way out wait (bounded) for the stages not yet seen full
-      if (*failed)
-        for (int q = 0; q < p.stages; ++q) {
-          const uint32_t uses = round + (q < s ? 1u : 0u);
-          for (uint32_t it = 0; uses > 0 && it < kWaitLimit; ++it) {
-            uint32_t done = 0;
-            asm volatile(
-                "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-                : "=r"(done) : "r"(smem_u32(bars.full + q)), "r"((uses - 1) & 1) : "memory");
-            if (done) break;
-          }
-        }
     }
   } else if (wid == 1) {
     // ================= MMAs
@@ -196,8 +185,7 @@ __global__ void __launch_bounds__(kThreads, 1) sage_forward_kernel(const __grid_
       // fp32 accumulate, tf32 operands, N / 8, M / 16
       const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(p.b_rows >> 3) << 17) | ((uint32_t)(kM >> 4) << 24);
       bool ok = !p.resident || wait_bar(&bars.weights, 0, failed);
-      int s = 0;
-      uint32_t round = 0, t = 0;
+      uint32_t t = 0;
       for (int tile = blockIdx.x; ok && tile < p.tiles; tile += gridDim.x, ++t) {
         const uint32_t buf = t & 1u;
         if (t >= 2) ok = wait_bar(bars.acc_empty + buf, ((t >> 1) - 1) & 1, failed);
@@ -218,11 +206,6 @@ __global__ void __launch_bounds__(kThreads, 1) sage_forward_kernel(const __grid_
         }
         if (ok) commit(bars.acc_full + buf);
       }
-      if (*failed) {  // MMAs in flight read this CTA's shared memory and write its TMEM
-        volatile int drained = 0;
-        commit(&bars.drain);
-        wait_bar(&bars.drain, 0, &drained);
-      }
     }
   } else {
     // ================= epilogue: warp w owns the TMEM lanes of its quarter; 32 x 32 pieces go through shared memory so that
@@ -231,11 +214,17 @@ __global__ void __launch_bounds__(kThreads, 1) sage_forward_kernel(const __grid_
     float* epi = epi_s + (wid - 2) * kEpiFloats;
     const bool vec = (p.n & 3) == 0 && (((uintptr_t)p.y) & 15) == 0;
     uint32_t t = 0;
+    bool lost = false;  // a wait ran out
     for (int tile = blockIdx.x; tile < p.tiles; tile += gridDim.x, ++t) {
       const uint32_t buf = t & 1u;
-      if (!__all_sync(0xffffffffu, wait_bar(bars.acc_full + buf, (t >> 1) & 1, failed))) break;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int64_t row0 = (int64_t)tile * kM + quarter * 32;
+      lost = lost || !__all_sync(0xffffffffu, wait_bar(bars.acc_full + buf, (t >> 1) & 1, failed));
+      if (lost) {
+        for (int64_t row = row0; row < row0 + 32 && row < p.m; ++row)
+          for (int c = lane; c < tile_cols; c += 32) p.y[row * p.n + col0 + c] = __int_as_float(0x7fffffff);
+        continue;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       for (int c0 = 0; c0 < tile_cols; c0 += 32) {
         uint32_t r1[32], r2[32];
         const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + buf * 256u + (uint32_t)c0;
@@ -285,11 +274,26 @@ __global__ void __launch_bounds__(kThreads, 1) sage_forward_kernel(const __grid_
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (bars.failed) {
+    // loads in flight write to this CTA's shared memory, MMAs in flight read it and write its TMEM: wait (bounded) for what was issued
+    volatile int expired = 0;  // (set by a wait that runs out again; the next one then gives up soon)
+    if (tid == 0) {
+      if (p.resident) wait_bar(&bars.weights, 0, &expired);
+      for (int q = 0; q < p.stages; ++q) {
+        const uint32_t uses = round + (q < s ? 1u : 0u);
+        if (uses > 0) wait_bar(bars.full + q, (uses - 1) & 1, &expired);
+      }
+    } else if (tid == 32) {
+      commit(&bars.drain);
+      wait_bar(&bars.drain, 0, &expired);
+    }
+    __syncthreads();
+  }
   if (wid == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
   }
-  if (tid == 0 && bars.failed && p.error != nullptr) atomicExch(p.error, 3);
+  if (tid == 0 && bars.failed) report_wait(p.error, 3);
 }
 
 using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,

@@ -72,7 +72,7 @@ template <int P> __device__ __forceinline__ void producer_barrier() { asm volati
 
 __device__ __forceinline__ void raise_abort(Sync* sync, int* error, int code) {
   st_release(&sync->abort, 1u);
-  if (error != nullptr) atomicExch(error, code);
+  report_wait(error, code);
 }
 
 // Consumer side (all 32 lanes call it): wait until edges [0, need) are staged.  `seen` caches the lowest value any lane

@@ -45,6 +45,14 @@ struct Status {  // library status inside a node (no Python exception there)
 };
 constexpr Status checked{};
 
+// Kernels run behind the host, so a bounded wait that ran out in one of them shows at a later call: here, without a wait of its own.
+void check_reported() {
+  int32_t code = 0;
+  if (f2c_device_status_seen(&code) == F2C_OK && code != 0)
+    TORCH_CHECK(false, "f2cgt_b200: a bounded wait ran out inside an earlier kernel of this device (code ", code,
+                "): results of that call are unfinished (device_status() reports and clears this)");
+}
+
 float* f32(const at::Tensor& t) { return (float*)t.data_ptr(); }
 
 at::Tensor mm(const Net& net, const at::Tensor& a, const at::Tensor& b) {
@@ -153,6 +161,7 @@ struct SageBackward : public torch::autograd::Node {
     at::NoGradGuard no_grad;
     const at::Tensor given = grads[0].to(at::kFloat);
     c10::cuda::CUDAGuard guard(given.device());
+    check_reported();
     const c10::cuda::CUDAStream main = at::cuda::getCurrentCUDAStream(given.device().index());
     cudaStream_t st = main.stream();
     auto self = shared_from_this();
@@ -281,6 +290,7 @@ PyObject* sage_net(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const bool record = at::GradMode::is_enabled() && torch::autograd::compute_requires_grad(w);
     at::Tensor result = unlocked([&] {
       c10::cuda::CUDAGuard guard(h_self.device());
+      check_reported();
       cudaStream_t st = stream_of(h_self);
       std::shared_ptr<SageBackward> node;
       if (record) {

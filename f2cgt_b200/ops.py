@@ -90,7 +90,8 @@ def _check_block(table, indptr, indices):
 
 
 def device_status(device=None):
-    """0, or the code of a bounded wait that ran out inside a kernel since the last query (synchronises the current stream)."""
+    """0, or the code of a bounded wait that ran out inside a kernel since the last query (synchronises the current stream).
+    ``sage.SAGE`` looks at the same word in every forward and backward pass, without waiting, and raises until it is read here."""
     import ctypes
     code = ctypes.c_int32(0)
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)

@@ -26,7 +26,7 @@ import torch.nn.functional as F
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 sys.path.insert(0, ROOT)
 
-from f2cgt_b200 import sage, synth  # noqa: E402
+from f2cgt_b200 import ops, sage, synth  # noqa: E402
 
 PRESETS = {
     # nodes, avg degree, feat dim, classes, train ids, hot fraction, hot bits, VQ (n_cb, cs), hidden, fan-out
@@ -215,6 +215,9 @@ def train(preset="small", table="replicated", rank=0, world=1, local_rank=0, epo
         if world > 1:
             dist.barrier()
         epoch_s.append(time.perf_counter() - t0)
+        code = ops.device_status(device)
+        if code != 0:
+            raise RuntimeError(f"a bounded wait ran out inside a kernel (code {code}): the weights of this epoch are not to be used")
         if first_layer_edges:
             edges = float(first_layer_edges)
         losses.append(float(loss.detach()))

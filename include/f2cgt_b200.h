@@ -8,7 +8,8 @@
  * Conventions (all entry points):
  *   - every pointer is a DEVICE pointer unless the parameter name ends in `_host`;
  *   - tensors are dense row-major ("contiguous" in torch terms); sizes are in elements;
- *   - the library allocates nothing that outlives a call and never synchronises the device; work
+ *   - the library allocates nothing that outlives a call (but for one word per device, see f2c_device_status) and never
+ *     synchronises the device; work
  *     is queued on `stream` (a cudaStream_t passed as void*; NULL = the legacy default stream,
  *     which is what the reference launches on, e.g. src/fusion_spmm.cu:261);
  *   - the return value is a status (F2C_OK = 0); on failure `f2c_last_error()` returns a message
@@ -75,8 +76,14 @@ int f2c_version(void);
 /* Kernels of this library never spin without a limit: a wait that runs out (a producer warp or a tensor-core
  * barrier that does not answer within ~0.2 s) makes the kernel return early and raises a per-device word.
  * f2c_device_status synchronises `stream`, copies that word of the current device to *code_host (0 = no wait ever
- * ran out since the last query) and clears it.  Allocates nothing.  No counterpart in the reference. */
+ * ran out since the last query) and clears it.
+ * f2c_device_status_seen tells the same without waiting and without clearing: what kernels that have run by now have reported.
+ * f2c_device_status_report queues such a report on `stream` (for tests of what a caller does then).
+ * The word's copy on the host is four bytes of pinned memory per device that the first call sets up; otherwise they allocate
+ * nothing.  No counterpart in the reference. */
 int f2c_device_status(int32_t* code_host, void* stream);
+int f2c_device_status_seen(int32_t* code_host);
+int f2c_device_status_report(int32_t code, void* stream);
 
 /* packbits(unpack, target_bits)  -  src/packbits.cu:44-64 (kernel :6-42).
  * unpack [rows, unpack_dim] u8 -> pack [rows, ceil(unpack_dim*bits/8)] u8; bits in {1,2,4}. */
@@ -133,7 +140,7 @@ int f2c_spmm_csr_backward(const float* grad_out, const void* indptr, const void*
 
 /* Forward product of a SAGE layer (fc_self and fc_neigh of examples/conv.py:62-76 together), fp32 storage, tf32 operands
  * (rounded to nearest), fp32 accumulation: y [m, n] = (x1 [m, k] w1 [n, k]^T + bias [n]) + x2 w2^T (bias may be NULL), then
- * max(0, .) when relu != 0 (a NaN stays NaN).  Row-major, operands 16-byte aligned, k % 4 == 0 (else F2C_ERR_UNSUPPORTED). */
+ * max(0, .) when relu != 0 (a NaN stays NaN).  Rows that a wait which ran out left unfinished (f2c_device_status) are NaN.  Row-major, operands 16-byte aligned, k % 4 == 0 (else F2C_ERR_UNSUPPORTED). */
 int f2c_sage_forward(const float* x1, const float* x2, const float* w1, const float* w2, const float* bias, float* y, int64_t m,
                      int64_t n, int64_t k, int relu, void* stream);
 

@@ -425,3 +425,36 @@ def test_network_as_one_node_keeps_not_a_number_where_the_layers_do(capi, tf32, 
     for i, (a, b) in enumerate(zip(*got)):
         assert torch.equal(a.isnan(), b.isnan()), (i, int(a.isnan().sum()), int(b.isnan().sum()))
         assert torch.equal(a.isinf(), b.isinf()), i
+
+
+def _report(code):
+    from f2cgt_b200._lib import check, lib
+    check(lib.f2c_device_status_report(code, torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+
+
+def test_network_raises_when_a_wait_ran_out_in_an_earlier_kernel(capi):
+    """A bounded wait that ran out leaves a report; the passes that follow raise until it has been read."""
+    from f2cgt_b200 import ops
+    model, blocks, _ = _small_network(0.5)
+    out = model(blocks)
+    assert ops.device_status() == 0
+    _report(3)
+    with pytest.raises(RuntimeError, match="bounded wait"):
+        model(blocks)
+    with pytest.raises(RuntimeError, match="bounded wait"):
+        out.sum().backward()
+    assert ops.device_status() == 3 and ops.device_status() == 0
+    model(blocks).sum().backward()
+    assert ops.device_status() == 0
+
+
+def test_training_does_not_return_when_a_wait_ran_out(capi, monkeypatch):
+    from f2cgt_b200 import ops, sage, train_graphsage as tg
+    monkeypatch.setitem(tg.PRESETS, "small", dict(tg.PRESETS["small"], nodes=5000, degree=10, train=512, fan_out=(3, 3)))
+    assert tg.train(epochs=1, batch_size=256)["epochs_run"] == 1
+    pokes = []
+    monkeypatch.setattr(sage.GPUSamplingDataloader, "poke", lambda self: pokes.append(0) or len(pokes) == 3 and _report(1))  # behind the last step
+    with pytest.raises(RuntimeError, match="bounded wait"):
+        tg.train(epochs=1, batch_size=256, max_steps=1)
+    assert ops.device_status() == 0
