@@ -140,6 +140,14 @@ Beside& beside(c10::DeviceIndex device) {
 }
 constexpr int64_t kBesideRows = 4096;  // fewer rows: a product is shorter than the calls that would move it
 
+// Stands behind gradients that were asked for with a graph (create_graph) and have none.
+struct NotTwice : public torch::autograd::Node {
+  std::string name() const override { return "SageNotTwiceDifferentiable"; }
+  variable_list apply(variable_list&&) override {
+    TORCH_CHECK(false, "a SAGE network of several layers cannot be differentiated twice: its aggregations have no second derivative here");
+  }
+};
+
 struct SageBackward : public torch::autograd::Node {
   Net net;
   std::vector<SavedVariable> weights;   // per layer: self, neigh, bias
@@ -155,11 +163,41 @@ struct SageBackward : public torch::autograd::Node {
 
   variable_list apply(variable_list&& grads) override {
     TORCH_CHECK(!released, "Trying to backward through the graph a second time: its saved tensors have been freed");
+    if (!grads[0].defined()) return variable_list(3 * net.layers.size());
+    if (!at::GradMode::is_enabled()) return gradients(grads[0]);
+    // create_graph: the gradients are to be differentiable themselves
+    if (net.layers.size() == 1) return one_layer_with_graph(grads[0]);
+    variable_list result = gradients(grads[0]), from = {grads[0]};
+    auto self = shared_from_this();
+    for (const SavedVariable& w : weights) from.push_back(w.unpack(self));
+    if (!torch::autograd::compute_requires_grad(from)) return result;
+    auto node = std::shared_ptr<NotTwice>(new NotTwice(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(from));
+    for (at::Tensor& r : result) {
+      if (!r.defined()) continue;
+      {
+        at::NoGradGuard no_grad;
+        r = r.clone();  // two of them share memory
+      }
+      torch::autograd::set_history(r, node);
+    }
+    return result;
+  }
+
+  // A single layer is linear in the gradient that it is given, so torch's own products make the graph.
+  variable_list one_layer_with_graph(const at::Tensor& given) {
+    const at::Tensor dy = given.to(at::kFloat), turned = dy.t();
+    auto of = [&](size_t i, auto&& make) { return task_should_compute_output(i) ? make() : at::Tensor(); };
+    auto bias = weights[2].unpack(shared_from_this());
+    return {of(0, [&] { return mm(net, turned, x1[0].narrow(0, 0, dy.size(0))); }), of(1, [&] { return mm(net, turned, x2[0].narrow(0, 0, dy.size(0))); }),
+            of(2, [&] { return bias.defined() ? dy.sum(0) : at::Tensor(); })};
+  }
+
+  variable_list gradients(const at::Tensor& grad_output) {
     const size_t L = net.layers.size();
     variable_list result(3 * L);
-    if (!grads[0].defined()) return result;
     at::NoGradGuard no_grad;
-    const at::Tensor given = grads[0].to(at::kFloat);
+    const at::Tensor given = grad_output.to(at::kFloat);
     c10::cuda::CUDAGuard guard(given.device());
     check_reported();
     const c10::cuda::CUDAStream main = at::cuda::getCurrentCUDAStream(given.device().index());

@@ -458,3 +458,28 @@ def test_training_does_not_return_when_a_wait_ran_out(capi, monkeypatch):
     with pytest.raises(RuntimeError, match="bounded wait"):
         tg.train(epochs=1, batch_size=256, max_steps=1)
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("layers", [1, 2, 3])
+def test_gradients_with_a_graph(capi, layers):
+    """create_graph=True: one layer is differentiable twice, as its products are; more layers give the same first gradients and
+    refuse the second derivative instead of leaving it out."""
+    model, blocks, _ = _small_network(0.0, layers=layers)
+    params = list(model.parameters())
+    plain = torch.autograd.grad(model(blocks).square().mean(), params)
+    grads = torch.autograd.grad(model(blocks).square().mean(), params, create_graph=True)
+    assert all(x.requires_grad for x in grads)
+    assert all(torch.allclose(a, b, rtol=1e-4, atol=1e-6) for a, b in zip(plain, grads))
+    if layers > 1:
+        with pytest.raises(RuntimeError, match="differentiated twice"):
+            sum(x.square().sum() for x in grads).backward()
+        with pytest.raises(RuntimeError, match="differentiated twice"):
+            torch.autograd.grad(grads[0].sum(), params)
+        return
+    sum(x.square().sum() for x in grads).backward()
+    got = [p.grad.clone() for p in params]
+    model.zero_grad(set_to_none=True)
+    model.layers[0].register_forward_pre_hook(lambda *_: None)  # a hook: the layer on its own
+    grads = torch.autograd.grad(model(blocks).square().mean(), params, create_graph=True)
+    sum(x.square().sum() for x in grads).backward()
+    assert all(torch.allclose(a, p.grad, rtol=1e-4, atol=1e-6) for a, p in zip(got, params))
