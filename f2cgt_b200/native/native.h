@@ -7,6 +7,7 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/Dtype.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "../../include/f2cgt_b200.h"
@@ -90,6 +91,8 @@ inline PyObject* guarded(F&& body) {
   try {
     return body();
   } catch (const PythonError&) {
+  } catch (python_error& e) {  // out of a Python hook that torch called
+    e.restore();
   } catch (const c10::Error& e) {
     PyErr_SetString(PyExc_RuntimeError, e.what_without_backtrace());
   } catch (const std::exception& e) {

@@ -148,17 +148,46 @@ struct NotTwice : public torch::autograd::Node {
   }
 };
 
+// A tensor kept for the backward pass, and what it has to be when it comes back: saved-tensor hooks (offloading, checkpointing) see
+// it like any other saved tensor, and may give back another one.
+class Kept {
+ public:
+  explicit Kept(const at::Tensor& t) : saved_(t, false) {
+    if (!t.defined()) return;
+    sizes_ = t.sizes().vec();
+    dtype_ = t.scalar_type();
+    device_ = t.device();
+  }
+  at::Tensor get(const std::shared_ptr<torch::autograd::Node>& node) const {
+    at::Tensor t = saved_.unpack(node);
+    if (!t.defined()) return t;
+    TORCH_CHECK(t.sizes() == sizes_ && t.scalar_type() == dtype_ && t.device() == device_,
+                "sage_net: a saved-tensor hook gave back a tensor of another shape, type or device");
+    return t.contiguous();
+  }
+
+ private:
+  SavedVariable saved_;
+  std::vector<int64_t> sizes_;
+  at::ScalarType dtype_ = at::kFloat;
+  at::Device device_ = at::kCPU;
+};
+
+// One layer of what the backward pass needs: inputs of the products (x1 is also the previous layer's output), what the ReLU gave and
+// dropout's mask (not in the last layer; undefined without dropout), the block (not in the first layer).
+template <typename T>
+struct PerLayer { T x1, x2, active, keep, indptr, indices; };
+
 struct SageBackward : public torch::autograd::Node {
   Net net;
-  std::vector<SavedVariable> weights;   // per layer: self, neigh, bias
-  std::vector<at::Tensor> x1, x2;       // inputs of the layers' products
-  std::vector<at::Tensor> out, active, keep;  // all layers but the last: output, what the ReLU gave, dropout's mask (undefined: none)
+  std::vector<Kept> weights;            // per layer: self, neigh, bias
+  std::vector<PerLayer<Kept>> layers;
   bool released = false;
 
   std::string name() const override { return "SageBackward"; }
   void release_variables() override {
     released = true;
-    weights.clear(); x1.clear(); x2.clear(); out.clear(); active.clear(); keep.clear();
+    weights.clear(); layers.clear();
   }
 
   variable_list apply(variable_list&& grads) override {
@@ -169,7 +198,7 @@ struct SageBackward : public torch::autograd::Node {
     if (net.layers.size() == 1) return one_layer_with_graph(grads[0]);
     variable_list result = gradients(grads[0]), from = {grads[0]};
     auto self = shared_from_this();
-    for (const SavedVariable& w : weights) from.push_back(w.unpack(self));
+    for (const Kept& w : weights) from.push_back(w.get(self));
     if (!torch::autograd::compute_requires_grad(from)) return result;
     auto node = std::shared_ptr<NotTwice>(new NotTwice(), torch::autograd::deleteNode);
     node->set_next_edges(torch::autograd::collect_next_edges(from));
@@ -187,10 +216,12 @@ struct SageBackward : public torch::autograd::Node {
   // A single layer is linear in the gradient that it is given, so torch's own products make the graph.
   variable_list one_layer_with_graph(const at::Tensor& given) {
     const at::Tensor dy = given.to(at::kFloat), turned = dy.t();
+    auto self = shared_from_this();
+    const at::Tensor x1 = layers[0].x1.get(self).narrow(0, 0, dy.size(0)), x2 = layers[0].x2.get(self).narrow(0, 0, dy.size(0));
     auto of = [&](size_t i, auto&& make) { return task_should_compute_output(i) ? make() : at::Tensor(); };
-    auto bias = weights[2].unpack(shared_from_this());
-    return {of(0, [&] { return mm(net, turned, x1[0].narrow(0, 0, dy.size(0))); }), of(1, [&] { return mm(net, turned, x2[0].narrow(0, 0, dy.size(0))); }),
-            of(2, [&] { return bias.defined() ? dy.sum(0) : at::Tensor(); })};
+    const bool bias = weights[2].get(self).defined();
+    return {of(0, [&] { return mm(net, turned, x1); }), of(1, [&] { return mm(net, turned, x2); }),
+            of(2, [&] { return bias ? dy.sum(0) : at::Tensor(); })};
   }
 
   variable_list gradients(const at::Tensor& grad_output) {
@@ -206,17 +237,19 @@ struct SageBackward : public torch::autograd::Node {
     std::vector<at::Tensor> w(3 * L);
     int64_t biases = 0;
     for (size_t i = 0; i < 3 * L; ++i) {
-      w[i] = weights[i].unpack(self);
+      w[i] = weights[i].get(self);
       if (i % 3 == 2 && w[i].defined()) biases += (w[i].numel() + 63) / 64 * 64;
     }
+    std::vector<PerLayer<at::Tensor>> of;
+    for (const PerLayer<Kept>& l : layers)
+      of.push_back({l.x1.get(self), l.x2.get(self), l.active.get(self), l.keep.get(self), l.indptr.get(self), l.indices.get(self)});
     at::Tensor bias_grads = empty({biases}, at::kFloat, given.device());  // the mask kernel adds to it
     // The weight gradients' products run over padded rows, where the gradients are zero; what they meet there must be finite.
     Zeros zeros;
     zeros.add(bias_grads.data_ptr(), biases * 4);
     for (size_t i = 0; i < L; ++i) {
-      if (i == 0) zeros.tail(x1[0], net.layers[0].rows);
-      zeros.tail(x2[i], net.layers[i].rows);
-      if (i + 1 < L) zeros.tail(out[i], net.layers[i].rows);
+      zeros.tail(of[i].x1, net.layers[i == 0 ? 0 : i - 1].rows);
+      zeros.tail(of[i].x2, net.layers[i].rows);
     }
 
     // gradient of the last layer's output on its padded rows
@@ -244,8 +277,8 @@ struct SageBackward : public torch::autograd::Node {
       at::Tensor dy = g;
       if (i + 1 < L) {
         dy = empty({m, n}, at::kFloat, g.device());
-        checked = f2c_sage_mask_dropout(f32(g), f32(active[i]), keep[i].defined() ? (const uint8_t*)keep[i].data_ptr() : nullptr, (float)net.scale(),
-                                        f32(dy), db.defined() ? f32(db) : nullptr, m, n, st);
+        checked = f2c_sage_mask_dropout(f32(g), f32(of[i].active), of[i].keep.defined() ? (const uint8_t*)of[i].keep.data_ptr() : nullptr,
+                                        (float)net.scale(), f32(dy), db.defined() ? f32(db) : nullptr, m, n, st);
       } else if (db.defined()) {
         checked = f2c_sage_mask(f32(dy), nullptr, 1.0f, nullptr, f32(db), m, n, st);
       }
@@ -256,22 +289,22 @@ struct SageBackward : public torch::autograd::Node {
         side.fork.record(main);
         side.fork.block(*side.stream);
         c10::cuda::CUDAStreamGuard on_side(*side.stream);
-        product(net, d_nb, dy, true, x2[i], false);
-        if (i > 0) product(net, d_self, dy, true, x1[i], false);
+        product(net, d_nb, dy, true, of[i].x2, false);
+        if (i > 0) product(net, d_self, dy, true, of[i].x1, false);
         side.join.record(*side.stream);
         forked = true;
         read_beside.push_back(dy);
       } else {
-        product(net, d_nb, dy, true, x2[i], false);
-        if (i > 0) product(net, d_self, dy, true, x1[i], false);
+        product(net, d_nb, dy, true, of[i].x2, false);
+        if (i > 0) product(net, d_self, dy, true, of[i].x1, false);
       }
-      if (i == 0) product(net, d_self, dy, true, x1[i], false);
+      if (i == 0) product(net, d_self, dy, true, of[i].x1, false);
       if (i > 0) {
         at::Tensor dh = empty({net.layers[i - 1].padded, k}, at::kFloat, g.device());  // gradient of the previous layer's output
         at::Tensor d_rows = empty({m, k}, at::kFloat, g.device());
         product(net, d_rows, dy, false, wi[1], false);
-        checked = f2c_spmm_csr_backward(f32(d_rows), l.indptr.data_ptr(), l.indices.data_ptr(), dtype_tag(l.indptr.scalar_type()), f32(dh), l.rows,
-                                        dh.size(0), k, F2C_MEAN, st);
+        checked = f2c_spmm_csr_backward(f32(d_rows), of[i].indptr.data_ptr(), of[i].indices.data_ptr(), dtype_tag(of[i].indptr.scalar_type()), f32(dh),
+                                        l.rows, dh.size(0), k, F2C_MEAN, st);
         at::Tensor head = dh.narrow(0, 0, m);
         product(net, head, dy, false, wi[0], true);
         g = dh;
@@ -336,6 +369,7 @@ PyObject* sage_net(PyObject*, PyObject* const* a, Py_ssize_t n) {
         node->set_next_edges(torch::autograd::collect_next_edges(w));
       }
       at::Tensor h;
+      std::vector<PerLayer<at::Tensor>> of;
       {
         at::AutoDispatchBelowADInplaceOrView below;
         at::Tensor x1 = h_self, x2 = h_neigh;
@@ -355,20 +389,15 @@ PyObject* sage_net(PyObject*, PyObject* const* a, Py_ssize_t n) {
             if (net.p < 1 && h.numel() > 0) std::tie(h, keep) = at::native_dropout(h, net.p, true);
             else h = at::dropout(h, net.p, true);
           }
-          if (record) {
-            node->x1.push_back(x1);
-            node->x2.push_back(x2);
-            if (!last) {
-              node->out.push_back(h);
-              node->active.push_back(active);
-              node->keep.push_back(keep);
-            }
-          }
+          if (record) of.push_back({x1, x2, last ? at::Tensor() : active, keep, l.indptr, l.indices});
         }
         if (h.size(0) > net.layers[L - 1].rows) h = h.narrow(0, 0, net.layers[L - 1].rows);
       }
       if (record) {
-        for (const at::Tensor& t : w) node->weights.emplace_back(t, false);
+        for (const at::Tensor& t : w) node->weights.emplace_back(t);
+        for (const PerLayer<at::Tensor>& l : of)
+          node->layers.push_back({Kept(l.x1), Kept(l.x2), Kept(l.active), Kept(l.keep), Kept(l.indptr), Kept(l.indices)});
+        for (Layer& l : net.layers) l.indptr = l.indices = at::Tensor();
         node->net = std::move(net);
         torch::autograd::set_history(h, node);
       }

@@ -483,3 +483,37 @@ def test_gradients_with_a_graph(capi, layers):
     grads = torch.autograd.grad(model(blocks).square().mean(), params, create_graph=True)
     sum(x.square().sum() for x in grads).backward()
     assert all(torch.allclose(a, p.grad, rtol=1e-4, atol=1e-6) for a, p in zip(got, params))
+
+
+def test_saved_tensor_hooks_see_the_activations(capi):
+    """What the backward pass needs goes through saved-tensor hooks (here: kept on the host) and checkpoint(): same gradients, and
+    the activations are among it.  A hook that gives back something else is refused."""
+    from torch.autograd.graph import saved_tensors_hooks
+    from torch.utils.checkpoint import checkpoint
+    model, blocks, g = _small_network(0.5)
+    weight = torch.randn(233, 10, generator=g, device="cuda")
+    seen = []
+
+    def pack(t):
+        seen.append(t.numel())
+        return t.cpu()
+
+    def run(forward):
+        torch.manual_seed(3)
+        model.zero_grad(set_to_none=True)
+        out = forward()
+        out.backward(weight)
+        return [out.detach()] + [p.grad.clone() for p in model.parameters()]
+
+    def hooked(unpack):
+        with saved_tensors_hooks(pack, unpack):
+            return model(blocks)
+    want = run(lambda: model(blocks))
+    rows = blocks[0]["dst_nodes"].numel()
+    for got in (run(lambda: hooked(lambda t: t.cuda())), run(lambda: checkpoint(model, blocks, use_reentrant=False))):
+        for a, b in zip(want, got):
+            assert torch.allclose(a, b, rtol=1e-4, atol=1e-5)
+    assert sum(n >= rows * 64 for n in seen) >= 5  # both inputs of the first two layers, what the first ReLU gave
+    for bad in (lambda t: t, lambda t: t.cuda()[:1], lambda t: t.cuda().double()):
+        with pytest.raises(RuntimeError):
+            run(lambda: hooked(bad))
