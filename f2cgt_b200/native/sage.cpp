@@ -13,6 +13,7 @@
 #include "native.h"
 
 #include <array>
+#include <atomic>
 
 #include <ATen/cuda/CUDAEvent.h>
 #include <cublas_v2.h>
@@ -36,9 +37,12 @@ struct Net {
   std::vector<Layer> layers;
   double p = 0.0;                     // dropout between the layers (0 outside training)
   bool tf32 = false;                  // forward products may be the library's
-  c10::optional<at::ScalarType> cast; // operand type of torch's products
+  c10::optional<at::ScalarType> cast; // operand type of torch's products (backward pass: the type in force then)
   double scale() const { return p < 1.0 ? 1.0 / (1.0 - p) : 0.0; }
 };
+
+// Operand type of torch's products in force (sage.products_in): a scalar type, or -1.
+std::atomic<int> g_product_type{-1};
 
 struct Status {  // library status inside a node (no Python exception there)
   void operator=(int rc) const { TORCH_CHECK(rc == F2C_OK, "f2cgt_b200: ", f2c_last_error()); }
@@ -193,6 +197,8 @@ struct SageBackward : public torch::autograd::Node {
   variable_list apply(variable_list&& grads) override {
     TORCH_CHECK(!released, "Trying to backward through the graph a second time: its saved tensors have been freed");
     if (!grads[0].defined()) return variable_list(3 * net.layers.size());
+    const int type = g_product_type.load();
+    net.cast = type < 0 ? c10::nullopt : c10::make_optional((at::ScalarType)type);
     if (!at::GradMode::is_enabled()) return gradients(grads[0]);
     // create_graph: the gradients are to be differentiable themselves
     if (net.layers.size() == 1) return one_layer_with_graph(grads[0]);
@@ -407,8 +413,18 @@ PyObject* sage_net(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
+PyObject* product_type(PyObject*, PyObject* o) {  // torch.dtype or None
+  return guarded([&]() -> PyObject* {
+    if (o != Py_None && !THPDtype_Check(o)) fail(PyExc_TypeError, "product_type: a torch.dtype or None");
+    g_product_type = o == Py_None ? -1 : (int)reinterpret_cast<THPDtype*>(o)->scalar_type;
+    Py_RETURN_NONE;
+  });
+}
+
 }  // namespace
 
-PyMethodDef g_sage_methods[] = {{"sage_net", (PyCFunction)(void*)sage_net, METH_FASTCALL, nullptr}, {nullptr, nullptr, 0, nullptr}};
+PyMethodDef g_sage_methods[] = {{"sage_net", (PyCFunction)(void*)sage_net, METH_FASTCALL, nullptr},
+                                {"product_type", product_type, METH_O, nullptr},
+                                {nullptr, nullptr, 0, nullptr}};
 
 }  // namespace f2c_native

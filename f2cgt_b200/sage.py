@@ -193,13 +193,17 @@ class products_in:
     def __init__(self, dtype):
         self.dtype = dtype
 
-    def __enter__(self):
+    def _set(self, dtype):
         global _PRODUCT_DTYPE
-        self.before, _PRODUCT_DTYPE = _PRODUCT_DTYPE, self.dtype
+        _PRODUCT_DTYPE = dtype
+        ops._native.product_type(dtype)  # the network's backward pass takes what is in force when it runs, as the layers' do
+
+    def __enter__(self):
+        self.before = _PRODUCT_DTYPE
+        self._set(self.dtype)
 
     def __exit__(self, *exc):
-        global _PRODUCT_DTYPE
-        _PRODUCT_DTYPE = self.before
+        self._set(self.before)
 
 
 def _mm(a, b):

@@ -517,3 +517,26 @@ def test_saved_tensor_hooks_see_the_activations(capi):
     for bad in (lambda t: t, lambda t: t.cuda()[:1], lambda t: t.cuda().double()):
         with pytest.raises(RuntimeError):
             run(lambda: hooked(bad))
+
+
+@pytest.mark.parametrize("forward,backward", [(torch.bfloat16, None), (None, torch.bfloat16)])
+def test_products_have_the_type_in_force_when_they_run(capi, forward, backward):
+    """Operand type of the forward products and of the backward products: each that of its own time, as with the layers on their
+    own.  Bound: values that differ by some 1e-6 (sums in another order) round to different bf16 numbers, 2^-8 apart, once in
+    1e-6 / 2^-8 times, so operands and results are off by 2^-8 sqrt(2.6e-4) = 6e-5 each, about 1e-4 together; 5e-4 is asked, and
+    products of the other type would be off by 4.6e-3."""
+    from f2cgt_b200 import sage
+    model, blocks, g = _small_network(0.0)
+    weight = torch.randn(233, 10, generator=g, device="cuda")
+    got = []
+    for one_node in (True, False):
+        if not one_node:
+            model.layers[1].register_forward_pre_hook(lambda *_: None)
+        model.zero_grad(set_to_none=True)
+        with sage.products_in(forward):
+            out = model(blocks)
+        with sage.products_in(backward):
+            out.backward(weight)
+        got.append([p.grad for p in model.parameters()])
+    for a, b in zip(*got):
+        assert float((a - b).norm() / b.norm()) < 5e-4
