@@ -11,18 +11,21 @@ namespace f2c {
 namespace {
 
 constexpr int kThreads = 256;
+constexpr int kPartCols = 8192;  // columns whose sums a CTA holds; wider rows are cut into parts (grid.y)
 
 enum Mask { kSums, kRelu, kReluDropout };  // only the column sums of g; h; h and keep
 
 template <bool VEC, Mask MASK>
 __global__ void __launch_bounds__(kThreads) sage_mask_kernel(const float* __restrict__ g, const float* __restrict__ h, const uint8_t* __restrict__ keep,
-                                                             float scale, float* __restrict__ dy, float* __restrict__ db, int64_t rows, int n,
-                                                             int units) {
+                                                             float scale, float* __restrict__ dy, float* __restrict__ db, int64_t rows,
+                                                             int64_t n) {
   dependency_wait();
   release_dependents();
   constexpr int E = VEC ? 4 : 1;
   extern __shared__ float sums[];
-  for (int i = threadIdx.x; i < n; i += kThreads) sums[i] = 0.0f;
+  const int64_t col0 = (int64_t)blockIdx.y * kPartCols;
+  const int cols = (int)(n - col0 < kPartCols ? n - col0 : kPartCols), units = cols / E;
+  for (int i = threadIdx.x; i < cols; i += kThreads) sums[i] = 0.0f;
   __syncthreads();
   const int lanes = units < kThreads ? kThreads / units : 1;  // rows a CTA works on at a time
   const int local = units < kThreads ? (int)threadIdx.x / units : 0;
@@ -36,7 +39,7 @@ __global__ void __launch_bounds__(kThreads) sage_mask_kernel(const float* __rest
     const int c = u * E;
 #pragma unroll 4
     for (int64_t r = (int64_t)blockIdx.x * lanes + local; r < rows; r += step) {
-      const int64_t at = r * n + c;
+      const int64_t at = r * n + col0 + c;
       if (VEC) {
         float4 v = __ldcs(reinterpret_cast<const float4*>(g + at));
         if (MASK != kSums) {
@@ -64,7 +67,7 @@ __global__ void __launch_bounds__(kThreads) sage_mask_kernel(const float* __rest
   }
   if (db == nullptr) return;
   __syncthreads();
-  for (int i = threadIdx.x; i < n; i += kThreads) atomicAdd(db + i, sums[i]);
+  for (int i = threadIdx.x; i < cols; i += kThreads) atomicAdd(db + col0 + i, sums[i]);
 }
 
 }  // namespace
@@ -75,18 +78,19 @@ using namespace f2c;
 extern "C" int f2c_sage_mask_dropout(const float* g, const float* h, const uint8_t* keep, float scale, float* dy, float* db, int64_t rows, int64_t n,
                                      void* stream) {
   const char* op = "sage_mask";
-  F2C_REQUIRE(rows >= 0 && n >= 0 && n <= 8192, F2C_ERR_LIMIT, "%s: bad shape", op);
+  F2C_REQUIRE(rows >= 0 && n >= 0 && n <= (int64_t)kPartCols * 65535, F2C_ERR_LIMIT, "%s: bad shape", op);
   if (rows * n == 0) return F2C_OK;
   F2C_REQUIRE(g && (h != nullptr ? dy != nullptr : db != nullptr && keep == nullptr), F2C_ERR_INVALID, "%s: null pointer", op);
   const bool vec = n % 4 == 0 && aligned(g, 16) && aligned(h, 16) && aligned(dy, 16) && aligned(keep, 4);
-  const int units = (int)(vec ? n / 4 : n);
+  const int cols = (int)(n < kPartCols ? n : kPartCols), units = vec ? cols / 4 : cols;
   const int lanes = units < kThreads ? kThreads / units : 1;
   int64_t grid = ceil_div(rows, (int64_t)lanes * 4);
   if (grid > 8 * current_sm_count()) grid = 8 * current_sm_count();
   auto kern = h == nullptr      ? (vec ? sage_mask_kernel<true, kSums> : sage_mask_kernel<false, kSums>)
               : keep == nullptr ? (vec ? sage_mask_kernel<true, kRelu> : sage_mask_kernel<false, kRelu>)
                                 : (vec ? sage_mask_kernel<true, kReluDropout> : sage_mask_kernel<false, kReluDropout>);
-  launch_dependent(kern, (unsigned)grid, kThreads, (size_t)n * 4, (cudaStream_t)stream, g, h, keep, scale, dy, db, rows, (int)n, units);
+  launch_dependent(kern, dim3((unsigned)grid, (unsigned)ceil_div(n, kPartCols)), kThreads, (size_t)cols * 4, (cudaStream_t)stream, g, h, keep, scale,
+                   dy, db, rows, n);
   return check_launch(op);
 }
 

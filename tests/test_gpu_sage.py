@@ -540,3 +540,36 @@ def test_products_have_the_type_in_force_when_they_run(capi, forward, backward):
         got.append([p.grad for p in model.parameters()])
     for a, b in zip(*got):
         assert float((a - b).norm() / b.norm()) < 5e-4
+
+
+@pytest.mark.parametrize("rows,n", [(40, 8191), (40, 8192), (37, 8193), (9, 16_388), (3, 30_000)])
+def test_relu_dropout_gradient_of_wide_rows(capi, rows, n):
+    from f2cgt_b200 import ops
+    from f2cgt_b200._lib import check, lib
+    g = torch.Generator(device="cuda").manual_seed(n)
+    grad, h = torch.randn(rows, n, generator=g, device="cuda"), torch.randn(rows, n, generator=g, device="cuda")
+    keep = torch.rand(rows, n, generator=g, device="cuda") < 0.5
+    dy, db = torch.empty_like(grad), torch.zeros(n, device="cuda")
+    check(lib.f2c_sage_mask_dropout(grad.data_ptr(), h.data_ptr(), keep.data_ptr(), 2.0, dy.data_ptr(), db.data_ptr(), rows, n, ops._stream(h)))
+    want = torch.where(h > 0, grad * keep * 2.0, 0.0)
+    assert torch.equal(dy, want) and torch.allclose(db.double(), want.double().sum(0), rtol=1e-5, atol=1e-5 * rows**0.5)
+
+
+def _one_node_and_layers(model, blocks, weight):
+    got = []
+    for one_node in (True, False):
+        if not one_node:
+            model.layers[1].register_forward_pre_hook(lambda *_: None)  # a hook: layer by layer
+        assert (model._plain_weights() is not None) == one_node
+        model.zero_grad(set_to_none=True)
+        out = model(blocks)
+        out.backward(weight)
+        got.append([out.detach()] + [p.grad for p in model.parameters()])
+    return got
+
+
+@pytest.mark.parametrize("classes,hidden", [(10_000, 64), (10, 9001)])
+def test_network_of_many_columns(capi, classes, hidden):
+    model, blocks, g = _small_network(0.0, classes=classes, hidden=hidden, layers=2)
+    for a, b in zip(*_one_node_and_layers(model, blocks, torch.randn(233, classes, generator=g, device="cuda"))):
+        assert float((a - b).norm()) <= 1e-4 * float(b.norm())
