@@ -73,19 +73,25 @@ bool use_own(const Net& net, int64_t rows, int64_t n, int64_t k, bool record) {
   return net.tf32 && k % 4 == 0 && k <= 65536 && n <= 65536 && rows > 1 && (!record || k % 32 == 0 || rows >= 16384);
 }
 
-// Ranges to be set to zero in one launch: a memset each costs the host as much as a kernel.
+// Ranges to be set to zero, as many in one launch as it takes: a memset each costs the host as much as a kernel.
 struct Zeros {
-  void* at[32];
-  int64_t bytes[32];
+  static constexpr int kMost = 32;  // of f2c_zero_ranges
+  explicit Zeros(cudaStream_t stream) : st(stream) {}
+  cudaStream_t st;
+  void* at[kMost];
+  int64_t bytes[kMost];
   int count = 0;
   void add(void* p, int64_t n) {
     if (n <= 0) return;
-    TORCH_CHECK(count < 32, "sage_net: too many layers");
+    if (count == kMost) run();
     at[count] = p;
     bytes[count++] = n;
   }
   void tail(const at::Tensor& t, int64_t rows) { add(f32(t) + rows * t.size(1), (t.size(0) - rows) * t.size(1) * 4); }
-  void run(cudaStream_t st) { checked = f2c_zero_ranges(at, bytes, count, st); }
+  void run() {
+    checked = f2c_zero_ranges(at, bytes, count, st);
+    count = 0;
+  }
 };
 
 // Products of the backward pass as at::mm computes them (same library call, same operands), without its dispatch: out is
@@ -251,7 +257,7 @@ struct SageBackward : public torch::autograd::Node {
       of.push_back({l.x1.get(self), l.x2.get(self), l.active.get(self), l.keep.get(self), l.indptr.get(self), l.indices.get(self)});
     at::Tensor bias_grads = empty({biases}, at::kFloat, given.device());  // the mask kernel adds to it
     // The weight gradients' products run over padded rows, where the gradients are zero; what they meet there must be finite.
-    Zeros zeros;
+    Zeros zeros(st);
     zeros.add(bias_grads.data_ptr(), biases * 4);
     for (size_t i = 0; i < L; ++i) {
       zeros.tail(of[i].x1, net.layers[i == 0 ? 0 : i - 1].rows);
@@ -266,7 +272,7 @@ struct SageBackward : public torch::autograd::Node {
       zeros.tail(padded, g.size(0));
       g = padded;
     }
-    zeros.run(st);
+    zeros.run();
     Beside& side = beside(given.device().index());
     bool forked = false;
     std::vector<at::Tensor> read_beside;  // what the side stream reads, until the streams have joined

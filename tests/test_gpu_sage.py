@@ -573,3 +573,16 @@ def test_network_of_many_columns(capi, classes, hidden):
     model, blocks, g = _small_network(0.0, classes=classes, hidden=hidden, layers=2)
     for a, b in zip(*_one_node_and_layers(model, blocks, torch.randn(233, classes, generator=g, device="cuda"))):
         assert float((a - b).norm()) <= 1e-4 * float(b.norm())
+
+
+def test_network_of_many_layers(capi):
+    from f2cgt_b200 import sage
+    first, blocks, g = _small_network(0.0, layers=1)
+    rows = blocks[0]["dst_nodes"].numel()
+    around = torch.arange(rows, device="cuda")
+    ring = dict(indptr=torch.arange(rows + 1, device="cuda"), indices_local=around.roll(1), dst_nodes=blocks[0]["dst_nodes"], n_edges=rows)
+    torch.manual_seed(2)
+    model = sage.SAGE(128, 16, 5, 20, 0.0, first.layers[0].sm).cuda()
+    got = _one_node_and_layers(model, list(blocks) + [ring] * 19, torch.randn(rows, 5, generator=g, device="cuda"))
+    for a, b in zip(*got):
+        assert float((a - b).norm()) <= 1e-4 * float(b.norm())
