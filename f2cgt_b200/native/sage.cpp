@@ -69,8 +69,12 @@ void addmm_(const Net& net, at::Tensor& y, const at::Tensor& a, const at::Tensor
 // Whether a layer's forward product is the library's kernel.  Its result equals torch's two products bit for bit for k % 32 == 0
 // (checked for k = 64 .. 256, n = 16 .. 256, 2 .. 61,440 rows) and, for other k, from some ten thousand rows on; below that cuBLAS sums in
 // another order, which a training run would notice (see above) and inference does not.
-bool use_own(const Net& net, int64_t rows, int64_t n, int64_t k, bool record) {
-  return net.tf32 && k % 4 == 0 && k <= 65536 && n <= 65536 && rows > 1 && (!record || k % 32 == 0 || rows >= 16384);
+bool use_own(const Net& net, const at::Tensor& x1, const at::Tensor& x2, const at::Tensor& w1, const at::Tensor& w2, int64_t rows, bool record) {
+  const int64_t n = w1.size(0), k = w1.size(1);
+  if (!net.tf32 || k % 4 != 0 || k > 65536 || n > 65536 || rows <= 1) return false;
+  for (const at::Tensor* t : {&x1, &x2, &w1, &w2})  // parameters may be views into a flat buffer
+    if ((reinterpret_cast<uintptr_t>(t->data_ptr()) & 15) != 0) return false;
+  return !record || k % 32 == 0 || rows >= 16384;
 }
 
 // Ranges to be set to zero, as many in one launch as it takes: a memset each costs the host as much as a kernel.
@@ -114,7 +118,7 @@ void product(const Net& net, at::Tensor& out, const at::Tensor& a, bool a_turned
 at::Tensor layer_forward(const Net& net, const at::Tensor& x1, const at::Tensor& x2, const at::Tensor* w, const Layer& l, bool relu, bool record,
                          cudaStream_t st) {
   const at::Tensor &w1 = w[0], &w2 = w[1], &bias = w[2];
-  if (use_own(net, l.rows, w1.size(0), w1.size(1), record)) {
+  if (use_own(net, x1, x2, w1, w2, l.rows, record)) {
     at::Tensor y = empty({l.padded, w1.size(0)}, at::kFloat, x1.device());
     checked = f2c_sage_forward(f32(x1), f32(x2), f32(w1), f32(w2), bias.defined() ? f32(bias) : nullptr, f32(y), l.rows, w1.size(0), w1.size(1),
                                relu ? 1 : 0, st);

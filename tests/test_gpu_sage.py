@@ -586,3 +586,30 @@ def test_network_of_many_layers(capi):
     got = _one_node_and_layers(model, list(blocks) + [ring] * 19, torch.randn(rows, 5, generator=g, device="cuda"))
     for a, b in zip(*got):
         assert float((a - b).norm()) <= 1e-4 * float(b.norm())
+
+
+@pytest.mark.parametrize("shift", [0, 1, 2, 3])
+def test_weights_that_are_views_of_a_flat_buffer(capi, shift):
+    """Parameters that start anywhere in one buffer: same outputs (to tf32's 10 bits, sums in another order) and gradients."""
+    model, blocks, g = _small_network(0.0)
+    weight = torch.randn(233, 10, generator=g, device="cuda")
+    before = torch.backends.cuda.matmul.allow_tf32
+    torch.backends.cuda.matmul.allow_tf32 = True
+    try:
+        got = []
+        for flat in (False, True):
+            if flat:
+                buffer, at = torch.empty(sum(p.numel() + 3 for p in model.parameters()) + 4, device="cuda"), shift
+                for p in model.parameters():
+                    part = buffer[at:at + p.numel()].view_as(p)
+                    part.copy_(p.data)
+                    p.data = part
+                    at += p.numel() + 3
+            model.zero_grad(set_to_none=True)
+            out = model(blocks)
+            out.backward(weight)
+            got.append([out.detach()] + [p.grad for p in model.parameters()])
+        for a, b in zip(*got):
+            assert float((a - b).norm() / b.norm()) < 5e-3
+    finally:
+        torch.backends.cuda.matmul.allow_tf32 = before
