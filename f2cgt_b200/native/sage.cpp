@@ -66,15 +66,21 @@ void addmm_(const Net& net, at::Tensor& y, const at::Tensor& a, const at::Tensor
   if (net.cast) y.add_(mm(net, a, b)); else y.addmm_(a, b);
 }
 
-// Whether a layer's forward product is the library's kernel.  Its result equals torch's two products bit for bit for k % 32 == 0
-// (checked for k = 64 .. 256, n = 16 .. 256, 2 .. 61,440 rows) and, for other k, from some ten thousand rows on; below that cuBLAS sums in
-// another order, which a training run would notice (see above) and inference does not.
+// Whether a layer's forward product is the library's kernel.  Both sides round operands to tf32 (2.9e-4 off in float64 terms for either)
+// except for one column or one row, where cuBLAS takes a matrix-vector product in fp32 (1e-7): those stay there.  Under a training run
+// (record) the result has to be the two library products' bit for bit (see above).  It is for k % 32 == 0 from 2 rows on, for k % 8 == 0
+// (checked for k = 8 .. 512, n = 4 .. 300, 2 .. 73,728 rows), and for k % 8 == 4, where cuBLAS adds in another order for few rows and for
+// few columns or odd numbers of them, from 32,768 rows of 64 columns on (k = 20 .. 300, n = 64 .. 256 in fours, to 102,400 rows; at 64 columns
+// 28,672 rows still differ).  k % 8 == 0 below 16,384 rows is left to cuBLAS, where a step has been timed that way only.
+// tests/test_gpu_sage.py compares both sides over this range: with another cuBLAS it tells whether the rule still holds.
 bool use_own(const Net& net, const at::Tensor& x1, const at::Tensor& x2, const at::Tensor& w1, const at::Tensor& w2, int64_t rows, bool record) {
   const int64_t n = w1.size(0), k = w1.size(1);
-  if (!net.tf32 || k % 4 != 0 || k > 65536 || n > 65536 || rows <= 1) return false;
+  if (!net.tf32 || k % 4 != 0 || k > 65536 || n < 2 || n > 65536 || rows < 2) return false;
   for (const at::Tensor* t : {&x1, &x2, &w1, &w2})  // parameters may be views into a flat buffer
     if ((reinterpret_cast<uintptr_t>(t->data_ptr()) & 15) != 0) return false;
-  return !record || k % 32 == 0 || rows >= 16384;
+  if (!record) return true;
+  if (n < 4) return false;  // (two columns of k = 512: another order)
+  return k % 32 == 0 || (k % 8 == 0 && rows >= 16384) || (n % 4 == 0 && n >= 64 && rows >= 32768);
 }
 
 // Ranges to be set to zero, as many in one launch as it takes: a memset each costs the host as much as a kernel.

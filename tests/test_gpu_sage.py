@@ -613,3 +613,43 @@ def test_weights_that_are_views_of_a_flat_buffer(capi, shift):
             assert float((a - b).norm() / b.norm()) < 5e-3
     finally:
         torch.backends.cuda.matmul.allow_tf32 = before
+
+
+@pytest.mark.parametrize("k,ms,ns", [(32, (2, 3, 128, 1024, 61_440), (4, 47, 256)), (64, (2, 128, 3072, 16_384), (10, 64, 172)), (128, (2, 640, 8192, 61_440), (4, 47, 128, 172)),
+                                     (256, (17, 2048, 40_960), (10, 128, 256, 300)), (104, (16_384, 28_672), (5, 64, 128)), (200, (16_384, 53_248), (47, 128, 256)),
+                                     (36, (32_768, 65_536), (64, 68, 128)), (100, (32_768, 40_960, 102_400), (64, 100, 128, 256)), (300, (32_768, 49_152), (64, 172))])
+def test_layer_product_equals_the_library_products_bit_for_bit(capi, k, ms, ns):
+    """Where a training network takes the library's own product it must not change a bit of what torch's two products give
+    (use_own() in native/sage.cpp)."""
+    from f2cgt_b200 import ops
+    from f2cgt_b200._lib import check, lib
+    g = torch.Generator(device="cuda").manual_seed(k)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    before = torch.backends.cuda.matmul.allow_tf32
+    torch.backends.cuda.matmul.allow_tf32 = True
+    try:
+        for m in ms:
+            for n in ns:
+                x1, x2, w1, w2, b = rnd(m, k), rnd(m, k), rnd(n, k), rnd(n, k), rnd(n)
+                y = torch.empty((m, n), device="cuda")
+                check(lib.f2c_sage_forward(x1.data_ptr(), x2.data_ptr(), w1.data_ptr(), w2.data_ptr(), b.data_ptr(), y.data_ptr(), m, n, k, 0, ops._stream(x1)))
+                assert torch.equal(y, torch.addmm(b, x1, w1.t()).addmm_(x2, w2.t())), (m, n, k)
+    finally:
+        torch.backends.cuda.matmul.allow_tf32 = before
+
+
+@pytest.mark.parametrize("classes", [1, 2, 47])
+def test_outputs_of_the_network_equal_the_layers_bit_for_bit(capi, classes):
+    """tf32 products allowed, with gradients: the one-node network gives the layers' outputs.  One output column: fp32 in both."""
+    before = torch.backends.cuda.matmul.allow_tf32
+    torch.backends.cuda.matmul.allow_tf32 = True
+    try:
+        model, blocks, g = _small_network(0.0, classes=classes, hidden=128)
+        got = _one_node_and_layers(model, blocks, torch.randn(233, classes, generator=g, device="cuda"))
+        assert torch.equal(got[0][0], got[1][0])
+        with torch.no_grad():
+            for layer in model.layers:
+                layer._forward_pre_hooks.clear()
+            assert model._plain_weights() is not None and torch.equal(model(blocks), got[0][0])
+    finally:
+        torch.backends.cuda.matmul.allow_tf32 = before
