@@ -357,9 +357,12 @@ class SAGE(nn.Module):
         return h if h.shape[0] == n_out else h[:n_out]
 
     def _plain_weights(self):
-        """[self, neigh, bias] of every layer, or None when the layers are not just these tensors (subclasses, hooks,
-        parametrisations, other dtypes, autocast): then every layer is called on its own."""
-        if torch.is_autocast_enabled("cuda") or type(self.dropout) is not nn.Dropout or _hooked(self.dropout):
+        """[self, neigh, bias] of every layer, or None when the layers are not just these tensors (subclasses, hooks - those of
+        all modules too -, parametrisations, other dtypes, autocast, forward-mode derivatives): then every layer is called on its
+        own."""
+        if torch.is_autocast_enabled("cuda") or type(self.dropout) is not nn.Dropout or self.dropout.inplace or _hooked(self.dropout):
+            return None
+        if nn.modules.module._has_any_global_hook() or torch.autograd.forward_ad._current_level >= 0:
             return None
         weights = []
         for i, layer in enumerate(self.layers._modules.values()):

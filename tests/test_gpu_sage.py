@@ -653,3 +653,38 @@ def test_outputs_of_the_network_equal_the_layers_bit_for_bit(capi, classes):
             assert model._plain_weights() is not None and torch.equal(model(blocks), got[0][0])
     finally:
         torch.backends.cuda.matmul.allow_tf32 = before
+
+
+def test_hooks_of_all_modules_see_the_dropout_layers(capi):
+    model, blocks, _ = _small_network(0.5)
+    torch.manual_seed(3)
+    want, seen = model(blocks), []
+    handle = torch.nn.modules.module.register_module_forward_hook(lambda module, *_: seen.append(type(module).__name__))
+    try:
+        torch.manual_seed(3)
+        got = model(blocks)
+    finally:
+        handle.remove()
+    assert seen.count("Dropout") == 2 and torch.allclose(got, want, rtol=1e-4, atol=1e-4)
+
+
+def test_forward_mode_derivatives_are_refused_not_left_out(capi):
+    import torch.autograd.forward_ad as fwd
+    model, blocks, _ = _small_network(0.0)
+    with fwd.dual_level():
+        weights = {name: fwd.make_dual(p.detach(), torch.ones_like(p)) for name, p in model.named_parameters()}
+        with pytest.raises((RuntimeError, NotImplementedError)):
+            torch.func.functional_call(model, weights, (blocks,))
+
+
+def test_dropout_in_place_draws_its_own_masks(capi):
+    """nn.Dropout(inplace=True) draws from the generator as torch's in-place dropout does, with or without hooks on a layer."""
+    model, blocks, _ = _small_network(0.5)
+    model.dropout.inplace = True
+    got = []
+    for _ in range(2):
+        torch.manual_seed(3)
+        with torch.no_grad():
+            got.append(model(blocks))
+        model.layers[1].register_forward_pre_hook(lambda *_: None)
+    assert torch.allclose(got[0], got[1], rtol=1e-4, atol=1e-4)
