@@ -15,6 +15,9 @@ struct Set {
   cudaEvent_t built = nullptr, consumed = nullptr;
   bool lent = false;  // handed out before: its last user must be through before it is overwritten
   ~Set() {
+    // A minibatch may still be under construction on the loader's stream, in memory that other streams (and, for the header, the
+    // host) would get next.
+    if (built != nullptr) (void)cudaEventSynchronize(built);
     if (built != nullptr) (void)cudaEventDestroy(built);
     if (consumed != nullptr) (void)cudaEventDestroy(consumed);
   }

@@ -194,3 +194,18 @@ def test_minibatch_kernel_rejects_ids_outside_the_graph(capi):
             ops.sample_minibatch_finish(b)
         ops.sample_minibatch_launch(b, torch.tensor([1], device="cuda"))
         assert ops.sample_minibatch_finish(b)[1].tolist() == [1, 2]
+
+
+def test_buffers_stay_until_their_minibatch_is_built(capi):
+    """Buffers dropped while a minibatch is being built in them on another stream: their memory is not given back before the kernel
+    that writes to it is through."""
+    from f2cgt_b200 import ops, synth
+    indptr, indices = synth.power_law_graph(500_000, 20, 2.1, seed=1, device="cuda")
+    seeds = torch.arange(20_000, device="cuda")
+    side = torch.cuda.Stream()
+    for _ in range(5):
+        buffers = ops.MinibatchBuffers(indptr, indices, 20_000, [15, 15])
+        torch.cuda.synchronize()
+        ops.sample_minibatch_launch(buffers, seeds, stream=side)
+        del buffers
+        assert side.query()
