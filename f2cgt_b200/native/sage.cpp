@@ -284,8 +284,22 @@ struct SageBackward : public torch::autograd::Node {
     }
     zeros.run();
     Beside& side = beside(given.device().index());
-    bool forked = false;
     std::vector<at::Tensor> read_beside;  // what the side stream reads, until the streams have joined
+    // Joins the streams again, also when something below throws (out of memory): until then what the other stream reads and writes must
+    // not serve anybody else.
+    struct Join {
+      Beside& side;
+      const c10::cuda::CUDAStream& main;
+      bool forked = false;
+      void now() {
+        if (!std::exchange(forked, false)) return;
+        side.join.record(*side.stream);
+        side.join.block(main);
+      }
+      ~Join() {
+        try { now(); } catch (...) {}
+      }
+    } join{side, main};
     int64_t bias_at = 0;
     for (size_t i = L; i-- > 0;) {
       const Layer& l = net.layers[i];
@@ -310,11 +324,10 @@ struct SageBackward : public torch::autograd::Node {
       if (m >= kBesideRows) {
         side.fork.record(main);
         side.fork.block(*side.stream);
+        join.forked = true;
         c10::cuda::CUDAStreamGuard on_side(*side.stream);
         product(net, d_nb, dy, true, of[i].x2, false);
         if (i > 0) product(net, d_self, dy, true, of[i].x1, false);
-        side.join.record(*side.stream);
-        forked = true;
         read_beside.push_back(dy);
       } else {
         product(net, d_nb, dy, true, of[i].x2, false);
@@ -332,7 +345,7 @@ struct SageBackward : public torch::autograd::Node {
         g = dh;
       }
     }
-    if (forked) side.join.block(main);
+    join.now();
     for (size_t i = 0; i < 3 * L; ++i)
       if (!task_should_compute_output(i)) result[i] = at::Tensor();
     return result;
