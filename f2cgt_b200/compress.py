@@ -182,27 +182,30 @@ def sq_compress_features(features, target_bits, column_slice, hotness=None, samp
         ready = None
         ws = torch.empty((max(lanes, 1), (lib.f2c_sq_statistics_workspace() + 255) // 256 * 256), dtype=torch.uint8, device=features.device)
         samples = []  # alive until the host has read the results
-    for i in range(s_lo, s_hi):
-        gen.manual_seed(seed * 1000003 + i)  # per slice, so that the row is the same whichever rank computes it
-        lo, hi = i * column_slice, min((i + 1) * column_slice, D)
-        idx = None if direct and sample_size >= n else _sample_rows(n, sample_size, hotness, gen)
-        n_sample = n if idx is None else idx.numel()
-        if not direct or not _by_kernel(n_sample, hi - lo):
-            rows[i - s_lo] = sq_metadata((features if idx is None else features[idx])[:, lo:hi])
-            continue
-        lane = len(pending) % lanes
-        if streams[lane] is not main:
-            if ready is None or idx is not None:
-                ready = main.record_event()  # the features, the workspaces, the sample's row numbers
-            if idx is not None or len(pending) < lanes:
-                streams[lane].wait_event(ready)
-        _statistics(features, idx, n_sample, lo, hi - lo, stats[i - s_lo], ws[lane], streams[lane])
-        samples.append(idx)
-        pending.append((i - s_lo, n_sample * (hi - lo)))
+    try:
+        for i in range(s_lo, s_hi):
+            gen.manual_seed(seed * 1000003 + i)  # per slice, so that the row is the same whichever rank computes it
+            lo, hi = i * column_slice, min((i + 1) * column_slice, D)
+            idx = None if direct and sample_size >= n else _sample_rows(n, sample_size, hotness, gen)
+            n_sample = n if idx is None else idx.numel()
+            if not direct or not _by_kernel(n_sample, hi - lo):
+                rows[i - s_lo] = sq_metadata((features if idx is None else features[idx])[:, lo:hi])
+                continue
+            lane = len(pending) % lanes
+            if streams[lane] is not main:
+                if ready is None or idx is not None:
+                    ready = main.record_event()  # the features, the workspaces, the sample's row numbers
+                if idx is not None or len(pending) < lanes:
+                    streams[lane].wait_event(ready)
+            samples.append(idx)
+            pending.append((i - s_lo, n_sample * (hi - lo)))
+            _statistics(features, idx, n_sample, lo, hi - lo, stats[i - s_lo], ws[lane], streams[lane])
+    finally:  # an exception too: what the other streams read and write is given back when this call ends
+        if pending:
+            for side in streams:
+                if side is not main:
+                    main.wait_stream(side)
     if pending:
-        for side in streams:
-            if side is not main:
-                main.wait_stream(side)
         staging = torch.empty(stats.shape, dtype=torch.float64, pin_memory=True)
         staging.copy_(stats, non_blocking=True)
         torch.cuda.current_stream(features.device).synchronize()

@@ -157,3 +157,26 @@ def test_sample_statistics_equal_a_sort(capi, rows, D, col, width, sampled):
         got = out.tolist()
         assert got[:4] == want, (kind, got, want)
         assert abs(got[4] - float(part.double().mean())) <= 1e-12 * max(1.0, got[4])
+
+
+def test_failing_statistics_leave_no_work_behind(capi, monkeypatch):
+    """An exception between two slices: the caller's stream waits for what the other streams were given, since its memory is free
+    for others from then on."""
+    from f2cgt_b200 import compress
+    queue, calls = compress._statistics, []
+
+    def statistics(*args):
+        calls.append(0)
+        if len(calls) == 2:
+            raise MemoryError
+        queue(*args)
+        with torch.cuda.stream(args[-1]):
+            torch.cuda._sleep(200_000_000)  # about 0.1 s
+    x = torch.randn(3000, 64, device="cuda")
+    compress.sq_compress_features(x, 4, 16)
+    torch.cuda.synchronize()
+    monkeypatch.setattr(compress, "_statistics", statistics)
+    with pytest.raises(MemoryError):
+        compress.sq_compress_features(x, 4, 16)
+    assert not torch.cuda.current_stream().query()
+    torch.cuda.synchronize()
