@@ -148,7 +148,7 @@ template <int DMAX, int METRIC>
 __global__ void __launch_bounds__(kListThreads) kmeans_listed_kernel(const float* __restrict__ x, const float* __restrict__ y,
                                                                      int64_t* __restrict__ labels, const int32_t* __restrict__ list,
                                                                      const int32_t* __restrict__ count_dev, const int32_t* __restrict__ all_dev,
-                                                                     int64_t max_count, int k, int d, int kc, int y_vec4) {
+                                                                     int64_t max_count, int k, int d, int kc, int y_vec4, int y_settled) {
   constexpr int STRIDE = DMAX + 4;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float* yc_s = reinterpret_cast<float*>(smem_raw);  // [kc][STRIDE]
@@ -180,10 +180,10 @@ __global__ void __launch_bounds__(kListThreads) kmeans_listed_kernel(const float
       __syncthreads();
     }
   };
-  // The kernel before on the stream, which makes the list, has waited for the centres, so they may be staged before it is done.
-  if (kc >= k) stage(0, k);
+  if (kc >= k && y_settled) stage(0, k);  // while the kernel before, which makes the list, still runs
   dependency_wait();
   release_dependents();
+  if (kc >= k && !y_settled) stage(0, k);
   const bool all = all_dev != nullptr && *all_dev != 0;  // every point instead of the listed ones
   const int64_t cnt = !all && *count_dev < max_count ? *count_dev : max_count;
   const int lane = threadIdx.x & 31;
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(kListThreads) kmeans_listed_kernel(const float
 
 template <int DMAX>
 static int launch_listed(const float* x, const float* y, int64_t* labels, const int32_t* list, const int32_t* count_dev, const int32_t* all_dev,
-                         int64_t max_count, int64_t k, int64_t d, int metric, cudaStream_t st) {
+                         int64_t max_count, int64_t k, int64_t d, int metric, bool y_settled, cudaStream_t st) {
   int kc = (int)k;
   while ((size_t)kc * (DMAX + 5) * sizeof(float) > 96 * 1024) kc = (kc + 1) / 2;
   const size_t smem = (size_t)kc * (DMAX + 5) * sizeof(float);
@@ -270,7 +270,7 @@ static int launch_listed(const float* x, const float* y, int64_t* labels, const 
   int64_t grid = ceil_div(max_count, kListThreads / 32);
   if (grid > 2 * current_sm_count()) grid = 2 * current_sm_count();
   launch_dependent(kern, (unsigned)grid, kListThreads, smem, st, x, y, labels, list, count_dev, all_dev, max_count, (int)k, (int)d, kc,
-                   d % 4 == 0 && aligned(y, 16) ? 1 : 0);
+                   d % 4 == 0 && aligned(y, 16) ? 1 : 0, y_settled ? 1 : 0);
   return check_launch("kmeans_assign");
 }
 
@@ -316,14 +316,16 @@ int kmeans_assign_exact(const float* x, const float* y, int64_t* labels, const i
 }
 
 // Exact assignment of the points listed in `list`; their number sits in device memory (*count_dev <= max_count).  Of all
-// max_count points instead when all_dev is set and *all_dev is not 0.
+// max_count points instead when all_dev is set and *all_dev is not 0.  y_settled: the kernel launched before this one on the stream has
+// dependency_wait() as its first statement and does not write y, so what y holds then is what it holds now, and the centres are staged
+// before that kernel is done.
 int kmeans_assign_exact_listed(const float* x, const float* y, int64_t* labels, const int32_t* list, const int32_t* count_dev,
-                               const int32_t* all_dev, int64_t max_count, int64_t k, int64_t d, int metric, cudaStream_t st) {
+                               const int32_t* all_dev, int64_t max_count, int64_t k, int64_t d, int metric, bool y_settled, cudaStream_t st) {
   if (max_count == 0) return F2C_OK;
-  if (d <= 8) return launch_listed<8>(x, y, labels, list, count_dev, all_dev, max_count, k, d, metric, st);
-  if (d <= 16) return launch_listed<16>(x, y, labels, list, count_dev, all_dev, max_count, k, d, metric, st);
-  if (d <= 32) return launch_listed<32>(x, y, labels, list, count_dev, all_dev, max_count, k, d, metric, st);
-  if (d <= 64) return launch_listed<64>(x, y, labels, list, count_dev, all_dev, max_count, k, d, metric, st);
+  if (d <= 8) return launch_listed<8>(x, y, labels, list, count_dev, all_dev, max_count, k, d, metric, y_settled, st);
+  if (d <= 16) return launch_listed<16>(x, y, labels, list, count_dev, all_dev, max_count, k, d, metric, y_settled, st);
+  if (d <= 32) return launch_listed<32>(x, y, labels, list, count_dev, all_dev, max_count, k, d, metric, y_settled, st);
+  if (d <= 64) return launch_listed<64>(x, y, labels, list, count_dev, all_dev, max_count, k, d, metric, y_settled, st);
   return set_error(F2C_ERR_UNSUPPORTED, "kmeans_assign: listed re-scoring needs d <= 64");
 }
 

@@ -37,7 +37,7 @@
 namespace f2c {
 
 int kmeans_assign_exact_listed(const float* x, const float* y, int64_t* labels, const int32_t* list, const int32_t* count_dev,
-                               const int32_t* all_dev, int64_t max_count, int64_t k, int64_t d, int metric, cudaStream_t st);
+                               const int32_t* all_dev, int64_t max_count, int64_t k, int64_t d, int metric, bool y_settled, cudaStream_t st);
 
 namespace tc {
 
@@ -146,7 +146,7 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 // [tmem slot][2 x 2 x 2 x 128 floats |x|^2]
 template <bool BF16>
 __global__ void __launch_bounds__(kCtaThreads, 1) kmeans_tc_kernel(const Params p) {
-  dependency_wait();
+  dependency_wait();  // first of all: the kernel launched behind this one relies on it (y_settled below)
   release_dependents();
   extern __shared__ __align__(128) unsigned char smem[];
   if (p.done != nullptr && *(volatile const int32_t*)p.done != 0) return;
@@ -535,7 +535,7 @@ int kmeans_assign_tc(const float* x, const float* y, int64_t* labels, int64_t n,
   int rc = check_launch("kmeans_assign (tensor cores)");
   if (rc) return rc;
   // undecided points (all of them after a wait that ran out): exact fp32 scorer over the device-side list
-  return kmeans_assign_exact_listed(x, y, labels, p.amb_list, p.amb_count, p.error, n, k, d, metric, st);
+  return kmeans_assign_exact_listed(x, y, labels, p.amb_list, p.amb_count, p.error, n, k, d, metric, /* y_settled */ true, st);
 }
 
 // ------------------------------------------------------------------------------------------------------

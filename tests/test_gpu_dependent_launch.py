@@ -73,15 +73,18 @@ def calls(capi):
     return out
 
 
-def test_no_kernel_reads_before_the_previous_one_is_through(capi):
+def clear_late(dummy, t):
+    """Queue one kernel that clears dummy and, last of all, t."""
     from f2cgt_b200 import ops
     from f2cgt_b200._lib import check, lib
-    dummy = torch.ones(1 << 27, device="cuda")
+    at = (ctypes.c_void_p * 2)(dummy.data_ptr(), t.data_ptr())
+    size = (ctypes.c_int64 * 2)(dummy.numel() * 4, t.numel() * t.element_size() // 4 * 4)
+    check(lib.f2c_zero_ranges(at, size, 2, ops._stream(t)))
 
-    def clear(t):
-        at = (ctypes.c_void_p * 2)(dummy.data_ptr(), t.data_ptr())
-        size = (ctypes.c_int64 * 2)(dummy.numel() * 4, t.numel() * t.element_size() // 4 * 4)
-        check(lib.f2c_zero_ranges(at, size, 2, ops._stream(t)))
+
+def test_no_kernel_reads_before_the_previous_one_is_through(capi):
+    dummy = torch.ones(1 << 27, device="cuda")
+    clear = lambda t: clear_late(dummy, t)  # noqa: E731
 
     def values(out):
         return [t.clone() for t in (out if isinstance(out, list) else [out])]
@@ -104,3 +107,30 @@ def test_no_kernel_reads_before_the_previous_one_is_through(capi):
             for a, b in zip(got, want):
                 assert np.array_equal(a.cpu().numpy(), b.cpu().numpy(), equal_nan=a.is_floating_point()), (name, i)
             inputs[i].copy_(kept)
+
+
+@pytest.mark.parametrize("n,d,k", [(5000, 8, 256), (3000, 64, 100), (2000, 32, 17)])
+def test_an_iteration_of_a_fit_reads_nothing_early(capi, n, d, k):
+    """Assignment, exact re-score (which stages the centres before the assignment is through) and sums, right behind the kernel that
+    writes the centres or the points: no copy or memset stands in between, as between the iterations of a fit."""
+    from f2cgt_b200 import ops
+    from f2cgt_b200._lib import check, lib
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x0, c0 = torch.randn(n, d, generator=g, device="cuda"), torch.randn(k, d, generator=g, device="cuda")
+    x, c = x0.clone(), c0.clone()
+    ws = torch.empty(lib.f2c_kmeans_fit_workspace(n, k, d), dtype=torch.uint8, device="cuda")
+    dummy = torch.ones(1 << 27, device="cuda")
+    for cleared in (c, x):
+        got = []
+        for apart in (False, False, True):  # the first call loads the kernels
+            x.copy_(x0)
+            c.copy_(c0)
+            check(lib.f2c_kmeans_fit_begin(x.data_ptr(), n, k, d, ws.data_ptr(), ops._stream(x)))
+            torch.cuda.synchronize()
+            clear_late(dummy, cleared[:len(cleared) // 2])
+            if apart:
+                torch.cuda.synchronize()
+            check(lib.f2c_kmeans_fit_iterate(x.data_ptr(), c.data_ptr(), n, k, d, 0, 0.0, 2, ws.data_ptr(), ops._stream(x)))
+            got.append(c.clone())
+            torch.cuda.synchronize()
+        assert torch.equal(got[1], got[2])

@@ -179,3 +179,13 @@ def test_fit_goes_on_after_an_assignment_whose_wait_ran_out(capi):
     got, spoiled = _fit(x, x[:64].clone(), 6, spoil=True)
     assert spoiled[:3] == words[:3]
     assert spoiled[3] == 3 and torch.equal(want, got)
+
+
+def test_iterations_in_a_row_equal_iterations_one_by_one(capi):
+    """Eight iterations queued at once, whose kernels start while the one before still runs, and eight with the device idle between."""
+    g = torch.Generator(device="cuda").manual_seed(0)
+    for n, d, k in ((5000, 16, 64), (30000, 8, 256), (20000, 64, 200)):
+        x = torch.randn(n, d, generator=g, device="cuda")
+        a, w1 = _fit(x, x[:k].clone(), 8)
+        b, w2 = _fit(x, x[:k].clone(), 0, each=[1] * 8)
+        assert torch.equal(a, b) and w1 == w2
