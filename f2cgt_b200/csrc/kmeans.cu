@@ -10,8 +10,9 @@
 //    distance matrix with coalesced rows and/or reduces the argmin in the warp.  pairwise_distance is
 //    bound by its n*k*4-byte output.
 //  * thread-per-point (d <= 128): x_i lives in registers, centres are broadcast from shared memory
-//    with 128-bit reads, four FMAs per read.  This is the exact fp32 scorer; the tensor-core kernel
-//    (kmeans_tc.cu) uses it to re-score the points whose best two candidates are too close to call.
+//    with 128-bit reads, four FMAs per read.  This is the exact fp32 scorer; the points whose best two
+//    candidates are too close to call for the tensor-core kernel (kmeans_tc.cu) go through
+//    kmeans_listed_kernel, which computes the same distances.
 #include "common.cuh"
 
 namespace f2c {
@@ -73,8 +74,8 @@ __global__ void __launch_bounds__(256) kmeans_warp_kernel(const float* __restric
 // Centres are staged KC at a time as [KC][DMAX] (zero padded) plus their squared norms.
 template <int DMAX, int METRIC>
 __global__ void __launch_bounds__(256) kmeans_thread_kernel(const float* __restrict__ x, const float* __restrict__ y,
-                                                            int64_t* __restrict__ labels, const int32_t* __restrict__ subset, int64_t n,
-                                                            int k, int d, int kc, const int32_t* done) {
+                                                            int64_t* __restrict__ labels, int64_t n, int k, int d, int kc,
+                                                            const int32_t* done) {
   dependency_wait();
   release_dependents();
   if (done != nullptr && *(volatile const int32_t*)done != 0) return;  // a fit that has converged (kmeans_fit.cu)
@@ -82,10 +83,8 @@ __global__ void __launch_bounds__(256) kmeans_thread_kernel(const float* __restr
   float* yc_s = reinterpret_cast<float*>(smem_raw);  // [kc][DMAX]
   float* cc_s = yc_s + (size_t)kc * DMAX;            // [kc]
   for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n; base += (int64_t)gridDim.x * blockDim.x) {
-  const int64_t slot = base + threadIdx.x;
-  const bool valid = slot < n;
-  // subset != nullptr: only the listed points are (re)scored
-  const int64_t i = valid ? (subset ? (int64_t)subset[slot] : slot) : 0;
+  const int64_t i = base + threadIdx.x;
+  const bool valid = i < n;
   float xr[DMAX];
   float xx = 0.0f;
 #pragma unroll
@@ -275,8 +274,8 @@ static int launch_listed(const float* x, const float* y, int64_t* labels, const 
 }
 
 template <int DMAX>
-static int launch_thread_assign(const float* x, const float* y, int64_t* labels, const int32_t* subset, int64_t n, int64_t k,
-                                int64_t d, int metric, cudaStream_t st, const int32_t* done) {
+static int launch_thread_assign(const float* x, const float* y, int64_t* labels, int64_t n, int64_t k, int64_t d, int metric, cudaStream_t st,
+                                const int32_t* done) {
   int kc = (int)k;
   const size_t budget = 96 * 1024;
   while ((size_t)kc * (DMAX + 1) * sizeof(float) > budget) kc = (kc + 1) / 2;
@@ -286,26 +285,25 @@ static int launch_thread_assign(const float* x, const float* y, int64_t* labels,
   if (metric == F2C_COSINE) {
     auto kern = kmeans_thread_kernel<DMAX, F2C_COSINE>;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) launch_dependent(kern, grid, 256, smem, st, x, y, labels, subset, n, (int)k, (int)d, kc, done);
+    if (e == cudaSuccess) launch_dependent(kern, grid, 256, smem, st, x, y, labels, n, (int)k, (int)d, kc, done);
   } else {
     auto kern = kmeans_thread_kernel<DMAX, F2C_L2>;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) launch_dependent(kern, grid, 256, smem, st, x, y, labels, subset, n, (int)k, (int)d, kc, done);
+    if (e == cudaSuccess) launch_dependent(kern, grid, 256, smem, st, x, y, labels, n, (int)k, (int)d, kc, done);
   }
   if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "kmeans_assign: %s", cudaGetErrorString(e));
   return check_launch("kmeans_assign");
 }
 
-// Exact fp32 assignment of all points (subset == nullptr) or of the listed ones.
-int kmeans_assign_exact(const float* x, const float* y, int64_t* labels, const int32_t* subset, int64_t n, int64_t k,
-                        int64_t d, int metric, cudaStream_t st, const int32_t* done) {
+// Exact fp32 assignment of all points.
+int kmeans_assign_exact(const float* x, const float* y, int64_t* labels, int64_t n, int64_t k, int64_t d, int metric, cudaStream_t st,
+                        const int32_t* done) {
   if (n == 0) return F2C_OK;
-  if (d <= 8) return launch_thread_assign<8>(x, y, labels, subset, n, k, d, metric, st, done);
-  if (d <= 16) return launch_thread_assign<16>(x, y, labels, subset, n, k, d, metric, st, done);
-  if (d <= 32) return launch_thread_assign<32>(x, y, labels, subset, n, k, d, metric, st, done);
-  if (d <= 64) return launch_thread_assign<64>(x, y, labels, subset, n, k, d, metric, st, done);
-  if (d <= 128) return launch_thread_assign<128>(x, y, labels, subset, n, k, d, metric, st, done);
-  if (subset != nullptr) return set_error(F2C_ERR_UNSUPPORTED, "kmeans_assign: subset re-scoring needs d <= 128");
+  if (d <= 8) return launch_thread_assign<8>(x, y, labels, n, k, d, metric, st, done);
+  if (d <= 16) return launch_thread_assign<16>(x, y, labels, n, k, d, metric, st, done);
+  if (d <= 32) return launch_thread_assign<32>(x, y, labels, n, k, d, metric, st, done);
+  if (d <= 64) return launch_thread_assign<64>(x, y, labels, n, k, d, metric, st, done);
+  if (d <= 128) return launch_thread_assign<128>(x, y, labels, n, k, d, metric, st, done);
   int64_t blocks = ceil_div(n, 8);
   if (blocks > current_sm_count() * 32) blocks = current_sm_count() * 32;
   if (metric == F2C_COSINE)
@@ -380,5 +378,5 @@ extern "C" int f2c_kmeans_assign(const float* x, const float* centers, int64_t* 
   const bool prefer_tc = d >= 4 || scorer == F2C_SCORER_TENSOR;
   if (workspace != nullptr && kmeans_tc_supported(n, k, d) && prefer_tc && scorer != F2C_SCORER_EXACT && aligned(workspace, 16))
     return kmeans_assign_tc(x, centers, labels, n, k, d, metric, workspace, (cudaStream_t)stream, nullptr, false);
-  return kmeans_assign_exact(x, centers, labels, nullptr, n, k, d, metric, (cudaStream_t)stream, nullptr);
+  return kmeans_assign_exact(x, centers, labels, n, k, d, metric, (cudaStream_t)stream, nullptr);
 }

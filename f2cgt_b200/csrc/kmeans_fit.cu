@@ -23,8 +23,8 @@ bool kmeans_tc_supported(int64_t n, int64_t k, int64_t d);
 int64_t kmeans_tc_workspace(int64_t n);
 int kmeans_assign_tc(const float* x, const float* y, int64_t* labels, int64_t n, int64_t k, int64_t d, int metric, void* workspace,
                      cudaStream_t st, const int32_t* done, bool head_is_clear);
-int kmeans_assign_exact(const float* x, const float* y, int64_t* labels, const int32_t* subset, int64_t n, int64_t k, int64_t d,
-                        int metric, cudaStream_t st, const int32_t* done);
+int kmeans_assign_exact(const float* x, const float* y, int64_t* labels, int64_t n, int64_t k, int64_t d, int metric, cudaStream_t st,
+                        const int32_t* done);
 
 namespace fit {
 
@@ -269,7 +269,7 @@ extern "C" int f2c_kmeans_fit_iterate(const float* x, float* centers, int64_t n,
   if (grid > current_sm_count()) grid = current_sm_count();
   for (int it = 0; it < iterations; ++it) {
     rc = tc ? kmeans_assign_tc(x, centers, labels, n, k, d, metric, ws + w.assign, st, &state->done, true)
-            : kmeans_assign_exact(x, centers, labels, nullptr, n, k, d, metric, st, &state->done);
+            : kmeans_assign_exact(x, centers, labels, n, k, d, metric, st, &state->done);
     if (rc) return rc;
     launch_dependent(kern, (unsigned)grid, fit::kThreads, shared ? smem : 0, st, x, labels, centers, sums, counts, n, (int)k, (int)d, tol, assign_head,
                      state);
