@@ -554,10 +554,13 @@ static int launch_sq_spmm(const void* codes, int code_dtype, const float* codebo
       const Plan wide = plan(true);
       if (wide.ok && (!q.ok || wide.parts < q.parts)) { q = wide; across = true; }
     }
-    // Three parts or more of 8-bit columns that fill less than two thirds of their lanes read the ids and offsets too often for
-    // their work: 30,000 rows of 255 columns 102 us against 97 of the general kernel, whose warps fill 8 x 32 columns; of 262, 99
-    // against 107; 6,000 rows, where the general kernel's launch counts more, 24 against 28.
-    const bool thin = BITS == 8 && q.parts >= 3 && 3 * D < 2 * q.parts * ((int64_t)kLaneCols << q.logG) && n_dst * D >= 3ll << 20;
+    // Three parts or more of 8-bit columns that fill less than two thirds of their lanes (249 to 255 columns) read the ids and offsets too
+    // often for their work; the general kernel's warps fill 8 x 32 columns there.  12 neighbours, parts against general kernel: 250 columns
+    // of 3,000 / 6,000 / 9,000 / 13,000 / 30,000 / 90,000 rows 14.9 / 24.8 / 35.0 / 47.5 / 102.0 / 291.8 against 15.6 / 25.4 / 32.3 / 43.5 / 98.8 / 275.2
+    // us (249, 251, 253 to 255 the same within 1 us), so the line lies between 1.5 and 2.2 million sums.  From 257 columns on the parts are
+    // better at every size: 257 columns 14.9 / 24.8 / 34.8 / 47.6 / 102.0 / 291.9 against 16.8 / 28.0 / 35.4 / 48.0 / 108.9 / 304.8, 373 columns 9,000 rows
+    // 45.2 against 48.6.
+    const bool thin = BITS == 8 && q.parts >= 3 && 3 * D < 2 * q.parts * ((int64_t)kLaneCols << q.logG) && n_dst * D >= 2ll << 20;
     if ((BITS < 16 || n_dst * D <= 1ll << 18) && q.ok && !thin) {
       SqParams p{};
       p.codes = (const uint8_t*)codes; p.codebooks = codebooks; p.indptr = indptr; p.indices = indices; p.out = out;
