@@ -108,14 +108,17 @@ static int launch_vq_ept(const CodeT* codes, const CbT* cbs, float* out, int64_t
   if constexpr (std::is_same<CbT, float>::value) {
     // Reads of single floats from narrow centroids spread a warp over many lines of L1, so 8 and 16 columns are staged once there
     // is work for the copy of up to 200 KB per multiprocessor: 200,000 x 110 of 8 columns 23.7 us against 33.6 from L1, x 375 of
-    // 16 69 against 78, but 27,000 x 110 8.9 against 7.5.  From 32 columns on L1 is as good or better (x 357 of 64: 88 against
-    // 71), and so it is for 16-byte reads up to some 100 M outputs, beyond which the copy is nothing (400,000 x 128 of 32 columns
-    // 35.0 us staged, 34.6 not; 1,000,003 x 128 86.8 and 90.5).
+    // 16 69 against 78, but 27,000 x 110 8.9 against 7.5.  From 32 columns on L1 is as good or better (x 357 of 64: 88 against 71).
+    // 16-byte reads from centroids of 16 columns or more gain from about 100 M outputs on, where the copy is nothing: calls in a row,
+    // 24 / 48 / 96 / 128 / 192 / 256 M outputs, 128 columns of 32 18.0 / 33.5 / 66.1 / 88.5 / 132.4 / 176.6 us staged, 17.1 / 32.6 / 67.4 / 90.4 / 136.0 /
+    // 180.2 not; 128 of 64 18.1 / 33.3 / 64.5 / 85.9 / 126.9 / 168.6 and 17.4 / 33.1 / 66.4 / 89.5 / 134.4 / 178.6; 192 of 32 18.3 / 33.5 / 66.5 / 89.2 /
+    // 134.6 / 179.3 and 18.2 / 33.4 / 73.9 / 102.5 / 179.5 / 242.0; 112 of 16 70.4 / 70.4 at 96 M, 142.0 / 142.7 at 192 M,
+    // 187.9 / 190.5 at 256 M.  Eight columns do not: 128 of 8 76.0 staged, 69.3 not at 96 M, 190.0 against 179.6 at 256 M.
     const int64_t used = ceil_div(D, cs);  // subspaces that hold columns
     const int spq = (cs & (cs - 1)) == 0 && cs < 32 ? (int)(32 / cs) : 1;
     const int64_t line = spq > 1 ? 128 * K : 4 * K * cs;  // bytes of spq subspaces
     const int64_t fit = (int64_t)kVqStagedSmem / line * spq;
-    const bool worth = EPT == 1 ? cs < 32 && rows * D >= (8 << 20) : used <= fit && rows * D >= (96 << 20);
+    const bool worth = EPT == 1 ? cs < 32 && rows * D >= (8 << 20) : cs >= 16 && used <= fit && rows * D >= (96 << 20);
     if (fit > 0 && worth && cs % 4 == 0 && aligned(cbs, 16)) {
       int64_t parts = ceil_div(used, fit);
       while (parts < used && ceil_div(ceil_div(used, parts), spq) * spq * cs / EPT > kVqStagedThreads) ++parts;
