@@ -116,6 +116,15 @@ def train(preset="small", table="replicated", rank=0, world=1, local_rank=0, epo
     process group); returns the record rank 0 reports (every rank gets it).  The first epoch is a discarded warm-up; when
     ``min_timed_steps`` is set, enough further epochs are run to time at least that many steps per rank.  Per-phase device
     times come from CUDA events on the current stream (sample / exchange / forward / backward / optimizer)."""
+    tf32_before = torch.backends.cuda.matmul.allow_tf32
+    try:
+        return _train(preset, table, rank, world, local_rank, epochs, min_timed_steps, batch_size, lr, dropout, index_dtype, max_steps, precision,
+                      ahead)
+    finally:
+        torch.backends.cuda.matmul.allow_tf32 = tf32_before
+
+
+def _train(preset, table, rank, world, local_rank, epochs, min_timed_steps, batch_size, lr, dropout, index_dtype, max_steps, precision, ahead):
     cfg = PRESETS[preset]
     device = torch.device("cuda", local_rank)
     idt = torch.int32 if index_dtype == "int32" else torch.int64
@@ -154,7 +163,6 @@ def train(preset="small", table="replicated", rank=0, world=1, local_rank=0, epo
     if precision not in ("tf32", "fp32", "bf16"):
         raise ValueError("precision must be tf32, fp32 or bf16")
     product_dtype = torch.bfloat16 if precision == "bf16" else None
-    tf32_before = torch.backends.cuda.matmul.allow_tf32
     torch.backends.cuda.matmul.allow_tf32 = precision == "tf32"
     steps = torch.tensor([len(loader)], device=device)
     if world > 1:
@@ -234,7 +242,6 @@ def train(preset="small", table="replicated", rank=0, world=1, local_rank=0, epo
         sm = stats.clone(); dist.all_reduce(sm, op=dist.ReduceOp.SUM)
         stats = torch.cat([mx[:1], sm[1:2], mx[2:]])
     stats = stats.tolist()
-    torch.backends.cuda.matmul.allow_tf32 = tf32_before
     if hasattr(cm, "close"):
         torch.cuda.synchronize()
         cm.close()

@@ -457,7 +457,7 @@ def test_training_does_not_return_when_a_wait_ran_out(capi, monkeypatch):
     monkeypatch.setattr(sage.GPUSamplingDataloader, "poke", lambda self: pokes.append(0) or len(pokes) == 3 and _report(1))  # behind the last step
     with pytest.raises(RuntimeError, match="bounded wait"):
         tg.train(epochs=1, batch_size=256, max_steps=1)
-    assert ops.device_status() == 0
+    assert ops.device_status() == 0 and not torch.backends.cuda.matmul.allow_tf32  # the switch is back where it was
 
 
 @pytest.mark.parametrize("layers", [1, 2, 3])
