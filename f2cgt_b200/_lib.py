@@ -68,7 +68,7 @@ SIGNATURES = {
     "f2c_spmm_csr_backward": [p, p, p, ci, p, i64, i64, i64, ci, p],
     "f2c_sage_forward": [p, p, p, p, p, p, i64, i64, i64, ci, p],
     "f2c_sage_mask": [p, p, f32, p, p, i64, i64, p],
-    "f2c_sage_mask_dropout": [p, p, p, f32, p, p, i64, i64, p],
+    "f2c_sage_mask_dropout": [p, p, p, p, f32, p, p, i64, i64, p],
     "f2c_zero_ranges": [C.POINTER(p), C.POINTER(i64), ci, p],
     "f2c_sq_spmm_csr": [p, ci, p, i64, p, p, ci, p, i64, i64, i64, i64, ci, i64, ci, EP, p],
     "f2c_sq_spmm_csr_peer": [p, ci, i64, ci, p, i64, p, p, ci, p, i64, i64, i64, i64, ci, i64, ci, EP, p],

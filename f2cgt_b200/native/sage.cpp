@@ -174,7 +174,7 @@ class Kept {
  public:
   explicit Kept(const at::Tensor& t) : saved_(t, false) {
     if (!t.defined()) return;
-    sizes_ = t.sizes().vec();
+    sizes_ = t.sizes();
     dtype_ = t.scalar_type();
     device_ = t.device();
   }
@@ -188,13 +188,13 @@ class Kept {
 
  private:
   SavedVariable saved_;
-  std::vector<int64_t> sizes_;
+  c10::DimVector sizes_;
   at::ScalarType dtype_ = at::kFloat;
   at::Device device_ = at::kCPU;
 };
 
 // One layer of what the backward pass needs: inputs of the products (x1 is also the previous layer's output), what the ReLU gave and
-// dropout's mask (not in the last layer; undefined without dropout), the block (not in the first layer).
+// dropout's mask (undefined in the last layer and without dropout), the block (not in the first layer).
 template <typename T>
 struct PerLayer { T x1, x2, active, keep, indptr, indices; };
 
@@ -313,8 +313,10 @@ struct SageBackward : public torch::autograd::Node {
       at::Tensor dy = g;
       if (i + 1 < L) {
         dy = empty({m, n}, at::kFloat, g.device());
-        checked = f2c_sage_mask_dropout(f32(g), f32(of[i].active), of[i].keep.defined() ? (const uint8_t*)of[i].keep.data_ptr() : nullptr,
-                                        (float)net.scale(), f32(dy), db.defined() ? f32(db) : nullptr, m, n, st);
+        const at::Tensor &active = of[i].active, &keep = of[i].keep;
+        checked = f2c_sage_mask_dropout(f32(g), f32(of[i + 1].x1), active.defined() ? f32(active) : nullptr,
+                                        keep.defined() ? (const uint8_t*)keep.data_ptr() : nullptr, (float)net.scale(), f32(dy),
+                                        db.defined() ? f32(db) : nullptr, m, n, st);
       } else if (db.defined()) {
         checked = f2c_sage_mask(f32(dy), nullptr, 1.0f, nullptr, f32(db), m, n, st);
       }
@@ -424,7 +426,7 @@ PyObject* sage_net(PyObject*, PyObject* const* a, Py_ssize_t n) {
             if (net.p < 1 && h.numel() > 0) std::tie(h, keep) = at::native_dropout(h, net.p, true);
             else h = at::dropout(h, net.p, true);
           }
-          if (record) of.push_back({x1, x2, last ? at::Tensor() : active, keep, l.indptr, l.indices});
+          if (record) of.push_back({x1, x2, last || net.p <= 0 ? at::Tensor() : active, keep, l.indptr, l.indices});
         }
         if (h.size(0) > net.layers[L - 1].rows) h = h.narrow(0, 0, net.layers[L - 1].rows);
       }

@@ -144,15 +144,15 @@ int f2c_spmm_csr_backward(const float* grad_out, const void* indptr, const void*
 int f2c_sage_forward(const float* x1, const float* x2, const float* w1, const float* w2, const float* bias, float* y, int64_t m,
                      int64_t n, int64_t k, int relu, void* stream);
 
-/* Gradient through ReLU and dropout of a layer, and its bias gradient: dy = h <= 0 ? 0 : g * keep * scale (h = what the ReLU
- * gave, keep [rows, n] = 0 where dropout dropped and 1 elsewhere, scale = what it multiplied survivors with), and db [n] += column
- * sums of dy (db may be NULL; no fixed order).  g, h, dy [rows, n] f32.  A NaN in h passes its gradient, and NaN or infinite
- * gradients of dropped elements give NaN, as in torch.  h == NULL (then keep == NULL): dy is not written, db += column sums of g.
- * f2c_sage_mask: keep all ones (h may then also be the output behind dropout, which is zero where dropout dropped, for
- * finite gradients). */
+/* Gradient through ReLU and dropout of a layer, and its bias gradient: dy = active <= 0 ? 0 : g * keep * scale (active = what the
+ * ReLU gave, keep [rows, n] = 0 where dropout dropped and 1 elsewhere, scale = what it multiplied survivors with), and db [n] +=
+ * column sums of dy (db may be NULL; no fixed order).  h = the output behind both; g, h, active, dy [rows, n] f32.  A NaN in h passes
+ * its gradient, and NaN or infinite gradients of dropped elements give NaN, as in torch: only there active and keep are read.
+ * active == NULL: h; keep == NULL: all ones.  h == NULL: dy is not written, db += column sums of g.
+ * f2c_sage_mask: active == keep == NULL (exact without dropout, and with it for finite g and h). */
 int f2c_sage_mask(const float* g, const float* h, float scale, float* dy, float* db, int64_t rows, int64_t n, void* stream);
-int f2c_sage_mask_dropout(const float* g, const float* h, const uint8_t* keep, float scale, float* dy, float* db, int64_t rows,
-                          int64_t n, void* stream);
+int f2c_sage_mask_dropout(const float* g, const float* h, const float* active, const uint8_t* keep, float scale, float* dy, float* db,
+                          int64_t rows, int64_t n, void* stream);
 
 /* Set up to 32 ranges of device memory (whole 4-byte words) to zero in one launch; the arrays are HOST arrays. */
 int f2c_zero_ranges(void* const* ranges_host, const int64_t* bytes_host, int count, void* stream);

@@ -361,11 +361,13 @@ def test_relu_dropout_gradient_equals_torch_for_every_value(capi, rows, n, dropo
     x.requires_grad_()
     active = torch.relu(x)
     keep = torch.rand(rows, n, generator=g, device="cuda") < 0.6
-    out = torch.ops.aten.native_dropout_backward(grad, keep, 2.5) if dropout else grad * 1.0
-    active.backward(out)
+    active.backward(torch.ops.aten.native_dropout_backward(grad, keep, 2.5) if dropout else grad)
+    active = active.detach()
     dy, db = torch.empty_like(grad), torch.zeros(n, device="cuda")
     if dropout:
-        check(lib.f2c_sage_mask_dropout(grad.data_ptr(), active.data_ptr(), keep.data_ptr(), 2.5, dy.data_ptr(), db.data_ptr(), rows, n, ops._stream(dy)))
+        h = active * keep * 2.5
+        check(lib.f2c_sage_mask_dropout(grad.data_ptr(), h.data_ptr(), active.data_ptr(), keep.data_ptr(), 2.5, dy.data_ptr(), db.data_ptr(), rows, n,
+                                        ops._stream(dy)))
     else:
         check(lib.f2c_sage_mask(grad.data_ptr(), active.data_ptr(), 1.0, dy.data_ptr(), db.data_ptr(), rows, n, ops._stream(dy)))
     assert torch.equal(dy.nan_to_num(7.0, 8.0, 9.0), x.grad.nan_to_num(7.0, 8.0, 9.0))
@@ -550,8 +552,10 @@ def test_relu_dropout_gradient_of_wide_rows(capi, rows, n):
     grad, h = torch.randn(rows, n, generator=g, device="cuda"), torch.randn(rows, n, generator=g, device="cuda")
     keep = torch.rand(rows, n, generator=g, device="cuda") < 0.5
     dy, db = torch.empty_like(grad), torch.zeros(n, device="cuda")
-    check(lib.f2c_sage_mask_dropout(grad.data_ptr(), h.data_ptr(), keep.data_ptr(), 2.0, dy.data_ptr(), db.data_ptr(), rows, n, ops._stream(h)))
-    want = torch.where(h > 0, grad * keep * 2.0, 0.0)
+    active, h = h, h * keep * 2.0
+    check(lib.f2c_sage_mask_dropout(grad.data_ptr(), h.data_ptr(), active.data_ptr(), keep.data_ptr(), 2.0, dy.data_ptr(), db.data_ptr(), rows, n,
+                                    ops._stream(h)))
+    want = torch.where(active > 0, grad * keep * 2.0, 0.0)
     assert torch.equal(dy, want) and torch.allclose(db.double(), want.double().sum(0), rtol=1e-5, atol=1e-5 * rows**0.5)
 
 
