@@ -407,6 +407,7 @@ PyObject* sage_net(PyObject*, PyObject* const* a, Py_ssize_t n) {
       }
       at::Tensor h;
       std::vector<PerLayer<at::Tensor>> of;
+      of.reserve(L);
       {
         at::AutoDispatchBelowADInplaceOrView below;
         at::Tensor x1 = h_self, x2 = h_neigh;
@@ -431,6 +432,8 @@ PyObject* sage_net(PyObject*, PyObject* const* a, Py_ssize_t n) {
         if (h.size(0) > net.layers[L - 1].rows) h = h.narrow(0, 0, net.layers[L - 1].rows);
       }
       if (record) {
+        node->weights.reserve(w.size());
+        node->layers.reserve(of.size());
         for (const at::Tensor& t : w) node->weights.emplace_back(t);
         for (const PerLayer<at::Tensor>& l : of)
           node->layers.push_back({Kept(l.x1), Kept(l.x2), Kept(l.active), Kept(l.keep), Kept(l.indptr), Kept(l.indices)});
