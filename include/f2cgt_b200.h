@@ -19,6 +19,11 @@
  *     instantiates int8/uint8/int16 indices, src/common.h:39-57, which no caller uses);
  *   - code tensors are uint8 / int8 / int16 (src/common.h:68-82).  Packed widths (1, 2, 4 bits)
  *     are raw bytes whatever the dtype says (src/sq_quantization.cu:131-132).
+ *   - the aggregations read code rows that do not start on a 4-, 8- or 16-byte boundary as the whole aligned
+ *     blocks of that size which hold a byte of them: up to 15 bytes before the first and behind the last row of a
+ *     table are read, and thrown away, when the table starts or ends inside such a block.  These bytes lie in the
+ *     same memory page as the table's own; a caller who packs tables without padding need not keep other work from
+ *     writing them.
  */
 #ifndef F2CGT_B200_H_
 #define F2CGT_B200_H_
