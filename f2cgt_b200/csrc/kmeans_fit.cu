@@ -7,7 +7,7 @@
 // every few of them; iterations queued behind the converged one change nothing.
 //
 //  * Sums are exact and independent of the order of the additions: a value becomes a fixed-point integer (43 fraction bits
-//    below the largest magnitude of the data set, fewer when more than 2^18 points could overflow 63 bits), and integers
+//    below the largest magnitude of its column, fewer when more than 2^18 points could overflow 63 bits), and integers
 //    commute.  A fit is therefore reproducible bit for bit, as it was with the sorted float64 prefix sums this replaces,
 //    and at least as accurate.
 //  * Inside a CTA the integers are added in shared memory as two 22-bit limbs with 32-bit atomics without a result (the
@@ -37,7 +37,7 @@ struct State {       // first 256 bytes of the workspace; the host reads the fir
   int32_t iterations;
   int32_t not_finite;   // the data hold inf or NaN: nothing is iterated, the caller says so
   int32_t assign_error; // code of the last bounded wait of the tensor-core kernel that ran out (the exact scorer then assigned every point)
-  uint32_t max_bits;    // largest |x| as float bits
+  uint32_t pad;
   uint32_t arrived;
   double shift;
 };
@@ -47,44 +47,76 @@ __device__ __forceinline__ int fraction_bits(int64_t n) {
   return min(43, 61 - lg);
 }
 
-__global__ void __launch_bounds__(256) max_abs_kernel(const float* __restrict__ x, int64_t numel, State* st) {
+// |x| <= 2^e for the float with these bits; a value of the column becomes an integer multiple of 2^(e - bits)
+__device__ __forceinline__ int exponent(uint32_t max_bits) { return max_bits == 0u ? 0 : (int)(max_bits >> 23) - 126; }
+__device__ __forceinline__ double power2(int e) { return __hiloint2double((1023 + e) << 20, 0); }  // |e| < 1023
+
+// Largest |x| of every column as float bits.  `threads` is a multiple of d, so that a thread stays in its column; d above the grid's
+// threads: every thread walks over columns.
+__global__ void __launch_bounds__(256) max_abs_kernel(const float* __restrict__ x, int64_t numel, int d, int64_t threads, uint32_t* __restrict__ maxima) {
   dependency_wait();
   release_dependents();
-  uint32_t m = 0;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < numel; i += (int64_t)gridDim.x * blockDim.x)
-    m = max(m, __float_as_uint(__ldg(x + i)) & 0x7fffffffu);  // NaN has larger bits than inf
-  m = __reduce_max_sync(0xffffffffu, m);
-  if ((threadIdx.x & 31) == 0 && m != 0u) atomicMax(&st->max_bits, m);
+  extern __shared__ uint32_t max_s[];
+  const int64_t me = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool shared = threads > 0 && d <= 4096;
+  if (shared) {
+    for (int j = threadIdx.x; j < d; j += blockDim.x) max_s[j] = 0u;
+    __syncthreads();
+  }
+  if (threads > 0) {
+    uint32_t m = 0;
+    if (me < threads)
+      for (int64_t i = me; i < numel; i += threads) m = max(m, __float_as_uint(__ldg(x + i)) & 0x7fffffffu);  // NaN has larger bits than inf
+    if (m != 0u) atomicMax(shared ? max_s + me % d : maxima + me % d, m);
+  } else {
+    for (int64_t j = me; j < d; j += (int64_t)gridDim.x * blockDim.x) {
+      uint32_t m = 0;
+      for (int64_t i = j; i < numel; i += d) m = max(m, __float_as_uint(__ldg(x + i)) & 0x7fffffffu);
+      maxima[j] = m;
+    }
+  }
+  if (shared) {
+    __syncthreads();
+    for (int j = threadIdx.x; j < d; j += blockDim.x)
+      if (max_s[j] != 0u) atomicMax(maxima + j, max_s[j]);
+  }
 }
 
-__global__ void begin_kernel(State* st) {
+__global__ void begin_kernel(const uint32_t* __restrict__ maxima, int d, State* st) {
   dependency_wait();
   release_dependents();
-  if (threadIdx.x == 0 && st->max_bits >= 0x7f800000u) { st->not_finite = 1; st->done = 1; }
+  for (int j = threadIdx.x; j < d; j += blockDim.x)
+    if (maxima[j] >= 0x7f800000u) { st->not_finite = 1; st->done = 1; }
 }
 
 // Centres <- sums / counts (clusters without points keep theirs), sums and counts <- 0, shift, done.  One CTA.
-__device__ void finish_iteration(float* __restrict__ centers, long long* sums, unsigned int* counts, int k, int d, double unit,
-                                 double tol, int32_t* assign_head, State* st) {
+// scale_of(j): what column j's values were multiplied with, a power of two.
+template <typename Scale>
+__device__ void finish_iteration(float* __restrict__ centers, long long* sums, unsigned int* counts, int k, int d, Scale scale_of, double tol,
+                                 int32_t* assign_head, State* st) {
   __shared__ double part[kThreads / 32];
   double shift = 0.0;
   // this CTA alone works now: the loads of eight entries are in flight together (one at a time: 11 of 23 us for 256 x 32)
   constexpr int U = 8;
   for (int i0 = threadIdx.x; i0 < k * d; i0 += U * kThreads) {
     unsigned int cnt[U];
+    int col[U];
     long long sum[U];
     float old[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int i = i0 + u * kThreads;
+      const int c = i / d;
       cnt[u] = 0u;
-      if (i < k * d) { cnt[u] = __ldcg(counts + i / d); sum[u] = __ldcg(sums + i); old[u] = centers[i]; }
+      col[u] = i - c * d;
+      if (i < k * d) { cnt[u] = __ldcg(counts + c); sum[u] = __ldcg(sums + i); old[u] = centers[i]; }
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int i = i0 + u * kThreads;
       if (cnt[u] != 0u) {  // sums of clusters without points are zero
         sums[i] = 0;
+        const double unit = __hiloint2double((2046 << 20) - __double2hiint(scale_of(col[u])), 0);  // 1 / scale
         const float next = (float)((double)sum[u] * unit) / (float)cnt[u];
         const float diff = next - old[u];
         shift += (double)(diff * diff);
@@ -116,10 +148,12 @@ __device__ void finish_iteration(float* __restrict__ centers, long long* sums, u
 template <bool SHARED>
 __global__ void __launch_bounds__(kThreads) accumulate_kernel(const float* __restrict__ x, const int64_t* __restrict__ labels,
                                                               float* __restrict__ centers, long long* sums, unsigned int* counts,
-                                                              int64_t n, int k, int d, double tol, int32_t* assign_head, State* st) {
+                                                              const uint32_t* __restrict__ maxima, int64_t n, int k, int d, double tol,
+                                                              int32_t* assign_head, State* st) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int kd = k * d;
-  uint32_t* lo = reinterpret_cast<uint32_t*>(smem);
+  double* scales = reinterpret_cast<double*>(smem);  // of the columns
+  uint32_t* lo = reinterpret_cast<uint32_t*>(scales + (SHARED ? d : 0));
   int32_t* hi = reinterpret_cast<int32_t*>(lo + (SHARED ? kd : 0));
   uint32_t* cnt = reinterpret_cast<uint32_t*>(hi + (SHARED ? kd : 0));
   uint16_t* lab = reinterpret_cast<uint16_t*>(cnt + (SHARED ? k : 0));  // labels of the chunk (k <= 65535 here)
@@ -129,12 +163,11 @@ __global__ void __launch_bounds__(kThreads) accumulate_kernel(const float* __res
     for (int i = tid; i < 2 * kd + k; i += kThreads) lo[i] = 0u;
   dependency_wait();
   release_dependents();
-  if (*(volatile int32_t*)&st->done != 0) return;
-  // |x| <= 2^e: unit of the last place = 2^(e - bits)
-  const uint32_t mb = st->max_bits;
-  const int e = mb == 0u ? 0 : (int)(mb >> 23) - 126;
   const int bits = fraction_bits(n);
-  const double scale = ldexp(1.0, bits - e), unit = ldexp(1.0, e - bits);
+  auto scale_of = [&](int j) { return SHARED ? scales[j] : power2(bits - exponent(__ldg(maxima + j))); };
+  if (SHARED)
+    for (int i = tid; i < d; i += kThreads) scales[i] = power2(bits - exponent(__ldg(maxima + i)));
+  if (*(volatile int32_t*)&st->done != 0) return;
 
   // chunks are dealt so that every CTA gets almost the same number of points
   const int64_t rounds = (n + (int64_t)gridDim.x * kChunk - 1) / ((int64_t)gridDim.x * kChunk);
@@ -156,7 +189,7 @@ __global__ void __launch_bounds__(kThreads) accumulate_kernel(const float* __res
     int p = tid / d, j = tid - p * d;
     const int dp = kThreads / d, dj = kThreads - dp * d;
     for (int t = tid; t < total; t += kThreads) {
-      const long long v = __double2ll_rn((double)__ldg(base + t) * scale);
+      const long long v = __double2ll_rn((double)__ldg(base + t) * scale_of(j));
       if (SHARED) {
         const int at = (int)lab[p] * d + j;
         atomicAdd(lo + at, (uint32_t)v & 0x3fffffu);
@@ -189,11 +222,11 @@ __global__ void __launch_bounds__(kThreads) accumulate_kernel(const float* __res
   __syncthreads();
   if (last) {
     __threadfence();
-    finish_iteration(centers, sums, counts, k, d, unit, tol, assign_head, st);
+    finish_iteration(centers, sums, counts, k, d, scale_of, tol, assign_head, st);
   }
 }
 
-struct Layout { size_t sums, counts, labels, assign, total; };
+struct Layout { size_t sums, counts, labels, assign, maxima, total; };
 
 static Layout plan(int64_t n, int64_t k, int64_t d) {
   auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
@@ -203,6 +236,7 @@ static Layout plan(int64_t n, int64_t k, int64_t d) {
   w.counts = at; at += up((size_t)k * 4);
   w.labels = at; at += up((size_t)n * 8);
   w.assign = at; at += kmeans_tc_supported(n, k, d) ? up((size_t)kmeans_tc_workspace(n)) : 0;
+  w.maxima = at; at += up((size_t)d * 4);
   w.total = at;
   return w;
 }
@@ -232,12 +266,14 @@ extern "C" int f2c_kmeans_fit_begin(const float* x, int64_t n, int64_t k, int64_
   const fit::Layout w = fit::plan(n, k, d);
   cudaError_t e = cudaMemsetAsync(workspace, 0, w.labels, st);  // state, sums and counts
   if (e == cudaSuccess && kmeans_tc_supported(n, k, d)) e = cudaMemsetAsync((unsigned char*)workspace + w.assign, 0, 256, st);
+  if (e == cudaSuccess) e = cudaMemsetAsync((unsigned char*)workspace + w.maxima, 0, (size_t)d * 4, st);
   if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "%s: %s", op, cudaGetErrorString(e));
   fit::State* state = (fit::State*)workspace;
   int64_t blocks = ceil_div(n * d, 256 * 8);
   if (blocks > 8 * current_sm_count()) blocks = 8 * current_sm_count();
-  launch_dependent(fit::max_abs_kernel, (unsigned)blocks, 256, 0, st, x, n * d, state);
-  launch_dependent(fit::begin_kernel, 1, 32, 0, st, state);
+  uint32_t* maxima = (uint32_t*)((unsigned char*)workspace + w.maxima);
+  launch_dependent(fit::max_abs_kernel, (unsigned)blocks, 256, d <= 4096 ? (size_t)d * 4 : 0, st, x, n * d, (int)d, blocks * 256 / d * d, maxima);
+  launch_dependent(fit::begin_kernel, 1, 256, 0, st, maxima, (int)d, state);
   return check_launch(op);
 }
 
@@ -257,7 +293,8 @@ extern "C" int f2c_kmeans_fit_iterate(const float* x, float* centers, int64_t n,
   int64_t* labels = (int64_t*)(ws + w.labels);
   const bool tc = kmeans_tc_supported(n, k, d) && d >= 4;
   int32_t* assign_head = tc ? (int32_t*)(ws + w.assign) : nullptr;  // [undecided points, error]; cleared by f2c_kmeans_fit_begin, then by every iteration
-  const size_t smem = ((size_t)2 * k * d + k) * 4 + fit::kChunk * 2;
+  const size_t smem = (size_t)d * 8 + ((size_t)2 * k * d + k) * 4 + fit::kChunk * 2;
+  const uint32_t* maxima = (const uint32_t*)(ws + w.maxima);
   const bool shared = smem <= fit::kSmemLimit && k <= 65535;
   auto kern = shared ? fit::accumulate_kernel<true> : fit::accumulate_kernel<false>;
   if (shared) {
@@ -271,8 +308,8 @@ extern "C" int f2c_kmeans_fit_iterate(const float* x, float* centers, int64_t n,
     rc = tc ? kmeans_assign_tc(x, centers, labels, n, k, d, metric, ws + w.assign, st, &state->done, true)
             : kmeans_assign_exact(x, centers, labels, n, k, d, metric, st, &state->done);
     if (rc) return rc;
-    launch_dependent(kern, (unsigned)grid, fit::kThreads, shared ? smem : 0, st, x, labels, centers, sums, counts, n, (int)k, (int)d, tol, assign_head,
-                     state);
+    launch_dependent(kern, (unsigned)grid, fit::kThreads, shared ? smem : 0, st, x, labels, centers, sums, counts, maxima, n, (int)k, (int)d, tol,
+                     assign_head, state);
     rc = check_launch(op);
     if (rc) return rc;
   }

@@ -189,3 +189,18 @@ def test_iterations_in_a_row_equal_iterations_one_by_one(capi):
         a, w1 = _fit(x, x[:k].clone(), 8)
         b, w2 = _fit(x, x[:k].clone(), 0, each=[1] * 8)
         assert torch.equal(a, b) and w1 == w2
+
+
+@pytest.mark.parametrize("n,k,d", [(5000, 8, 5), (40_000, 16, 64), (3000, 4, 300), (700, 2, 5000)])
+def test_fit_keeps_the_precision_of_small_columns(capi, n, k, d):
+    """Columns of very different sizes: a centre's entries are as precise as fp32 in each of them (exact sums, one rounding to float32,
+    one division), whatever the largest column holds."""
+    g = torch.Generator(device="cuda").manual_seed(d)
+    size = torch.logspace(9, -12, d, device="cuda")[torch.randperm(d, generator=g, device="cuda")]
+    x = torch.rand(n, d, generator=g, device="cuda").add_(0.5) * size
+    start = x[:k].clone()
+    labels = capi.kmeans_assign(x, start, "l2")
+    got, words = _fit(x, start.clone(), 1)
+    want = torch.zeros(k, d, dtype=torch.float64, device="cuda").index_add_(0, labels, x.double())
+    want /= torch.bincount(labels, minlength=k).double()[:, None]
+    assert words[1] == 1 and float(((got.double() - want).abs() / want).max()) < 2.0**-22  # two roundings of 2^-24, doubled
