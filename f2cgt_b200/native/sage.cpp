@@ -395,6 +395,11 @@ PyObject* sage_net(PyObject*, PyObject* const* a, Py_ssize_t n) {
     net.tf32 = PyObject_IsTrue(a[8]) == 1;
     if (a[9] != Py_None) net.cast = reinterpret_cast<THPDtype*>(a[9])->scalar_type;
     if (h_self.dim() != 2 || h_self.sizes() != h_neigh.sizes() || h_self.size(0) < net.layers[0].padded) fail(PyExc_RuntimeError, "sage_net: bad inputs");
+    auto elsewhere = [&](const at::Tensor& t) { return t.defined() && t.device() != h_self.device(); };
+    bool apart = elsewhere(h_neigh);
+    for (const at::Tensor& t : w) apart = apart || elsewhere(t);
+    for (const Layer& l : net.layers) apart = apart || elsewhere(l.indptr) || elsewhere(l.indices);
+    if (apart) fail(PyExc_RuntimeError, "sage_net: expected all tensors on the same device");
     const bool record = at::GradMode::is_enabled() && torch::autograd::compute_requires_grad(w);
     at::Tensor result = unlocked([&] {
       c10::cuda::CUDAGuard guard(h_self.device());

@@ -692,3 +692,11 @@ def test_dropout_in_place_draws_its_own_masks(capi):
             got.append(model(blocks))
         model.layers[1].register_forward_pre_hook(lambda *_: None)
     assert torch.allclose(got[0], got[1], rtol=1e-4, atol=1e-4)
+
+
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two GPUs")
+def test_network_on_another_device_than_its_blocks_is_refused(capi):
+    model, blocks, _ = _small_network(0.0)
+    model.layers[1].to("cuda:1")
+    with pytest.raises(RuntimeError, match="same device"):
+        model(blocks)
