@@ -1,4 +1,8 @@
-"""GPU: calls that wait for a place in the launch queue leave the interpreter to the other Python threads."""
+"""GPU: calls that wait for a place in the launch queue leave the interpreter to the other Python threads; first calls of a process
+under capture."""
+import os
+import subprocess
+import sys
 import threading
 import time
 
@@ -73,3 +77,27 @@ def test_other_threads_run_while_the_launch_queue_is_full(capi, which):
     pause, longest = _longest_pause_beside(call)
     assert longest > 0.05, "the queue did not fill"
     assert pause < 0.5 * longest
+
+
+CAPTURED = """
+import torch
+import F2CGTLib as capi
+g = torch.Generator(device="cuda").manual_seed(0)
+codes = torch.randint(-128, 128, (20000, 32), generator=g, device="cuda", dtype=torch.int8)
+cb = torch.tensor([[1e-3, 4.0, -9.97, 2.0, 0.8]], device="cuda")
+ip = torch.arange(0, 12 * 40000 + 1, 12, device="cuda")
+ix = torch.randint(0, 20000, (12 * 40000,), generator=g, device="cuda")
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    out = capi.sq_decompress_spmm_csr(codes, cb, ip, ix, 2, 128, 128)
+graph.replay()
+assert torch.equal(out, capi.sq_decompress_spmm_csr(codes, cb, ip, ix, 2, 128, 128, kernel="general"))
+from f2cgt_b200 import ops
+assert ops.device_status() == 0
+"""
+
+
+def test_first_use_of_the_status_word_under_capture(capi):
+    """The streamed kernel's status word and its host copy are set up by the first call, which here is part of a graph."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    subprocess.run([sys.executable, "-c", CAPTURED], cwd=root, check=True, timeout=120)
