@@ -73,18 +73,15 @@ def calls(capi):
     return out
 
 
-def clear_late(dummy, t):
-    """Queue one kernel that clears dummy and, last of all, t."""
+def test_no_kernel_reads_before_the_previous_one_is_through(capi):
     from f2cgt_b200 import ops
     from f2cgt_b200._lib import check, lib
-    at = (ctypes.c_void_p * 2)(dummy.data_ptr(), t.data_ptr())
-    size = (ctypes.c_int64 * 2)(dummy.numel() * 4, t.numel() * t.element_size() // 4 * 4)
-    check(lib.f2c_zero_ranges(at, size, 2, ops._stream(t)))
-
-
-def test_no_kernel_reads_before_the_previous_one_is_through(capi):
     dummy = torch.ones(1 << 27, device="cuda")
-    clear = lambda t: clear_late(dummy, t)  # noqa: E731
+
+    def clear(t):
+        at = (ctypes.c_void_p * 2)(dummy.data_ptr(), t.data_ptr())
+        size = (ctypes.c_int64 * 2)(dummy.numel() * 4, t.numel() * t.element_size() // 4 * 4)
+        check(lib.f2c_zero_ranges(at, size, 2, ops._stream(t)))
 
     def values(out):
         return [t.clone() for t in (out if isinstance(out, list) else [out])]
@@ -107,6 +104,15 @@ def test_no_kernel_reads_before_the_previous_one_is_through(capi):
             for a, b in zip(got, want):
                 assert np.array_equal(a.cpu().numpy(), b.cpu().numpy(), equal_nan=a.is_floating_point()), (name, i)
             inputs[i].copy_(kept)
+
+
+def clear_late(dummy, t):
+    """Queue one kernel that clears dummy and, last of all, t."""
+    from f2cgt_b200 import ops
+    from f2cgt_b200._lib import check, lib
+    at = (ctypes.c_void_p * 2)(dummy.data_ptr(), t.data_ptr())
+    size = (ctypes.c_int64 * 2)(dummy.numel() * 4, t.numel() * t.element_size() // 4 * 4)
+    check(lib.f2c_zero_ranges(at, size, 2, ops._stream(t)))
 
 
 @pytest.mark.parametrize("n,d,k", [(5000, 8, 256), (3000, 64, 100), (2000, 32, 17)])
