@@ -374,7 +374,7 @@ extern "C" int f2c_kmeans_assign(const float* x, const float* centers, int64_t* 
   F2C_REQUIRE(x && centers && labels, F2C_ERR_INVALID, "kmeans_assign: null pointer");
   // tensor-core path when a scratch buffer is supplied and the shape fits; the exact fp32 scorer otherwise, and below four
   // dimensions, where many points' best two centres are too close for the split product (2,449,029 x 4 against 256 centres:
-  // exact scorer 982 us, tensor cores 159)
+  // exact scorer 982 us, tensor cores 104)
   const bool prefer_tc = d >= 4 || scorer == F2C_SCORER_TENSOR;
   if (workspace != nullptr && kmeans_tc_supported(n, k, d) && prefer_tc && scorer != F2C_SCORER_EXACT && aligned(workspace, 16))
     return kmeans_assign_tc(x, centers, labels, n, k, d, metric, workspace, (cudaStream_t)stream, nullptr, false);

@@ -2,37 +2,38 @@
 // Reference operator: KMeans.predict (src/kmeans.cu:77-98, RAFT kmeans_predict), i.e.
 // labels[i] = first argmin_c dist(x_i, y_c) with dist = squared L2 or cosine distance.
 //
-// The n*k*d contraction S = X * Y^T is the only dense GEMM on the path, so it runs as
-// tcgen05.mma.kind::tf32 with M = 128 points per tile, N = all (<= 256) centres, accumulators in TMEM,
-// operands in shared memory in the canonical no-swizzle K-major layout.
+// The n*k*d contraction S = X * Y^T is the only dense GEMM on the path, so it runs as tcgen05.mma.kind::f16 with M = 128
+// points per tile, N = all (<= 256) centres, fp32 accumulators in TMEM, operands in shared memory in the canonical
+// no-swizzle K-major layout.
 //
-//  * Accuracy.  TF32 keeps 10 mantissa bits, which would flip near ties, so both operands are split
-//    x = hi + lo (hi = top 19 bits) and the products hi*hi + lo*hi + hi*lo are obtained in ONE GEMM by
-//    concatenating along K:  A' = [x_hi | x_lo | x_hi],  B' = [y_hi | y_hi | y_lo]  (K = 3d), which is
-//    fp32-accurate to ~2^-19.  For 32 < d <= 64 those operands would not fit in shared memory; there the split is
-//    into bf16 pairs x = b1 + b2 (+ a rest below 2^-18 |x|) with the same concatenation on kind::f16
-//    (half the bytes per value), accurate to ~2^-16.
-//  * The whole score comes out of the GEMM.  argmin_c |y_c|^2 - 2 x.y_c = argmax_c (x.y_c - |y_c|^2 / 2): one
-//    more K step carries [1, 1, 0...] on the point side and the split of -|y_c|^2/2 on the centre side
-//    (cosine: the centre rows are pre-scaled by 1/|y_c| instead), so the epilogue is a pure arg-max - one three-operand
-//    max per (point, centre) - with no per-centre term to fetch.
+//  * Accuracy.  A value is split into two f16 numbers, x = h1 + h2 + (rest below 2^-22 |x|, or 2^-25 where h2 is subnormal),
+//    and the products h1*g1 + h2*g1 + h1*g2 are obtained in ONE GEMM by concatenating along K:
+//    A' = [x1 | x2 | x1], B' = [y1 | y1 | y2] (K = 3d).  f16 has five exponent bits, so operands are scaled by powers of two
+//    first: the rows of X each by their own largest value (a common factor of a point's scores does not change its arg-max;
+//    squared L2: only rows that lie further out than the centres), the rows of Y by their norm (cosine) or by the largest
+//    norm of all (squared L2).  (Two f16 carry 22 bits where 3 x tf32 carried 21 at half the rate and twice the bytes, and
+//    3 x bf16 16, which sent several per cent of 64-dimensional points to the exact scorer.)
+//  * The whole score comes out of the GEMM.  argmin_c |y_c|^2 - 2 x.y_c = argmax_c (x.y_c - |y_c|^2 / 2): one more chunk of K
+//    carries powers of two on the point side and three f16 pieces of -|y_c|^2/2 on the centre side, so the epilogue is a pure
+//    arg-max.  A column that is padding carries -65504 in that chunk.
 //  * The epilogue reads the 128 x 256 scores with tcgen05.ld (one point per thread) and finds the best score and whether it is
 //    the only one within the error bound of the product.  A point where it is not is NOT decided here: its index is appended to
 //    a scratch list and the exact fp32 scorer (kmeans.cu) assigns it afterwards, so every label equals the label of the exact
 //    fp32 kernel.  (Squared distances of points that lie some 10^3 times further out than the centres differ by less than their
-//    own fp32 rounding; there the score, which leaves |x|^2 out, still decides, for the nearer centre: 40,001 x 8 around the origin,
-//    200 centres, 1 point of 40,001 at 2^10 times the centres' norm, 322 at 2^16, all nearer in float64.)
-//  * Overlap.  A CTA is two groups of eight warps that share the staged centre tile; each group has its own
-//    point tile, mbarrier and 256 TMEM columns and runs load -> MMA -> epilogue on alternate tiles, so the
-//    tensor pipe works on one group's tile while the other group is in its epilogue.  A point of the tile
-//    belongs to two threads of its group (same TMEM lane, warps w and w + 4): they load and split alternate
-//    chunks of its row and scan one half of the centres each - the epilogue, not the MMA, is what the kernel
-//    spends its issue slots on, and twice the warps fill them better.  The group's first thread issues the
-//    MMAs.  Every wait on an MMA-completion mbarrier is bounded; on expiry an error code is recorded, which makes the exact
-//    scorer assign every point, no further wait is made, and the CTA frees its TMEM at the common exit.
+//    own fp32 rounding; there the score, which leaves |x|^2 out, still decides, for the nearer centre.)
+//  * Overlap.  A CTA has 22 warps with fixed roles: three groups of four epilogue warps, two of four producer warps, which have their
+//    points' rows copied to shared memory ahead, split them and store them into a ring of A tiles, and two warps whose first lanes issue the
+//    MMAs, each into its pair of accumulators of 128 columns.  They meet at mbarriers only: a half of the columns is made while the epilogue
+//    reads another, and a group ends a tile while the two others read theirs.
+//    What bounds it: up to 16 dimensions the maxima (one per point and centre and direction, two cycles per three-operand instruction: ALU
+//    pipe 66 % busy) and the latency of the chain accumulator free - MMAs - accumulator full; more dimensions: the producers' chains of
+//    dependent instructions, whatever memory and the tensor pipe do (without the splitting 147 us of 2,449,029 x 32 become 110).
+//    Measured, 2,449,029 points against 256 centres, whole call (before: sixteen warps that all loaded, split, waited and searched, one barrier
+//    per tile, 3 x tf32 or 3 x bf16): 8 dimensions 154 -> 102 us, 16: 193 -> 117, 24: 228 -> 141, 32: 267 -> 154, 64: 401 -> 313; 100 centres
+//    of 8 dimensions 119 -> 77, of 64: 359 -> 217.  Two epilogue groups instead of three: 8 dimensions 107.
+//    Every wait on an mbarrier is bounded; on expiry an error code is recorded, which makes the exact scorer assign every point, no further
+//    wait is made and no copy started, and the CTA frees its TMEM at the common exit once its own copies and MMAs are complete.
 #include <mutex>
-
-#include <cuda_bf16.h>
 
 #include "common.cuh"
 
@@ -45,7 +46,11 @@ namespace tc {
 
 constexpr int kTileM = 128;
 constexpr int kMaxN = 256;
-constexpr uint32_t kWaitLimit = 1u << 22;
+constexpr uint32_t kWaitLimit = 1u << 18, kWaitHint = 4000;  // tries, and nanoseconds that one may take: about a second
+constexpr int kEpilogueGroups = 3, kEpilogueWarps = 4 * kEpilogueGroups, kProducerWarps = 8;
+constexpr int kMmaWarp = kEpilogueWarps + kProducerWarps, kMmaWarps = 2;  // one per pair of accumulators of 128 columns
+constexpr int kThreads = 32 * (kMmaWarp + kMmaWarps);
+constexpr int kBoundRing = 8;  // tiles whose error bounds are kept; more than the A ring and the two accumulators hold together
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -57,17 +62,7 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t addr, uint32_t lbo, uint3
   return ((uint64_t)hi << 32) | lo;
 }
 
-__device__ __forceinline__ void mma_tf32(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t"
-      "}\n" ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
-      : "memory");
-}
-
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t"
       ".reg .pred p;\n\t"
@@ -77,20 +72,37 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint6
       : "memory");
 }
 
-// x = b1 + b2 + (rest below 2^-18 |x|) with b1, b2 bf16 (round to nearest): eight values -> two 16-byte chunks
-__device__ __forceinline__ void split8_bf16(const float (&v)[8], uint4& c1, uint4& c2) {
-  uint32_t w1[4], w2[4];
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const __nv_bfloat16 a1 = __float2bfloat16_rn(v[2 * e]), b1 = __float2bfloat16_rn(v[2 * e + 1]);
-    const __nv_bfloat16 a2 = __float2bfloat16_rn(v[2 * e] - __bfloat162float(a1));
-    const __nv_bfloat16 b2 = __float2bfloat16_rn(v[2 * e + 1] - __bfloat162float(b1));
-    w1[e] = (uint32_t)__bfloat16_as_ushort(a1) | ((uint32_t)__bfloat16_as_ushort(b1) << 16);
-    w2[e] = (uint32_t)__bfloat16_as_ushort(a2) | ((uint32_t)__bfloat16_as_ushort(b2) << 16);
-  }
-  c1 = make_uint4(w1[0], w1[1], w1[2], w1[3]);
-  c2 = make_uint4(w2[0], w2[1], w2[2], w2[3]);
+__device__ __forceinline__ void mma_commit(uint32_t mbar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
 }
+
+__device__ __forceinline__ void mbar_init(uint32_t mbar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
+  asm volatile("{\n\t.reg .b64 s;\n\tmbarrier.arrive.shared::cta.b64 s, [%0];\n\t}" ::"r"(mbar) : "memory");
+}
+
+// A role's waits.  One that runs out is reported (code = 1 + tiles done) and no later one waits.
+struct Waiter {
+  int32_t* error;
+  bool gave_up;
+  __device__ __forceinline__ bool operator()(uint32_t mbar, uint32_t parity, int code) {
+    if (gave_up) return false;
+    for (uint32_t it = 0; it < kWaitLimit; ++it) {
+      uint32_t done;
+      asm volatile(
+          "{\n\t.reg .pred p;\n\t"
+          "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+          "selp.u32 %0, 1, 0, p;\n\t}\n"
+          : "=r"(done) : "r"(mbar), "r"(parity), "r"(kWaitHint) : "memory");
+      if (done) return true;
+    }
+    gave_up = true;
+    atomicExch(error, code);
+    return false;
+  }
+};
 
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
@@ -116,27 +128,12 @@ struct Params {
   int32_t* error;      // scratch: non-zero when a bounded wait expired
   int64_t n;
   int k, d;
-  int dp;      // d padded to a multiple of 8
-  int bf16;    // 1: operands are bf16 pairs (x = b1 + b2), A' = [x1 | x2 | x1], B' = [y1 | y1 | y2], kind::f16 (32 < d <= 64)
-  int n_pad;   // k padded to a multiple of 32 (epilogue reads 32 columns at a time; MMA N needs 16)
   int metric;
-  int vec4;    // rows of x can be read as float4
-  int y_vec4;  // and rows of y
+  int x_aligned;       // x starts on a 16-byte boundary
+  int x_wide, y_wide;  // rows can be read as float4
   float eps;   // relative error bound of one score
   const int32_t* done;  // when set and non-zero: nothing to do (a fit that has converged, kmeans_fit.cu)
 };
-
-constexpr int kGroupThreads = 256;  // two threads per point of the tile
-constexpr int kCtaThreads = 2 * kGroupThreads;
-
-__device__ __forceinline__ void group_sync(int g) { asm volatile("bar.sync %0, 256;" ::"r"(g + 1) : "memory"); }
-
-__device__ __forceinline__ void split4(const float (&v)[4], float4& hi, float4& lo) {
-  hi.x = __uint_as_float(__float_as_uint(v[0]) & 0xFFFFE000u); lo.x = v[0] - hi.x;
-  hi.y = __uint_as_float(__float_as_uint(v[1]) & 0xFFFFE000u); lo.y = v[1] - hi.y;
-  hi.z = __uint_as_float(__float_as_uint(v[2]) & 0xFFFFE000u); lo.z = v[2] - hi.z;
-  hi.w = __uint_as_float(__float_as_uint(v[3]) & 0xFFFFE000u); lo.w = v[3] - hi.w;
-}
 
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float r;
@@ -144,310 +141,414 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   return r;
 }
 
-// Shared memory: [B tile][A tile group 0][A tile group 1][scratch 256 floats][exchange 2 x 2 x 128 x 8 B][2 mbarriers]
-// [tmem slot][2 x 2 x 2 x 128 floats |x|^2]
-template <bool BF16>
-__global__ void __launch_bounds__(kCtaThreads, 1) kmeans_tc_kernel(const Params p) {
+__device__ __forceinline__ float sqrt_approx(float v) {
+  float r;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ void add_if_ge(int& sum, float a, float b, int add) {
+  asm("{\n\t.reg .pred q;\n\tsetp.ge.f32 q, %1, %2;\n\t@q add.s32 %0, %0, %3;\n\t}" : "+r"(sum) : "f"(a), "f"(b), "r"(add));
+}
+
+__device__ __forceinline__ float power2f(int e) { return __int_as_float((127 + e) << 23); }  // -127 < e < 128
+// |v| < 2^e for the largest such v; 0 for v = 0 and for what is not finite
+__device__ __forceinline__ int exponent_above(float v) {
+  const int b = (int)((__float_as_uint(v) & 0x7fffffffu) >> 23);
+  return b == 0 || b == 255 ? 0 : b - 126;
+}
+
+// v = c1 + c2 + rest: eight values -> two 16-byte chunks of f16
+__device__ __forceinline__ void split8(const float (&v)[8], uint4& c1, uint4& c2) {
+  uint32_t w1[4], w2[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const __half2 a = __floats2half2_rn(v[2 * e], v[2 * e + 1]);
+    const float2 f = __half22float2(a);
+    const __half2 b = __floats2half2_rn(v[2 * e] - f.x, v[2 * e + 1] - f.y);
+    w1[e] = *reinterpret_cast<const uint32_t*>(&a);
+    w2[e] = *reinterpret_cast<const uint32_t*>(&b);
+  }
+  c1 = make_uint4(w1[0], w1[1], w1[2], w1[3]);
+  c2 = make_uint4(w2[0], w2[1], w2[2], w2[3]);
+}
+
+// Eight values of a row from column t on; zeros behind its end and where !on.
+__device__ __forceinline__ void load8(const float* __restrict__ row, int t, int d, bool wide, bool on, float (&v)[8]) {
+  if (wide) {  // d % 4 == 0
+    const uint4 a = ldg_u128_if(row + t, on && t < d), b = ldg_u128_if(row + t + 4, on && t + 4 < d);
+    v[0] = __uint_as_float(a.x); v[1] = __uint_as_float(a.y); v[2] = __uint_as_float(a.z); v[3] = __uint_as_float(a.w);
+    v[4] = __uint_as_float(b.x); v[5] = __uint_as_float(b.y); v[6] = __uint_as_float(b.z); v[7] = __uint_as_float(b.w);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = on && t + e < d ? __ldg(row + t + e) : 0.0f;
+  }
+}
+
+// How a warp reads rows of C chunks of eight columns: lane = (row of R, chunk of CL), chunk fastest.  PAD bytes between the operands'
+// chunks make the eight lanes of a 16-byte store touch eight bank groups.
+template <int C>
+struct Lanes {
+  static constexpr int CL = C <= 2 ? C : C <= 4 ? 4 : 8;  // lanes per row
+  static constexpr int R = 32 / CL;                       // rows of one read
+  static constexpr int PAD = CL == 1 ? 0 : 128 / CL;
+  // A producer warp's rows of a tile come in PARTS of ROWS rows, one bulk copy each.
+  static constexpr int ROWS = C <= 4 ? 32 : 16, PARTS = 32 / ROWS, READS = ROWS / R;
+  static constexpr int PART_BYTES = ROWS * C * 32;
+};
+
+// Which 16-byte chunks the operands of the concatenated GEMM take.  Along K: [x1 | x2 | x1 | norm] against [y1 | y1 | y2 | norm], C
+// chunks each and one (C even: two, the second zero) for the norm; one MMA takes two neighbours of that sequence, whose distance
+// in shared memory a descriptor states.  So x1 is stored once, and y1 where no pair starts in one copy of it and ends in the next.
+template <int C>
+struct Operands {
+  static constexpr int steps = (3 * C + 2) / 2;
+  static constexpr int zero = C % 2 == 0 ? 1 : 0;  // a zero chunk behind the norm chunk
+  static constexpr int a_chunks = 2 * C + 1 + zero, b_chunks = C % 2 == 0 ? 2 * C + 2 : 3 * C + 1;
+  static constexpr int a_norm = 2 * C, b_norm = C % 2 == 0 ? 2 * C : 3 * C, b_low = C % 2 == 0 ? C : 2 * C;  // where norm and y2 start
+  static constexpr int a(int q) { return q < 2 * C ? q : q < 3 * C ? q - 2 * C : q - C; }
+  static constexpr int b(int q) { return C % 2 != 0 || q < C ? q : q - C; }
+};
+
+// What shared memory holds: A tiles in the ring, and parts of rows in flight per producer warp: 32 to 64 KB per SM (the DRAM's latency
+// holds about 35 at its full rate).  Tiles go to two producer groups and two MMA threads in turn, so with an odd number of stages a stage
+// changes hands; its barriers, of which each side has to see every phase, are then those of t % (2 * stages).
+template <int C, int NB>
+struct Ring {
+  static constexpr int stages = C >= 7 && NB == 8 ? 3 : 4, turns = stages % 2 ? 2 * stages : stages;
+  static constexpr int slots = C == 1 ? 8 : C == 2 ? 4 : C >= 7 ? 1 : 2;
+  static constexpr size_t bytes = (size_t)Operands<C>::b_chunks * (NB * 512 + Lanes<C>::PAD) + (size_t)Operands<C>::a_chunks * stages * (kTileM * 16 + Lanes<C>::PAD) +
+                                  (size_t)kProducerWarps * slots * Lanes<C>::PART_BYTES + kMaxN * 4 + kBoundRing * kTileM * 4 +
+                                  8 * (2 * turns + 4 * kEpilogueGroups + 6 + kProducerWarps * slots) + 16;
+  static_assert(bytes <= 227 * 1024, "shared memory of a CTA");
+};
+
+// Shared memory: [B tile][A ring][rows in flight][norms 256 floats][bounds kBoundRing x 128 floats][mbarriers, tmem slot]
+// C: chunks of eight dimensions of a row (1 to 8); NB: blocks of 32 columns (4: up to 128 centres, 8: up to 256).
+template <int C, int NB>
+__global__ void __launch_bounds__(kThreads, 1) kmeans_tc_kernel(const Params p) {
+  using L = Lanes<C>;
+  using O = Operands<C>;
+  using Q = Ring<C, NB>;
+  constexpr int N = 32 * NB;
+  constexpr uint32_t lbo_b = N * 16 + L::PAD, lbo_a = kTileM * 16 + L::PAD, sbo = 128;
   dependency_wait();  // first of all: the kernel launched behind this one relies on it (y_settled below)
   release_dependents();
   extern __shared__ __align__(128) unsigned char smem[];
   if (p.done != nullptr && *(volatile const int32_t*)p.done != 0) return;
-  const int tid = threadIdx.x;
-  const int g = tid >> 8;            // group
-  const int lt = tid & 255;          // thread within the group
-  const int pt = lt & 127;           // its point of the tile = its TMEM lane
-  const int half = lt >> 7;          // which half of the row's K chunks it loads and which half of the centres it scans
-  const int lane_quarter = (lt >> 5) & 3;
-  // 16-byte K chunks per operand row (the last two carry the norm term): 4 tf32 or 8 bf16 values per chunk
-  const int kc_x = BF16 ? 3 * p.dp / 8 : 3 * p.dp / 4;
-  const int kc = kc_x + 2;
-  const uint32_t lbo_b = kMaxN * 16, lbo_a = kTileM * 16, sbo = 128;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr uint32_t a_bytes = O::a_chunks * lbo_a;
   unsigned char* b_tile = smem;
-  unsigned char* a_tile = smem + (size_t)kc * lbo_b + (size_t)g * kc * lbo_a;
-  float* scratch = reinterpret_cast<float*>(smem + (size_t)kc * lbo_b + (size_t)2 * kc * lbo_a);
-  float2* exch = reinterpret_cast<float2*>(scratch + kMaxN) + g * 2 * kTileM;  // (best, its centre or -1) of half 1, for two tiles
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(scratch + kMaxN + 4 * kTileM * 2);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mbar + 2);
-  float* xx_all = reinterpret_cast<float*>(mbar + 8) + g * 4 * kTileM;  // |x|^2 of the points (tf32: two parts of it) of two tiles
+  unsigned char* a_ring = smem + O::b_chunks * lbo_b;
+  unsigned char* rows = a_ring + Q::stages * a_bytes;
+  float* norms = reinterpret_cast<float*>(rows + kProducerWarps * Q::slots * L::PART_BYTES);
+  float* bounds = norms + kMaxN;
+  uint64_t* mbars = reinterpret_cast<uint64_t*>(bounds + kBoundRing * kTileM);
+  // a_full[turns], a_free[turns], acc_full[kFull][HALVES], acc_free[4], drained[2], row_full[producer warp][slots].  A wait names the parity of a
+  // phase only, so whoever waits has to have seen the phase before, and the next one must not end before it has looked.  That an accumulator
+  // has become full is therefore a matter of its tile, t % kFull, where t + kFull has the same accumulator and the same epilogue group: its
+  // MMAs wait for those of all tiles between that have this accumulator, t among them, to have been read.
+  constexpr int HALVES = NB / 4, kFull = 4 * kEpilogueGroups / HALVES;
+  const uint32_t a_full = smem_u32(mbars), a_free = a_full + 8 * Q::turns, acc_full = a_free + 8 * Q::turns, acc_free = acc_full + 8 * kFull * HALVES,
+                 drained = acc_free + 32, row_full = drained + 16;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mbars + 2 * Q::turns + 6 + kFull * HALVES + kProducerWarps * Q::slots);
 
-  // ---- one-time setup: TMEM (all 512 columns: 256 per group), mbarriers, centre tile ----
-  if (tid < 32) {
+  const int64_t n_tiles = (p.n + kTileM - 1) / kTileM;
+  const int turns = (int)((n_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x);  // tiles of this CTA: blockIdx.x + t * gridDim.x
+  Waiter wait{p.error, false};
+
+  const int group = warp >= kEpilogueWarps ? (warp - kEpilogueWarps) >> 2 : warp >> 2;
+  const int row_l = lane / L::CL, chunk_l = lane % L::CL;
+  const bool producer = warp >= kEpilogueWarps && warp < kMmaWarp;
+  const int own = producer ? warp - kEpilogueWarps : 0;
+  unsigned char* own_rows = rows + own * (Q::slots * L::PART_BYTES);
+  const uint32_t own_full = row_full + (uint32_t)own * (8 * Q::slots);
+  // rows of part q of this warp's share of tile t: how many there are, and whether one bulk copy fetches them
+  auto part_base = [&](int t, int q) { return ((int64_t)blockIdx.x + (int64_t)t * gridDim.x) * kTileM + (warp & 3) * 32 + q * L::ROWS; };
+  auto part_bulk = [&](int64_t base) { return p.x_aligned && base + L::ROWS <= p.n; };
+  uint32_t fetched = 0;  // lane 0: bit s, slot s has had a bulk copy; bit 8 + s, the parity of its last one's phase
+  auto fetch = [&](int t, int q, int slot) {
+    if (t < turns && !wait.gave_up) {
+      const int64_t base = part_base(t, q);
+      const float* src = p.x + base * p.d;
+      const uint32_t dst = smem_u32(own_rows + slot * L::PART_BYTES);
+      if (part_bulk(base)) {
+        if (lane == 0) {
+          fetched = (fetched ^ (((fetched >> slot) & 1u) << (8 + slot))) | (1u << slot);
+          const uint32_t bytes = (uint32_t)(L::ROWS * 4 * p.d), full = own_full + 8u * slot;
+          asm volatile("{\n\t.reg .b64 s;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 s, [%0], %1;\n\t}" ::"r"(full), "r"(bytes) : "memory");
+          asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(full)
+                       : "memory");
+        }
+      } else {  // the last rows of x, or an x that starts off a 16-byte boundary
+        const int some = (int)max((int64_t)0, min((int64_t)L::ROWS, p.n - base)) * p.d;
+        for (int e = lane; e < some; e += 32) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + 4u * e), "l"(src + e) : "memory");
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+
+  // ---- one-time setup: mbarriers, TMEM (all 512 columns), centre tile ----
+  if (threadIdx.x == 32 * kMmaWarp) {
+    for (int s = 0; s < Q::turns; ++s) { mbar_init(a_full + 8 * s, 4); mbar_init(a_free + 8 * s, 1); }
+    for (int u = 0; u < kFull * HALVES; ++u) mbar_init(acc_full + 8 * u, 1);
+    for (int u = 0; u < 4; ++u) mbar_init(acc_free + 8 * u, 4);
+    for (int g = 0; g < 2; ++g) mbar_init(drained + 8 * g, 1);
+    for (int u = 0; u < kProducerWarps * Q::slots; ++u) mbar_init(row_full + 8 * u, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  if (warp == kMmaWarp) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(mbar)) : "memory");
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(mbar + 1)) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  if (producer) {  // the first rows, on their way while the centres are staged
+#pragma unroll
+    for (int u = 0; u < Q::slots; ++u) fetch(group + 2 * (u / L::PARTS), u % L::PARTS, u);
   }
-  // centre c = tid (first 256 threads, 256 rows); padded rows are zero with a norm term that never wins
-  if (tid < kMaxN) {
-    const int c = tid;
-    const int G = p.dp / 4;
-    // sixteen numbers of the row at a time, their loads in flight together (one at a time: 31 us for 256 x 64 and few points, now 18)
-    auto row16 = [&](int t0, float (&v)[16]) {
-      const float* yc = p.y + (int64_t)c * p.d;
+  constexpr int kStagers = 8;
+  constexpr int STEPS = (N / kStagers + L::R - 1) / L::R;  // reads that make a warp's share of the centres
+  static_assert(N / kStagers % L::R == 0 || STEPS == 1, "shares of whole reads");
+  const int c0 = warp * (STEPS * L::R);  // C = 1: the first N / 32 warps have 32 centres each
+  constexpr bool KEEP = STEPS <= 4;  // in registers between the two passes; more than 32 dimensions are read twice
+  float yv[KEEP ? STEPS : 1][8];
+  auto load_centres = [&](int s, float (&v)[8]) {
+    const int c = c0 + s * L::R + row_l;
+    load8(p.y + (int64_t)c * p.d, 8 * chunk_l, p.d, p.y_wide, c < p.k, v);
+  };
+  if (warp < kStagers) {
+    if constexpr (KEEP) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int t = t0 + 4 * q;
-        float4 w = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (c < p.k && p.y_vec4) {
-          if (t < p.d) w = __ldg(reinterpret_cast<const float4*>(yc + t));
-        } else if (c < p.k) {
-          if (t < p.d) w.x = __ldg(yc + t);
-          if (t + 1 < p.d) w.y = __ldg(yc + t + 1);
-          if (t + 2 < p.d) w.z = __ldg(yc + t + 2);
-          if (t + 3 < p.d) w.w = __ldg(yc + t + 3);
-        }
-        v[4 * q] = w.x; v[4 * q + 1] = w.y; v[4 * q + 2] = w.z; v[4 * q + 3] = w.w;
-      }
-    };
-    float nrm = 0.0f;
-    for (int t0 = 0; t0 < p.d; t0 += 16) {
-      float v[16];
-      row16(t0, v);
-#pragma unroll
-      for (int e = 0; e < 16; ++e) nrm = fmaf(v[e], v[e], nrm);
+      for (int s = 0; s < STEPS; ++s) load_centres(s, yv[s]);
     }
-    // cosine: rows are scaled to unit length (zero rows stay zero); L2: rows as they are
-    const float row_scale = p.metric == F2C_COSINE ? (nrm > 0.0f ? 1.0f / sqrtf(nrm) : 0.0f) : 1.0f;
-    for (int t0 = 0; t0 < p.dp; t0 += 16) {
-      float v[16];
-      row16(t0, v);
 #pragma unroll
-      for (int e = 0; e < 16; ++e) v[e] *= row_scale;
-      if constexpr (BF16) {
-        const int C = p.dp / 8;
+    for (int s = 0; s < STEPS; ++s) {
+      float (&v)[8] = yv[KEEP ? s : 0];
+      if constexpr (!KEEP) load_centres(s, v);
+      float nrm = 0.0f;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int cq = t0 / 8 + h;
-          const float w[8] = {v[8 * h], v[8 * h + 1], v[8 * h + 2], v[8 * h + 3], v[8 * h + 4], v[8 * h + 5], v[8 * h + 6], v[8 * h + 7]};
-          uint4 c1, c2;
-          split8_bf16(w, c1, c2);  // B' = [y1 | y1 | y2]; dp is a multiple of 16
-          *reinterpret_cast<uint4*>(b_tile + (size_t)(cq) * lbo_b + c * 16) = c1;
-          *reinterpret_cast<uint4*>(b_tile + (size_t)(C + cq) * lbo_b + c * 16) = c1;
-          *reinterpret_cast<uint4*>(b_tile + (size_t)(2 * C + cq) * lbo_b + c * 16) = c2;
-        }
-      } else {
+      for (int e = 0; e < 8; ++e) nrm = fmaf(v[e], v[e], nrm);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int gq = t0 / 4 + q;
-          if (gq < G) {
-            const float w[4] = {v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]};
-            float4 hi, lo;
-            split4(w, hi, lo);  // B' = [y_hi | y_hi | y_lo]
-            *reinterpret_cast<float4*>(b_tile + (size_t)(gq) * lbo_b + c * 16) = hi;
-            *reinterpret_cast<float4*>(b_tile + (size_t)(G + gq) * lbo_b + c * 16) = hi;
-            *reinterpret_cast<float4*>(b_tile + (size_t)(2 * G + gq) * lbo_b + c * 16) = lo;
-          }
-        }
-      }
+      for (int o = 1; o < L::CL; o <<= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
+      if (chunk_l == 0 && c0 + s * L::R + row_l < kMaxN) norms[c0 + s * L::R + row_l] = nrm;
     }
-    // norm term: -|y_c|^2 / 2 split in two TF32 values (L2), 0 (cosine), a value that never wins (padding)
-    float h = c < p.k ? (p.metric == F2C_L2 ? -0.5f * nrm : 0.0f) : -1e30f;
-    if (BF16) {  // three bf16 pieces of h against three ones on the point side
-      const __nv_bfloat16 h1 = __float2bfloat16_rn(h);
-      const __nv_bfloat16 h2 = __float2bfloat16_rn(h - __bfloat162float(h1));
-      const __nv_bfloat16 h3 = __float2bfloat16_rn(h - __bfloat162float(h1) - __bfloat162float(h2));
-      *reinterpret_cast<uint4*>(b_tile + (size_t)kc_x * lbo_b + c * 16) =
-          make_uint4((uint32_t)__bfloat16_as_ushort(h1) | ((uint32_t)__bfloat16_as_ushort(h2) << 16), (uint32_t)__bfloat16_as_ushort(h3), 0u, 0u);
-    } else {
-      const float h_hi = __uint_as_float(__float_as_uint(h) & 0xFFFFE000u);
-      *reinterpret_cast<float4*>(b_tile + (size_t)kc_x * lbo_b + c * 16) = make_float4(h_hi, h - h_hi, 0.0f, 0.0f);
-    }
-    *reinterpret_cast<float4*>(b_tile + (size_t)(kc_x + 1) * lbo_b + c * 16) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    scratch[c] = c < p.k ? nrm : 0.0f;
   }
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem_base = *tmem_slot + (uint32_t)g * 256u;
-  // largest centre norm (tolerance of the L2 score); a non-finite centre sends every point to the exact scorer
+  // largest centre norm (scale and tolerance of the L2 score); a non-finite centre sends every point to the exact scorer
   float cmax = 0.0f, poison = 0.0f;
 #pragma unroll
-  for (int c = threadIdx.x & 31; c < kMaxN; c += 32) { cmax = fmaxf(cmax, scratch[c]); poison = fmaf(scratch[c], 0.0f, poison); }  // inf, NaN -> NaN
+  for (int c = lane; c < N; c += 32) { cmax = fmaxf(cmax, norms[c]); poison = fmaf(norms[c], 0.0f, poison); }  // inf, NaN -> NaN
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     cmax = fmaxf(cmax, __shfl_xor_sync(0xffffffffu, cmax, o));
     poison += __shfl_xor_sync(0xffffffffu, poison, o);
   }
   const bool bad_centres = !(poison == 0.0f);
-  cmax = sqrtf(cmax);
-
-  // instruction descriptor: fp32 accumulate; A and B formats tf32 (2, kind::tf32) or bf16 (1, kind::f16); N / 8; M / 16
-  const uint32_t fmt = BF16 ? 1u : 2u;
-  const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(p.n_pad >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
-  const int ksteps = kc / 2;  // one MMA consumes 8 tf32 = two 16-byte chunks of K
-  const uint32_t mbar_addr = smem_u32(mbar + g);
-  uint32_t parity = 0;
-
-  const int64_t n_tiles = (p.n + kTileM - 1) / kTileM;
-  const int64_t first = (int64_t)blockIdx.x * 2 + g, stride = (int64_t)gridDim.x * 2;
-  // This thread's chunks of its point's row, fetched one tile ahead so that the global-load latency hides behind the
-  // previous tile's MMA and epilogue: chunk q of the thread is 16-byte chunk half + 2q of the row (tf32: d <= 32).
-  constexpr int kMaxChunks = BF16 ? 8 : 4;
-  float4 xv[kMaxChunks];
-  // bf16 path (rows of 132 to 256 bytes): the tile's rows are fetched and split by a different thread mapping than the
-  // one of the epilogue, so that a warp-wide load covers 8 rows x 128 contiguous bytes instead of 32 rows x 16 bytes
-  // (the load queue was the limiter): lane = (row pl of 8, 32-byte chunk cl of 4), warp wq of the group, item
-  // j = 0..3 -> row block 2 wq + (j >> 1), chunk cl + 4 (j & 1).  Shared-memory stores stay conflict-free (8 lanes =
-  // 8 consecutive rows of one chunk), |x|^2 goes through shared memory to the epilogue thread of the point.
-  const int wq = lt >> 5, pl = lt & 7, cl = (lt >> 3) & 3;
-  auto fetch_row = [&](int64_t tile_) {
-    const int64_t i_own = tile_ * kTileM + pt;
-    const int G = p.dp / 4;
+  const bool l2 = p.metric == F2C_L2;
+  const int e_y = l2 ? max(-120, min(120, exponent_above(sqrtf(cmax)))) : 0;  // squared L2: everything times 2^-e_y
+  const float scale_y = power2f(-e_y);
+  cmax = l2 ? sqrtf(cmax) * scale_y : 1.0f;
+  if (warp < kStagers) {
 #pragma unroll
-    for (int q = 0; q < kMaxChunks; ++q) {
-      const int gq = BF16 ? 2 * (cl + 4 * ((q >> 1) & 1)) + (q & 1) : half + 2 * q;
-      const int64_t i_ = BF16 ? tile_ * kTileM + (wq * 2 + (q >> 2)) * 8 + pl : i_own;
-      xv[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      if (gq < G && tile_ < n_tiles && i_ < p.n) {
-        if (p.vec4 && 4 * gq + 3 < p.d) {
-          xv[q] = __ldg(reinterpret_cast<const float4*>(p.x + i_ * p.d) + gq);
-        } else {
-          float v[4];
+    for (int s = 0; s < STEPS; ++s) {
+      const int c = c0 + s * L::R + row_l;
+      float (&v)[8] = yv[KEEP ? s : 0];
+      if constexpr (!KEEP) load_centres(s, v);
+      if (c < N) {
+        const float nrm = norms[c];
+        // cosine: rows of unit length (zero rows stay zero)
+        const float f = l2 ? scale_y : (nrm > 0.0f ? 1.0f / sqrtf(nrm) : 0.0f);
+        float own_sq = 0.0f;  // squared length of the scaled row, which the norm term takes: |y|^2 itself may overflow
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int t = 4 * gq + e;
-            v[e] = t < p.d ? __ldg(p.x + i_ * p.d + t) : 0.0f;
-          }
-          xv[q] = make_float4(v[0], v[1], v[2], v[3]);
+        for (int e = 0; e < 8; ++e) { v[e] *= f; own_sq = fmaf(v[e], v[e], own_sq); }
+        if (C == L::CL || chunk_l < C) {
+          uint4 c1, c2;
+          split8(v, c1, c2);
+          *reinterpret_cast<uint4*>(b_tile + (size_t)chunk_l * lbo_b + c * 16) = c1;
+          if (O::b_low > C) *reinterpret_cast<uint4*>(b_tile + (size_t)(C + chunk_l) * lbo_b + c * 16) = c1;
+          *reinterpret_cast<uint4*>(b_tile + (size_t)(O::b_low + chunk_l) * lbo_b + c * 16) = c2;
+        }
+#pragma unroll
+        for (int o = 1; o < L::CL; o <<= 1) own_sq += __shfl_xor_sync(0xffffffffu, own_sq, o);
+        if (chunk_l == 0) {
+          const float h = l2 && c < p.k ? -0.5f * own_sq : 0.0f;
+          const __half h1 = __float2half_rn(h), h2 = __float2half_rn(h - __half2float(h1));
+          const __half h3 = __float2half_rn(h - __half2float(h1) - __half2float(h2));
+          const __half never = __float2half_rn(c < p.k ? 0.0f : -65504.0f);
+          *reinterpret_cast<uint4*>(b_tile + (size_t)O::b_norm * lbo_b + c * 16) =
+              make_uint4((uint32_t)__half_as_ushort(h1) | ((uint32_t)__half_as_ushort(h2) << 16),
+                         (uint32_t)__half_as_ushort(h3) | ((uint32_t)__half_as_ushort(never) << 16), 0u, 0u);
+          if (O::zero) *reinterpret_cast<uint4*>(b_tile + (size_t)(O::b_norm + 1) * lbo_b + c * 16) = make_uint4(0u, 0u, 0u, 0u);
         }
       }
     }
-  };
-  // One barrier of the group per tile: it completes the A tile, ends the reading of the previous tile's accumulators and hands
-  // half 1's result for that tile to half 0, which writes the labels while the next MMAs run.  What crosses it is kept for two
-  // tiles in turn.
-  bool gave_up = false;  // a wait ran out: the error word makes the exact scorer assign every point, so just leave the loop's rhythm intact
-  float best = 0.0f, tol2 = 0.0f, xx = 0.0f;
-  int centre = -1;
-  int64_t i = -1;  // this thread's point of the tile before
-  int turn = 0;
-  auto finish = [&](int t) {  // half 0: labels of the tile before
-    const float2 o = exch[t * kTileM + pt];
-    const bool mine = best - tol2 > o.x, other = o.x - tol2 > best;
-    const int c = mine ? centre : (other ? __float_as_int(o.y) : -1);
-    const bool odd = bad_centres || !(xx < INFINITY) || !(fmaxf(best, o.x) > -INFINITY);  // NaN / inf somewhere: exact scorer
-    const bool mine_to_write = i >= 0 && i < p.n, undecided = mine_to_write && (odd || c < 0);
-    const uint32_t listed = __ballot_sync(0xffffffffu, undecided);  // the exact scorer assigns them afterwards
-    if (listed != 0u) {
-      int slot = 0;
-      if ((threadIdx.x & 31) == 0) slot = atomicAdd(p.amb_count, __popc(listed));
-      slot = __shfl_sync(0xffffffffu, slot, 0);
-      if (undecided) p.amb_list[slot + __popc(listed & ((1u << (threadIdx.x & 31)) - 1u))] = (int32_t)i;
+  } else if (producer) {
+    // what the norm chunk holds in every A tile (cosine: a one against the padding's number), and the zeros behind it
+    for (int i = threadIdx.x - 32 * kEpilogueWarps; i < Q::stages * kTileM; i += 32 * kProducerWarps) {
+      unsigned char* at = a_ring + (size_t)(i / kTileM) * a_bytes + (size_t)O::a_norm * lbo_a + i % kTileM * 16;
+      *reinterpret_cast<uint4*>(at) = make_uint4(0u, 0x3C000000u, 0u, 0u);
+      if (O::zero) *reinterpret_cast<uint4*>(at + lbo_a) = make_uint4(0u, 0u, 0u, 0u);
     }
-    if (mine_to_write && !undecided) p.labels[i] = c;
-  };
-  fetch_row(first);
-  for (int64_t tile = first; tile < n_tiles; tile += stride, turn ^= 1) {
-    float* xx_s = xx_all + turn * 2 * kTileM;
-    // ---- A tile: the two threads of point tile*128 + pt split and store alternate 16-byte chunks of its row ----
-    {
-      float sum = 0.0f;
-      const int G = p.dp / 4;
-      if (BF16) {
-        const int C = p.dp / 8;
-        float part[2] = {0.0f, 0.0f};  // this thread's share of |x|^2 of its two rows
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem_base = *tmem_slot;
+  // Tile t's columns 128 h .. 128 h + 127 are in accumulator (t, h) of four.
+  auto accumulator = [](int t, int h) { return 2 * (t & 1) + (NB == 8 ? h : (t >> 1) & 1); };
+
+  if (producer) {
+    const float eps = 2.0f * cmax * (bad_centres ? INFINITY : p.eps);  // what two scores may be off by together, per |x|
+    int unit = 0;
+    for (int t = group; t < turns; t += 2) {
+      unsigned char* a_tile = a_ring + (size_t)(t % Q::stages) * a_bytes;
+      if (t >= Q::stages) wait(a_free + 8 * ((t - Q::stages) % Q::turns), (uint32_t)((t - Q::stages) / Q::turns) & 1u, 1 + t);
 #pragma unroll
-        for (int q2 = 0; q2 < kMaxChunks / 2; ++q2) {
-          const int cq = cl + 4 * (q2 & 1);  // bf16 chunk = float4 chunks 2 cq, 2 cq + 1 = xv[2 q2], xv[2 q2 + 1]
-          const int ptl = (wq * 2 + (q2 >> 1)) * 8 + pl;
-          if (cq < C) {
-            const float v[8] = {xv[2 * q2].x, xv[2 * q2].y, xv[2 * q2].z, xv[2 * q2].w,
-                                xv[2 * q2 + 1].x, xv[2 * q2 + 1].y, xv[2 * q2 + 1].z, xv[2 * q2 + 1].w};
+      for (int q = 0; q < L::PARTS; ++q, ++unit) {
+        const int slot = unit % Q::slots;
+        asm volatile("cp.async.wait_group %0;" ::"n"(Q::slots - 1) : "memory");
+        if (part_bulk(part_base(t, q))) wait(own_full + 8 * slot, (uint32_t)(unit / Q::slots) & 1u, 1 + t);
+        __syncwarp();
+        // The reads go through every step side by side: their chains of dependent instructions are what a lone warp waits for.
+        float v[L::READS][8], top[L::READS], sum[L::READS], factor[L::READS];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) part[q2 >> 1] = fmaf(v[e], v[e], part[q2 >> 1]);
-            uint4 c1, c2;
-            split8_bf16(v, c1, c2);  // A' = [x1 | x2 | x1]
-            *reinterpret_cast<uint4*>(a_tile + (size_t)(cq) * lbo_a + ptl * 16) = c1;
-            *reinterpret_cast<uint4*>(a_tile + (size_t)(C + cq) * lbo_a + ptl * 16) = c2;
-            *reinterpret_cast<uint4*>(a_tile + (size_t)(2 * C + cq) * lbo_a + ptl * 16) = c1;
+        for (int b = 0; b < L::READS; ++b) {
+          const float* row = reinterpret_cast<const float*>(own_rows + slot * L::PART_BYTES) + (b * L::R + row_l) * p.d + 8 * chunk_l;
+          if (p.x_wide) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              float4 w = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+              if (8 * chunk_l + 4 * h < p.d) w = *reinterpret_cast<const float4*>(row + 4 * h);
+              v[b][4 * h] = w.x; v[b][4 * h + 1] = w.y; v[b][4 * h + 2] = w.z; v[b][4 * h + 3] = w.w;
+            }
+          } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[b][e] = 8 * chunk_l + e < p.d ? row[e] : 0.0f;
           }
         }
+        float any = 0.0f;
 #pragma unroll
-        for (int b = 0; b < 2; ++b) {
-          float v = part[b];
-          v += __shfl_xor_sync(0xffffffffu, v, 8);
-          v += __shfl_xor_sync(0xffffffffu, v, 16);
-          if (cl == 0) xx_s[(wq * 2 + b) * 8 + pl] = v;
+        for (int b = 0; b < L::READS; ++b) {
+          top[b] = max3(max3(fabsf(v[b][0]), fabsf(v[b][1]), fabsf(v[b][2])), max3(fabsf(v[b][3]), fabsf(v[b][4]), fabsf(v[b][5])),
+                        fmaxf(fabsf(v[b][6]), fabsf(v[b][7])));
+          any = fmaxf(any, top[b]);
+        }
+        // The slot's next copy may start when all lanes' reads have arrived, not merely been issued: the vote waits for what was read (it is always
+        // true; a barrier of the warp in its place let rows be overwritten before they were read).
+        if (__any_sync(0xffffffffu, !(any < 0.0f))) fetch(t + 2 * ((q + Q::slots) / L::PARTS), (q + Q::slots) % L::PARTS, slot);
+        if (l2) {
+#pragma unroll
+          for (int b = 0; b < L::READS; ++b) {
+            top[b] *= scale_y;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[b][e] *= scale_y;
+          }
+        }
+#pragma unroll
+        for (int b = 0; b < L::READS; ++b) {
+#pragma unroll
+          for (int o = 1; o < L::CL; o <<= 1) top[b] = fmaxf(top[b], __shfl_xor_sync(0xffffffffu, top[b], o));
+          // |v| < 2^ex.  Squared L2: among the centres the factor stays that of the centres, so that the norm term is not scaled up
+          const int biased = min(max(__float_as_int(top[b]) & 0x7f800000, l2 ? 126 << 23 : 0), 252 << 23);
+          factor[b] = __int_as_float((253 << 23) - biased);  // 2^-ex, ex = biased - 126
+        }
+#pragma unroll
+        for (int b = 0; b < L::READS; ++b) {
+          unsigned char* at = a_tile + (size_t)chunk_l * lbo_a + ((warp & 3) * 32 + q * L::ROWS + b * L::R + row_l) * 16;
+          float even = 0.0f, odd = 0.0f;
+#pragma unroll
+          for (int e = 0; e < 8; e += 2) {
+            v[b][e] *= factor[b]; v[b][e + 1] *= factor[b];
+            even = fmaf(v[b][e], v[b][e], even); odd = fmaf(v[b][e + 1], v[b][e + 1], odd);
+          }
+          sum[b] = even + odd;
+          uint4 c1, c2;
+          split8(v[b], c1, c2);
+          if (C == L::CL || chunk_l < C) {
+            *reinterpret_cast<uint4*>(at) = c1;
+            *reinterpret_cast<uint4*>(at + C * lbo_a) = c2;
+          }
+        }
+#pragma unroll
+        for (int b = 0; b < L::READS; ++b)
+#pragma unroll
+          for (int o = 1; o < L::CL; o <<= 1) sum[b] += __shfl_xor_sync(0xffffffffu, sum[b], o);
+        // one lane per row: its error bound, and (squared L2) its part of the norm term: powers of two against the pieces of -|y|^2 / 2 (0 for a
+        // point so far out that its own is no f16: the term is below the bound there), a one against the padding's
+        float own_sum = sum[0], own_factor = factor[0];
+#pragma unroll
+        for (int b = 1; b < L::READS; ++b)
+          if (chunk_l == b) { own_sum = sum[b]; own_factor = factor[b]; }
+        const int row = (warp & 3) * 32 + q * L::ROWS + chunk_l * L::R + row_l;
+        const float floor = 2.0f * cmax * (l2 ? fmaxf(0x1p-19f * own_factor, 0x1p-126f) : 0x1p-21f);  // f16 at its lower end, and the norm term
+        const float unscale = __int_as_float((254 << 23) - __float_as_int(own_factor)) * power2f(e_y);  // 1 / all that x was multiplied with
+        // INFINITY for NaN, and for a point whose |x|^2 is more than fp32 holds: the exact scorer's distance says so
+        const float bound = own_sum * unscale * unscale < INFINITY ? fminf(fmaf(eps, sqrt_approx(own_sum), floor), INFINITY) : INFINITY;
+        if (chunk_l < L::READS) {
+          bounds[(t & (kBoundRing - 1)) * kTileM + row] = bound;
+          if (l2) {
+            const uint32_t one = (uint32_t)__half_as_ushort(__float2half_rn(own_factor));
+            *reinterpret_cast<uint4*>(a_tile + (size_t)O::a_norm * lbo_a + row * 16) = make_uint4(one | (one << 16), one | 0x3C000000u, 0u, 0u);
+          }
         }
       }
-#pragma unroll
-      for (int q = 0; q < (BF16 ? 0 : kMaxChunks); ++q) {
-        const int gq = half + 2 * q;
-        if (gq < G) {
-          const float v[4] = {xv[q].x, xv[q].y, xv[q].z, xv[q].w};
-          sum = fmaf(v[0], v[0], sum); sum = fmaf(v[1], v[1], sum); sum = fmaf(v[2], v[2], sum); sum = fmaf(v[3], v[3], sum);
-          float4 hi, lo;
-          split4(v, hi, lo);
-          // A' = [x_hi | x_lo | x_hi]
-          *reinterpret_cast<float4*>(a_tile + (size_t)(gq) * lbo_a + pt * 16) = hi;
-          *reinterpret_cast<float4*>(a_tile + (size_t)(G + gq) * lbo_a + pt * 16) = lo;
-          *reinterpret_cast<float4*>(a_tile + (size_t)(2 * G + gq) * lbo_a + pt * 16) = hi;
-        }
-      }
-      if (!BF16) xx_s[half * kTileM + pt] = sum;
-      // norm-term columns: ones against the pieces of -|y|^2 / 2 (two tf32 ones, or three bf16 ones = 0x3F80 each)
-      *reinterpret_cast<uint4*>(a_tile + (size_t)(kc_x + half) * lbo_a + pt * 16) =
-          half != 0 ? make_uint4(0u, 0u, 0u, 0u)
-                    : (BF16 ? make_uint4(0x3F803F80u, 0x00003F80u, 0u, 0u) : make_uint4(0x3F800000u, 0x3F800000u, 0u, 0u));
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(a_full + 8 * (t % Q::turns));
     }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    group_sync(g);
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-
-    // ---- S = A' * B'^T into this group's TMEM columns ----
-    if (lt == 0) {
-      const uint32_t a_addr = smem_u32(a_tile), b_addr = smem_u32(b_tile);
-      for (int s_ = 0; s_ < ksteps; ++s_) {
-        const uint64_t a_desc = make_desc(a_addr + (uint32_t)s_ * 2u * lbo_a, lbo_a, sbo);
-        const uint64_t b_desc = make_desc(b_addr + (uint32_t)s_ * 2u * lbo_b, lbo_b, sbo);
-        if (BF16) mma_bf16(tmem_base, a_desc, b_desc, idesc, s_ > 0 ? 1u : 0u);
-        else mma_tf32(tmem_base, a_desc, b_desc, idesc, s_ > 0 ? 1u : 0u);
-      }
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar_addr) : "memory");
-    }
-    fetch_row(tile + stride);  // next tile's row, in flight during this tile's MMA and epilogue
-    if (half == 0) finish(turn ^ 1);
-    i = tile * kTileM + pt;
-    xx = BF16 ? xx_s[pt] : xx_s[pt] + xx_s[kTileM + pt];
-    // ---- bounded wait for the MMAs ----
-    uint32_t done = 0;
-    for (uint32_t it = 0; it < kWaitLimit && !done && !gave_up; ++it) {
-      asm volatile(
-          "{\n\t.reg .pred p;\n\t"
-          "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-          "selp.u32 %0, 1, 0, p;\n\t}\n"
-          : "=r"(done) : "r"(mbar_addr), "r"(parity) : "memory");
-    }
-    parity ^= 1u;
-    if (!done && !gave_up) {
-      gave_up = true;
-      atomicExch(p.error, 1 + (int)((tile - first) / stride));  // 1 + how many tiles this group had finished
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    if (wait.gave_up && lane == 0) {  // copies that have not been waited for: one per slot at most, since nothing was fetched after that wait
+      Waiter last{p.error, false};
+      for (int slot = 0; slot < Q::slots; ++slot)
+        if ((fetched >> slot) & 1u) last(own_full + 8 * slot, (fetched >> (8 + slot)) & 1u, 1 + turns);
     }
     __syncwarp();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-
-    // ---- epilogue: TMEM lane pt = point i; its two threads scan one half of the centres each ----
-    // Maxima only, one three-operand max per score: of the 16-column groups (row_max) and of the columns with the same number in
-    // their group (col_max).  Scores within 2 tol of the best lie in the crossings of the groups and columns whose maximum does,
-    // so the best centre is decided exactly when that is one group and one column - at the crossing.  (A running best, second
-    // best and index took five compare instructions per score, which issue at half rate: 2,449,029 points of 8 columns
-    // against 256 centres 275 us, 152 with this and one barrier per tile instead of three.)
-    const float xn = sqrtf(xx);
-    // error bound of a score: L2  eps*|x||y|max ;  cosine  eps*|x|
-    tol2 = 2.0f * (p.metric == F2C_L2 ? p.eps * xn * cmax : p.eps * xn);
-    const uint32_t lane_addr = tmem_base + ((uint32_t)(lane_quarter * 32) << 16);
-    const int c_split = ((p.n_pad / 32 + 1) / 2) * 32;
-    const int c_begin = half == 0 ? 0 : c_split, c_end = half == 0 ? c_split : p.n_pad;
-    constexpr int kGroups = kMaxN / 2 / 16;
-    float row_max[kGroups], col_max[16];
+  } else if (warp >= kMmaWarp) {
+    // One thread per pair of accumulators, with nothing but constants to add: its instructions follow one another at their full latency (one
+    // thread for both, descriptors made in the loop: 740 cycles a tile, more than the epilogue takes; a thread for each of the four: the
+    // same at 8 dimensions and 24 us slower at 2,449,029 x 32, whose MMAs then get in each other's way).
+    if (lane == 0) {
+      // instruction descriptor: fp32 accumulate; A and B f16 (0); 128 columns; M / 16
+      constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
+      const int g = warp - kMmaWarp;
+      const uint64_t b_base = make_desc(smem_u32(b_tile), 0, sbo);
+      bool on = true;
+      for (int t = g; t < turns && on; t += 2) {
+        const uint64_t a_base = make_desc(smem_u32(a_ring) + (uint32_t)(t % Q::stages) * a_bytes, 0, sbo);
+        on = wait(a_full + 8 * (t % Q::turns), (uint32_t)(t / Q::turns) & 1u, 1 + t);
 #pragma unroll
-    for (int j = 0; j < 16; ++j) col_max[j] = -INFINITY;
-    {
+        for (int h = 0; h < HALVES; ++h) {  // the epilogue reads one half of the columns while the other is made
+          const int a = accumulator(t, h);
+          on = on && wait(acc_free + 8 * a, ((uint32_t)(t >> (NB == 8 ? 1 : 2)) & 1u) ^ 1u, 1 + t);
+          if (!on) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+          for (int s = 0; s < O::steps; ++s) {  // one MMA consumes 16 f16 = two 16-byte chunks of K
+            constexpr auto part = [](int first, int second, uint32_t lbo) { return (uint64_t)((uint32_t)first * lbo >> 4) | (uint64_t)((uint32_t)(second - first) * lbo >> 4) << 16; };
+            mma_f16(tmem_base + (uint32_t)a * 128u, a_base + part(O::a(2 * s), O::a(2 * s + 1), lbo_a),
+                    b_base + part(O::b(2 * s), O::b(2 * s + 1), lbo_b) + (uint64_t)(h * 128), idesc, s > 0 ? 1u : 0u);
+          }
+          mma_commit(acc_full + 8 * (HALVES * (t % kFull) + h));
+        }
+        if (on) mma_commit(a_free + 8 * (t % Q::turns));
+      }
+      mma_commit(drained + 8 * g);  // after a wait that ran out nobody else has waited for the MMAs in flight
+      Waiter last{p.error, false};
+      last(drained + 8 * g, 0u, 1 + turns);
+    }
+    __syncwarp();
+  } else {
+    // ---- epilogue: TMEM lane pt = point; its thread scans all centres ----
+    // Maxima only, one three-operand max per score: of the 16-column groups (row_max) and of the columns with the same number in
+    // their group (col_max).  Scores within the bound of the best lie in the crossings of the groups and columns whose maximum does,
+    // so the best centre is decided exactly when that is one group and one column - at the crossing.  (A running best, second
+    // best and index took five compare instructions per score, which issue at half rate.)
+    const int pt = (warp & 3) * 32 + lane;
+    const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
+    constexpr int kGroups = 2 * NB;
+    uint32_t turn = 0;  // which of this group's tiles
+    for (int t = group; t < turns; t += kEpilogueGroups, ++turn) {
+      float row_max[kGroups], col_max[16], bound = 0.0f;
       uint32_t ra[16], rb[16];  // two 16-column loads alternate: one is consumed while the other is in flight
       auto group_max = [&](const uint32_t (&r)[16]) {
         auto f = [&](int j) { return __uint_as_float(r[j]); };
@@ -455,48 +556,92 @@ __global__ void __launch_bounds__(kCtaThreads, 1) kmeans_tc_kernel(const Params 
         const float m4 = max3(f(12), f(13), f(14));
         return fmaxf(max3(m0, m1, m2), max3(m3, m4, f(15)));
       };
-      if (c_begin < c_end) tmem_ld16(lane_addr + (uint32_t)c_begin, ra);
 #pragma unroll
-      for (int q = 0; q < kGroups; q += 2) {  // c_end - c_begin is a multiple of 32
-        const int c0 = c_begin + 16 * q;
-        row_max[q] = -INFINITY;
-        row_max[q + 1] = -INFINITY;
-        if (c0 < c_end) {
+      for (int h = 0; h < HALVES; ++h) {
+        constexpr uint32_t laps = kFull / kEpilogueGroups;  // barriers that this group uses in turn
+        const int a = accumulator(t, h);
+        wait(acc_full + 8 * (HALVES * (group + kEpilogueGroups * (turn % laps)) + h), (turn / laps) & 1u, 1 + t);
+        __syncwarp();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (h == 0) bound = bounds[(t & (kBoundRing - 1)) * kTileM + pt];  // before acc_free: a later tile's takes its place
+        const uint32_t addr = lane_addr + (uint32_t)a * 128u;
+        tmem_ld16(addr, ra);
+#pragma unroll
+        for (int q = 0; q < 8; q += 2) {
           tmem_wait(ra);
-          tmem_ld16(lane_addr + (uint32_t)(c0 + 16), rb);
-          row_max[q] = group_max(ra);
+          tmem_ld16(addr + (uint32_t)(16 * q + 16), rb);
+          row_max[8 * h + q] = group_max(ra);
           float own[16];
 #pragma unroll
           for (int j = 0; j < 16; ++j) own[j] = __uint_as_float(ra[j]);
           tmem_wait(rb);
-          if (c0 + 32 < c_end) tmem_ld16(lane_addr + (uint32_t)(c0 + 32), ra);
-          row_max[q + 1] = group_max(rb);
+          if (q + 2 < 8) {
+            tmem_ld16(addr + (uint32_t)(16 * q + 32), ra);
+          } else {  // the next MMAs may overwrite the accumulator
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(acc_free + 8 * a);
+          }
+          row_max[8 * h + q + 1] = group_max(rb);
 #pragma unroll
-          for (int j = 0; j < 16; ++j) col_max[j] = max3(col_max[j], own[j], __uint_as_float(rb[j]));
+          for (int j = 0; j < 16; ++j)
+            col_max[j] = h == 0 && q == 0 ? fmaxf(own[j], __uint_as_float(rb[j])) : max3(col_max[j], own[j], __uint_as_float(rb[j]));
         }
       }
+      float best = row_max[0];
+#pragma unroll
+      for (int q = 1; q + 1 < kGroups; q += 2) best = max3(best, row_max[q], row_max[q + 1]);
+      best = fmaxf(best, row_max[kGroups - 1]);
+      // hits, each counted as 64 + its number: from 64 to 127 there was one
+      const float from = best - bound;
+      int rows_hit[2] = {0, 0}, cols_hit[2] = {0, 0};
+#pragma unroll
+      for (int q = 0; q < kGroups; ++q) add_if_ge(rows_hit[q & 1], row_max[q], from, 64 + q);
+#pragma unroll
+      for (int j = 0; j < 16; ++j) add_if_ge(cols_hit[j & 1], col_max[j], from, 64 + j);
+      const int r_hit = rows_hit[0] + rows_hit[1], c_hit = cols_hit[0] + cols_hit[1];
+      const int centre = 16 * r_hit + c_hit - (16 * 64 + 64);
+      const bool decided = (r_hit >> 6) == 1 && (c_hit >> 6) == 1 && best > -INFINITY;
+      const int64_t i = ((int64_t)blockIdx.x + (int64_t)t * gridDim.x) * kTileM + pt;
+      const bool undecided = i < p.n && !decided;
+      const uint32_t listed = __ballot_sync(0xffffffffu, undecided);  // the exact scorer assigns them afterwards
+      if (listed != 0u) {
+        int slot = 0;
+        if (lane == 0) slot = atomicAdd(p.amb_count, __popc(listed));
+        slot = __shfl_sync(0xffffffffu, slot, 0);
+        if (undecided) p.amb_list[slot + __popc(listed & ((1u << lane) - 1u))] = (int32_t)i;
+      }
+      if (i < p.n && decided) p.labels[i] = centre;
     }
-    static_assert(kGroups == 8, "the tree below");
-    best = max3(max3(row_max[0], row_max[1], row_max[2]), max3(row_max[3], row_max[4], row_max[5]), fmaxf(row_max[6], row_max[7]));
-    // hits, each counted as 64 + its number: below 128 there was one
-    const float from = best - tol2;
-    int rows_hit = 0, cols_hit = 0;
-#pragma unroll
-    for (int q = 0; q < kGroups; ++q) rows_hit += row_max[q] >= from ? 64 + q : 0;
-#pragma unroll
-    for (int j = 0; j < 16; ++j) cols_hit += col_max[j] >= from ? 64 + j : 0;
-    centre = rows_hit < 128 && cols_hit < 128 ? c_begin + 16 * (rows_hit - 64) + cols_hit - 64 : -1;
-    if (half == 1) exch[turn * kTileM + pt] = make_float2(best, __int_as_float(centre));
   }
-  group_sync(g);
-  if (half == 0) finish(turn ^ 1);
 
   // ---- common exit: all TMEM reads retired, then the allocating warp frees the columns ----
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (tid < 32) {
+  if (warp == kMmaWarp) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(*tmem_slot), "r"(512u) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+  }
+}
+
+struct Kernel {
+  void (*kern)(const Params);
+  size_t smem;
+};
+template <int C>
+static Kernel kernel_for(int64_t k) {
+  return k <= 128 ? Kernel{kmeans_tc_kernel<C, 4>, Ring<C, 4>::bytes} : Kernel{kmeans_tc_kernel<C, 8>, Ring<C, 8>::bytes};
+}
+static Kernel kernel_for(int64_t k, int64_t d) {
+  switch ((d + 7) / 8) {
+    case 1: return kernel_for<1>(k);
+    case 2: return kernel_for<2>(k);
+    case 3: return kernel_for<3>(k);
+    case 4: return kernel_for<4>(k);
+    case 5: return kernel_for<5>(k);
+    case 6: return kernel_for<6>(k);
+    case 7: return kernel_for<7>(k);
+    default: return kernel_for<8>(k);
   }
 }
 
@@ -511,29 +656,22 @@ int kmeans_assign_tc(const float* x, const float* y, int64_t* labels, int64_t n,
   tc::Params p{};
   p.done = done;
   p.x = x; p.y = y; p.labels = labels; p.n = n; p.k = (int)k; p.d = (int)d; p.metric = metric;
-  p.dp = (int)((d + 7) / 8 * 8);
-  p.bf16 = p.dp > 32 ? 1 : 0;  // 3 x tf32 does not fit in shared memory beyond d = 32; 3 x bf16 does up to d = 64
-  if (p.bf16) p.dp = (int)((d + 15) / 16 * 16);  // one bf16 MMA consumes 16 values of K
-  p.n_pad = (int)((k + 31) / 32 * 32);
-  p.vec4 = d % 4 == 0 && aligned(x, 16);
-  p.y_vec4 = d % 4 == 0 && aligned(y, 16);
-  // relative error bound of one score: 2^-16 for the tf32 split (true error ~2^-18.4); 2^-14 for the bf16 split
-  // (neglected terms x2.y2 + x.y3 + x3.y <= 3 * 2^-18 |x||y| = 2^-16.4)
-  p.eps = p.bf16 ? 1.0f / 16384.0f : 1.0f / 65536.0f;
+  p.x_aligned = aligned(x, 16);
+  p.x_wide = d % 4 == 0;  // of the copy in shared memory
+  p.y_wide = d % 4 == 0 && aligned(y, 16);
+  // relative error bound of one score: the split leaves 3 * 2^-22 of |x||y|, the rest is the sums of up to 13 MMAs of 16 products
+  p.eps = d <= 32 ? 1.0f / 65536.0f : 1.0f / 32768.0f;
   int32_t* head = reinterpret_cast<int32_t*>(workspace);
   p.amb_count = head; p.error = head + 1; p.amb_list = head + 64;
   cudaError_t e = head_is_clear ? cudaSuccess : cudaMemsetAsync(head, 0, 256, st);
   if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "kmeans_assign: %s", cudaGetErrorString(e));
-  const int kc = (p.bf16 ? 3 * p.dp / 8 : 3 * p.dp / 4) + 2;
-  size_t smem = (size_t)kc * (tc::kMaxN + 2 * tc::kTileM) * 16 + tc::kMaxN * 4 + 4 * tc::kTileM * 8 + 64 + 8 * tc::kTileM * 4;
+  auto [kern, smem] = tc::kernel_for(k, d);
   if (smem < 120 * 1024) smem = 120 * 1024;  // one CTA per SM: a second one would only wait for the TMEM columns
-  auto kern = p.bf16 ? tc::kmeans_tc_kernel<true> : tc::kmeans_tc_kernel<false>;
   e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "kmeans_assign: %s", cudaGetErrorString(e));
-  int64_t tiles = ceil_div(n, tc::kTileM);
-  int64_t grid = ceil_div(tiles, 2);  // one CTA per SM (it owns all 512 TMEM columns), two tiles in flight per CTA
-  if (grid > current_sm_count()) grid = current_sm_count();
-  launch_dependent(kern, (unsigned)grid, tc::kCtaThreads, smem, st, p);
+  int64_t grid = ceil_div(n, tc::kTileM);
+  if (grid > current_sm_count()) grid = current_sm_count();  // one CTA per SM (it owns all 512 TMEM columns)
+  launch_dependent(kern, (unsigned)grid, tc::kThreads, smem, st, p);
   int rc = check_launch("kmeans_assign (tensor cores)");
   if (rc) return rc;
   // undecided points (all of them after a wait that ran out): exact fp32 scorer over the device-side list

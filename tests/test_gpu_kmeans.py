@@ -204,3 +204,22 @@ def test_fit_keeps_the_precision_of_small_columns(capi, n, k, d):
     want = torch.zeros(k, d, dtype=torch.float64, device="cuda").index_add_(0, labels, x.double())
     want /= torch.bincount(labels, minlength=k).double()[:, None]
     assert words[1] == 1 and float(((got.double() - want).abs() / want).max()) < 2.0**-22  # two roundings of 2^-24, doubled
+
+
+@pytest.mark.parametrize("d", [1, 7, 8, 13, 16, 24, 31, 32, 40, 48, 52, 56, 64])
+def test_tensor_core_assignment_at_the_edges_of_its_tiles(capi, d):
+    """Chunk counts, both column counts, one to four tiles per CTA with ragged ends, rows that start off a 16-byte boundary, magnitudes far
+    from one: labels of the exact fp32 scorer, call after call (a lost wait shows now and then only)."""
+    from f2cgt_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(d)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for n in (1, 127, 129, sms * 128 + 1, 3 * sms * 128 + 77):
+        for k in (1, 128, 129, 256):
+            offset = (n + k) % 3
+            x = torch.randn(n * d + offset, device="cuda", generator=g)[offset:].view(n, d)
+            c = torch.randn(k * d + offset, device="cuda", generator=g)[offset:].view(k, d)
+            for metric, size in (("l2", 1.0), ("cosine", 1.0), ("cosine", 1e-15), ("cosine", 1e15)):
+                y = x if size == 1.0 else (x * size).contiguous()
+                exact = ops.kmeans_assign(y, c, metric, scorer="exact")
+                for _ in range(3):
+                    assert torch.equal(ops.kmeans_assign(y, c, metric, scorer="tensor"), exact), (n, k, metric, size)
