@@ -13,14 +13,9 @@
 //    with 128-bit reads, four FMAs per read.  This is the exact fp32 scorer; the points whose best two
 //    candidates are too close to call for the tensor-core kernel (kmeans_tc.cu) go through
 //    kmeans_listed_kernel, which computes the same distances.
-#include "common.cuh"
+#include "kmeans_fit.cuh"
 
 namespace f2c {
-
-__device__ __forceinline__ float finish_cosine(float dot, float xx, float cc) {
-  float den = sqrtf(xx) * sqrtf(cc);
-  return den > 0.0f ? 1.0f - dot / den : 1.0f;
-}
 
 // ---------------------------------------------------------------- warp per point
 template <int METRIC, bool WRITE_DIST, bool WRITE_LABEL>
@@ -330,7 +325,7 @@ int kmeans_assign_exact_listed(const float* x, const float* y, int64_t* labels, 
 bool kmeans_tc_supported(int64_t n, int64_t k, int64_t d);
 int64_t kmeans_tc_workspace(int64_t n);
 int kmeans_assign_tc(const float* x, const float* y, int64_t* labels, int64_t n, int64_t k, int64_t d, int metric, void* workspace,
-                     cudaStream_t st, const int32_t* done, bool head_is_clear);
+                     cudaStream_t st);
 
 static int validate_km(const char* op, int64_t n, int64_t k, int64_t d, int metric) {
   F2C_REQUIRE(n >= 0 && k >= 1 && d >= 1, F2C_ERR_INVALID, "%s: bad shape n=%lld k=%lld d=%lld", op, (long long)n, (long long)k,
@@ -377,6 +372,6 @@ extern "C" int f2c_kmeans_assign(const float* x, const float* centers, int64_t* 
   // exact scorer 982 us, tensor cores 104)
   const bool prefer_tc = d >= 4 || scorer == F2C_SCORER_TENSOR;
   if (workspace != nullptr && kmeans_tc_supported(n, k, d) && prefer_tc && scorer != F2C_SCORER_EXACT && aligned(workspace, 16))
-    return kmeans_assign_tc(x, centers, labels, n, k, d, metric, workspace, (cudaStream_t)stream, nullptr, false);
+    return kmeans_assign_tc(x, centers, labels, n, k, d, metric, workspace, (cudaStream_t)stream);
   return kmeans_assign_exact(x, centers, labels, n, k, d, metric, (cudaStream_t)stream, nullptr);
 }

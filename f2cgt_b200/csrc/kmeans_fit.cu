@@ -1,10 +1,11 @@
 // Lloyd iterations of KMeans.fit (reference: RAFT kmeans::fit behind src/kmeans.cu:61-75, and the torch loop of
 // examples/my_kmeans.py:73-113) queued on the device without a host read per iteration.
 //
-// One iteration = the assignment kernels (kmeans_tc.cu / kmeans.cu) + ONE kernel that sums every cluster's points and, in
-// the CTA that finishes last, replaces the centres, measures their shift and raises the `done` word.  All kernels of an
-// iteration return at once when that word is set, so the caller queues several iterations ahead and looks at the word
-// every few of them; iterations queued behind the converged one change nothing.
+// Shapes of the tensor cores (up to 256 centres, 4 to 64 dimensions): kmeans_fit_tc.cu, a kernel for many iterations.  All others, here:
+// one iteration = the exact assignment (kmeans.cu) + ONE kernel that sums every cluster's points and, in the CTA that finishes last,
+// replaces the centres, measures their shift and raises the `done` word.  All kernels return at once when that word is set, so the
+// caller queues several iterations ahead and looks at the word every few of them; iterations queued behind the converged one change
+// nothing.
 //
 //  * Sums are exact and independent of the order of the additions: a value becomes a fixed-point integer (43 fraction bits
 //    below the largest magnitude of its column, fewer when more than 2^18 points could overflow 63 bits), and integers
@@ -13,16 +14,13 @@
 //  * Inside a CTA the integers are added in shared memory as two 22-bit limbs with 32-bit atomics without a result (the
 //    64-bit ones are a compare-and-swap loop); at most 1023 points can be added before a limb could overflow, so a CTA
 //    takes chunks of at most 1000 points and adds the touched clusters to the 64-bit sums in global memory.
-//
-// Measured on B200, 147,000 points x 32 dimensions, 256 centres: see launch_accumulate().
-#include "common.cuh"
+#include "kmeans_fit.cuh"
 
 namespace f2c {
 
 bool kmeans_tc_supported(int64_t n, int64_t k, int64_t d);
-int64_t kmeans_tc_workspace(int64_t n);
-int kmeans_assign_tc(const float* x, const float* y, int64_t* labels, int64_t n, int64_t k, int64_t d, int metric, void* workspace,
-                     cudaStream_t st, const int32_t* done, bool head_is_clear);
+int kmeans_fit_tc(const float* x, float* centers, int64_t n, int64_t k, int64_t d, int metric, double tol, int iterations, FitState* state, long long* sums,
+                  uint32_t* counts, const uint32_t* maxima, uint16_t* labels, double* shifts, int32_t* error, cudaStream_t st);
 int kmeans_assign_exact(const float* x, const float* y, int64_t* labels, int64_t n, int64_t k, int64_t d, int metric, cudaStream_t st,
                         const int32_t* done);
 
@@ -31,25 +29,6 @@ namespace fit {
 constexpr int kThreads = 512;
 constexpr int kChunk = 1000;                 // points whose limbs cannot overflow 32 bits
 constexpr size_t kSmemLimit = 200 * 1024;
-
-struct State {       // first 256 bytes of the workspace; the host reads the first four words
-  int32_t done;
-  int32_t iterations;
-  int32_t not_finite;   // the data hold inf or NaN: nothing is iterated, the caller says so
-  int32_t assign_error; // code of the last bounded wait of the tensor-core kernel that ran out (the exact scorer then assigned every point)
-  uint32_t pad;
-  uint32_t arrived;
-  double shift;
-};
-
-__device__ __forceinline__ int fraction_bits(int64_t n) {
-  const int lg = 64 - __clzll((unsigned long long)n);  // 2^lg > n
-  return min(43, 61 - lg);
-}
-
-// |x| <= 2^e for the float with these bits; a value of the column becomes an integer multiple of 2^(e - bits)
-__device__ __forceinline__ int exponent(uint32_t max_bits) { return max_bits == 0u ? 0 : (int)(max_bits >> 23) - 126; }
-__device__ __forceinline__ double power2(int e) { return __hiloint2double((1023 + e) << 20, 0); }  // |e| < 1023
 
 // Largest |x| of every column as float bits.  `threads` is a multiple of d, so that a thread stays in its column; d above the grid's
 // threads: every thread walks over columns.
@@ -82,7 +61,7 @@ __global__ void __launch_bounds__(256) max_abs_kernel(const float* __restrict__ 
   }
 }
 
-__global__ void begin_kernel(const uint32_t* __restrict__ maxima, int d, State* st) {
+__global__ void begin_kernel(const uint32_t* __restrict__ maxima, int d, FitState* st) {
   dependency_wait();
   release_dependents();
   for (int j = threadIdx.x; j < d; j += blockDim.x)
@@ -93,7 +72,7 @@ __global__ void begin_kernel(const uint32_t* __restrict__ maxima, int d, State* 
 // scale_of(j): what column j's values were multiplied with, a power of two.
 template <typename Scale>
 __device__ void finish_iteration(float* __restrict__ centers, long long* sums, unsigned int* counts, int k, int d, Scale scale_of, double tol,
-                                 int32_t* assign_head, State* st) {
+                                 FitState* st) {
   __shared__ double part[kThreads / 32];
   double shift = 0.0;
   // this CTA alone works now: the loads of eight entries are in flight together (one at a time: 11 of 23 us for 256 x 32)
@@ -135,11 +114,6 @@ __device__ void finish_iteration(float* __restrict__ centers, long long* sums, u
     st->shift = total;
     st->iterations += 1;
     st->arrived = 0u;
-    if (assign_head != nullptr) {
-      // after a wait that ran out the labels are the exact scorer's, so the iteration counts and the next one starts afresh
-      if (assign_head[1] != 0) st->assign_error = assign_head[1];
-      assign_head[0] = assign_head[1] = 0;
-    }
     if ((double)(float)total <= tol) st->done = 1;
   }
 }
@@ -149,7 +123,7 @@ template <bool SHARED>
 __global__ void __launch_bounds__(kThreads) accumulate_kernel(const float* __restrict__ x, const int64_t* __restrict__ labels,
                                                               float* __restrict__ centers, long long* sums, unsigned int* counts,
                                                               const uint32_t* __restrict__ maxima, int64_t n, int k, int d, double tol,
-                                                              int32_t* assign_head, State* st) {
+                                                              FitState* st) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int kd = k * d;
   double* scales = reinterpret_cast<double*>(smem);  // of the columns
@@ -222,11 +196,11 @@ __global__ void __launch_bounds__(kThreads) accumulate_kernel(const float* __res
   __syncthreads();
   if (last) {
     __threadfence();
-    finish_iteration(centers, sums, counts, k, d, scale_of, tol, assign_head, st);
+    finish_iteration(centers, sums, counts, k, d, scale_of, tol, st);
   }
 }
 
-struct Layout { size_t sums, counts, labels, assign, maxima, total; };
+struct Layout { size_t sums, counts, labels, assign, maxima, shifts, total; };
 
 static Layout plan(int64_t n, int64_t k, int64_t d) {
   auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
@@ -235,8 +209,9 @@ static Layout plan(int64_t n, int64_t k, int64_t d) {
   w.sums = at; at += up((size_t)k * d * 8);
   w.counts = at; at += up((size_t)k * 4);
   w.labels = at; at += up((size_t)n * 8);
-  w.assign = at; at += kmeans_tc_supported(n, k, d) ? up((size_t)kmeans_tc_workspace(n)) : 0;
+  w.assign = at; at += 256;  // second word: code of a bounded wait of the tensor-core kernel that ran out
   w.maxima = at; at += up((size_t)d * 4);
+  w.shifts = at; at += up((size_t)current_sm_count() * 8);
   w.total = at;
   return w;
 }
@@ -265,10 +240,10 @@ extern "C" int f2c_kmeans_fit_begin(const float* x, int64_t n, int64_t k, int64_
   cudaStream_t st = (cudaStream_t)stream;
   const fit::Layout w = fit::plan(n, k, d);
   cudaError_t e = cudaMemsetAsync(workspace, 0, w.labels, st);  // state, sums and counts
-  if (e == cudaSuccess && kmeans_tc_supported(n, k, d)) e = cudaMemsetAsync((unsigned char*)workspace + w.assign, 0, 256, st);
-  if (e == cudaSuccess) e = cudaMemsetAsync((unsigned char*)workspace + w.maxima, 0, (size_t)d * 4, st);
+  if (e == cudaSuccess) e = cudaMemsetAsync((unsigned char*)workspace + w.assign, 0, w.shifts - w.assign, st);  // error, maxima
+  if (e == cudaSuccess && kmeans_tc_supported(n, k, d)) e = cudaMemsetAsync((uint16_t*)((unsigned char*)workspace + w.labels) + n, 0xff, (size_t)n * 2, st);  // summed: none
   if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "%s: %s", op, cudaGetErrorString(e));
-  fit::State* state = (fit::State*)workspace;
+  FitState* state = (FitState*)workspace;
   int64_t blocks = ceil_div(n * d, 256 * 8);
   if (blocks > 8 * current_sm_count()) blocks = 8 * current_sm_count();
   uint32_t* maxima = (uint32_t*)((unsigned char*)workspace + w.maxima);
@@ -287,12 +262,16 @@ extern "C" int f2c_kmeans_fit_iterate(const float* x, float* centers, int64_t n,
   cudaStream_t st = (cudaStream_t)stream;
   const fit::Layout w = fit::plan(n, k, d);
   unsigned char* ws = (unsigned char*)workspace;
-  fit::State* state = (fit::State*)ws;
+  FitState* state = (FitState*)ws;
   long long* sums = (long long*)(ws + w.sums);
   unsigned int* counts = (unsigned int*)(ws + w.counts);
   int64_t* labels = (int64_t*)(ws + w.labels);
-  const bool tc = kmeans_tc_supported(n, k, d) && d >= 4;
-  int32_t* assign_head = tc ? (int32_t*)(ws + w.assign) : nullptr;  // [undecided points, error]; cleared by f2c_kmeans_fit_begin, then by every iteration
+  // the line is that of the assignment (kmeans.cu)
+  if (kmeans_tc_supported(n, k, d) && d >= 4) {
+    if (iterations == 0) return F2C_OK;
+    return kmeans_fit_tc(x, centers, n, k, d, metric, tol, iterations, state, sums, counts, (const uint32_t*)(ws + w.maxima), (uint16_t*)labels,
+                         (double*)(ws + w.shifts), (int32_t*)(ws + w.assign) + 1, st);
+  }
   const size_t smem = (size_t)d * 8 + ((size_t)2 * k * d + k) * 4 + fit::kChunk * 2;
   const uint32_t* maxima = (const uint32_t*)(ws + w.maxima);
   const bool shared = smem <= fit::kSmemLimit && k <= 65535;
@@ -305,11 +284,10 @@ extern "C" int f2c_kmeans_fit_iterate(const float* x, float* centers, int64_t n,
   int64_t grid = shared ? ceil_div(n, 256) : ceil_div(n * d, fit::kThreads);
   if (grid > current_sm_count()) grid = current_sm_count();
   for (int it = 0; it < iterations; ++it) {
-    rc = tc ? kmeans_assign_tc(x, centers, labels, n, k, d, metric, ws + w.assign, st, &state->done, true)
-            : kmeans_assign_exact(x, centers, labels, n, k, d, metric, st, &state->done);
+    rc = kmeans_assign_exact(x, centers, labels, n, k, d, metric, st, &state->done);
     if (rc) return rc;
     launch_dependent(kern, (unsigned)grid, fit::kThreads, shared ? smem : 0, st, x, labels, centers, sums, counts, maxima, n, (int)k, (int)d, tol,
-                     assign_head, state);
+                     state);
     rc = check_launch(op);
     if (rc) return rc;
   }

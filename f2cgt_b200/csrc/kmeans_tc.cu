@@ -1,41 +1,7 @@
-// K-means assignment on the 5th-generation tensor cores (tcgen05, TMEM accumulators).
-// Reference operator: KMeans.predict (src/kmeans.cu:77-98, RAFT kmeans_predict), i.e.
-// labels[i] = first argmin_c dist(x_i, y_c) with dist = squared L2 or cosine distance.
-//
-// The n*k*d contraction S = X * Y^T is the only dense GEMM on the path, so it runs as tcgen05.mma.kind::f16 with M = 128
-// points per tile, N = all (<= 256) centres, fp32 accumulators in TMEM, operands in shared memory in the canonical
-// no-swizzle K-major layout.
-//
-//  * Accuracy.  A value is split into two f16 numbers, x = h1 + h2 + (rest below 2^-22 |x|, or 2^-25 where h2 is subnormal),
-//    and the products h1*g1 + h2*g1 + h1*g2 are obtained in ONE GEMM by concatenating along K:
-//    A' = [x1 | x2 | x1], B' = [y1 | y1 | y2] (K = 3d).  f16 has five exponent bits, so operands are scaled by powers of two
-//    first: the rows of X each by their own largest value (a common factor of a point's scores does not change its arg-max;
-//    squared L2: only rows that lie further out than the centres), the rows of Y by their norm (cosine) or by the largest
-//    norm of all (squared L2).  (Two f16 carry 22 bits where 3 x tf32 carried 21 at half the rate and twice the bytes, and
-//    3 x bf16 16, which sent several per cent of 64-dimensional points to the exact scorer.)
-//  * The whole score comes out of the GEMM.  argmin_c |y_c|^2 - 2 x.y_c = argmax_c (x.y_c - |y_c|^2 / 2): one more chunk of K
-//    carries powers of two on the point side and three f16 pieces of -|y_c|^2/2 on the centre side, so the epilogue is a pure
-//    arg-max.  A column that is padding carries -65504 in that chunk.
-//  * The epilogue reads the 128 x 256 scores with tcgen05.ld (one point per thread) and finds the best score and whether it is
-//    the only one within the error bound of the product.  A point where it is not is NOT decided here: its index is appended to
-//    a scratch list and the exact fp32 scorer (kmeans.cu) assigns it afterwards, so every label equals the label of the exact
-//    fp32 kernel.  (Squared distances of points that lie some 10^3 times further out than the centres differ by less than their
-//    own fp32 rounding; there the score, which leaves |x|^2 out, still decides, for the nearer centre.)
-//  * Overlap.  A CTA has 22 warps with fixed roles: three groups of four epilogue warps, two of four producer warps, which have their
-//    points' rows copied to shared memory ahead, split them and store them into a ring of A tiles, and two warps whose first lanes issue the
-//    MMAs, each into its pair of accumulators of 128 columns.  They meet at mbarriers only: a half of the columns is made while the epilogue
-//    reads another, and a group ends a tile while the two others read theirs.
-//    What bounds it: up to 16 dimensions the maxima (one per point and centre and direction, two cycles per three-operand instruction: ALU
-//    pipe 66 % busy) and the latency of the chain accumulator free - MMAs - accumulator full; more dimensions: the producers' chains of
-//    dependent instructions, whatever memory and the tensor pipe do (without the splitting 147 us of 2,449,029 x 32 become 110).
-//    Measured, 2,449,029 points against 256 centres, whole call (before: sixteen warps that all loaded, split, waited and searched, one barrier
-//    per tile, 3 x tf32 or 3 x bf16): 8 dimensions 154 -> 102 us, 16: 193 -> 117, 24: 228 -> 141, 32: 267 -> 154, 64: 401 -> 313; 100 centres
-//    of 8 dimensions 119 -> 77, of 64: 359 -> 217.  Two epilogue groups instead of three: 8 dimensions 107.
-//    Every wait on an mbarrier is bounded; on expiry an error code is recorded, which makes the exact scorer assign every point, no further
-//    wait is made and no copy started, and the CTA frees its TMEM at the common exit once its own copies and MMAs are complete.
+// Entry points of the tensor-core k-means assignment (the kernel: kmeans_tc.cuh).
 #include <mutex>
 
-#include "common.cuh"
+#include "kmeans_tc.cuh"
 
 namespace f2c {
 
@@ -44,584 +10,11 @@ int kmeans_assign_exact_listed(const float* x, const float* y, int64_t* labels, 
 
 namespace tc {
 
-constexpr int kTileM = 128;
-constexpr int kMaxN = 256;
-constexpr uint32_t kWaitLimit = 1u << 18, kWaitHint = 4000;  // tries, and nanoseconds that one may take: about a second
-constexpr int kEpilogueGroups = 3, kEpilogueWarps = 4 * kEpilogueGroups, kProducerWarps = 8;
-constexpr int kMmaWarp = kEpilogueWarps + kProducerWarps, kMmaWarps = 2;  // one per pair of accumulators of 128 columns
-constexpr int kThreads = 32 * (kMmaWarp + kMmaWarps);
-constexpr int kBoundRing = 8;  // tiles whose error bounds are kept; more than the A ring and the two accumulators hold together
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-// Shared-memory matrix descriptor, K-major, no swizzle: element (row r, 16-byte K chunk c) lives at
-// start + (r % 8) * 16 + (r / 8) * SBO + c * LBO.
-__device__ __forceinline__ uint64_t make_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-  uint32_t lo = ((addr & 0x3FFFFu) >> 4) | ((lbo >> 4) << 16);
-  uint32_t hi = (sbo >> 4) | (1u << 14);  // bits 46-47: descriptor version 1 (sm_100); layout type 0 = no swizzle
-  return ((uint64_t)hi << 32) | lo;
-}
-
-__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t"
-      "}\n" ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
-      : "memory");
-}
-
-__device__ __forceinline__ void mma_commit(uint32_t mbar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
-}
-
-__device__ __forceinline__ void mbar_init(uint32_t mbar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
-  asm volatile("{\n\t.reg .b64 s;\n\tmbarrier.arrive.shared::cta.b64 s, [%0];\n\t}" ::"r"(mbar) : "memory");
-}
-
-// A role's waits.  One that runs out is reported (code = 1 + tiles done) and no later one waits.
-struct Waiter {
-  int32_t* error;
-  bool gave_up;
-  __device__ __forceinline__ bool operator()(uint32_t mbar, uint32_t parity, int code) {
-    if (gave_up) return false;
-    for (uint32_t it = 0; it < kWaitLimit; ++it) {
-      uint32_t done;
-      asm volatile(
-          "{\n\t.reg .pred p;\n\t"
-          "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-          "selp.u32 %0, 1, 0, p;\n\t}\n"
-          : "=r"(done) : "r"(mbar), "r"(parity), "r"(kWaitHint) : "memory");
-      if (done) return true;
-    }
-    gave_up = true;
-    atomicExch(error, code);
-    return false;
-  }
-};
-
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-}
-
-// The loads issued so far are complete; naming the registers keeps their uses behind the wait.
-__device__ __forceinline__ void tmem_wait(uint32_t (&r)[16]) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]),
-                 "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])::"memory");
-}
-
-struct Params {
-  const float* x;
-  const float* y;
-  int64_t* labels;
-  int32_t* amb_list;   // scratch: indices of undecided points
-  int32_t* amb_count;  // scratch: their number
-  int32_t* error;      // scratch: non-zero when a bounded wait expired
-  int64_t n;
-  int k, d;
-  int metric;
-  int x_aligned;       // x starts on a 16-byte boundary
-  int x_wide, y_wide;  // rows can be read as float4
-  float eps;   // relative error bound of one score
-  const int32_t* done;  // when set and non-zero: nothing to do (a fit that has converged, kmeans_fit.cu)
-};
-
-__device__ __forceinline__ float max3(float a, float b, float c) {
-  float r;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
-}
-
-__device__ __forceinline__ float sqrt_approx(float v) {
-  float r;
-  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(v));
-  return r;
-}
-__device__ __forceinline__ void add_if_ge(int& sum, float a, float b, int add) {
-  asm("{\n\t.reg .pred q;\n\tsetp.ge.f32 q, %1, %2;\n\t@q add.s32 %0, %0, %3;\n\t}" : "+r"(sum) : "f"(a), "f"(b), "r"(add));
-}
-
-__device__ __forceinline__ float power2f(int e) { return __int_as_float((127 + e) << 23); }  // -127 < e < 128
-// |v| < 2^e for the largest such v; 0 for v = 0 and for what is not finite
-__device__ __forceinline__ int exponent_above(float v) {
-  const int b = (int)((__float_as_uint(v) & 0x7fffffffu) >> 23);
-  return b == 0 || b == 255 ? 0 : b - 126;
-}
-
-// v = c1 + c2 + rest: eight values -> two 16-byte chunks of f16
-__device__ __forceinline__ void split8(const float (&v)[8], uint4& c1, uint4& c2) {
-  uint32_t w1[4], w2[4];
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const __half2 a = __floats2half2_rn(v[2 * e], v[2 * e + 1]);
-    const float2 f = __half22float2(a);
-    const __half2 b = __floats2half2_rn(v[2 * e] - f.x, v[2 * e + 1] - f.y);
-    w1[e] = *reinterpret_cast<const uint32_t*>(&a);
-    w2[e] = *reinterpret_cast<const uint32_t*>(&b);
-  }
-  c1 = make_uint4(w1[0], w1[1], w1[2], w1[3]);
-  c2 = make_uint4(w2[0], w2[1], w2[2], w2[3]);
-}
-
-// Eight values of a row from column t on; zeros behind its end and where !on.
-__device__ __forceinline__ void load8(const float* __restrict__ row, int t, int d, bool wide, bool on, float (&v)[8]) {
-  if (wide) {  // d % 4 == 0
-    const uint4 a = ldg_u128_if(row + t, on && t < d), b = ldg_u128_if(row + t + 4, on && t + 4 < d);
-    v[0] = __uint_as_float(a.x); v[1] = __uint_as_float(a.y); v[2] = __uint_as_float(a.z); v[3] = __uint_as_float(a.w);
-    v[4] = __uint_as_float(b.x); v[5] = __uint_as_float(b.y); v[6] = __uint_as_float(b.z); v[7] = __uint_as_float(b.w);
-  } else {
-#pragma unroll
-    for (int e = 0; e < 8; ++e) v[e] = on && t + e < d ? __ldg(row + t + e) : 0.0f;
-  }
-}
-
-// How a warp reads rows of C chunks of eight columns: lane = (row of R, chunk of CL), chunk fastest.  PAD bytes between the operands'
-// chunks make the eight lanes of a 16-byte store touch eight bank groups.
-template <int C>
-struct Lanes {
-  static constexpr int CL = C <= 2 ? C : C <= 4 ? 4 : 8;  // lanes per row
-  static constexpr int R = 32 / CL;                       // rows of one read
-  static constexpr int PAD = CL == 1 ? 0 : 128 / CL;
-  // A producer warp's rows of a tile come in PARTS of ROWS rows, one bulk copy each.
-  static constexpr int ROWS = C <= 4 ? 32 : 16, PARTS = 32 / ROWS, READS = ROWS / R;
-  static constexpr int PART_BYTES = ROWS * C * 32;
-};
-
-// Which 16-byte chunks the operands of the concatenated GEMM take.  Along K: [x1 | x2 | x1 | norm] against [y1 | y1 | y2 | norm], C
-// chunks each and one (C even: two, the second zero) for the norm; one MMA takes two neighbours of that sequence, whose distance
-// in shared memory a descriptor states.  So x1 is stored once, and y1 where no pair starts in one copy of it and ends in the next.
-template <int C>
-struct Operands {
-  static constexpr int steps = (3 * C + 2) / 2;
-  static constexpr int zero = C % 2 == 0 ? 1 : 0;  // a zero chunk behind the norm chunk
-  static constexpr int a_chunks = 2 * C + 1 + zero, b_chunks = C % 2 == 0 ? 2 * C + 2 : 3 * C + 1;
-  static constexpr int a_norm = 2 * C, b_norm = C % 2 == 0 ? 2 * C : 3 * C, b_low = C % 2 == 0 ? C : 2 * C;  // where norm and y2 start
-  static constexpr int a(int q) { return q < 2 * C ? q : q < 3 * C ? q - 2 * C : q - C; }
-  static constexpr int b(int q) { return C % 2 != 0 || q < C ? q : q - C; }
-};
-
-// What shared memory holds: A tiles in the ring, and parts of rows in flight per producer warp: 32 to 64 KB per SM (the DRAM's latency
-// holds about 35 at its full rate).  Tiles go to two producer groups and two MMA threads in turn, so with an odd number of stages a stage
-// changes hands; its barriers, of which each side has to see every phase, are then those of t % (2 * stages).
-template <int C, int NB>
-struct Ring {
-  static constexpr int stages = C >= 7 && NB == 8 ? 3 : 4, turns = stages % 2 ? 2 * stages : stages;
-  static constexpr int slots = C == 1 ? 8 : C == 2 ? 4 : C >= 7 ? 1 : 2;
-  static constexpr size_t bytes = (size_t)Operands<C>::b_chunks * (NB * 512 + Lanes<C>::PAD) + (size_t)Operands<C>::a_chunks * stages * (kTileM * 16 + Lanes<C>::PAD) +
-                                  (size_t)kProducerWarps * slots * Lanes<C>::PART_BYTES + kMaxN * 4 + kBoundRing * kTileM * 4 +
-                                  8 * (2 * turns + 4 * kEpilogueGroups + 6 + kProducerWarps * slots) + 16;
-  static_assert(bytes <= 227 * 1024, "shared memory of a CTA");
-};
-
-// Shared memory: [B tile][A ring][rows in flight][norms 256 floats][bounds kBoundRing x 128 floats][mbarriers, tmem slot]
-// C: chunks of eight dimensions of a row (1 to 8); NB: blocks of 32 columns (4: up to 128 centres, 8: up to 256).
 template <int C, int NB>
 __global__ void __launch_bounds__(kThreads, 1) kmeans_tc_kernel(const Params p) {
-  using L = Lanes<C>;
-  using O = Operands<C>;
-  using Q = Ring<C, NB>;
-  constexpr int N = 32 * NB;
-  constexpr uint32_t lbo_b = N * 16 + L::PAD, lbo_a = kTileM * 16 + L::PAD, sbo = 128;
   dependency_wait();  // first of all: the kernel launched behind this one relies on it (y_settled below)
   release_dependents();
-  extern __shared__ __align__(128) unsigned char smem[];
-  if (p.done != nullptr && *(volatile const int32_t*)p.done != 0) return;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  constexpr uint32_t a_bytes = O::a_chunks * lbo_a;
-  unsigned char* b_tile = smem;
-  unsigned char* a_ring = smem + O::b_chunks * lbo_b;
-  unsigned char* rows = a_ring + Q::stages * a_bytes;
-  float* norms = reinterpret_cast<float*>(rows + kProducerWarps * Q::slots * L::PART_BYTES);
-  float* bounds = norms + kMaxN;
-  uint64_t* mbars = reinterpret_cast<uint64_t*>(bounds + kBoundRing * kTileM);
-  // a_full[turns], a_free[turns], acc_full[kFull][HALVES], acc_free[4], drained[2], row_full[producer warp][slots].  A wait names the parity of a
-  // phase only, so whoever waits has to have seen the phase before, and the next one must not end before it has looked.  That an accumulator
-  // has become full is therefore a matter of its tile, t % kFull, where t + kFull has the same accumulator and the same epilogue group: its
-  // MMAs wait for those of all tiles between that have this accumulator, t among them, to have been read.
-  constexpr int HALVES = NB / 4, kFull = 4 * kEpilogueGroups / HALVES;
-  const uint32_t a_full = smem_u32(mbars), a_free = a_full + 8 * Q::turns, acc_full = a_free + 8 * Q::turns, acc_free = acc_full + 8 * kFull * HALVES,
-                 drained = acc_free + 32, row_full = drained + 16;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mbars + 2 * Q::turns + 6 + kFull * HALVES + kProducerWarps * Q::slots);
-
-  const int64_t n_tiles = (p.n + kTileM - 1) / kTileM;
-  const int turns = (int)((n_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x);  // tiles of this CTA: blockIdx.x + t * gridDim.x
-  Waiter wait{p.error, false};
-
-  const int group = warp >= kEpilogueWarps ? (warp - kEpilogueWarps) >> 2 : warp >> 2;
-  const int row_l = lane / L::CL, chunk_l = lane % L::CL;
-  const bool producer = warp >= kEpilogueWarps && warp < kMmaWarp;
-  const int own = producer ? warp - kEpilogueWarps : 0;
-  unsigned char* own_rows = rows + own * (Q::slots * L::PART_BYTES);
-  const uint32_t own_full = row_full + (uint32_t)own * (8 * Q::slots);
-  // rows of part q of this warp's share of tile t: how many there are, and whether one bulk copy fetches them
-  auto part_base = [&](int t, int q) { return ((int64_t)blockIdx.x + (int64_t)t * gridDim.x) * kTileM + (warp & 3) * 32 + q * L::ROWS; };
-  auto part_bulk = [&](int64_t base) { return p.x_aligned && base + L::ROWS <= p.n; };
-  uint32_t fetched = 0;  // lane 0: bit s, slot s has had a bulk copy; bit 8 + s, the parity of its last one's phase
-  auto fetch = [&](int t, int q, int slot) {
-    if (t < turns && !wait.gave_up) {
-      const int64_t base = part_base(t, q);
-      const float* src = p.x + base * p.d;
-      const uint32_t dst = smem_u32(own_rows + slot * L::PART_BYTES);
-      if (part_bulk(base)) {
-        if (lane == 0) {
-          fetched = (fetched ^ (((fetched >> slot) & 1u) << (8 + slot))) | (1u << slot);
-          const uint32_t bytes = (uint32_t)(L::ROWS * 4 * p.d), full = own_full + 8u * slot;
-          asm volatile("{\n\t.reg .b64 s;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 s, [%0], %1;\n\t}" ::"r"(full), "r"(bytes) : "memory");
-          asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(full)
-                       : "memory");
-        }
-      } else {  // the last rows of x, or an x that starts off a 16-byte boundary
-        const int some = (int)max((int64_t)0, min((int64_t)L::ROWS, p.n - base)) * p.d;
-        for (int e = lane; e < some; e += 32) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + 4u * e), "l"(src + e) : "memory");
-      }
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-
-  // ---- one-time setup: mbarriers, TMEM (all 512 columns), centre tile ----
-  if (threadIdx.x == 32 * kMmaWarp) {
-    for (int s = 0; s < Q::turns; ++s) { mbar_init(a_full + 8 * s, 4); mbar_init(a_free + 8 * s, 1); }
-    for (int u = 0; u < kFull * HALVES; ++u) mbar_init(acc_full + 8 * u, 1);
-    for (int u = 0; u < 4; ++u) mbar_init(acc_free + 8 * u, 4);
-    for (int g = 0; g < 2; ++g) mbar_init(drained + 8 * g, 1);
-    for (int u = 0; u < kProducerWarps * Q::slots; ++u) mbar_init(row_full + 8 * u, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
-  if (warp == kMmaWarp) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  if (producer) {  // the first rows, on their way while the centres are staged
-#pragma unroll
-    for (int u = 0; u < Q::slots; ++u) fetch(group + 2 * (u / L::PARTS), u % L::PARTS, u);
-  }
-  constexpr int kStagers = 8;
-  constexpr int STEPS = (N / kStagers + L::R - 1) / L::R;  // reads that make a warp's share of the centres
-  static_assert(N / kStagers % L::R == 0 || STEPS == 1, "shares of whole reads");
-  const int c0 = warp * (STEPS * L::R);  // C = 1: the first N / 32 warps have 32 centres each
-  constexpr bool KEEP = STEPS <= 4;  // in registers between the two passes; more than 32 dimensions are read twice
-  float yv[KEEP ? STEPS : 1][8];
-  auto load_centres = [&](int s, float (&v)[8]) {
-    const int c = c0 + s * L::R + row_l;
-    load8(p.y + (int64_t)c * p.d, 8 * chunk_l, p.d, p.y_wide, c < p.k, v);
-  };
-  if (warp < kStagers) {
-    if constexpr (KEEP) {
-#pragma unroll
-      for (int s = 0; s < STEPS; ++s) load_centres(s, yv[s]);
-    }
-#pragma unroll
-    for (int s = 0; s < STEPS; ++s) {
-      float (&v)[8] = yv[KEEP ? s : 0];
-      if constexpr (!KEEP) load_centres(s, v);
-      float nrm = 0.0f;
-#pragma unroll
-      for (int e = 0; e < 8; ++e) nrm = fmaf(v[e], v[e], nrm);
-#pragma unroll
-      for (int o = 1; o < L::CL; o <<= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
-      if (chunk_l == 0 && c0 + s * L::R + row_l < kMaxN) norms[c0 + s * L::R + row_l] = nrm;
-    }
-  }
-  __syncthreads();
-  // largest centre norm (scale and tolerance of the L2 score); a non-finite centre sends every point to the exact scorer
-  float cmax = 0.0f, poison = 0.0f;
-#pragma unroll
-  for (int c = lane; c < N; c += 32) { cmax = fmaxf(cmax, norms[c]); poison = fmaf(norms[c], 0.0f, poison); }  // inf, NaN -> NaN
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    cmax = fmaxf(cmax, __shfl_xor_sync(0xffffffffu, cmax, o));
-    poison += __shfl_xor_sync(0xffffffffu, poison, o);
-  }
-  const bool bad_centres = !(poison == 0.0f);
-  const bool l2 = p.metric == F2C_L2;
-  const int e_y = l2 ? max(-120, min(120, exponent_above(sqrtf(cmax)))) : 0;  // squared L2: everything times 2^-e_y
-  const float scale_y = power2f(-e_y);
-  cmax = l2 ? sqrtf(cmax) * scale_y : 1.0f;
-  if (warp < kStagers) {
-#pragma unroll
-    for (int s = 0; s < STEPS; ++s) {
-      const int c = c0 + s * L::R + row_l;
-      float (&v)[8] = yv[KEEP ? s : 0];
-      if constexpr (!KEEP) load_centres(s, v);
-      if (c < N) {
-        const float nrm = norms[c];
-        // cosine: rows of unit length (zero rows stay zero)
-        const float f = l2 ? scale_y : (nrm > 0.0f ? 1.0f / sqrtf(nrm) : 0.0f);
-        float own_sq = 0.0f;  // squared length of the scaled row, which the norm term takes: |y|^2 itself may overflow
-#pragma unroll
-        for (int e = 0; e < 8; ++e) { v[e] *= f; own_sq = fmaf(v[e], v[e], own_sq); }
-        if (C == L::CL || chunk_l < C) {
-          uint4 c1, c2;
-          split8(v, c1, c2);
-          *reinterpret_cast<uint4*>(b_tile + (size_t)chunk_l * lbo_b + c * 16) = c1;
-          if (O::b_low > C) *reinterpret_cast<uint4*>(b_tile + (size_t)(C + chunk_l) * lbo_b + c * 16) = c1;
-          *reinterpret_cast<uint4*>(b_tile + (size_t)(O::b_low + chunk_l) * lbo_b + c * 16) = c2;
-        }
-#pragma unroll
-        for (int o = 1; o < L::CL; o <<= 1) own_sq += __shfl_xor_sync(0xffffffffu, own_sq, o);
-        if (chunk_l == 0) {
-          const float h = l2 && c < p.k ? -0.5f * own_sq : 0.0f;
-          const __half h1 = __float2half_rn(h), h2 = __float2half_rn(h - __half2float(h1));
-          const __half h3 = __float2half_rn(h - __half2float(h1) - __half2float(h2));
-          const __half never = __float2half_rn(c < p.k ? 0.0f : -65504.0f);
-          *reinterpret_cast<uint4*>(b_tile + (size_t)O::b_norm * lbo_b + c * 16) =
-              make_uint4((uint32_t)__half_as_ushort(h1) | ((uint32_t)__half_as_ushort(h2) << 16),
-                         (uint32_t)__half_as_ushort(h3) | ((uint32_t)__half_as_ushort(never) << 16), 0u, 0u);
-          if (O::zero) *reinterpret_cast<uint4*>(b_tile + (size_t)(O::b_norm + 1) * lbo_b + c * 16) = make_uint4(0u, 0u, 0u, 0u);
-        }
-      }
-    }
-  } else if (producer) {
-    // what the norm chunk holds in every A tile (cosine: a one against the padding's number), and the zeros behind it
-    for (int i = threadIdx.x - 32 * kEpilogueWarps; i < Q::stages * kTileM; i += 32 * kProducerWarps) {
-      unsigned char* at = a_ring + (size_t)(i / kTileM) * a_bytes + (size_t)O::a_norm * lbo_a + i % kTileM * 16;
-      *reinterpret_cast<uint4*>(at) = make_uint4(0u, 0x3C000000u, 0u, 0u);
-      if (O::zero) *reinterpret_cast<uint4*>(at + lbo_a) = make_uint4(0u, 0u, 0u, 0u);
-    }
-  }
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem_base = *tmem_slot;
-  // Tile t's columns 128 h .. 128 h + 127 are in accumulator (t, h) of four.
-  auto accumulator = [](int t, int h) { return 2 * (t & 1) + (NB == 8 ? h : (t >> 1) & 1); };
-
-  if (producer) {
-    const float eps = 2.0f * cmax * (bad_centres ? INFINITY : p.eps);  // what two scores may be off by together, per |x|
-    int unit = 0;
-    for (int t = group; t < turns; t += 2) {
-      unsigned char* a_tile = a_ring + (size_t)(t % Q::stages) * a_bytes;
-      if (t >= Q::stages) wait(a_free + 8 * ((t - Q::stages) % Q::turns), (uint32_t)((t - Q::stages) / Q::turns) & 1u, 1 + t);
-#pragma unroll
-      for (int q = 0; q < L::PARTS; ++q, ++unit) {
-        const int slot = unit % Q::slots;
-        asm volatile("cp.async.wait_group %0;" ::"n"(Q::slots - 1) : "memory");
-        if (part_bulk(part_base(t, q))) wait(own_full + 8 * slot, (uint32_t)(unit / Q::slots) & 1u, 1 + t);
-        __syncwarp();
-        // The reads go through every step side by side: their chains of dependent instructions are what a lone warp waits for.
-        float v[L::READS][8], top[L::READS], sum[L::READS], factor[L::READS];
-#pragma unroll
-        for (int b = 0; b < L::READS; ++b) {
-          const float* row = reinterpret_cast<const float*>(own_rows + slot * L::PART_BYTES) + (b * L::R + row_l) * p.d + 8 * chunk_l;
-          if (p.x_wide) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              float4 w = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-              if (8 * chunk_l + 4 * h < p.d) w = *reinterpret_cast<const float4*>(row + 4 * h);
-              v[b][4 * h] = w.x; v[b][4 * h + 1] = w.y; v[b][4 * h + 2] = w.z; v[b][4 * h + 3] = w.w;
-            }
-          } else {
-#pragma unroll
-            for (int e = 0; e < 8; ++e) v[b][e] = 8 * chunk_l + e < p.d ? row[e] : 0.0f;
-          }
-        }
-        float any = 0.0f;
-#pragma unroll
-        for (int b = 0; b < L::READS; ++b) {
-          top[b] = max3(max3(fabsf(v[b][0]), fabsf(v[b][1]), fabsf(v[b][2])), max3(fabsf(v[b][3]), fabsf(v[b][4]), fabsf(v[b][5])),
-                        fmaxf(fabsf(v[b][6]), fabsf(v[b][7])));
-          any = fmaxf(any, top[b]);
-        }
-        // The slot's next copy may start when all lanes' reads have arrived, not merely been issued: the vote waits for what was read (it is always
-        // true; a barrier of the warp in its place let rows be overwritten before they were read).
-        if (__any_sync(0xffffffffu, !(any < 0.0f))) fetch(t + 2 * ((q + Q::slots) / L::PARTS), (q + Q::slots) % L::PARTS, slot);
-        if (l2) {
-#pragma unroll
-          for (int b = 0; b < L::READS; ++b) {
-            top[b] *= scale_y;
-#pragma unroll
-            for (int e = 0; e < 8; ++e) v[b][e] *= scale_y;
-          }
-        }
-#pragma unroll
-        for (int b = 0; b < L::READS; ++b) {
-#pragma unroll
-          for (int o = 1; o < L::CL; o <<= 1) top[b] = fmaxf(top[b], __shfl_xor_sync(0xffffffffu, top[b], o));
-          // |v| < 2^ex.  Squared L2: among the centres the factor stays that of the centres, so that the norm term is not scaled up
-          const int biased = min(max(__float_as_int(top[b]) & 0x7f800000, l2 ? 126 << 23 : 0), 252 << 23);
-          factor[b] = __int_as_float((253 << 23) - biased);  // 2^-ex, ex = biased - 126
-        }
-#pragma unroll
-        for (int b = 0; b < L::READS; ++b) {
-          unsigned char* at = a_tile + (size_t)chunk_l * lbo_a + ((warp & 3) * 32 + q * L::ROWS + b * L::R + row_l) * 16;
-          float even = 0.0f, odd = 0.0f;
-#pragma unroll
-          for (int e = 0; e < 8; e += 2) {
-            v[b][e] *= factor[b]; v[b][e + 1] *= factor[b];
-            even = fmaf(v[b][e], v[b][e], even); odd = fmaf(v[b][e + 1], v[b][e + 1], odd);
-          }
-          sum[b] = even + odd;
-          uint4 c1, c2;
-          split8(v[b], c1, c2);
-          if (C == L::CL || chunk_l < C) {
-            *reinterpret_cast<uint4*>(at) = c1;
-            *reinterpret_cast<uint4*>(at + C * lbo_a) = c2;
-          }
-        }
-#pragma unroll
-        for (int b = 0; b < L::READS; ++b)
-#pragma unroll
-          for (int o = 1; o < L::CL; o <<= 1) sum[b] += __shfl_xor_sync(0xffffffffu, sum[b], o);
-        // one lane per row: its error bound, and (squared L2) its part of the norm term: powers of two against the pieces of -|y|^2 / 2 (0 for a
-        // point so far out that its own is no f16: the term is below the bound there), a one against the padding's
-        float own_sum = sum[0], own_factor = factor[0];
-#pragma unroll
-        for (int b = 1; b < L::READS; ++b)
-          if (chunk_l == b) { own_sum = sum[b]; own_factor = factor[b]; }
-        const int row = (warp & 3) * 32 + q * L::ROWS + chunk_l * L::R + row_l;
-        const float floor = 2.0f * cmax * (l2 ? fmaxf(0x1p-19f * own_factor, 0x1p-126f) : 0x1p-21f);  // f16 at its lower end, and the norm term
-        const float unscale = __int_as_float((254 << 23) - __float_as_int(own_factor)) * power2f(e_y);  // 1 / all that x was multiplied with
-        // INFINITY for NaN, and for a point whose |x|^2 is more than fp32 holds: the exact scorer's distance says so
-        const float bound = own_sum * unscale * unscale < INFINITY ? fminf(fmaf(eps, sqrt_approx(own_sum), floor), INFINITY) : INFINITY;
-        if (chunk_l < L::READS) {
-          bounds[(t & (kBoundRing - 1)) * kTileM + row] = bound;
-          if (l2) {
-            const uint32_t one = (uint32_t)__half_as_ushort(__float2half_rn(own_factor));
-            *reinterpret_cast<uint4*>(a_tile + (size_t)O::a_norm * lbo_a + row * 16) = make_uint4(one | (one << 16), one | 0x3C000000u, 0u, 0u);
-          }
-        }
-      }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) mbar_arrive(a_full + 8 * (t % Q::turns));
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    if (wait.gave_up && lane == 0) {  // copies that have not been waited for: one per slot at most, since nothing was fetched after that wait
-      Waiter last{p.error, false};
-      for (int slot = 0; slot < Q::slots; ++slot)
-        if ((fetched >> slot) & 1u) last(own_full + 8 * slot, (fetched >> (8 + slot)) & 1u, 1 + turns);
-    }
-    __syncwarp();
-  } else if (warp >= kMmaWarp) {
-    // One thread per pair of accumulators, with nothing but constants to add: its instructions follow one another at their full latency (one
-    // thread for both, descriptors made in the loop: 740 cycles a tile, more than the epilogue takes; a thread for each of the four: the
-    // same at 8 dimensions and 24 us slower at 2,449,029 x 32, whose MMAs then get in each other's way).
-    if (lane == 0) {
-      // instruction descriptor: fp32 accumulate; A and B f16 (0); 128 columns; M / 16
-      constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
-      const int g = warp - kMmaWarp;
-      const uint64_t b_base = make_desc(smem_u32(b_tile), 0, sbo);
-      bool on = true;
-      for (int t = g; t < turns && on; t += 2) {
-        const uint64_t a_base = make_desc(smem_u32(a_ring) + (uint32_t)(t % Q::stages) * a_bytes, 0, sbo);
-        on = wait(a_full + 8 * (t % Q::turns), (uint32_t)(t / Q::turns) & 1u, 1 + t);
-#pragma unroll
-        for (int h = 0; h < HALVES; ++h) {  // the epilogue reads one half of the columns while the other is made
-          const int a = accumulator(t, h);
-          on = on && wait(acc_free + 8 * a, ((uint32_t)(t >> (NB == 8 ? 1 : 2)) & 1u) ^ 1u, 1 + t);
-          if (!on) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-          for (int s = 0; s < O::steps; ++s) {  // one MMA consumes 16 f16 = two 16-byte chunks of K
-            constexpr auto part = [](int first, int second, uint32_t lbo) { return (uint64_t)((uint32_t)first * lbo >> 4) | (uint64_t)((uint32_t)(second - first) * lbo >> 4) << 16; };
-            mma_f16(tmem_base + (uint32_t)a * 128u, a_base + part(O::a(2 * s), O::a(2 * s + 1), lbo_a),
-                    b_base + part(O::b(2 * s), O::b(2 * s + 1), lbo_b) + (uint64_t)(h * 128), idesc, s > 0 ? 1u : 0u);
-          }
-          mma_commit(acc_full + 8 * (HALVES * (t % kFull) + h));
-        }
-        if (on) mma_commit(a_free + 8 * (t % Q::turns));
-      }
-      mma_commit(drained + 8 * g);  // after a wait that ran out nobody else has waited for the MMAs in flight
-      Waiter last{p.error, false};
-      last(drained + 8 * g, 0u, 1 + turns);
-    }
-    __syncwarp();
-  } else {
-    // ---- epilogue: TMEM lane pt = point; its thread scans all centres ----
-    // Maxima only, one three-operand max per score: of the 16-column groups (row_max) and of the columns with the same number in
-    // their group (col_max).  Scores within the bound of the best lie in the crossings of the groups and columns whose maximum does,
-    // so the best centre is decided exactly when that is one group and one column - at the crossing.  (A running best, second
-    // best and index took five compare instructions per score, which issue at half rate.)
-    const int pt = (warp & 3) * 32 + lane;
-    const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
-    constexpr int kGroups = 2 * NB;
-    uint32_t turn = 0;  // which of this group's tiles
-    for (int t = group; t < turns; t += kEpilogueGroups, ++turn) {
-      float row_max[kGroups], col_max[16], bound = 0.0f;
-      uint32_t ra[16], rb[16];  // two 16-column loads alternate: one is consumed while the other is in flight
-      auto group_max = [&](const uint32_t (&r)[16]) {
-        auto f = [&](int j) { return __uint_as_float(r[j]); };
-        const float m0 = max3(f(0), f(1), f(2)), m1 = max3(f(3), f(4), f(5)), m2 = max3(f(6), f(7), f(8)), m3 = max3(f(9), f(10), f(11));
-        const float m4 = max3(f(12), f(13), f(14));
-        return fmaxf(max3(m0, m1, m2), max3(m3, m4, f(15)));
-      };
-#pragma unroll
-      for (int h = 0; h < HALVES; ++h) {
-        constexpr uint32_t laps = kFull / kEpilogueGroups;  // barriers that this group uses in turn
-        const int a = accumulator(t, h);
-        wait(acc_full + 8 * (HALVES * (group + kEpilogueGroups * (turn % laps)) + h), (turn / laps) & 1u, 1 + t);
-        __syncwarp();
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (h == 0) bound = bounds[(t & (kBoundRing - 1)) * kTileM + pt];  // before acc_free: a later tile's takes its place
-        const uint32_t addr = lane_addr + (uint32_t)a * 128u;
-        tmem_ld16(addr, ra);
-#pragma unroll
-        for (int q = 0; q < 8; q += 2) {
-          tmem_wait(ra);
-          tmem_ld16(addr + (uint32_t)(16 * q + 16), rb);
-          row_max[8 * h + q] = group_max(ra);
-          float own[16];
-#pragma unroll
-          for (int j = 0; j < 16; ++j) own[j] = __uint_as_float(ra[j]);
-          tmem_wait(rb);
-          if (q + 2 < 8) {
-            tmem_ld16(addr + (uint32_t)(16 * q + 32), ra);
-          } else {  // the next MMAs may overwrite the accumulator
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(acc_free + 8 * a);
-          }
-          row_max[8 * h + q + 1] = group_max(rb);
-#pragma unroll
-          for (int j = 0; j < 16; ++j)
-            col_max[j] = h == 0 && q == 0 ? fmaxf(own[j], __uint_as_float(rb[j])) : max3(col_max[j], own[j], __uint_as_float(rb[j]));
-        }
-      }
-      float best = row_max[0];
-#pragma unroll
-      for (int q = 1; q + 1 < kGroups; q += 2) best = max3(best, row_max[q], row_max[q + 1]);
-      best = fmaxf(best, row_max[kGroups - 1]);
-      // hits, each counted as 64 + its number: from 64 to 127 there was one
-      const float from = best - bound;
-      int rows_hit[2] = {0, 0}, cols_hit[2] = {0, 0};
-#pragma unroll
-      for (int q = 0; q < kGroups; ++q) add_if_ge(rows_hit[q & 1], row_max[q], from, 64 + q);
-#pragma unroll
-      for (int j = 0; j < 16; ++j) add_if_ge(cols_hit[j & 1], col_max[j], from, 64 + j);
-      const int r_hit = rows_hit[0] + rows_hit[1], c_hit = cols_hit[0] + cols_hit[1];
-      const int centre = 16 * r_hit + c_hit - (16 * 64 + 64);
-      const bool decided = (r_hit >> 6) == 1 && (c_hit >> 6) == 1 && best > -INFINITY;
-      const int64_t i = ((int64_t)blockIdx.x + (int64_t)t * gridDim.x) * kTileM + pt;
-      const bool undecided = i < p.n && !decided;
-      const uint32_t listed = __ballot_sync(0xffffffffu, undecided);  // the exact scorer assigns them afterwards
-      if (listed != 0u) {
-        int slot = 0;
-        if (lane == 0) slot = atomicAdd(p.amb_count, __popc(listed));
-        slot = __shfl_sync(0xffffffffu, slot, 0);
-        if (undecided) p.amb_list[slot + __popc(listed & ((1u << lane) - 1u))] = (int32_t)i;
-      }
-      if (i < p.n && decided) p.labels[i] = centre;
-    }
-  }
-
-  // ---- common exit: all TMEM reads retired, then the allocating warp frees the columns ----
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  if (warp == kMmaWarp) {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
-  }
+  run<C, NB>(p);
 }
 
 struct Kernel {
@@ -652,21 +45,16 @@ bool kmeans_tc_supported(int64_t n, int64_t k, int64_t d) { return n >= 1 && n <
 int64_t kmeans_tc_workspace(int64_t n) { return 256 + 4 * n; }  // [count, error, pad][index list]
 
 int kmeans_assign_tc(const float* x, const float* y, int64_t* labels, int64_t n, int64_t k, int64_t d, int metric, void* workspace,
-                     cudaStream_t st, const int32_t* done, bool head_is_clear) {
+                     cudaStream_t st) {
   tc::Params p{};
-  p.done = done;
-  p.x = x; p.y = y; p.labels = labels; p.n = n; p.k = (int)k; p.d = (int)d; p.metric = metric;
-  p.x_aligned = aligned(x, 16);
-  p.x_wide = d % 4 == 0;  // of the copy in shared memory
-  p.y_wide = d % 4 == 0 && aligned(y, 16);
-  // relative error bound of one score: the split leaves 3 * 2^-22 of |x||y|, the rest is the sums of up to 13 MMAs of 16 products
-  p.eps = d <= 32 ? 1.0f / 65536.0f : 1.0f / 32768.0f;
+  tc::describe(p, x, y, n, k, d, metric);
+  p.labels = labels;
   int32_t* head = reinterpret_cast<int32_t*>(workspace);
   p.amb_count = head; p.error = head + 1; p.amb_list = head + 64;
-  cudaError_t e = head_is_clear ? cudaSuccess : cudaMemsetAsync(head, 0, 256, st);
+  cudaError_t e = cudaMemsetAsync(head, 0, 256, st);
   if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "kmeans_assign: %s", cudaGetErrorString(e));
   auto [kern, smem] = tc::kernel_for(k, d);
-  if (smem < 120 * 1024) smem = 120 * 1024;  // one CTA per SM: a second one would only wait for the TMEM columns
+  if (smem < tc::kOneCta) smem = tc::kOneCta;
   e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "kmeans_assign: %s", cudaGetErrorString(e));
   int64_t grid = ceil_div(n, tc::kTileM);
@@ -737,7 +125,7 @@ extern "C" int f2c_kmeans_assign_static(const float* x, const float* centers, in
   int rc = tc::static_scratch(op, &scratch);
   if (rc) return rc;
   // same kernels as kmeans_assign; the header (count, error code) is cleared inside
-  return kmeans_assign_tc(x, centers, labels, n, k, d, metric, scratch, (cudaStream_t)stream, nullptr, false);
+  return kmeans_assign_tc(x, centers, labels, n, k, d, metric, scratch, (cudaStream_t)stream);
 }
 
 // What the last f2c_kmeans_assign_static call on the current device left in the header of the built-in array: the

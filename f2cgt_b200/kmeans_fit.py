@@ -36,7 +36,7 @@ def _init_kmeanspp(x, k, gen):
     return centers
 
 
-_AHEAD = 8  # iterations queued between two looks at the convergence flag (those behind the converged one cost a few empty launches)
+_AHEAD = 16  # iterations queued between two looks at the convergence flag (those behind the converged one do nothing)
 
 
 def _iterate(x, centers, metric, max_iter, tol):

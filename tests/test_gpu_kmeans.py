@@ -223,3 +223,26 @@ def test_tensor_core_assignment_at_the_edges_of_its_tiles(capi, d):
                 exact = ops.kmeans_assign(y, c, metric, scorer="exact")
                 for _ in range(3):
                     assert torch.equal(ops.kmeans_assign(y, c, metric, scorer="tensor"), exact), (n, k, metric, size)
+
+
+@pytest.mark.parametrize("n,k,d", [(1, 1, 4), (127, 128, 8), (1025, 129, 24), (70_000, 256, 13), (200_003, 33, 64), (40_000, 200, 40)])
+def test_fit_kernel_at_the_edges_of_its_tiles(capi, n, k, d):
+    """Ragged tiles, one to many chunks of points per CTA, many points that the tensor cores leave open (every second centre is a copy,
+    a third of the rows is zero), rows off a 16-byte boundary: the centres of a loop over the exact assignment with float64 sums."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn(n * d + 1, generator=g, device="cuda")[1:].view(n, d)
+    x[::3] = 0
+    start = torch.randn(k, d, generator=g, device="cuda")
+    start[1::2] = start[:k - k % 2:2]
+    from f2cgt_b200 import ops
+    for metric in ("l2", "cosine"):
+        want = start.clone()
+        for _ in range(3):
+            labels = ops.kmeans_assign(x.contiguous(), want, metric, scorer="exact")
+            sums = torch.zeros(k, d, dtype=torch.float64, device="cuda").index_add_(0, labels, x.double())
+            cnt = torch.bincount(labels, minlength=k).unsqueeze(1)
+            want = torch.where(cnt > 0, sums.float() / cnt.clamp_min(1), want)
+        km = capi.KMeans(start.clone(), metric, max_iter=3, tol=-1.0)
+        km.fit(x)
+        # fixed-point sums are exact, float64 ones to 2^-53 of the largest partial sum: both round to the same float32 but for its last bit
+        assert float((km.get_centers() - want).abs().max()) <= 2.0**-22 * float(want.abs().max())
