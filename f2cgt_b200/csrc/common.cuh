@@ -176,6 +176,23 @@ __device__ __forceinline__ float div_exact_fast(float a, float b, float rcp) {
   return fmaf(r, rcp, q);
 }
 
+// a / b for four values, b a small positive integer, rcp = 1 / b; div_exact's corrections with one range check for all
+__device__ __forceinline__ float4 div4(float4 a, float b, float rcp) {
+  const float big = fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w)));
+  const float small = fminf(fminf(fabsf(a.x), fabsf(a.y)), fminf(fabsf(a.z), fabsf(a.w)));
+  if (big < 1e30f && small > 1e-30f && b <= 1048576.0f)
+    return make_float4(div_exact_fast(a.x, b, rcp), div_exact_fast(a.y, b, rcp), div_exact_fast(a.z, b, rcp), div_exact_fast(a.w, b, rcp));
+  return make_float4(a.x / b, a.y / b, a.z / b, a.w / b);
+}
+
+// Two floats in one 64-bit register, as add.f32x2 takes them.
+__device__ __forceinline__ void lds_2x64(uint32_t a, unsigned long long& x, unsigned long long& y) {
+  asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "r"(a));
+}
+__device__ __forceinline__ void add2(unsigned long long& acc, unsigned long long v) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(acc) : "l"(v)); }
+__device__ __forceinline__ float lo32(unsigned long long v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float hi32(unsigned long long v) { return __uint_as_float((uint32_t)(v >> 32)); }
+
 // Philox4x32-10 (Salmon et al., SC'11).  One call yields four 32-bit words for counter ctr.
 struct Philox {
   uint32_t k0, k1, o0, o1;

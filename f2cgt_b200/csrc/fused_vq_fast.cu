@@ -135,11 +135,39 @@ __global__ void __launch_bounds__(VqCta<HB>::kThreads, 1) vq_fast_kernel(const V
   const uint8_t* __restrict__ codes = reinterpret_cast<const uint8_t*>(p.codes) + (ANY ? s_begin : 0);
   const uint32_t code_bytes = ANY ? (uint32_t)p.n_cb : (uint32_t)ROWB;  // from one row to the next
 
+  // This lane's four columns: in pairs, which one instruction adds (VQ alone: 16 subspaces of 8 columns 30.4 -> 28.9 us with that, one
+  // vector store of the codes and one reciprocal per row), or single where hot rows arrive column by column (8 bits, pairs: 36.9 -> 40.7).
+  unsigned long long acc_lo, acc_hi;
   float4 acc;
   auto add_vq = [&](uint32_t edge_byte_addr) {
     const uint32_t code = lds_u8(edge_byte_addr);
-    const float4 v = lds_f4(cb_addr + code * (uint32_t)stride);
-    acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+    if constexpr (HB == 0) {
+      unsigned long long a, b;
+      lds_2x64(cb_addr + code * (uint32_t)stride, a, b);
+      add2(acc_lo, a); add2(acc_hi, b);
+    } else {
+      const float4 v = lds_f4(cb_addr + code * (uint32_t)stride);
+      acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+    }
+  };
+  // four edges whose reads are in flight together
+  auto add_vq4 = [&](uint32_t first) {
+    uint32_t c[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) c[i] = lds_u8(first + i * ROWB);
+    if constexpr (HB == 0) {
+      unsigned long long a[4], b[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) lds_2x64(cb_addr + c[i] * (uint32_t)stride, a[i], b[i]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) { add2(acc_lo, a[i]); add2(acc_hi, b[i]); }
+    } else {
+      float4 v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[i] = lds_f4(cb_addr + c[i] * (uint32_t)stride);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) { acc.x += v[i].x; acc.y += v[i].y; acc.z += v[i].z; acc.w += v[i].w; }
+    }
   };
   const uint32_t lane_off = (uint32_t)lane * (HB == 4 ? 8u : 4u);  // < 256: fits the low byte of the permute result
   const uint32_t lut_base = smem_u32(lut_s);
@@ -177,17 +205,20 @@ __global__ void __launch_bounds__(VqCta<HB>::kThreads, 1) vq_fast_kernel(const V
   };
   auto stage_codes = [&](const CodeRow<ROWW>& c, int cnt) {
     if (lane < cnt) {
+      uint32_t x[ROWW];
 #pragma unroll
       for (int w = 0; w < ROWW; ++w) {
-        uint32_t x = c.w[w];
+        x[w] = c.w[w];
         if (clamp) {  // codes >= K read the last centroid, as the general kernel does
           uint32_t y = 0;
 #pragma unroll
-          for (int b = 0; b < 4; ++b) y |= min((x >> (8 * b)) & 0xFFu, (uint32_t)(K - 1)) << (8 * b);
-          x = y;
+          for (int b = 0; b < 4; ++b) y |= min((x[w] >> (8 * b)) & 0xFFu, (uint32_t)(K - 1)) << (8 * b);
+          x[w] = y;
         }
-        wbuf[lane * ROWW + w] = x;
       }
+      if constexpr (ROWW == 4) *reinterpret_cast<uint4*>(wbuf + lane * 4) = make_uint4(x[0], x[1], x[2], x[3]);
+      else if constexpr (ROWW == 2) *reinterpret_cast<uint2*>(wbuf + lane * 2) = make_uint2(x[0], x[1]);
+      else wbuf[lane] = x[0];
     }
   };
 
@@ -218,14 +249,25 @@ __global__ void __launch_bounds__(VqCta<HB>::kThreads, 1) vq_fast_kernel(const V
     if (rE >= n_dst) break;
     // ================= stage 4: aggregate row rE
     if (rE >= r0) {
+      acc_lo = acc_hi = 0ull;
       acc = make_float4(0.f, 0.f, 0.f, 0.f);
       const int cnt0 = min(deg4, 32);
       __syncwarp();
       stage_codes(code4, cnt0);
       __syncwarp();
-      if (HB != 0) {
+      // Rows without hot neighbours - 74 % of 15-neighbour rows where 2 % of the nodes are hot, 46 % at 5 % - in a short loop of four edges
+      // whose reads overlap; the others one edge at a time, in code that the hot rows' registers need unrolled.  (59,000 rows x 12, 128
+      // columns of 32, 8-bit hot rows: 1 % hot 33.9 -> 29.1 us, 5 % 37.0 -> 35.6, 65 % 43.2 -> 43.4; 36,000 x 15, 256 columns of 64, 4 bits,
+      // 2 %: 51.0 -> 46.2.  Groups of four in the unrolled code of all rows: 58.)
+      if (HB == 0 || mask4 == 0u) {
+        int u = 0;
+#pragma unroll 1
+        for (; u + 4 <= cnt0; u += 4) add_vq4(wb_addr + u * ROWB);
+#pragma unroll 1
+        for (; u < cnt0; ++u) add_vq(wb_addr + u * ROWB);
+      } else {
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
+        for (int u = 0; u < (HB != 0 ? U : 0); ++u) {
           if (u >= cnt0) break;
           if ((mask4 >> u) & 1u) add_hot(hot[u]);
           else add_vq(wb_addr + u * ROWB);
@@ -235,19 +277,6 @@ __global__ void __launch_bounds__(VqCta<HB>::kThreads, 1) vq_fast_kernel(const V
           if (sl_ >= 0) add_hot(load_hot(sl_));
           else add_vq(wb_addr + u * ROWB);
         }
-      } else {
-        int u = 0;
-        for (; u + 4 <= cnt0; u += 4) {
-          const uint32_t c0 = lds_u8(wb_addr + u * ROWB), c1 = lds_u8(wb_addr + (u + 1) * ROWB);
-          const uint32_t c2 = lds_u8(wb_addr + (u + 2) * ROWB), c3 = lds_u8(wb_addr + (u + 3) * ROWB);
-          const float4 v0 = lds_f4(cb_addr + c0 * (uint32_t)stride), v1 = lds_f4(cb_addr + c1 * (uint32_t)stride);
-          const float4 v2 = lds_f4(cb_addr + c2 * (uint32_t)stride), v3 = lds_f4(cb_addr + c3 * (uint32_t)stride);
-          acc.x += v0.x; acc.y += v0.y; acc.z += v0.z; acc.w += v0.w;
-          acc.x += v1.x; acc.y += v1.y; acc.z += v1.z; acc.w += v1.w;
-          acc.x += v2.x; acc.y += v2.y; acc.z += v2.z; acc.w += v2.w;
-          acc.x += v3.x; acc.y += v3.y; acc.z += v3.z; acc.w += v3.w;
-        }
-        for (; u < cnt0; ++u) add_vq(wb_addr + u * ROWB);
       }
       // rows with more than 32 neighbours: further batches, fetched on the spot
       for (int64_t k0 = beg4 + 32; k0 < beg4 + deg4; k0 += 32) {
@@ -271,10 +300,8 @@ __global__ void __launch_bounds__(VqCta<HB>::kThreads, 1) vq_fast_kernel(const V
         }
       }
       if (active) {
-        if (p.reduce == F2C_MEAN) {
-          const float degf = deg4 == 0 ? 1.0f : (float)deg4;
-          acc.x = acc.x / degf; acc.y = acc.y / degf; acc.z = acc.z / degf; acc.w = acc.w / degf;
-        }
+        if constexpr (HB == 0) acc = make_float4(lo32(acc_lo), hi32(acc_lo), lo32(acc_hi), hi32(acc_hi));
+        if (p.reduce == F2C_MEAN && deg4 > 1) acc = div4(acc, (float)deg4, 1.0f / (float)deg4);
         const int64_t flat = (int64_t)rE * p.feat_dim + col;
         if (p.drop.enabled) acc = dropout_apply4(acc, (uint64_t)flat, p.drop);
         stg_cs_f4(p.out + flat, acc);

@@ -39,24 +39,9 @@ __device__ __forceinline__ uint4 lds_u128(uint32_t a) {
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
   return v;
 }
-__device__ __forceinline__ void lds_2x64(uint32_t a, unsigned long long& x, unsigned long long& y) {
-  asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "r"(a));
-}
 __device__ __forceinline__ void add_if(unsigned long long& acc, unsigned long long v, bool on) {
   asm("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q add.rn.f32x2 %0, %0, %1;\n\t}" : "+l"(acc) : "l"(v), "r"((uint32_t)on));
 }
-__device__ __forceinline__ float lo32(unsigned long long v) { return __uint_as_float((uint32_t)v); }
-__device__ __forceinline__ float hi32(unsigned long long v) { return __uint_as_float((uint32_t)(v >> 32)); }
-
-// a / b for four values, b a small positive integer, rcp = 1 / b; div_exact's corrections with one range check for all
-__device__ __forceinline__ float4 div4(float4 a, float b, float rcp) {
-  const float big = fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w)));
-  const float small = fminf(fminf(fabsf(a.x), fabsf(a.y)), fminf(fabsf(a.z), fabsf(a.w)));
-  if (big < 1e30f && small > 1e-30f && b <= 1048576.0f)
-    return make_float4(div_exact_fast(a.x, b, rcp), div_exact_fast(a.y, b, rcp), div_exact_fast(a.z, b, rcp), div_exact_fast(a.w, b, rcp));
-  return make_float4(a.x / b, a.y / b, a.z / b, a.w / b);
-}
-
 // NCH: 64-column chunks per part (1, 2).  WORDS: words of a row's code bytes in the part.  ANY: any alignment.  EB: bytes per code.
 template <typename IdxT, int NCH, int WORDS, bool ANY, int EB>
 __global__ void __launch_bounds__(kThreads, 1) vq_rows_kernel(const VqParams p) {
