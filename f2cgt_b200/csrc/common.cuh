@@ -93,12 +93,6 @@ __device__ __forceinline__ uint4 ldg_nc_u128_if(const void* p, bool on) {
                : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w) : "l"(p), "r"((uint32_t)on));
   return v;
 }
-__device__ __forceinline__ uint4 ldg_u128_if(const void* p, bool on) {  // the same through L1: the rest of a line is read soon
-  uint4 v = make_uint4(0u, 0u, 0u, 0u);
-  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %5, 0;\n\t@q ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];\n\t}"
-               : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w) : "l"(p), "r"((uint32_t)on));
-  return v;
-}
 // low 32 bits of a neighbour id, 0 without a load when !on
 __device__ __forceinline__ uint32_t ld_id_if(const int32_t* p, bool on) {
   uint32_t v = 0u;

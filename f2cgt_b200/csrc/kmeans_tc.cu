@@ -5,14 +5,11 @@
 
 namespace f2c {
 
-int kmeans_assign_exact_listed(const float* x, const float* y, int64_t* labels, const int32_t* list, const int32_t* count_dev,
-                               const int32_t* all_dev, int64_t max_count, int64_t k, int64_t d, int metric, bool y_settled, cudaStream_t st);
-
 namespace tc {
 
 template <int C, int NB>
-__global__ void __launch_bounds__(kThreads, 1) kmeans_tc_kernel(const Params p) {
-  dependency_wait();  // first of all: the kernel launched behind this one relies on it (y_settled below)
+__global__ void __launch_bounds__(kThreads, 1) kmeans_tc_kernel(const __grid_constant__ Params p) {
+  dependency_wait();
   release_dependents();
   run<C, NB>(p);
 }
@@ -42,7 +39,8 @@ static Kernel kernel_for(int64_t k, int64_t d) {
 
 // Eligibility and scratch size of the tensor-core path.
 bool kmeans_tc_supported(int64_t n, int64_t k, int64_t d) { return n >= 1 && n < (1ll << 31) && k >= 1 && k <= tc::kMaxN && d >= 1 && d <= 64; }
-int64_t kmeans_tc_workspace(int64_t n) { return 256 + 4 * n; }  // [count, error, pad][index list]
+constexpr int64_t kTcWorkspace = 256;  // [points that the exact scorer assigned, error]
+int64_t kmeans_tc_workspace() { return kTcWorkspace; }
 
 int kmeans_assign_tc(const float* x, const float* y, int64_t* labels, int64_t n, int64_t k, int64_t d, int metric, void* workspace,
                      cudaStream_t st) {
@@ -50,8 +48,8 @@ int kmeans_assign_tc(const float* x, const float* y, int64_t* labels, int64_t n,
   tc::describe(p, x, y, n, k, d, metric);
   p.labels = labels;
   int32_t* head = reinterpret_cast<int32_t*>(workspace);
-  p.amb_count = head; p.error = head + 1; p.amb_list = head + 64;
-  cudaError_t e = cudaMemsetAsync(head, 0, 256, st);
+  p.undecided = head; p.error = head + 1;
+  cudaError_t e = cudaMemsetAsync(head, 0, 8, st);
   if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "kmeans_assign: %s", cudaGetErrorString(e));
   auto [kern, smem] = tc::kernel_for(k, d);
   if (smem < tc::kOneCta) smem = tc::kOneCta;
@@ -60,32 +58,26 @@ int kmeans_assign_tc(const float* x, const float* y, int64_t* labels, int64_t n,
   int64_t grid = ceil_div(n, tc::kTileM);
   if (grid > current_sm_count()) grid = current_sm_count();  // one CTA per SM (it owns all 512 TMEM columns)
   launch_dependent(kern, (unsigned)grid, tc::kThreads, smem, st, p);
-  int rc = check_launch("kmeans_assign (tensor cores)");
-  if (rc) return rc;
-  // undecided points (all of them after a wait that ran out): exact fp32 scorer over the device-side list
-  return kmeans_assign_exact_listed(x, y, labels, p.amb_list, p.amb_count, p.error, n, k, d, metric, /* y_settled */ true, st);
+  return check_launch("kmeans_assign (tensor cores)");
 }
 
 // ------------------------------------------------------------------------------------------------------
 // K-means assignment for callers that cannot allocate device memory.
 //
-// f2c_kmeans_assign leaves the undecided-point list to the caller, which means one device allocation per
-// call (or a buffer the caller has to carry around).  Some callers cannot do that: a data-loader or serving
-// thread that lives inside a process whose framework allocator already owns almost all of HBM (a raw
-// cudaMalloc there can fail, or make the framework drop its cache), and callers on a latency-critical
-// path, where cudaMalloc / cudaFree would stall every stream of the device.  For them the scratch lives in
-// a fixed array in the library's device image: 4 MiB + 256 B on every GPU that loads the library, held until
-// the process exits, enough for kStaticMaxPoints points per call.
+// f2c_kmeans_assign reports to a buffer of the caller's, which means one small device allocation per call (or a buffer the caller
+// has to carry around).  Some callers cannot do that: a data-loader or serving thread that lives inside a process whose framework
+// allocator already owns almost all of HBM (a raw cudaMalloc there can fail, or make the framework drop its cache), and callers on
+// a latency-critical path, where cudaMalloc / cudaFree would stall every stream of the device.  For them the report lives in a
+// fixed array in the library's device image.  (It held a list of undecided points, too, which is where the limit of points per
+// call comes from.)
 //
 // The array's name below is only a host-side handle; the device address is obtained once per device with
 // cudaGetSymbolAddress while that device is current.  That happens on the first call made on a device (a
-// synchronising runtime query, once).  All calls on a device share the one array: the header is
-// cleared at the start of every call, the list behind it keeps whatever the previous call left and is only
-// read up to the new count.  Two calls that overlap on the GPU (different streams, or threads) would
-// overwrite each other's list - serialise them.
+// synchronising runtime query, once).  All calls on a device share the one array, which is cleared at the start of every call:
+// two calls that overlap on the GPU (different streams, or threads) would mix their reports - serialise them.
 namespace tc {
 constexpr int64_t kStaticMaxPoints = 1 << 20;
-static __device__ __align__(256) unsigned char g_static_scratch[256 + 4 * kStaticMaxPoints];
+static __device__ __align__(256) unsigned char g_static_scratch[kTcWorkspace];
 
 // Device address of the scratch array on the current device, looked up once per device (with that device current).
 static int static_scratch(const char* op, void** scratch) {

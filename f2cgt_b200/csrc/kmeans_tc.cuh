@@ -17,9 +17,8 @@
 //    carries powers of two on the point side and three f16 pieces of -|y_c|^2/2 on the centre side, so the epilogue is a pure
 //    arg-max.  A column that is padding carries -65504 in that chunk.
 //  * The epilogue reads the 128 x 256 scores with tcgen05.ld (one point per thread) and finds the best score and whether it is
-//    the only one within the error bound of the product.  A point where it is not is NOT decided here: its index is appended to
-//    a scratch list and the exact fp32 scorer (kmeans.cu) assigns it afterwards, so every label equals the label of the exact
-//    fp32 kernel.  (Squared distances of points that lie some 10^3 times further out than the centres differ by less than their
+//    the only one within the error bound of the product.  A point where it is not goes to a list of the CTA, whose warps give it
+//    the label of the exact fp32 scorer (kmeans.cu) at the end, so every label equals the label of that kernel.  (Squared distances of points that lie some 10^3 times further out than the centres differ by less than their
 //    own fp32 rounding; there the score, which leaves |x|^2 out, still decides, for the nearer centre.)
 //  * Overlap.  A CTA has 22 warps with fixed roles: three groups of four epilogue warps, two of four producer warps, which have their
 //    points' rows copied to shared memory ahead, split them and store them into a ring of A tiles, and two warps whose first lanes issue the
@@ -29,8 +28,10 @@
 //    pipe 66 % busy) and the latency of the chain accumulator free - MMAs - accumulator full; more dimensions: the producers' chains of
 //    dependent instructions, whatever memory and the tensor pipe do (without the splitting 147 us of 2,449,029 x 32 become 110).
 //    Measured, 2,449,029 points against 256 centres, whole call (before: sixteen warps that all loaded, split, waited and searched, one barrier
-//    per tile, 3 x tf32 or 3 x bf16): 8 dimensions 154 -> 102 us, 16: 193 -> 117, 24: 228 -> 141, 32: 267 -> 154, 64: 401 -> 313; 100 centres
-//    of 8 dimensions 119 -> 77, of 64: 359 -> 217.  Two epilogue groups instead of three: 8 dimensions 107.
+//    per tile, 3 x tf32 or 3 x bf16, undecided points in a second kernel): 8 dimensions 153 -> 98 us, 16: 193 -> 112, 24: 227 -> 142, 32: 265
+//    -> 157, 64: 400 -> 305; 100 centres of 8 dimensions 118 -> 72, of 64: 357 -> 229.  Two epilogue groups instead of three: 8 dimensions 107.
+//    Few points: 5000 x 8 20 -> 11, 40,000 x 8 20 -> 12.5, 149,000 x 32 37 -> 26 (without the second kernel, its list and the clearing of it;
+//    with them 20, 18 and 28), 149,000 x 64 47 -> 48.
 //    Every wait on an mbarrier is bounded; on expiry an error code is recorded, which makes the exact scorer assign every point, no further
 //    wait is made and no copy started, and the CTA frees its TMEM at the common exit once its own copies and MMAs are complete.
 #pragma once
@@ -51,6 +52,7 @@ constexpr uint32_t kWaitLimit = 1u << 18, kWaitHint = 4000;  // tries, and nanos
 constexpr int kEpilogueGroups = 3, kEpilogueWarps = 4 * kEpilogueGroups, kProducerWarps = 8;
 constexpr int kMmaWarp = kEpilogueWarps + kProducerWarps, kMmaWarps = 2;  // one per pair of accumulators of 128 columns
 constexpr int kThreads = 32 * (kMmaWarp + kMmaWarps);
+constexpr int kList = 1024;    // undecided points that a CTA keeps in shared memory
 constexpr int kBoundRing = 8;  // tiles whose error bounds are kept; more than the A ring and the two accumulators hold together
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -124,9 +126,8 @@ struct Params {
   const float* x;
   const float* y;
   int64_t* labels;
-  int32_t* amb_list;   // scratch: indices of undecided points
-  int32_t* amb_count;  // scratch: their number
-  int32_t* error;      // scratch: non-zero when a bounded wait expired
+  int32_t* undecided;  // how many points the exact scorer assigned
+  int32_t* error;      // non-zero when a bounded wait expired
   int64_t n;
   int k, d;
   int metric;
@@ -234,47 +235,215 @@ struct Ring {
   static constexpr int slots = C == 1 ? 8 : C == 2 ? 4 : C >= 7 ? 1 : 2;
   static constexpr size_t bytes = (size_t)Operands<C>::b_chunks * (NB * 512 + Lanes<C>::PAD) + (size_t)Operands<C>::a_chunks * stages * (kTileM * 16 + Lanes<C>::PAD) +
                                   (size_t)kProducerWarps * slots * Lanes<C>::PART_BYTES + kMaxN * 4 + kBoundRing * kTileM * 4 +
-                                  8 * (2 * turns + 4 * kEpilogueGroups + 6 + kProducerWarps * slots) + 16;
+                                  8 * (2 * turns + 4 * kEpilogueGroups + 6 + kProducerWarps * slots) + 16 + 4 * kList;
   static_assert(bytes <= 227 * 1024, "shared memory of a CTA");
 };
 
-// ---------------------------------------------------------------- the second half of a Lloyd iteration
-// Label of one point by the exact scorer, by a whole warp: the sums of kmeans.cu's kernels, term by term.  yc: centres of DP floats, zero
-// padded, STRIDE apart (eight lanes that read a piece of eight centres touch eight bank groups); cc: their squared norms; xs: the point.
-template <int DP>
-__device__ __forceinline__ int nearest(const float* yc, const float* cc, const float* xs, int k, bool cosine) {
-  constexpr int STRIDE = DP + 4;
-  const int lane = threadIdx.x & 31;
-  float xx = 0.0f;
-  if (cosine)
-    for (int t = 0; t < DP; ++t) xx = fmaf(xs[t], xs[t], xx);
-  float best = INFINITY;
-  int best_c = 0x7fffffff;
-  for (int c = lane; c < k; c += 32) {
-    float acc = 0.0f;
+// ---------------------------------------------------------------- points that the tensor cores leave undecided
+// Shared memory, behind the assignment, of a list of undecided points (numbered inside the CTA: 128 * tile + row) and of their labels.
+constexpr int kFew = 8;     // points up to which the centres are not staged for them
+constexpr int kMany = 400;  // points from which on a thread scores one
+struct Scores {
+  unsigned long long nearest[kFew];
+  uint16_t label[kList];
+};
+
+// Labels of the listed points by exact distances, term by term those of kmeans.cu's kernels; called by all threads.
+//  * A few points: a warp scores one of them against 32 centres where these lie; the smallest distance, then the smallest index.  (Staging
+//    the centres for them took 7 to 28 thousand cycles, and in a fit all other CTAs waited for the few that had such points.)
+//  * More: the centres are staged in a_ring, rows padded so that eight lanes touch eight bank groups, and a warp scores a point.
+//  * Many, as where rows are zero: a thread scores a point, a centre is read once for 32 of them.
+template <int C>
+__device__ __noinline__ void score_exactly(const Params& p, const uint32_t* list, int count, Scores* out, unsigned char* a_ring, float* points, bool& staged) {
+  constexpr int DP = 8 * C, STRIDE = DP + 4, kWarps = kThreads / 32;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const bool cosine = p.metric == F2C_COSINE;
+  auto point = [&](int w) {
+    const int at = (int)list[w];
+    return p.x + (((int64_t)blockIdx.x + (int64_t)(at >> 7) * gridDim.x) * kTileM + (at & 127)) * p.d;
+  };
+  auto distance = [&](float acc, float x_norm, float c_norm) {  // finish_cosine() with the square roots taken before
+    const float den = x_norm * c_norm, v = !cosine ? acc : den > 0.0f ? 1.0f - acc / den : 1.0f;
+    return v != v ? 1.0f : v;
+  };
+  if (count <= kFew) {
+    if (tid < kFew) out->nearest[tid] = ~0ull;
+    for (int e = tid; e < count * DP; e += kThreads) points[e] = e % DP < p.d ? __ldg(point(e / DP) + e % DP) : 0.0f;
+    __syncthreads();
+    const int blocks = (p.k + 31) / 32;
+    for (int w = warp; w < count * blocks; w += kWarps) {
+      const int c = w % blocks * 32 + lane;
+      const float* xs = points + w / blocks * DP;
+      const float* yc = p.y + min(c, p.k - 1) * p.d;
+      float acc = 0.0f, xx = 0.0f, cc = 0.0f;
+#pragma unroll 1
+      for (int b = 0; b < DP; b += 32) {
+        constexpr int IN_FLIGHT = C < 4 ? C : 4;
+        float y[IN_FLIGHT][8];
 #pragma unroll
-    for (int t = 0; t < DP; t += 4) {
-      const float4 a = *reinterpret_cast<const float4*>(xs + t), b = *reinterpret_cast<const float4*>(yc + c * STRIDE + t);
-      if (!cosine) {
-        const float d0 = a.x - b.x, d1 = a.y - b.y, d2 = a.z - b.z, d3 = a.w - b.w;
-        acc = fmaf(d0, d0, acc); acc = fmaf(d1, d1, acc); acc = fmaf(d2, d2, acc); acc = fmaf(d3, d3, acc);
-      } else {
-        acc = fmaf(a.x, b.x, acc); acc = fmaf(a.y, b.y, acc); acc = fmaf(a.z, b.z, acc); acc = fmaf(a.w, b.w, acc);
+        for (int q = 0; q < IN_FLIGHT; ++q) load8(yc, b + 8 * q, p.d, p.y_wide, true, y[q]);
+#pragma unroll
+        for (int q = 0; q < IN_FLIGHT; ++q) {
+          if (b + 8 * q >= DP) break;
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const float a = xs[b + 8 * q + e];
+            if (cosine) {
+              acc = fmaf(a, y[q][e], acc);
+              xx = fmaf(a, a, xx);
+              cc = fmaf(y[q][e], y[q][e], cc);
+            } else {
+              const float df = a - y[q][e];
+              acc = fmaf(df, df, acc);
+            }
+          }
+        }
       }
+      const uint32_t bits = __float_as_uint(distance(acc, sqrtf(xx), sqrtf(cc))), order = bits ^ ((int32_t)bits < 0 ? 0xffffffffu : 0x80000000u);
+      if (c < p.k) atomicMin(out->nearest + w / blocks, (unsigned long long)order << 32 | (uint32_t)c);
     }
-    float v = cosine ? finish_cosine(acc, xx, cc[c]) : acc;
-    if (v != v) v = 1.0f;
-    if (v < best) { best = v; best_c = c; }
+    __syncthreads();
+    if (tid < count) out->label[tid] = (uint16_t)out->nearest[tid];
+    __syncthreads();
+    return;
   }
+  float* yc = reinterpret_cast<float*>(a_ring);
+  float* norm = yc + p.k * STRIDE;
+  if (!staged) {
+#pragma unroll 12
+    for (int e = tid; e < p.k * DP; e += kThreads) {  // many reads in flight
+      const int c = e / DP, t = e - c * DP;
+      yc[c * STRIDE + t] = t < p.d ? __ldcg(p.y + c * p.d + t) : 0.0f;
+    }
+    __syncthreads();
+    for (int c = tid; c < p.k; c += kThreads) {
+      float s = 0.0f;
+      for (int t = 0; t < DP; ++t) s = fmaf(yc[c * STRIDE + t], yc[c * STRIDE + t], s);
+      norm[c] = sqrtf(s);
+    }
+    __syncthreads();
+    staged = true;
+  }
+  if (count < kMany) {
+    float* xs = points + warp * DP;
+    for (int w = warp; w < count; w += kWarps) {
+      const float* xi = point(w);
+      __syncwarp();
+      for (int t = lane; t < DP; t += 32) xs[t] = t < p.d ? __ldg(xi + t) : 0.0f;
+      __syncwarp();
+      float xx = 0.0f, best = INFINITY;
+      int best_c = 0x7fffffff;
+      if (cosine)
+        for (int t = 0; t < DP; ++t) xx = fmaf(xs[t], xs[t], xx);
+      const float x_norm = sqrtf(xx);
+      for (int c = lane; c < p.k; c += 32) {
+        float acc = 0.0f;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-    const int oc = __shfl_xor_sync(0xffffffffu, best_c, o);
-    if (ob < best || (ob == best && oc < best_c)) { best = ob; best_c = oc; }
+        for (int t = 0; t < DP; t += 4) {
+          const float4 a = *reinterpret_cast<const float4*>(xs + t), b = *reinterpret_cast<const float4*>(yc + c * STRIDE + t);
+          if (!cosine) {
+            const float d0 = a.x - b.x, d1 = a.y - b.y, d2 = a.z - b.z, d3 = a.w - b.w;
+            acc = fmaf(d0, d0, acc); acc = fmaf(d1, d1, acc); acc = fmaf(d2, d2, acc); acc = fmaf(d3, d3, acc);
+          } else {
+            acc = fmaf(a.x, b.x, acc); acc = fmaf(a.y, b.y, acc); acc = fmaf(a.z, b.z, acc); acc = fmaf(a.w, b.w, acc);
+          }
+        }
+        const float v = distance(acc, x_norm, norm[c]);
+        if (v < best) { best = v; best_c = c; }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+        const int oc = __shfl_xor_sync(0xffffffffu, best_c, o);
+        if (ob < best || (ob == best && oc < best_c)) { best = ob; best_c = oc; }
+      }
+      if (lane == 0) out->label[w] = (uint16_t)(best_c == 0x7fffffff ? 0 : best_c);
+    }
+  } else {
+    for (int w = tid; w < count; w += kThreads) {
+      const float* xi = point(w);
+      float xr[DP], xx = 0.0f, best = INFINITY;
+      int best_c = 0;
+#pragma unroll
+      for (int t = 0; t < DP; ++t) {
+        xr[t] = t < p.d ? __ldg(xi + t) : 0.0f;
+        xx = fmaf(xr[t], xr[t], xx);
+      }
+      const float x_norm = sqrtf(xx);
+#pragma unroll 1
+      for (int c = 0; c < p.k; ++c) {
+        float acc = 0.0f;
+#pragma unroll
+        for (int t = 0; t < DP; t += 4) {
+          const float4 b = *reinterpret_cast<const float4*>(yc + c * STRIDE + t);
+          if (!cosine) {
+            const float d0 = xr[t] - b.x, d1 = xr[t + 1] - b.y, d2 = xr[t + 2] - b.z, d3 = xr[t + 3] - b.w;
+            acc = fmaf(d0, d0, acc); acc = fmaf(d1, d1, acc); acc = fmaf(d2, d2, acc); acc = fmaf(d3, d3, acc);
+          } else {
+            acc = fmaf(xr[t], b.x, acc); acc = fmaf(xr[t + 1], b.y, acc); acc = fmaf(xr[t + 2], b.z, acc); acc = fmaf(xr[t + 3], b.w, acc);
+          }
+        }
+        const float v = distance(acc, x_norm, norm[c]);
+        if (v < best) { best = v; best_c = c; }
+      }
+      out->label[w] = (uint16_t)best_c;
+    }
   }
-  return best_c == 0x7fffffff ? 0 : best_c;
+  __syncthreads();
 }
 
+// What an assignment does with its undecided points: the CTA's list holds the first kList of them; if there are more, or a wait has run out,
+// they are found by their labels, -1, and scored as many at a time as there are threads.
+template <int C>
+__device__ __noinline__ void settle(const Params& p, int turns, bool all, const uint32_t* open_list, uint32_t* counter, unsigned char* a_ring, unsigned char* rows) {
+  Scores* scores = reinterpret_cast<Scores*>(rows);
+  uint32_t* list = reinterpret_cast<uint32_t*>(scores + 1);  // [2 * kThreads]
+  float* points = reinterpret_cast<float*>(list + 2 * kThreads);
+  static_assert(sizeof(Scores) % 16 == 0 && kThreads <= kList && sizeof(Scores) + 8 * kThreads + kThreads / 32 * 8 * C * 4 <= kProducerWarps * Ring<C, 4>::slots * Lanes<C>::PART_BYTES,
+                "fits the rows' place");
+  const int tid = threadIdx.x;
+  const uint32_t open = *counter;
+  bool staged = false;
+  auto index_of = [&](uint32_t at) { return ((int64_t)blockIdx.x + (int64_t)(at >> 7) * gridDim.x) * kTileM + (at & 127u); };
+  auto score = [&](const uint32_t* which, int count) {
+    score_exactly<C>(p, which, count, scores, a_ring, points, staged);
+    for (int w = tid; w < count; w += kThreads) p.labels[index_of(which[w])] = scores->label[w];
+    __syncthreads();
+  };
+  uint32_t total = open;
+  if (!all && open <= (uint32_t)kList) {
+    if (open == 0u) return;
+    score(open_list, (int)open);
+  } else {
+    total = 0u;
+    __syncthreads();
+    if (tid == 0) *counter = 0u;
+    for (int first = 0; first < turns * kTileM; first += kThreads) {
+      __syncthreads();
+      const uint32_t at = (uint32_t)(first + tid);
+      const int64_t i = index_of(at);
+      if (first + tid < turns * kTileM && i < p.n && (all || __ldcg(p.labels + i) < 0)) list[atomicAdd(counter, 1u)] = at;
+      __syncthreads();
+      int count = (int)*counter;
+      const bool last = first + kThreads >= turns * kTileM;
+      for (int from = 0; count >= kThreads || (last && count > 0); from += kThreads, count -= min(count, kThreads)) {
+        score(list + from, min(count, kThreads));
+        total += (uint32_t)min(count, kThreads);
+        if (count < kThreads) break;
+        if (count - kThreads < kThreads && !last) {  // the rest moves to the front
+          const uint32_t rest = tid < count - kThreads ? list[from + kThreads + tid] : 0u;
+          __syncthreads();
+          if (tid < count - kThreads) list[tid] = rest;
+          if (tid == 0) *counter = (uint32_t)(count - kThreads);
+          break;
+        }
+      }
+    }
+  }
+  if (tid == 0) atomicAdd(p.undecided, (int32_t)total);
+}
+
+// ---------------------------------------------------------------- the second half of a Lloyd iteration
 // Behind the labels of this CTA's points: those that are still undecided, the clusters' sums, and, all CTAs together, the new centres.
 // Returns whether the fit has converged.  `number`: of this iteration; `all`: score every point exactly.  a_ring, rows: shared memory that
 // the assignment has done with.
@@ -291,7 +460,6 @@ __device__ __noinline__ bool end_of_iteration(const FitParams& p, int number, in
   constexpr int W = C == 1 ? 8 : C == 2 ? 16 : 32, CPL = C > 4 ? 2 : 1;  // lanes per point, columns per lane
   uint2* sorted = reinterpret_cast<uint2*>(rows);  // cluster and, where it lost the point, kLost; where the point's row starts behind the chunk's first
   constexpr uint32_t kLost = 1u << 16;
-  constexpr int kFew = 32;  // open points up to which the centres are not staged for them
   uint32_t* hist = reinterpret_cast<uint32_t*>(sorted + 2 * kChunk);
   uint32_t* start = hist + kMaxN;  // [257]
   int32_t* gained = reinterpret_cast<int32_t*>(start + kMaxN + 4);
@@ -299,8 +467,6 @@ __device__ __noinline__ bool end_of_iteration(const FitParams& p, int number, in
   double* part = reinterpret_cast<double*>(point + kWarps * DP);
   static_assert((4 * kChunk + 3 * kMaxN + 4 + kWarps * DP + 2 * kWarps) * 4 <= kProducerWarps * Ring<C, 4>::slots * Lanes<C>::PART_BYTES &&
                     (4 * kChunk + 3 * kMaxN + 4 + kWarps * DP + 2 * kWarps) * 4 <= kProducerWarps * Ring<C, 8>::slots * Lanes<C>::PART_BYTES, "fits the rows' place");
-  float* yc = reinterpret_cast<float*>(a_ring);
-  float* cc = yc + p.k * (DP + 4);
   static_assert(kMaxN * (DP + 5) * 4 <= Ring<C, 8>::stages * Operands<C>::a_chunks * (kTileM * 16 + Lanes<C>::PAD), "fits the A ring's place");
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bool all = lost || *(volatile const int32_t*)p.error != 0;
@@ -329,95 +495,33 @@ __device__ __noinline__ bool end_of_iteration(const FitParams& p, int number, in
     for (int c = tid; c < kMaxN; c += kThreads) { hist[c] = 0u; gained[c] = 0; }
     if (tid == 0) start[0] = 0u;  // length of the list of open points
     uint32_t label[kShares], before[kShares], rank[kShares], rank_before[kShares];
-    auto read_labels = [&] {
-      bool open = false;
+    bool open = false;
+#pragma unroll
+    for (int s = 0; s < kShares; ++s) {
+      const int g = warp + kWarps * s;
+      const int64_t i = index_of(t0 + (g >> 2), (g & 3) * 32 + lane);
+      label[s] = g < shares && i < p.n ? __ldcg(p.labels16 + i) : kUndecided + 1u;
+      open |= label[s] == kUndecided;
+    }
+    if (__syncthreads_or(open || all)) {
+      uint32_t* list = reinterpret_cast<uint32_t*>(rows);
+      Scores* scores = reinterpret_cast<Scores*>(rows + kChunk * 4);
+      static_assert(kChunk <= kList && kChunk * 4 + sizeof(Scores) <= 2 * kChunk * sizeof(uint2), "in the place of the sorted changes");
+      int entry[kShares];
 #pragma unroll
       for (int s = 0; s < kShares; ++s) {
-        const int g = warp + kWarps * s;
-        const int64_t i = index_of(t0 + (g >> 2), (g & 3) * 32 + lane);
-        label[s] = g < shares && i < p.n ? __ldcg(p.labels16 + i) : kUndecided + 1u;
-        open |= label[s] == kUndecided;
+        entry[s] = -1;
+        if (label[s] == kUndecided || (all && label[s] < kUndecided)) {
+          entry[s] = (int)atomicAdd(start, 1u);
+          list[entry[s]] = (uint32_t)(t0 * kTileM + (warp + kWarps * s) * 32 + lane);
+        }
       }
-      return open;
-    };
-    const bool open = read_labels();
-    if (__syncthreads_or(open || all)) {
-      // the open points in a list, which all warps work on
-      uint32_t* open_points = reinterpret_cast<uint32_t*>(rows);
-      unsigned long long* nearest_of = reinterpret_cast<unsigned long long*>(rows + kChunk * 4);
+      __syncthreads();
+      score_exactly<C>(p, list, (int)start[0], scores, a_ring, point, staged);
 #pragma unroll
       for (int s = 0; s < kShares; ++s)
-        if (label[s] == kUndecided || (all && label[s] < kUndecided))
-          open_points[atomicAdd(start, 1u)] = (uint32_t)((warp + kWarps * s) * 32 + lane);
-      if (tid < kFew) nearest_of[tid] = ~0ull;
-      __syncthreads();
-      const int list = (int)start[0];
-      if (list <= kFew) {
-        // a few points: a warp scores one of them against 32 centres where these lie; the smallest distance, then the smallest index
-        // (staging the centres for them took 7 to 28 thousand cycles, and all other CTAs waited for the few that had such points)
-        const int blocks = (p.k + 31) / 32;
-        for (int w = warp; w < list * blocks; w += kWarps) {
-          const int at = (int)open_points[w / blocks], c = w % blocks * 32 + lane;
-          const float* xi = p.x + index_of(t0 + (at >> 7), at & 127) * p.d;
-          const float* yc = p.centers + min(c, p.k - 1) * p.d;
-          const bool cosine = p.metric == F2C_COSINE;
-          float acc = 0.0f, xx = 0.0f, cc = 0.0f;
-#pragma unroll 2
-          for (int b = 0; b < DP; b += 8) {
-            float a[8], y[8];
-            load8(xi, b, p.d, p.x_wide && p.x_aligned, true, a);
-            load8(yc, b, p.d, p.y_wide, true, y);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              if (cosine) {
-                acc = fmaf(a[e], y[e], acc);
-                xx = fmaf(a[e], a[e], xx);
-                cc = fmaf(y[e], y[e], cc);
-              } else {
-                const float df = a[e] - y[e];
-                acc = fmaf(df, df, acc);
-              }
-            }
-          }
-          float v = cosine ? finish_cosine(acc, xx, cc) : acc;
-          if (v != v) v = 1.0f;
-          const uint32_t bits_v = __float_as_uint(v), order = bits_v ^ ((int32_t)bits_v < 0 ? 0xffffffffu : 0x80000000u);
-          if (c < p.k) atomicMin(nearest_of + w / blocks, (unsigned long long)order << 32 | (uint32_t)c);
-        }
-        __syncthreads();
-        if (tid < list) {
-          const int at = (int)open_points[tid];
-          __stcg(p.labels16 + index_of(t0 + (at >> 7), at & 127), (uint16_t)nearest_of[tid]);
-        }
-      } else {
-        if (!staged) {
-#pragma unroll 12
-          for (int e = tid; e < p.k * DP; e += kThreads) {
-            const int c = e / DP, t = e - c * DP;
-            yc[c * (DP + 4) + t] = t < p.d ? __ldcg(p.centers + c * p.d + t) : 0.0f;
-          }
-          __syncthreads();
-          for (int c = tid; c < p.k; c += kThreads) {
-            float s = 0.0f;
-            for (int t = 0; t < DP; ++t) s = fmaf(yc[c * (DP + 4) + t], yc[c * (DP + 4) + t], s);
-            cc[c] = s;
-          }
-          __syncthreads();
-          staged = true;
-        }
-        float* xs = point + warp * DP;
-        for (int w = warp; w < list; w += kWarps) {
-          const int at = (int)open_points[w];
-          const int64_t i = index_of(t0 + (at >> 7), at & 127);
-          __syncwarp();
-          for (int t = lane; t < DP; t += 32) xs[t] = t < p.d ? __ldg(p.x + i * p.d + t) : 0.0f;
-          __syncwarp();
-          const int c = nearest<DP>(yc, cc, xs, p.k, p.metric == F2C_COSINE);
-          if (lane == 0) __stcg(p.labels16 + i, (uint16_t)c);
-        }
-      }
-      __syncthreads();
-      read_labels();
+        if (entry[s] >= 0) label[s] = scores->label[entry[s]];
+      __syncthreads();  // the sorted changes take their place
     }
     bool any = false;
 #pragma unroll
@@ -568,7 +672,7 @@ __device__ __noinline__ bool end_of_iteration(const FitParams& p, int number, in
   return converged;
 }
 
-// Shared memory: [B tile][A ring][rows in flight][norms 256 floats][bounds kBoundRing x 128 floats][mbarriers, tmem slot]
+// Shared memory: [B tile][A ring][rows in flight][norms 256 floats][bounds kBoundRing x 128 floats][mbarriers, tmem slot, count and list of undecided points]
 // C: chunks of eight dimensions of a row (1 to 8); NB: blocks of 32 columns (4: up to 128 centres, 8: up to 256).
 // P = Params: one assignment.  FitParams: Lloyd iterations, by CTAs that are all resident (kmeans_fit_tc.cu); tiles are then counted on
 // from iteration to iteration, so that the barriers' phases go on.
@@ -597,6 +701,8 @@ __device__ __forceinline__ void run(const P& p) {
   const uint32_t a_full = smem_u32(mbars), a_free = a_full + 8 * Q::turns, acc_full = a_free + 8 * Q::turns, acc_free = acc_full + 8 * kFull * HALVES,
                  drained = acc_free + 32, row_full = drained + 16;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mbars + 2 * Q::turns + 6 + kFull * HALVES + kProducerWarps * Q::slots);
+  uint32_t* open_count = tmem_slot + 1;  // undecided points of this CTA, the first kList of them in the list
+  uint32_t* open_list = tmem_slot + 4;
 
   const int64_t n_tiles = (p.n + kTileM - 1) / kTileM;
   const int turns = (int)((n_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x);  // tiles of this CTA: blockIdx.x + t * gridDim.x
@@ -636,6 +742,7 @@ __device__ __forceinline__ void run(const P& p) {
 
   // ---- one-time setup: mbarriers, TMEM (all 512 columns), centre tile ----
   if (threadIdx.x == 32 * kMmaWarp) {
+    *open_count = 0u;
     for (int s = 0; s < Q::turns; ++s) { mbar_init(a_full + 8 * s, 4); mbar_init(a_free + 8 * s, 1); }
     for (int u = 0; u < kFull * HALVES; ++u) mbar_init(acc_full + 8 * u, 1);
     for (int u = 0; u < 4; ++u) mbar_init(acc_free + 8 * u, 4);
@@ -840,7 +947,8 @@ __device__ __forceinline__ void run(const P& p) {
             const float floor = 2.0f * cmax * (l2 ? fmaxf(0x1p-19f * own_factor, 0x1p-126f) : 0x1p-21f);  // f16 at its lower end, and the norm term
             const float unscale = __int_as_float((254 << 23) - __float_as_int(own_factor)) * power2f(e_y);  // 1 / all that x was multiplied with
             // INFINITY for NaN, and for a point whose |x|^2 is more than fp32 holds: the exact scorer's distance says so
-            const float bound = own_sum * unscale * unscale < INFINITY ? fminf(fmaf(eps, sqrt_approx(own_sum), floor), INFINITY) : INFINITY;
+            // (-1 for a row of zeros under the cosine metric: all its distances are 1, its label is 0)
+            const float bound = !l2 && own_sum == 0.0f ? -1.0f : own_sum * unscale * unscale < INFINITY ? fminf(fmaf(eps, sqrt_approx(own_sum), floor), INFINITY) : INFINITY;
             if (chunk_l < L::READS) {
               bounds[(t & (kBoundRing - 1)) * kTileM + row] = bound;
               if (l2) {
@@ -947,21 +1055,22 @@ __device__ __forceinline__ void run(const P& p) {
 #pragma unroll
           for (int j = 0; j < 16; ++j) add_if_ge(cols_hit[j & 1], col_max[j], from, 64 + j);
           const int r_hit = rows_hit[0] + rows_hit[1], c_hit = cols_hit[0] + cols_hit[1];
-          const int centre = 16 * r_hit + c_hit - (16 * 64 + 64);
-          const bool decided = (r_hit >> 6) == 1 && (c_hit >> 6) == 1 && best > -INFINITY;
+          const bool zero = bound < 0.0f;
+          const int centre = zero ? 0 : 16 * r_hit + c_hit - (16 * 64 + 64);
+          const bool decided = zero || ((r_hit >> 6) == 1 && (c_hit >> 6) == 1 && best > -INFINITY);
           const int64_t i = ((int64_t)blockIdx.x + (int64_t)(t - base) * gridDim.x) * kTileM + pt;
           if constexpr (FIT) {
             if (i < p.n) p.labels16[i] = (uint16_t)(decided ? (uint32_t)centre : kUndecided);
           } else {
             const bool undecided = i < p.n && !decided;
-            const uint32_t listed = __ballot_sync(0xffffffffu, undecided);  // the exact scorer assigns them afterwards
+            const uint32_t listed = __ballot_sync(0xffffffffu, undecided);
             if (listed != 0u) {
-              int slot = 0;
-              if (lane == 0) slot = atomicAdd(p.amb_count, __popc(listed));
-              slot = __shfl_sync(0xffffffffu, slot, 0);
-              if (undecided) p.amb_list[slot + __popc(listed & ((1u << lane) - 1u))] = (int32_t)i;
+              uint32_t slot = 0;
+              if (lane == 0) slot = atomicAdd(open_count, (uint32_t)__popc(listed));
+              slot = __shfl_sync(0xffffffffu, slot, 0) + __popc(listed & ((1u << lane) - 1u));
+              if (undecided && slot < (uint32_t)kList) open_list[slot] = (uint32_t)(t * kTileM + pt);
             }
-            if (i < p.n && decided) p.labels[i] = centre;
+            if (i < p.n) p.labels[i] = decided ? centre : -1;
           }
         }
       }
@@ -969,6 +1078,9 @@ __device__ __forceinline__ void run(const P& p) {
     if constexpr (FIT) {
       lost = __syncthreads_or(wait.gave_up) != 0;
       if (end_of_iteration<C>(p, done_before + it, turns, lost, a_ring, rows)) break;
+    } else {
+      lost = __syncthreads_or(wait.gave_up) != 0;
+      settle<C>(p, turns, lost, open_list, open_count, a_ring, rows);
     }
   }
 

@@ -226,23 +226,16 @@ PyObject* kmeans_assign(PyObject*, PyObject* const* a, Py_ssize_t n) {  // x, ce
     if (x.dim() != 2 || centers.dim() != 2 || x.size(1) != centers.size(1)) fail(PyExc_RuntimeError, "data must be [n, d] and centers [k, d]");
     const int metric = (int)integer(a[2]);
     const int64_t rows = x.size(0), k = centers.size(0), d = x.size(1);
-    at::Tensor labels, head;
+    at::Tensor labels, head;  // the workspace starts with what the second result is
     check_status(unlocked([&] {
       c10::cuda::CUDAGuard guard(x.device());
       const cudaStream_t st = stream_of(x);
       labels = empty({rows}, at::kLong, x.device());
-      head = empty({2}, at::kInt, x.device());
       const int64_t bytes = f2c_kmeans_assign_workspace(rows, k, d);
-      at::Tensor ws;
-      if (bytes > 0) {
-        ws = empty({bytes}, at::kByte, x.device());
-        C10_CUDA_CHECK(cudaMemsetAsync(ws.data_ptr(), 0, 256, st));  // the exact scorer leaves it as it is
-      }
-      const int rc = f2c_kmeans_assign(x.const_data_ptr<float>(), centers.const_data_ptr<float>(), labels.mutable_data_ptr<int64_t>(), rows, k, d,
-                                       metric, bytes > 0 ? ws.data_ptr() : nullptr, st);
-      if (bytes > 0) C10_CUDA_CHECK(cudaMemcpyAsync(head.data_ptr(), ws.data_ptr(), 8, cudaMemcpyDeviceToDevice, st));
-      else C10_CUDA_CHECK(cudaMemsetAsync(head.data_ptr(), 0, 8, st));
-      return rc;
+      head = empty({std::max(bytes, (int64_t)8) / 4}, at::kInt, x.device());
+      if (bytes == 0) C10_CUDA_CHECK(cudaMemsetAsync(head.data_ptr(), 0, 8, st));
+      return f2c_kmeans_assign(x.const_data_ptr<float>(), centers.const_data_ptr<float>(), labels.mutable_data_ptr<int64_t>(), rows, k, d, metric,
+                               bytes > 0 ? head.data_ptr() : nullptr, st);
     }));
     PyObject* l = THPVariable_Wrap(std::move(labels));
     PyObject* h = THPVariable_Wrap(std::move(head));

@@ -293,7 +293,7 @@ int f2c_kmeans_fit_iterate(const float* x, float* centers, int64_t n, int64_t k,
                            void* workspace, void* stream);
 
 /* K-means assignment for callers that cannot allocate device memory - no counterpart in the reference.
- * Same result as f2c_kmeans_assign, but the scratch it needs is a fixed 4 MiB + 256 B array inside the library
+ * Same result as f2c_kmeans_assign, but the scratch it needs is a fixed array of 256 B inside the library
  * (present on every GPU that loads it, until exit) instead of a caller-supplied workspace, and the call itself
  * allocates nothing.  Meant for threads inside a process whose framework allocator owns nearly all of HBM, or on
  * a latency-critical path where cudaMalloc / cudaFree would stall the device.  Limits: n <= 1,048,576 points per
