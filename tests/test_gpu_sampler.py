@@ -183,6 +183,12 @@ def test_minibatch_kernel_equals_hops_one_by_one(capi, idx, picks, n_seeds):
         assert torch.equal(nodes, frontier)
 
 
+@pytest.mark.parametrize("n_seeds", [1024, 2050, 2051, 2600])
+def test_minibatch_kernel_around_the_line_of_the_first_hop(capi, n_seeds):
+    """Up to 2048 seeds every CTA scans the first hop's lists itself, more are scanned in shares (a step takes 0 to 3 seeds less)."""
+    test_minibatch_kernel_equals_hops_one_by_one(capi, torch.int64, (13, 4), n_seeds)
+
+
 def test_minibatch_kernel_rejects_ids_outside_the_graph(capi):
     from f2cgt_b200 import ops
     indptr = torch.tensor([0, 2, 3, 3], device="cuda")
