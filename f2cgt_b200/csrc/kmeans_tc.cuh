@@ -133,6 +133,7 @@ struct Params {
   int metric;
   int x_aligned;       // x starts on a 16-byte boundary
   int x_wide, y_wide;  // rows can be read as float4
+  uint32_t never;      // ~0, which the kernel does not know: see arrived()
   float eps;   // relative error bound of one score
 };
 
@@ -156,6 +157,10 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
   return r;
 }
+
+// True once `any`, a maximum over magnitudes that were read, is there: its bits are never `never`.  The compiler does not know that, so whoever
+// branches on it waits for the reads.  (any >= 0 in its place is folded to a constant, and with it goes the wait.)
+__device__ __forceinline__ bool arrived(float any, uint32_t never) { return __float_as_uint(any) != never; }
 
 __device__ __forceinline__ float sqrt_approx(float v) {
   float r;
@@ -897,9 +902,10 @@ __device__ __forceinline__ void run(const P& p) {
                             fmaxf(fabsf(v[b][6]), fabsf(v[b][7])));
               any = fmaxf(any, top[b]);
             }
-            // The slot's next copy may start when all lanes' reads have arrived, not merely been issued: the vote waits for what was read (it is always
-            // true; a barrier of the warp in its place let rows be overwritten before they were read).
-            if (__any_sync(0xffffffffu, !(any < 0.0f))) fetch(t - base + 2 * ((q + Q::slots) / L::PARTS), (q + Q::slots) % L::PARTS, slot);
+            // The slot's next copy may start when all lanes' reads have arrived, not merely been issued: every lane's vote needs what it has read
+            // (a barrier of the warp alone let rows be overwritten before they were read), and its fence puts the reads before the copy's writes.
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            if (__all_sync(0xffffffffu, arrived(any, p.never))) fetch(t - base + 2 * ((q + Q::slots) / L::PARTS), (q + Q::slots) % L::PARTS, slot);
             if (l2) {
 #pragma unroll
               for (int b = 0; b < L::READS; ++b) {
@@ -1111,6 +1117,7 @@ inline void describe(Params& p, const float* x, const float* y, int64_t n, int64
   p.x_aligned = aligned(x, 16);
   p.x_wide = d % 4 == 0;  // of the copy in shared memory
   p.y_wide = d % 4 == 0 && aligned(y, 16);
+  p.never = ~0u;
   // relative error bound of one score: the split leaves 3 * 2^-22 of |x||y|, the rest is the sums of up to 13 MMAs of 16 products
   p.eps = d <= 32 ? 1.0f / 65536.0f : 1.0f / 32768.0f;
 }
