@@ -13,7 +13,7 @@ LIB_PATH = os.environ.get("F2CGT_B200_LIB") or os.path.join(_PKG, "libf2cgt_b200
 U8, I8, I16, I32, I64, F16, F32, F64 = range(8)
 MEAN, SUM = 0, 1
 L2, COSINE = 0, 1
-SCORER_EXACT, SCORER_TENSOR = 0x100, 0x200
+SCORER_EXACT, SCORER_TENSOR, NO_WAITS = 0x100, 0x200, 0x400
 # f2c_kernel: kernel family of a fused aggregation call
 KERNELS = {"auto": 0, "stream": 1, "prefetch": 2, "general": 3, "prefetch_arith": 4}
 

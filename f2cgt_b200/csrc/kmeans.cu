@@ -170,7 +170,7 @@ int kmeans_assign_exact(const float* x, const float* y, int64_t* labels, int64_t
 bool kmeans_tc_supported(int64_t n, int64_t k, int64_t d);
 int64_t kmeans_tc_workspace();
 int kmeans_assign_tc(const float* x, const float* y, int64_t* labels, int64_t n, int64_t k, int64_t d, int metric, void* workspace,
-                     cudaStream_t st);
+                     cudaStream_t st, int flags);
 
 static int validate_km(const char* op, int64_t n, int64_t k, int64_t d, int metric) {
   F2C_REQUIRE(n >= 0 && k >= 1 && d >= 1, F2C_ERR_INVALID, "%s: bad shape n=%lld k=%lld d=%lld", op, (long long)n, (long long)k,
@@ -207,7 +207,8 @@ extern "C" int64_t f2c_kmeans_assign_workspace(int64_t n, int64_t k, int64_t d) 
 extern "C" int f2c_kmeans_assign(const float* x, const float* centers, int64_t* labels, int64_t n, int64_t k, int64_t d,
                                  int metric, void* workspace, void* stream) {
   const int scorer = metric & (F2C_SCORER_EXACT | F2C_SCORER_TENSOR);  // per-call choice of the scorer (tests, benchmarks)
-  metric &= ~(F2C_SCORER_EXACT | F2C_SCORER_TENSOR);
+  const int flags = metric & F2C_NO_WAITS;
+  metric &= ~(F2C_SCORER_EXACT | F2C_SCORER_TENSOR | F2C_NO_WAITS);
   int rc = validate_km("kmeans_assign", n, k, d, metric);
   if (rc) return rc;
   if (n == 0) return F2C_OK;
@@ -217,7 +218,7 @@ extern "C" int f2c_kmeans_assign(const float* x, const float* centers, int64_t* 
   // exact scorer 982 us, tensor cores 104)
   const bool prefer_tc = d >= 4 || scorer == F2C_SCORER_TENSOR;
   if (workspace != nullptr && kmeans_tc_supported(n, k, d) && prefer_tc && scorer != F2C_SCORER_EXACT && aligned(workspace, 16))
-    return kmeans_assign_tc(x, centers, labels, n, k, d, metric, workspace, (cudaStream_t)stream);
+    return kmeans_assign_tc(x, centers, labels, n, k, d, metric, workspace, (cudaStream_t)stream, flags);
   if (workspace != nullptr && kmeans_tc_supported(n, k, d)) {  // nothing was undecided
     const cudaError_t e = cudaMemsetAsync(workspace, 0, 8, (cudaStream_t)stream);
     if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "kmeans_assign: %s", cudaGetErrorString(e));

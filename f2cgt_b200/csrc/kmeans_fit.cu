@@ -20,7 +20,7 @@ namespace f2c {
 
 bool kmeans_tc_supported(int64_t n, int64_t k, int64_t d);
 int kmeans_fit_tc(const float* x, float* centers, int64_t n, int64_t k, int64_t d, int metric, double tol, int iterations, FitState* state, long long* sums,
-                  uint32_t* counts, const uint32_t* maxima, uint16_t* labels, double* shifts, int32_t* error, cudaStream_t st);
+                  uint32_t* counts, const uint32_t* maxima, uint16_t* labels, double* shifts, int32_t* error, cudaStream_t st, int flags);
 int kmeans_assign_exact(const float* x, const float* y, int64_t* labels, int64_t n, int64_t k, int64_t d, int metric, cudaStream_t st,
                         const int32_t* done);
 
@@ -257,6 +257,8 @@ extern "C" int f2c_kmeans_fit_iterate(const float* x, float* centers, int64_t n,
   const char* op = "kmeans_fit_iterate";
   int rc = fit::validate(op, n, k, d);
   if (rc) return rc;
+  const int flags = metric & F2C_NO_WAITS;
+  metric &= ~F2C_NO_WAITS;
   F2C_REQUIRE(metric == F2C_L2 || metric == F2C_COSINE, F2C_ERR_INVALID, "%s: unknown metric", op);
   F2C_REQUIRE(x && centers && workspace && aligned(workspace, 256) && iterations >= 0, F2C_ERR_INVALID, "%s: bad argument", op);
   cudaStream_t st = (cudaStream_t)stream;
@@ -270,7 +272,7 @@ extern "C" int f2c_kmeans_fit_iterate(const float* x, float* centers, int64_t n,
   if (kmeans_tc_supported(n, k, d) && d >= 4) {
     if (iterations == 0) return F2C_OK;
     return kmeans_fit_tc(x, centers, n, k, d, metric, tol, iterations, state, sums, counts, (const uint32_t*)(ws + w.maxima), (uint16_t*)labels,
-                         (double*)(ws + w.shifts), (int32_t*)(ws + w.assign) + 1, st);
+                         (double*)(ws + w.shifts), (int32_t*)(ws + w.assign) + 1, st, flags);
   }
   const size_t smem = (size_t)d * 8 + ((size_t)2 * k * d + k) * 4 + fit::kChunk * 2;
   const uint32_t* maxima = (const uint32_t*)(ws + w.maxima);

@@ -11,10 +11,10 @@
 namespace f2c {
 namespace tc {
 
-template <int C, int NB>
+template <int C, int NB, bool NO_WAITS = false>
 __global__ void __launch_bounds__(kThreads, 1) kmeans_fit_kernel(const __grid_constant__ FitParams p) {
   if (*(volatile const int32_t*)&p.state->done != 0) return;  // converged, or not finite
-  run<C, NB>(p);
+  run<C, NB, NO_WAITS>(p);
 }
 
 struct Kernel {
@@ -25,7 +25,8 @@ template <int C>
 static Kernel kernel_for(int64_t k) {
   return k <= 128 ? Kernel{kmeans_fit_kernel<C, 4>, Ring<C, 4>::bytes} : Kernel{kmeans_fit_kernel<C, 8>, Ring<C, 8>::bytes};
 }
-static Kernel kernel_for(int64_t k, int64_t d) {
+static Kernel kernel_for(int64_t k, int64_t d, bool no_waits) {
+  if (no_waits) return Kernel{kmeans_fit_kernel<8, 8, true>, Ring<8, 8>::bytes};  // for any number of dimensions
   switch ((d + 7) / 8) {
     case 1: return kernel_for<1>(k);
     case 2: return kernel_for<2>(k);
@@ -43,14 +44,14 @@ static Kernel kernel_for(int64_t k, int64_t d) {
 // labels: 2 n numbers; those from n on are 0xffff and sums and counts zero before the first call, and theirs from call to call.
 // shifts: one number per SM.
 int kmeans_fit_tc(const float* x, float* centers, int64_t n, int64_t k, int64_t d, int metric, double tol, int iterations, FitState* state, long long* sums,
-                  uint32_t* counts, const uint32_t* maxima, uint16_t* labels, double* shifts, int32_t* error, cudaStream_t st) {
+                  uint32_t* counts, const uint32_t* maxima, uint16_t* labels, double* shifts, int32_t* error, cudaStream_t st, int flags) {
   const char* op = "kmeans_fit_iterate";
   tc::FitParams p{};
   tc::describe(p, x, centers, n, k, d, metric);
   p.error = error;
   p.state = state; p.centers = centers; p.labels16 = labels; p.summed16 = labels + n; p.sums = sums; p.counts = counts; p.maxima = maxima;
   p.shifts = shifts; p.iterations = iterations; p.tol = tol;
-  auto [kern, smem] = tc::kernel_for(k, d);
+  auto [kern, smem] = tc::kernel_for(k, d, (flags & F2C_NO_WAITS) != 0);
   if (smem < tc::kOneCta) smem = tc::kOneCta;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "%s: %s", op, cudaGetErrorString(e));

@@ -7,11 +7,11 @@ namespace f2c {
 
 namespace tc {
 
-template <int C, int NB>
+template <int C, int NB, bool NO_WAITS = false>
 __global__ void __launch_bounds__(kThreads, 1) kmeans_tc_kernel(const __grid_constant__ Params p) {
   dependency_wait();
   release_dependents();
-  run<C, NB>(p);
+  run<C, NB, NO_WAITS>(p);
 }
 
 struct Kernel {
@@ -22,7 +22,8 @@ template <int C>
 static Kernel kernel_for(int64_t k) {
   return k <= 128 ? Kernel{kmeans_tc_kernel<C, 4>, Ring<C, 4>::bytes} : Kernel{kmeans_tc_kernel<C, 8>, Ring<C, 8>::bytes};
 }
-static Kernel kernel_for(int64_t k, int64_t d) {
+static Kernel kernel_for(int64_t k, int64_t d, bool no_waits) {
+  if (no_waits) return Kernel{kmeans_tc_kernel<8, 8, true>, Ring<8, 8>::bytes};  // for any number of dimensions
   switch ((d + 7) / 8) {
     case 1: return kernel_for<1>(k);
     case 2: return kernel_for<2>(k);
@@ -43,7 +44,7 @@ constexpr int64_t kTcWorkspace = 256;  // [points that the exact scorer assigned
 int64_t kmeans_tc_workspace() { return kTcWorkspace; }
 
 int kmeans_assign_tc(const float* x, const float* y, int64_t* labels, int64_t n, int64_t k, int64_t d, int metric, void* workspace,
-                     cudaStream_t st) {
+                     cudaStream_t st, int flags) {
   tc::Params p{};
   tc::describe(p, x, y, n, k, d, metric);
   p.labels = labels;
@@ -51,7 +52,7 @@ int kmeans_assign_tc(const float* x, const float* y, int64_t* labels, int64_t n,
   p.undecided = head; p.error = head + 1;
   cudaError_t e = cudaMemsetAsync(head, 0, 8, st);
   if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "kmeans_assign: %s", cudaGetErrorString(e));
-  auto [kern, smem] = tc::kernel_for(k, d);
+  auto [kern, smem] = tc::kernel_for(k, d, (flags & F2C_NO_WAITS) != 0);
   if (smem < tc::kOneCta) smem = tc::kOneCta;
   e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "kmeans_assign: %s", cudaGetErrorString(e));
@@ -117,7 +118,7 @@ extern "C" int f2c_kmeans_assign_static(const float* x, const float* centers, in
   int rc = tc::static_scratch(op, &scratch);
   if (rc) return rc;
   // same kernels as kmeans_assign; the header (count, error code) is cleared inside
-  return kmeans_assign_tc(x, centers, labels, n, k, d, metric, scratch, (cudaStream_t)stream);
+  return kmeans_assign_tc(x, centers, labels, n, k, d, metric, scratch, (cudaStream_t)stream, 0);
 }
 
 // What the last f2c_kmeans_assign_static call on the current device left in the header of the built-in array: the

@@ -32,8 +32,9 @@
 //    -> 157, 64: 400 -> 305; 100 centres of 8 dimensions 118 -> 72, of 64: 357 -> 229.  Two epilogue groups instead of three: 8 dimensions 107.
 //    Few points: 5000 x 8 20 -> 11, 40,000 x 8 20 -> 12.5, 149,000 x 32 37 -> 26 (without the second kernel, its list and the clearing of it;
 //    with them 20, 18 and 28), 149,000 x 64 47 -> 48.
-//    Every wait on an mbarrier is bounded; on expiry an error code is recorded, which makes the exact scorer assign every point, no further
-//    wait is made and no copy started, and the CTA frees its TMEM at the common exit once its own copies and MMAs are complete.
+//    Every wait on an mbarrier is bounded; on expiry an error code is recorded, no further wait is made and no copy started, and the exact
+//    scorer assigns all points of the CTA.  Rows that were asked for may still arrive then, so it works where no copy is aimed, over the operands.
+//    The copies and MMAs are waited for at the common exit, in front of the freeing of the TMEM.
 #pragma once
 #include <cooperative_groups.h>
 #include <cuda_fp16.h>
@@ -246,6 +247,9 @@ struct Ring {
 
 // ---------------------------------------------------------------- points that the tensor cores leave undecided
 // Shared memory, behind the assignment, of a list of undecided points (numbered inside the CTA: 128 * tile + row) and of their labels.
+// Bytes of what the second half of an assignment, or of a Lloyd iteration, keeps in shared memory beside the centres.
+template <int C>
+constexpr size_t kListsPlace = 20480 + 1024 * C;
 constexpr int kFew = 8;     // points up to which the centres are not staged for them
 constexpr int kMany = 400;  // points from which on a thread scores one
 struct Scores {
@@ -397,15 +401,15 @@ __device__ __noinline__ void score_exactly(const Params& p, const uint32_t* list
   __syncthreads();
 }
 
-// What an assignment does with its undecided points: the CTA's list holds the first kList of them; if there are more, or a wait has run out,
+// What an assignment does with its undecided points: the CTA's list holds the first kList of them; if there are more, or a wait has run out (lost),
 // they are found by their labels, -1, and scored as many at a time as there are threads.
 template <int C>
-__device__ __noinline__ void settle(const Params& p, int turns, bool all, const uint32_t* open_list, uint32_t* counter, unsigned char* a_ring, unsigned char* rows) {
+__device__ __noinline__ void settle(const Params& p, int turns, bool lost, const uint32_t* open_list, uint32_t* counter, unsigned char* a_ring, unsigned char* rows) {
   Scores* scores = reinterpret_cast<Scores*>(rows);
   uint32_t* list = reinterpret_cast<uint32_t*>(scores + 1);  // [2 * kThreads]
   float* points = reinterpret_cast<float*>(list + 2 * kThreads);
-  static_assert(sizeof(Scores) % 16 == 0 && kThreads <= kList && sizeof(Scores) + 8 * kThreads + kThreads / 32 * 8 * C * 4 <= kProducerWarps * Ring<C, 4>::slots * Lanes<C>::PART_BYTES,
-                "fits the rows' place");
+  static_assert(sizeof(Scores) % 16 == 0 && kThreads <= kList && sizeof(Scores) + 8 * kThreads + kThreads / 32 * 8 * C * 4 <= kListsPlace<C>,
+                "fits");
   const int tid = threadIdx.x;
   const uint32_t open = *counter;
   bool staged = false;
@@ -416,7 +420,7 @@ __device__ __noinline__ void settle(const Params& p, int turns, bool all, const 
     __syncthreads();
   };
   uint32_t total = open;
-  if (!all && open <= (uint32_t)kList) {
+  if (!lost && open <= (uint32_t)kList) {
     if (open == 0u) return;
     score(open_list, (int)open);
   } else {
@@ -427,7 +431,7 @@ __device__ __noinline__ void settle(const Params& p, int turns, bool all, const 
       __syncthreads();
       const uint32_t at = (uint32_t)(first + tid);
       const int64_t i = index_of(at);
-      if (first + tid < turns * kTileM && i < p.n && (all || __ldcg(p.labels + i) < 0)) list[atomicAdd(counter, 1u)] = at;
+      if (first + tid < turns * kTileM && i < p.n && (lost || __ldcg(p.labels + i) < 0)) list[atomicAdd(counter, 1u)] = at;
       __syncthreads();
       int count = (int)*counter;
       const bool last = first + kThreads >= turns * kTileM;
@@ -450,15 +454,16 @@ __device__ __noinline__ void settle(const Params& p, int turns, bool all, const 
 
 // ---------------------------------------------------------------- the second half of a Lloyd iteration
 // Behind the labels of this CTA's points: those that are still undecided, the clusters' sums, and, all CTAs together, the new centres.
-// Returns whether the fit has converged.  `number`: of this iteration; `all`: score every point exactly.  a_ring, rows: shared memory that
-// the assignment has done with.
+// Returns whether the fit has converged.  `number`: of this iteration; a_ring, rows: shared memory that the assignment has done with; `instead`: if
+// not null, a wait of this CTA has run out and this is where nothing may still arrive.
 //  * The sums are integers and exact, so they are kept from iteration to iteration, and only points that have changed their cluster are
 //    taken off one sum and added to another.  From the second iteration on these are few: an iteration of 149,000 x 32 that added up
 //    everything anew took 40 us, 35 with this (a 64-bit reduction per cluster, column and CTA; L2 does about a hundred of them a cycle).
 //  * A CTA sorts its changes by cluster (a counting sort of up to 1024 points' at a time), and 8, 16 or 32 lanes walk a part of them, hold
 //    their columns' sums in registers and add them to the global ones where the cluster changes.
 template <int C>
-__device__ __noinline__ bool end_of_iteration(const FitParams& p, int number, int turns, bool lost, unsigned char* a_ring, unsigned char* rows) {
+__device__ __noinline__ bool end_of_iteration(const FitParams& p, int number, int turns, unsigned char* instead, unsigned char* a_ring, unsigned char* rows) {
+  if (instead != nullptr) { rows = instead; a_ring = instead + kListsPlace<C>; }
   namespace cg = cooperative_groups;
   constexpr int DP = 8 * C, kWarps = kThreads / 32;
   constexpr int kChunkTiles = 8, kChunk = kChunkTiles * kTileM, kShares = (kChunk / 32 + kWarps - 1) / kWarps;
@@ -470,11 +475,10 @@ __device__ __noinline__ bool end_of_iteration(const FitParams& p, int number, in
   int32_t* gained = reinterpret_cast<int32_t*>(start + kMaxN + 4);
   float* point = reinterpret_cast<float*>(gained + kMaxN);  // one per warp
   double* part = reinterpret_cast<double*>(point + kWarps * DP);
-  static_assert((4 * kChunk + 3 * kMaxN + 4 + kWarps * DP + 2 * kWarps) * 4 <= kProducerWarps * Ring<C, 4>::slots * Lanes<C>::PART_BYTES &&
-                    (4 * kChunk + 3 * kMaxN + 4 + kWarps * DP + 2 * kWarps) * 4 <= kProducerWarps * Ring<C, 8>::slots * Lanes<C>::PART_BYTES, "fits the rows' place");
+  static_assert((4 * kChunk + 3 * kMaxN + 4 + kWarps * DP + 2 * kWarps) * 4 <= kListsPlace<C>, "fits");
   static_assert(kMaxN * (DP + 5) * 4 <= Ring<C, 8>::stages * Operands<C>::a_chunks * (kTileM * 16 + Lanes<C>::PAD), "fits the A ring's place");
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const bool all = lost || *(volatile const int32_t*)p.error != 0;
+  const bool all = instead != nullptr || *(volatile const int32_t*)p.error != 0;  // a wait has run out, here or in another CTA: score every point exactly
   auto index_of = [&](int t, int row) { return ((int64_t)blockIdx.x + (int64_t)t * gridDim.x) * kTileM + row; };
   bool staged = false;
   const int bits = fraction_bits(p.n);
@@ -679,9 +683,10 @@ __device__ __noinline__ bool end_of_iteration(const FitParams& p, int number, in
 
 // Shared memory: [B tile][A ring][rows in flight][norms 256 floats][bounds kBoundRing x 128 floats][mbarriers, tmem slot, count and list of undecided points]
 // C: chunks of eight dimensions of a row (1 to 8); NB: blocks of 32 columns (4: up to 128 centres, 8: up to 256).
+// NO_WAITS: every wait runs out at once, for tests of what follows.
 // P = Params: one assignment.  FitParams: Lloyd iterations, by CTAs that are all resident (kmeans_fit_tc.cu); tiles are then counted on
 // from iteration to iteration, so that the barriers' phases go on.
-template <int C, int NB, typename P>
+template <int C, int NB, bool NO_WAITS, typename P>
 __device__ __forceinline__ void run(const P& p) {
   constexpr bool FIT = std::is_same<P, FitParams>::value;
   using L = Lanes<C>;
@@ -864,7 +869,10 @@ __device__ __forceinline__ void run(const P& p) {
       // Tile t's columns 128 h .. 128 h + 127 are in accumulator (t, h) of four.
       auto accumulator = [](int t, int h) { return 2 * (t & 1) + (NB == 8 ? h : (t >> 1) & 1); };
 
-      if (producer) {
+      if constexpr (NO_WAITS) {  // the first rows are on their way
+        wait.gave_up = true;
+        if (threadIdx.x == 0) atomicExch(p.error, 1);
+      } else if (producer) {
         const float eps = 2.0f * cmax * (bad_centres ? INFINITY : p.eps);  // what two scores may be off by together, per |x|
         for (int t = base + ((group ^ base) & 1); t < base + turns; t += 2) {
           unsigned char* a_tile = a_ring + (size_t)(t % Q::stages) * a_bytes;
@@ -1081,12 +1089,15 @@ __device__ __forceinline__ void run(const P& p) {
         }
       }
     }
+    // Behind a wait that has run out copies may still arrive in `rows`, and MMAs still read the operands: the second half's lists and centres
+    // lie over the operands then, which are not used again.
+    lost = __syncthreads_or(wait.gave_up) != 0;
+    constexpr size_t place = kListsPlace<C>;
+    static_assert(place + N * (8 * C + 5) * 4 <= O::b_chunks * lbo_b + Q::stages * a_bytes && place <= kProducerWarps * Q::slots * L::PART_BYTES, "room in both places");
     if constexpr (FIT) {
-      lost = __syncthreads_or(wait.gave_up) != 0;
-      if (end_of_iteration<C>(p, done_before + it, turns, lost, a_ring, rows)) break;
+      if (end_of_iteration<C>(p, done_before + it, turns, lost ? smem : nullptr, a_ring, rows)) break;
     } else {
-      lost = __syncthreads_or(wait.gave_up) != 0;
-      settle<C>(p, turns, lost, open_list, open_count, a_ring, rows);
+      settle<C>(p, turns, lost, open_list, open_count, lost ? smem + place : a_ring, lost ? smem : rows);
     }
   }
 

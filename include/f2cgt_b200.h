@@ -44,6 +44,9 @@ typedef enum { F2C_L2 = 0, F2C_COSINE = 1 } f2c_metric;  /* src/kmeans.cu:16-22,
  * without one the library picks by shape.  Both give the same labels. */
 #define F2C_SCORER_EXACT 0x100   /* fp32 FMA scorer */
 #define F2C_SCORER_TENSOR 0x200  /* tcgen05 scorer + exact re-score of undecided points (needs a workspace) */
+/* f2c_kmeans_assign and f2c_kmeans_fit_iterate: every bounded wait of the tensor-core kernel runs out at once.  Same results; for
+ * tests of what follows a wait that has run out. */
+#define F2C_NO_WAITS 0x400
 
 typedef enum {
   F2C_OK = 0,

@@ -151,7 +151,7 @@ def test_fit_iterations_equal_the_restated_loop(capi, metric, n, k, d):
         assert torch.equal(got, again.get_centers())
 
 
-def _fit(x, centers, iterations, spoil=False, each=None):
+def _fit(x, centers, iterations, spoil=False, each=None, metric=0):
     """Lloyd iterations by the C entry points, queued at once or (each) one call after the other; centres and state words."""
     from f2cgt_b200 import ops
     from f2cgt_b200._lib import check, lib
@@ -164,7 +164,7 @@ def _fit(x, centers, iterations, spoil=False, each=None):
     for take in each or [iterations]:
         if spoil:
             head[1] = 3
-        check(lib.f2c_kmeans_fit_iterate(x.data_ptr(), centers.data_ptr(), n, k, d, 0, 0.0, take, ws.data_ptr(), ops._stream(x)))
+        check(lib.f2c_kmeans_fit_iterate(x.data_ptr(), centers.data_ptr(), n, k, d, metric, 0.0, take, ws.data_ptr(), ops._stream(x)))
         if each:
             torch.cuda.synchronize()
     return centers, ws[:16].view(torch.int32).tolist()
@@ -179,6 +179,26 @@ def test_fit_goes_on_after_an_assignment_whose_wait_ran_out(capi):
     got, spoiled = _fit(x, x[:64].clone(), 6, spoil=True)
     assert spoiled[:3] == words[:3]
     assert spoiled[3] == 3 and torch.equal(want, got)
+
+
+@pytest.mark.parametrize("n,k,d", [(1, 1, 4), (129, 100, 8), (40_000, 256, 13), (70_001, 200, 64)])
+def test_a_lost_wait_leaves_the_exact_labels_and_sums(capi, n, k, d):
+    """Every bounded wait of the tensor-core kernel runs out at once, with the first rows on their way into shared memory: the error word says
+    so, all points have the exact scorer's labels, and a fit ends at the centres, bit for bit, of one without such waits."""
+    from f2cgt_b200 import _lib, _native, ops
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn(n, d, generator=g, device="cuda")
+    c = torch.randn(k, d, generator=g, device="cuda")
+    x[::5] = 0
+    for metric in ("l2", "cosine"):
+        flags = ops._metric(metric) | _lib.SCORER_TENSOR
+        labels, head = _native.kmeans_assign(x, c, flags | _lib.NO_WAITS)
+        assert torch.equal(labels, ops.kmeans_assign(x, c, metric, scorer="exact"))
+        assert head[:2].tolist() == [n, 1]
+        assert torch.equal(_native.kmeans_assign(x, c, flags)[0], labels)  # and the next call finds the device as it was
+        want, words = _fit(x, c.clone(), 4, metric=ops._metric(metric))
+        got, lost = _fit(x, c.clone(), 4, each=[1, 3], metric=ops._metric(metric) | _lib.NO_WAITS)
+        assert torch.equal(want, got) and lost[:3] == words[:3] and words[3] == 0 and lost[3] == 1
 
 
 def test_iterations_in_a_row_equal_iterations_one_by_one(capi):
