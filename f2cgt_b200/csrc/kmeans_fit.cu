@@ -211,7 +211,7 @@ static Layout plan(int64_t n, int64_t k, int64_t d) {
   w.labels = at; at += up((size_t)n * 8);
   w.assign = at; at += 256;  // second word: code of a bounded wait of the tensor-core kernel that ran out
   w.maxima = at; at += up((size_t)d * 4);
-  w.shifts = at; at += up((size_t)current_sm_count() * 8);
+  w.shifts = at; at += up((size_t)kFitMaxCtas * 8);
   w.total = at;
   return w;
 }

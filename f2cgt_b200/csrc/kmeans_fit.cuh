@@ -21,6 +21,8 @@ struct FitState {       // first 256 bytes of the workspace; the host reads the 
   double shift;
 };
 
+constexpr int kFitMaxCtas = 256;  // of the cooperative kernel: what a workspace has room for, whatever device was current when its size was asked for
+
 // Sums are exact and independent of the order of the additions: a value becomes a fixed-point integer, this many bits below the largest
 // magnitude of its column, and integers commute.
 __device__ __forceinline__ int fraction_bits(int64_t n) {

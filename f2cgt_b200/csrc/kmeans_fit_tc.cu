@@ -42,7 +42,7 @@ static Kernel kernel_for(int64_t k, int64_t d, bool no_waits) {
 }  // namespace tc
 
 // labels: 2 n numbers; those from n on are 0xffff and sums and counts zero before the first call, and theirs from call to call.
-// shifts: one number per SM.
+// shifts: one number per CTA, kFitMaxCtas at most.
 int kmeans_fit_tc(const float* x, float* centers, int64_t n, int64_t k, int64_t d, int metric, double tol, int iterations, FitState* state, long long* sums,
                   uint32_t* counts, const uint32_t* maxima, uint16_t* labels, double* shifts, int32_t* error, cudaStream_t st, int flags) {
   const char* op = "kmeans_fit_iterate";
@@ -57,6 +57,7 @@ int kmeans_fit_tc(const float* x, float* centers, int64_t n, int64_t k, int64_t 
   if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "%s: %s", op, cudaGetErrorString(e));
   int64_t grid = ceil_div(n, tc::kTileM);
   if (grid > current_sm_count()) grid = current_sm_count();
+  if (grid > kFitMaxCtas) grid = kFitMaxCtas;
   void* args[] = {(void*)&p};
   e = cudaLaunchCooperativeKernel((const void*)kern, dim3((unsigned)grid), dim3(tc::kThreads), args, smem, st);
   if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "%s: cooperative launch: %s", op, cudaGetErrorString(e));

@@ -46,12 +46,12 @@ def _iterate(x, centers, metric, max_iter, tol):
         raise RuntimeError("data must be [n, d] and centers [k, d]")
     n, d = x.shape
     k = centers.shape[0]
-    ws = torch.empty((lib.f2c_kmeans_fit_workspace(n, k, d),), dtype=torch.uint8, device=x.device)
-    words = ws[:16].view(torch.int32)
     seen = [(torch.empty(4, dtype=torch.int32, pin_memory=True), torch.cuda.Event()) for _ in range(2)]
     stream = torch.cuda.current_stream(x.device)
     queued = rounds = 0
     with ops._on(x):
+        ws = torch.empty((lib.f2c_kmeans_fit_workspace(n, k, d),), dtype=torch.uint8, device=x.device)
+        words = ws[:16].view(torch.int32)
         check(lib.f2c_kmeans_fit_begin(x.data_ptr(), n, k, d, ws.data_ptr(), stream.cuda_stream))
         while True:
             take = min(_AHEAD, max_iter - queued)

@@ -31,6 +31,12 @@ def test_library_exports_every_declared_symbol():
         assert name in _lib.SIGNATURES, f"{name} has no ctypes signature"
 
 
+def test_fit_workspace_does_not_depend_on_the_current_device():
+    # 256 bytes each of state, sums, counts, labels, error words and maxima, and a number for every CTA that a fit may have on any device
+    from f2cgt_b200 import _lib
+    assert _lib.lib.f2c_kmeans_fit_workspace(1, 1, 4) == 6 * 256 + 256 * 8
+
+
 def test_argument_validation_needs_no_gpu():
     # bad arguments are rejected before any CUDA call, so this runs on a CPU-only machine
     from f2cgt_b200 import _lib
