@@ -54,6 +54,7 @@ constexpr int kEpilogueGroups = 3, kEpilogueWarps = 4 * kEpilogueGroups, kProduc
 constexpr int kMmaWarp = kEpilogueWarps + kProducerWarps, kMmaWarps = 2;  // one per pair of accumulators of 128 columns
 constexpr int kThreads = 32 * (kMmaWarp + kMmaWarps);
 constexpr int kList = 1024;    // undecided points that a CTA keeps in shared memory
+constexpr float kTiny = 0x1p-100f;  // squared lengths below: the exact scorer's products run out of exponent, and a score says nothing of its labels
 constexpr int kBoundRing = 8;  // tiles whose error bounds are kept; more than the A ring and the two accumulators hold together
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -806,16 +807,20 @@ __device__ __forceinline__ void run(const P& p) {
         }
       }
       __syncthreads();
-      // largest centre norm (scale and tolerance of the L2 score); a non-finite centre sends every point to the exact scorer
+      // largest centre norm (scale and tolerance of the L2 score); a centre that is not finite or (cosine; squared L2: all of them) so short that its
+      // squared length has lost bits sends every point to the exact scorer
       float cmax = 0.0f, poison = 0.0f;
 #pragma unroll
-      for (int c = lane; c < N; c += 32) { cmax = fmaxf(cmax, norms[c]); poison = fmaf(norms[c], 0.0f, poison); }  // inf, NaN -> NaN
+      for (int c = lane; c < N; c += 32) {
+        cmax = fmaxf(cmax, norms[c]);
+        poison = fmaf(norms[c], !l2 && norms[c] > 0.0f && norms[c] < kTiny ? INFINITY : 0.0f, poison);  // inf, NaN -> NaN
+      }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
         cmax = fmaxf(cmax, __shfl_xor_sync(0xffffffffu, cmax, o));
         poison += __shfl_xor_sync(0xffffffffu, poison, o);
       }
-      const bool bad_centres = !(poison == 0.0f);
+      const bool bad_centres = !(poison == 0.0f) || (l2 && cmax < kTiny);
       const int e_y = l2 ? max(-120, min(120, exponent_above(sqrtf(cmax)))) : 0;  // squared L2: everything times 2^-e_y
       const float scale_y = power2f(-e_y);
       cmax = l2 ? sqrtf(cmax) * scale_y : 1.0f;
@@ -960,9 +965,11 @@ __device__ __forceinline__ void run(const P& p) {
             const int row = (warp & 3) * 32 + q * L::ROWS + chunk_l * L::R + row_l;
             const float floor = 2.0f * cmax * (l2 ? fmaxf(0x1p-19f * own_factor, 0x1p-126f) : 0x1p-21f);  // f16 at its lower end, and the norm term
             const float unscale = __int_as_float((254 << 23) - __float_as_int(own_factor)) * power2f(e_y);  // 1 / all that x was multiplied with
-            // INFINITY for NaN, and for a point whose |x|^2 is more than fp32 holds: the exact scorer's distance says so
+            const float length2 = own_sum * unscale * unscale;  // |x|^2
+            // INFINITY for NaN, for a point whose |x|^2 is more than fp32 holds, and for one whose |x|^2 is next to nothing under the cosine metric (the
+            // exact scorer takes 0 for it, all distances are 1 then): the exact scorer's distance says so
             // (-1 for a row of zeros under the cosine metric: all its distances are 1, its label is 0)
-            const float bound = !l2 && own_sum == 0.0f ? -1.0f : own_sum * unscale * unscale < INFINITY ? fminf(fmaf(eps, sqrt_approx(own_sum), floor), INFINITY) : INFINITY;
+            const float bound = !l2 && own_sum == 0.0f ? -1.0f : length2 < INFINITY && (l2 || length2 >= kTiny) ? fminf(fmaf(eps, sqrt_approx(own_sum), floor), INFINITY) : INFINITY;
             if (chunk_l < L::READS) {
               bounds[(t & (kBoundRing - 1)) * kTileM + row] = bound;
               if (l2) {

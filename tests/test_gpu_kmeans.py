@@ -245,6 +245,25 @@ def test_tensor_core_assignment_at_the_edges_of_its_tiles(capi, d):
                     assert torch.equal(ops.kmeans_assign(y, c, metric, scorer="tensor"), exact), (n, k, metric, size)
 
 
+@pytest.mark.parametrize("d", [5, 8, 32, 64])
+def test_rows_and_centres_whose_squared_length_underflows(capi, d):
+    """fp32 holds no square below 1.4e-45: the exact scorer gives short rows label 0 (all cosine distances are 1, all squared ones 0) and loses bits
+    before that.  The tensor cores, which scale their operands, must not know better; nor where half the rows or one centre are that short."""
+    from f2cgt_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(d)
+    x = torch.randn(3001, d, device="cuda", generator=g)
+    c = torch.randn(100, d, device="cuda", generator=g)
+    x[7], c[7] = 0, 0
+    for size in (1e-14, 1e-17, 1e-20, 1e-22, 1e-30, 1e-41):
+        tiny, mixed, one = x * size, x.clone(), c.clone()
+        mixed[::2] *= size
+        one[11] *= size
+        for metric in ("l2", "cosine"):
+            for data, centres in ((tiny, c), (mixed, c), (x, one), (tiny, c * size), (tiny, one), (mixed, one)):
+                exact = ops.kmeans_assign(data, centres, metric, scorer="exact")
+                assert torch.equal(ops.kmeans_assign(data, centres, metric, scorer="tensor"), exact), (size, metric)
+
+
 @pytest.mark.parametrize("n,k,d", [(1, 1, 4), (127, 128, 8), (1025, 129, 24), (70_000, 256, 13), (200_003, 33, 64), (40_000, 200, 40)])
 def test_fit_kernel_at_the_edges_of_its_tiles(capi, n, k, d):
     """Ragged tiles, one to many chunks of points per CTA, many points that the tensor cores leave open (every second centre is a copy,
