@@ -264,6 +264,26 @@ def test_rows_and_centres_whose_squared_length_underflows(capi, d):
                 assert torch.equal(ops.kmeans_assign(data, centres, metric, scorer="tensor"), exact), (size, metric)
 
 
+@pytest.mark.parametrize("d,k", [(8, 40), (40, 200)])
+@pytest.mark.parametrize("twins", [1.0, 0.5])
+def test_more_undecided_points_than_a_cta_lists(capi, d, k, twins):
+    """A CTA lists 1024 undecided points and finds them by their labels when there are more, as many at a time as it has threads: all of its 1536
+    points and more are undecided here (every centre has a twin: whole rounds), or about half of 5120 (the rest of a round moves on)."""
+    from f2cgt_b200 import ops
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n = sms * 128 * (12 if twins == 1.0 else 40) + 77
+    g = torch.Generator(device="cuda").manual_seed(d)
+    x = torch.randn(n, d, device="cuda", generator=g)
+    c = torch.randn(k, d, device="cuda", generator=g)
+    own = int(k / 2 if twins == 1.0 else k * twins / (1 + twins))
+    c[k - own:] = c[:own]
+    for metric in ("l2", "cosine"):
+        labels = ops.kmeans_assign(x, c, metric, scorer="tensor")
+        undecided = ops.kmeans_assign.last_undecided
+        assert torch.equal(labels, ops.kmeans_assign(x, c, metric, scorer="exact"))
+        assert undecided == n if twins == 1.0 else 1400 * sms < undecided < n - 704 * sms
+
+
 @pytest.mark.parametrize("n,k,d", [(1, 1, 4), (127, 128, 8), (1025, 129, 24), (70_000, 256, 13), (200_003, 33, 64), (40_000, 200, 40)])
 def test_fit_kernel_at_the_edges_of_its_tiles(capi, n, k, d):
     """Ragged tiles, one to many chunks of points per CTA, many points that the tensor cores leave open (every second centre is a copy,
