@@ -50,7 +50,7 @@ int kmeans_fit_tc(const float* x, float* centers, int64_t n, int64_t k, int64_t 
   tc::describe(p, x, centers, n, k, d, metric);
   p.error = error;
   p.state = state; p.centers = centers; p.labels16 = labels; p.summed16 = labels + n; p.sums = sums; p.counts = counts; p.maxima = maxima;
-  p.shifts = shifts; p.iterations = iterations; p.tol = tol;
+  p.shifts = shifts; p.tol = tol;
   auto [kern, smem] = tc::kernel_for(k, d, (flags & F2C_NO_WAITS) != 0);
   if (smem < tc::kOneCta) smem = tc::kOneCta;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -59,8 +59,15 @@ int kmeans_fit_tc(const float* x, float* centers, int64_t n, int64_t k, int64_t 
   if (grid > current_sm_count()) grid = current_sm_count();
   if (grid > kFitMaxCtas) grid = kFitMaxCtas;
   void* args[] = {(void*)&p};
-  e = cudaLaunchCooperativeKernel((const void*)kern, dim3((unsigned)grid), dim3(tc::kThreads), args, smem, st);
-  if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "%s: cooperative launch: %s", op, cudaGetErrorString(e));
+  // A launch takes every SM, registers and all, so that kernels of other streams wait for its end: it has as many iterations as take about a
+  // millisecond, one at least (2,449,029 x 32: 3 of 280 us; 149,000 x 32, 32 us each: all that are queued at a time).
+  const int64_t most = (1ll << 28) / (n * (d < 16 ? 16 : d));
+  while (iterations > 0) {
+    p.iterations = most < 1 ? 1 : most < iterations ? (int)most : iterations;
+    e = cudaLaunchCooperativeKernel((const void*)kern, dim3((unsigned)grid), dim3(tc::kThreads), args, smem, st);
+    if (e != cudaSuccess) return set_error(F2C_ERR_CUDA, "%s: cooperative launch: %s", op, cudaGetErrorString(e));
+    iterations -= p.iterations;
+  }
   return check_launch(op);
 }
 

@@ -211,6 +211,27 @@ def test_iterations_in_a_row_equal_iterations_one_by_one(capi):
         assert torch.equal(a, b) and w1 == w2
 
 
+def test_a_launch_of_a_large_fit_has_few_iterations(capi):
+    """Other streams' kernels get in between: 3,000,000 points have five iterations per launch, so seven are two launches (or seven, one by one)."""
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x = torch.randn(3_000_000, 8, generator=g, device="cuda")
+    a, w1 = _fit(x, x[:100].clone(), 7)
+    b, w2 = _fit(x, x[:100].clone(), 0, each=[1] * 7)
+    assert torch.equal(a, b) and w1 == w2 and w1[:2] == [0, 7]
+    import ctypes
+    from f2cgt_b200._lib import check, lib
+    rt = ctypes.CDLL("libcudart.so.12")  # torch's: the launches of a call are the nodes of its capture
+    ws = torch.empty(lib.f2c_kmeans_fit_workspace(x.shape[0], 100, 8), dtype=torch.uint8, device="cuda")
+    stream, graph, launches = torch.cuda.Stream(), ctypes.c_void_p(), ctypes.c_size_t()
+    handle = ctypes.c_void_p(stream.cuda_stream)
+    assert rt.cudaStreamBeginCapture(handle, 2) == 0
+    rc = lib.f2c_kmeans_fit_iterate(x.data_ptr(), a.data_ptr(), x.shape[0], 100, 8, 0, 0.0, 7, ws.data_ptr(), stream.cuda_stream)
+    assert rt.cudaStreamEndCapture(handle, ctypes.byref(graph)) == 0
+    check(rc)
+    assert rt.cudaGraphGetNodes(graph, None, ctypes.byref(launches)) == 0 and rt.cudaGraphDestroy(graph) == 0
+    assert launches.value == 2
+
+
 @pytest.mark.parametrize("n,k,d", [(5000, 8, 5), (40_000, 16, 64), (3000, 4, 300), (700, 2, 5000)])
 def test_fit_keeps_the_precision_of_small_columns(capi, n, k, d):
     """Columns of very different sizes: a centre's entries are as precise as fp32 in each of them (exact sums, one rounding to float32,
