@@ -18,22 +18,13 @@ struct Kernel {
   void (*kern)(const Params);
   size_t smem;
 };
-template <int C>
-static Kernel kernel_for(int64_t k) {
-  return k <= 128 ? Kernel{kmeans_tc_kernel<C, 4>, Ring<C, 4>::bytes} : Kernel{kmeans_tc_kernel<C, 8>, Ring<C, 8>::bytes};
-}
+struct Kernels {
+  template <int C, int NB>
+  static Kernel of() { return {kmeans_tc_kernel<C, NB>, Ring<C, NB>::bytes}; }
+};
 static Kernel kernel_for(int64_t k, int64_t d, bool no_waits) {
-  if (no_waits) return Kernel{kmeans_tc_kernel<8, 8, true>, Ring<8, 8>::bytes};  // for any number of dimensions
-  switch ((d + 7) / 8) {
-    case 1: return kernel_for<1>(k);
-    case 2: return kernel_for<2>(k);
-    case 3: return kernel_for<3>(k);
-    case 4: return kernel_for<4>(k);
-    case 5: return kernel_for<5>(k);
-    case 6: return kernel_for<6>(k);
-    case 7: return kernel_for<7>(k);
-    default: return kernel_for<8>(k);
-  }
+  if (no_waits) return {kmeans_tc_kernel<8, 8, true>, Ring<8, 8>::bytes};  // for any number of dimensions
+  return kernel_for<Kernels>(k, d);
 }
 
 }  // namespace tc
@@ -108,7 +99,7 @@ extern "C" int f2c_kmeans_assign_static(const float* x, const float* centers, in
               (long long)d);
   F2C_REQUIRE(metric == F2C_L2 || metric == F2C_COSINE, F2C_ERR_INVALID, "%s: unknown metric", op);
   F2C_REQUIRE(n <= tc::kStaticMaxPoints, F2C_ERR_LIMIT,
-              "%s: %lld points exceed the %lld the built-in scratch holds; split the call or use kmeans_assign with a workspace", op,
+              "%s: %lld points exceed the %lld of one call; split it or use kmeans_assign with a workspace", op,
               (long long)n, (long long)tc::kStaticMaxPoints);
   F2C_REQUIRE(k <= tc::kMaxN && d <= 64, F2C_ERR_LIMIT, "%s: at most %d centres of at most 64 dimensions", op, tc::kMaxN);
   if (n == 0) return F2C_OK;

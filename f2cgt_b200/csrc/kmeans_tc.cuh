@@ -18,8 +18,9 @@
 //    arg-max.  A column that is padding carries -65504 in that chunk.
 //  * The epilogue reads the 128 x 256 scores with tcgen05.ld (one point per thread) and finds the best score and whether it is
 //    the only one within the error bound of the product.  A point where it is not goes to a list of the CTA, whose warps give it
-//    the label of the exact fp32 scorer (kmeans.cu) at the end, so every label equals the label of that kernel.  (Squared distances of points that lie some 10^3 times further out than the centres differ by less than their
-//    own fp32 rounding; there the score, which leaves |x|^2 out, still decides, for the nearer centre.)
+//    the label of the exact fp32 scorer (kmeans.cu) at the end, so every label equals the label of that kernel.  (Squared distances of points
+//    that lie some 10^3 times further out than the centres differ by less than their own fp32 rounding; there the score, which leaves |x|^2
+//    out, still decides, for the nearer centre.)
 //  * Overlap.  A CTA has 22 warps with fixed roles: three groups of four epilogue warps, two of four producer warps, which have their
 //    points' rows copied to shared memory ahead, split them and store them into a ring of A tiles, and two warps whose first lanes issue the
 //    MMAs, each into its pair of accumulators of 128 columns.  They meet at mbarriers only: a half of the columns is made while the epilogue
@@ -1138,6 +1139,24 @@ inline void describe(Params& p, const float* x, const float* y, int64_t n, int64
   p.never = ~0u;
   // relative error bound of one score: the split leaves 3 * 2^-22 of |x||y|, the rest is the sums of up to 13 MMAs of 16 products
   p.eps = d <= 32 ? 1.0f / 65536.0f : 1.0f / 32768.0f;
+}
+
+// Kernels::of<C, NB>() for k centres of d dimensions.
+template <typename Kernels>
+auto kernel_for(int64_t k, int64_t d) {
+#define F2C_CHUNKS(C) \
+  case C: return k <= 128 ? Kernels::template of<C, 4>() : Kernels::template of<C, 8>()
+  switch ((d + 7) / 8) {
+    F2C_CHUNKS(1);
+    F2C_CHUNKS(2);
+    F2C_CHUNKS(3);
+    F2C_CHUNKS(4);
+    F2C_CHUNKS(5);
+    F2C_CHUNKS(6);
+    F2C_CHUNKS(7);
+    default: return k <= 128 ? Kernels::template of<8, 4>() : Kernels::template of<8, 8>();
+  }
+#undef F2C_CHUNKS
 }
 
 }  // namespace tc

@@ -100,7 +100,7 @@ def test_tensor_core_assignment_equals_exact_fp32_kernel(capi, oracle, metric, n
         undecided = ops.kmeans_assign.last_undecided
         exact = ops.kmeans_assign(x, centers, metric, scorer="exact")
         assert torch.equal(tc, exact), (metric, n, k, d, int((tc != exact).sum()))
-        # the split product (3 x tf32 up to d = 32, 3 x bf16 up to d = 64) decides almost everything itself
+        # the split product (three products of f16 pairs) decides almost everything itself
         # (a duplicated centre makes every point that prefers it an exact tie: about 1/k of the points)
         assert undecided <= (0.02 if d <= 32 else 0.05) * n + 8 + (3.0 * n / k if centers is c2 else 0)
         if centers is c:
@@ -202,7 +202,7 @@ def test_a_lost_wait_leaves_the_exact_labels_and_sums(capi, n, k, d):
 
 
 def test_iterations_in_a_row_equal_iterations_one_by_one(capi):
-    """Eight iterations queued at once, whose kernels start while the one before still runs, and eight with the device idle between."""
+    """Eight iterations queued at once, which one kernel makes, and eight with the device idle between."""
     g = torch.Generator(device="cuda").manual_seed(0)
     for n, d, k in ((5000, 16, 64), (30000, 8, 256), (20000, 64, 200)):
         x = torch.randn(n, d, generator=g, device="cuda")
