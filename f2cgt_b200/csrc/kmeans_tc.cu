@@ -14,17 +14,27 @@ __global__ void __launch_bounds__(kThreads, 1) kmeans_tc_kernel(const __grid_con
   run<C, NB, NO_WAITS>(p);
 }
 
+// (All of this is the file's own, as `static` says: a type of that name, and a dispatch alike, is in the other file too.)
 struct Kernel {
   void (*kern)(const Params);
   size_t smem;
 };
-struct Kernels {
-  template <int C, int NB>
-  static Kernel of() { return {kmeans_tc_kernel<C, NB>, Ring<C, NB>::bytes}; }
-};
+template <int C>
+static Kernel kernel_for(int64_t k) {
+  return k <= 128 ? Kernel{kmeans_tc_kernel<C, 4>, Ring<C, 4>::bytes} : Kernel{kmeans_tc_kernel<C, 8>, Ring<C, 8>::bytes};
+}
 static Kernel kernel_for(int64_t k, int64_t d, bool no_waits) {
-  if (no_waits) return {kmeans_tc_kernel<8, 8, true>, Ring<8, 8>::bytes};  // for any number of dimensions
-  return kernel_for<Kernels>(k, d);
+  if (no_waits) return Kernel{kmeans_tc_kernel<8, 8, true>, Ring<8, 8>::bytes};  // for any number of dimensions
+  switch ((d + 7) / 8) {
+    case 1: return kernel_for<1>(k);
+    case 2: return kernel_for<2>(k);
+    case 3: return kernel_for<3>(k);
+    case 4: return kernel_for<4>(k);
+    case 5: return kernel_for<5>(k);
+    case 6: return kernel_for<6>(k);
+    case 7: return kernel_for<7>(k);
+    default: return kernel_for<8>(k);
+  }
 }
 
 }  // namespace tc

@@ -1141,23 +1141,5 @@ inline void describe(Params& p, const float* x, const float* y, int64_t n, int64
   p.eps = d <= 32 ? 1.0f / 65536.0f : 1.0f / 32768.0f;
 }
 
-// Kernels::of<C, NB>() for k centres of d dimensions.
-template <typename Kernels>
-auto kernel_for(int64_t k, int64_t d) {
-#define F2C_CHUNKS(C) \
-  case C: return k <= 128 ? Kernels::template of<C, 4>() : Kernels::template of<C, 8>()
-  switch ((d + 7) / 8) {
-    F2C_CHUNKS(1);
-    F2C_CHUNKS(2);
-    F2C_CHUNKS(3);
-    F2C_CHUNKS(4);
-    F2C_CHUNKS(5);
-    F2C_CHUNKS(6);
-    F2C_CHUNKS(7);
-    default: return k <= 128 ? Kernels::template of<8, 4>() : Kernels::template of<8, 8>();
-  }
-#undef F2C_CHUNKS
-}
-
 }  // namespace tc
 }  // namespace f2c
