@@ -966,11 +966,11 @@ __device__ __forceinline__ void run(const P& p) {
             const int row = (warp & 3) * 32 + q * L::ROWS + chunk_l * L::R + row_l;
             const float floor = 2.0f * cmax * (l2 ? fmaxf(0x1p-19f * own_factor, 0x1p-126f) : 0x1p-21f);  // f16 at its lower end, and the norm term
             const float unscale = __int_as_float((254 << 23) - __float_as_int(own_factor)) * power2f(e_y);  // 1 / all that x was multiplied with
-            const float length2 = own_sum * unscale * unscale;  // |x|^2
-            // INFINITY for NaN, for a point whose |x|^2 is more than fp32 holds, and for one whose |x|^2 is next to nothing under the cosine metric (the
-            // exact scorer takes 0 for it, all distances are 1 then): the exact scorer's distance says so
-            // (-1 for a row of zeros under the cosine metric: all its distances are 1, its label is 0)
-            const float bound = !l2 && own_sum == 0.0f ? -1.0f : length2 < INFINITY && (l2 || length2 >= kTiny) ? fminf(fmaf(eps, sqrt_approx(own_sum), floor), INFINITY) : INFINITY;
+            // INFINITY for NaN, for a point whose |x|^2 is more than fp32 holds, and, cosine, for one whose values are all below 2^-51, as kTiny is for
+            // centres (the exact scorer may take 0 for its length, all distances are 1 then): the exact scorer's distance says so
+            // (-1 for a row of zeros under the cosine metric: all its distances are 1, its label is 0).  (The length in the factor's place: 175 us
+            // instead of 162 for 2,449,029 x 32.)
+            const float bound = !l2 && own_factor > 0x1p50f ? (own_sum == 0.0f ? -1.0f : INFINITY) : own_sum * unscale * unscale < INFINITY ? fminf(fmaf(eps, sqrt_approx(own_sum), floor), INFINITY) : INFINITY;
             if (chunk_l < L::READS) {
               bounds[(t & (kBoundRing - 1)) * kTileM + row] = bound;
               if (l2) {
