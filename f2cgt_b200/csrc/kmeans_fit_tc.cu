@@ -3,8 +3,8 @@
 // before, each near its own latency (a set-up, a list of undecided points that is usually a few hundred long, a last CTA that replaced the
 // centres alone); the CTAs keep their TMEM and barriers, score their own undecided points, and replace a share of the centres each.
 //
-// Measured, one iteration (before: three kernels): 149,000 x 32, 256 centres 54 -> 31 us, x 8 30 -> 24, x 64 78 -> 59; 30,000 x 32 28 -> 20;
-// 2,449,029 x 32 577 -> 277.  Of the 31 us the assignment takes 10, the centres' way into shared memory 2.5, the two barriers with what CTAs
+// Measured, one iteration (before: three kernels): 149,000 x 32, 256 centres 54 -> 32 us, x 8 30 -> 24, x 64 78 -> 56; 30,000 x 32 28 -> 21;
+// 2,449,029 x 32 577 -> 287.  Of the 32 us the assignment takes 10, the centres' way into shared memory 2.5, the two barriers with what CTAs
 // wait for one another 8 (those with undecided points come 4 later than the rest).
 #include "kmeans_tc.cuh"
 
@@ -61,7 +61,7 @@ int kmeans_fit_tc(const float* x, float* centers, int64_t n, int64_t k, int64_t 
   if (grid > kFitMaxCtas) grid = kFitMaxCtas;
   void* args[] = {(void*)&p};
   // A launch takes every SM, registers and all, so that kernels of other streams wait for its end: it has as many iterations as take about a
-  // millisecond, one at least (2,449,029 x 32: 3 of 280 us; 149,000 x 32, 32 us each: all that are queued at a time).
+  // millisecond, one at least (2,449,029 x 32: 3 of 287 us; 149,000 x 32, 32 us each: all that are queued at a time).
   const int64_t most = (1ll << 28) / (n * (d < 16 ? 16 : d));
   while (iterations > 0) {
     p.iterations = most < 1 ? 1 : most < iterations ? (int)most : iterations;

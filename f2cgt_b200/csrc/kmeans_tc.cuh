@@ -26,13 +26,13 @@
 //    MMAs, each into its pair of accumulators of 128 columns.  They meet at mbarriers only: a half of the columns is made while the epilogue
 //    reads another, and a group ends a tile while the two others read theirs.
 //    What bounds it: up to 16 dimensions the maxima (one per point and centre and direction, two cycles per three-operand instruction: ALU
-//    pipe 66 % busy) and the latency of the chain accumulator free - MMAs - accumulator full; more dimensions: the producers' chains of
-//    dependent instructions, whatever memory and the tensor pipe do (without the splitting 147 us of 2,449,029 x 32 become 110).
-//    Measured, 2,449,029 points against 256 centres, whole call (before: sixteen warps that all loaded, split, waited and searched, one barrier
-//    per tile, 3 x tf32 or 3 x bf16, undecided points in a second kernel): 8 dimensions 153 -> 98 us, 16: 193 -> 112, 24: 227 -> 142, 32: 265
-//    -> 157, 64: 400 -> 305; 100 centres of 8 dimensions 118 -> 72, of 64: 357 -> 229.  Two epilogue groups instead of three: 8 dimensions 107.
-//    Few points: 5000 x 8 20 -> 11, 40,000 x 8 20 -> 12.5, 149,000 x 32 37 -> 26 (without the second kernel, its list and the clearing of it;
-//    with them 20, 18 and 28), 149,000 x 64 47 -> 48.
+//    pipe 68 % busy) and the latency of the chain accumulator free - MMAs - accumulator full; more dimensions: no unit alone (61 % at 32, 45 % at 64),
+//    warps wait for accumulators and rows and, at 64, for instructions.
+//    Measured, 2,449,029 points against 256 centres, whole call between two events, L2 flushed (before, calls in a row: sixteen warps that all
+//    loaded, split, waited and searched, one barrier per tile, 3 x tf32 or 3 x bf16, undecided points in a second kernel): 8 dimensions 153 ->
+//    107 us (102 in a row), 16: 193 -> 119, 24: 227 -> 148, 32: 265 -> 160, 64: 400 -> 318; 100 centres of 8 dimensions 118 -> 79, of 64: 357 ->
+//    240.  Two epilogue groups instead of three: 8 dimensions 9 more.  Few points: 5000 x 8 20 -> 14, 40,000 x 8 20 -> 16, 149,000 x 32 37 -> 31
+//    (the events alone are 3 of these); slower: 149,000 x 64 47 -> 48 in a row.
 //    Every wait on an mbarrier is bounded; on expiry an error code is recorded, no further wait is made and no copy started, and the exact
 //    scorer assigns all points of the CTA.  Rows that were asked for may still arrive then, so it works where no copy is aimed, over the operands.
 //    The copies and MMAs are waited for at the common exit, in front of the freeing of the TMEM.
